@@ -31,6 +31,7 @@
 #include "layered_gqa.cuh"
 #include "layered_recurrent.cuh"
 #include "layered_tc.cuh"
+#include "layered_stream.cuh"
 #include "st_header.h"
 
 using namespace xl;
@@ -753,11 +754,73 @@ static int launch_ltc(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& m
   return 0;
 }
 
+// launches a kernel in clusters of `cluster` CTAs along x, free to start before the kernel in front of it has finished (the kernel waits itself)
+template <typename... KA, typename... A>
+static int launch_early(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threads, size_t smem, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = e->stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim = {(unsigned)cluster, 1, 1};
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  CK(cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...));
+  e->launches++;
+  return 0;
+}
+
+// CTAs that share a column tile of a product with few rows by cutting K: doubled while two CTAs per SM are not exceeded and every CTA
+// keeps two K blocks or more (a CTA with less spends its time on the barriers)
+static int stream_splits(const xotb200_lm* e, int N, int K, int z) {
+  const long tiles = (long)cdiv(N, LTC_M) * z;
+  const int nkb = cdiv(K, LTC_BK);
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= 2L * e->sm_count && nkb >= 4 * s) s *= 2;
+  return s;
+}
+
+template <int NB, int EPI, typename TC>
+static int launch_stream(xotb200_lm* e, const CUtensorMap& mw, const CUtensorMap& mx, const LtcArgs& a, int splits, int z) {
+  auto kern = stream_gemm_kernel<NB, EPI, TC>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, lst_smem_bytes(NB)));
+  TRY(launch_early(e, kern, dim3(splits, cdiv(a.N, LTC_M), z), LST_THREADS, lst_smem_bytes(NB), splits, mw, mx, a));
+  e->tc_launches++;
+  return 0;
+}
+
+// rows of a row tile that holds M rows (M <= LST_MAX_ROWS)
+static int stream_tile_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
+
+// 1 = launched, 0 = the operands cannot be described to TMA.  Not NULL `tile_batch`: `batch` row tiles of stream_tile_rows(M) rows of A and C,
+// each with the B matrix its entry names.
+template <typename TC, int EPI>
+static int product_stream(xotb200_lm* e, const bf16* A, long lda, long a_batch, const bf16* B, long ldb, long b_batch, int b_count, TC* C, long ldc, long c_batch, int M,
+                          int N, int K, int batch, const EpiArgs& epi, const int* tile_batch = nullptr) {
+  const int nb = stream_tile_rows(M);
+  CUtensorMap mw, mx;
+  if (!make_map3(&mw, B, N, K, ldb, b_batch, b_count, LTC_M)) return 0;
+  if (!(tile_batch ? make_map3(&mx, A, (long)batch * nb, K, lda, 0, 1, nb) : make_map3(&mx, A, M, K, lda, a_batch, batch, nb))) return 0;
+  const LtcArgs a{M, N, K, C, ldc, c_batch, e->d_err, epi, tile_batch, 0};
+  const int s = stream_splits(e, N, K, batch);
+  if (nb == 16) TRY((launch_stream<16, EPI, TC>(e, mw, mx, a, s, batch)));
+  else if (nb == 32) TRY((launch_stream<32, EPI, TC>(e, mw, mx, a, s, batch)));
+  else if (nb == 64) TRY((launch_stream<64, EPI, TC>(e, mw, mx, a, s, batch)));
+  else TRY((launch_stream<128, EPI, TC>(e, mw, mx, a, s, batch)));
+  return 1;
+}
+
 // 1 = launched, 0 = not eligible (the caller falls back), < 0 = error
 template <typename TC, int EPI>
 static int product_tc(xotb200_lm* e, const bf16* A, long lda, long a_batch, const bf16* B, long ldb, long b_batch, TC* C, long ldc, long c_batch, int M,
                       int N, int K, int batch, const EpiArgs& epi) {
-  const int nt = (N > 64 && M > LTC_M) ? 128 : 64;   // one row tile: narrower column tiles, twice the CTAs streaming weights
+  // one row tile or less: bound by reading B (measured up to 128 rows: 24.8 -> 17.8 us a launch at 64 .. 128 rows, width 2048)
+  if (M <= LST_MAX_ROWS) return product_stream<TC, EPI>(e, A, lda, a_batch, B, ldb, b_batch, batch, C, ldc, c_batch, M, N, K, batch, epi);
+  const int nt = N > 64 ? 128 : 64;
   CUtensorMap ma, mb;
   if (!make_map3(&ma, A, M, K, lda, a_batch, batch, LTC_M) || !make_map3(&mb, B, N, K, ldb, b_batch, batch, nt)) return 0;
   LtcArgs a{M, N, K, C, ldc, c_batch, e->d_err, epi, nullptr, 0};
@@ -1379,8 +1442,10 @@ static int mamba2_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
 // Rows sorted by expert, every run padded to whole row tiles: C[p, :] = A[p, :] B[tile_batch[p / 128]]^T on the tensor cores.
 // 1 = launched, 0 = the operands cannot be described to TMA
 template <int EPI, typename TC>
-static int grouped_product(xotb200_lm* e, const bf16* A, long lda, const bf16* B, long ldb, long b_batch, int n_batch, TC* C, long ldc, int m_pad, int N,
+static int grouped_product(xotb200_lm* e, const bf16* A, long lda, const bf16* B, long ldb, long b_batch, int n_batch, TC* C, long ldc, int M, int m_pad, int N,
                            int K, const int* tile_batch, const EpiArgs& epi = EpiArgs{}) {
+  if (M <= LST_MAX_ROWS)
+    return product_stream<TC, EPI>(e, A, lda, 0, B, ldb, b_batch, n_batch, C, ldc, 0, M, N, K, m_pad / stream_tile_rows(M), epi, tile_batch);
   const int nt = N > 64 ? 128 : 64;
   CUtensorMap ma, mb;
   if (!make_map3(&ma, A, m_pad, K, lda, 0, 1, LTC_M) || !make_map3(&mb, B, N, K, ldb, b_batch, n_batch, nt)) return 0;
@@ -1440,23 +1505,25 @@ static int feed_forward(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
     e->launches++;
     if constexpr (std::is_same<T, bf16>::value) {
       if (grouped_ok) {
-        const int pairs = M * top, tiles = cdiv(pairs, LTC_M) + E, m_pad = tiles * LTC_M;
+        // few rows: an expert has at most M of them (a row picks an expert once), one row tile each, and the products stream the chosen experts
+        const int tile_rows = M <= LST_MAX_ROWS ? stream_tile_rows(M) : LTC_M;
+        const int pairs = M * top, tiles = M <= LST_MAX_ROWS ? std::min(E, pairs) : cdiv(pairs, LTC_M) + E, m_pad = tiles * tile_rows;
         REQUIRE(tiles <= e->moe_tiles_cap, "internal: the expert tile list was not sized for this step");
         int *counts = e->moe_plan, *starts = counts + e->max_experts, *cursor = starts + e->max_experts + 1, *place = cursor + e->max_experts,
             *tile_expert = place + (size_t)e->m_cap * e->max_top;
         bf16* xg = static_cast<bf16*>(e->moe_xg);
         moe_count_kernel<<<cdiv(pairs, 256), 256, 0, e->stream>>>(e->moe_ids, pairs, counts);
-        moe_plan_kernel<<<1, 256, 0, e->stream>>>(counts, E, LTC_M, tiles, starts, cursor, tile_expert);
+        moe_plan_kernel<<<1, 256, 0, e->stream>>>(counts, E, tile_rows, tiles, starts, cursor, tile_expert);
         moe_scatter_kernel<bf16><<<cdiv(pairs, 8), 256, 0, e->stream>>>(h, D, e->moe_ids, pairs, top, starts, cursor, place, xg);
         CK(cudaGetLastError());
         e->launches += 3;
         bf16* ma = static_cast<bf16*>(e->mact);
         int r = s.expert_act == XOTB200_LM_EXPERT_CLAMPED_GLU
-                    ? grouped_product<EPI_CLAMPED_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, m_pad, 2 * F, D, tile_expert, glu)
-                : gated ? grouped_product<EPI_SILU_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, m_pad, 2 * F, D, tile_expert, glu)
-                        : grouped_product<EPI_RELU2, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)F * D, E, ma, F, m_pad, F, D, tile_expert);
+                    ? grouped_product<EPI_CLAMPED_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, M, m_pad, 2 * F, D, tile_expert, glu)
+                : gated ? grouped_product<EPI_SILU_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, M, m_pad, 2 * F, D, tile_expert, glu)
+                        : grouped_product<EPI_RELU2, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)F * D, E, ma, F, M, m_pad, F, D, tile_expert);
         if (r < 0) return r;
-        if (r == 1) r = grouped_product<EPI_NONE, float>(e, ma, F, at<bf16>(e, L.w_edown), F, (long)D * F, E, e->moe_yg, D, m_pad, D, F, tile_expert);
+        if (r == 1) r = grouped_product<EPI_NONE, float>(e, ma, F, at<bf16>(e, L.w_edown), F, (long)D * F, E, e->moe_yg, D, M, m_pad, D, F, tile_expert);
         if (r < 0) return r;
         if (r == 1) {
           moe_combine_kernel<bf16><<<row_grid(e, M, D, 256), 256, 0, e->stream>>>(e->moe_yg, place, e->moe_wts, top, D, shared, yout, close);

@@ -1,0 +1,181 @@
+// layered_stream.cuh — products with few activation rows on the tensor cores: the weights are streamed once, at the memory's pace.
+//
+//   C[z][m, n] = sum_k A[z][m, k] * B[zb][n, k]      A, B bf16 and K-major, m < M <= NB, fp32 accumulation
+//
+// With few rows a product is bound by reading B.  The operands change places for it: 128 rows of B are the 128-row operand of
+// tcgen05.mma and the NB activation rows its N side, so a CTA's shared memory holds almost nothing but weights in flight and no tensor
+// time goes to empty rows.  K is cut over the CTAs of a cluster (gridDim.x = cluster size, up to 8), so that every matrix, also a narrow one, has
+// about two CTAs per SM streaming it; each CTA leaves its fp32 partial tile in its own shared memory, and after one cluster barrier CTA r
+// adds the rows m = r, r + S, ... of all S partial tiles in order through distributed shared memory (deterministic, no workspace, no second
+// launch) and applies the epilogue of layered_kernels.cuh to them.  Stores are whole 128-column runs of a row.
+//
+// A weight never depends on a kernel of the same step: the first stages' weight copies are issued BEFORE the kernel waits for the one in front
+// of it (griddepcontrol.wait), so a product that was launched early has its ring full when its rows arrive.
+// Grouped products (`tile_batch`): row tile t = blockIdx.z holds NB rows of one expert, tile_batch[t] names it (negative: empty).
+// Measured (B200, per launch in a decode step, 128 x 64 tiles of layered_tc.cuh -> this kernel): 8 rows, a 2048-wide model: 26.4 -> 12.5 us on average
+// over the projections, 28.5 -> 11.2 for the 8192 x 2048 up product, experts' gate/up (14 of 16 experts of 4096 x 2048) 64.7 -> 39.6 us = 5.9 TB/s; 16
+// rows, width 4096: 34.6 -> 21.6 us on average, 14336 x 4096 33.1 -> 29.4 us; 64 .. 128 rows, width 2048: 24.8 -> 17.8 us.  What is left above
+// the weights' time is the launch, the first copies' latency and the cluster's exchange (6 .. 8 us a launch).
+// Every mbarrier wait is bounded: one that expires sets *err, the CTA waits for its own copies, still takes part in the cluster's barriers,
+// frees its tensor memory and returns.
+#pragma once
+#include "layered_tc.cuh"
+
+namespace xl {
+
+constexpr int LST_THREADS = 256, LST_MAX_ROWS = 128;
+
+// ring stages that let two CTAs share an SM (its 227 KB): the weights in flight per SM are then 2 * stages * 16 KB
+__host__ __device__ constexpr int lst_stage_bytes(int nb) { return LTC_M * LTC_BK * 2 + nb * LTC_BK * 2; }
+__host__ __device__ constexpr int lst_stages(int nb) { return nb <= 16 ? 6 : nb <= 32 ? 5 : nb <= 64 ? 4 : 3; }
+__host__ __device__ constexpr int lst_smem_bytes(int nb) { return lst_stages(nb) * lst_stage_bytes(nb) + 1024 + 256; }
+static_assert(lst_smem_bytes(128) <= 112 * 1024 && lst_smem_bytes(16) <= 112 * 1024 && lst_smem_bytes(32) <= 112 * 1024 && lst_smem_bytes(64) <= 112 * 1024, "two CTAs per SM");
+static_assert(LTC_M * 128 * 4 <= lst_stages(128) * lst_stage_bytes(128), "the partial tile reuses the ring");
+
+// entry (m, n) of a float in the shared memory of CTA `rank` of the cluster
+__device__ __forceinline__ float ld_dsmem_f32(uint32_t addr, uint32_t rank) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(xb::mapa_shared(addr, rank)) : "memory");
+  return v;
+}
+
+template <int NB, int EPI, typename TC>
+__global__ void __launch_bounds__(LST_THREADS, 2)
+stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const LtcArgs a) {
+  extern __shared__ __align__(1024) uint8_t lst_smem[];
+  constexpr int NS = lst_stages(NB), STAGE = lst_stage_bytes(NB), W_BYTES = LTC_M * LTC_BK * 2;
+  constexpr int TMEM_COLS = NB < 32 ? 32 : NB;
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(lst_smem) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + NS * STAGE);
+  uint64_t* empty = full + NS;
+  uint64_t* tmem_full = empty + NS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+  float* part = reinterpret_cast<float*>(base);              // [NB][128] once the ring is done
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S = gridDim.x, split = blockIdx.x, n0 = blockIdx.y * LTC_M, z = blockIdx.z;
+  const int nkb = (a.K + LTC_BK - 1) / LTC_BK, per = (nkb + S - 1) / S;
+  const int kb0 = min(nkb, split * per), nk = min(nkb, kb0 + per) - kb0;
+  pdl_launch_dependents();
+  int zb = z, mx = 0, zx = z;
+  if (a.tile_batch) {                                        // which expert this row tile belongs to: known once the plan has been made
+    pdl_wait();
+    zb = a.tile_batch[z];
+    mx = z * NB;
+    zx = 0;
+    if (zb < 0) return;                                      // an empty tile: the whole cluster leaves before anything is set up
+  }
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < NS; ++i) { xb::mbar_init(&full[i], 1); xb::mbar_init(&empty[i], 1); }
+    xb::mbar_init(tmem_full, 1);
+    xb::fence_mbar_init();
+  }
+  if (warp == 2) xb::tmem_alloc(tmem_slot, TMEM_COLS);
+  xb::tc_fence_before();
+  __syncthreads();
+  xb::tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ===== TMA producer =====
+      const int pre = min(NS, nk);
+      for (int i = 0; i < pre; ++i) {
+        xb::mbar_expect_tx(&full[i], STAGE);
+        xb::tma_load_3d(base + (size_t)i * STAGE, &tmW, (kb0 + i) * LTC_BK, n0, zb, &full[i]);
+      }
+      pdl_wait();
+      for (int i = 0; i < pre; ++i) xb::tma_load_3d(base + (size_t)i * STAGE + W_BYTES, &tmX, (kb0 + i) * LTC_BK, mx, zx, &full[i]);
+      int issued = pre;
+      bool ok = true;
+      for (int i = pre; i < nk && ok; ++i) {
+        const int st = i % NS;
+        ok = ltc_wait(&empty[st], (((unsigned)i / NS) & 1u) ^ 1u, a.err);
+        if (!ok) break;
+        uint8_t* sw = base + (size_t)st * STAGE;
+        xb::mbar_expect_tx(&full[st], STAGE);
+        xb::tma_load_3d(sw, &tmW, (kb0 + i) * LTC_BK, n0, zb, &full[st]);
+        xb::tma_load_3d(sw + W_BYTES, &tmX, (kb0 + i) * LTC_BK, mx, zx, &full[st]);
+        issued = i + 1;
+      }
+      if (!ok)   // gave up: let the copies still in flight land before the CTA's shared memory goes away
+        for (int i = max(0, issued - NS); i < issued; ++i) ltc_wait(&full[i % NS], ((unsigned)i / NS) & 1u, a.err);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // ===== MMA issuer =====
+      constexpr uint32_t idesc = ltc_idesc(LTC_M, NB);
+      bool ok = true;
+      for (int i = 0; i < nk; ++i) {
+        const int st = i % NS;
+        ok = ltc_wait(&full[st], ((unsigned)i / NS) & 1u, a.err);
+        if (!ok) break;
+        xb::tc_fence_after();
+        const uint32_t sw = xb::smem_u32(base + (size_t)st * STAGE), sx = sw + W_BYTES;
+#pragma unroll
+        for (int k = 0; k < LTC_BK / 16; ++k)
+          xb::umma_bf16(tmem_base, xb::umma_desc_sw128(sw + k * 32), xb::umma_desc_sw128(sx + k * 32), idesc, (i | k) != 0 ? 1u : 0u);
+        xb::umma_commit(&empty[st]);
+      }
+      if (ok && nk > 0) xb::umma_commit(tmem_full);
+    }
+  } else if (warp >= 4) {
+    // ===== accumulator -> shared memory: warp q holds weight rows 32q .. 32q+31 =====
+    const int q = warp - 4;
+    if (nk > 0 && ltc_wait(tmem_full, 0, a.err)) {
+      xb::tc_fence_after();
+#pragma unroll 1
+      for (int c0 = 0; c0 < NB && c0 < a.M; c0 += 16) {
+        uint32_t v[16];
+        xb::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) part[(c0 + j) * LTC_M + q * 32 + lane] = __uint_as_float(v[j]);
+      }
+    } else if (nk == 0) {
+      for (int c = 0; c < NB; ++c) part[c * LTC_M + q * 32 + lane] = 0.f;
+    }
+  }
+  xb::tc_fence_before();
+  __syncthreads();
+  if (S > 1) xb::cluster_sync_all();
+  pdl_wait();                                                // every thread: the stores below follow all earlier kernels
+  float ap = 0.f, aq = 0.f;
+  if (EPI == EPI_XIELU) {
+    const __nv_bfloat16* raw = static_cast<const __nv_bfloat16*>(a.epi.p);
+    ap = softplusf_(__bfloat162float(raw[0]));
+    aq = 0.5f + softplusf_(__bfloat162float(raw[1]));
+  }
+  const uint32_t part_addr = xb::smem_u32(part);
+  auto total = [&](int m, int c) {                           // sum of the cluster's partial tiles, in the order of K
+    if (S == 1) return part[m * LTC_M + c];
+    float v = 0.f;
+    for (int r = 0; r < S; ++r) v += ld_dsmem_f32(part_addr + (uint32_t)(m * LTC_M + c) * 4, r);
+    return v;
+  };
+  TC* C = static_cast<TC*>(a.C) + (a.tile_batch ? (size_t)mx * a.ldc : (size_t)z * a.c_batch);
+  constexpr int W = epi_is_glu(EPI) ? LTC_M / 2 : LTC_M;     // outputs per row of the tile
+  for (int i = threadIdx.x; i < ((a.M - split + S - 1) / S) * W; i += LST_THREADS) {
+    const int m = split + i / W * S, c = i % W;
+    if constexpr (epi_is_glu(EPI)) {                         // 8 gate rows, then their 8 up rows
+      const int cg = c / 8 * 16 + c % 8;
+      if (n0 + cg + 8 < a.N) ltc_store<TC>(C + (size_t)m * a.ldc + (n0 >> 1) + c, glu_f<EPI>(total(m, cg), total(m, cg + 8), a.epi));
+    } else if (n0 + c < a.N) {
+      float v = total(m, c);
+      if constexpr (EPI == EPI_CLOSE) {
+        stream_close<__nv_bfloat16>(a.epi, m, n0 + c, v);
+      } else {
+        if (EPI == EPI_RELU2) { v = fmaxf(v, 0.f); v *= v; }
+        if (EPI == EPI_XIELU) v = xielu_f(v, ap, aq);
+        if (EPI == EPI_GELU) v = gelu_erf_f(v);
+        ltc_store<TC>(C + (size_t)m * a.ldc + n0 + c, v);
+      }
+    }
+  }
+  xb::tc_fence_after();
+  if (S > 1) {
+    __syncthreads();
+    xb::cluster_sync_all();                                  // nobody's shared memory goes away while a peer reads it
+  }
+  if (warp == 2) xb::tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+}  // namespace xl
