@@ -1,0 +1,47 @@
+"""The row kernels of the layered engine that keep a row in registers (group norm, layer norm and RMS norm that close a sublayer, embedding
+rows, arg-max): widths at the edges of their pieces (one, two or four per thread, rows that end inside a warp), against the float64 oracles."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from tests import bufulorn_oracle as bo, tunavik_oracle as to, zokuvik_oracle as zo
+from tests import bufulorn_util as bu, layered_util as lu, tunavik_util as tu
+
+DTYPES = ["float32", "bfloat16"]
+
+
+def run(cfg, w, oracle, dtype, vocab):
+  eng = lu.make_engine(cfg, w, dtype)
+  toks = lu.rand_tokens(vocab, 9, 3)
+  got = lu.run_cut(eng, 0, toks, [6, 1])
+  ref, _ = oracle(cfg, w, toks)
+  assert lu.row_err(got, ref) < lu.TOL[dtype]
+  eng.clear_request(0)
+  lg, best = eng.step([0], [toks])                             # both results of one step
+  assert int(best[0]) == int(np.argmax(lg[0]))
+  eng.clear_request(0)
+  none, alone = eng.step([0], [toks], logits=False)            # the arg-max without the logits
+  assert none is None and int(alone[0]) == int(best[0])
+  eng.close()
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width,groups", [(128, 1), (1024, 4), (1152, 3), (2048, 16), (8320, 5), (192, 1)])   # 192: parts that are no whole pieces
+def test_grouped_norms(width, groups, dtype):
+  cfg = lu.config([lu.attn(heads=2, dim=8, rot_dim=4, vdim=8, kv_rank=16, q_rank=8, ff=24)], width=width, vocab=67, groups=groups)
+  run(cfg, zo.random_weights(cfg, 3), lu.oracle_logits, dtype, 67)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [8, 132, 1024, 1028, 4100, 8196, 70])                                        # 70: not whole pieces of four
+def test_layer_norms(width, dtype):
+  cfg = bu.config([bu.attention(heads=2, kv_heads=1, dim=8, vdim=8, mlp=bu.dense(24))], width=width, vocab=4099, max_positions=32)
+  run(cfg, bo.random_weights(cfg, 4), bu.oracle_logits, dtype, 4099)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [132, 1028, 8196])
+def test_rms_norms(width, dtype):
+  cfg = tu.config([tu.attention(heads=2, kv_heads=1, dim=8, vdim=8)], width=width, vocab=66)
+  run(cfg, to.random_weights(cfg, 5), tu.oracle_logits, dtype, 66)

@@ -1617,6 +1617,17 @@ static void finish_logits(xotb200_lm* e, int n_want) {
   e->launches++;
 }
 
+// How a block holds a row of D entries in registers: pieces of four per thread (nv of them, 1, 2 or 4; 0 = the row is not whole pieces or too long,
+// the kernels that walk it take it).  One piece per thread while the block stays at 256 threads, then two: a single row is over soonest with
+// few warps at the block's barriers and two loads of everything in flight per thread.  (1 row: width 1024 grouped norm 6.2 -> 3.9 us a launch in a step.)
+struct RowShape { int nv, threads; };
+static RowShape row_shape(int D) {
+  if (D % 4 != 0) return {0, 0};
+  const int nv = D <= 1024 ? 1 : D <= 8192 ? 2 : D <= 16384 ? 4 : 0;
+  return {nv, nv ? cdiv(D, 4 * nv * 32) * 32 : 0};
+}
+static int embed_threads(int D) { return std::min(512, cdiv(D, 4 * 32) * 32); }
+
 // layers of the form x += norm(sublayer(x)): the sublayer reads the stream itself (its T copy h); a layer norm (weight and bias)
 // or an RMS norm (weight stored around zero) closes it and adds the bias of the mixer's output projection on the way
 template <typename T>
@@ -1630,13 +1641,20 @@ static int run_layers_post(xotb200_lm* e, const StepPlan& sp, int n_want) {
   auto kern_rms = residual_rmsnorm_kernel<T>;
   TRY(opt_in_smem(kern, (size_t)D * 4));
   TRY(opt_in_smem(kern_rms, (size_t)D * 4));
-  auto close = [&](size_t w, size_t b, const T* y_bias) -> int {
-    if (rms) kern_rms<<<M, nt, (size_t)D * 4, e->stream>>>(e->x, e->y, y_bias, at<T>(e, w), 1.0f, h, nullptr, D, eps);
-    else kern<<<M, nt, (size_t)D * 4, e->stream>>>(e->x, e->y, y_bias, at<T>(e, w), at<T>(e, b), h, nullptr, D, eps);
+  const RowShape rs = row_shape(D);
+  // closes a sublayer (y), or norms gathered rows of the stream (rows)
+  auto norm_rows = [&](const float* y, const T* y_bias, size_t w, size_t b, T* out, const int* rows, int n) -> int {
+    if (rs.nv) {
+      auto vk = rms ? (rs.nv == 1 ? residual_norm_vec_kernel<T, 1, true> : rs.nv == 2 ? residual_norm_vec_kernel<T, 2, true> : residual_norm_vec_kernel<T, 4, true>)
+                    : (rs.nv == 1 ? residual_norm_vec_kernel<T, 1, false> : rs.nv == 2 ? residual_norm_vec_kernel<T, 2, false> : residual_norm_vec_kernel<T, 4, false>);
+      vk<<<n, rs.threads, 0, e->stream>>>(e->x, y, y_bias, at<T>(e, w), rms ? nullptr : at<T>(e, b), 1.0f, out, rows, D, eps);
+    } else if (rms) kern_rms<<<n, nt, (size_t)D * 4, e->stream>>>(e->x, y, y_bias, at<T>(e, w), 1.0f, out, rows, D, eps);
+    else kern<<<n, nt, (size_t)D * 4, e->stream>>>(e->x, y, y_bias, at<T>(e, w), at<T>(e, b), out, rows, D, eps);
     CK(cudaGetLastError());
     e->launches++;
     return 0;
   };
+  auto close = [&](size_t w, size_t b, const T* y_bias) -> int { return norm_rows(e->y, y_bias, w, b, h, nullptr, M); };
   if (e->first) {
     if (e->cfg.pos_sinusoid || e->cfg.embed_norm) {
       auto ek = embed_sinusoid_rows_kernel<T>;
@@ -1644,8 +1662,9 @@ static int run_layers_post(xotb200_lm* e, const StepPlan& sp, int n_want) {
       ek<<<M, nt, (size_t)D * 4, e->stream>>>(at<T>(e, e->embed), e->cfg.max_positions > 0 ? at<T>(e, e->pos_table) : nullptr, e->pos_freqs, sp.tokens, sp.row_pos,
                                               e->cfg.embed_norm ? at<T>(e, e->embed_norm) : nullptr, 1.0f, eps, e->x, h, D);
     } else {
-      embed_pos_rows_kernel<T><<<M, 128, 0, e->stream>>>(at<T>(e, e->embed), e->cfg.max_positions > 0 ? at<T>(e, e->pos_table) : nullptr, sp.tokens, sp.row_pos,
-                                                         e->x, h, D);
+      auto ek = D % 4 == 0 ? embed_pos_rows_kernel<T, 4> : embed_pos_rows_kernel<T, 1>;
+      ek<<<M, D % 4 == 0 ? embed_threads(D) : 128, 0, e->stream>>>(at<T>(e, e->embed), e->cfg.max_positions > 0 ? at<T>(e, e->pos_table) : nullptr, sp.tokens, sp.row_pos,
+                                                                   e->x, h, D);
     }
   } else {
     cast_rows_kernel<T><<<std::min(4096, cdiv((long)M * D, 256)), 256, 0, e->stream>>>(e->x, h, (size_t)M * D);
@@ -1665,10 +1684,7 @@ static int run_layers_post(xotb200_lm* e, const StepPlan& sp, int n_want) {
   if (e->trace) e->trace_floats = e->layers.size() * (size_t)M * D;
   if (e->last && n_want > 0) {
     T* hw = static_cast<T*>(e->hw);
-    if (rms) kern_rms<<<n_want, nt, (size_t)D * 4, e->stream>>>(e->x, nullptr, nullptr, at<T>(e, e->final_norm), 1.0f, hw, sp.want, D, eps);
-    else kern<<<n_want, nt, (size_t)D * 4, e->stream>>>(e->x, nullptr, nullptr, at<T>(e, e->final_norm), at<T>(e, e->final_norm_b), hw, sp.want, D, eps);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(norm_rows(nullptr, nullptr, e->final_norm, e->final_norm_b, hw, sp.want, n_want));
     TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
     finish_logits(e, n_want);
     CK(cudaGetLastError());
@@ -1882,18 +1898,29 @@ static int run_layers(xotb200_lm* e, const StepPlan& sp, int n_want) {
   T* h = static_cast<T*>(e->h);
   const float* pend_y = nullptr;
   const T* pend_w = nullptr;
+  const RowShape rs = (D / G) % 128 == 0 ? row_shape(D) : RowShape{0, 0};   // parts of whole 128-entry pieces: the row stays in registers
+  auto norm_rows = [&](const float* y, const T* w_post, const T* w_pre, T* out, const int* rows, int n) -> int {
+    if (rs.nv) {
+      auto vk = rs.nv == 1 ? residual_groupnorm_vec_kernel<T, 1> : rs.nv == 2 ? residual_groupnorm_vec_kernel<T, 2> : residual_groupnorm_vec_kernel<T, 4>;
+      vk<<<n, rs.threads, 0, e->stream>>>(e->x, y, w_post, w_pre, out, rows, D, G, eps);
+    } else {
+      residual_groupnorm_kernel<T><<<n, norm_threads(D, G), 0, e->stream>>>(e->x, y, w_post, w_pre, out, rows, D, G, eps);
+    }
+    CK(cudaGetLastError());
+    e->launches++;
+    return 0;
+  };
   // x += groupnorm(pending sublayer output) * its post-norm weight;  h = groupnorm(x) * w_pre  (either half may be absent)
   auto open = [&](const T* w_pre) -> int {
     if (!pend_y && !w_pre) return 0;
-    residual_groupnorm_kernel<T><<<M, norm_threads(D, G), 0, e->stream>>>(e->x, pend_y, pend_w, w_pre, w_pre ? h : nullptr, nullptr, D, G, eps);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(norm_rows(pend_y, pend_w, w_pre, w_pre ? h : nullptr, nullptr, M));
     pend_y = nullptr;
     pend_w = nullptr;
     return 0;
   };
   if (e->first) {
-    embed_rows_kernel<T><<<M, 128, 0, e->stream>>>(at<T>(e, e->embed), sp.tokens, e->x, D);
+    auto ek = D % 4 == 0 ? embed_rows_kernel<T, 4> : embed_rows_kernel<T, 1>;
+    ek<<<M, D % 4 == 0 ? embed_threads(D) : 128, 0, e->stream>>>(at<T>(e, e->embed), sp.tokens, e->x, D);
     CK(cudaGetLastError());
     e->launches++;
   }
@@ -1918,9 +1945,7 @@ static int run_layers(xotb200_lm* e, const StepPlan& sp, int n_want) {
   if (e->trace) e->trace_floats = e->layers.size() * (size_t)M * D;
   if (e->last && n_want > 0) {
     T* hw = static_cast<T*>(e->hw);
-    residual_groupnorm_kernel<T><<<n_want, norm_threads(D, G), 0, e->stream>>>(e->x, nullptr, nullptr, at<T>(e, e->final_norm), hw, sp.want, D, G, eps);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(norm_rows(nullptr, nullptr, at<T>(e, e->final_norm), hw, sp.want, n_want));
     TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
     finish_logits(e, n_want);
     CK(cudaGetLastError());
