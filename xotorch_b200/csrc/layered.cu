@@ -184,7 +184,6 @@ struct xotb200_lm {
   float* part = nullptr;                               // key-run partial results of the absorbed attention kernel
   size_t part_cap = 0;
   int max_w = 0;                                       // widest cached row (kv_rank + rot_dim)
-  int* d_argmax = nullptr;
   float* h_out = nullptr;                              // pinned staging for results
   size_t h_out_cap = 0;
   int max_in = 0, max_q = 0, max_qfull = 0, max_qr = 0, max_hdn = 0, max_olat = 0, max_oh = 0, max_ff = 0, max_hd = 0, max_lr = 0;
@@ -192,6 +191,7 @@ struct xotb200_lm {
   float* trace_buf = nullptr;
   size_t trace_floats = 0, trace_cap = 0;
   int gemm_mode = 0;
+  bool early = false;                                  // this step's kernels may start before the one in front has finished (launch_early)
   bool graphs_on = true;                               // decode steps are replayed from CUDA graphs
   std::map<std::array<long, 5>, GraphSlot> graphs;
   int64_t graph_replays = 0;
@@ -741,20 +741,10 @@ static bool make_map3(CUtensorMap* m, const void* ptr, long rows, long K, long l
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int NT, int EPI, typename TC>
-static int launch_ltc(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& mb, const LtcArgs& a, int batch) {
-  constexpr int NS = 3;
-  auto kern = ltc_gemm_kernel<NT, EPI, NS, TC>;
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ltc_smem_bytes(NT, NS)));
-  const dim3 grid = a.cols_first ? dim3(cdiv(a.N, NT), cdiv(a.M, LTC_M), batch) : dim3(cdiv(a.M, LTC_M), cdiv(a.N, NT), batch);
-  kern<<<grid, LTC_THREADS, ltc_smem_bytes(NT, NS), e->stream>>>(ma, mb, a);
-  CK(cudaGetLastError());
-  e->launches++;
-  e->tc_launches++;
-  return 0;
-}
-
-// launches a kernel in clusters of `cluster` CTAs along x, free to start before the kernel in front of it has finished (the kernel waits itself)
+// Launches a kernel in clusters of `cluster` CTAs along x.  In a step of few rows (e->early) it may start before the kernel in front of it has
+// finished: it waits itself (pdl_wait), its launch and what it loads ahead of that are hidden.  Such a step is a chain of some forty short
+// kernels, and the launches are most of it (one request, width 1024: 5979 -> 4913 us for 25 steps).  With many rows the kernels are long, and
+// blocks that were placed early, around a kernel still running, are spread worse over the SMs (1024 rows, width 4096: 2503 -> 2588 us).
 template <typename... KA, typename... A>
 static int launch_early(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threads, size_t smem, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -763,14 +753,37 @@ static int launch_early(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threa
   cfg.dynamicSmemBytes = smem;
   cfg.stream = e->stream;
   cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim = {(unsigned)cluster, 1, 1};
   cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cfg.numAttrs = 0;
+  if (e->early) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs++].val.clusterDim = {(unsigned)cluster, 1, 1};
+  }
   CK(cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...));
   e->launches++;
+  return 0;
+}
+// the ordinary way: kernels whose blocks compute for long (about one to an SM) and so depend on where they are placed
+template <typename... KA, typename... A>
+static int launch_late(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threads, size_t smem, A&&... args) {
+  kern<<<grid, threads, smem, e->stream>>>(static_cast<KA>(args)...);
+  CK(cudaGetLastError());
+  e->launches++;
+  return 0;
+}
+
+template <int NT, int EPI, typename TC>
+static int launch_ltc(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& mb, const LtcArgs& a, int batch) {
+  constexpr int NS = 3;
+  auto kern = ltc_gemm_kernel<NT, EPI, NS, TC>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ltc_smem_bytes(NT, NS)));
+  const dim3 grid = a.cols_first ? dim3(cdiv(a.N, NT), cdiv(a.M, LTC_M), batch) : dim3(cdiv(a.M, LTC_M), cdiv(a.N, NT), batch);
+  TRY(launch_late(e, kern, grid, LTC_THREADS, ltc_smem_bytes(NT, NS), ma, mb, a));
+  e->tc_launches++;
   return 0;
 }
 
@@ -851,8 +864,7 @@ static int product(xotb200_lm* e, const TA* A, long lda, long a_batch, const TB*
   do {                                                                                                                         \
     auto kern = gemv_rows_kernel<TA, TB, TC, EPI, MR>;                                                                         \
     TRY(opt_in_smem(kern, sm));                                                                                                \
-    kern<<<dim3(blocks, 1, batch), 256, sm, e->stream>>>(A, lda, a_batch, B, sbn, b_batch, C, ldc, c_batch, M, N, K, wsplit,    \
-                                                         epi);                                                                \
+    TRY(launch_early(e, kern, dim3(blocks, 1, batch), 256, sm, 1, A, lda, a_batch, B, sbn, b_batch, C, ldc, c_batch, M, N, K, wsplit, epi)); \
   } while (0)
     if (M == 1) LAUNCH_GEMV(1);
     else if (M == 2) LAUNCH_GEMV(2);
@@ -860,11 +872,8 @@ static int product(xotb200_lm* e, const TA* A, long lda, long a_batch, const TB*
     else LAUNCH_GEMV(8);
 #undef LAUNCH_GEMV
   } else {
-    gemm_tiled_kernel<TA, TB, TC, EPI><<<dim3(cdiv(N, 64), cdiv(M, 64), batch), 256, 0, e->stream>>>(A, lda, a_batch, B, sbn, sbk, b_batch, C, ldc,
-                                                                                                  c_batch, M, N, K, epi);
+    TRY(launch_late(e, gemm_tiled_kernel<TA, TB, TC, EPI>, dim3(cdiv(N, 64), cdiv(M, 64), batch), 256, 0, A, lda, a_batch, B, sbn, sbk, b_batch, C, ldc, c_batch, M, N, K, epi));
   }
-  CK(cudaGetLastError());
-  e->launches++;
   return 0;
 }
 
@@ -957,8 +966,7 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
     drop_graphs(e);
     const size_t w = (size_t)std::max(n_want, 16);
     TRY(regrow(e->hw, w * D * e->esz));
-    TRY(regrow(e->logits, w * e->cfg.vocab * 4));
-    TRY(regrow(e->d_argmax, w * 4));
+    TRY(regrow(e->logits, (w * ((size_t)e->cfg.vocab + 1) + 1) * 4));   // with the rows' argmax and the error word behind them
     e->want_cap = (int)w;
   }
   if (e->trace && e->trace_cap < (size_t)e->layers.size() * e->m_cap * D) {
@@ -1028,9 +1036,7 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   const float* qraw = e->proj;
   int q_ld = L.n_in;
   if (s.q_rank > 0) {
-    rmsnorm_cols_kernel<T><<<cdiv(M, 8), 256, 0, e->stream>>>(e->proj, L.n_in, L.c_q, s.q_rank, at<T>(e, L.dq_norm), static_cast<T*>(e->cqn), s.q_rank, M, eps);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(launch_early(e, rmsnorm_cols_kernel<T>, cdiv(M, 8), 256, 0, 1, e->proj, L.n_in, L.c_q, s.q_rank, at<T>(e, L.dq_norm), static_cast<T*>(e->cqn), s.q_rank, M, eps));
     TRY((product<T, T, float, 0>(e, static_cast<T*>(e->cqn), s.q_rank, 0, at<T>(e, L.uq), s.q_rank, 1, 0, e->qraw, HQ, 0, M, HQ, s.q_rank, 1)));
     qraw = e->qraw;
     q_ld = HQ;
@@ -1043,12 +1049,10 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
     if (f != sp.flash.end() && f->second.n_tiles > 0) fl = &f->second;
   }
   const bool absorbed = sp.any_short || !fl;
-  latent_prepare_kernel<T><<<cdiv((long)M * (H + 1), 8), 256, 0, e->stream>>>(qraw, q_ld, H, dn, dr, e->proj, L.n_in, L.c_kv, R, at<T>(e, L.dkv_norm), eps, L.freqs,
+  TRY(launch_early(e, latent_prepare_kernel<T>, cdiv((long)M * (H + 1), 8), 256, 0, 1, qraw, q_ld, H, dn, dr, e->proj, L.n_in, L.c_kv, R, at<T>(e, L.dkv_norm), eps, L.freqs,
                                                                               s.rot_dims, s.rot_layout, sp.row_slot, sp.row_pos, pg, static_cast<T*>(L.pool),
                                                                               absorbed ? static_cast<T*>(e->qn) : nullptr, e->qfull,
-                                                                              fl ? static_cast<bf16*>(e->q16) : nullptr, M);
-  CK(cudaGetLastError());
-  e->launches++;
+                                                                              fl ? static_cast<bf16*>(e->q16) : nullptr, M));
   const float* gate = s.out_gate ? e->proj : nullptr;
   const T* sink = s.sink ? at<T>(e, L.sink) : nullptr;
   if (absorbed) {
@@ -1070,20 +1074,16 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   do {                                                                                                                                          \
     auto kern = latent_attention_kernel<T, NACC>;                                                                                               \
     TRY(opt_in_smem(kern, smem));                                                                                                               \
-    kern<<<grid, nw * 32, smem, e->stream>>>(e->qfull, static_cast<const T*>(L.pool), pg, it.first, H, R, dr, s.scale, s.window, gate, L.n_in, \
-                                             L.c_g, sink, static_cast<T*>(e->olat), chunk, e->part, nbuf);                                      \
+    TRY(launch_early(e, kern, grid, nw * 32, smem, 1, e->qfull, static_cast<const T*>(L.pool), pg, it.first, H, R, dr, s.scale, s.window, gate, L.n_in, \
+                                             L.c_g, sink, static_cast<T*>(e->olat), chunk, e->part, nbuf));                                      \
   } while (0)
       if (R <= 64) LAUNCH_ATTN(2);
       else if (R <= 128) LAUNCH_ATTN(4);
       else if (R <= 256) LAUNCH_ATTN(8);
       else LAUNCH_ATTN(16);
 #undef LAUNCH_ATTN
-      CK(cudaGetLastError());
-      e->launches++;
       if (splits > 1) {
-        latent_attention_combine_kernel<T><<<dim3(it.second, cdiv(pairs, 8), it.second * cdiv(pairs, 8) < e->sm_count ? std::min(16, cdiv(R, 32)) : 1), 256, 0, e->stream>>>(e->part, it.first, H, R, splits, gate, L.n_in, L.c_g, sink, static_cast<T*>(e->olat));
-        CK(cudaGetLastError());
-        e->launches++;
+        TRY(launch_early(e, latent_attention_combine_kernel<T>, dim3(it.second, cdiv(pairs, 8), it.second * cdiv(pairs, 8) < e->sm_count ? std::min(16, cdiv(R, 32)) : 1), 256, 0, 1, e->part, it.first, H, R, splits, gate, L.n_in, L.c_g, sink, static_cast<T*>(e->olat)));
       }
     }
     // value expansion per head
@@ -1094,9 +1094,7 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
     if (fl) {
       // expanded form for the requests that bring many rows (it overwrites their rows of `oh`)
       bf16 *q16 = static_cast<bf16*>(e->q16), *cbuf = static_cast<bf16*>(e->cbuf), *knx = static_cast<bf16*>(e->knx), *vxx = static_cast<bf16*>(e->vxx);
-      latent_gather_kernel<bf16><<<dim3(cdiv(fl->max_keys, 8), fl->n_reqs), 256, 0, e->stream>>>(static_cast<const bf16*>(L.pool), pg, fl->reqs, R + dr, cbuf);
-      CK(cudaGetLastError());
-      e->launches++;
+      TRY(launch_early(e, latent_gather_kernel<bf16>, dim3(cdiv(fl->max_keys, 8), fl->n_reqs), 256, 0, 1, static_cast<const bf16*>(L.pool), pg, fl->reqs, R + dr, cbuf));
       TRY((product<bf16, bf16, bf16, 0>(e, cbuf, R + dr, 0, at<bf16>(e, L.uk_rows), R, 1, 0, knx, (long)H * dn, 0, fl->n_keys, H * dn, R, 1)));
       TRY((product<bf16, bf16, bf16, 0>(e, cbuf, R + dr, 0, at<bf16>(e, L.uv), R, 1, 0, vxx, (long)H * dv, 0, fl->n_keys, H * dv, R, 1)));
       const int dqp = (dn + dr + 15) & ~15, dvt = dv <= 64 ? 8 : 16;
@@ -1106,8 +1104,8 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   do {                                                                                                                                            \
     auto kern = KERN;                                                                                                                             \
     TRY(opt_in_smem(kern, SMEM));                                                                                                                 \
-    kern<<<grid, 128, SMEM, e->stream>>>(q16, knx, cbuf, vxx, fl->tiles, H, dn, dr, dv, R, s.scale, s.window, gate, L.n_in, L.c_g, sink,         \
-                                         static_cast<bf16*>(e->oh));                                                                              \
+    TRY(launch_late(e, kern, grid, 128, SMEM, q16, knx, cbuf, vxx, fl->tiles, H, dn, dr, dv, R, s.scale, s.window, gate, L.n_in, L.c_g, sink,         \
+                                         static_cast<bf16*>(e->oh)));                                                                              \
   } while (0)
       if (aligned) {   // whole 16-byte chunks: cp.async double buffering, ldmatrix fragments
         const size_t smem = ((size_t)3 * 64 * (dqp + 8) + (size_t)2 * 64 * (8 * dvt + 8)) * 2;
@@ -1119,8 +1117,6 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
         else LAUNCH_FLASH(latent_flash_kernel<16>, smem);
       }
 #undef LAUNCH_FLASH
-      CK(cudaGetLastError());
-      e->launches++;
       e->flash_launches++;
     }
   }
@@ -1137,10 +1133,8 @@ static int launch_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc 
   const dim3 grid(sp.n_seq * s.heads, cdiv(dv, warps * CPW));
   const int HD = s.heads * dk;
   const int vec4 = (dk % 4 == 0 && dv % 4 == 0 && HD % 4 == 0 && (ks.ld | ks.col | rs.ld | rs.col | vs.ld | vs.col) % 4 == 0) ? 1 : 0;
-  delta_rule_kernel<KPT, P, NC><<<grid, warps * 32, 0, e->stream>>>(ks, rs, vs, e->wlog, removal ? e->du : nullptr, removal ? e->dau : nullptr, sp.seqs, s.heads, dk, dv,
-                                                                    e->state + L.state_off, e->state_floats, e->oraw, vec4);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, delta_rule_kernel<KPT, P, NC>, grid, warps * 32, 0, 1, ks, rs, vs, e->wlog, removal ? e->du : nullptr, removal ? e->dau : nullptr, sp.seqs, s.heads, dk, dv,
+                                                                    e->state + L.state_off, e->state_floats, e->oraw, vec4));
   return 0;
 }
 // The recurrence is bound by the instructions one warp issues per token (measured: ~2.8 cycles each with one warp per scheduler):
@@ -1170,19 +1164,13 @@ static int delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   const int D = e->cfg.width, M = sp.M, HD = s.heads * s.dim;
   T* h = static_cast<T*>(e->h);
   TRY((product<T, T, float, 0>(e, h, D, 0, at<T>(e, L.w_in), D, 1, 0, e->proj, L.n_in, 0, M, L.n_in, D, 1)));
-  tanh_cols_kernel<T><<<cdiv((long)M * s.low_rank, 256), 256, 0, e->stream>>>(e->proj, L.n_in, L.c_w1, s.low_rank, static_cast<T*>(e->th), M);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, tanh_cols_kernel<T>, cdiv((long)M * s.low_rank, 256), 256, 0, 1, e->proj, L.n_in, L.c_w1, s.low_rank, static_cast<T*>(e->th), M));
   TRY((product<T, T, float, 0>(e, static_cast<T*>(e->th), s.low_rank, 0, at<T>(e, L.w2), s.low_rank, 1, 0, e->wlog, HD, 0, M, HD, s.low_rank, 1)));
-  delta_prepare_kernel<T><<<cdiv((long)M * s.heads, 8), 256, 0, e->stream>>>(e->proj, L.n_in, L.c_k, L.c_a, e->wlog, at<T>(e, L.w0), at<T>(e, L.a_b), e->du, e->dau,
-                                                                              s.heads, s.dim, M);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, delta_prepare_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->proj, L.n_in, L.c_k, L.c_a, e->wlog, at<T>(e, L.w0), at<T>(e, L.a_b), e->du, e->dau,
+                                                                              s.heads, s.dim, M));
   TRY(run_delta(e, L, sp, DeltaSrc{e->proj, L.n_in, L.c_k}, DeltaSrc{e->proj, L.n_in, L.c_r}, DeltaSrc{e->proj, L.n_in, L.c_v}, s.dim, s.vdim, true));
-  head_norm_gate_kernel<T><<<cdiv((long)M * s.heads, 8), 256, 0, e->stream>>>(e->oraw, nullptr, nullptr, at<T>(e, L.onorm), s.vdim, e->proj, L.n_in, L.c_g, 0,
-                                                                               static_cast<T*>(e->oh), s.heads, s.vdim, e->cfg.norm_eps, M);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), s.vdim, e->proj, L.n_in, L.c_g, 0,
+                                                                               static_cast<T*>(e->oh), s.heads, s.vdim, e->cfg.norm_eps, M));
   TRY(output_product<T>(e, static_cast<T*>(e->oh), L.wo, HD, e->y, M));
   return 0;
 }
@@ -1225,9 +1213,9 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
     auto pk = gqa_prepare_row_kernel<T>;
     const size_t psm = (size_t)(H + (own ? G : 0)) * dk * 4;
     TRY(opt_in_smem(pk, psm));
-    pk<<<M, nt, psm, e->stream>>>(e->proj, L.ld_in, L.c_q, L.c_kk, L.c_vv, s.proj_bias ? at<T>(e, L.b_in) : nullptr, at<T>(e, L.q_norm),
+    TRY(launch_early(e, pk, M, nt, psm, 1, e->proj, L.ld_in, L.c_q, L.c_kk, L.c_vv, s.proj_bias ? at<T>(e, L.b_in) : nullptr, at<T>(e, L.q_norm),
                                                         own ? at<T>(e, L.k_norm) : nullptr, e->cfg.norm_eps, H, G, dk, dv, own ? 1 : 0, s.q_temp_coef,
-                                                        s.q_temp_every, sp.row_slot, sp.row_pos, pg, pool, e->qfull, q16);
+                                                        s.q_temp_every, sp.row_slot, sp.row_pos, pg, pool, e->qfull, q16));
   } else if (s.conv_taps > 0 || rotated_norm || L.rot_mul != 1.f || L.vmix_mode) {
     GqaPrep a{};
     a.proj = e->proj; a.ld = L.ld_in; a.col_q = L.c_q; a.col_k = L.c_kk; a.col_v = L.c_vv;
@@ -1256,8 +1244,8 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
       const dim3 grid(sp.n_seq, cdiv(slots, 8), zs);
 #define LAUNCH_PREP(TAPS)                                                                                                          \
   do {                                                                                                                             \
-    if (hmax <= 128) gqa_filter_prepare_vec_kernel<T, TAPS, 1><<<grid, 256, vsm, e->stream>>>(a, sp.seqs, pg, pool, qf, q16);      \
-    else gqa_filter_prepare_vec_kernel<T, TAPS, 2><<<grid, 256, vsm, e->stream>>>(a, sp.seqs, pg, pool, qf, q16);                  \
+    if (hmax <= 128) TRY(launch_early(e, gqa_filter_prepare_vec_kernel<T, TAPS, 1>, grid, 256, vsm, 1, a, sp.seqs, pg, pool, qf, q16));      \
+    else TRY(launch_early(e, gqa_filter_prepare_vec_kernel<T, TAPS, 2>, grid, 256, vsm, 1, a, sp.seqs, pg, pool, qf, q16));                  \
   } while (0)
       if (taps == 1) LAUNCH_PREP(1);
       else if (taps == 2) LAUNCH_PREP(2);
@@ -1270,23 +1258,19 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
       const size_t psm = (size_t)GQA_PREP_ROWS * (dk + s.rot_dims) * 4;
       auto pk = gqa_filter_prepare_kernel<T>;
       TRY(opt_in_smem(pk, psm));
-      pk<<<dim3(sp.n_seq, cdiv(slots, a.spc), zs), 128, psm, e->stream>>>(a, sp.seqs, pg, pool, qf, q16);
+      TRY(launch_early(e, pk, dim3(sp.n_seq, cdiv(slots, a.spc), zs), 128, psm, 1, a, sp.seqs, pg, pool, qf, q16));
     }
   } else {
-    gqa_prepare_kernel<T><<<cdiv((long)M * slots, 8), 256, 0, e->stream>>>(
+    TRY(launch_early(e, gqa_prepare_kernel<T>, cdiv((long)M * slots, 8), 256, 0, 1,
         e->proj, L.ld_in, L.c_q, L.c_kk, L.c_vv, s.proj_bias ? at<T>(e, L.b_in) : nullptr, weighted ? at<T>(e, L.q_norm) : nullptr,
         weighted && own ? at<T>(e, L.k_norm) : nullptr, e->cfg.norm_eps, H, G, dk, dv, own ? 1 : 0, s.q_temp_coef, s.q_temp_every, sp.row_slot, sp.row_pos,
-        pg, pool, e->qfull, q16, M, s.qk_norm != XOTB200_LM_QKNORM_NONE ? 1 : 0, s.rot_dims > 0 ? L.freqs : nullptr, s.rot_dims, s.rot_layout);
+        pg, pool, e->qfull, q16, M, s.qk_norm != XOTB200_LM_QKNORM_NONE ? 1 : 0, s.rot_dims > 0 ? L.freqs : nullptr, s.rot_dims, s.rot_layout));
   }
-  CK(cudaGetLastError());
-  e->launches++;
   const size_t pool_rows = (size_t)e->n_pages * e->page_size;
   if (s.pool > 0) {
     // blocks whose last token this step appended get their pooled row (after the append, before any reader)
-    gqa_pool_blocks_kernel<T><<<dim3(sp.n_seq, sp.max_rows / s.pool + 1, cdiv(G * (dk + dv), 128)), 128, 0, e->stream>>>(pool, pg, pool_rows, sp.seqs, s.pool,
-                                                                                                                       G * (dk + dv));
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(launch_early(e, gqa_pool_blocks_kernel<T>, dim3(sp.n_seq, sp.max_rows / s.pool + 1, cdiv(G * (dk + dv), 128)), 128, 0, 1, pool, pg, pool_rows, sp.seqs, s.pool,
+                                                                                                                       G * (dk + dv)));
   }
   const GqaScore sc{s.scale, s.softcap, s.window, s.chunk, s.dist_bias ? at<T>(e, L.r1) : nullptr, s.dist_bias ? at<T>(e, L.r2) : nullptr,
                     s.rel_buckets > 0 ? L.rel_tab : nullptr, L.rel_n, s.sink == XOTB200_LM_SINK_LEARNED ? at<T>(e, L.sink) : nullptr, s.keep_first, s.pool, pool_rows,
@@ -1305,8 +1289,8 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
   do {                                                                                                                                       \
     auto kern = gqa_attention_kernel<T, NACC>;                                                                                               \
     TRY(opt_in_smem(kern, smem));                                                                                                            \
-    kern<<<grid, nw * 32, smem, e->stream>>>(e->qfull, pool, pg, it.first, H, G, dk, dv, sc, gate, s.out_gate, L.ld_in, L.c_g,               \
-                                             static_cast<T*>(e->oh), run, e->part);                                                          \
+    TRY(launch_early(e, kern, grid, nw * 32, smem, 1, e->qfull, pool, pg, it.first, H, G, dk, dv, sc, gate, s.out_gate, L.ld_in, L.c_g,               \
+                                             static_cast<T*>(e->oh), run, e->part));                                                          \
   } while (0)
     if (dv <= 32) LAUNCH_GQA(1);
     else if (dv <= 64) LAUNCH_GQA(2);
@@ -1314,13 +1298,9 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
     else if (dv <= 256) LAUNCH_GQA(8);
     else LAUNCH_GQA(16);
 #undef LAUNCH_GQA
-    CK(cudaGetLastError());
-    e->launches++;
     if (splits > 1) {
       // few pairs: their value columns are cut over grid.z
-      gqa_combine_kernel<T><<<dim3(it.second, cdiv(qpi * H, 8), it.second * cdiv(qpi * H, 8) < 4 * e->sm_count ? cdiv(dv, 32) : 1), 256, 0, e->stream>>>(e->part, it.first, H, dv, splits, static_cast<const T*>(sc.sink), sc.sink_one, gate, s.out_gate, L.ld_in, L.c_g, static_cast<T*>(e->oh));
-      CK(cudaGetLastError());
-      e->launches++;
+      TRY(launch_early(e, gqa_combine_kernel<T>, dim3(it.second, cdiv(qpi * H, 8), it.second * cdiv(qpi * H, 8) < 4 * e->sm_count ? cdiv(dv, 32) : 1), 256, 0, 1, e->part, it.first, H, dv, splits, static_cast<const T*>(sc.sink), sc.sink_one, gate, s.out_gate, L.ld_in, L.c_g, static_cast<T*>(e->oh)));
     }
   }
   if constexpr (std::is_same<T, bf16>::value) {
@@ -1335,22 +1315,18 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
       if (s.window > 0) dist_n = std::min(dist_n, s.window + 64);
       if (s.dist_bias) {
         if ((size_t)H * dist_n > e->dist_cap) { TRY(regrow(e->dist_tab, (size_t)H * dist_n * 4)); e->dist_cap = (size_t)H * dist_n; }
-        gqa_dist_table_kernel<<<cdiv((long)H * dist_n, 256), 256, 0, e->stream>>>(at<bf16>(e, L.r1), at<bf16>(e, L.r2), H, dist_n, e->dist_tab);
-        CK(cudaGetLastError());
-        e->launches++;
+        TRY(launch_early(e, gqa_dist_table_kernel, cdiv((long)H * dist_n, 256), 256, 0, 1, at<bf16>(e, L.r1), at<bf16>(e, L.r2), H, dist_n, e->dist_tab));
       }
 #define LAUNCH_GQA_FLASH(DVT)                                                                                                              \
   do {                                                                                                                                     \
     auto kern = gqa_flash_kernel<DVT>;                                                                                                     \
     TRY(opt_in_smem(kern, fsm));                                                                                                           \
-    kern<<<grid, 128, fsm, e->stream>>>(static_cast<const bf16*>(e->q16), pool, pg, sp.gqa_tiles, H, G, dk, dv, sc,                        \
-                                        s.dist_bias ? e->dist_tab : nullptr, dist_n, gate, s.out_gate, L.ld_in, L.c_g, static_cast<bf16*>(e->oh)); \
+    TRY(launch_late(e, kern, grid, 128, fsm, static_cast<const bf16*>(e->q16), pool, pg, sp.gqa_tiles, H, G, dk, dv, sc,                        \
+                                        s.dist_bias ? e->dist_tab : nullptr, dist_n, gate, s.out_gate, L.ld_in, L.c_g, static_cast<bf16*>(e->oh))); \
   } while (0)
       if (dvt == 8) LAUNCH_GQA_FLASH(8);
       else LAUNCH_GQA_FLASH(16);
 #undef LAUNCH_GQA_FLASH
-      CK(cudaGetLastError());
-      e->launches++;
       e->flash_launches++;
     }
   }
@@ -1365,10 +1341,8 @@ static int filter_channels(xotb200_lm* e, LmLayer& L, const StepPlan& sp, int co
   const xotb200_lm_layer& s = L.s;
   float* cstate = e->state + L.conv_off;
   const int zrows = std::max(1, std::min(128, cdiv(sp.max_rows, 8)));
-  short_conv_kernel<T, float><<<dim3(sp.n_seq, cdiv(C, 256), zrows), 256, 0, e->stream>>>(e->proj, L.ld_in, col0, C, at<T>(e, L.conv_w), bias, s.conv_taps, 1, 0,
-                                                                                          sp.seqs, cstate, e->state_floats, e->cvb, C);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, short_conv_kernel<T, float>, dim3(sp.n_seq, cdiv(C, 256), zrows), 256, 0, 1, e->proj, L.ld_in, col0, C, at<T>(e, L.conv_w), bias, s.conv_taps, 1, 0,
+                                                                                          sp.seqs, cstate, e->state_floats, e->cvb, C));
   return 0;
 }
 
@@ -1377,15 +1351,11 @@ static int gated_delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, floa
   const xotb200_lm_layer& s = L.s;
   const int M = sp.M, H = s.heads, G = s.kv_heads, dk = s.dim, dv = s.vdim, C = L.conv_ch;
   TRY(filter_channels<T>(e, L, sp, L.c_r, C, nullptr));
-  gated_delta_prepare_kernel<T><<<cdiv((long)M * H, 8), 256, 0, e->stream>>>(e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
-                                                                            e->du, e->dau, e->dkk, e->drr, H, G, dk, M);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, gated_delta_prepare_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
+                                                                            e->du, e->dau, e->dkk, e->drr, H, G, dk, M));
   TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, H * dk, 0}, DeltaSrc{e->drr, H * dk, 0}, DeltaSrc{e->cvb, C, 2 * G * dk}, dk, dv, true));
-  head_norm_gate_kernel<T><<<cdiv((long)M * H, 8), 256, 0, e->stream>>>(e->oraw, nullptr, nullptr, at<T>(e, L.onorm), 0, e->proj, L.ld_in, L.c_g, 1, static_cast<T*>(ohbuf),
-                                                                       H, dv, e->cfg.norm_eps, M);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), 0, e->proj, L.ld_in, L.c_g, 1, static_cast<T*>(ohbuf),
+                                                                       H, dv, e->cfg.norm_eps, M));
   TRY(output_product<T>(e, static_cast<T*>(ohbuf), L.wo, H * dv, yout, M));
   return 0;
 }
@@ -1396,20 +1366,14 @@ template <typename T>
 static int matrix_lstm_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout, void* ohbuf) {
   const xotb200_lm_layer& s = L.s;
   const int M = sp.M, H = s.heads, dk = s.dim, dv = s.vdim;
-  mlstm_gates_kernel<T><<<cdiv((long)sp.n_seq * H, 4), 128, 0, e->stream>>>(e->proj, L.ld_in, L.c_i, L.c_f, at<T>(e, L.i_b), at<T>(e, L.f_b), s.gate_cap, sp.seqs, sp.n_seq, H,
-                                                                          e->state + L.m_off, e->state_floats, e->gdec, e->ginw, e->gfloor);
-  CK(cudaGetLastError());
-  mlstm_expand_kernel<<<cdiv((long)M * H, 8), 256, 0, e->stream>>>(e->proj, L.ld_in, L.c_r, L.c_k, e->gdec, e->ginw, e->wlog, e->dkk, e->drr, H, dk, M);
-  CK(cudaGetLastError());
-  mlstm_normaliser_kernel<<<sp.n_seq * H, 32 * std::max(1, std::min(16, sp.max_rows / 16)), 0, e->stream>>>(e->dkk, e->drr, e->gdec, sp.seqs, H, dk, e->state + L.n_off,
-                                                                                                        e->state_floats, e->gnq);
-  CK(cudaGetLastError());
-  e->launches += 3;
+  TRY(launch_early(e, mlstm_gates_kernel<T>, cdiv((long)sp.n_seq * H, 4), 128, 0, 1, e->proj, L.ld_in, L.c_i, L.c_f, at<T>(e, L.i_b), at<T>(e, L.f_b), s.gate_cap, sp.seqs, sp.n_seq, H,
+                                                                          e->state + L.m_off, e->state_floats, e->gdec, e->ginw, e->gfloor));
+  TRY(launch_early(e, mlstm_expand_kernel, cdiv((long)M * H, 8), 256, 0, 1, e->proj, L.ld_in, L.c_r, L.c_k, e->gdec, e->ginw, e->wlog, e->dkk, e->drr, H, dk, M));
+  TRY(launch_early(e, mlstm_normaliser_kernel, sp.n_seq * H, 32 * std::max(1, std::min(16, sp.max_rows / 16)), 0, 1, e->dkk, e->drr, e->gdec, sp.seqs, H, dk, e->state + L.n_off,
+                                                                                                        e->state_floats, e->gnq));
   TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, H * dk, 0}, DeltaSrc{e->drr, H * dk, 0}, DeltaSrc{e->proj, L.ld_in, L.c_v}, dk, dv, false));
-  head_norm_gate_kernel<T><<<cdiv((long)M * H, 8), 256, 0, e->stream>>>(e->oraw, e->gnq, e->gfloor, at<T>(e, L.onorm), dv, e->proj, L.ld_in, L.c_g, 0,
-                                                                       static_cast<T*>(ohbuf), H, dv, e->cfg.norm_eps, M);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->oraw, e->gnq, e->gfloor, at<T>(e, L.onorm), dv, e->proj, L.ld_in, L.c_g, 0,
+                                                                       static_cast<T*>(ohbuf), H, dv, e->cfg.norm_eps, M));
   TRY(output_product<T>(e, static_cast<T*>(ohbuf), L.wo, H * dv, yout, M));
   return 0;
 }
@@ -1421,20 +1385,16 @@ static int mamba2_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
   const xotb200_lm_layer& s = L.s;
   const int M = sp.M, H = s.heads, G = s.kv_heads, N = s.dim, dv = s.vdim, C = L.conv_ch, inner = H * dv;
   TRY(filter_channels<T>(e, L, sp, L.c_v, C, at<T>(e, L.conv_b)));
-  mamba2_prepare_kernel<T><<<cdiv((long)M * H, 8), 256, 0, e->stream>>>(e->cvb, C, e->proj, L.ld_in, L.c_dt, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog, e->dkk, e->drr,
-                                                                       H, G, N, dv, M);
-  CK(cudaGetLastError());
-  e->launches++;
+  TRY(launch_early(e, mamba2_prepare_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_dt, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog, e->dkk, e->drr,
+                                                                       H, G, N, dv, M));
   TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, H * N, 0}, DeltaSrc{e->drr, H * N, 0}, DeltaSrc{e->cvb, C, 0}, N, dv, false));
   {
     const int part = inner / s.out_norm_groups;
     auto ok = mamba2_out_kernel<T>;
     TRY(opt_in_smem(ok, (size_t)part * 4));
-    ok<<<M * s.out_norm_groups, std::min(1024, std::max(32, cdiv(part, 4 * 32) * 32)), (size_t)part * 4, e->stream>>>(
-        e->oraw, e->cvb, C, e->proj, L.ld_in, L.c_z, at<T>(e, L.d_skip), at<T>(e, L.onorm), H, dv, s.out_norm_groups, e->cfg.norm_eps, static_cast<T*>(ohbuf));
+    TRY(launch_early(e, ok, M * s.out_norm_groups, std::min(1024, std::max(32, cdiv(part, 4 * 32) * 32)), (size_t)part * 4, 1,
+        e->oraw, e->cvb, C, e->proj, L.ld_in, L.c_z, at<T>(e, L.d_skip), at<T>(e, L.onorm), H, dv, s.out_norm_groups, e->cfg.norm_eps, static_cast<T*>(ohbuf)));
   }
-  CK(cudaGetLastError());
-  e->launches++;
   TRY(output_product<T>(e, static_cast<T*>(ohbuf), L.wo, inner, yout, M));
   return 0;
 }
@@ -1497,12 +1457,10 @@ static int feed_forward(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
       auto kern = multi ? moe_router_kernel<T, RPB> : moe_router_kernel<T, 1>;
       const size_t rsm = (multi ? RPB : 1) * row_sm;
       TRY(opt_in_smem(kern, rsm));
-      kern<<<multi ? cdiv(M, RPB) : M, std::min(1024, std::max(32 * RPB, (M <= 16 ? E : cdiv(E, 2)) * 32)), rsm, e->stream>>>(
+      TRY(launch_early(e, kern, multi ? cdiv(M, RPB) : M, std::min(1024, std::max(32 * RPB, (M <= 16 ? E : cdiv(E, 2)) * 32)), rsm, 1,
           h, D, at<T>(e, L.router), s.router_bias ? at<T>(e, L.router_b) : nullptr, s.router_kind, E, s.groups, s.groups_keep, top,
-          s.router_correction ? at<T>(e, L.correction) : nullptr, s.group_best, s.router_scale, e->moe_ids, e->moe_wts, M);
+          s.router_correction ? at<T>(e, L.correction) : nullptr, s.group_best, s.router_scale, e->moe_ids, e->moe_wts, M));
     }
-    CK(cudaGetLastError());
-    e->launches++;
     if constexpr (std::is_same<T, bf16>::value) {
       if (grouped_ok) {
         // few rows: an expert has at most M of them (a row picks an expert once), one row tile each, and the products stream the chosen experts
@@ -1512,11 +1470,9 @@ static int feed_forward(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
         int *counts = e->moe_plan, *starts = counts + e->max_experts, *cursor = starts + e->max_experts + 1, *place = cursor + e->max_experts,
             *tile_expert = place + (size_t)e->m_cap * e->max_top;
         bf16* xg = static_cast<bf16*>(e->moe_xg);
-        moe_count_kernel<<<cdiv(pairs, 256), 256, 0, e->stream>>>(e->moe_ids, pairs, counts);
-        moe_plan_kernel<<<1, 256, 0, e->stream>>>(counts, E, tile_rows, tiles, starts, cursor, tile_expert);
-        moe_scatter_kernel<bf16><<<cdiv(pairs, 8), 256, 0, e->stream>>>(h, D, e->moe_ids, pairs, top, starts, cursor, place, xg);
-        CK(cudaGetLastError());
-        e->launches += 3;
+        TRY(launch_early(e, moe_count_kernel, cdiv(pairs, 256), 256, 0, 1, e->moe_ids, pairs, counts));
+        TRY(launch_early(e, moe_plan_kernel, 1, 256, 0, 1, counts, E, tile_rows, tiles, starts, cursor, tile_expert));
+        TRY(launch_early(e, moe_scatter_kernel<bf16>, cdiv(pairs, 8), 256, 0, 1, h, D, e->moe_ids, pairs, top, starts, cursor, place, xg));
         bf16* ma = static_cast<bf16*>(e->mact);
         int r = s.expert_act == XOTB200_LM_EXPERT_CLAMPED_GLU
                     ? grouped_product<EPI_CLAMPED_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, M, m_pad, 2 * F, D, tile_expert, glu)
@@ -1526,9 +1482,7 @@ static int feed_forward(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
         if (r == 1) r = grouped_product<EPI_NONE, float>(e, ma, F, at<bf16>(e, L.w_edown), F, (long)D * F, E, e->moe_yg, D, M, m_pad, D, F, tile_expert);
         if (r < 0) return r;
         if (r == 1) {
-          moe_combine_kernel<bf16><<<row_grid(e, M, D, 256), 256, 0, e->stream>>>(e->moe_yg, place, e->moe_wts, top, D, shared, yout, close);
-          CK(cudaGetLastError());
-          e->launches++;
+          TRY(launch_early(e, moe_combine_kernel<bf16>, row_grid(e, M, D, 256), 256, 0, 1, e->moe_yg, place, e->moe_wts, top, D, shared, yout, close));
           e->closed = e->close != nullptr;
           return 0;
         }
@@ -1538,19 +1492,15 @@ static int feed_forward(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
       auto kern = moe_rows_up_kernel<T>;
       TRY(opt_in_smem(kern, (size_t)D * 4));
       // a warp takes two weight rows per pass with gated experts (a gate row and its up row), four with ungated ones
-      kern<<<dim3(M, top + (ride ? 1 : 0), std::max(1, std::min(cdiv(std::max(F, ride ? Fs : 0), gated ? 8 : 32), M <= 16 ? 1024 : 16))), 256, (size_t)D * 4, e->stream>>>(
-          h, D, at<T>(e, L.w_gu), F, s.expert_act == XOTB200_LM_EXPERT_CLAMPED_GLU ? 2 : gated ? 1 : 0, glu, e->moe_ids, top, static_cast<T*>(e->mact), ride ? at<T>(e, L.up) : nullptr, Fs, static_cast<T*>(e->act));
-      CK(cudaGetLastError());
-      e->launches++;
+      TRY(launch_early(e, kern, dim3(M, top + (ride ? 1 : 0), std::max(1, std::min(cdiv(std::max(F, ride ? Fs : 0), gated ? 8 : 32), M <= 16 ? 1024 : 16))), 256, (size_t)D * 4, 1,
+          h, D, at<T>(e, L.w_gu), F, s.expert_act == XOTB200_LM_EXPERT_CLAMPED_GLU ? 2 : gated ? 1 : 0, glu, e->moe_ids, top, static_cast<T*>(e->mact), ride ? at<T>(e, L.up) : nullptr, Fs, static_cast<T*>(e->act)));
     }
     {
       auto kern = moe_rows_down_kernel<T>;
       const size_t dsm = ((size_t)top * F + (ride ? Fs + 4 : 0)) * 4;
       TRY(opt_in_smem(kern, dsm));
-      kern<<<dim3(M, std::max(1, std::min(cdiv(D, 16), M <= 16 ? 1024 : 16))), 256, dsm, e->stream>>>(static_cast<T*>(e->mact), F, at<T>(e, L.w_edown), D, e->moe_ids, e->moe_wts, top,
-                                                                                                   shared, yout, static_cast<T*>(e->act), ride ? at<T>(e, L.down) : nullptr, Fs, close);
-      CK(cudaGetLastError());
-      e->launches++;
+      TRY(launch_early(e, kern, dim3(M, std::max(1, std::min(cdiv(D, 16), M <= 16 ? 1024 : 16))), 256, dsm, 1, static_cast<T*>(e->mact), F, at<T>(e, L.w_edown), D, e->moe_ids, e->moe_wts, top,
+                                                                                                   shared, yout, static_cast<T*>(e->act), ride ? at<T>(e, L.down) : nullptr, Fs, close));
       e->closed = e->close != nullptr;
     }
     return 0;
@@ -1611,10 +1561,11 @@ static int run_mixer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   return 0;
 }
 
-static void finish_logits(xotb200_lm* e, int n_want) {
+static int finish_logits(xotb200_lm* e, int n_want) {
   const float scale = e->cfg.logit_scale != 0.f ? e->cfg.logit_scale : 1.0f;
-  argmax_rows_kernel<<<n_want, 1024, 0, e->stream>>>(e->logits, e->cfg.vocab, scale, e->cfg.logit_softcap, e->d_argmax);
-  e->launches++;
+  // the rows' results and the error word lie behind the logits: [n_want, vocab] fp32, [n_want] int, one int
+  int* tail = reinterpret_cast<int*>(e->logits + (size_t)n_want * e->cfg.vocab);
+  return launch_early(e, argmax_rows_kernel, n_want, 1024, 0, 1, e->logits, e->cfg.vocab, scale, e->cfg.logit_softcap, tail, e->d_err);
 }
 
 // How a block holds a row of D entries in registers: pieces of four per thread (nv of them, 1, 2 or 4; 0 = the row is not whole pieces or too long,
@@ -1647,11 +1598,9 @@ static int run_layers_post(xotb200_lm* e, const StepPlan& sp, int n_want) {
     if (rs.nv) {
       auto vk = rms ? (rs.nv == 1 ? residual_norm_vec_kernel<T, 1, true> : rs.nv == 2 ? residual_norm_vec_kernel<T, 2, true> : residual_norm_vec_kernel<T, 4, true>)
                     : (rs.nv == 1 ? residual_norm_vec_kernel<T, 1, false> : rs.nv == 2 ? residual_norm_vec_kernel<T, 2, false> : residual_norm_vec_kernel<T, 4, false>);
-      vk<<<n, rs.threads, 0, e->stream>>>(e->x, y, y_bias, at<T>(e, w), rms ? nullptr : at<T>(e, b), 1.0f, out, rows, D, eps);
-    } else if (rms) kern_rms<<<n, nt, (size_t)D * 4, e->stream>>>(e->x, y, y_bias, at<T>(e, w), 1.0f, out, rows, D, eps);
-    else kern<<<n, nt, (size_t)D * 4, e->stream>>>(e->x, y, y_bias, at<T>(e, w), at<T>(e, b), out, rows, D, eps);
-    CK(cudaGetLastError());
-    e->launches++;
+      TRY(launch_early(e, vk, n, rs.threads, 0, 1, e->x, y, y_bias, at<T>(e, w), rms ? nullptr : at<T>(e, b), 1.0f, out, rows, D, eps));
+    } else if (rms) TRY(launch_early(e, kern_rms, n, nt, (size_t)D * 4, 1, e->x, y, y_bias, at<T>(e, w), 1.0f, out, rows, D, eps));
+    else TRY(launch_early(e, kern, n, nt, (size_t)D * 4, 1, e->x, y, y_bias, at<T>(e, w), at<T>(e, b), out, rows, D, eps));
     return 0;
   };
   auto close = [&](size_t w, size_t b, const T* y_bias) -> int { return norm_rows(e->y, y_bias, w, b, h, nullptr, M); };
@@ -1659,18 +1608,16 @@ static int run_layers_post(xotb200_lm* e, const StepPlan& sp, int n_want) {
     if (e->cfg.pos_sinusoid || e->cfg.embed_norm) {
       auto ek = embed_sinusoid_rows_kernel<T>;
       TRY(opt_in_smem(ek, (size_t)D * 4));
-      ek<<<M, nt, (size_t)D * 4, e->stream>>>(at<T>(e, e->embed), e->cfg.max_positions > 0 ? at<T>(e, e->pos_table) : nullptr, e->pos_freqs, sp.tokens, sp.row_pos,
-                                              e->cfg.embed_norm ? at<T>(e, e->embed_norm) : nullptr, 1.0f, eps, e->x, h, D);
+      TRY(launch_early(e, ek, M, nt, (size_t)D * 4, 1, at<T>(e, e->embed), e->cfg.max_positions > 0 ? at<T>(e, e->pos_table) : nullptr, e->pos_freqs, sp.tokens, sp.row_pos,
+                                              e->cfg.embed_norm ? at<T>(e, e->embed_norm) : nullptr, 1.0f, eps, e->x, h, D));
     } else {
       auto ek = D % 4 == 0 ? embed_pos_rows_kernel<T, 4> : embed_pos_rows_kernel<T, 1>;
-      ek<<<M, D % 4 == 0 ? embed_threads(D) : 128, 0, e->stream>>>(at<T>(e, e->embed), e->cfg.max_positions > 0 ? at<T>(e, e->pos_table) : nullptr, sp.tokens, sp.row_pos,
-                                                                   e->x, h, D);
+      TRY(launch_early(e, ek, M, D % 4 == 0 ? embed_threads(D) : 128, 0, 1, at<T>(e, e->embed), e->cfg.max_positions > 0 ? at<T>(e, e->pos_table) : nullptr, sp.tokens, sp.row_pos,
+                                                                   e->x, h, D));
     }
   } else {
-    cast_rows_kernel<T><<<std::min(4096, cdiv((long)M * D, 256)), 256, 0, e->stream>>>(e->x, h, (size_t)M * D);
+    TRY(launch_early(e, cast_rows_kernel<T>, std::min(4096, cdiv((long)M * D, 256)), 256, 0, 1, e->x, h, (size_t)M * D));
   }
-  CK(cudaGetLastError());
-  e->launches++;
   for (size_t li = 0; li < e->layers.size(); ++li) {
     LmLayer& L = e->layers[li];
     TRY(run_mixer<T>(e, L, sp));
@@ -1686,8 +1633,7 @@ static int run_layers_post(xotb200_lm* e, const StepPlan& sp, int n_want) {
     T* hw = static_cast<T*>(e->hw);
     TRY(norm_rows(nullptr, nullptr, e->final_norm, e->final_norm_b, hw, sp.want, n_want));
     TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    finish_logits(e, n_want);
-    CK(cudaGetLastError());
+    TRY(finish_logits(e, n_want));
   }
   return 0;
 }
@@ -1714,25 +1660,19 @@ static int run_layers_pre_scalar(xotb200_lm* e, const StepPlan& sp, int n_want) 
     const T* g = L ? at<T>(e, q ? L->norm2 : L->norm1) : nullptr;
     const T* inc = L && hc ? at<T>(e, L->hc_in[q]) : nullptr;
     const bool conv = L && CT > 0;
-    okern<<<M, nt, (size_t)D * 4, e->stream>>>(e->x, S, pend.y, pend.y2, pend.ya, pend.yb, mult, pend.mix, pend.out, inc, g, eps, nullptr,
-                                               L ? (conv ? e->h0 : nullptr) : sum_out, L && !conv ? h : nullptr, D);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(launch_early(e, okern, M, nt, (size_t)D * 4, 1, e->x, S, pend.y, pend.y2, pend.ya, pend.yb, mult, pend.mix, pend.out, inc, g, eps, nullptr,
+                                               L ? (conv ? e->h0 : nullptr) : sum_out, L && !conv ? h : nullptr, D));
     pend = Pending{};
     if (conv) {
       float* cstate = e->state + L->canon_off[q];
       const int zrows = std::max(1, std::min(128, cdiv(sp.max_rows, 8)));
-      short_conv_kernel<T, T><<<dim3(sp.n_seq, cdiv(D, 256), zrows), 256, 0, e->stream>>>(e->h0, D, 0, D, at<T>(e, L->canon[q]), nullptr, CT, 0, 1, sp.seqs, cstate,
-                                                                                          e->state_floats, h, D);
-      CK(cudaGetLastError());
-      e->launches++;
+      TRY(launch_early(e, short_conv_kernel<T, T>, dim3(sp.n_seq, cdiv(D, 256), zrows), 256, 0, 1, e->h0, D, 0, D, at<T>(e, L->canon[q]), nullptr, CT, 0, 1, sp.seqs, cstate,
+                                                                                          e->state_floats, h, D));
     }
     return 0;
   };
   if (e->first) {
-    embed_streams_kernel<T><<<M, nt, 0, e->stream>>>(at<T>(e, e->embed), sp.tokens, e->cfg.embed_norm ? at<T>(e, e->embed_norm) : nullptr, eps, e->x, S, D);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(launch_early(e, embed_streams_kernel<T>, M, nt, 0, 1, at<T>(e, e->embed), sp.tokens, e->cfg.embed_norm ? at<T>(e, e->embed_norm) : nullptr, eps, e->x, S, D));
   }
   for (size_t li = 0; li < e->layers.size(); ++li) {
     LmLayer& L = e->layers[li];
@@ -1754,13 +1694,10 @@ static int run_layers_pre_scalar(xotb200_lm* e, const StepPlan& sp, int n_want) 
   if (e->last && n_want > 0) {
     // the final norm of the wanted rows closes the last sublayer for them on the way (the other rows' streams are not needed again)
     T* hw = static_cast<T*>(e->hw);
-    okern<<<n_want, nt, (size_t)D * 4, e->stream>>>(e->x, S, pend.y, pend.y2, pend.ya, pend.yb, mult, pend.mix, pend.out, nullptr, at<T>(e, e->final_norm), eps, sp.want,
-                                                    nullptr, hw, D);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(launch_early(e, okern, n_want, nt, (size_t)D * 4, 1, e->x, S, pend.y, pend.y2, pend.ya, pend.yb, mult, pend.mix, pend.out, nullptr, at<T>(e, e->final_norm), eps, sp.want,
+                                                    nullptr, hw, D));
     TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    finish_logits(e, n_want);
-    CK(cudaGetLastError());
+    TRY(finish_logits(e, n_want));
   }
   return 0;
 }
@@ -1775,10 +1712,8 @@ static int run_layers_pre_dyt(xotb200_lm* e, const StepPlan& sp, int n_want) {
   T* h = static_cast<T*>(e->h);
   const int nt = std::min(256, std::max(32, cdiv(D, 32) * 32));
   LmLayer& L0 = e->layers.front();
-  if (e->first) embed_dyt_rows_kernel<T><<<row_grid(e, M, D, nt), nt, 0, e->stream>>>(at<T>(e, e->embed), sp.tokens, at<T>(e, L0.norm1a), at<T>(e, L0.norm1), at<T>(e, L0.norm1b), e->x, h, D);
-  else dyt_rows_kernel<T><<<row_grid(e, M, D, nt), nt, 0, e->stream>>>(e->x, nullptr, at<T>(e, L0.norm1a), at<T>(e, L0.norm1), at<T>(e, L0.norm1b), h, D);
-  CK(cudaGetLastError());
-  e->launches++;
+  if (e->first) TRY(launch_early(e, embed_dyt_rows_kernel<T>, row_grid(e, M, D, nt), nt, 0, 1, at<T>(e, e->embed), sp.tokens, at<T>(e, L0.norm1a), at<T>(e, L0.norm1), at<T>(e, L0.norm1b), e->x, h, D));
+  else TRY(launch_early(e, dyt_rows_kernel<T>, row_grid(e, M, D, nt), nt, 0, 1, e->x, nullptr, at<T>(e, L0.norm1a), at<T>(e, L0.norm1), at<T>(e, L0.norm1b), h, D));
   // runs one sublayer: `ls` scales its result; the norm that follows it (a = NULL: none) makes the next operand
   EpiArgs close;
   auto sublayer = [&](auto&& body, size_t ls, const LmLayer* next, int q) -> int {
@@ -1798,9 +1733,7 @@ static int run_layers_pre_dyt(xotb200_lm* e, const StepPlan& sp, int n_want) {
     e->close = nullptr;
     if (rc < 0) return rc;
     if (!e->closed) {
-      close_rows_kernel<T><<<row_grid(e, M, D, nt), nt, 0, e->stream>>>(close, e->y, D);
-      CK(cudaGetLastError());
-      e->launches++;
+      TRY(launch_early(e, close_rows_kernel<T>, row_grid(e, M, D, nt), nt, 0, 1, close, e->y, D));
     }
     return 0;
   };
@@ -1815,12 +1748,9 @@ static int run_layers_pre_dyt(xotb200_lm* e, const StepPlan& sp, int n_want) {
   if (e->trace) e->trace_floats = e->layers.size() * (size_t)M * D;
   if (e->last && n_want > 0) {
     T* hw = static_cast<T*>(e->hw);
-    dyt_rows_kernel<T><<<row_grid(e, n_want, D, nt), nt, 0, e->stream>>>(e->x, sp.want, at<T>(e, e->final_norm_a), at<T>(e, e->final_norm), at<T>(e, e->final_norm_b), hw, D);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(launch_early(e, dyt_rows_kernel<T>, row_grid(e, n_want, D, nt), nt, 0, 1, e->x, sp.want, at<T>(e, e->final_norm_a), at<T>(e, e->final_norm), at<T>(e, e->final_norm_b), hw, D));
     TRY((product<T, T, float, EPI_NONE>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    finish_logits(e, n_want);
-    CK(cudaGetLastError());
+    TRY(finish_logits(e, n_want));
   }
   return 0;
 }
@@ -1839,10 +1769,8 @@ static int run_layers_parallel(xotb200_lm* e, const StepPlan& sp, int n_want) {
   const float *pend = nullptr, *pend2 = nullptr;
   auto pass = [&](bool embed, const T* w, T* out, const int* rows, int n) -> int {
     if (!embed && !pend && !w) return 0;
-    kern<<<n, nt, (size_t)D * 4, e->stream>>>(e->x, pend, pend2, embed ? at<T>(e, e->embed) : nullptr, sp.tokens, e->cfg.embed_scale != 0.f ? e->cfg.embed_scale : 1.0f,
-                                              e->cfg.bigram_buckets > 0 ? at<T>(e, e->bigram) : nullptr, sp.bigram_row, rows, w, eps, out, D);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(launch_early(e, kern, n, nt, (size_t)D * 4, 1, e->x, pend, pend2, embed ? at<T>(e, e->embed) : nullptr, sp.tokens, e->cfg.embed_scale != 0.f ? e->cfg.embed_scale : 1.0f,
+                                              e->cfg.bigram_buckets > 0 ? at<T>(e, e->bigram) : nullptr, sp.bigram_row, rows, w, eps, out, D));
     if (!rows) pend = pend2 = nullptr;
     return 0;
   };
@@ -1874,8 +1802,7 @@ static int run_layers_parallel(xotb200_lm* e, const StepPlan& sp, int n_want) {
     T* hw = static_cast<T*>(e->hw);
     TRY(pass(false, at<T>(e, e->final_norm), hw, sp.want, n_want));
     TRY((product<T, T, float, EPI_NONE>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    finish_logits(e, n_want);
-    CK(cudaGetLastError());
+    TRY(finish_logits(e, n_want));
   }
   return 0;
 }
@@ -1902,12 +1829,10 @@ static int run_layers(xotb200_lm* e, const StepPlan& sp, int n_want) {
   auto norm_rows = [&](const float* y, const T* w_post, const T* w_pre, T* out, const int* rows, int n) -> int {
     if (rs.nv) {
       auto vk = rs.nv == 1 ? residual_groupnorm_vec_kernel<T, 1> : rs.nv == 2 ? residual_groupnorm_vec_kernel<T, 2> : residual_groupnorm_vec_kernel<T, 4>;
-      vk<<<n, rs.threads, 0, e->stream>>>(e->x, y, w_post, w_pre, out, rows, D, G, eps);
+      TRY(launch_early(e, vk, n, rs.threads, 0, 1, e->x, y, w_post, w_pre, out, rows, D, G, eps));
     } else {
-      residual_groupnorm_kernel<T><<<n, norm_threads(D, G), 0, e->stream>>>(e->x, y, w_post, w_pre, out, rows, D, G, eps);
+      TRY(launch_early(e, residual_groupnorm_kernel<T>, n, norm_threads(D, G), 0, 1, e->x, y, w_post, w_pre, out, rows, D, G, eps));
     }
-    CK(cudaGetLastError());
-    e->launches++;
     return 0;
   };
   // x += groupnorm(pending sublayer output) * its post-norm weight;  h = groupnorm(x) * w_pre  (either half may be absent)
@@ -1920,9 +1845,7 @@ static int run_layers(xotb200_lm* e, const StepPlan& sp, int n_want) {
   };
   if (e->first) {
     auto ek = D % 4 == 0 ? embed_rows_kernel<T, 4> : embed_rows_kernel<T, 1>;
-    ek<<<M, D % 4 == 0 ? embed_threads(D) : 128, 0, e->stream>>>(at<T>(e, e->embed), sp.tokens, e->x, D);
-    CK(cudaGetLastError());
-    e->launches++;
+    TRY(launch_early(e, ek, M, D % 4 == 0 ? embed_threads(D) : 128, 0, 1, at<T>(e, e->embed), sp.tokens, e->x, D));
   }
   for (size_t li = 0; li < e->layers.size(); ++li) {
     LmLayer& L = e->layers[li];
@@ -1947,8 +1870,7 @@ static int run_layers(xotb200_lm* e, const StepPlan& sp, int n_want) {
     T* hw = static_cast<T*>(e->hw);
     TRY(norm_rows(nullptr, nullptr, at<T>(e, e->final_norm), hw, sp.want, n_want));
     TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    finish_logits(e, n_want);
-    CK(cudaGetLastError());
+    TRY(finish_logits(e, n_want));
   }
   return 0;
 }
@@ -2122,7 +2044,7 @@ int xotb200_lm_destroy(xotb200_lm* e) {
     if (L.rel_tab) cudaFree(L.rel_tab);
   }
   void* ptrs[] = {e->vfirst, e->oh2, e->y2, e->h0, e->gdec, e->ginw, e->gfloor, e->gnq, e->pos_freqs, e->dist_tab, e->moe_xg, e->moe_yg, e->moe_plan, e->dkk, e->drr, e->cvb, e->moe_ids, e->moe_wts, e->mact, e->du, e->dau, e->part, e->q16, e->cbuf, e->knx, e->vxx, e->blob, e->d_stage, e->x, e->y, e->proj, e->qraw, e->qfull, e->wlog, e->oraw, e->logits, e->h, e->cqn, e->qn, e->olat, e->oh, e->act,
-                  e->th, e->hw, e->d_argmax, e->trace_buf};
+                  e->th, e->hw, e->trace_buf};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (e->h_stage) cudaFreeHost(e->h_stage);
@@ -2315,8 +2237,7 @@ int xotb200_lm_clear_request(xotb200_lm* e, int slot) {
   e->slot_pages[slot] = 0;
   e->slot_len[slot] = 0;
   if (e->state_floats) {
-    CK(cudaMemsetAsync(e->state + (size_t)slot * e->state_floats, 0, e->state_floats * 4, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
+    CK(cudaMemsetAsync(e->state + (size_t)slot * e->state_floats, 0, e->state_floats * 4, e->stream));   // in stream order before the next step
   }
   return 0;
 }
@@ -2360,6 +2281,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   if (e->first)
     for (long m = 0; m < M; ++m) REQUIRE(tokens[m] >= 0 && tokens[m] < V, "token id %d outside the vocabulary of %d", tokens[m], V);
   TRY(ensure_scratch(e, (int)M, n_want));
+  e->early = M <= LST_MAX_ROWS;
   TRY(refresh_tables(e));
   // ---- commit: pages and lengths; the step's index arrays are built in one host vector and copied once
   const bool use_flash = e->esz == 2 && e->flash_on && e->flash_fits;
@@ -2476,7 +2398,8 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     e->stage_cap = cap;
   }
   memcpy(e->h_stage, st.data(), off * 4);
-  if (e->last && n_want > 0) TRY(ensure_host_out(e, (size_t)n_want * V + n_want));
+  const bool results = e->last && n_want > 0;
+  if (results) TRY(ensure_host_out(e, (size_t)n_want * V + n_want + 1));
   else if (!e->last) TRY(ensure_host_out(e, (size_t)M * (D + e->carry_out)));
   // Decoding — every request brings one row — has the same launches step after step: only the contents of the index arrays and
   // the lengths differ.  Such a step is captured into a CUDA graph the second time its shape is seen and replayed from then on.
@@ -2539,15 +2462,15 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
         if (e->carry_in) TRY(copy_rows(e->vfirst, e->carry_in, hidden_f32 + D, ld, e->carry_in, cudaMemcpyHostToDevice));
       }
       TRY(e->esz == 2 ? run_layers<bf16>(e, sp, n_want) : run_layers<float>(e, sp, n_want));
-      if (e->last && n_want > 0) {
-        if (logits_f32) CK(cudaMemcpyAsync(e->h_out, e->logits, (size_t)n_want * V * 4, cudaMemcpyDeviceToHost, e->stream));
-        if (argmax_i32) CK(cudaMemcpyAsync(e->h_out + (size_t)n_want * V, e->d_argmax, (size_t)n_want * 4, cudaMemcpyDeviceToHost, e->stream));
+      if (results) {
+        const size_t skip = logits_f32 ? 0 : (size_t)n_want * V;   // one copy: the logits when they are asked for, argmax, error word
+        CK(cudaMemcpyAsync(e->h_out + skip, e->logits + skip, ((size_t)n_want * V + n_want + 1 - skip) * 4, cudaMemcpyDeviceToHost, e->stream));
       } else if (!e->last) {
         const size_t ld = (size_t)D + e->carry_out;
         TRY(copy_rows(e->h_out, ld, e->x, D, D, cudaMemcpyDeviceToHost));
         if (e->carry_out) TRY(copy_rows(e->h_out + D, ld, e->vfirst, e->carry_out, e->carry_out, cudaMemcpyDeviceToHost));
       }
-      CK(cudaMemcpyAsync(e->h_err, e->d_err, 4, cudaMemcpyDeviceToHost, e->stream));
+      if (!results) CK(cudaMemcpyAsync(e->h_err, e->d_err, 4, cudaMemcpyDeviceToHost, e->stream));
       return 0;
     };
     rc = body();
@@ -2570,11 +2493,12 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   CK(cudaEventRecord(e->ev1, e->stream));
   CK(cudaStreamSynchronize(e->stream));
   CK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
-  if (*e->h_err != 0) {
-    set_err("a kernel gave up a bounded wait (device error word %d); the step's results are not valid", *e->h_err);
+  const int err = results ? reinterpret_cast<const int*>(e->h_out)[(size_t)n_want * V + n_want] : *e->h_err;
+  if (err != 0) {
+    set_err("a kernel gave up a bounded wait (device error word %d); the step's results are not valid", err);
     return XOTB200_ECUDA;
   }
-  if (e->last && n_want > 0) {
+  if (results) {
     if (logits_f32) memcpy(logits_f32, e->h_out, (size_t)n_want * V * 4);
     if (argmax_i32) memcpy(argmax_i32, e->h_out + (size_t)n_want * V, (size_t)n_want * 4);
   } else if (!e->last) {

@@ -32,6 +32,7 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 template <typename T, int VEC>
 __global__ void embed_pos_rows_kernel(const T* __restrict__ embed, const T* __restrict__ pos_table, const int* __restrict__ tokens,
                                       const int* __restrict__ row_pos, float* __restrict__ x, T* __restrict__ h, int D) {
+  pdl_enter();
   const int m = blockIdx.x;
   const T* src = embed + (size_t)tokens[m] * D;
   const T* ps = pos_table ? pos_table + (size_t)row_pos[m] * D : nullptr;
@@ -52,6 +53,7 @@ __global__ void embed_pos_rows_kernel(const T* __restrict__ embed, const T* __re
 // the T copy of an fp32 stream (a later shard starts from the residual stream it is given)
 template <typename T>
 __global__ void cast_rows_kernel(const float* __restrict__ x, T* __restrict__ h, size_t n) {
+  pdl_enter();
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) stf(h + i, x[i]);
 }
 
@@ -64,6 +66,7 @@ __global__ void cast_rows_kernel(const float* __restrict__ x, T* __restrict__ h,
 template <typename T>
 __global__ void residual_layernorm_kernel(float* __restrict__ x, const float* __restrict__ y, const T* __restrict__ y_bias, const T* __restrict__ w,
                                           const T* __restrict__ b, T* __restrict__ h, const int* __restrict__ src_rows, int D, float eps) {
+  pdl_enter();
   extern __shared__ float ln_row[];
   __shared__ float red[32];
   const int m = blockIdx.x;
@@ -94,6 +97,7 @@ template <typename T>
 __global__ void embed_sinusoid_rows_kernel(const T* __restrict__ embed, const T* __restrict__ pos_table, const float* __restrict__ freqs,
                                            const int* __restrict__ tokens, const int* __restrict__ row_pos, const T* __restrict__ w_norm, float w_offset,
                                            float eps, float* __restrict__ x, T* __restrict__ h, int D) {
+  pdl_enter();
   extern __shared__ float ln_row[];
   __shared__ float red[32];
   const int m = blockIdx.x;
@@ -127,6 +131,7 @@ __global__ void embed_sinusoid_rows_kernel(const T* __restrict__ embed, const T*
 template <typename T>
 __global__ void residual_rmsnorm_kernel(float* __restrict__ x, const float* __restrict__ y, const T* __restrict__ y_bias, const T* __restrict__ w,
                                         float w_offset, T* __restrict__ h, const int* __restrict__ src_rows, int D, float eps) {
+  pdl_enter();
   extern __shared__ float ln_row[];
   __shared__ float red[32];
   const int m = blockIdx.x;
@@ -159,6 +164,7 @@ __global__ void residual_norm_vec_kernel(float* __restrict__ x, const float* __r
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   float4 t[NV], xv[NV], wv[NV], bv[NV];
   int d[NV];
+  pdl_launch_dependents();
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     d[v] = (v * blockDim.x + threadIdx.x) * 4;
@@ -167,6 +173,7 @@ __global__ void residual_norm_vec_kernel(float* __restrict__ x, const float* __r
     bv[v] = on && !RMS ? ld4f(b + d[v]) : zero;
     t[v] = on && y && y_bias ? ld4f(y_bias + d[v]) : zero;
   }
+  pdl_wait();                                                  // the weights were under way meanwhile
   const size_t xm = y ? m : (src_rows ? src_rows[m] : m);
   float s = 0.f;
 #pragma unroll
@@ -215,6 +222,7 @@ template <typename T, int VEC>
 __global__ void parallel_rows_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ y2, const T* __restrict__ embed,
                                      const int* __restrict__ tokens, float embed_scale, const T* __restrict__ bigram, const int* __restrict__ bigram_row,
                                      const int* __restrict__ src_rows, const T* __restrict__ w, float eps, T* __restrict__ h, int D) {
+  pdl_enter();
   extern __shared__ __align__(16) float par_row[];             // read back by the writing thread only
   __shared__ float red[32];
   const size_t m = blockIdx.x, src = src_rows ? src_rows[m] : m;
@@ -265,6 +273,7 @@ __global__ void parallel_rows_kernel(float* __restrict__ x, const float* __restr
 template <typename T>
 __global__ void embed_dyt_rows_kernel(const T* __restrict__ embed, const int* __restrict__ tokens, const T* __restrict__ alpha, const T* __restrict__ w,
                                       const T* __restrict__ b, float* __restrict__ x, T* __restrict__ h, int D) {
+  pdl_enter();
   const size_t m = blockIdx.x;
   const T* src = embed + (size_t)tokens[m] * D;
   const float a = ldf(alpha);
@@ -277,12 +286,14 @@ __global__ void embed_dyt_rows_kernel(const T* __restrict__ embed, const int* __
 template <typename T>
 __global__ void dyt_rows_kernel(const float* __restrict__ x, const int* __restrict__ src_rows, const T* __restrict__ alpha, const T* __restrict__ w,
                                 const T* __restrict__ b, T* __restrict__ h, int D) {
+  pdl_enter();
   const size_t m = blockIdx.x, xm = src_rows ? src_rows[m] : m;
   const float a = ldf(alpha);
   for (int d = blockIdx.y * blockDim.x + threadIdx.x; d < D; d += gridDim.y * blockDim.x) stf(h + m * D + d, dyt_f(x[xm * D + d], a, ldf(w + d), ldf(b + d)));
 }
 template <typename T>
 __global__ void close_rows_kernel(const EpiArgs close, const float* __restrict__ y, int D) {
+  pdl_enter();
   const size_t m = blockIdx.x;
   for (int d = blockIdx.y * blockDim.x + threadIdx.x; d < D; d += gridDim.y * blockDim.x) stream_close<T>(close, m, d, y[m * D + d]);
 }
@@ -301,6 +312,7 @@ template <typename T, typename TO>
 __global__ void short_conv_kernel(const float* __restrict__ proj, int ld, int col0, int C, const T* __restrict__ w, const T* __restrict__ bias, int taps,
                                   int act, int residual, const Item* __restrict__ seqs, float* __restrict__ state, size_t state_slot_stride,
                                   TO* __restrict__ out, int ld_out) {
+  pdl_enter();
   const Item sq = seqs[blockIdx.x];
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= C) return;
@@ -360,6 +372,7 @@ __global__ void gated_delta_prepare_kernel(const float* __restrict__ cv, int C, 
                                            const T* __restrict__ a_log, const T* __restrict__ dt_bias, float* __restrict__ w_out,
                                            float* __restrict__ u_out, float* __restrict__ au_out, float* __restrict__ kk_out,
                                            float* __restrict__ r_out, int H, int G, int dk, int M) {
+  pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= M * H) return;
   const size_t m = idx / H;
@@ -517,6 +530,7 @@ template <typename T, int RPB>
 __global__ void __launch_bounds__(1024) moe_router_kernel(const T* __restrict__ h, int D, const T* __restrict__ w_router, const T* __restrict__ bias, int kind, int E,
                                   int groups, int keep, int top, const T* __restrict__ correction, int group_best, float wscale, int* __restrict__ ids,
                                   float* __restrict__ wts, int M) {
+  pdl_enter();
   extern __shared__ __align__(16) float rsm[];                 // [RPB][D] the rows (fp32), then [RPB] scores
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int m0 = blockIdx.x * RPB, nr = min(RPB, M - m0), Dp = (D + 3) & ~3, ns = moe_router_scores(kind, E, groups);
@@ -677,6 +691,7 @@ __global__ void __launch_bounds__(1024) moe_router_kernel(const T* __restrict__ 
 template <typename T>
 __global__ void moe_rows_up_kernel(const T* __restrict__ h, int D, const T* __restrict__ w_gu, int F, int expert_glu, const EpiArgs glu, const int* __restrict__ ids,
                                    int top, T* __restrict__ act, const T* __restrict__ w_shared, int Fs, T* __restrict__ act_shared) {
+  pdl_enter();
   extern __shared__ __align__(16) float hs[];                  // the row, fp32
   const int m = blockIdx.x, k = blockIdx.y;
   stage_f32(hs, h + (size_t)m * D, D);
@@ -715,6 +730,7 @@ template <typename T>
 __global__ void moe_rows_down_kernel(const T* __restrict__ act, int F, const T* __restrict__ w_down, int D, const int* __restrict__ ids,
                                      const float* __restrict__ wts, int top, int accumulate, float* __restrict__ y, const T* __restrict__ act_shared,
                                      const T* __restrict__ w_sdown, int Fs, const EpiArgs close) {
+  pdl_enter();
   extern __shared__ __align__(16) float as[];                  // [top][F] fp32, then [Fs] of the shared expert (from a 16-byte boundary)
   const int m = blockIdx.x;
   float* as_s = as + (((size_t)top * F + 3) & ~(size_t)3);
@@ -798,11 +814,13 @@ __global__ void moe_rows_down_kernel(const T* __restrict__ act, int F, const T* 
 // pair's result does not (rows of a product are independent).
 // ---------------------------------------------------------------------------------------------------------------------------
 __global__ void moe_count_kernel(const int* __restrict__ ids, int n_pairs, int* __restrict__ counts) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_pairs) atomicAdd(counts + ids[i], 1);
 }
 __global__ void moe_plan_kernel(int* __restrict__ counts, int E, int tile_rows, int n_tiles, int* __restrict__ starts, int* __restrict__ cursor,
                                 int* __restrict__ tile_expert) {
+  pdl_enter();
   __shared__ int s_total;
   if (threadIdx.x == 0) {
     int at = 0;
@@ -834,6 +852,7 @@ __global__ void moe_plan_kernel(int* __restrict__ counts, int E, int tile_rows, 
 template <typename T>
 __global__ void moe_scatter_kernel(const T* __restrict__ h, int D, const int* __restrict__ ids, int n_pairs, int top, const int* __restrict__ starts,
                                    int* __restrict__ cursor, int* __restrict__ place, T* __restrict__ xg) {
+  pdl_enter();
   const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= n_pairs) return;
   int p = 0;
@@ -855,6 +874,7 @@ __global__ void moe_scatter_kernel(const T* __restrict__ h, int D, const int* __
 template <typename T>
 __global__ void moe_combine_kernel(const float* __restrict__ yg, const int* __restrict__ place, const float* __restrict__ wts, int top, int D,
                                    int accumulate, float* __restrict__ y, const EpiArgs close) {
+  pdl_enter();
   const size_t m = blockIdx.x;
   for (int d = blockIdx.y * blockDim.x + threadIdx.x; d < D; d += gridDim.y * blockDim.x) {
     float acc = 0.f;
@@ -884,6 +904,7 @@ constexpr int HC_MAX_STREAMS = 8;
 template <typename T>
 __global__ void embed_streams_kernel(const T* __restrict__ embed, const int* __restrict__ tokens, const T* __restrict__ g, float eps, float* __restrict__ X,
                                      int S, int D) {
+  pdl_enter();
   __shared__ float red[32];
   const int m = blockIdx.x;
   const T* src = embed + (size_t)tokens[m] * D;
@@ -900,6 +921,7 @@ template <typename T, int SM, int VEC>   // SM: copies held per entry (>= S); VE
 __global__ void hc_open_kernel(float* __restrict__ X, int S, const float* __restrict__ y, const float* __restrict__ y2, float ya, float yb, float mult,
                                const T* __restrict__ mix, const T* __restrict__ outc, const T* __restrict__ inc, const T* __restrict__ g, float eps,
                                const int* __restrict__ src_rows, float* __restrict__ out_f32, T* __restrict__ out_t, int D) {
+  pdl_enter();
   extern __shared__ __align__(16) float hc_row[];
   __shared__ float red[32];
   __shared__ float c_mix[HC_MAX_STREAMS * HC_MAX_STREAMS], c_out[HC_MAX_STREAMS], c_in[HC_MAX_STREAMS];

@@ -106,6 +106,7 @@ __global__ void gqa_prepare_kernel(const float* __restrict__ proj, int ld, int c
                                    float q_temp_coef, int q_temp_every, const int* __restrict__ row_slot, const int* __restrict__ row_pos, Paging pg,
                                    T* __restrict__ pool, float* __restrict__ qf, bf16* __restrict__ q16, int M, int norm_on,
                                    const float* __restrict__ freqs, int rot_dims, int rot_layout) {
+  pdl_enter();
   const int slots = H + (own_kv ? 2 * G : 0);
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= M * slots) return;
@@ -157,6 +158,7 @@ __global__ void gqa_prepare_row_kernel(const float* __restrict__ proj, int ld, i
                                        const T* __restrict__ q_norm, const T* __restrict__ k_norm, float eps, int H, int G, int dk, int dv, int own_kv,
                                        float q_temp_coef, int q_temp_every, const int* __restrict__ row_slot, const int* __restrict__ row_pos, Paging pg,
                                        T* __restrict__ pool, float* __restrict__ qf, bf16* __restrict__ q16) {
+  pdl_enter();
   extern __shared__ float qk_row[];                            // [nq] q * q_norm, then [nk] k * k_norm; read back by the writing thread only
   __shared__ float red[2][32];
   const int m = blockIdx.x, nq = H * dk, nk = own_kv ? G * dk : 0, nv = own_kv ? G * dv : 0;
@@ -230,6 +232,7 @@ struct GqaPrep {
 template <typename T>
 __global__ void __launch_bounds__(128) gqa_filter_prepare_kernel(const GqaPrep a, const Item* __restrict__ seqs, Paging pg, T* __restrict__ pool, float* __restrict__ qf,
                                                                  bf16* __restrict__ q16) {
+  pdl_enter();
   extern __shared__ float prep_sm[];
   float* fs = prep_sm;                                         // [GQA_PREP_ROWS][dk]: filtered entries of the head being prepared
   float* cs = prep_sm + GQA_PREP_ROWS * a.dk;                  // [GQA_PREP_ROWS][rot_dims]: cosine, sine of every plane
@@ -382,6 +385,7 @@ __device__ __forceinline__ float4 fma4(float4 a, float4 b, float4 c) { return ma
 template <typename T, int TAPS, int NV>
 __global__ void __launch_bounds__(256, NV == 1 ? 3 : 2) gqa_filter_prepare_vec_kernel(const GqaPrep a, const Item* __restrict__ seqs, Paging pg, T* __restrict__ pool, float* __restrict__ qf,
                                                                      bf16* __restrict__ q16) {
+  pdl_enter();
   extern __shared__ __align__(16) float cs[];                  // [RB][rs]: cosine, sine of every plane
   constexpr int KEEP = TAPS - 1, RB = GQA_PREP_VEC_ROWS / NV;  // rows held at once
   __shared__ size_t prow[RB];                                  // their places in the pool
@@ -576,6 +580,7 @@ __device__ __forceinline__ float gqa_gate(const float* gate, int mode, size_t m,
 // ---------------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void gqa_pool_blocks_kernel(T* __restrict__ pool, Paging pg, size_t pool_rows, const Item* __restrict__ seqs, int P, int rowlen) {
+  pdl_enter();
   const Item sq = seqs[blockIdx.x];
   const int b = sq.pos0 / P + blockIdx.y;
   if (b >= (sq.pos0 + sq.n_rows) / P) return;
@@ -600,6 +605,7 @@ template <typename T, int NACC>
 __global__ void gqa_attention_kernel(const float* __restrict__ qf, const T* __restrict__ pool, Paging pg, const Item* __restrict__ items, int H,
                                      int G, int dk, int dv, GqaScore sc, const float* __restrict__ gate, int gate_mode, int gate_ld, int gate_col0,
                                      T* __restrict__ out, int chunk_keys, float* __restrict__ part) {
+  pdl_enter();
   extern __shared__ float smem[];
   const Item it = items[blockIdx.x];
   const int rep = H / G, W = dk + dv, WS = W | 1;
@@ -703,6 +709,7 @@ __global__ void gqa_attention_kernel(const float* __restrict__ qf, const T* __re
 template <typename T>
 __global__ void gqa_combine_kernel(const float* __restrict__ part, const Item* __restrict__ items, int H, int dv, int splits, const T* __restrict__ sink,
                                    int sink_one, const float* __restrict__ gate, int gate_mode, int gate_ld, int gate_col0, T* __restrict__ out) {
+  pdl_enter();
   const Item it = items[blockIdx.x];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int pair = blockIdx.y * nw + warp;
@@ -741,6 +748,7 @@ __global__ void gqa_combine_kernel(const float* __restrict__ part, const Item* _
 // dist_table[a][d] = r1[a] * ln(1 + r2[a] * d) for d < n: the distance penalty of head a, made once per step and layer so that the
 // prompt kernel reads it instead of taking a logarithm per score
 __global__ void gqa_dist_table_kernel(const bf16* __restrict__ r1, const bf16* __restrict__ r2, int H, int n, float* __restrict__ table) {
+  pdl_enter();
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= (size_t)H * n) return;
   const int a = (int)(i / n), d = (int)(i % n);
@@ -759,6 +767,7 @@ __global__ void __launch_bounds__(128)
 gqa_flash_kernel(const bf16* __restrict__ q16, const bf16* __restrict__ pool, Paging pg, const GqaTile* __restrict__ tiles, int H, int G, int dk, int dv,
                  GqaScore sc, const float* __restrict__ dist_table, int dist_n, const float* __restrict__ gate, int gate_mode, int gate_ld, int gate_col0,
                  bf16* __restrict__ out) {
+  pdl_enter();
   extern __shared__ __align__(16) uint8_t gsm[];
   __shared__ size_t krow[2][64];                    // pool rows of the keys of the tile in flight / in use
   __shared__ float dpen[2][128];                    // distance terms (learned bias - penalty) a (64 rows x 64 keys) tile can meet: distance = dbase + index

@@ -25,6 +25,11 @@ typedef __nv_bfloat16 bf16;
 // Both do nothing in a kernel launched the ordinary way.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// first statement of a kernel with nothing to do before its inputs are there: its launch latency is hidden, no more
+__device__ __forceinline__ void pdl_enter() {
+  pdl_launch_dependents();
+  pdl_wait();
+}
 
 template <typename T> __device__ __forceinline__ float ldf(const T* p);
 template <> __device__ __forceinline__ float ldf<float>(const float* p) { return *p; }
@@ -170,6 +175,7 @@ struct Paging {
 // trip instead of one per loop pass.
 template <typename T, int VEC>
 __global__ void embed_rows_kernel(const T* __restrict__ embed, const int* __restrict__ tokens, float* __restrict__ x, int D) {
+  pdl_enter();
   const int m = blockIdx.x;
   const T* src = embed + (size_t)tokens[m] * D;
 #pragma unroll 4
@@ -189,6 +195,7 @@ template <typename T>
 __global__ void residual_groupnorm_kernel(float* __restrict__ x, const float* __restrict__ y, const T* __restrict__ w_post,
                                           const T* __restrict__ w_pre, T* __restrict__ h, const int* __restrict__ src_rows, int D, int G,
                                           float eps) {
+  pdl_enter();
   // `wpg` warps share one part (each a slice of it); their sums of squares meet in shared memory.  All warps walk the same
   // number of rounds, so the barriers are uniform.
   __shared__ float red[2][32];
@@ -253,6 +260,7 @@ __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   float4 xv[NV], yv[NV], wo[NV], wp[NV];
   int d[NV];
+  pdl_launch_dependents();
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     d[v] = (v * blockDim.x + threadIdx.x) * 4;
@@ -260,6 +268,7 @@ __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float
     wo[v] = on && y ? ld4f(w_post + d[v]) : zero;
     wp[v] = on && h ? ld4f(w_pre + d[v]) : zero;
   }
+  pdl_wait();                                                  // the weights were under way meanwhile
   const size_t xm = src_rows ? src_rows[m] : m;
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
@@ -311,6 +320,7 @@ __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float
 template <typename T>
 __global__ void rmsnorm_cols_kernel(const float* __restrict__ in, int ld_in, int col0, int n, const T* __restrict__ w, T* __restrict__ out,
                                     int ld_out, int M, float eps) {
+  pdl_enter();
   const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (m >= M) return;
   const float* r = in + (size_t)m * ld_in + col0;
@@ -342,6 +352,7 @@ __global__ void latent_prepare_kernel(const float* __restrict__ qraw, int q_ld, 
                                       const T* __restrict__ w_norm, float eps, const float* __restrict__ freqs, int rot_dims, int layout,
                                       const int* __restrict__ row_slot, const int* __restrict__ row_pos, Paging pg, T* __restrict__ pool, T* __restrict__ qn,
                                       float* __restrict__ qfull, bf16* __restrict__ q16, int M) {
+  pdl_enter();
   const long idx = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (idx >= (long)M * (H + 1)) return;
@@ -428,6 +439,7 @@ __global__ void __launch_bounds__(NACC > 8 ? 512 : 1024)
 latent_attention_kernel(const float* __restrict__ qfull, const T* __restrict__ pool, Paging pg, const Item* __restrict__ items, int H, int R, int dr, float scale,
                         int window, const float* __restrict__ gate, int gate_ld, int gate_col0, const T* __restrict__ sink, T* __restrict__ olat, int chunk,
                         float* __restrict__ part, int nbuf) {
+  pdl_enter();
   extern __shared__ __align__(16) uint32_t lsm[];
   constexpr int VPW = 4 / sizeof(T);                // values per word
   const Item it = items[blockIdx.x];
@@ -554,6 +566,7 @@ latent_attention_kernel(const float* __restrict__ qfull, const T* __restrict__ p
 template <typename T>
 __global__ void latent_attention_combine_kernel(const float* __restrict__ part, const Item* __restrict__ items, int H, int R, int splits,
                                                 const float* __restrict__ gate, int gate_ld, int gate_col0, const T* __restrict__ sink, T* __restrict__ olat) {
+  pdl_enter();
   const Item it = items[blockIdx.x];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int pair = blockIdx.y * nw + warp;
@@ -597,6 +610,7 @@ __global__ void latent_attention_combine_kernel(const float* __restrict__ part, 
 template <typename T>
 __global__ void delta_prepare_kernel(const float* __restrict__ proj, int ld, int col_k, int col_a, float* __restrict__ wlog, const T* __restrict__ w_bias,
                                      const T* __restrict__ a_bias, float* __restrict__ u_out, float* __restrict__ au_out, int H, int dk, int M) {
+  pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= M * H) return;
   const size_t m = idx / H;
@@ -628,6 +642,7 @@ template <int KPT, int P, int NC>
 __global__ void delta_rule_kernel(DeltaSrc ksrc, DeltaSrc rsrc, DeltaSrc vsrc, const float* __restrict__ wdec,
                                   const float* __restrict__ uvec, const float* __restrict__ auvec, const Item* __restrict__ seqs, int H, int dk,
                                   int dv, float* __restrict__ state, size_t state_slot_stride, float* __restrict__ o_raw, int vec4) {
+  pdl_enter();
   constexpr int DKP = KPT * P;                       // padded size: >= dk and >= dv
   constexpr int CH = DKP <= 64 ? 16 : DKP <= 128 ? 8 : 4;   // tokens per buffer: two buffers fill the 48 KB of static shared memory
   __shared__ __align__(16) float buf[2][CH][6][DKP]; // per token: w, a*u, u, k, r, v
@@ -743,6 +758,7 @@ template <typename T>
 __global__ void head_norm_gate_kernel(const float* __restrict__ o_raw, const float* __restrict__ nq, const float* __restrict__ den_floor,
                                       const T* __restrict__ w_norm, int w_head_stride, const float* __restrict__ gate, int gate_ld, int gate_col0, int gate_silu,
                                       T* __restrict__ out, int H, int dv, float eps, int M) {
+  pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= M * H) return;
   const int m = idx / H, h = idx % H;
@@ -760,6 +776,7 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o_raw, const flo
 // out[m, :n] = tanh(in[m, col0 : col0 + n])  (fp32 in, T out): the low-rank decay branch between its two products
 template <typename T>
 __global__ void tanh_cols_kernel(const float* __restrict__ in, int ld, int col0, int n, T* __restrict__ out, int M) {
+  pdl_enter();
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= (size_t)M * n) return;
   const size_t m = i / n, d = i % n;
@@ -776,6 +793,7 @@ template <typename TA, typename TB, typename TC, int EPI>
 __global__ void __launch_bounds__(256)
 gemm_tiled_kernel(const TA* __restrict__ A, long lda, long a_batch, const TB* __restrict__ B, long sbn, long sbk, long b_batch, TC* __restrict__ C,
                   long ldc, long c_batch, int M, int N, int K, const EpiArgs epi) {
+  pdl_enter();
   constexpr int BM = 64, BN = 64, BK = 16;
   __shared__ float As[BK][BM + 4], Bs[BK][BN + 4];
   A += (size_t)blockIdx.z * a_batch;
@@ -853,9 +871,7 @@ gemv_rows_kernel(const TA* __restrict__ A, long lda, long a_batch, const TB* __r
   A += (size_t)blockIdx.z * a_batch;
   B += (size_t)blockIdx.z * b_batch;
   C += (size_t)blockIdx.z * c_batch;
-  for (int m = 0; m < M; ++m) stage_f32(a_s + (size_t)m * K, A + (size_t)m * lda, K);
-  float* red = a_s + (size_t)M * K;
-  __syncthreads();
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gpb = 8 / wsplit, grp = warp / wsplit, slice = warp % wsplit;
   constexpr int VEC = 16 / sizeof(TB);
@@ -863,14 +879,37 @@ gemv_rows_kernel(const TA* __restrict__ A, long lda, long a_batch, const TB* __r
   const int step = vec_ok ? 32 * VEC : 32;
   const int ksl = ((K + wsplit - 1) / wsplit + step - 1) / step * step;
   const int kbeg = slice * ksl, kend = min(K, kbeg + ksl);
-  for (int nb = blockIdx.x * gpb * RB; nb < N; nb += gridDim.x * gpb * RB) {   // uniform trip count for the whole block
-    const int n0 = nb + grp * RB;
-    size_t brow[RB];                                 // element offset of the group's weight rows
+  auto rows_of = [&](int n0, size_t (&brow)[RB]) {     // element offset of a group's weight rows
 #pragma unroll
     for (int r = 0; r < RB; ++r) {
       brow[r] = (size_t)(n0 + r) * sbn;
       if constexpr (epi_is_glu(EPI)) brow[r] = (r & 1 ? glu_up_row((n0 + r) >> 1, N >> 1, epi.il8) : glu_gate_row((n0 + r) >> 1, N >> 1, epi.il8)) * (size_t)sbn;
     }
+  };
+  auto load = [&](uint4 (&raw)[2][RB], int n0, const size_t (&brow)[RB], int k) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int r = 0; r < RB; ++r)
+        raw[u][r] = (n0 + r < N && k + u * 32 * VEC < kend) ? *reinterpret_cast<const uint4*>(B + brow[r] + k + u * 32 * VEC) : make_uint4(0, 0, 0, 0);
+  };
+  // the first weights do not depend on the kernel in front: they are on their way while it ends and the rows are staged
+  uint4 raw[2][RB];
+  bool have = vec_ok;
+  if (have) {
+    const int n0 = blockIdx.x * gpb * RB + grp * RB;
+    size_t brow[RB];
+    rows_of(n0, brow);
+    load(raw, n0, brow, kbeg + lane * VEC);
+  }
+  pdl_wait();
+  for (int m = 0; m < M; ++m) stage_f32(a_s + (size_t)m * K, A + (size_t)m * lda, K);
+  float* red = a_s + (size_t)M * K;
+  __syncthreads();
+  for (int nb = blockIdx.x * gpb * RB; nb < N; nb += gridDim.x * gpb * RB) {   // uniform trip count for the whole block
+    const int n0 = nb + grp * RB;
+    size_t brow[RB];
+    rows_of(n0, brow);
     float acc[RB][MR];
 #pragma unroll
     for (int r = 0; r < RB; ++r)
@@ -879,13 +918,8 @@ gemv_rows_kernel(const TA* __restrict__ A, long lda, long a_batch, const TB* __r
     if (vec_ok) {
       // two steps of the slice at a time: 2 x RB independent 16-byte loads per lane are in flight before the first FMA
       for (int k = kbeg + lane * VEC; k < kend; k += 64 * VEC) {
-        uint4 raw[2][RB];
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int r = 0; r < RB; ++r)
-            raw[u][r] = (n0 + r < N && k + u * 32 * VEC < kend) ? *reinterpret_cast<const uint4*>(B + brow[r] + k + u * 32 * VEC)
-                                                                : make_uint4(0, 0, 0, 0);
+        if (!have) load(raw, n0, brow, k);
+        have = false;
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const int ku = min(k + u * 32 * VEC, K - VEC);     // past the slice the weights read as zero; the index stays inside a_s
@@ -951,7 +985,9 @@ gemv_rows_kernel(const TA* __restrict__ A, long lda, long a_batch, const TB* __r
 
 // finishes the logits of every row in place — l <- l * scale, then l <- cap * tanh(l / cap) when cap > 0 — and takes the
 // lowest-index argmax of the row (greedy sampling on the device)
-__global__ void argmax_rows_kernel(float* __restrict__ logits, int V, float scale, float cap, int* __restrict__ out) {
+// also hands the step's error word on behind the rows' results, so that all of them reach the host in one copy
+__global__ void argmax_rows_kernel(float* __restrict__ logits, int V, float scale, float cap, int* __restrict__ out, const int* __restrict__ err) {
+  pdl_enter();
   __shared__ float bv[32];
   __shared__ int bi[32];
   float* r = logits + (size_t)blockIdx.x * V;
@@ -1000,6 +1036,7 @@ __global__ void argmax_rows_kernel(float* __restrict__ logits, int V, float scal
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
       if (bv[w] > best || (bv[w] == best && bi[w] < idx)) { best = bv[w]; idx = bi[w]; }
     out[blockIdx.x] = idx;
+    if (blockIdx.x == 0) out[gridDim.x] = *err;
   }
 }
 
@@ -1089,6 +1126,7 @@ struct FlashTile {
 
 template <typename T>
 __global__ void latent_gather_kernel(const T* __restrict__ pool, Paging pg, const GatherReq* __restrict__ reqs, int W, T* __restrict__ cbuf) {
+  pdl_enter();
   const GatherReq rq = reqs[blockIdx.y];
   const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= rq.nkeys) return;
@@ -1121,6 +1159,7 @@ __global__ void __launch_bounds__(128)
 latent_flash_kernel(const bf16* __restrict__ q16, const bf16* __restrict__ kn, const bf16* __restrict__ cbuf, const bf16* __restrict__ vx,
                     const FlashTile* __restrict__ tiles, int H, int dn, int dr, int dv, int R, float scale, int window, const float* __restrict__ gate,
                     int gate_ld, int gate_col0, const bf16* __restrict__ sink, bf16* __restrict__ out) {
+  pdl_enter();
   extern __shared__ __align__(16) uint8_t fsm[];
   const FlashTile tl = tiles[blockIdx.x];
   const int h = blockIdx.y;
@@ -1285,6 +1324,7 @@ __global__ void __launch_bounds__(128)
 latent_flash_aligned_kernel(const bf16* __restrict__ q16, const bf16* __restrict__ kn, const bf16* __restrict__ cbuf, const bf16* __restrict__ vx,
                             const FlashTile* __restrict__ tiles, int H, int dn, int dr, int dv, int R, float scale, int window,
                             const float* __restrict__ gate, int gate_ld, int gate_col0, const bf16* __restrict__ sink, bf16* __restrict__ out) {
+  pdl_enter();
   extern __shared__ __align__(16) uint8_t fsm[];
   const FlashTile tl = tiles[blockIdx.x];
   const int h = blockIdx.y;

@@ -26,6 +26,7 @@ template <typename T>
 __global__ void mlstm_gates_kernel(const float* __restrict__ proj, int ld, int col_i, int col_f, const T* __restrict__ b_i, const T* __restrict__ b_f,
                                    float cap, const Item* __restrict__ seqs, int n_seq, int H, float* __restrict__ m_state, size_t state_slot_stride,
                                    float* __restrict__ decay, float* __restrict__ inw, float* __restrict__ floor_out) {
+  pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= n_seq * H) return;
   const Item sq = seqs[idx / H];
@@ -63,6 +64,7 @@ __global__ void mlstm_gates_kernel(const float* __restrict__ proj, int ld, int c
 __global__ void mlstm_expand_kernel(const float* __restrict__ proj, int ld, int col_q, int col_k, const float* __restrict__ decay,
                                     const float* __restrict__ inw, float* __restrict__ w_out, float* __restrict__ kk_out, float* __restrict__ r_out,
                                     int H, int dk, int M) {
+  pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= M * H) return;
   const size_t m = idx / H;
@@ -85,6 +87,7 @@ __global__ void mlstm_expand_kernel(const float* __restrict__ proj, int ld, int 
 // the new state.  (One row per request, decoding: one warp, one pass.)
 __global__ void mlstm_normaliser_kernel(const float* __restrict__ kk, const float* __restrict__ r, const float* __restrict__ decay, const Item* __restrict__ seqs,
                                         int H, int dk, float* __restrict__ n_state, size_t state_slot_stride, float* __restrict__ nq) {
+  pdl_enter();
   constexpr int E = 8, TB = 4;
   __shared__ float seg_n[32][E * 32];
   __shared__ float seg_p[32];
@@ -153,6 +156,7 @@ template <typename T>
 __global__ void mamba2_prepare_kernel(const float* __restrict__ cv, int C, const float* __restrict__ proj, int ld, int col_dt, const T* __restrict__ a_log,
                                       const T* __restrict__ dt_bias, float* __restrict__ w_out, float* __restrict__ kk_out, float* __restrict__ r_out,
                                       int H, int G, int N, int dv, int M) {
+  pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= M * H) return;
   const size_t m = idx / H;
@@ -175,6 +179,7 @@ __global__ void mamba2_prepare_kernel(const float* __restrict__ cv, int C, const
 template <typename T>
 __global__ void mamba2_out_kernel(const float* __restrict__ o_raw, const float* __restrict__ cv, int C, const float* __restrict__ proj, int ld, int col_z,
                                   const T* __restrict__ Dskip, const T* __restrict__ w_norm, int H, int dv, int parts, float eps, T* __restrict__ out) {
+  pdl_enter();
   extern __shared__ float gated[];
   __shared__ float red[32];
   const size_t m = blockIdx.x / parts;

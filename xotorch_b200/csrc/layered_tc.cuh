@@ -59,6 +59,7 @@ __device__ __forceinline__ void ltc_load16(__nv_bfloat16* dst, const __nv_bfloat
 template <int NT, int EPI, int NS, typename TC>
 __global__ void __launch_bounds__(LTC_THREADS, 2 * ltc_smem_bytes(NT, NS) <= 226 * 1024 ? 2 : 1)
 ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LtcArgs a) {
+  pdl_enter();
   extern __shared__ __align__(1024) uint8_t ltc_smem[];
   constexpr int A_BYTES = LTC_M * LTC_BK * 2;
   constexpr int STAGE = ltc_stage_bytes(NT);
