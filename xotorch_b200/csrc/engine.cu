@@ -123,6 +123,11 @@ struct LayerW {
   bf16* router;                                           // MoE: [E, D] row-major
 };
 
+// tensor maps of one activation buffer: box of 128 rows (token tiles), and of 64, 32, 16 rows (few token rows)
+struct ActMaps {
+  CUtensorMap full, r64, r32, r16;
+};
+
 struct xotb200_engine {
   xotb200_model_cfg cfg;
   int device = 0, sm_count = 148;
@@ -189,13 +194,10 @@ struct xotb200_engine {
   int l2_ahead = 0;                // decode producer look-ahead into L2 (stages per CTA)
   int max_inflight = 0;            // decode producer window (bulk copies in flight per CTA, 0 = ring depth)
   unsigned int pace_q = 0;         // decode producer pacing, 2^-16 ns per byte per CTA (0 = off)
-  float* tc_ws = nullptr;          // split-K partial tiles of the one-tile prefill GEMMs, and their tickets
-  size_t tc_ws_bytes = 0;
-  unsigned int* tc_ws_ticket = nullptr;
   bool tc_fuse = true;             // RoPE/KV-append and SwiGLU fused into GEMM epilogues (XOTB200_TC_FUSE=0: separate kernels, A/B)
-  int prefill_mode = 0;            // 0 auto (TC when n_tokens >= 8), 1 always the decode kernel, 2 always TC
+  int prefill_mode = 0;            // 0 auto (runs_as_gemms), 1 always the decode kernel, 2 always TC
   bf16 *tc_x = nullptr, *tc_xn = nullptr, *tc_qkv = nullptr, *tc_q = nullptr, *tc_ao = nullptr, *tc_gu = nullptr, *tc_act = nullptr;
-  CUtensorMap tm_xn, tm_ao, tm_act;
+  ActMaps tm_xn, tm_ao, tm_act;
   std::map<int, std::vector<CUtensorMap>> tm_w;   // per N-tile width: 4 per local layer (qkv, o, gu, down) + head
   int tc_cap = 0;                  // token rows the tensor-core scratch buffers currently hold
   // sparse MoE prefill: gathered per-expert row blocks (rows_max = 2 * tc_cap + E * 128) and the device-side plan
@@ -373,18 +375,24 @@ static encode_tiled_fn get_encode_tiled() {
   }
   return fn;
 }
-// activations [rows, K] row-major bf16 (rows a multiple of 128) -> box {64 k, 128 rows}, SWIZZLE_128B
-static int make_tmap_act(CUtensorMap* m, bf16* ptr, int K, int rows = TC_M) {
+// activations [rows, K] row-major bf16 (rows a multiple of 128) -> box {64 k, box_rows rows}, SWIZZLE_128B
+static int make_tmap_act(CUtensorMap* m, bf16* ptr, int K, int rows = TC_M, int box_rows = TC_M) {
   encode_tiled_fn enc = get_encode_tiled();
   REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled not available from the driver");
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)TC_M};
+  const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
   const cuuint32_t es[2] = {1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(activation K=%d) failed: %d", K, (int)r);
   return 0;
+}
+static int make_act_maps(ActMaps* m, bf16* ptr, int K, int rows) {
+  if (int rc = make_tmap_act(&m->full, ptr, K, rows)) return rc;
+  if (int rc = make_tmap_act(&m->r64, ptr, K, rows, 64)) return rc;
+  if (int rc = make_tmap_act(&m->r32, ptr, K, rows, 32)) return rc;
+  return make_tmap_act(&m->r16, ptr, K, rows, 16);
 }
 // weights in K-panel layout [K/tk][N][tk] -> 3-D map {tk, N, K/tk}, box {64 k, nt rows, 1}, SWIZZLE_128B
 static int make_tmap_w(CUtensorMap* m, const bf16* ptr, int N, int K, int tk, int nt) {
@@ -433,6 +441,53 @@ static int ensure_smem_attr(int device, const void* fn, int bytes) {
   return 0;
 }
 
+// A launch that may start before the kernel in front of it has finished (every kernel of the dense prompt path waits for it itself: pdl_wait), in
+// clusters of `cluster` CTAs along x (0 or 1: none, or the kernel fixes its cluster shape itself).
+template <typename... KA, typename... A>
+static int launch_early(xotb200_engine* e, cudaStream_t st, void (*fn)(KA...), dim3 grid, int threads, size_t smem, int cluster, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim = {(unsigned)cluster, 1, 1};
+  cfg.attrs = at;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  CK(cudaLaunchKernelEx(&cfg, fn, static_cast<KA>(args)...));
+  e->launches++;
+  return 0;
+}
+
+// GEMM of one tile of token rows (a.S <= 128; HEAD_LAST: one row) as a weight stream: tc_stream_kernel.  K is cut over 1, 2, 4 or 8 CTAs, doubled
+// while two CTAs per SM are not exceeded and each keeps two K blocks or more.
+template <int NB>
+static int launch_tc_stream_nb(xotb200_engine* e, const CUtensorMap& tmW, const CUtensorMap& tmX, const TcGemmArgs& a, int epi, int splits, cudaStream_t st) {
+  void (*fn)(CUtensorMap, CUtensorMap, TcGemmArgs) = nullptr;
+  const bool f16 = e->cfg.dtype == XOTB200_DTYPE_F16;
+  switch (epi) {
+    case TCE_STORE: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_STORE> : xb::bf::tc_stream_kernel<NB, TCE_STORE>; break;
+    case TCE_RESID: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_RESID> : xb::bf::tc_stream_kernel<NB, TCE_RESID>; break;
+    case TCE_QKV: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_QKV> : xb::bf::tc_stream_kernel<NB, TCE_QKV>; break;
+    case TCE_SWIGLU: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_SWIGLU> : xb::bf::tc_stream_kernel<NB, TCE_SWIGLU>; break;
+    default: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_HEAD_LAST> : xb::bf::tc_stream_kernel<NB, TCE_HEAD_LAST>; break;
+  }
+  if (int rc = ensure_smem_attr(e->device, (const void*)fn, tcs_smem_bytes(NB))) return rc;
+  return launch_early(e, st, fn, dim3(splits, a.N / TC_M), TC_THREADS, tcs_smem_bytes(NB), splits, tmW, tmX, a);
+}
+static int launch_tc_stream(xotb200_engine* e, const CUtensorMap& tmW, const ActMaps& x, const TcGemmArgs& a_in, int epi, cudaStream_t st) {
+  TcGemmArgs a = a_in;
+  a.err = &e->ctl->err;
+  const int nb = epi == TCE_HEAD_LAST || a.S <= 16 ? 16 : a.S <= 32 ? 32 : a.S <= 64 ? 64 : 128, tiles = a.N / TC_M, nkb = a.K / TC_BK;
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= 2 * e->sm_count && nkb >= 4 * s) s *= 2;
+  return nb == 16 ? launch_tc_stream_nb<16>(e, tmW, x.r16, a, epi, s, st) : nb == 32 ? launch_tc_stream_nb<32>(e, tmW, x.r32, a, epi, s, st)
+       : nb == 64 ? launch_tc_stream_nb<64>(e, tmW, x.r64, a, epi, s, st) : launch_tc_stream_nb<128>(e, tmW, x.full, a, epi, s, st);
+}
+
 template <int NT, int NS>
 static int launch_tc_gemm_nt(xotb200_engine* e, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcGemmArgs& a, int epi,
                              cudaStream_t st) {
@@ -447,10 +502,7 @@ static int launch_tc_gemm_nt(xotb200_engine* e, const CUtensorMap& tmA, const CU
   }
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, tc_smem_bytes(NT, NS))) return rc;
   const int mtiles = a.grid_m > 0 ? a.grid_m : (epi == TCE_HEAD_LAST ? 1 : (a.S + TC_M - 1) / TC_M - a.mt0);
-  fn<<<dim3(mtiles, a.N / NT, a.ksplit > 1 ? a.ksplit : 1), TC_THREADS, tc_smem_bytes(NT, NS), st>>>(tmA, tmB, a);
-  CK(cudaGetLastError());
-  e->launches++;
-  return 0;
+  return launch_early(e, st, fn, dim3(mtiles, a.N / NT), TC_THREADS, tc_smem_bytes(NT, NS), 1, tmA, tmB, a);
 }
 // persistent variant (one CTA per SM, two TMEM accumulators): used when a launch has more output tiles than SMs
 template <int NT, int NS>
@@ -466,10 +518,7 @@ static int launch_tc_gemm_persistent(xotb200_engine* e, const CUtensorMap& tmA, 
     default: fn = f16 ? xb::fp::tc_gemm_persistent_kernel<NT, TCE_HEAD_LAST, NS> : xb::bf::tc_gemm_persistent_kernel<NT, TCE_HEAD_LAST, NS>; break;
   }
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, tc_smem_bytes(NT, NS))) return rc;
-  fn<<<std::min(tiles, e->sm_count), TC_THREADS, tc_smem_bytes(NT, NS), st>>>(tmA, tmB, a);
-  CK(cudaGetLastError());
-  e->launches++;
-  return 0;
+  return launch_early(e, st, fn, std::min(tiles, e->sm_count), TC_THREADS, tc_smem_bytes(NT, NS), 1, tmA, tmB, a);
 }
 
 // CTA-pair variant (cta_group::2): clusters of two CTAs, one 256-token x NT tile per pair; tmB is the weight map with a box of NT/2 rows
@@ -489,10 +538,7 @@ static int launch_tc_gemm_2sm(xotb200_engine* e, const CUtensorMap& tmA, const C
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, tc2_smem_bytes(NT, NS))) return rc;
   const int total = ((a.S + 2 * TC_M - 1) / (2 * TC_M)) * (a.N / NT);
   const int pairs = std::max(1, std::min(total, e->sm_count / 2));
-  fn<<<2 * pairs, TC_THREADS, tc2_smem_bytes(NT, NS), st>>>(tmA, tmB_half, a);
-  CK(cudaGetLastError());
-  e->launches++;
-  return 0;
+  return launch_early(e, st, fn, 2 * pairs, TC_THREADS, tc2_smem_bytes(NT, NS), 0, tmA, tmB_half, a);
 }
 
 static int launch_tc_gemm(xotb200_engine* e, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcGemmArgs& a_in, int epi, TcCfg c,
@@ -579,46 +625,23 @@ static int prepare_tc(xotb200_engine* e, int n_tokens) {
       if (int rc = make_tmap_act(&e->tm_moe_xg, e->moe_xg, (int)D, (int)rows)) return rc;
       if (int rc = make_tmap_act(&e->tm_moe_act, e->moe_act, (int)F, (int)rows)) return rc;
     }
-    if (int rc = make_tmap_act(&e->tm_xn, e->tc_xn, (int)D, need)) return rc;
-    if (int rc = make_tmap_act(&e->tm_ao, e->tc_ao, (int)qd, need)) return rc;
+    if (int rc = make_act_maps(&e->tm_xn, e->tc_xn, (int)D, need)) return rc;
+    if (int rc = make_act_maps(&e->tm_ao, e->tc_ao, (int)qd, need)) return rc;
     if (c.n_experts == 0)
-      if (int rc = make_tmap_act(&e->tm_act, e->tc_act, (int)F, need)) return rc;
+      if (int rc = make_act_maps(&e->tm_act, e->tc_act, (int)F, need)) return rc;
   }
   return 0;
 }
 
 // one GEMM of the prefill: weight `widx` of the shard (see ensure_tm_w), tile configuration from (N, tokens in flight)
-static int tc_gemm(xotb200_engine* e, const CUtensorMap& tmA, int widx, const TcGemmArgs& a, int epi, cudaStream_t st) {
+static int tc_gemm(xotb200_engine* e, const ActMaps& tm, int widx, const TcGemmArgs& a, int epi, cudaStream_t st) {
   const TcCfg c = tc_cfg(a.N, epi == TCE_HEAD_LAST ? 1 : a.S);
-  // ONE token tile (S <= 128): the GEMM streams the weight once and is bound by how many SMs pull on it.  N / NT tiles
-  // of the narrow GEMMs (O, down: 32 tiles of 128; QKV: 48) leave most SMs idle and every CTA re-reads the whole [128, K]
-  // activation tile; split-K puts ksplit CTAs on each tile, each reading only its K slice of both operands.
-  static const bool use_splitk = !(getenv("XOTB200_TC_SPLITK") && atoi(getenv("XOTB200_TC_SPLITK")) == 0);
-  if (use_splitk && a.S <= TC_M && a.mt0 == 0 && a.tile_info == nullptr && a.N % 128 == 0 &&
-      (epi == TCE_STORE || epi == TCE_RESID || epi == TCE_QKV)) {
-    const int tiles = a.N / 128, nkb = a.K / TC_BK;
-    int ks = std::min(4, e->sm_count / std::max(1, tiles));
-    while (ks > 1 && nkb % ks != 0) --ks;
-    if (ks >= 2 && nkb / ks >= 4) {
-      const size_t need = (size_t)tiles * ks * TC_M * 128 * 4;
-      if (need > e->tc_ws_bytes) {
-        CK(cudaStreamSynchronize(st));
-        if (e->tc_ws) CK(cudaFree(e->tc_ws));
-        e->tc_ws = nullptr;
-        CK(cudaMalloc(&e->tc_ws, need));
-        e->tc_ws_bytes = need;
-      }
-      if (!e->tc_ws_ticket) {
-        CK(cudaMalloc(&e->tc_ws_ticket, 4096 * 4));
-        MEMSET_SYNC(e, e->tc_ws_ticket, 0, 4096 * 4);
-      }
-      REQUIRE(tiles <= 4096, "split-K ticket table too small for N=%d", a.N);
-      if (int rc = ensure_tm_w(e, 128)) return rc;
-      TcGemmArgs b = a;
-      b.ksplit = ks; b.ws = e->tc_ws; b.ws_ticket = e->tc_ws_ticket; b.err = &e->ctl->err;
-      return launch_tc_gemm_nt<128, 6>(e, tmA, e->tm_w[128][widx], b, epi, st);
-    }
+  // ONE token tile (S <= 128), or the head's one row: the GEMM streams the weight once
+  if ((epi == TCE_HEAD_LAST || (a.S <= TC_M && a.mt0 == 0)) && a.tile_info == nullptr && a.N % TC_M == 0) {
+    if (int rc = ensure_tm_w(e, TC_M)) return rc;
+    return launch_tc_stream(e, e->tm_w[TC_M][widx], tm, a, epi, st);
   }
+  const CUtensorMap& tmA = tm.full;
   // several 256-token tiles in flight and a 256-wide N tile: CTA pairs (each CTA stages half of the weight tile)
   static const bool use_2sm = !(getenv("XOTB200_TC_2SM") && atoi(getenv("XOTB200_TC_2SM")) == 0);
   if (use_2sm && epi != TCE_HEAD_LAST && a.tile_info == nullptr && a.mt0 == 0 && c.nt == 256 && a.S > 2 * TC_M && a.N % 256 == 0 &&
@@ -648,10 +671,7 @@ static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, i
   auto fn = f16 ? xb::fp::tc_flash_attn_kernel<HD> : xb::bf::tc_flash_attn_kernel<HD>;
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, SMEM)) return rc;
   const float scale_log2 = 1.4426950408889634f / sqrtf((float)HD);
-  fn<<<dim3((S + 63) / 64, e->cfg.n_heads), 128, SMEM, st>>>(e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
-  CK(cudaGetLastError());
-  e->launches++;
-  return 0;
+  return launch_early(e, st, fn, dim3((S + 63) / 64, e->cfg.n_heads), 128, SMEM, 1, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
 }
 
 // Prefill n_tokens positions starting at pos0 on the tensor cores, in chunks of up to TC_CHUNK tokens (layer-major
@@ -662,12 +682,11 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
   const xotb200_model_cfg& c = e->cfg;
   const int D = c.dim, F = c.ffn, Hq = c.n_heads, Hkv = c.n_kv_heads, hd = c.head_dim;
   const int qd = Hq * hd, nqkv = (Hq + 2 * Hkv) * hd, nl = e->end - e->start + 1;
+  auto rmsnorm = c.dtype == XOTB200_DTYPE_F16 ? xb::fp::tc_rmsnorm_kernel : xb::bf::tc_rmsnorm_kernel;
   for (int m0 = 0; m0 < n_tokens; m0 += TC_CHUNK) {
     const int S = std::min(TC_CHUNK, n_tokens - m0);
     if (e->first) {
-      tc_gather_kernel<<<S, 128, 0, st>>>(e->stage_tokens + m0, e->embed, e->tc_x, D);
-      CK(cudaGetLastError());
-      e->launches++;
+      if (int rc = launch_early(e, st, tc_gather_kernel, S, 128, 0, 1, e->stage_tokens + m0, e->embed, e->tc_x, D)) return rc;
     } else {
       CK(cudaMemcpyAsync(e->tc_x, e->stage_in + (size_t)m0 * D, (size_t)S * D * 2, cudaMemcpyDeviceToDevice, st));
     }
@@ -675,8 +694,7 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
       const LayerW& w = e->layers[li];
       bf16* kc = e->kv + (size_t)e->cur_req * e->kv_req_stride + ((size_t)li * 2 + 0) * Hkv * e->L * hd;
       bf16* vc = e->kv + (size_t)e->cur_req * e->kv_req_stride + ((size_t)li * 2 + 1) * Hkv * e->L * hd;
-      DT_LAUNCH(e, (tc_rmsnorm_kernel<<<S, 256, 0, st>>>(e->tc_x, w.attn_norm, e->tc_xn, D, c.norm_eps)));
-      CK(cudaGetLastError());
+      if (int rc = launch_early(e, st, rmsnorm, S, 256, 0, 1, e->tc_x, w.attn_norm, e->tc_xn, D, c.norm_eps)) return rc;
       if (e->tc_fuse) {     // RoPE + KV append in the QKV GEMM's epilogue: rotated q -> tc_q, k / v -> the cache rows of this chunk
         TcGemmArgs g{S, nqkv, D, e->tk, e->tc_q, nullptr, qd, 0};
         g.kc = kc; g.vc = vc; g.rope = e->rope; g.q_rows = qd; g.kv_rows = Hkv * hd; g.hd = hd; g.L = e->L; g.pos0 = pos0 + m0;
@@ -693,8 +711,7 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
         return rc;
       TcGemmArgs o{S, D, qd, e->tk, e->tc_x, nullptr, D, 0};
       if (int rc = tc_gemm(e, e->tm_ao, 4 * li + 1, o, TCE_RESID, st)) return rc;
-      DT_LAUNCH(e, (tc_rmsnorm_kernel<<<S, 256, 0, st>>>(e->tc_x, w.mlp_norm, e->tc_xn, D, c.norm_eps)));
-      CK(cudaGetLastError());
+      if (int rc = launch_early(e, st, rmsnorm, S, 256, 0, 1, e->tc_x, w.mlp_norm, e->tc_xn, D, c.norm_eps)) return rc;
       if (c.n_experts > 0) {
         // ---- sparse MoE MLP: router -> plan -> gather -> per-expert gate/up -> SwiGLU -> per-expert down -> combine ----
         const int E = c.n_experts, rows = e->moe_rows, max_tiles = (S + TC_M - 1) / TC_M, avg_rows = std::max(1, 2 * S / E);
@@ -717,7 +734,7 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
         }
         DT_LAUNCH(e, (moe_combine_kernel<<<S, 256, 0, st>>>(e->tc_x, e->moe_y, e->moe_row_of, e->moe_route_w, D)));
         CK(cudaGetLastError());
-        e->launches += 7;   // 2 RMSNorm + router, plan, gather, SwiGLU, combine (RoPE/KV counted above when it is a kernel)
+        e->launches += 5;   // router, plan, gather, SwiGLU, combine
         continue;
       }
       if (e->tc_fuse) {     // SwiGLU in the gate/up GEMM's epilogue: [S, F] written instead of [S, 2F] + a kernel
@@ -732,18 +749,14 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
       }
       TcGemmArgs d{S, D, F, e->tk, e->tc_x, nullptr, D, 0};
       if (int rc = tc_gemm(e, e->tm_act, 4 * li + 3, d, TCE_RESID, st)) return rc;
-      e->launches += 2;   // the two RMSNorm kernels (the GEMM / attention launchers count themselves)
     }
     if (e->last) {
       if (m0 + S == n_tokens) {   // logits of the last position only (sharded_inference_engine.py:365-368)
-        const int mt_last = (S - 1) / TC_M, r0 = mt_last * TC_M;   // only the tile holding the last position
-        DT_LAUNCH(e, (tc_rmsnorm_kernel<<<S - r0, 256, 0, st>>>(e->tc_x + (size_t)r0 * D, e->final_norm, e->tc_xn + (size_t)r0 * D, D, c.norm_eps)));
-        CK(cudaGetLastError());
+        const int mt_last = (S - 1) / TC_M, r0 = c.vocab % TC_M == 0 ? S - 1 : mt_last * TC_M;   // the last position, or the tile holding it
+        if (int rc = launch_early(e, st, rmsnorm, S - r0, 256, 0, 1, e->tc_x + (size_t)r0 * D, e->final_norm, e->tc_xn + (size_t)r0 * D, D, c.norm_eps)) return rc;
         TcGemmArgs h{S, c.vocab, D, e->tk, nullptr, e->logits, 0, mt_last};
         if (int rc = tc_gemm(e, e->tm_xn, 4 * nl, h, TCE_HEAD_LAST, st)) return rc;
-        tc_argmax_kernel<<<1, 1024, 0, st>>>(e->logits, c.vocab, e->ctl);
-        CK(cudaGetLastError());
-        e->launches += 2;
+        if (int rc = launch_early(e, st, tc_argmax_kernel, 1, 1024, 0, 1, e->logits, c.vocab, e->ctl)) return rc;
       }
     } else {
       CK(cudaMemcpyAsync(e->stage_out + (size_t)m0 * D, e->tc_x, (size_t)S * D * 2, cudaMemcpyDeviceToDevice, st));
@@ -959,7 +972,7 @@ int xotb200_destroy(xotb200_engine* e) {
   cudaDeviceSynchronize();
   free_shard(e);
   if (e->next_ipc && e->next_inbox) cudaIpcCloseMemHandle(e->next_inbox);
-  void* tcp[] = {e->tc_ws, e->tc_ws_ticket, e->tc_x, e->tc_xn, e->tc_qkv, e->tc_q, e->tc_ao, e->tc_gu, e->tc_act, e->moe_xg, e->moe_gu, e->moe_act, e->moe_y,
+  void* tcp[] = {e->tc_x, e->tc_xn, e->tc_qkv, e->tc_q, e->tc_ao, e->tc_gu, e->tc_act, e->moe_xg, e->moe_gu, e->moe_act, e->moe_y,
                  e->moe_route_e, e->moe_route_w, e->moe_row_of, e->moe_row_token, e->moe_exp_info};
   for (void* p : tcp)
     if (p) cudaFree(p);
@@ -1308,6 +1321,12 @@ static int ensure_staging(xotb200_engine* e, int n) {
   return 0;
 }
 
+// Positions from which a call runs as GEMMs (prefill_tc) instead of one after the other through the decode kernel.  A dense shard streams its
+// weights once either way for one position, and once instead of n times for more; a sparse-MoE shard pays its per-expert launches first.
+static bool runs_as_gemms(const xotb200_engine* e, int n_tokens) {
+  return e->prefill_mode == 2 || (e->prefill_mode == 0 && n_tokens >= (e->cfg.n_experts > 0 ? 8 : 2));
+}
+
 int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidden_f32, int n_tokens, int pos0,
                     float* out_f32) {
   REQUIRE(e && e->start >= 0, "no shard set");
@@ -1333,7 +1352,7 @@ int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidde
     CK(cudaGetLastError());
     e->launches++;
   }
-  const bool use_tc = e->prefill_mode == 2 || (e->prefill_mode == 0 && n_tokens >= 8);
+  const bool use_tc = runs_as_gemms(e, n_tokens);
   if (use_tc) {
     if (int rc = prefill_tc(e, n_tokens, pos0, st)) return rc;     // GEMM-shaped: 5th-gen tensor cores
   } else {
@@ -1378,7 +1397,7 @@ int xotb200_forward_device(xotb200_engine* e, const int32_t* tokens, const void*
   } else {
     CK(cudaMemcpyAsync(e->stage_in, hidden_dev, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
   }
-  const bool use_tc = e->prefill_mode == 2 || (e->prefill_mode == 0 && n_tokens >= 8);
+  const bool use_tc = runs_as_gemms(e, n_tokens);
   if (use_tc) {
     if (int rc = prefill_tc(e, n_tokens, pos0, st)) return rc;
   } else {
@@ -1438,7 +1457,7 @@ int xotb200_forward_hop(xotb200_engine* e, const int32_t* tokens, int64_t seq_in
   e->hop_out = (!e->last && decode) ? 1 : 0;
   e->hop_seq_in = (unsigned int)seq_in;
   e->hop_seq_out = seq;
-  const bool use_tc = e->prefill_mode == 2 || (e->prefill_mode == 0 && n_tokens >= 8);
+  const bool use_tc = runs_as_gemms(e, n_tokens);
   int rc = use_tc ? prefill_tc(e, n_tokens, pos0, st) : launch_mega(e, 1, n_tokens, 0, pos0, st);
   e->hop_in = e->hop_out = 0;
   if (rc) return rc;
@@ -1698,12 +1717,14 @@ int xotb200_debug_gemm(xotb200_engine* e, const void* a_bf16, const void* w_bf16
   MEMCPY_SYNC(e, dW0, w_bf16, (size_t)N * K * 2, cudaMemcpyHostToDevice);
   relayout_rows_kernel<<<N, 128, 0, e->stream>>>(dW0, dW, N, K, 0, e->cfg.head_dim, 1, 0, N, tk);
   CK(cudaGetLastError());
-  CUtensorMap tA, tB;
-  int rc = make_tmap_act(&tA, dA, K);
-  if (!rc) rc = make_tmap_w(&tB, dW, N, K, tk, tc_nt(N));
+  ActMaps tA;
+  CUtensorMap tB;
+  const bool stream = N % TC_M == 0;                     // as tc_gemm chooses
+  int rc = make_act_maps(&tA, dA, K, TC_M);
+  if (!rc) rc = make_tmap_w(&tB, dW, N, K, tk, stream ? TC_M : tc_nt(N));
   if (!rc) {
     TcGemmArgs g{S, N, K, tk, dO, nullptr, N, 0};
-    rc = launch_tc_gemm(e, tA, tB, g, TCE_STORE, tc_cfg(N, S), e->stream);
+    rc = stream ? launch_tc_stream(e, tB, tA, g, TCE_STORE, e->stream) : launch_tc_gemm(e, tA.full, tB, g, TCE_STORE, tc_cfg(N, S), e->stream);
   }
   cudaError_t er = cudaStreamSynchronize(e->stream);
   if (!rc && er == cudaSuccess) {

@@ -41,12 +41,6 @@ struct TcGemmArgs {
   bf16 *kc, *vc;          // K / V cache of (request, layer): [Hkv][L][hd]
   const float2* rope;     // [L][hd/2] (cos, sin)
   int q_rows, kv_rows, hd, L, pos0;
-  // split-K (one 128-token tile: the GEMM is weight-streaming bound and N / NT tiles do not fill the GPU): grid.z = ksplit CTAs
-  // share an output tile, each sweeps K / ksplit; fp32 partial tiles go through `ws`, the CTA drawing the last ticket of the tile
-  // adds them in split order (deterministic) and runs the epilogue
-  int ksplit;             // 1 = off
-  float* ws;              // [tile][ksplit][128][NT] fp32
-  unsigned int* ws_ticket;   // [tile], zero between launches (the last CTA resets its entry)
   int* err;               // sticky device error word (StepCtl::err): 3 = a bounded wait of the persistent GEMM expired
 };
 
@@ -157,11 +151,25 @@ __device__ __forceinline__ void umma_commit_2sm(uint64_t* bar, uint16_t mask) {
 __host__ __device__ constexpr int tc2_stage_bytes(int nt) { return TC_M * TC_BK * 2 + (nt / 2) * TC_BK * 2; }   // per CTA: own A rows + half of B
 __host__ __device__ constexpr int tc2_smem_bytes(int nt, int ns) { return ns * tc2_stage_bytes(nt) + 1024 + 256; }
 
+// ---- few token rows (tc_stream_kernel): 128 weight rows are the M operand, NB token rows the N side; two CTAs share an SM's shared memory
+__host__ __device__ constexpr int tcs_stage_bytes(int nb) { return TC_M * TC_BK * 2 + nb * TC_BK * 2; }
+__host__ __device__ constexpr int tcs_stages(int nb) { return nb <= 16 ? 6 : nb <= 32 ? 5 : nb <= 64 ? 4 : 3; }
+__host__ __device__ constexpr int tcs_smem_bytes(int nb) { return tcs_stages(nb) * tcs_stage_bytes(nb) + 1024 + 256; }
+constexpr int TCS_LD = TC_M + 4;      // floats per row of a CTA's partial tile (16-byte pieces of neighbouring rows in different banks)
+static_assert(tcs_smem_bytes(16) <= 112 * 1024 && tcs_smem_bytes(32) <= 112 * 1024 && tcs_smem_bytes(64) <= 112 * 1024 && tcs_smem_bytes(128) <= 112 * 1024, "two CTAs per SM");
+static_assert(128 * TCS_LD * 4 <= tcs_stages(128) * tcs_stage_bytes(128), "the partial tile reuses the ring");
+__device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr, uint32_t rank) {   // from the shared memory of CTA `rank` of the cluster
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(mapa_shared(addr, rank)) : "memory");
+  return v;
+}
+
 // ------------------------------------------------------------------------------------------------------------
 // row-parallel helpers around the GEMMs
 // ------------------------------------------------------------------------------------------------------------
 // x[s, :] = embed[tokens[s], :]   (first shard)
 __global__ void tc_gather_kernel(const int* tokens, const bf16* embed, bf16* x, int D) {
+  pdl_enter();
   const uint4* s4 = reinterpret_cast<const uint4*>(embed + (size_t)tokens[blockIdx.x] * D);
   uint4* d4 = reinterpret_cast<uint4*>(x + (size_t)blockIdx.x * D);
   for (int c = threadIdx.x; c < D / 8; c += blockDim.x) d4[c] = s4[c];
@@ -169,6 +177,7 @@ __global__ void tc_gather_kernel(const int* tokens, const bf16* embed, bf16* x, 
 
 // lowest-index arg-max of logits[0..V) -> ctl->token   (single block of 1024 threads)
 __global__ void __launch_bounds__(1024) tc_argmax_kernel(const float* logits, int V, StepCtl* ctl) {
+  pdl_enter();
   __shared__ float sv[32];
   __shared__ int si[32];
   float bv = -INFINITY;
