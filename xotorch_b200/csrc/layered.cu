@@ -32,6 +32,7 @@
 #include "layered_recurrent.cuh"
 #include "layered_tc.cuh"
 #include "layered_stream.cuh"
+#include "layered_fma.cuh"
 #include "st_header.h"
 
 using namespace xl;
@@ -842,6 +843,35 @@ static int product_tc(xotb200_lm* e, const bf16* A, long lda, long a_batch, cons
   return 1;
 }
 
+// 32-bit product of more rows than the decode kernel takes; 1 = launched, 0 = operands that are not whole 16-byte pieces
+template <int RM, int EPI>
+static int launch_fma(xotb200_lm* e, const float* A, long lda, long a_batch, const float* B, long ldb, long b_batch, float* C, long ldc, long c_batch, int M, int N, int K,
+                      int batch, const EpiArgs& epi) {
+  auto kern = gemm_fma_kernel<RM, EPI>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fma_smem_bytes(RM)));
+  const int n_tiles = cdiv(N, FMA_BN), tiles = n_tiles * cdiv(M, 8 * RM), nkb = cdiv(K, FMA_BK);
+  int s = 1;
+  while (s < 8 && (long)tiles * batch * s * 2 <= 2L * e->sm_count && nkb >= 4 * s) s *= 2;
+  return launch_early(e, kern, dim3(s, tiles, batch), FMA_THREADS, fma_smem_bytes(RM), s, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, n_tiles, epi);
+}
+template <int EPI>
+static int product_fma(xotb200_lm* e, const float* A, long lda, long a_batch, const float* B, long ldb, long b_batch, float* C, long ldc, long c_batch, int M, int N, int K,
+                       int batch, const EpiArgs& epi) {
+  if (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) || (lda | ldb | K) % 4 || (batch > 1 && (a_batch | b_batch) % 4) || (long)cdiv(N, FMA_BN) * cdiv(M, 16) > 65535)
+    return 0;
+  // rows per tile: the height that leaves the fewest empty rows in all, the taller one when equal (B is read once per row tile)
+  int best = 2;
+  for (int rm : {4, 6, 8, 10, 12})
+    if (cdiv(M, 8 * rm) * rm <= cdiv(M, 8 * best) * best) best = rm;
+  const int r = best == 2   ? launch_fma<2, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi)
+                : best == 4 ? launch_fma<4, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi)
+                : best == 6 ? launch_fma<6, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi)
+                : best == 8 ? launch_fma<8, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi)
+                : best == 10 ? launch_fma<10, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi)
+                             : launch_fma<12, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi);
+  return r < 0 ? r : 1;
+}
+
 template <typename TA, typename TB, typename TC, int EPI>
 static int product(xotb200_lm* e, const TA* A, long lda, long a_batch, const TB* B, long sbn, long sbk, long b_batch, TC* C, long ldc, long c_batch,
                    int M, int N, int K, int batch, const EpiArgs& epi = EpiArgs{}) {
@@ -872,6 +902,11 @@ static int product(xotb200_lm* e, const TA* A, long lda, long a_batch, const TB*
     else LAUNCH_GEMV(8);
 #undef LAUNCH_GEMV
   } else {
+    if constexpr (std::is_same<TA, float>::value && std::is_same<TB, float>::value && std::is_same<TC, float>::value)
+      if (e->gemm_mode != 1 && sbk == 1) {
+        const int r = product_fma<EPI>(e, A, lda, a_batch, B, sbn, b_batch, C, ldc, c_batch, M, N, K, batch, epi);
+        if (r != 0) return r < 0 ? r : 0;
+      }
     TRY(launch_late(e, gemm_tiled_kernel<TA, TB, TC, EPI>, dim3(cdiv(N, 64), cdiv(M, 64), batch), 256, 0, A, lda, a_batch, B, sbn, sbk, b_batch, C, ldc, c_batch, M, N, K, epi));
   }
   return 0;
@@ -1125,37 +1160,37 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   return 0;
 }
 
+// which of the recurrence's forms a mixer uses (delta_rule_kernel)
+enum DeltaForm { DELTA_VECTOR, DELTA_VECTOR_NO_REMOVAL, DELTA_SCALAR };
 template <int KPT, int P, int NC>
-static int launch_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks, DeltaSrc rs, DeltaSrc vs, int dk, int dv, bool removal) {
+static int launch_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks, DeltaSrc rs, DeltaSrc vs, int dk, int dv, DeltaForm form) {
   const xotb200_lm_layer& s = L.s;
   constexpr int CPW = (32 / P) * NC;
   const int warps = std::max(1, std::min(4, cdiv(dv, CPW)));
   const dim3 grid(sp.n_seq * s.heads, cdiv(dv, warps * CPW));
   const int HD = s.heads * dk;
   const int vec4 = (dk % 4 == 0 && dv % 4 == 0 && HD % 4 == 0 && (ks.ld | ks.col | rs.ld | rs.col | vs.ld | vs.col) % 4 == 0) ? 1 : 0;
-  TRY(launch_early(e, delta_rule_kernel<KPT, P, NC>, grid, warps * 32, 0, 1, ks, rs, vs, e->wlog, removal ? e->du : nullptr, removal ? e->dau : nullptr, sp.seqs, s.heads, dk, dv,
-                                                                    e->state + L.state_off, e->state_floats, e->oraw, vec4));
-  return 0;
+  auto kern = form == DELTA_SCALAR ? delta_rule_kernel<KPT, P, NC, true, true> : form == DELTA_VECTOR ? delta_rule_kernel<KPT, P, NC, false, true> : delta_rule_kernel<KPT, P, NC, false, false>;
+  return launch_early(e, kern, grid, warps * 32, 0, 1, ks, rs, vs, e->wlog, e->du, e->dau, sp.seqs, s.heads, dk, dv, e->state + L.state_off, e->state_floats, e->oraw, vec4);
 }
-// The recurrence is bound by the instructions one warp issues per token (measured: ~2.8 cycles each with one warp per scheduler):
-// key rows over 4 or 8 lanes, few columns per thread, four warps per block.  The variant is chosen by the larger of the key and
-// value sizes; of the columns-per-thread choices the widest that still gives CTAs for three quarters of the SMs (a single prompt has only
-// heads x column groups CTAs: narrower threads mean more CTAs and more warps per scheduler to hide the dependent latency).
-// dk x dv: the state of a head (the mixers that ride on this kernel say what that is); removal: the rule has its - au (u^T S) term
-static int run_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks, DeltaSrc rs, DeltaSrc vs, int dk, int dv, bool removal) {
+// The recurrence is bound by the chain of one token and by instruction issue: key rows over 4 or 8 lanes, few columns per thread, four warps
+// per block.  The variant is chosen by the larger of the key and value sizes; of the columns-per-thread choices the widest that still gives CTAs
+// for three quarters of the SMs (a single prompt has only heads x column groups CTAs: narrower threads mean more CTAs and more warps per
+// scheduler to hide the dependent latency).  dk x dv: the state of a head (the mixers that ride on this kernel say what that is).
+static int run_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks, DeltaSrc rs, DeltaSrc vs, int dk, int dv, DeltaForm form) {
   const int d = std::max(dk, dv);
   auto fills = [&](int P, int NC) {                    // CTAs of a variant against the SMs
     const int cpw = (32 / P) * NC, warps = std::max(1, std::min(4, cdiv(dv, cpw)));
     return 4L * sp.n_seq * L.s.heads * cdiv(dv, warps * cpw) >= 3L * e->sm_count;
   };
-  if (d <= 16) return launch_delta<4, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, removal);
-  if (d <= 32) return fills(4, 2) ? launch_delta<8, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, removal) : launch_delta<8, 4, 1>(e, L, sp, ks, rs, vs, dk, dv, removal);
+  if (d <= 16) return launch_delta<4, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, form);
+  if (d <= 32) return fills(4, 2) ? launch_delta<8, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, form) : launch_delta<8, 4, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
   if (d <= 64)
-    return fills(8, 4) ? launch_delta<8, 8, 4>(e, L, sp, ks, rs, vs, dk, dv, removal)
-         : fills(8, 2) ? launch_delta<8, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, removal)
-                       : launch_delta<8, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, removal);
-  if (d <= 128) return fills(8, 2) ? launch_delta<16, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, removal) : launch_delta<16, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, removal);
-  return launch_delta<32, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, removal);
+    return fills(8, 4) ? launch_delta<8, 8, 4>(e, L, sp, ks, rs, vs, dk, dv, form)
+         : fills(8, 2) ? launch_delta<8, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form)
+                       : launch_delta<8, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
+  if (d <= 128) return fills(8, 2) ? launch_delta<16, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form) : launch_delta<16, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
+  return launch_delta<32, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
 }
 
 template <typename T>
@@ -1168,7 +1203,7 @@ static int delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   TRY((product<T, T, float, 0>(e, static_cast<T*>(e->th), s.low_rank, 0, at<T>(e, L.w2), s.low_rank, 1, 0, e->wlog, HD, 0, M, HD, s.low_rank, 1)));
   TRY(launch_early(e, delta_prepare_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->proj, L.n_in, L.c_k, L.c_a, e->wlog, at<T>(e, L.w0), at<T>(e, L.a_b), e->du, e->dau,
                                                                               s.heads, s.dim, M));
-  TRY(run_delta(e, L, sp, DeltaSrc{e->proj, L.n_in, L.c_k}, DeltaSrc{e->proj, L.n_in, L.c_r}, DeltaSrc{e->proj, L.n_in, L.c_v}, s.dim, s.vdim, true));
+  TRY(run_delta(e, L, sp, DeltaSrc{e->proj, L.n_in, L.c_k}, DeltaSrc{e->proj, L.n_in, L.c_r}, DeltaSrc{e->proj, L.n_in, L.c_v}, s.dim, s.vdim, DELTA_VECTOR));
   TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), s.vdim, e->proj, L.n_in, L.c_g, 0,
                                                                                static_cast<T*>(e->oh), s.heads, s.vdim, e->cfg.norm_eps, M));
   TRY(output_product<T>(e, static_cast<T*>(e->oh), L.wo, HD, e->y, M));
@@ -1351,9 +1386,9 @@ static int gated_delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, floa
   const xotb200_lm_layer& s = L.s;
   const int M = sp.M, H = s.heads, G = s.kv_heads, dk = s.dim, dv = s.vdim, C = L.conv_ch;
   TRY(filter_channels<T>(e, L, sp, L.c_r, C, nullptr));
-  TRY(launch_early(e, gated_delta_prepare_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
-                                                                            e->du, e->dau, e->dkk, e->drr, H, G, dk, M));
-  TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, H * dk, 0}, DeltaSrc{e->drr, H * dk, 0}, DeltaSrc{e->cvb, C, 2 * G * dk}, dk, dv, true));
+  TRY(launch_early(e, gated_delta_prepare_kernel<T>, cdiv((long)M * G, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
+                   e->dau, e->dkk, e->drr, H, G, dk, M));
+  TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, G * dk, 0, H / G}, DeltaSrc{e->drr, G * dk, 0, H / G}, DeltaSrc{e->cvb, C, 2 * G * dk}, dk, dv, DELTA_SCALAR));
   TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), 0, e->proj, L.ld_in, L.c_g, 1, static_cast<T*>(ohbuf),
                                                                        H, dv, e->cfg.norm_eps, M));
   TRY(output_product<T>(e, static_cast<T*>(ohbuf), L.wo, H * dv, yout, M));
@@ -1371,7 +1406,7 @@ static int matrix_lstm_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, floa
   TRY(launch_early(e, mlstm_expand_kernel, cdiv((long)M * H, 8), 256, 0, 1, e->proj, L.ld_in, L.c_r, L.c_k, e->gdec, e->ginw, e->wlog, e->dkk, e->drr, H, dk, M));
   TRY(launch_early(e, mlstm_normaliser_kernel, sp.n_seq * H, 32 * std::max(1, std::min(16, sp.max_rows / 16)), 0, 1, e->dkk, e->drr, e->gdec, sp.seqs, H, dk, e->state + L.n_off,
                                                                                                         e->state_floats, e->gnq));
-  TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, H * dk, 0}, DeltaSrc{e->drr, H * dk, 0}, DeltaSrc{e->proj, L.ld_in, L.c_v}, dk, dv, false));
+  TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, H * dk, 0}, DeltaSrc{e->drr, H * dk, 0}, DeltaSrc{e->proj, L.ld_in, L.c_v}, dk, dv, DELTA_VECTOR_NO_REMOVAL));
   TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->oraw, e->gnq, e->gfloor, at<T>(e, L.onorm), dv, e->proj, L.ld_in, L.c_g, 0,
                                                                        static_cast<T*>(ohbuf), H, dv, e->cfg.norm_eps, M));
   TRY(output_product<T>(e, static_cast<T*>(ohbuf), L.wo, H * dv, yout, M));
@@ -1387,7 +1422,7 @@ static int mamba2_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
   TRY(filter_channels<T>(e, L, sp, L.c_v, C, at<T>(e, L.conv_b)));
   TRY(launch_early(e, mamba2_prepare_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_dt, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog, e->dkk, e->drr,
                                                                        H, G, N, dv, M));
-  TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, H * N, 0}, DeltaSrc{e->drr, H * N, 0}, DeltaSrc{e->cvb, C, 0}, N, dv, false));
+  TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, H * N, 0}, DeltaSrc{e->drr, H * N, 0}, DeltaSrc{e->cvb, C, 0}, N, dv, DELTA_VECTOR_NO_REMOVAL));
   {
     const int part = inner / s.out_norm_groups;
     auto ok = mamba2_out_kernel<T>;

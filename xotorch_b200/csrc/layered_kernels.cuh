@@ -628,66 +628,104 @@ __global__ void delta_prepare_kernel(const float* __restrict__ proj, int ld, int
   }
 }
 
-// A thread owns NC value columns x KPT key rows of the state (row i = e * P + part), so the token's vectors, read from shared
-// memory once, serve NC columns and the NC recurrences run as independent chains.  vec4: every source row is 16-byte aligned
-// (sizes and offsets multiples of 4 floats), so the staging uses 16-byte cp.async.
-// uvec == NULL: the rule has no removal term (S <- diag(w) S + k v^T): u and a * u are neither staged nor applied.
-// The write key k, the read-out vector r and the value v each come from their own fp32 matrix (pointer, leading dimension, first
-// column; head a's vector at column a * dk, resp. a * dv): a projection output or a prepared buffer.
+// A thread owns NC value columns x KPT key rows of the state.  The rows come in runs of four, row 4 (q P + part) + r, so that a token's vector is
+// read four entries per shared-memory load, and state and vectors are kept as PAIRS of fp32 that one packed instruction (fma.rn.f32x2: two
+// independent fp32 FMAs) works on: a head of 128 x 128 takes some 130 instructions a token and warp instead of 270.  The chain from token to
+// token is dot product -> sum over the P lanes -> update; the read-outs of four tokens are summed over the lanes together afterwards, off it.
+// SCALAR: the head has ONE decay and ONE write strength per token, S <- g S + k (beta (v - g (k^T S)))^T: three vectors and two numbers are staged
+// instead of six vectors (wdec = g, auvec = beta, both [M, H]).  Else S <- diag(w) S - au (u^T S) + k v^T with wdec, uvec, auvec [M, H * dk]; REMOVAL 0:
+// without the u term (u and au are neither staged nor applied).  vec4: every source row is 16-byte aligned (sizes and offsets multiples of 4
+// floats), so the staging uses 16-byte cp.async.
+// The write key k, the read-out vector r and the value v each come from their own fp32 matrix (pointer, leading dimension, first column; head a's
+// vector at column a / rep * dk, resp. a * dv): a projection output or a prepared buffer.
+// Bound by the latency of the chain and the issue of one or two warps per scheduler, not by memory.
 struct DeltaSrc {
   const float* p;
   int ld, col;
+  int rep = 1;                                       // heads that share a vector
 };
-template <int KPT, int P, int NC>
-__global__ void delta_rule_kernel(DeltaSrc ksrc, DeltaSrc rsrc, DeltaSrc vsrc, const float* __restrict__ wdec,
+typedef unsigned long long f32x2;                    // two fp32 in a register pair
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+template <int KPT, int P, int NC, bool SCALAR, bool REMOVAL>
+__global__ void __launch_bounds__(128) delta_rule_kernel(DeltaSrc ksrc, DeltaSrc rsrc, DeltaSrc vsrc, const float* __restrict__ wdec,
                                   const float* __restrict__ uvec, const float* __restrict__ auvec, const Item* __restrict__ seqs, int H, int dk,
                                   int dv, float* __restrict__ state, size_t state_slot_stride, float* __restrict__ o_raw, int vec4) {
   pdl_enter();
   constexpr int DKP = KPT * P;                       // padded size: >= dk and >= dv
-  constexpr int CH = DKP <= 64 ? 16 : DKP <= 128 ? 8 : 4;   // tokens per buffer: two buffers fill the 48 KB of static shared memory
-  __shared__ __align__(16) float buf[2][CH][6][DKP]; // per token: w, a*u, u, k, r, v
+  constexpr int NVEC = SCALAR ? 3 : 6;               // k, r, v (then w, u, au)
+  constexpr int CH = DKP <= 64 ? 16 : DKP <= 128 ? 8 : 4;   // tokens per buffer: two buffers fit the 48 KB of static shared memory
+  constexpr int Q = KPT / 4, TG = 4;                 // runs of four rows per thread; tokens whose read-outs are summed together
+  __shared__ __align__(16) float buf[2][CH][NVEC][DKP];
+  __shared__ float gb[2][CH][2];                     // SCALAR: g, beta
   const Item sq = seqs[blockIdx.x / H];
   const int h = blockIdx.x % H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int CPW = (32 / P) * NC;                 // columns per warp
   const int col0 = (blockIdx.y * (blockDim.x >> 5) + warp) * CPW + (lane / P) * NC, part = lane % P;   // grid.y splits the value columns
   float* S = state + (size_t)sq.slot * state_slot_stride + (size_t)h * dk * dv;
-  float s[KPT][NC];
+  f32x2 s[NC][Q][2];
 #pragma unroll
-  for (int e = 0; e < KPT; ++e)
+  for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const int i = e * P + part;
-      s[e][c] = (col0 + c < dv && i < dk) ? S[(size_t)i * dv + col0 + c] : 0.f;
+    for (int q = 0; q < Q; ++q) {
+      float v[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int i = 4 * (q * P + part) + r;
+        v[r] = (col0 + c < dv && i < dk) ? S[(size_t)i * dv + col0 + c] : 0.f;
+      }
+      s[c][q][0] = pack2(v[0], v[1]);
+      s[c][q][1] = pack2(v[2], v[3]);
     }
-  for (int e = threadIdx.x; e < 2 * CH * 6 * DKP; e += blockDim.x) (&buf[0][0][0][0])[e] = 0.f;   // the padding stays zero
+  for (int e = threadIdx.x; e < 2 * CH * NVEC * DKP; e += blockDim.x) (&buf[0][0][0][0])[e] = 0.f;   // the padding stays zero
   __syncthreads();
   const int HD = H * dk;
   // A thread copies the same pieces (vector, offset) of every token of a chunk: which pieces is worked out per piece, not per copy
   // (the divisions stay out of the token loop), and the token loop only adds the source's row stride.
   const int perk = vec4 ? dk / 4 : dk, perv = vec4 ? dv / 4 : dv;   // copies per key-sized vector / per value vector
-  const int per_tok = 5 * perk + perv;
+  const int per_tok = (NVEC - 1) * perk + perv;
   auto issue = [&](int c) {
     const int t0 = c * CH, nt = min(CH, sq.n_rows - t0);
     const size_t m0 = (size_t)sq.row0 + t0;
     for (int piece = threadIdx.x; piece < per_tok; piece += blockDim.x) {
-      const int vec = piece / perk < 5 ? piece / perk : 5, i = (piece - vec * perk) * (vec4 ? 4 : 1);
+      // order of the pieces: v, then k, r (, w, u, au)
+      const int vec = piece < perv ? 2 : (piece - perv) / perk < 2 ? (piece - perv) / perk : (piece - perv) / perk + 1;
+      const int i = (piece < perv ? piece : (piece - perv) % perk) * (vec4 ? 4 : 1);
       const float* src;
       size_t stride;
-      if (!uvec && (vec == 1 || vec == 2)) continue;          // no removal term: these two stay zero
-      if (vec == 0) { src = wdec + m0 * HD + h * dk + i; stride = HD; }
-      else if (vec == 1) { src = auvec + m0 * HD + h * dk + i; stride = HD; }
-      else if (vec == 2) { src = uvec + m0 * HD + h * dk + i; stride = HD; }
-      else if (vec == 3) { src = ksrc.p + m0 * ksrc.ld + ksrc.col + h * dk + i; stride = ksrc.ld; }
-      else if (vec == 4) { src = rsrc.p + m0 * rsrc.ld + rsrc.col + h * dk + i; stride = rsrc.ld; }
-      else { src = vsrc.p + m0 * vsrc.ld + vsrc.col + h * dv + i; stride = vsrc.ld; }
+      if (!SCALAR && !REMOVAL && vec >= 4) continue;         // no removal term
+      if (vec == 0) { src = ksrc.p + m0 * ksrc.ld + ksrc.col + h / ksrc.rep * dk + i; stride = ksrc.ld; }
+      else if (vec == 1) { src = rsrc.p + m0 * rsrc.ld + rsrc.col + h / rsrc.rep * dk + i; stride = rsrc.ld; }
+      else if (vec == 2) { src = vsrc.p + m0 * vsrc.ld + vsrc.col + h * dv + i; stride = vsrc.ld; }
+      else { src = (vec == 3 ? wdec : vec == 4 ? uvec : auvec) + m0 * HD + h * dk + i; stride = HD; }
       float* dst = &buf[c & 1][0][vec][i];
       if (vec4) {
-        for (int t = 0; t < nt; ++t) cp_async16(dst + (size_t)t * 6 * DKP, src + t * stride);
+        for (int t = 0; t < nt; ++t) cp_async16(dst + (size_t)t * NVEC * DKP, src + t * stride);
       } else {
-        for (int t = 0; t < nt; ++t) cp_async4(dst + (size_t)t * 6 * DKP, src + t * stride);
+        for (int t = 0; t < nt; ++t) cp_async4(dst + (size_t)t * NVEC * DKP, src + t * stride);
       }
     }
+    if (SCALAR && (int)threadIdx.x < 2 * nt) cp_async4(&gb[c & 1][threadIdx.x >> 1][threadIdx.x & 1], (threadIdx.x & 1 ? auvec : wdec) + (m0 + (threadIdx.x >> 1)) * H + h);
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const int nch = (sq.n_rows + CH - 1) / CH;
@@ -701,52 +739,140 @@ __global__ void delta_rule_kernel(DeltaSrc ksrc, DeltaSrc rsrc, DeltaSrc vsrc, c
     }
     __syncthreads();
     const int nt = min(CH, sq.n_rows - c * CH);
-    float(*b)[6][DKP] = buf[c & 1];
-    for (int t = 0; t < nt; ++t) {
-      float dot[NC], out[NC], vj[NC];
+    float(*b)[NVEC][DKP] = buf[c & 1];
+#pragma unroll 1
+    for (int t0 = 0; t0 < nt; t0 += TG) {
+      float out[TG][NC];
 #pragma unroll
-      for (int x = 0; x < NC; ++x) { dot[x] = 0.f; out[x] = 0.f; vj[x] = col0 + x < DKP ? b[t][5][col0 + x] : 0.f; }
-      if (uvec) {                                          // block-uniform
+      for (int g = 0; g < TG; ++g) {
+        const int t = t0 + g;
 #pragma unroll
-        for (int e = 0; e < KPT; ++e) {
-          const float u = b[t][2][e * P + part];
+        for (int x = 0; x < NC; ++x) out[g][x] = 0.f;
+        if (t >= nt) continue;                               // block-uniform
+        auto vec = [&](int v, int q) { return *reinterpret_cast<const ulonglong2*>(&b[t][v][4 * (q * P + part)]); };
+        float vj[NC], dot[NC];
 #pragma unroll
-          for (int x = 0; x < NC; ++x) dot[x] = fmaf(u, s[e][x], dot[x]);
+        for (int x = 0; x < NC; ++x) vj[x] = col0 + x < DKP ? b[t][2][col0 + x] : 0.f;
+        if constexpr (REMOVAL) {
+          f32x2 d2[NC][2];
+#pragma unroll
+          for (int x = 0; x < NC; ++x) d2[x][0] = d2[x][1] = 0;
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            const ulonglong2 u = vec(SCALAR ? 0 : 4, q);
+#pragma unroll
+            for (int x = 0; x < NC; ++x) { d2[x][0] = fma2(u.x, s[x][q][0], d2[x][0]); d2[x][1] = fma2(u.y, s[x][q][1], d2[x][1]); }
+          }
+#pragma unroll
+          for (int x = 0; x < NC; ++x) {
+            const float2 p = unpack2(d2[x][0]), r = unpack2(d2[x][1]);
+            dot[x] = (p.x + p.y) + (r.x + r.y);
+          }
+#pragma unroll
+          for (int o = P / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int x = 0; x < NC; ++x) dot[x] += __shfl_xor_sync(0xffffffffu, dot[x], o);
         }
+        f32x2 o2[NC][2];
 #pragma unroll
-        for (int o = P / 2; o > 0; o >>= 1)
+        for (int x = 0; x < NC; ++x) o2[x][0] = o2[x][1] = 0;
+        if constexpr (SCALAR) {
+          const float gd = gb[c & 1][t][0], beta = gb[c & 1][t][1];
+          const f32x2 g2 = pack2(gd, gd);
+          f32x2 c2[NC];
 #pragma unroll
-          for (int x = 0; x < NC; ++x) dot[x] += __shfl_xor_sync(0xffffffffu, dot[x], o);
-      }
+          for (int x = 0; x < NC; ++x) {
+            const float cx = REMOVAL ? beta * fmaf(-gd, dot[x], vj[x]) : beta * vj[x];
+            c2[x] = pack2(cx, cx);
+          }
 #pragma unroll
-      for (int e = 0; e < KPT; ++e) {
-        const int i = e * P + part;
-        const float w = b[t][0][i], au = b[t][1][i], kk = b[t][3][i], rr = b[t][4][i];
+          for (int q = 0; q < Q; ++q) {
+            const ulonglong2 k = vec(0, q), r = vec(1, q);
+#pragma unroll
+            for (int x = 0; x < NC; ++x) {
+              s[x][q][0] = fma2(k.x, c2[x], mul2(g2, s[x][q][0]));
+              s[x][q][1] = fma2(k.y, c2[x], mul2(g2, s[x][q][1]));
+              o2[x][0] = fma2(s[x][q][0], r.x, o2[x][0]);
+              o2[x][1] = fma2(s[x][q][1], r.y, o2[x][1]);
+            }
+          }
+        } else {
+          f32x2 v2[NC], n2[NC];
+#pragma unroll
+          for (int x = 0; x < NC; ++x) {
+            v2[x] = pack2(vj[x], vj[x]);
+            if constexpr (REMOVAL) n2[x] = pack2(-dot[x], -dot[x]);
+          }
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            const ulonglong2 k = vec(0, q), r = vec(1, q), w = vec(3, q);
+            ulonglong2 au;
+            if constexpr (REMOVAL) au = vec(5, q);
+#pragma unroll
+            for (int x = 0; x < NC; ++x) {
+              f32x2 t0v = mul2(k.x, v2[x]), t1v = mul2(k.y, v2[x]);
+              if constexpr (REMOVAL) { t0v = fma2(au.x, n2[x], t0v); t1v = fma2(au.y, n2[x], t1v); }
+              s[x][q][0] = fma2(w.x, s[x][q][0], t0v);
+              s[x][q][1] = fma2(w.y, s[x][q][1], t1v);
+              o2[x][0] = fma2(s[x][q][0], r.x, o2[x][0]);
+              o2[x][1] = fma2(s[x][q][1], r.y, o2[x][1]);
+            }
+          }
+        }
 #pragma unroll
         for (int x = 0; x < NC; ++x) {
-          s[e][x] = fmaf(w, s[e][x], fmaf(-au, dot[x], kk * vj[x]));
-          out[x] = fmaf(s[e][x], rr, out[x]);
+          const float2 p = unpack2(o2[x][0]), r = unpack2(o2[x][1]);
+          out[g][x] = (p.x + p.y) + (r.x + r.y);
         }
       }
+      // sums over the P lanes of TG * NC read-outs at once: each step halves the values a lane still holds
+      if constexpr (TG * NC >= P) {
+        float v[TG * NC];
 #pragma unroll
-      for (int o = P / 2; o > 0; o >>= 1)
+        for (int g = 0; g < TG; ++g)
 #pragma unroll
-        for (int x = 0; x < NC; ++x) out[x] += __shfl_xor_sync(0xffffffffu, out[x], o);
-      if (part == 0) {
-        float* dst = o_raw + ((size_t)sq.row0 + c * CH + t) * (size_t)(H * dv) + h * dv + col0;
+          for (int x = 0; x < NC; ++x) v[g * NC + x] = out[g][x];
 #pragma unroll
-        for (int x = 0; x < NC; ++x)
-          if (col0 + x < dv) dst[x] = out[x];
+        for (int o = P / 2, n = TG * NC; o > 0; o >>= 1, n >>= 1) {
+          const bool up = part & o;
+#pragma unroll
+          for (int i = 0; i < TG * NC / 2; ++i)
+            if (i < n / 2) {
+              const float keep = up ? v[i + n / 2] : v[i], give = up ? v[i] : v[i + n / 2];
+              v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+        constexpr int LEFT = TG * NC / P;                    // values this lane ends with: LEFT * part ..
+#pragma unroll
+        for (int i = 0; i < LEFT; ++i) {
+          const int idx = part * LEFT + i, g = idx / NC, x = idx % NC;
+          if (t0 + g < nt && col0 + x < dv) o_raw[((size_t)sq.row0 + c * CH + t0 + g) * (size_t)(H * dv) + h * dv + col0 + x] = v[i];
+        }
+      } else {
+#pragma unroll
+        for (int g = 0; g < TG; ++g)
+#pragma unroll
+          for (int x = 0; x < NC; ++x) {
+#pragma unroll
+            for (int o = P / 2; o > 0; o >>= 1) out[g][x] += __shfl_xor_sync(0xffffffffu, out[g][x], o);
+            if (part == (g * NC + x) % P && t0 + g < nt && col0 + x < dv)
+              o_raw[((size_t)sq.row0 + c * CH + t0 + g) * (size_t)(H * dv) + h * dv + col0 + x] = out[g][x];
+          }
       }
     }
     __syncthreads();                                 // the buffer is refilled two chunks later
   }
 #pragma unroll
-  for (int e = 0; e < KPT; ++e)
+  for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const int i = e * P + part;
-      if (col0 + c < dv && i < dk) S[(size_t)i * dv + col0 + c] = s[e][c];
+    for (int q = 0; q < Q; ++q) {
+      const float2 a = unpack2(s[c][q][0]), d = unpack2(s[c][q][1]);
+      const float v[4] = {a.x, a.y, d.x, d.y};
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const int i = 4 * (q * P + part) + r;
+        if (col0 + c < dv && i < dk) S[(size_t)i * dv + col0 + c] = v[r];
+      }
     }
 }
 
