@@ -46,3 +46,30 @@ def test_expert_products_match_oracle(rows):
   ref, _ = bu.oracle_logits(cfg, w, toks)
   err = lambda a, b: sorted(lu.row_err(a[i:i + 1], b[i:i + 1]) for i in range(rows))   # noqa: E731
   assert err(got, ref)[int(0.9 * (rows - 1))] < lu.TOL["bfloat16"] and err(got, fma)[int(0.9 * (rows - 1))] < lu.TOL["bfloat16"] / 2
+
+
+@pytest.mark.parametrize("rows,width,ff", [(129, 200, 2072), (700, 1032, 5904), (1030, 520, 3580)])
+def test_many_rows_on_cta_pairs_match_oracle(rows, width, ff):
+  """256 x 256 tiles of CTA pairs where they fill the GPU (700 rows x 5904: 3 x 24 tiles, the last row tile with 188 rows, the last column tile with 16
+  columns; 1030 x 3580: a row tile with 6 rows), 128 x 128 tiles elsewhere; closing epilogues of both forms"""
+  cfg = lu.config([lu.attn("latent_attention_2", heads=2, dim=16, rot_dim=8, vdim=16, kv_rank=24, window=40, ff=ff)], width=width, vocab=331, groups=1)
+  w = zo.random_weights(cfg, 21)
+  toks = lu.rand_tokens(331, rows, 4)
+  eng = lu.make_engine(cfg, w, "bfloat16", max_tokens=rows + 8)
+  got, _ = eng.step([0], [toks], want=list(range(rows)), argmax=False)
+  eng.close()
+  ref, _ = lu.oracle_logits(cfg, w, toks)
+  assert lu.row_err(got, ref) < lu.TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("rows", [600])
+def test_closing_products_on_cta_pairs_match_oracle(rows):
+  from tests import rinutar_oracle as ro, rinutar_util as ru
+  cfg = ru.config([ru.attn(heads=2, mlp=ru.dense(1032))], width=6136, vocab=64)   # down product: 600 x 6136 with K = 1032: 3 x 24 tiles
+  w = ro.random_weights(cfg, 8)
+  toks = lu.rand_tokens(64, rows, 5)
+  eng = lu.make_engine(cfg, w, "bfloat16", max_tokens=rows + 8)
+  got, _ = eng.step([0], [toks], want=list(range(rows)), argmax=False)
+  eng.close()
+  ref, _ = ru.oracle_logits(cfg, w, toks)
+  assert lu.row_err(got, ref) < lu.TOL["bfloat16"]

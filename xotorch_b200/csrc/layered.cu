@@ -828,15 +828,35 @@ static int product_stream(xotb200_lm* e, const bf16* A, long lda, long a_batch, 
   return 1;
 }
 
+// Pairs of CTAs on 256 x 256 tiles: 1.4 times the rate of 128 x 128 tiles while the tiles fill the pairs, so they are taken when at least 0.72 of
+// the pairs' time goes to rows and columns that exist (a last wave that is nearly empty, and rows or columns beyond the matrix, count against it).
+template <int EPI, typename TC>
+static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& mb, const LtcArgs& a) {
+  auto kern = ltc_pair_kernel<EPI, TC>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LTP_SMEM));
+  const int tiles = cdiv(a.M, 2 * LTC_M) * cdiv(a.N, LTP_N), pairs = std::min(tiles, e->sm_count / 2);
+  TRY(launch_late(e, kern, 2 * pairs, LTC_THREADS, LTP_SMEM, ma, mb, a));
+  e->tc_launches++;
+  return 0;
+}
+static bool pairs_pay(const xotb200_lm* e, int M, int N, int K) {
+  const long tiles = (long)cdiv(M, 2 * LTC_M) * cdiv(N, LTP_N), pairs = std::max(1, e->sm_count / 2), waves = (tiles + pairs - 1) / pairs;
+  return K >= 512 && (double)M * N >= 0.72 * (double)waves * pairs * (2.0 * LTC_M * LTP_N);
+}
+
 // 1 = launched, 0 = not eligible (the caller falls back), < 0 = error
 template <typename TC, int EPI>
 static int product_tc(xotb200_lm* e, const bf16* A, long lda, long a_batch, const bf16* B, long ldb, long b_batch, TC* C, long ldc, long c_batch, int M,
                       int N, int K, int batch, const EpiArgs& epi) {
   // one row tile or less: bound by reading B (measured up to 128 rows: 24.8 -> 17.8 us a launch at 64 .. 128 rows, width 2048)
   if (M <= LST_MAX_ROWS) return product_stream<TC, EPI>(e, A, lda, a_batch, B, ldb, b_batch, batch, C, ldc, c_batch, M, N, K, batch, epi);
-  const int nt = N > 64 ? 128 : 64;
+  const int nt = N > 64 ? 128 : 64;                            // 128: also a CTA's half of a pair's column tile
   CUtensorMap ma, mb;
   if (!make_map3(&ma, A, M, K, lda, a_batch, batch, LTC_M) || !make_map3(&mb, B, N, K, ldb, b_batch, batch, nt)) return 0;
+  if (batch == 1 && pairs_pay(e, M, N, K)) {
+    TRY((launch_pair<EPI, TC>(e, ma, mb, LtcArgs{M, N, K, C, ldc, 0, e->d_err, epi, nullptr, 0})));
+    return 1;
+  }
   LtcArgs a{M, N, K, C, ldc, c_batch, e->d_err, epi, nullptr, 0};
   if (nt == 128) TRY((launch_ltc<128, EPI, TC>(e, ma, mb, a, batch)));
   else TRY((launch_ltc<64, EPI, TC>(e, ma, mb, a, batch)));
@@ -1387,7 +1407,7 @@ static int gated_delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, floa
   const int M = sp.M, H = s.heads, G = s.kv_heads, dk = s.dim, dv = s.vdim, C = L.conv_ch;
   TRY(filter_channels<T>(e, L, sp, L.c_r, C, nullptr));
   TRY(launch_early(e, gated_delta_prepare_kernel<T>, cdiv((long)M * G, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
-                   e->dau, e->dkk, e->drr, H, G, dk, M));
+                   e->dau, e->du, e->dkk, e->drr, H, G, dk, M));
   TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, G * dk, 0, H / G}, DeltaSrc{e->drr, G * dk, 0, H / G}, DeltaSrc{e->cvb, C, 2 * G * dk}, dk, dv, DELTA_SCALAR));
   TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), 0, e->proj, L.ld_in, L.c_g, 1, static_cast<T*>(ohbuf),
                                                                        H, dv, e->cfg.norm_eps, M));

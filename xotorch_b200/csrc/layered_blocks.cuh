@@ -364,12 +364,13 @@ __global__ void short_conv_kernel(const float* __restrict__ proj, int ld, int co
 // What the gated delta rule needs per token, in the scalar form of delta_rule_kernel:  S <- g S + k (beta (v - g (k^T S)))^T, o = S^T r
 // with unit key k, step size beta and decay g of the head.  cv [M, C] holds the filtered q (G * dk), k (G * dk), v (H * dv) channels; value
 // head a reads query/key head a / (H / G).  proj columns col_b + a / col_a + a are the step-size and decay logits.  One warp per (row, query/key
-// head): unit key and scaled query [M, G * dk] each, and g, beta [M, H] of the value heads that read it.
+// head): unit key and scaled query [M, G * dk] each, the unit key times the unit key of the row behind it ([M, G]; the last row's is not used),
+// and g, beta [M, H] of the value heads that read it.
 // ---------------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void gated_delta_prepare_kernel(const float* __restrict__ cv, int C, const float* __restrict__ proj, int ld, int col_b, int col_a,
                                            const T* __restrict__ a_log, const T* __restrict__ dt_bias, float* __restrict__ g_out, float* __restrict__ beta_out,
-                                           float* __restrict__ k_out, float* __restrict__ r_out, int H, int G, int dk, int M) {
+                                           float* __restrict__ kk_out, float* __restrict__ k_out, float* __restrict__ r_out, int H, int G, int dk, int M) {
   pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= M * G) return;
@@ -377,9 +378,17 @@ __global__ void gated_delta_prepare_kernel(const float* __restrict__ cv, int C, 
   const int kh = idx % G, rep = H / G;
   const float* q = cv + m * C + (size_t)kh * dk;
   const float* k = cv + m * C + (size_t)G * dk + (size_t)kh * dk;
-  float sq = 0.f, sk = 0.f;
-  for (int i = lane; i < dk; i += 32) { sq = fmaf(q[i], q[i], sq); sk = fmaf(k[i], k[i], sk); }
+  const float* kn = m + 1 < (size_t)M ? k + C : k;             // the row behind (of another request: its product is not used)
+  float sq = 0.f, sk = 0.f, sn = 0.f, kk = 0.f;
+  for (int i = lane; i < dk; i += 32) {
+    sq = fmaf(q[i], q[i], sq);
+    sk = fmaf(k[i], k[i], sk);
+    sn = fmaf(kn[i], kn[i], sn);
+    kk = fmaf(k[i], kn[i], kk);
+  }
   const float iq = 1.0f / (sqrtf(warp_sum(sq) + 1e-6f) * sqrtf((float)dk)), ik = 1.0f / sqrtf(warp_sum(sk) + 1e-6f);
+  kk = warp_sum(kk) * ik * (1.0f / sqrtf(warp_sum(sn) + 1e-6f));
+  if (lane == 0) kk_out[m * G + kh] = kk;
   for (int a = kh * rep + lane; a < (kh + 1) * rep; a += 32) {
     beta_out[m * H + a] = sigmoidf_(proj[m * ld + col_b + a]);
     g_out[m * H + a] = expf(-expf(ldf(a_log + a)) * softplusf_(proj[m * ld + col_a + a] + ldf(dt_bias + a)));

@@ -632,8 +632,8 @@ __global__ void delta_prepare_kernel(const float* __restrict__ proj, int ld, int
 // read four entries per shared-memory load, and state and vectors are kept as PAIRS of fp32 that one packed instruction (fma.rn.f32x2: two
 // independent fp32 FMAs) works on: a head of 128 x 128 takes some 130 instructions a token and warp instead of 270.  The chain from token to
 // token is dot product -> sum over the P lanes -> update; the read-outs of four tokens are summed over the lanes together afterwards, off it.
-// SCALAR: the head has ONE decay and ONE write strength per token, S <- g S + k (beta (v - g (k^T S)))^T: three vectors and two numbers are staged
-// instead of six vectors (wdec = g, auvec = beta, both [M, H]).  Else S <- diag(w) S - au (u^T S) + k v^T with wdec, uvec, auvec [M, H * dk]; REMOVAL 0:
+// SCALAR: the head has ONE decay and ONE write strength per token, S <- g S + k (beta (v - g (k^T S)))^T: three vectors and three numbers are
+// staged instead of six vectors (wdec = g, auvec = beta, both [M, H], uvec [M, H / ksrc.rep] = a token's key times the next one's).  Else S <- diag(w) S - au (u^T S) + k v^T with wdec, uvec, auvec [M, H * dk]; REMOVAL 0:
 // without the u term (u and au are neither staged nor applied).  vec4: every source row is 16-byte aligned (sizes and offsets multiples of 4
 // floats), so the staging uses 16-byte cp.async.
 // The write key k, the read-out vector r and the value v each come from their own fp32 matrix (pointer, leading dimension, first column; head a's
@@ -667,7 +667,7 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 }
 
 template <int KPT, int P, int NC, bool SCALAR, bool REMOVAL>
-__global__ void __launch_bounds__(128) delta_rule_kernel(DeltaSrc ksrc, DeltaSrc rsrc, DeltaSrc vsrc, const float* __restrict__ wdec,
+__global__ void __launch_bounds__(128, 2) delta_rule_kernel(DeltaSrc ksrc, DeltaSrc rsrc, DeltaSrc vsrc, const float* __restrict__ wdec,
                                   const float* __restrict__ uvec, const float* __restrict__ auvec, const Item* __restrict__ seqs, int H, int dk,
                                   int dv, float* __restrict__ state, size_t state_slot_stride, float* __restrict__ o_raw, int vec4) {
   pdl_enter();
@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(128) delta_rule_kernel(DeltaSrc ksrc, DeltaSrc
   constexpr int CH = DKP <= 64 ? 16 : DKP <= 128 ? 8 : 4;   // tokens per buffer: two buffers fit the 48 KB of static shared memory
   constexpr int Q = KPT / 4, TG = 4;                 // runs of four rows per thread; tokens whose read-outs are summed together
   __shared__ __align__(16) float buf[2][CH][NVEC][DKP];
-  __shared__ float gb[2][CH][2];                     // SCALAR: g, beta
+  __shared__ __align__(16) float gb[2][CH][4];       // SCALAR: g, beta, k of the token . k of the next one
   const Item sq = seqs[blockIdx.x / H];
   const int h = blockIdx.x % H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -725,7 +725,11 @@ __global__ void __launch_bounds__(128) delta_rule_kernel(DeltaSrc ksrc, DeltaSrc
         for (int t = 0; t < nt; ++t) cp_async4(dst + (size_t)t * NVEC * DKP, src + t * stride);
       }
     }
-    if (SCALAR && (int)threadIdx.x < 2 * nt) cp_async4(&gb[c & 1][threadIdx.x >> 1][threadIdx.x & 1], (threadIdx.x & 1 ? auvec : wdec) + (m0 + (threadIdx.x >> 1)) * H + h);
+    if (SCALAR)
+      for (int p = threadIdx.x; p < 3 * nt; p += blockDim.x) {
+        const int t = p / 3, n = p % 3;
+        cp_async4(&gb[c & 1][t][n], n == 0 ? wdec + (m0 + t) * H + h : n == 1 ? auvec + (m0 + t) * H + h : uvec + (m0 + t) * (H / ksrc.rep) + h / ksrc.rep);
+      }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   const int nch = (sq.n_rows + CH - 1) / CH;
@@ -740,89 +744,112 @@ __global__ void __launch_bounds__(128) delta_rule_kernel(DeltaSrc ksrc, DeltaSrc
     __syncthreads();
     const int nt = min(CH, sq.n_rows - c * CH);
     float(*b)[NVEC][DKP] = buf[c & 1];
+    float(*sc)[4] = gb[c & 1];
+    auto vec = [&](int t, int v, int q) { return *reinterpret_cast<const ulonglong2*>(&b[t][v][4 * (q * P + part)]); };
+    // sum over the key rows of vector v of token t times the state, for each column of the thread
+    auto dots = [&](int t, int v, float (&d)[NC]) {
+      f32x2 d2[NC][2];
+#pragma unroll
+      for (int x = 0; x < NC; ++x) d2[x][0] = d2[x][1] = 0;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const ulonglong2 u = vec(t, v, q);
+#pragma unroll
+        for (int x = 0; x < NC; ++x) { d2[x][0] = fma2(u.x, s[x][q][0], d2[x][0]); d2[x][1] = fma2(u.y, s[x][q][1], d2[x][1]); }
+      }
+#pragma unroll
+      for (int x = 0; x < NC; ++x) {
+        const float2 p = unpack2(d2[x][0]), r = unpack2(d2[x][1]);
+        d[x] = (p.x + p.y) + (r.x + r.y);
+      }
+#pragma unroll
+      for (int o = P / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int x = 0; x < NC; ++x) d[x] += __shfl_xor_sync(0xffffffffu, d[x], o);
+    };
+    float dot[NC];                                           // k^T S of the next token, per column (SCALAR with removal)
+#pragma unroll
+    for (int x = 0; x < NC; ++x) dot[x] = 0.f;
+    if constexpr (SCALAR && REMOVAL) dots(0, 0, dot);
+    // one token: the state moves on, out <- this thread's part of S^T r
+    auto token = [&](int t, float (&out)[NC]) {
+      float vj[NC];
+#pragma unroll
+      for (int x = 0; x < NC; ++x) vj[x] = col0 + x < DKP ? b[t][2][col0 + x] : 0.f;
+      f32x2 o2[NC][2];
+#pragma unroll
+      for (int x = 0; x < NC; ++x) o2[x][0] = o2[x][1] = 0;
+      if constexpr (SCALAR) {
+        const float4 g4 = *reinterpret_cast<const float4*>(sc[t]);               // g, beta, k_t . k_{t+1}
+        float nxt[NC], cx[NC];
+        // k_{t+1}^T S_t = g_t (k_{t+1}^T S_{t-1}) + (k_{t+1} . k_t) c_t: the sum over the lanes is taken on the OLD state, beside this token's
+        // update, and only two multiply-adds are left between c_t and c_{t+1}
+        if constexpr (REMOVAL) dots(t + 1 < nt ? t + 1 : t, 0, nxt);
+        const f32x2 g2 = pack2(g4.x, g4.x);
+        f32x2 c2[NC];
+#pragma unroll
+        for (int x = 0; x < NC; ++x) {
+          cx[x] = REMOVAL ? g4.y * fmaf(-g4.x, dot[x], vj[x]) : g4.y * vj[x];
+          c2[x] = pack2(cx[x], cx[x]);
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const ulonglong2 kk = vec(t, 0, q), r = vec(t, 1, q);
+#pragma unroll
+          for (int x = 0; x < NC; ++x) {
+            s[x][q][0] = fma2(kk.x, c2[x], mul2(g2, s[x][q][0]));
+            s[x][q][1] = fma2(kk.y, c2[x], mul2(g2, s[x][q][1]));
+            o2[x][0] = fma2(s[x][q][0], r.x, o2[x][0]);
+            o2[x][1] = fma2(s[x][q][1], r.y, o2[x][1]);
+          }
+        }
+        if constexpr (REMOVAL) {
+#pragma unroll
+          for (int x = 0; x < NC; ++x) dot[x] = fmaf(g4.z, cx[x], g4.x * nxt[x]);
+        }
+      } else {
+        float d[NC];
+        if constexpr (REMOVAL) dots(t, 4, d);
+        f32x2 v2[NC], n2[NC];
+#pragma unroll
+        for (int x = 0; x < NC; ++x) {
+          v2[x] = pack2(vj[x], vj[x]);
+          if constexpr (REMOVAL) n2[x] = pack2(-d[x], -d[x]);
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const ulonglong2 kk = vec(t, 0, q), r = vec(t, 1, q), w = vec(t, 3, q);
+          ulonglong2 au;
+          if constexpr (REMOVAL) au = vec(t, 5, q);
+#pragma unroll
+          for (int x = 0; x < NC; ++x) {
+            f32x2 t0v = mul2(kk.x, v2[x]), t1v = mul2(kk.y, v2[x]);
+            if constexpr (REMOVAL) { t0v = fma2(au.x, n2[x], t0v); t1v = fma2(au.y, n2[x], t1v); }
+            s[x][q][0] = fma2(w.x, s[x][q][0], t0v);
+            s[x][q][1] = fma2(w.y, s[x][q][1], t1v);
+            o2[x][0] = fma2(s[x][q][0], r.x, o2[x][0]);
+            o2[x][1] = fma2(s[x][q][1], r.y, o2[x][1]);
+          }
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < NC; ++x) {
+        const float2 p = unpack2(o2[x][0]), r = unpack2(o2[x][1]);
+        out[x] = (p.x + p.y) + (r.x + r.y);
+      }
+    };
 #pragma unroll 1
     for (int t0 = 0; t0 < nt; t0 += TG) {
       float out[TG][NC];
+      if (t0 + TG <= nt) {                                   // block-uniform; straight-line code lets the loads of a token run ahead of the one before
 #pragma unroll
-      for (int g = 0; g < TG; ++g) {
-        const int t = t0 + g;
+        for (int g = 0; g < TG; ++g) token(t0 + g, out[g]);
+      } else {
 #pragma unroll
-        for (int x = 0; x < NC; ++x) out[g][x] = 0.f;
-        if (t >= nt) continue;                               // block-uniform
-        auto vec = [&](int v, int q) { return *reinterpret_cast<const ulonglong2*>(&b[t][v][4 * (q * P + part)]); };
-        float vj[NC], dot[NC];
+        for (int g = 0; g < TG; ++g) {
 #pragma unroll
-        for (int x = 0; x < NC; ++x) vj[x] = col0 + x < DKP ? b[t][2][col0 + x] : 0.f;
-        if constexpr (REMOVAL) {
-          f32x2 d2[NC][2];
-#pragma unroll
-          for (int x = 0; x < NC; ++x) d2[x][0] = d2[x][1] = 0;
-#pragma unroll
-          for (int q = 0; q < Q; ++q) {
-            const ulonglong2 u = vec(SCALAR ? 0 : 4, q);
-#pragma unroll
-            for (int x = 0; x < NC; ++x) { d2[x][0] = fma2(u.x, s[x][q][0], d2[x][0]); d2[x][1] = fma2(u.y, s[x][q][1], d2[x][1]); }
-          }
-#pragma unroll
-          for (int x = 0; x < NC; ++x) {
-            const float2 p = unpack2(d2[x][0]), r = unpack2(d2[x][1]);
-            dot[x] = (p.x + p.y) + (r.x + r.y);
-          }
-#pragma unroll
-          for (int o = P / 2; o > 0; o >>= 1)
-#pragma unroll
-            for (int x = 0; x < NC; ++x) dot[x] += __shfl_xor_sync(0xffffffffu, dot[x], o);
-        }
-        f32x2 o2[NC][2];
-#pragma unroll
-        for (int x = 0; x < NC; ++x) o2[x][0] = o2[x][1] = 0;
-        if constexpr (SCALAR) {
-          const float gd = gb[c & 1][t][0], beta = gb[c & 1][t][1];
-          const f32x2 g2 = pack2(gd, gd);
-          f32x2 c2[NC];
-#pragma unroll
-          for (int x = 0; x < NC; ++x) {
-            const float cx = REMOVAL ? beta * fmaf(-gd, dot[x], vj[x]) : beta * vj[x];
-            c2[x] = pack2(cx, cx);
-          }
-#pragma unroll
-          for (int q = 0; q < Q; ++q) {
-            const ulonglong2 k = vec(0, q), r = vec(1, q);
-#pragma unroll
-            for (int x = 0; x < NC; ++x) {
-              s[x][q][0] = fma2(k.x, c2[x], mul2(g2, s[x][q][0]));
-              s[x][q][1] = fma2(k.y, c2[x], mul2(g2, s[x][q][1]));
-              o2[x][0] = fma2(s[x][q][0], r.x, o2[x][0]);
-              o2[x][1] = fma2(s[x][q][1], r.y, o2[x][1]);
-            }
-          }
-        } else {
-          f32x2 v2[NC], n2[NC];
-#pragma unroll
-          for (int x = 0; x < NC; ++x) {
-            v2[x] = pack2(vj[x], vj[x]);
-            if constexpr (REMOVAL) n2[x] = pack2(-dot[x], -dot[x]);
-          }
-#pragma unroll
-          for (int q = 0; q < Q; ++q) {
-            const ulonglong2 k = vec(0, q), r = vec(1, q), w = vec(3, q);
-            ulonglong2 au;
-            if constexpr (REMOVAL) au = vec(5, q);
-#pragma unroll
-            for (int x = 0; x < NC; ++x) {
-              f32x2 t0v = mul2(k.x, v2[x]), t1v = mul2(k.y, v2[x]);
-              if constexpr (REMOVAL) { t0v = fma2(au.x, n2[x], t0v); t1v = fma2(au.y, n2[x], t1v); }
-              s[x][q][0] = fma2(w.x, s[x][q][0], t0v);
-              s[x][q][1] = fma2(w.y, s[x][q][1], t1v);
-              o2[x][0] = fma2(s[x][q][0], r.x, o2[x][0]);
-              o2[x][1] = fma2(s[x][q][1], r.y, o2[x][1]);
-            }
-          }
-        }
-#pragma unroll
-        for (int x = 0; x < NC; ++x) {
-          const float2 p = unpack2(o2[x][0]), r = unpack2(o2[x][1]);
-          out[g][x] = (p.x + p.y) + (r.x + r.y);
+          for (int x = 0; x < NC; ++x) out[g][x] = 0.f;
+          if (t0 + g < nt) token(t0 + g, out[g]);
         }
       }
       // sums over the P lanes of TG * NC read-outs at once: each step halves the values a lane still holds

@@ -56,6 +56,112 @@ __device__ __forceinline__ void ltc_load16(__nv_bfloat16* dst, const __nv_bfloat
   reinterpret_cast<uint4*>(dst)[1] = reinterpret_cast<const uint4*>(src)[1];
 }
 
+// What happens to 16 consecutive columns n .. n + 15 of output row `row` (row < M, n < N), as tcgen05.ld hands them to a thread: the epilogue,
+// then the store in the widest pieces that the operands allow.
+template <int EPI, typename TC>
+struct LtcEpilogue {
+  bool vec, vec16, vecx;
+  float ap = 0.f, aq = 0.f, alpha = 0.f;
+  __device__ __forceinline__ explicit LtcEpilogue(const LtcArgs& a) {
+    vec = (sizeof(TC) == 4) && ((a.ldc | a.c_batch) % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.C) & 15) == 0);
+    vec16 = (sizeof(TC) == 2) && ((a.ldc | a.c_batch) % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.C) & 15) == 0);
+    // CLOSE: whole 16-entry pieces of the stream row, its operand row and the per-entry vectors move in 16-byte accesses
+    vecx = EPI == EPI_CLOSE && a.epi.ld % 8 == 0;
+    if (EPI == EPI_XIELU) {
+      const __nv_bfloat16* raw = static_cast<const __nv_bfloat16*>(a.epi.p);
+      ap = softplusf_(__bfloat162float(raw[0]));
+      aq = 0.5f + softplusf_(__bfloat162float(raw[1]));
+    }
+    if (EPI == EPI_CLOSE && a.epi.h) alpha = __bfloat162float(*static_cast<const __nv_bfloat16*>(a.epi.alpha));
+  }
+  __device__ __forceinline__ void store16(const LtcArgs& a, TC* crow, int row, int n, const uint32_t (&v)[16]) const {
+    float f[16];
+    if constexpr (EPI == EPI_CLOSE) {
+      if (vecx && n + 16 <= a.N) {
+        float4* x4 = reinterpret_cast<float4*>(a.epi.x + (size_t)row * a.epi.ld + n);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float4 t = x4[j];
+          f[4 * j] = t.x; f[4 * j + 1] = t.y; f[4 * j + 2] = t.z; f[4 * j + 3] = t.w;
+        }
+        __align__(16) __nv_bfloat16 t[16];
+        if (a.epi.ls) {
+          ltc_load16(t, static_cast<const __nv_bfloat16*>(a.epi.ls) + n);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) f[j] = fmaf(__uint_as_float(v[j]), __bfloat162float(t[j]), f[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) f[j] += __uint_as_float(v[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x4[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+        if (a.epi.h) {
+          __align__(16) __nv_bfloat16 tb[16];
+          ltc_load16(t, static_cast<const __nv_bfloat16*>(a.epi.w) + n);
+          ltc_load16(tb, static_cast<const __nv_bfloat16*>(a.epi.b) + n);
+          uint32_t pk[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            __nv_bfloat162 h2 = __floats2bfloat162_rn(dyt_f(f[2 * j], alpha, __bfloat162float(t[2 * j]), __bfloat162float(tb[2 * j])),
+                                                      dyt_f(f[2 * j + 1], alpha, __bfloat162float(t[2 * j + 1]), __bfloat162float(tb[2 * j + 1])));
+            pk[j] = *reinterpret_cast<uint32_t*>(&h2);
+          }
+          uint4* d4 = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.epi.h) + (size_t)row * a.epi.ld + n);
+          d4[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          d4[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+        }
+      } else {
+#pragma unroll 1
+        for (int j = 0; j < 16; ++j)
+          if (n + j < a.N) stream_close<__nv_bfloat16>(a.epi, row, n + j, __uint_as_float(v[j]));
+      }
+    } else if constexpr (epi_is_glu(EPI)) {        // 8 gate values, then their 8 up values -> 8 outputs at columns n / 2 ..
+      const int no = n >> 1;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = glu_f<EPI>(__uint_as_float(v[j]), __uint_as_float(v[j + 8]), a.epi);
+      if (sizeof(TC) == 2 && a.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0) {
+        uint32_t pk[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+          pk[j] = *reinterpret_cast<uint32_t*>(&h2);
+        }
+        *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(crow) + no) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ltc_store<TC>(crow + no + j, f[j]);
+      }
+    } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      f[j] = __uint_as_float(v[j]);
+      if (EPI == EPI_RELU2) { f[j] = fmaxf(f[j], 0.f); f[j] *= f[j]; }
+      if (EPI == EPI_XIELU) f[j] = xielu_f(f[j], ap, aq);
+      if (EPI == EPI_GELU) f[j] = gelu_erf_f(f[j]);
+    }
+    if (vec && n + 16 <= a.N) {
+      float4* d4 = reinterpret_cast<float4*>(reinterpret_cast<float*>(crow) + n);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) d4[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+    } else if (vec16 && n + 16 <= a.N) {
+      uint32_t pk[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+        pk[j] = *reinterpret_cast<uint32_t*>(&h2);
+      }
+      uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(crow) + n);
+      d4[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      d4[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (n + j < a.N) ltc_store<TC>(crow + n + j, f[j]);
+    }
+    }
+  }
+};
+
 template <int NT, int EPI, int NS, typename TC>
 __global__ void __launch_bounds__(LTC_THREADS, 2 * ltc_smem_bytes(NT, NS) <= 226 * 1024 ? 2 : 1)
 ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LtcArgs a) {
@@ -126,114 +232,128 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int row = m0 + q * 32 + lane;
     if (ltc_wait(tmem_full, 0, a.err)) {
       xb::tc_fence_after();
-      TC* crow = static_cast<TC*>(a.C) + (size_t)z * a.c_batch + (size_t)row * a.ldc;
-      const bool vec = (sizeof(TC) == 4) && ((a.ldc | a.c_batch) % 4 == 0) && ((reinterpret_cast<uintptr_t>(a.C) & 15) == 0);
-      const bool vec16 = (sizeof(TC) == 2) && ((a.ldc | a.c_batch) % 8 == 0) && ((reinterpret_cast<uintptr_t>(a.C) & 15) == 0);
-      float ap = 0.f, aq = 0.f;
-      if (EPI == EPI_XIELU) {
-        const __nv_bfloat16* raw = static_cast<const __nv_bfloat16*>(a.epi.p);
-        ap = softplusf_(__bfloat162float(raw[0]));
-        aq = 0.5f + softplusf_(__bfloat162float(raw[1]));
-      }
-      // CLOSE: whole 16-entry pieces of the stream row, its operand row and the per-entry vectors move in 16-byte accesses
-      const bool vecx = EPI == EPI_CLOSE && a.epi.ld % 8 == 0;
-      const float alpha = EPI == EPI_CLOSE && a.epi.h ? __bfloat162float(*static_cast<const __nv_bfloat16*>(a.epi.alpha)) : 0.f;
+      const LtcEpilogue<EPI, TC> ep(a);
 #pragma unroll 1
       for (int c0 = 0; c0 < NT; c0 += 16) {
         uint32_t v[16];
         xb::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);   // warp-collective: before any row / column test
         const int n = n0 + c0;
         if (row >= a.M || n >= a.N) continue;
-        float f[16];
-        if constexpr (EPI == EPI_CLOSE) {
-          if (vecx && n + 16 <= a.N) {
-            float4* x4 = reinterpret_cast<float4*>(a.epi.x + (size_t)row * a.epi.ld + n);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float4 t = x4[j];
-              f[4 * j] = t.x; f[4 * j + 1] = t.y; f[4 * j + 2] = t.z; f[4 * j + 3] = t.w;
-            }
-            __align__(16) __nv_bfloat16 t[16];
-            if (a.epi.ls) {
-              ltc_load16(t, static_cast<const __nv_bfloat16*>(a.epi.ls) + n);
-#pragma unroll
-              for (int j = 0; j < 16; ++j) f[j] = fmaf(__uint_as_float(v[j]), __bfloat162float(t[j]), f[j]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 16; ++j) f[j] += __uint_as_float(v[j]);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) x4[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-            if (a.epi.h) {
-              __align__(16) __nv_bfloat16 tb[16];
-              ltc_load16(t, static_cast<const __nv_bfloat16*>(a.epi.w) + n);
-              ltc_load16(tb, static_cast<const __nv_bfloat16*>(a.epi.b) + n);
-              uint32_t pk[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                __nv_bfloat162 h2 = __floats2bfloat162_rn(dyt_f(f[2 * j], alpha, __bfloat162float(t[2 * j]), __bfloat162float(tb[2 * j])),
-                                                          dyt_f(f[2 * j + 1], alpha, __bfloat162float(t[2 * j + 1]), __bfloat162float(tb[2 * j + 1])));
-                pk[j] = *reinterpret_cast<uint32_t*>(&h2);
-              }
-              uint4* d4 = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(a.epi.h) + (size_t)row * a.epi.ld + n);
-              d4[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-              d4[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-            }
-          } else {
-#pragma unroll 1
-            for (int j = 0; j < 16; ++j)
-              if (n + j < a.N) stream_close<__nv_bfloat16>(a.epi, row, n + j, __uint_as_float(v[j]));
-          }
-        } else if constexpr (epi_is_glu(EPI)) {        // 8 gate values, then their 8 up values -> 8 outputs at columns n / 2 ..
-          const int no = n >> 1;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) f[j] = glu_f<EPI>(__uint_as_float(v[j]), __uint_as_float(v[j + 8]), a.epi);
-          if (sizeof(TC) == 2 && a.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0) {
-            uint32_t pk[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-              pk[j] = *reinterpret_cast<uint32_t*>(&h2);
-            }
-            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(crow) + no) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) ltc_store<TC>(crow + no + j, f[j]);
-          }
-        } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          f[j] = __uint_as_float(v[j]);
-          if (EPI == EPI_RELU2) { f[j] = fmaxf(f[j], 0.f); f[j] *= f[j]; }
-          if (EPI == EPI_XIELU) f[j] = xielu_f(f[j], ap, aq);
-          if (EPI == EPI_GELU) f[j] = gelu_erf_f(f[j]);
-        }
-        if (vec && n + 16 <= a.N) {
-          float4* d4 = reinterpret_cast<float4*>(reinterpret_cast<float*>(crow) + n);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) d4[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-        } else if (vec16 && n + 16 <= a.N) {
-          uint32_t pk[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-            pk[j] = *reinterpret_cast<uint32_t*>(&h2);
-          }
-          uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(crow) + n);
-          d4[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-          d4[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (n + j < a.N) ltc_store<TC>(crow + n + j, f[j]);
-        }
-        }
+        ep.store16(a, static_cast<TC*>(a.C) + (size_t)z * a.c_batch + (size_t)row * a.ldc, row, n, v);
       }
     }
   }
   xb::tc_fence_before();
   __syncthreads();
   if (warp == 2) xb::tmem_dealloc(tmem_base, TMEM_COLS);
+}
+
+// ---- CTA pairs (cta_group::2): many rows ------------------------------------------------------------------------------------------------
+// A 128 x 128 tile pulls 32 KB of operands through L2 for 2.1 MFLOP per K block, and that, not the tensor pipe, sets the pace of the kernel above.
+// Here two CTAs share one 256 x 256 tile: each stages its own 128 rows of A and HALF of the B tile (32 KB per 4.2 MFLOP of its own), the
+// leader's thread issues tcgen05.mma.cta_group::2 over both CTAs' shared memory, and every CTA keeps its 128 rows of the accumulator.  Persistent: 74
+// pairs walk the tiles (row tile fastest, so that pairs running together share weight tiles in L2) with two accumulators in tensor memory (all
+// 512 columns), so the epilogue of one tile runs under the products of the next.  Plain loads, no multicast.  Every wait is bounded.
+constexpr int LTP_N = 256, LTP_STAGES = 6, LTP_STAGE_BYTES = LTC_M * LTC_BK * 2 + LTP_N / 2 * LTC_BK * 2;
+constexpr int LTP_SMEM = LTP_STAGES * LTP_STAGE_BYTES + 1024 + 256;
+
+template <int EPI, typename TC>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LTC_THREADS, 1)
+ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LtcArgs a) {
+  pdl_enter();
+  extern __shared__ __align__(1024) uint8_t ltc_smem[];
+  constexpr int A_BYTES = LTC_M * LTC_BK * 2, NS = LTP_STAGES, NT = LTP_N;
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ltc_smem) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + NS * LTP_STAGE_BYTES);   // the leader's count both CTAs' copies
+  uint64_t* empty = full + NS;
+  uint64_t* tmem_full = empty + NS;       // [2]
+  uint64_t* tmem_empty = tmem_full + 2;   // [2], the leader's: 4 warps of both CTAs
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = xb::cluster_ctarank();
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const int mtiles = (a.M + 2 * LTC_M - 1) / (2 * LTC_M), total = mtiles * ((a.N + NT - 1) / NT), nkb = (a.K + LTC_BK - 1) / LTC_BK;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < NS; ++i) { xb::mbar_init(&full[i], 1); xb::mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { xb::mbar_init(&tmem_full[i], 1); xb::mbar_init(&tmem_empty[i], 8); }
+    xb::fence_mbar_init();
+  }
+  __syncthreads();
+  if (warp == 2) xb::tmem_alloc_2sm(tmem_slot, 2 * NT);
+  xb::tc_fence_before();
+  xb::cluster_sync_all();                 // both CTAs' barriers are initialised before anybody signals across the pair
+  xb::tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0 && lane == 0) {
+    // ===== TMA producer (both CTAs): own rows of A, own half of B; completion is counted on the leader's barrier =====
+    unsigned it = 0;
+    bool ok = true;
+    for (int t = pair; t < total && ok; t += npairs) {
+      const int m0 = (t % mtiles) * 2 * LTC_M + (int)rank * LTC_M, n0 = (t / mtiles) * NT + (int)rank * (NT / 2);
+      for (int kb = 0; kb < nkb; ++kb, ++it) {
+        const int st = it % NS;
+        ok = ltc_wait(&empty[st], ((it / NS) & 1u) ^ 1u, a.err);
+        if (!ok) break;
+        uint8_t* sa = base + (size_t)st * LTP_STAGE_BYTES;
+        if (rank == 0) xb::mbar_expect_tx(&full[st], 2 * LTP_STAGE_BYTES);
+        const uint32_t bar = xb::mapa_shared(xb::smem_u32(&full[st]), 0);
+        xb::tma_load_3d_2sm(sa, &tmA, kb * LTC_BK, m0, 0, bar);
+        xb::tma_load_3d_2sm(sa + A_BYTES, &tmB, kb * LTC_BK, n0, 0, bar);
+      }
+    }
+    if (rank == 0)   // the copies still in flight (there are any only after giving up) land before the pair's shared memory goes away
+      for (unsigned i = it > NS ? it - NS : 0; i < it && !ok; ++i) ltc_wait(&full[i % NS], (i / NS) & 1u, a.err);
+  } else if (warp == 1 && lane == 0 && rank == 0) {
+    // ===== MMA issuer: one thread of the leader for the pair =====
+    constexpr uint32_t idesc = ltc_idesc(2 * LTC_M, NT);
+    unsigned it = 0, ti = 0;
+    bool ok = true;
+    for (int t = pair; t < total && ok; t += npairs, ++ti) {
+      const uint32_t buf = ti & 1u, acc = tmem_base + buf * NT;
+      ok = ltc_wait(&tmem_empty[buf], ((ti >> 1) & 1u) ^ 1u, a.err);     // both CTAs' epilogues have drained it
+      if (!ok) break;
+      xb::tc_fence_after();
+      for (int kb = 0; kb < nkb; ++kb, ++it) {
+        const int st = it % NS;
+        ok = ltc_wait(&full[st], (it / NS) & 1u, a.err);
+        if (!ok) break;
+        xb::tc_fence_after();
+        const uint32_t sa = xb::smem_u32(base + (size_t)st * LTP_STAGE_BYTES), sb = sa + A_BYTES;
+#pragma unroll
+        for (int k = 0; k < LTC_BK / 16; ++k)
+          xb::umma_bf16_2sm(acc, xb::umma_desc_sw128(sa + k * 32), xb::umma_desc_sw128(sb + k * 32), idesc, (kb | k) != 0 ? 1u : 0u);
+        xb::umma_commit_2sm(&empty[st], 3);                              // frees the stage in both CTAs
+      }
+      if (ok) xb::umma_commit_2sm(&tmem_full[buf], 3);
+    }
+  } else if (warp >= 4) {
+    // ===== epilogue (both CTAs): warp q holds tensor-memory lanes 32q .. 32q+31 = this CTA's rows of the tile =====
+    const int q = warp - 4;
+    const uint32_t leader_empty = xb::mapa_shared(xb::smem_u32(&tmem_empty[0]), 0);
+    const LtcEpilogue<EPI, TC> ep(a);
+    unsigned ti = 0;
+    for (int t = pair; t < total; t += npairs, ++ti) {
+      const uint32_t buf = ti & 1u;
+      const int row = (t % mtiles) * 2 * LTC_M + (int)rank * LTC_M + q * 32 + lane, n0 = (t / mtiles) * NT;
+      if (!ltc_wait(&tmem_full[buf], (ti >> 1) & 1u, a.err)) break;
+      xb::tc_fence_after();
+#pragma unroll 1
+      for (int c0 = 0; c0 < NT; c0 += 16) {
+        uint32_t v[16];
+        xb::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + buf * NT + (uint32_t)c0, v);   // warp-collective: before any row / column test
+        if (row < a.M && n0 + c0 < a.N) ep.store16(a, static_cast<TC*>(a.C) + (size_t)row * a.ldc, row, n0 + c0, v);
+      }
+      xb::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) xb::mbar_arrive_cluster(leader_empty + buf * 8);
+    }
+  }
+  __syncwarp();
+  xb::tc_fence_before();
+  __syncthreads();
+  xb::cluster_sync_all();                 // nobody leaves while the peer may still signal its barriers or read its shared memory
+  if (warp == 2) xb::tmem_dealloc_2sm(tmem_base, 2 * NT);
 }
 
 }  // namespace xl
