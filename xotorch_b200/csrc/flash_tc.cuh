@@ -1,0 +1,360 @@
+// flash_tc.cuh — prompt attention on the 5th-generation tensor cores (both engines): one CTA = 128 query rows of one request x one query head.
+//
+//   warp 0   one thread brings Q once and then the key / value tiles of 64 tokens by TMA (SWIZZLE_128B) into their rings;
+//   warp 1   one thread issues tcgen05.mma: S_j = Q K_j^T (128 x 64, fp32, tensor memory) one tile ahead, then O += P_j V_j with P read from tensor
+//            memory and V as it lies in memory ([token][value], the MN-major form of the B operand);
+//   warps 2-5  thread = query row: the row's 64 scores come by tcgen05.ld, so scale, soft cap, distance terms, mask, maximum and sum need no
+//            shuffle; the weights go back over the scores as the packed A operand of the value product.
+// PAIR: the weights enter the value product as a 16-bit PAIR (high part + remainder, two MMAs), 16 mantissa bits instead of 8.
+// The output is rescaled only when a row's maximum has grown by more than 2^8 since the last time (the reference the exponentials are taken
+// against is then stale by that factor at most, which fp32 sums and floating-point weights carry without loss).  Scores are kept in units of
+// ln 2.  Two CTAs share an SM (256 of the 512 tensor-memory columns and at most 112 KB each), so one's exponentials run under the other's MMAs: bound
+// by the exponentials and the arithmetic around them, not by the tensor pipe.
+// Every wait is bounded: one that expires sets *err, all roles of the CTA run out, it frees its tensor memory and returns.
+#pragma once
+#include "prefill_tc.cuh"
+
+namespace xf {
+
+constexpr int FT_Q = 128, FT_K = 64, FT_THREADS = 192;
+constexpr unsigned FT_SPIN_LIMIT = 1u << 22;   // try_wait rounds (each blocks for a while in hardware): seconds, not forever
+constexpr float LOG2E = 1.4426950408889634f;
+
+struct FlashTile128 {
+  int row0;      // first packed row
+  int n_rows;    // <= 128 consecutive rows of one request
+  int pos0;      // position of row0
+  int kbase;     // contiguous keys: index of position kfirst's key; paged keys: the request's slot
+  int kfirst;    // contiguous keys: position of the first key that is there
+};
+
+struct FlashArgs {
+  const FlashTile128* tiles;   // NULL: one request, tile t holds rows 128 t .. of n_rows rows from position pos0 (kbase, kfirst = 0)
+  int n_rows, pos0;
+  int H, rep, head_rows;       // query heads; query heads per key/value head; contiguous keys: rows between two key/value heads (0: heads lie side by side)
+  int kx, kx_head, k2_from, k2x, vx, vx_head;   // first column of the keys / per (key/value or query) head; chunk from which keys come from the second map, its first column
+  int kv_per_query_head;       // 1: every query head has keys and values of its own
+  const int* page_table;       // paged keys (NULL: contiguous)
+  int pages_per_slot, page_size;
+  float scale, cap;
+  int window, chunk;
+  const float *dist, *rel;     // [H][dist_n] subtracted, [H][rel_n] added per distance (NULL: none)
+  int dist_n, rel_n;
+  const void* sink;            // per query head, bf16 (NULL: none)
+  int sink_one;
+  const float* gate;
+  int gate_mode, gate_ld, gate_col0;   // 0 none, 1 sigmoid per head, 2 per entry
+  void* out;                   // [rows][H * dv], 16-bit
+  int* err;
+};
+
+__host__ __device__ constexpr int ft_k_stages(int) { return 2; }
+__host__ __device__ constexpr int ft_v_stages(int dkc, int dvc) { return dkc * 2 + dvc <= 6 ? 2 : 1; }
+__host__ __device__ constexpr int ft_smem_bytes(int dkc, int dvc) {
+  return dkc * FT_Q * 128 + ft_k_stages(dkc) * dkc * FT_K * 128 + ft_v_stages(dkc, dvc) * dvc * FT_K * 128 + 256 + 512;
+}
+
+__device__ __forceinline__ bool ft_wait(uint64_t* bar, uint32_t parity, volatile int* abort, int* err) {
+  for (unsigned i = 0; i < FT_SPIN_LIMIT; ++i) {
+    if (xb::mbar_try_wait(bar, parity)) return true;
+    if (*abort) return false;
+  }
+  *abort = 1;
+  if (err) atomicExch(err, 3);
+  return false;
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(xb::smem_u32(bar)) : "memory"); }
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+                 "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),
+                 "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+               : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+               "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+               "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+               "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// A from tensor memory (one 32-bit column = two consecutive k of a row), B from shared memory
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      : "memory");
+}
+// B [n][k] stored k row by k row ([64 tokens][64 values] chunks of 8 KB, 128-byte swizzle), the MN-major form: leading offset = from one 64-value chunk to
+// the next, stride offset = from 8 tokens to the next 8 (1024 bytes)
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)((FT_K * 128) >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+// instruction descriptor of kind::f16: fp32 accumulator, A and B both bf16 or both fp16; bit 16: B is MN-major
+__host__ __device__ constexpr uint32_t ft_idesc(int m, int n, bool f16, bool b_mn) {
+  return (1u << 4) | ((f16 ? 0u : 1u) << 7) | ((f16 ? 0u : 1u) << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+template <bool F16>
+__device__ __forceinline__ uint32_t pack16(float lo, float hi) {
+  uint32_t r;
+  if (F16) asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ int ft_first_key(int pos, int window, int chunk) {
+  int f = 0;
+  if (window > 0 && pos - window + 1 > f) f = pos - window + 1;
+  if (chunk > 0 && pos / chunk * chunk > f) f = pos / chunk * chunk;
+  return f;
+}
+
+// DKC, DVC: 64-wide chunks of a query / key row and of a value row
+template <int DKC, int DVC, bool PAIR, bool F16>
+__global__ void __launch_bounds__(FT_THREADS, 2)
+flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmK2,
+                const __grid_constant__ CUtensorMap tmV, const FlashArgs a) {
+  extern __shared__ __align__(1024) uint8_t ft_smem[];
+  constexpr int KS = ft_k_stages(DKC), VS = ft_v_stages(DKC, DVC), Q_BYTES = DKC * FT_Q * 128, K_BYTES = DKC * FT_K * 128, V_BYTES = DVC * FT_K * 128;
+  constexpr int COLS = 256;                          // tensor memory: S / P [2][64], then O [64 DVC]
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ft_smem) + 1023) & ~(uintptr_t)1023);
+  uint8_t *qs = base, *ks = qs + Q_BYTES, *vs = ks + KS * K_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(vs + VS * V_BYTES);
+  uint64_t *q_full = bars, *k_full = bars + 1, *k_empty = k_full + KS, *v_full = k_empty + KS, *v_empty = v_full + VS, *s_full = v_empty + VS, *p_full = s_full + 2,
+           *pv_done = p_full + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+  volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  xb::pdl_enter();
+  if (base - ft_smem > 512) {                        // cannot be (the shared window starts on a 1 KB boundary); the sizes leave 512 bytes for it
+    if (threadIdx.x == 0 && a.err) atomicExch(a.err, 4);
+    return;
+  }
+  FlashTile128 tl;
+  if (a.tiles) tl = a.tiles[gridDim.x - 1 - blockIdx.x];   // later tiles of a request see more keys: the long ones start first
+  else {
+    const int t = gridDim.x - 1 - blockIdx.x;
+    tl = FlashTile128{t * FT_Q, min(FT_Q, a.n_rows - t * FT_Q), a.pos0 + t * FT_Q, 0, 0};
+  }
+  const int h = blockIdx.y, g = a.kv_per_query_head ? h : h / a.rep;
+  const int last = tl.pos0 + tl.n_rows - 1;
+  int jstart = ft_first_key(tl.pos0, a.window, a.chunk);
+  if (a.page_table) jstart &= ~(FT_K - 1);           // a tile of paged keys lies in one page
+  const int nt = (last - jstart) / FT_K + 1;
+  if (threadIdx.x == 0) {
+    *abort = 0;
+    xb::mbar_init(q_full, 1);
+    for (int i = 0; i < KS; ++i) { xb::mbar_init(&k_full[i], 1); xb::mbar_init(&k_empty[i], 1); }
+    for (int i = 0; i < VS; ++i) { xb::mbar_init(&v_full[i], 1); xb::mbar_init(&v_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { xb::mbar_init(&s_full[i], 1); xb::mbar_init(&p_full[i], 128); xb::mbar_init(&pv_done[i], 1); }
+    xb::fence_mbar_init();
+  }
+  if (warp == 1) xb::tmem_alloc(tmem_slot, COLS);
+  xb::tc_fence_before();
+  __syncthreads();
+  xb::tc_fence_after();
+  const uint32_t tmem = *tmem_slot, tm_o = tmem + 128;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // ===== TMA producer =====
+      xb::mbar_expect_tx(q_full, Q_BYTES);
+      for (int c = 0; c < DKC; ++c) xb::tma_load_3d(qs + c * FT_Q * 128, &tmQ, c * 64, h, tl.row0, q_full);
+      bool ok = true;
+      int nk = 0, nv = 0;                            // tiles issued
+      for (int j = 0; j < nt && ok; ++j) {
+        const int pos = jstart + j * FT_K;
+        const int row = a.page_table ? a.page_table[(size_t)tl.kbase * a.pages_per_slot + pos / a.page_size] * a.page_size + pos % a.page_size
+                                     : tl.kbase + pos - tl.kfirst + g * a.head_rows;
+        ok = ft_wait(&k_empty[j % KS], ((j / KS) & 1) ^ 1, abort, a.err);
+        if (!ok) break;
+        xb::mbar_expect_tx(&k_full[j % KS], K_BYTES);
+        for (int c = 0; c < DKC; ++c) {
+          uint8_t* dst = ks + (j % KS) * K_BYTES + c * FT_K * 128;
+          if (c < a.k2_from) xb::tma_load_3d(dst, &tmK, a.kx + g * a.kx_head + c * 64, row, 0, &k_full[j % KS]);
+          else xb::tma_load_3d(dst, &tmK2, a.k2x + (c - a.k2_from) * 64, row, 0, &k_full[j % KS]);
+        }
+        nk = j + 1;
+        ok = ft_wait(&v_empty[j % VS], ((j / VS) & 1) ^ 1, abort, a.err);
+        if (!ok) break;
+        xb::mbar_expect_tx(&v_full[j % VS], V_BYTES);
+        for (int c = 0; c < DVC; ++c) xb::tma_load_3d(vs + (j % VS) * V_BYTES + c * FT_K * 128, &tmV, a.vx + g * a.vx_head + c * 64, row, 0, &v_full[j % VS]);
+        nv = j + 1;
+      }
+      if (!ok) {   // gave up: the copies still in flight land before the CTA's shared memory goes away
+        volatile int never = 0;
+        ft_wait(q_full, 0, &never, nullptr);
+        for (int j = max(0, nk - KS); j < nk; ++j) ft_wait(&k_full[j % KS], (j / KS) & 1, &never, nullptr);
+        for (int j = max(0, nv - VS); j < nv; ++j) ft_wait(&v_full[j % VS], (j / VS) & 1, &never, nullptr);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // ===== MMA issuer =====
+      constexpr uint32_t id_s = ft_idesc(FT_Q, FT_K, F16, false), id_o = ft_idesc(FT_Q, 64 * DVC, F16, true);
+      bool ok = ft_wait(q_full, 0, abort, a.err);
+      for (int j = 0; j <= nt && ok; ++j) {
+        if (j < nt) {
+          ok = ft_wait(&k_full[j % KS], (j / KS) & 1, abort, a.err);
+          if (ok && j >= 2) ok = ft_wait(&pv_done[j & 1], ((j - 2) >> 1) & 1, abort, a.err);   // the weights that lie over these scores have been used
+          if (!ok) break;
+          xb::tc_fence_after();
+          const uint32_t sq = xb::smem_u32(qs), sk = xb::smem_u32(ks + (j % KS) * K_BYTES);
+#pragma unroll
+          for (int c = 0; c < DKC; ++c)
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              xb::umma_bf16(tmem + (j & 1) * 64, xb::umma_desc_sw128(sq + c * FT_Q * 128 + k * 32), xb::umma_desc_sw128(sk + c * FT_K * 128 + k * 32), id_s, (c | k) != 0 ? 1u : 0u);
+          xb::umma_commit(&k_empty[j % KS]);
+          xb::umma_commit(&s_full[j & 1]);
+        }
+        if (j >= 1) {
+          const int i = j - 1;
+          ok = ft_wait(&p_full[i & 1], (i >> 1) & 1, abort, a.err) && ft_wait(&v_full[i % VS], (i / VS) & 1, abort, a.err);
+          if (!ok) break;
+          xb::tc_fence_after();
+          const uint32_t sv = xb::smem_u32(vs + (i % VS) * V_BYTES), p = tmem + (i & 1) * 64;
+#pragma unroll
+          for (int part = 0; part < (PAIR ? 2 : 1); ++part)
+#pragma unroll
+            for (int k = 0; k < FT_K / 16; ++k) umma_ts(tm_o, p + part * 32 + k * 8, umma_desc_mn(sv + k * 2048), id_o, (i | part | k) != 0 ? 1u : 0u);
+          xb::umma_commit(&v_empty[i % VS]);
+          xb::umma_commit(&pv_done[i & 1]);
+        }
+      }
+    }
+  } else {
+    // ===== softmax: warp w reads tensor-memory lanes 32 (w mod 4) .. =====
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const int r = (warp & 3) * 32 + lane, pos = tl.pos0 + r;
+    const int lo = ft_first_key(pos, a.window, a.chunk), lo_last = ft_first_key(last, a.window, a.chunk);
+    const float scale2 = a.scale * LOG2E, inv_cap2 = a.cap > 0.f ? 2.0f * LOG2E * a.scale / a.cap : 0.f, cap2 = a.cap * LOG2E;
+    const float* dist = a.dist ? a.dist + (size_t)h * a.dist_n : nullptr;
+    const float* rel = a.rel ? a.rel + (size_t)h * a.rel_n : nullptr;
+    float m = -INFINITY, den = 0.f;                  // reference of the exponentials (units of ln 2), sum of the weights
+    bool ok = true;
+    for (int j = 0; j < nt; ++j) {
+      ok = __all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err));
+      if (!ok) break;
+      xb::tc_fence_after();
+      const uint32_t ts = tmem + lane_base + (j & 1) * 64;
+      uint32_t raw[2][32];
+      tmem_ld32(ts, raw[0]);
+      tmem_ld32(ts + 32, raw[1]);
+      float s[64];
+#pragma unroll
+      for (int c = 0; c < 64; ++c) s[c] = __uint_as_float(raw[c >> 5][c & 31]);
+      const int j0 = jstart + j * FT_K;
+      if (a.cap > 0.f) {                             // cap tanh(x / cap) with tanh y = 1 - 2 / (e^2y + 1)
+#pragma unroll
+        for (int c = 0; c < 64; ++c) {
+          const float t = ex2(fminf(fmaxf(s[c] * inv_cap2, -43.3f), 43.3f));
+          s[c] = cap2 * __fdividef(t - 1.0f, t + 1.0f);
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < 64; ++c) s[c] *= scale2;
+      }
+      if (dist) {
+#pragma unroll
+        for (int c = 0; c < 64; ++c) s[c] = fmaf(-LOG2E, __ldg(dist + min(max(pos - j0 - c, 0), a.dist_n - 1)), s[c]);
+      }
+      if (rel) {
+#pragma unroll
+        for (int c = 0; c < 64; ++c) s[c] = fmaf(LOG2E, __ldg(rel + min(max(pos - j0 - c, 0), a.rel_n - 1)), s[c]);
+      }
+      if (j0 + FT_K - 1 > tl.pos0 || j0 < lo_last) { // some row of the tile does not see all keys
+        const int clo = lo - j0, chi = pos - j0;
+#pragma unroll
+        for (int c = 0; c < 64; ++c) s[c] = c >= clo && c <= chi ? s[c] : -INFINITY;
+      }
+      float t0 = fmaxf(s[0], s[1]), t1 = fmaxf(s[2], s[3]);
+#pragma unroll
+      for (int c = 4; c < 64; c += 4) { t0 = fmaxf(t0, fmaxf(s[c], s[c + 1])); t1 = fmaxf(t1, fmaxf(s[c + 2], s[c + 3])); }
+      const float tmax = fmaxf(t0, t1);
+      const bool grow = tmax > m + 8.0f || (m == -INFINITY && tmax > -INFINITY);
+      if (__any_sync(0xffffffffu, grow)) {
+        const float nm = fmaxf(m, tmax), corr = m == -INFINITY ? 0.f : ex2(m - nm);
+        if (j > 0) {
+          ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort, a.err));   // the output as it is
+          if (!ok) break;
+          xb::tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < 64 * DVC; c += 32) {
+            uint32_t o[32];
+            tmem_ld32(tm_o + lane_base + c, o);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+            tmem_st32(tm_o + lane_base + c, o);
+          }
+          tmem_st_wait();
+        }
+        den *= corr;
+        m = nm;
+      }
+      const float mm = m == -INFINITY ? 0.f : m;     // a row that has not seen a key yet: every weight is ex2(-inf) = 0
+      float d0 = 0.f, d1 = 0.f;
+      uint32_t hi[32], rest[32];
+#pragma unroll
+      for (int c = 0; c < 64; c += 2) {
+        const float p0 = ex2(s[c] - mm), p1 = ex2(s[c + 1] - mm);
+        d0 += p0;
+        d1 += p1;
+        hi[c >> 1] = pack16<F16>(p0, p1);
+        if constexpr (PAIR)   // bf16: the high parts as fp32 are the packed words' halves
+          rest[c >> 1] = pack16<F16>(p0 - __uint_as_float(hi[c >> 1] << 16), p1 - __uint_as_float(hi[c >> 1] & 0xffff0000u));
+      }
+      den += d0 + d1;
+      tmem_st32(ts, hi);
+      if constexpr (PAIR) tmem_st32(ts + 32, rest);
+      tmem_st_wait();
+      xb::tc_fence_before();
+      mbar_arrive(&p_full[j & 1]);
+    }
+    if (ok) ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(nt - 1) & 1], ((nt - 1) >> 1) & 1, abort, a.err));
+    if (ok) {
+      xb::tc_fence_after();
+      float f = 1.0f;
+      if (a.sink || a.sink_one) {
+        const float sk = a.sink ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.sink)[h]) * LOG2E : 0.f, nm = fmaxf(m, sk);
+        f = m == -INFINITY ? 0.f : ex2(m - nm);
+        den = den * f + ex2(sk - nm);
+      }
+      f /= den;
+      const size_t row = (size_t)tl.row0 + r;
+      const float* gt = a.gate_mode && r < tl.n_rows ? a.gate + row * a.gate_ld + a.gate_col0 + (a.gate_mode == 1 ? h : h * 64 * DVC) : nullptr;
+      if (a.gate_mode == 1 && gt) f *= 1.0f / (1.0f + expf(-*gt));
+      uint16_t* dst = static_cast<uint16_t*>(a.out) + (row * a.H + h) * (64 * DVC);
+#pragma unroll 1
+      for (int c = 0; c < 64 * DVC; c += 32) {
+        uint32_t o[32];
+        tmem_ld32(tm_o + lane_base + c, o);
+        if (r < tl.n_rows) {
+          float v[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * f;
+          if (a.gate_mode == 2) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] *= 1.0f / (1.0f + expf(-gt[c + i]));
+          }
+#pragma unroll
+          for (int i = 0; i < 32; i += 8)
+            *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(pack16<F16>(v[i], v[i + 1]), pack16<F16>(v[i + 2], v[i + 3]), pack16<F16>(v[i + 4], v[i + 5]), pack16<F16>(v[i + 6], v[i + 7]));
+        }
+        __syncwarp();
+      }
+    }
+  }
+  xb::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) xb::tmem_dealloc(tmem, COLS);
+}
+
+}  // namespace xf

@@ -33,6 +33,7 @@
 #include "layered_tc.cuh"
 #include "layered_stream.cuh"
 #include "layered_fma.cuh"
+#include "flash_tc.cuh"
 #include "st_header.h"
 
 using namespace xl;
@@ -835,7 +836,7 @@ static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& 
   auto kern = ltc_pair_kernel<EPI, TC>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LTP_SMEM));
   const int tiles = cdiv(a.M, 2 * LTC_M) * cdiv(a.N, LTP_N), pairs = std::min(tiles, e->sm_count / 2);
-  TRY(launch_late(e, kern, 2 * pairs, LTC_THREADS, LTP_SMEM, ma, mb, a));
+  TRY(launch_late(e, kern, 2 * pairs, LTP_THREADS, LTP_SMEM, ma, mb, a));
   e->tc_launches++;
   return 0;
 }
@@ -1053,6 +1054,8 @@ struct StepPlan {
   struct Flash {
     const GatherReq* reqs = nullptr;
     const FlashTile* tiles = nullptr;
+    const xf::FlashTile128* tiles128 = nullptr;        // the same rows in 128-row tiles
+    int n_tiles128 = 0;
     int n_reqs = 0, n_tiles = 0, n_keys = 0, max_keys = 0;
   };
   std::map<int, Flash> flash;
@@ -1060,6 +1063,8 @@ struct StepPlan {
   int max_rows = 0;                                    // most rows one request brings
   const GqaTile* gqa_tiles = nullptr;                  // key/value-cache attention, long portions (bf16): 64-row tiles
   int n_gqa_tiles = 0;
+  const xf::FlashTile128* gqa_tiles128 = nullptr;      // the same rows in 128-row tiles
+  int n_gqa_tiles128 = 0;
   bool any_short = true;                               // some request goes through the absorbed kernel
 };
 
@@ -1078,6 +1083,31 @@ static int latent_key_runs(const xotb200_lm* e, const xotb200_lm_layer& s, int n
   if (ctas > 0 && ctas < e->sm_count) splits = std::max(1, std::min(std::min(32, cdiv(span, 32)), cdiv(2 * e->sm_count, ctas)));
   *run = cdiv(cdiv(span, splits), 32) * 32;
   return cdiv(span, *run);
+}
+
+// ---- prompt attention on tcgen05 (flash_tc.cuh) ---------------------------------------------------------------------------------
+// queries [M][H][d] as a 3-D map {d, H, M} with a box of 64 entries of one head of 128 rows
+static bool make_query_map(CUtensorMap* m, const bf16* q, int M, int H, int d) {
+  encode_tiled_fn enc = get_encode_tiled();
+  if (!enc || (reinterpret_cast<uintptr_t>(q) & 15) || d % 8) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)d, (cuuint64_t)H, (cuuint64_t)M};
+  const cuuint64_t strides[2] = {(cuuint64_t)d * 2, (cuuint64_t)H * d * 2};
+  const cuuint32_t box[3] = {64, 1, xf::FT_Q}, es[3] = {1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(q), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+template <int DKC, int DVC>
+static int launch_flash_tc(xotb200_lm* e, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mk2, const CUtensorMap& mv, const xf::FlashArgs& a, int n_tiles) {
+  auto kern = xf::flash_tc_kernel<DKC, DVC, true, false>;
+  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, xf::ft_smem_bytes(DKC, DVC)));
+  TRY(launch_late(e, kern, dim3(n_tiles, a.H), xf::FT_THREADS, xf::ft_smem_bytes(DKC, DVC), mq, mk, mk2, mv, a));
+  e->flash_launches++;
+  return 0;
+}
+static int run_flash_tc(xotb200_lm* e, int dkc, int dvc, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mk2, const CUtensorMap& mv, const xf::FlashArgs& a,
+                        int n_tiles) {
+  if (dvc == 1) return dkc == 1 ? launch_flash_tc<1, 1>(e, mq, mk, mk2, mv, a, n_tiles) : dkc == 2 ? launch_flash_tc<2, 1>(e, mq, mk, mk2, mv, a, n_tiles) : launch_flash_tc<3, 1>(e, mq, mk, mk2, mv, a, n_tiles);
+  return dkc == 1 ? launch_flash_tc<1, 2>(e, mq, mk, mk2, mv, a, n_tiles) : dkc == 2 ? launch_flash_tc<2, 2>(e, mq, mk, mk2, mv, a, n_tiles) : launch_flash_tc<3, 2>(e, mq, mk, mk2, mv, a, n_tiles);
 }
 
 template <typename T>
@@ -1152,6 +1182,18 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
       TRY(launch_early(e, latent_gather_kernel<bf16>, dim3(cdiv(fl->max_keys, 8), fl->n_reqs), 256, 0, 1, static_cast<const bf16*>(L.pool), pg, fl->reqs, R + dr, cbuf));
       TRY((product<bf16, bf16, bf16, 0>(e, cbuf, R + dr, 0, at<bf16>(e, L.uk_rows), R, 1, 0, knx, (long)H * dn, 0, fl->n_keys, H * dn, R, 1)));
       TRY((product<bf16, bf16, bf16, 0>(e, cbuf, R + dr, 0, at<bf16>(e, L.uv), R, 1, 0, vxx, (long)H * dv, 0, fl->n_keys, H * dv, R, 1)));
+      // heads of whole 64-entry chunks (the rotated part may end inside one: beyond its row the loads read zeros): tcgen05; else mma.sync
+      const int dkc = dn / 64 + cdiv(dr, 64);
+      CUtensorMap mq, mk, mk2, mv;
+      if (dn % 64 == 0 && dn > 0 && dkc <= 3 && dr % 8 == 0 && R % 8 == 0 && (dv == 64 || dv == 128) && make_query_map(&mq, q16, M, H, dn + dr) &&
+          make_map3(&mk, knx, fl->n_keys, (long)H * dn, (long)H * dn, 0, 1, xf::FT_K) && make_map3(&mk2, cbuf, fl->n_keys, R + dr, R + dr, 0, 1, xf::FT_K) &&
+          make_map3(&mv, vxx, fl->n_keys, (long)H * dv, (long)H * dv, 0, 1, xf::FT_K)) {
+        xf::FlashArgs a = {};
+        a.tiles = fl->tiles128; a.H = H; a.rep = 1; a.kv_per_query_head = 1; a.kx_head = dn; a.k2_from = dn / 64; a.k2x = R; a.vx_head = dv;
+        a.scale = s.scale; a.window = s.window; a.sink = sink;
+        a.gate = gate; a.gate_mode = gate ? 1 : 0; a.gate_ld = L.n_in; a.gate_col0 = L.c_g; a.out = e->oh; a.err = e->d_err;
+        TRY(run_flash_tc(e, dkc, dv / 64, mq, mk, mk2, mv, a, fl->n_tiles128));
+      } else {
       const int dqp = (dn + dr + 15) & ~15, dvt = dv <= 64 ? 8 : 16;
       const dim3 grid(fl->n_tiles, H);
       const bool aligned = dn % 8 == 0 && dr % 8 == 0 && R % 8 == 0 && dv % 8 == 0;
@@ -1173,6 +1215,7 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
       }
 #undef LAUNCH_FLASH
       e->flash_launches++;
+      }
     }
   }
   // the output projection
@@ -1361,6 +1404,7 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
   if constexpr (std::is_same<T, bf16>::value) {
     if (sp.n_gqa_tiles > 0) {
       // long portions: streaming softmax on the tensor cores, keys and values straight from the pages
+      // whole 64-entry chunks, whole 64-token pieces of pages, no keys in front of the token stretch: tcgen05; else mma.sync
       const int dqp = (dk + 15) & ~15, dvt = dv <= 64 ? 8 : 16;
       const size_t fsm = ((size_t)3 * 64 * (dqp + 8) + (size_t)2 * 64 * (8 * dvt + 8)) * 2;
       const dim3 grid(sp.n_gqa_tiles, H);
@@ -1372,6 +1416,18 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
         if ((size_t)H * dist_n > e->dist_cap) { TRY(regrow(e->dist_tab, (size_t)H * dist_n * 4)); e->dist_cap = (size_t)H * dist_n; }
         TRY(launch_early(e, gqa_dist_table_kernel, cdiv((long)H * dist_n, 256), 256, 0, 1, at<bf16>(e, L.r1), at<bf16>(e, L.r2), H, dist_n, e->dist_tab));
       }
+      CUtensorMap mq, mkv;
+      const long rowlen = (long)G * (dk + dv);
+      if (dk % 64 == 0 && dk <= 192 && (dv == 64 || dv == 128) && e->page_size % xf::FT_K == 0 && !(s.window > 0 && (s.keep_first > 0 || s.pool > 0)) &&
+          make_query_map(&mq, static_cast<const bf16*>(e->q16), M, H, dk) && make_map3(&mkv, pool, (long)e->n_pages * e->page_size, rowlen, rowlen, 0, 1, xf::FT_K)) {
+        xf::FlashArgs a = {};
+        a.tiles = sp.gqa_tiles128; a.H = H; a.rep = H / G; a.kx_head = dk; a.k2_from = dk / 64; a.vx = G * dk; a.vx_head = dv;
+        a.page_table = pg.page_table; a.pages_per_slot = pg.pages_per_slot; a.page_size = pg.page_size;
+        a.scale = sc.scale; a.cap = sc.cap; a.window = sc.window; a.chunk = sc.chunk;
+        a.dist = s.dist_bias ? e->dist_tab : nullptr; a.dist_n = dist_n; a.rel = sc.rel; a.rel_n = sc.rel_n; a.sink = sc.sink; a.sink_one = sc.sink_one;
+        a.gate = gate; a.gate_mode = s.out_gate; a.gate_ld = L.ld_in; a.gate_col0 = L.c_g; a.out = e->oh; a.err = e->d_err;
+        TRY(run_flash_tc(e, dk / 64, dv / 64, mq, mkv, mkv, mkv, a, sp.n_gqa_tiles128));
+      } else {
 #define LAUNCH_GQA_FLASH(DVT)                                                                                                              \
   do {                                                                                                                                     \
     auto kern = gqa_flash_kernel<DVT>;                                                                                                     \
@@ -1383,6 +1439,7 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
       else LAUNCH_GQA_FLASH(16);
 #undef LAUNCH_GQA_FLASH
       e->flash_launches++;
+      }
     }
   }
   TRY(output_product<T>(e, static_cast<T*>(e->oh), L.wo, H * dv, yout, M));
@@ -2403,22 +2460,29 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     item_off[qk] = {push(it.data(), 4 * it.size()), (int)it.size()};
     if (!it.empty() && qk > 0) sp.any_short = true;
   }
-  size_t gqa_tiles_off = 0;
-  int n_gqa_tiles = 0;
+  size_t gqa_tiles_off = 0, gqa_tiles128_off = 0;
+  int n_gqa_tiles = 0, n_gqa_tiles128 = 0;
   if (use_gqa_flash && std::any_of(qpis.begin(), qpis.end(), [](int q) { return q < 0; })) {
     std::vector<GqaTile> gt;
     for (int i = 0; i < n_seq; ++i)
       if (is_long_gqa(i))
         for (int t = 0; t < counts[i]; t += 64) gt.push_back(GqaTile{seqs[i].row0 + t, std::min(64, counts[i] - t), seqs[i].pos0 + t, seqs[i].slot});
+    std::vector<xf::FlashTile128> g2;
+    for (int i = 0; i < n_seq; ++i)
+      if (is_long_gqa(i))
+        for (int t = 0; t < counts[i]; t += xf::FT_Q) g2.push_back(xf::FlashTile128{seqs[i].row0 + t, std::min(xf::FT_Q, counts[i] - t), seqs[i].pos0 + t, seqs[i].slot, 0});
+    gqa_tiles128_off = push(g2.data(), 5 * g2.size());
+    n_gqa_tiles128 = (int)g2.size();
     gqa_tiles_off = push(gt.data(), 4 * gt.size());
     n_gqa_tiles = (int)gt.size();
   }
-  struct FlashOff { size_t reqs, tiles; int n_reqs, n_tiles, n_keys, max_keys; };
+  struct FlashOff { size_t reqs, tiles, tiles128; int n_reqs, n_tiles, n_tiles128, n_keys, max_keys; };
   std::map<int, FlashOff> flash_off;
   size_t flash_keys = 0;
   for (int w : windows) {
     std::vector<GatherReq> gr;
     std::vector<FlashTile> ft;
+    std::vector<xf::FlashTile128> f2;
     int kbase = 0, max_keys = 0;
     for (int i = 0; i < n_seq; ++i)
       if (is_long(i)) {
@@ -2426,11 +2490,12 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
         const int nkeys = seqs[i].pos0 + counts[i] - kfirst;
         gr.push_back(GatherReq{seqs[i].slot, kfirst, nkeys, kbase});
         for (int t = 0; t < counts[i]; t += 64) ft.push_back(FlashTile{seqs[i].row0 + t, std::min(64, counts[i] - t), seqs[i].pos0 + t, kbase, kfirst});
+        for (int t = 0; t < counts[i]; t += xf::FT_Q) f2.push_back(xf::FlashTile128{seqs[i].row0 + t, std::min(xf::FT_Q, counts[i] - t), seqs[i].pos0 + t, kbase, kfirst});
         kbase += nkeys;
         max_keys = std::max(max_keys, nkeys);
       }
     if (gr.empty()) continue;
-    flash_off[w] = FlashOff{push(gr.data(), 4 * gr.size()), push(ft.data(), 5 * ft.size()), (int)gr.size(), (int)ft.size(), kbase, max_keys};
+    flash_off[w] = FlashOff{push(gr.data(), 4 * gr.size()), push(ft.data(), 5 * ft.size()), push(f2.data(), 5 * f2.size()), (int)gr.size(), (int)ft.size(), (int)f2.size(), kbase, max_keys};
     flash_keys = std::max(flash_keys, (size_t)kbase);
   }
   if (flash_keys > e->flash_keys_cap) {
@@ -2499,10 +2564,14 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
       for (auto& kv : item_off) sp.items[kv.first] = {reinterpret_cast<const Item*>(e->d_stage + kv.second.first), kv.second.second};
       sp.gqa_tiles = reinterpret_cast<const GqaTile*>(e->d_stage + gqa_tiles_off);
       sp.n_gqa_tiles = n_gqa_tiles;
+      sp.gqa_tiles128 = reinterpret_cast<const xf::FlashTile128*>(e->d_stage + gqa_tiles128_off);
+      sp.n_gqa_tiles128 = n_gqa_tiles128;
       for (auto& kv : flash_off) {
         StepPlan::Flash f;
         f.reqs = reinterpret_cast<const GatherReq*>(e->d_stage + kv.second.reqs);
         f.tiles = reinterpret_cast<const FlashTile*>(e->d_stage + kv.second.tiles);
+        f.tiles128 = reinterpret_cast<const xf::FlashTile128*>(e->d_stage + kv.second.tiles128);
+        f.n_tiles128 = kv.second.n_tiles128;
         f.n_reqs = kv.second.n_reqs; f.n_tiles = kv.second.n_tiles; f.n_keys = kv.second.n_keys; f.max_keys = kv.second.max_keys;
         sp.flash[kv.first] = f;
       }

@@ -254,11 +254,11 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // leader's thread issues tcgen05.mma.cta_group::2 over both CTAs' shared memory, and every CTA keeps its 128 rows of the accumulator.  Persistent: 74
 // pairs walk the tiles (row tile fastest, so that pairs running together share weight tiles in L2) with two accumulators in tensor memory (all
 // 512 columns), so the epilogue of one tile runs under the products of the next.  Plain loads, no multicast.  Every wait is bounded.
-constexpr int LTP_N = 256, LTP_STAGES = 6, LTP_STAGE_BYTES = LTC_M * LTC_BK * 2 + LTP_N / 2 * LTC_BK * 2;
+constexpr int LTP_N = 256, LTP_STAGES = 6, LTP_THREADS = 384, LTP_STAGE_BYTES = LTC_M * LTC_BK * 2 + LTP_N / 2 * LTC_BK * 2;
 constexpr int LTP_SMEM = LTP_STAGES * LTP_STAGE_BYTES + 1024 + 256;
 
 template <int EPI, typename TC>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LTC_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LTP_THREADS, 1)
 ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LtcArgs a) {
   pdl_enter();
   extern __shared__ __align__(1024) uint8_t ltc_smem[];
@@ -267,7 +267,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   uint64_t* full = reinterpret_cast<uint64_t*>(base + NS * LTP_STAGE_BYTES);   // the leader's count both CTAs' copies
   uint64_t* empty = full + NS;
   uint64_t* tmem_full = empty + NS;       // [2]
-  uint64_t* tmem_empty = tmem_full + 2;   // [2], the leader's: 4 warps of both CTAs
+  uint64_t* tmem_empty = tmem_full + 2;   // [2], the leader's: 8 warps of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = xb::cluster_ctarank();
@@ -275,7 +275,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const int mtiles = (a.M + 2 * LTC_M - 1) / (2 * LTC_M), total = mtiles * ((a.N + NT - 1) / NT), nkb = (a.K + LTC_BK - 1) / LTC_BK;
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) { xb::mbar_init(&full[i], 1); xb::mbar_init(&empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { xb::mbar_init(&tmem_full[i], 1); xb::mbar_init(&tmem_empty[i], 8); }
+    for (int i = 0; i < 2; ++i) { xb::mbar_init(&tmem_full[i], 1); xb::mbar_init(&tmem_empty[i], 16); }
     xb::fence_mbar_init();
   }
   __syncthreads();
@@ -328,8 +328,9 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       if (ok) xb::umma_commit_2sm(&tmem_full[buf], 3);
     }
   } else if (warp >= 4) {
-    // ===== epilogue (both CTAs): warp q holds tensor-memory lanes 32q .. 32q+31 = this CTA's rows of the tile =====
-    const int q = warp - 4;
+    // ===== epilogue (both CTAs): warps q and q + 4 hold tensor-memory lanes 32q .. 32q+31 = this CTA's rows of the tile, half of the columns each
+    // (the last tile's epilogue runs under nothing, and a heavy activation must not take longer than the next tile's products) =====
+    const int q = warp & 3, half = (warp - 4) >> 2;
     const uint32_t leader_empty = xb::mapa_shared(xb::smem_u32(&tmem_empty[0]), 0);
     const LtcEpilogue<EPI, TC> ep(a);
     unsigned ti = 0;
@@ -339,7 +340,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       if (!ltc_wait(&tmem_full[buf], (ti >> 1) & 1u, a.err)) break;
       xb::tc_fence_after();
 #pragma unroll 1
-      for (int c0 = 0; c0 < NT; c0 += 16) {
+      for (int c0 = half * (NT / 2); c0 < (half + 1) * (NT / 2); c0 += 16) {
         uint32_t v[16];
         xb::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + buf * NT + (uint32_t)c0, v);   // warp-collective: before any row / column test
         if (row < a.M && n0 + c0 < a.N) ep.store16(a, static_cast<TC*>(a.C) + (size_t)row * a.ldc, row, n0 + c0, v);
