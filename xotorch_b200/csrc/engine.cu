@@ -39,6 +39,7 @@
 #include "kernels.cuh"
 #include "megakernel.cuh"
 #include "prefill_tc.cuh"
+#include "flash_tc.cuh"
 #include "st_header.h"
 
 // Decode GEMV inner loop: 1 = mma.sync tensor-core path (default), 0 = the round-1 packed-FFMA2 loop (kept for A/B builds:
@@ -664,8 +665,36 @@ static int tc_gemm_expert(xotb200_engine* e, const CUtensorMap& tmA, int widx, T
   return launch_tc_gemm(e, tmA, e->tm_w[c.nt][widx], a, TCE_STORE, c, st);
 }
 
+// 16-bit matrix [rows][heads][cols] as a 3-D map {cols, heads, rows}, box {64, 1, box_rows}; heads 1: [rows][cols] as {cols, rows, 1}, box {64, box_rows, 1}
+static int make_tmap_heads(CUtensorMap* m, const bf16* ptr, int cols, int heads, long rows, int box_rows) {
+  encode_tiled_fn enc = get_encode_tiled();
+  REQUIRE(enc != nullptr, "cuTensorMapEncodeTiled not available from the driver");
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)(heads > 1 ? heads : rows), (cuuint64_t)(heads > 1 ? rows : 1)};
+  const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)cols * 2 * (heads > 1 ? heads : rows)};
+  const cuuint32_t box[3] = {64, (cuuint32_t)(heads > 1 ? 1 : box_rows), (cuuint32_t)(heads > 1 ? box_rows : 1)}, es[3] = {1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(heads, %d columns) failed: %d", cols, (int)r);
+  return 0;
+}
+// causal attention of a chunk on tcgen05 (flash_tc.cuh): q [S][Hq][HD], K / V [Hkv][L][HD]
+template <int HD>
+static int launch_tc_flash(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, int pos0, cudaStream_t st) {
+  const int Hq = e->cfg.n_heads;
+  CUtensorMap mq, mk, mv;
+  if (int rc = make_tmap_heads(&mq, e->tc_q, HD, Hq, S, xf::FT_Q)) return rc;
+  if (int rc = make_tmap_heads(&mk, kc, HD, 1, (long)e->cfg.n_kv_heads * e->L, xf::FT_K)) return rc;
+  if (int rc = make_tmap_heads(&mv, vc, HD, 1, (long)e->cfg.n_kv_heads * e->L, xf::FT_K)) return rc;
+  xf::FlashArgs a = {};
+  a.n_rows = S; a.pos0 = pos0; a.H = Hq; a.rep = R; a.head_rows = e->L; a.k2_from = HD / 64; a.scale = 1.0f / sqrtf((float)HD); a.out = e->tc_ao; a.err = &e->ctl->err;
+  auto fn = e->cfg.dtype == XOTB200_DTYPE_F16 ? xf::flash_tc_kernel<HD / 64, HD / 64, false, true> : xf::flash_tc_kernel<HD / 64, HD / 64, false, false>;
+  if (int rc = ensure_smem_attr(e->device, (const void*)fn, xf::ft_smem_bytes(HD / 64, HD / 64))) return rc;
+  return launch_early(e, st, fn, dim3((S + xf::FT_Q - 1) / xf::FT_Q, Hq), xf::FT_THREADS, xf::ft_smem_bytes(HD / 64, HD / 64), 1, mq, mk, mk, mv, a);
+}
+
 template <int HD>
 static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, int pos0, cudaStream_t st) {
+  if (S >= 64 && e->cfg.n_heads > 1) return launch_tc_flash<HD>(e, S, R, kc, vc, pos0, st);
   constexpr int SMEM = (64 + 4 * 64) * HD * 2;          // Q tile + 2 x (K, V) tiles
   const bool f16 = e->cfg.dtype == XOTB200_DTYPE_F16;
   auto fn = f16 ? xb::fp::tc_flash_attn_kernel<HD> : xb::bf::tc_flash_attn_kernel<HD>;

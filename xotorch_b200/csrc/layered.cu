@@ -1246,12 +1246,16 @@ static int run_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks,
     const int cpw = (32 / P) * NC, warps = std::max(1, std::min(4, cdiv(dv, cpw)));
     return 4L * sp.n_seq * L.s.heads * cdiv(dv, warps * cpw) >= 3L * e->sm_count;
   };
+  // a prompt of one request: with the P = 8 variants a scheduler has one warp, which waits four cycles of five; sixteen lanes per column make
+  // it two warps of half the work each
+  auto busy = [&](int P, int NC) { return (long)sp.n_seq * L.s.heads * cdiv(dv, 4 * (32 / P) * NC) > e->sm_count; };
   if (d <= 16) return launch_delta<4, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, form);
   if (d <= 32) return fills(4, 2) ? launch_delta<8, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, form) : launch_delta<8, 4, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
   if (d <= 64)
     return fills(8, 4) ? launch_delta<8, 8, 4>(e, L, sp, ks, rs, vs, dk, dv, form)
          : fills(8, 2) ? launch_delta<8, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form)
-                       : launch_delta<8, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
+                       : launch_delta<4, 16, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
+  if (d <= 128 && !busy(8, 2)) return launch_delta<8, 16, 2>(e, L, sp, ks, rs, vs, dk, dv, form);
   if (d <= 128) return fills(8, 2) ? launch_delta<16, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form) : launch_delta<16, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
   return launch_delta<32, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
 }

@@ -674,7 +674,7 @@ __global__ void __launch_bounds__(128, 2) delta_rule_kernel(DeltaSrc ksrc, Delta
   constexpr int DKP = KPT * P;                       // padded size: >= dk and >= dv
   constexpr int NVEC = SCALAR ? 3 : 6;               // k, r, v (then w, u, au)
   constexpr int CH = DKP <= 64 ? 16 : DKP <= 128 ? 8 : 4;   // tokens per buffer: two buffers fit the 48 KB of static shared memory
-  constexpr int Q = KPT / 4, TG = 4;                 // runs of four rows per thread; tokens whose read-outs are summed together
+  constexpr int Q = KPT / 4, TG = P / NC < 4 ? 4 : P / NC < CH ? P / NC : CH;   // runs of four rows per thread; tokens whose read-outs are summed together
   __shared__ __align__(16) float buf[2][CH][NVEC][DKP];
   __shared__ __align__(16) float gb[2][CH][4];       // SCALAR: g, beta, k of the token . k of the next one
   const Item sq = seqs[blockIdx.x / H];
@@ -852,39 +852,31 @@ __global__ void __launch_bounds__(128, 2) delta_rule_kernel(DeltaSrc ksrc, Delta
           if (t0 + g < nt) token(t0 + g, out[g]);
         }
       }
-      // sums over the P lanes of TG * NC read-outs at once: each step halves the values a lane still holds
-      if constexpr (TG * NC >= P) {
-        float v[TG * NC];
+      // sums over the P lanes of TG * NC read-outs at once: each step halves the values a lane still holds, down to one
+      constexpr int NV = TG * NC, LEFT = NV > P ? NV / P : 1, SAME = NV < P ? P / NV : 1;   // values a lane ends with; lanes that end with the same one
+      float v[NV];
 #pragma unroll
-        for (int g = 0; g < TG; ++g)
+      for (int g = 0; g < TG; ++g)
 #pragma unroll
-          for (int x = 0; x < NC; ++x) v[g * NC + x] = out[g][x];
+        for (int x = 0; x < NC; ++x) v[g * NC + x] = out[g][x];
 #pragma unroll
-        for (int o = P / 2, n = TG * NC; o > 0; o >>= 1, n >>= 1) {
+      for (int o = P / 2, n = NV; o > 0; o >>= 1, n = n > 1 ? n >> 1 : 1) {
+        if (n > 1) {
           const bool up = part & o;
 #pragma unroll
-          for (int i = 0; i < TG * NC / 2; ++i)
+          for (int i = 0; i < NV / 2; ++i)
             if (i < n / 2) {
               const float keep = up ? v[i + n / 2] : v[i], give = up ? v[i] : v[i + n / 2];
               v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
             }
+        } else {
+          v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
         }
-        constexpr int LEFT = TG * NC / P;                    // values this lane ends with: LEFT * part ..
+      }
 #pragma unroll
-        for (int i = 0; i < LEFT; ++i) {
-          const int idx = part * LEFT + i, g = idx / NC, x = idx % NC;
-          if (t0 + g < nt && col0 + x < dv) o_raw[((size_t)sq.row0 + c * CH + t0 + g) * (size_t)(H * dv) + h * dv + col0 + x] = v[i];
-        }
-      } else {
-#pragma unroll
-        for (int g = 0; g < TG; ++g)
-#pragma unroll
-          for (int x = 0; x < NC; ++x) {
-#pragma unroll
-            for (int o = P / 2; o > 0; o >>= 1) out[g][x] += __shfl_xor_sync(0xffffffffu, out[g][x], o);
-            if (part == (g * NC + x) % P && t0 + g < nt && col0 + x < dv)
-              o_raw[((size_t)sq.row0 + c * CH + t0 + g) * (size_t)(H * dv) + h * dv + col0 + x] = out[g][x];
-          }
+      for (int i = 0; i < LEFT; ++i) {
+        const int idx = part / SAME * LEFT + i, g = idx / NC, x = idx % NC;
+        if (part % SAME == 0 && t0 + g < nt && col0 + x < dv) o_raw[((size_t)sq.row0 + c * CH + t0 + g) * (size_t)(H * dv) + h * dv + col0 + x] = v[i];
       }
     }
     __syncthreads();                                 // the buffer is refilled two chunks later
