@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libxotb200.so"
@@ -35,10 +36,13 @@ class XotB200Error(RuntimeError):
 
 
 _lib = None
+_pools, _pools_lock = {}, threading.Lock()      # one per loaded library (libraries stay loaded)
 
 _SIGS = {
   "xotb200_last_error": (C.c_char_p, []),
   "xotb200_version": (C.c_char_p, []),
+  "xotb200_host_alloc": (C.c_int, [C.c_int64, C.POINTER(C.c_void_p)]),
+  "xotb200_host_free": (C.c_int, [C.c_void_p]),
   "xotb200_create": (C.c_int, [C.POINTER(ModelCfg), C.c_int, C.POINTER(C.c_void_p)]),
   "xotb200_destroy": (C.c_int, [C.c_void_p]),
   "xotb200_set_shard": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
@@ -148,6 +152,8 @@ _I32P = C.POINTER(C.c_int32)
 _LM_SIGS = {
   "xotb200_lm_last_error": (C.c_char_p, []),
   "xotb200_lm_version": (C.c_char_p, []),
+  "xotb200_lm_host_alloc": (C.c_int, [C.c_int64, C.POINTER(C.c_void_p)]),
+  "xotb200_lm_host_free": (C.c_int, [C.c_void_p]),
   "xotb200_lm_create": (C.c_int, [C.POINTER(LmCfg), C.POINTER(LmLayer), C.c_int, C.POINTER(C.c_void_p)]),
   "xotb200_lm_destroy": (C.c_int, [C.c_void_p]),
   "xotb200_lm_load_dir": (C.c_int, [C.c_void_p, C.c_char_p]),
@@ -204,6 +210,16 @@ def load_lm(path: os.PathLike | None = None, build: bool = True) -> C.CDLL:
   if path is None:
     _lm_lib = lib
   return lib
+
+
+def results(lib, prefix: str) -> "ResultPool":
+  """the process's pool of page-locked result arrays of a loaded library"""
+  pool = _pools.get(id(lib))
+  if pool is None:
+    from .pinned import library_pool
+    with _pools_lock:
+      pool = _pools.setdefault(id(lib), library_pool(lib, prefix))
+  return pool
 
 
 def check_lm(rc: int) -> int:

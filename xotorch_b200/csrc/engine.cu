@@ -927,6 +927,16 @@ extern "C" {
 const char* xotb200_last_error(void) { return g_err; }
 const char* xotb200_version(void) { return "xotb200 0.1.0 sm_100a"; }
 
+int xotb200_host_alloc(int64_t bytes, void** out) {
+  REQUIRE(bytes > 0 && out, "bad argument");
+  CK(cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable));
+  return 0;
+}
+int xotb200_host_free(void* p) {
+  if (p) CK(cudaFreeHost(p));
+  return 0;
+}
+
 int xotb200_create(const xotb200_model_cfg* cfg, int device, xotb200_engine** out) {
   REQUIRE(cfg && out, "null argument");
   REQUIRE(cfg->dtype == XOTB200_DTYPE_BF16 || cfg->dtype == XOTB200_DTYPE_F16, "dtype must be bf16 (0) or f16 (1), got %d", cfg->dtype);

@@ -2008,6 +2008,16 @@ extern "C" {
 const char* xotb200_lm_last_error(void) { return g_err; }
 const char* xotb200_lm_version(void) { return "xotb200_lm 0.1.0 sm_100a"; }
 
+int xotb200_lm_host_alloc(int64_t bytes, void** out) {
+  REQUIRE(bytes > 0 && out, "bad argument");
+  CK(cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable));
+  return 0;
+}
+int xotb200_lm_host_free(void* p) {
+  if (p) CK(cudaFreeHost(p));
+  return 0;
+}
+
 int xotb200_lm_create(const xotb200_lm_cfg* cfg, const xotb200_lm_layer* layers, int device, xotb200_lm** out) {
   REQUIRE(cfg && layers && out, "null argument");
   REQUIRE(cfg->dtype == XOTB200_LM_DTYPE_BF16 || cfg->dtype == XOTB200_LM_DTYPE_F32, "dtype must be bf16 (0) or f32 (2), got %d", cfg->dtype);
@@ -2523,6 +2533,13 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   }
   memcpy(e->h_stage, st.data(), off * 4);
   const bool results = e->last && n_want > 0;
+  // page-locked output memory takes the results directly
+  bool direct = false;
+  if (float* dst = e->last ? logits_f32 : hidden_out_f32) {
+    cudaPointerAttributes at;
+    direct = (results || !e->last) && cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    cudaGetLastError();                                  // a pointer the runtime cannot classify is ordinary memory
+  }
   if (results) TRY(ensure_host_out(e, (size_t)n_want * V + n_want + 1));
   else if (!e->last) TRY(ensure_host_out(e, (size_t)M * (D + e->carry_out)));
   // Decoding — every request brings one row — has the same launches step after step: only the contents of the index arrays and
@@ -2590,13 +2607,11 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
         if (e->carry_in) TRY(copy_rows(e->vfirst, e->carry_in, hidden_f32 + D, ld, e->carry_in, cudaMemcpyHostToDevice));
       }
       TRY(e->esz == 2 ? run_layers<bf16>(e, sp, n_want) : run_layers<float>(e, sp, n_want));
-      if (results) {
-        const size_t skip = logits_f32 ? 0 : (size_t)n_want * V;   // one copy: the logits when they are asked for, argmax, error word
-        CK(cudaMemcpyAsync(e->h_out + skip, e->logits + skip, ((size_t)n_want * V + n_want + 1 - skip) * 4, cudaMemcpyDeviceToHost, e->stream));
-      } else if (!e->last) {
+      if (!e->last) {
         const size_t ld = (size_t)D + e->carry_out;
-        TRY(copy_rows(e->h_out, ld, e->x, D, D, cudaMemcpyDeviceToHost));
-        if (e->carry_out) TRY(copy_rows(e->h_out + D, ld, e->vfirst, e->carry_out, e->carry_out, cudaMemcpyDeviceToHost));
+        float* dst = direct ? hidden_out_f32 : e->h_out;
+        TRY(copy_rows(dst, ld, e->x, D, D, cudaMemcpyDeviceToHost));
+        if (e->carry_out) TRY(copy_rows(dst + D, ld, e->vfirst, e->carry_out, e->carry_out, cudaMemcpyDeviceToHost));
       }
       if (!results) CK(cudaMemcpyAsync(e->h_err, e->d_err, 4, cudaMemcpyDeviceToHost, e->stream));
       return 0;
@@ -2618,6 +2633,14 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     }
     if (rc < 0) { cudaStreamSynchronize(e->stream); return rc; }
   }
+  if (results) {
+    // behind the (replayed) kernels, not part of a captured step: the caller's pointer is another one each time.  The argmax and the error word lie behind
+    // the logits; one copy when the logits go through the staging buffer or are not asked for.
+    const size_t n = (size_t)n_want * V;
+    if (direct) CK(cudaMemcpyAsync(logits_f32, e->logits, n * 4, cudaMemcpyDeviceToHost, e->stream));
+    const size_t skip = direct || !logits_f32 ? n : 0;
+    CK(cudaMemcpyAsync(e->h_out + skip, e->logits + skip, (n + n_want + 1 - skip) * 4, cudaMemcpyDeviceToHost, e->stream));
+  }
   CK(cudaEventRecord(e->ev1, e->stream));
   CK(cudaStreamSynchronize(e->stream));
   CK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
@@ -2627,9 +2650,9 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     return XOTB200_ECUDA;
   }
   if (results) {
-    if (logits_f32) memcpy(logits_f32, e->h_out, (size_t)n_want * V * 4);
+    if (logits_f32 && !direct) memcpy(logits_f32, e->h_out, (size_t)n_want * V * 4);
     if (argmax_i32) memcpy(argmax_i32, e->h_out + (size_t)n_want * V, (size_t)n_want * 4);
-  } else if (!e->last) {
+  } else if (!e->last && !direct) {
     memcpy(hidden_out_f32, e->h_out, (size_t)M * (D + e->carry_out) * 4);
   }
   return 0;

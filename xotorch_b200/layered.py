@@ -453,6 +453,7 @@ class LayeredShard:
     if dtype not in ("bfloat16", "float32"):
       raise ValueError(f"dtype {dtype!r}: the layered engine serves in bfloat16 and has an all-float32 mode")
     self.lib = _lib.load_lm()
+    self.results = _lib.results(self.lib, "xotb200_lm")
     self.config, self.family, self.device, self.dtype = dict(config), fam, int(device), dtype
     self.globals = LAYERED_FAMILIES[fam][1](config)
     self.n_layers = len(config["layers"])
@@ -584,10 +585,10 @@ class LayeredShard:
     wn = np.ascontiguousarray(want, dtype=np.int32).reshape(-1)
     lg = am = ho = None
     if self.is_last:
-      lg = np.empty((wn.size, self.vocab), dtype=np.float32) if logits else None
+      lg = self.results.empty((wn.size, self.vocab)) if logits else None
       am = np.empty(wn.size, dtype=np.int32) if argmax else None
     else:
-      ho = np.empty((M, self.hidden_out), dtype=np.float32)
+      ho = self.results.empty((M, self.hidden_out))
     p = lambda a: a.ctypes.data_as(C.c_void_p) if a is not None else None
     check_lm(self.lib.xotb200_lm_step(self.h, n_seq, p(sl), p(counts), tok_p, hid_p, p(wn), int(wn.size) if self.is_last else 0, p(lg), p(am), p(ho)))
     if self.is_last:

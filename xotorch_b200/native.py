@@ -71,6 +71,7 @@ def cfg_from_hf(hf: dict) -> ModelCfg:
 class NativeShard:
   def __init__(self, hf_config: dict, device: int = 0):
     self.lib = _lib.load()
+    self.results = _lib.results(self.lib, "xotb200")
     self.hf_config = dict(hf_config)
     self.cfg = cfg_from_hf(hf_config)
     self.device = device
@@ -140,10 +141,7 @@ class NativeShard:
       tok_p, hid_p = None, hid.ctypes.data_as(C.c_void_p)
     else:
       raise ValueError(f"input_data.ndim must be 2 (token ids) or 3 (hidden state), got {input_data.ndim}")
-    if self.is_last:
-      out = np.empty((1, self.cfg.vocab), dtype=np.float32)
-    else:
-      out = np.empty((1, n, self.cfg.dim), dtype=np.float32)
+    out = self.results.empty((1, self.cfg.vocab) if self.is_last else (1, n, self.cfg.dim))
     check(self.lib.xotb200_forward(self.h, tok_p, hid_p, n, int(pos0), out.ctypes.data_as(C.c_void_p)))
     return out
 
@@ -156,7 +154,7 @@ class NativeShard:
     if ids is not None:
       ids = np.ascontiguousarray(ids, dtype=np.int32)
       tok_p = ids.ctypes.data_as(C.c_void_p)
-    logits = np.empty((1, self.cfg.vocab), dtype=np.float32) if self.is_last else None
+    logits = self.results.empty((1, self.cfg.vocab)) if self.is_last else None
     check(self.lib.xotb200_forward_device(self.h, tok_p, C.c_void_p(hidden_dev_ptr) if hidden_dev_ptr else None, int(n_tokens),
                                           int(pos0), C.c_void_p(out_dev_ptr) if out_dev_ptr else None,
                                           logits.ctypes.data_as(C.c_void_p) if logits is not None else None))
@@ -170,7 +168,7 @@ class NativeShard:
     if ids is not None:
       ids = np.ascontiguousarray(ids, dtype=np.int32)
       tok_p = ids.ctypes.data_as(C.c_void_p)
-    logits = np.empty((1, self.cfg.vocab), dtype=np.float32) if self.is_last else None
+    logits = self.results.empty((1, self.cfg.vocab)) if self.is_last else None
     seq_out = C.c_int64(-1)
     check(self.lib.xotb200_forward_hop(self.h, tok_p, C.c_int64(int(seq_in)), int(n_tokens), int(pos0), C.byref(seq_out),
                                        logits.ctypes.data_as(C.c_void_p) if logits is not None else None))
