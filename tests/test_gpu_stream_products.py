@@ -1,5 +1,5 @@
 """Products with few rows on the tensor cores (the streaming form of the layered engine's products): edges of its row tiles (16, 32,
-64, 128 rows), column and K remainders, K cut over clusters of up to eight CTAs (the last of them without a block of its own), experts' row
+64, 128, 256 rows), column and K remainders, K cut over clusters of up to eight CTAs (the last of them without a block of its own), experts' row
 tiles — against the float64 oracles, with the error bound of the other 16-bit tests."""
 import pytest
 
@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 from tests import bufulorn_oracle as bo, zokuvik_oracle as zo
 from tests import bufulorn_util as bu, layered_util as lu
 
-ROWS = [3, 15, 16, 17, 32, 33, 64, 65, 127, 128, 129]
+ROWS = [3, 15, 16, 17, 32, 33, 64, 65, 127, 128, 129, 255, 256, 257]
 
 
 @pytest.mark.parametrize("rows", ROWS)
@@ -18,7 +18,7 @@ def test_dense_products_match_oracle(rows):
                   width=200, vocab=331, groups=4)
   w = zo.random_weights(cfg, 11)
   toks = lu.rand_tokens(331, rows, rows)
-  eng = lu.make_engine(cfg, w, "bfloat16", max_tokens=256)
+  eng = lu.make_engine(cfg, w, "bfloat16", max_tokens=264)
   before = eng.tensor_core_launches()
   got = lu.run_cut(eng, 0, toks, [rows])
   assert eng.tensor_core_launches() - before >= 11
@@ -37,7 +37,7 @@ def test_expert_products_match_oracle(rows):
                    bu.delta(heads=4, kv_heads=2, dim=16, vdim=24, mlp=bu.moe(experts=5, top=2, groups=None, ff=520))], width=136, vocab=150)
   w = bo.random_weights(cfg, 5)
   toks = lu.rand_tokens(150, rows, rows + 1)
-  eng = lu.make_engine(cfg, w, "bfloat16", max_tokens=256)
+  eng = lu.make_engine(cfg, w, "bfloat16", max_tokens=264)
   got = lu.run_cut(eng, 0, toks, [rows])
   eng.set_gemm_mode(1)
   eng.clear_request(0)

@@ -464,7 +464,9 @@ static int launch_early(xotb200_engine* e, cudaStream_t st, void (*fn)(KA...), d
 }
 
 // GEMM of one tile of token rows (a.S <= 128; HEAD_LAST: one row) as a weight stream: tc_stream_kernel.  K is cut over 1, 2, 4 or 8 CTAs, doubled
-// while two CTAs per SM are not exceeded and each keeps two K blocks or more.
+// while two CTAs per SM (with 128 rows, whose partial tiles are 64 KB: one) are not exceeded and each keeps two K blocks or more.  Measured on an 8B layer
+// (16 / 128 rows; 128 x 64..128 token tiles with split-K through a workspace took 36.5 us for O and down on average, 30.6 for QKV, 54.9 for
+// gate/up at 128 rows): O and down 18.3 / 28.7 us, QKV 14.5 / 23.6, gate/up 41.4 (5.7 TB/s) / 47.9.
 template <int NB>
 static int launch_tc_stream_nb(xotb200_engine* e, const CUtensorMap& tmW, const CUtensorMap& tmX, const TcGemmArgs& a, int epi, int splits, cudaStream_t st) {
   void (*fn)(CUtensorMap, CUtensorMap, TcGemmArgs) = nullptr;
@@ -484,7 +486,7 @@ static int launch_tc_stream(xotb200_engine* e, const CUtensorMap& tmW, const Act
   a.err = &e->ctl->err;
   const int nb = epi == TCE_HEAD_LAST || a.S <= 16 ? 16 : a.S <= 32 ? 32 : a.S <= 64 ? 64 : 128, tiles = a.N / TC_M, nkb = a.K / TC_BK;
   int s = 1;
-  while (s < 8 && tiles * s * 2 <= 2 * e->sm_count && nkb >= 4 * s) s *= 2;
+  while (s < 8 && tiles * s * 2 <= (nb >= 128 ? 1 : 2) * e->sm_count && nkb >= 4 * s) s *= 2;
   return nb == 16 ? launch_tc_stream_nb<16>(e, tmW, x.r16, a, epi, s, st) : nb == 32 ? launch_tc_stream_nb<32>(e, tmW, x.r32, a, epi, s, st)
        : nb == 64 ? launch_tc_stream_nb<64>(e, tmW, x.r64, a, epi, s, st) : launch_tc_stream_nb<128>(e, tmW, x.full, a, epi, s, st);
 }
@@ -705,8 +707,10 @@ static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, i
 
 // Prefill n_tokens positions starting at pos0 on the tensor cores, in chunks of up to TC_CHUNK tokens (layer-major
 // inside a chunk, so a chunk streams the shard's weights once).  Inputs: stage_tokens /
-// stage_in; outputs: stage_out (non-last shard) or logits + ctl->token of the last position (last shard).
-static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st) {
+// stage_in or `in` (device memory); outputs: stage_out or `out` (non-last shard) or logits + ctl->token of the last position (last shard).
+static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st, const void* in = nullptr, void* out = nullptr) {
+  const bf16* hidden_in = in ? static_cast<const bf16*>(in) : e->stage_in;
+  bf16* hidden_out = out ? static_cast<bf16*>(out) : e->stage_out;
   if (int rc = prepare_tc(e, n_tokens)) return rc;
   const xotb200_model_cfg& c = e->cfg;
   const int D = c.dim, F = c.ffn, Hq = c.n_heads, Hkv = c.n_kv_heads, hd = c.head_dim;
@@ -717,7 +721,7 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
     if (e->first) {
       if (int rc = launch_early(e, st, tc_gather_kernel, S, 128, 0, 1, e->stage_tokens + m0, e->embed, e->tc_x, D)) return rc;
     } else {
-      CK(cudaMemcpyAsync(e->tc_x, e->stage_in + (size_t)m0 * D, (size_t)S * D * 2, cudaMemcpyDeviceToDevice, st));
+      CK(cudaMemcpyAsync(e->tc_x, hidden_in + (size_t)m0 * D, (size_t)S * D * 2, cudaMemcpyDeviceToDevice, st));
     }
     for (int li = 0; li < nl; ++li) {
       const LayerW& w = e->layers[li];
@@ -788,7 +792,7 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
         if (int rc = launch_early(e, st, tc_argmax_kernel, 1, 1024, 0, 1, e->logits, c.vocab, e->ctl)) return rc;
       }
     } else {
-      CK(cudaMemcpyAsync(e->stage_out + (size_t)m0 * D, e->tc_x, (size_t)S * D * 2, cudaMemcpyDeviceToDevice, st));
+      CK(cudaMemcpyAsync(hidden_out + (size_t)m0 * D, e->tc_x, (size_t)S * D * 2, cudaMemcpyDeviceToDevice, st));
     }
   }
   // the residual stream of the last position is what xotb200_post_to_next hands to the next shard
@@ -1433,17 +1437,16 @@ int xotb200_forward_device(xotb200_engine* e, const int32_t* tokens, const void*
     for (int i = 0; i < n_tokens; ++i)
       REQUIRE(tokens[i] >= 0 && tokens[i] < e->cfg.vocab, "token id %d out of range", tokens[i]);
     CK(cudaMemcpyAsync(e->stage_tokens, tokens, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, st));
-  } else {
-    CK(cudaMemcpyAsync(e->stage_in, hidden_dev, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
   }
   const bool use_tc = runs_as_gemms(e, n_tokens);
-  if (use_tc) {
-    if (int rc = prefill_tc(e, n_tokens, pos0, st)) return rc;
+  if (use_tc) {   // the caller's buffers are read and written in place, no copy through the staging buffers
+    if (int rc = prefill_tc(e, n_tokens, pos0, st, hidden_dev, e->last ? nullptr : out_hidden_dev)) return rc;
   } else {
+    if (!tokens) CK(cudaMemcpyAsync(e->stage_in, hidden_dev, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
     if (int rc = launch_mega(e, 1, n_tokens, 0, pos0, st)) return rc;
   }
   if (e->last) CK(cudaMemcpyAsync(logits_f32, e->logits, (size_t)e->cfg.vocab * 4, cudaMemcpyDeviceToHost, st));
-  else CK(cudaMemcpyAsync(out_hidden_dev, e->stage_out, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
+  else if (!use_tc) CK(cudaMemcpyAsync(out_hidden_dev, e->stage_out, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
   CK(cudaStreamSynchronize(st));
   e->have_result = true;
   return 0;

@@ -69,6 +69,11 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
@@ -252,17 +257,19 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
       for (int c = 0; c < 64; ++c) s[c] = __uint_as_float(raw[c >> 5][c & 31]);
       const int j0 = jstart + j * FT_K;
-      if (a.cap > 0.f) {                             // cap tanh(x / cap) with tanh y = 1 - 2 / (e^2y + 1)
+      if (a.cap > 0.f) {                             // cap tanh(x / cap) with tanh y = 1 - 2 / (e^2y + 1): right at both ends too (e^2y = inf, 0)
 #pragma unroll
-        for (int c = 0; c < 64; ++c) {
-          const float t = ex2(fminf(fmaxf(s[c] * inv_cap2, -43.3f), 43.3f));
-          s[c] = cap2 * __fdividef(t - 1.0f, t + 1.0f);
-        }
+        for (int c = 0; c < 64; ++c) s[c] = fmaf(-2.0f * cap2, rcp(ex2(s[c] * inv_cap2) + 1.0f), cap2);
       } else {
 #pragma unroll
         for (int c = 0; c < 64; ++c) s[c] *= scale2;
       }
-      if (dist) {
+      const bool all = j0 + FT_K - 1 <= tl.pos0 && j0 >= lo_last;   // every row of the tile sees every key of it
+      if (dist && all && pos - j0 < a.dist_n) {              // no distance outside the table: one address for the tile
+        const float* dp = dist + (pos - j0);
+#pragma unroll
+        for (int c = 0; c < 64; ++c) s[c] = fmaf(-LOG2E, __ldg(dp - c), s[c]);
+      } else if (dist) {
 #pragma unroll
         for (int c = 0; c < 64; ++c) s[c] = fmaf(-LOG2E, __ldg(dist + min(max(pos - j0 - c, 0), a.dist_n - 1)), s[c]);
       }
@@ -270,7 +277,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
         for (int c = 0; c < 64; ++c) s[c] = fmaf(LOG2E, __ldg(rel + min(max(pos - j0 - c, 0), a.rel_n - 1)), s[c]);
       }
-      if (j0 + FT_K - 1 > tl.pos0 || j0 < lo_last) { // some row of the tile does not see all keys
+      if (!all) {
         const int clo = lo - j0, chi = pos - j0;
 #pragma unroll
         for (int c = 0; c < 64; ++c) s[c] = c >= clo && c <= chi ? s[c] : -INFINITY;
@@ -341,8 +348,15 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * f;
           if (a.gate_mode == 2) {
+            const bool vec = ((reinterpret_cast<uintptr_t>(gt) | (uintptr_t)c) & 15) == 0;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] *= 1.0f / (1.0f + expf(-gt[c + i]));
+            for (int i = 0; i < 32; i += 4) {
+              const float4 z = vec ? *reinterpret_cast<const float4*>(gt + c + i) : make_float4(gt[c + i], gt[c + i + 1], gt[c + i + 2], gt[c + i + 3]);
+              v[i] *= 1.0f / (1.0f + expf(-z.x));
+              v[i + 1] *= 1.0f / (1.0f + expf(-z.y));
+              v[i + 2] *= 1.0f / (1.0f + expf(-z.z));
+              v[i + 3] *= 1.0f / (1.0f + expf(-z.w));
+            }
           }
 #pragma unroll
           for (int i = 0; i < 32; i += 8)

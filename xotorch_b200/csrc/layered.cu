@@ -789,13 +789,13 @@ static int launch_ltc(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& m
   return 0;
 }
 
-// CTAs that share a column tile of a product with few rows by cutting K: doubled while two CTAs per SM are not exceeded and every CTA
+// CTAs that share a column tile of a product with few rows by cutting K: doubled while two CTAs per SM (256 rows: one) are not exceeded and every CTA
 // keeps two K blocks or more (a CTA with less spends its time on the barriers)
-static int stream_splits(const xotb200_lm* e, int N, int K, int z) {
+static int stream_splits(const xotb200_lm* e, int N, int K, int z, int nb) {
   const long tiles = (long)cdiv(N, LTC_M) * z;
   const int nkb = cdiv(K, LTC_BK);
   int s = 1;
-  while (s < 8 && tiles * s * 2 <= 2L * e->sm_count && nkb >= 4 * s) s *= 2;
+  while (s < 8 && tiles * s * 2 <= lst_ctas_per_sm(nb) * (long)e->sm_count && nkb >= 4 * s) s *= 2;
   return s;
 }
 
@@ -809,7 +809,7 @@ static int launch_stream(xotb200_lm* e, const CUtensorMap& mw, const CUtensorMap
 }
 
 // rows of a row tile that holds M rows (M <= LST_MAX_ROWS)
-static int stream_tile_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128; }
+static int stream_tile_rows(int M) { return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256; }
 
 // 1 = launched, 0 = the operands cannot be described to TMA.  Not NULL `tile_batch`: `batch` row tiles of stream_tile_rows(M) rows of A and C,
 // each with the B matrix its entry names.
@@ -821,11 +821,12 @@ static int product_stream(xotb200_lm* e, const bf16* A, long lda, long a_batch, 
   if (!make_map3(&mw, B, N, K, ldb, b_batch, b_count, LTC_M)) return 0;
   if (!(tile_batch ? make_map3(&mx, A, (long)batch * nb, K, lda, 0, 1, nb) : make_map3(&mx, A, M, K, lda, a_batch, batch, nb))) return 0;
   const LtcArgs a{M, N, K, C, ldc, c_batch, e->d_err, epi, tile_batch, 0};
-  const int s = stream_splits(e, N, K, batch);
+  const int s = stream_splits(e, N, K, tile_batch ? std::min(batch, b_count) : batch, nb);
   if (nb == 16) TRY((launch_stream<16, EPI, TC>(e, mw, mx, a, s, batch)));
   else if (nb == 32) TRY((launch_stream<32, EPI, TC>(e, mw, mx, a, s, batch)));
   else if (nb == 64) TRY((launch_stream<64, EPI, TC>(e, mw, mx, a, s, batch)));
-  else TRY((launch_stream<128, EPI, TC>(e, mw, mx, a, s, batch)));
+  else if (nb == 128) TRY((launch_stream<128, EPI, TC>(e, mw, mx, a, s, batch)));
+  else TRY((launch_stream<256, EPI, TC>(e, mw, mx, a, s, batch)));
   return 1;
 }
 
@@ -1100,7 +1101,7 @@ template <int DKC, int DVC>
 static int launch_flash_tc(xotb200_lm* e, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mk2, const CUtensorMap& mv, const xf::FlashArgs& a, int n_tiles) {
   auto kern = xf::flash_tc_kernel<DKC, DVC, true, false>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, xf::ft_smem_bytes(DKC, DVC)));
-  TRY(launch_late(e, kern, dim3(n_tiles, a.H), xf::FT_THREADS, xf::ft_smem_bytes(DKC, DVC), mq, mk, mk2, mv, a));
+  TRY(launch_early(e, kern, dim3(n_tiles, a.H), xf::FT_THREADS, xf::ft_smem_bytes(DKC, DVC), 1, mq, mk, mk2, mv, a));
   e->flash_launches++;
   return 0;
 }
@@ -1229,7 +1230,7 @@ template <int KPT, int P, int NC>
 static int launch_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks, DeltaSrc rs, DeltaSrc vs, int dk, int dv, DeltaForm form) {
   const xotb200_lm_layer& s = L.s;
   constexpr int CPW = (32 / P) * NC;
-  const int warps = std::max(1, std::min(4, cdiv(dv, CPW)));
+  const int warps = std::max(1, std::min(P == 32 ? 8 : 4, cdiv(dv, CPW)));
   const dim3 grid(sp.n_seq * s.heads, cdiv(dv, warps * CPW));
   const int HD = s.heads * dk;
   const int vec4 = (dk % 4 == 0 && dv % 4 == 0 && HD % 4 == 0 && (ks.ld | ks.col | rs.ld | rs.col | vs.ld | vs.col) % 4 == 0) ? 1 : 0;
@@ -1247,7 +1248,8 @@ static int run_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks,
     return 4L * sp.n_seq * L.s.heads * cdiv(dv, warps * cpw) >= 3L * e->sm_count;
   };
   // a prompt of one request: with the P = 8 variants a scheduler has one warp, which waits four cycles of five; sixteen lanes per column make
-  // it two warps of half the work each
+  // it two warps of half the work each.  Heads of 128: all lanes along the key rows, four columns a thread — a shared-memory load then brings 128
+  // different entries instead of 32 four times over, and loading the five vectors no longer takes half of a token's time.
   auto busy = [&](int P, int NC) { return (long)sp.n_seq * L.s.heads * cdiv(dv, 4 * (32 / P) * NC) > e->sm_count; };
   if (d <= 16) return launch_delta<4, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, form);
   if (d <= 32) return fills(4, 2) ? launch_delta<8, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, form) : launch_delta<8, 4, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
@@ -1255,7 +1257,7 @@ static int run_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks,
     return fills(8, 4) ? launch_delta<8, 8, 4>(e, L, sp, ks, rs, vs, dk, dv, form)
          : fills(8, 2) ? launch_delta<8, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form)
                        : launch_delta<4, 16, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
-  if (d <= 128 && !busy(8, 2)) return launch_delta<8, 16, 2>(e, L, sp, ks, rs, vs, dk, dv, form);
+  if (d <= 128 && !busy(8, 2)) return launch_delta<4, 32, 4>(e, L, sp, ks, rs, vs, dk, dv, form);
   if (d <= 128) return fills(8, 2) ? launch_delta<16, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form) : launch_delta<16, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
   return launch_delta<32, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
 }
@@ -1520,7 +1522,7 @@ static int mamba2_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
 template <int EPI, typename TC>
 static int grouped_product(xotb200_lm* e, const bf16* A, long lda, const bf16* B, long ldb, long b_batch, int n_batch, TC* C, long ldc, int M, int m_pad, int N,
                            int K, const int* tile_batch, const EpiArgs& epi = EpiArgs{}) {
-  if (M <= LST_MAX_ROWS)
+  if (M <= LST_EXPERT_ROWS)
     return product_stream<TC, EPI>(e, A, lda, 0, B, ldb, b_batch, n_batch, C, ldc, 0, M, N, K, m_pad / stream_tile_rows(M), epi, tile_batch);
   const int nt = N > 64 ? 128 : 64;
   CUtensorMap ma, mb;
@@ -1580,15 +1582,19 @@ static int feed_forward(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
     if constexpr (std::is_same<T, bf16>::value) {
       if (grouped_ok) {
         // few rows: an expert has at most M of them (a row picks an expert once), one row tile each, and the products stream the chosen experts
-        const int tile_rows = M <= LST_MAX_ROWS ? stream_tile_rows(M) : LTC_M;
-        const int pairs = M * top, tiles = M <= LST_MAX_ROWS ? std::min(E, pairs) : cdiv(pairs, LTC_M) + E, m_pad = tiles * tile_rows;
+        const int tile_rows = M <= LST_EXPERT_ROWS ? stream_tile_rows(M) : LTC_M;
+        const int pairs = M * top, tiles = M <= LST_EXPERT_ROWS ? std::min(E, pairs) : cdiv(pairs, LTC_M) + E, m_pad = tiles * tile_rows;
         REQUIRE(tiles <= e->moe_tiles_cap, "internal: the expert tile list was not sized for this step");
         int *counts = e->moe_plan, *starts = counts + e->max_experts, *cursor = starts + e->max_experts + 1, *place = cursor + e->max_experts,
             *tile_expert = place + (size_t)e->m_cap * e->max_top;
         bf16* xg = static_cast<bf16*>(e->moe_xg);
+        const bool few = M <= LST_EXPERT_ROWS && pairs <= MOE_FEW_PAIRS && E <= MOE_FEW_EXPERTS;
+        if (few) TRY(launch_early(e, moe_place_few_kernel<bf16>, cdiv(pairs, 8), 256, (size_t)(pairs + E) * 4, 1, h, D, e->moe_ids, pairs, top, E, tile_rows, tiles, place, tile_expert, xg));
+        else {
         TRY(launch_early(e, moe_count_kernel, cdiv(pairs, 256), 256, 0, 1, e->moe_ids, pairs, counts));
         TRY(launch_early(e, moe_plan_kernel, 1, 256, 0, 1, counts, E, tile_rows, tiles, starts, cursor, tile_expert));
         TRY(launch_early(e, moe_scatter_kernel<bf16>, cdiv(pairs, 8), 256, 0, 1, h, D, e->moe_ids, pairs, top, starts, cursor, place, xg));
+        }
         bf16* ma = static_cast<bf16*>(e->mact);
         int r = s.expert_act == XOTB200_LM_EXPERT_CLAMPED_GLU
                     ? grouped_product<EPI_CLAMPED_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, M, m_pad, 2 * F, D, tile_expert, glu)

@@ -876,6 +876,55 @@ __global__ void moe_scatter_kernel(const T* __restrict__ h, int D, const int* __
     for (int d = lane; d < D; d += 32) dst[d] = src[d];
   }
 }
+// The same three steps in one launch for few rows, where an expert has one tile of `tile_rows` >= rows (a row picks an expert once): every block
+// counts all pairs in shared memory for itself (a few hundred numbers), so places need no order between blocks, and come out in the order of the
+// pairs.  Block 0 writes the tile -> expert map.  One warp per pair.  Dynamic shared memory: n_pairs + E ints.
+constexpr int MOE_FEW_PAIRS = 2048, MOE_FEW_EXPERTS = 1024;
+template <typename T>
+__global__ void __launch_bounds__(256) moe_place_few_kernel(const T* __restrict__ h, int D, const int* __restrict__ ids, int n_pairs, int top, int E, int tile_rows, int n_tiles,
+                                                            int* __restrict__ place, int* __restrict__ tile_expert, T* __restrict__ xg) {
+  pdl_enter();
+  extern __shared__ int few_sm[];
+  int *sid = few_sm, *tile = few_sm + n_pairs;                 // the pairs' experts; per expert: used or not, then its tile
+  for (int e = threadIdx.x; e < E; e += blockDim.x) tile[e] = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_pairs; i += blockDim.x) {
+    const int e = ids[i];
+    sid[i] = e;
+    tile[e] = 1;
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == 0) {                                             // running number of the experts in use
+    int at = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane;
+      const unsigned used = __ballot_sync(0xffffffffu, e < E && tile[e]);
+      if (e < E) {
+        const int t = at + __popc(used & ((1u << lane) - 1u));
+        if (blockIdx.x == 0 && (used >> lane & 1u)) tile_expert[t] = e;
+        tile[e] = t;
+      }
+      at += __popc(used);
+    }
+    if (blockIdx.x == 0)
+      for (int t = at + lane; t < n_tiles; t += 32) tile_expert[t] = -1;
+  }
+  __syncthreads();
+  const int i = blockIdx.x * (blockDim.x >> 5) + warp;
+  if (i >= n_pairs) return;
+  const int e = sid[i];
+  int rank = 0;
+  for (int j = lane; j < i; j += 32) rank += sid[j] == e ? 1 : 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+  const int p = tile[e] * tile_rows + rank;
+  if (lane == 0) place[i] = p;
+  const T* src = h + (size_t)(i / top) * D;
+  T* dst = xg + (size_t)p * D;
+  constexpr int VEC = 16 / sizeof(T);                          // D is a multiple of 8 here
+  for (int d = lane * VEC; d < D; d += 32 * VEC) *reinterpret_cast<uint4*>(dst + d) = *reinterpret_cast<const uint4*>(src + d);
+}
 template <typename T>
 __global__ void moe_combine_kernel(const float* __restrict__ yg, const int* __restrict__ place, const float* __restrict__ wts, int top, int D,
                                    int accumulate, float* __restrict__ y, const EpiArgs close) {

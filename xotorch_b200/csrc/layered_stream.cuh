@@ -23,14 +23,15 @@
 
 namespace xl {
 
-constexpr int LST_THREADS = 256, LST_MAX_ROWS = 128;
+constexpr int LST_THREADS = 256, LST_MAX_ROWS = 256, LST_EXPERT_ROWS = 128;   // rows of a product; rows up to which experts have one row tile each
 
 // ring stages that let two CTAs share an SM (its 227 KB): the weights in flight per SM are then 2 * stages * 16 KB
 __host__ __device__ constexpr int lst_stage_bytes(int nb) { return LTC_M * LTC_BK * 2 + nb * LTC_BK * 2; }
-__host__ __device__ constexpr int lst_stages(int nb) { return nb <= 16 ? 6 : nb <= 32 ? 5 : nb <= 64 ? 4 : 3; }
+__host__ __device__ constexpr int lst_stages(int nb) { return nb <= 16 ? 6 : nb <= 32 ? 5 : nb <= 64 ? 4 : nb <= 128 ? 3 : 4; }
+__host__ __device__ constexpr int lst_ctas_per_sm(int nb) { return nb <= 128 ? 2 : 1; }   // 256 rows: half of a stage is rows, one CTA per SM with a deeper ring
 __host__ __device__ constexpr int lst_smem_bytes(int nb) { return lst_stages(nb) * lst_stage_bytes(nb) + 1024 + 256; }
 static_assert(lst_smem_bytes(128) <= 112 * 1024 && lst_smem_bytes(16) <= 112 * 1024 && lst_smem_bytes(32) <= 112 * 1024 && lst_smem_bytes(64) <= 112 * 1024, "two CTAs per SM");
-static_assert(LTC_M * 128 * 4 <= lst_stages(128) * lst_stage_bytes(128), "the partial tile reuses the ring");
+static_assert(LTC_M * 128 * 4 <= lst_stages(128) * lst_stage_bytes(128) && LTC_M * 256 * 4 <= lst_stages(256) * lst_stage_bytes(256), "the partial tile reuses the ring");
 
 // entry (m, n) of a float in the shared memory of CTA `rank` of the cluster
 __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr, uint32_t rank) {
@@ -40,7 +41,7 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t addr, uint32_t rank) {
 }
 
 template <int NB, int EPI, typename TC>
-__global__ void __launch_bounds__(LST_THREADS, 2)
+__global__ void __launch_bounds__(LST_THREADS, lst_ctas_per_sm(NB))
 stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const LtcArgs a) {
   extern __shared__ __align__(1024) uint8_t lst_smem[];
   constexpr int NS = lst_stages(NB), STAGE = lst_stage_bytes(NB), W_BYTES = LTC_M * LTC_BK * 2;
