@@ -541,7 +541,7 @@ static int launch_tc_gemm_2sm(xotb200_engine* e, const CUtensorMap& tmA, const C
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, tc2_smem_bytes(NT, NS))) return rc;
   const int total = ((a.S + 2 * TC_M - 1) / (2 * TC_M)) * (a.N / NT);
   const int pairs = std::max(1, std::min(total, e->sm_count / 2));
-  return launch_early(e, st, fn, 2 * pairs, TC_THREADS, tc2_smem_bytes(NT, NS), 0, tmA, tmB_half, a);
+  return launch_early(e, st, fn, 2 * pairs, TC2_THREADS, tc2_smem_bytes(NT, NS), 0, tmA, tmB_half, a);
 }
 
 static int launch_tc_gemm(xotb200_engine* e, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcGemmArgs& a_in, int epi, TcCfg c,

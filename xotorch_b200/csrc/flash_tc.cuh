@@ -137,7 +137,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  xb::pdl_enter();
+  xb::pdl_wait();
   if (base - ft_smem > 512) {                        // cannot be (the shared window starts on a 1 KB boundary); the sizes leave 512 bytes for it
     if (threadIdx.x == 0 && a.err) atomicExch(a.err, 4);
     return;
@@ -166,6 +166,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   xb::tc_fence_after();
   const uint32_t tmem = *tmem_slot, tm_o = tmem + 128;
+  xb::pdl_launch_dependents();   // not before: a later kernel's CTA that takes tensor memory and then waits for this kernel must not take it first
 
   if (warp == 0) {
     if (lane == 0) {

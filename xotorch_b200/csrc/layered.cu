@@ -1230,7 +1230,7 @@ template <int KPT, int P, int NC>
 static int launch_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks, DeltaSrc rs, DeltaSrc vs, int dk, int dv, DeltaForm form) {
   const xotb200_lm_layer& s = L.s;
   constexpr int CPW = (32 / P) * NC;
-  const int warps = std::max(1, std::min(P == 32 ? 8 : 4, cdiv(dv, CPW)));
+  const int warps = std::max(1, std::min(4, cdiv(dv, CPW)));
   const dim3 grid(sp.n_seq * s.heads, cdiv(dv, warps * CPW));
   const int HD = s.heads * dk;
   const int vec4 = (dk % 4 == 0 && dv % 4 == 0 && HD % 4 == 0 && (ks.ld | ks.col | rs.ld | rs.col | vs.ld | vs.col) % 4 == 0) ? 1 : 0;
@@ -1248,8 +1248,8 @@ static int run_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks,
     return 4L * sp.n_seq * L.s.heads * cdiv(dv, warps * cpw) >= 3L * e->sm_count;
   };
   // a prompt of one request: with the P = 8 variants a scheduler has one warp, which waits four cycles of five; sixteen lanes per column make
-  // it two warps of half the work each.  Heads of 128: all lanes along the key rows, four columns a thread — a shared-memory load then brings 128
-  // different entries instead of 32 four times over, and loading the five vectors no longer takes half of a token's time.
+  // it two warps of half the work each (1024 tokens, 32 heads of 128: 364 us a pass against 377; 3500 tokens, 32 heads of 64: 528 us against 800).
+  // All 32 lanes along the key rows and four columns a thread read less shared memory but cost 391 us there: the sums over lanes grow by a step.
   auto busy = [&](int P, int NC) { return (long)sp.n_seq * L.s.heads * cdiv(dv, 4 * (32 / P) * NC) > e->sm_count; };
   if (d <= 16) return launch_delta<4, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, form);
   if (d <= 32) return fills(4, 2) ? launch_delta<8, 4, 2>(e, L, sp, ks, rs, vs, dk, dv, form) : launch_delta<8, 4, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
@@ -1257,8 +1257,8 @@ static int run_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks,
     return fills(8, 4) ? launch_delta<8, 8, 4>(e, L, sp, ks, rs, vs, dk, dv, form)
          : fills(8, 2) ? launch_delta<8, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form)
                        : launch_delta<4, 16, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
-  if (d <= 128 && !busy(8, 2)) return launch_delta<4, 32, 4>(e, L, sp, ks, rs, vs, dk, dv, form);
-  if (d <= 128) return fills(8, 2) ? launch_delta<16, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form) : launch_delta<16, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
+  if (d <= 128 && !busy(8, 2)) return launch_delta<8, 16, 2>(e, L, sp, ks, rs, vs, dk, dv, form);
+  if (d <= 128) return launch_delta<16, 8, 2>(e, L, sp, ks, rs, vs, dk, dv, form);
   return launch_delta<32, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
 }
 

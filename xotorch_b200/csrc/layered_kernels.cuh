@@ -667,7 +667,7 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 }
 
 // sums of NC values over P neighbouring lanes, every lane gets all: the lanes halve the values while they add (each holds fewer and fewer), and
-// hand the sums round at the end — NC = 4 over 32 lanes: 9 shuffles instead of 20
+// hand the sums round at the end — NC = 4 over 8 lanes: 7 shuffles instead of 12
 template <int NC, int P>
 __device__ __forceinline__ void lane_sums(float (&d)[NC], int part) {
   if constexpr (NC == 1) {
@@ -700,7 +700,7 @@ __device__ __forceinline__ void lane_sums(float (&d)[NC], int part) {
 }
 
 template <int KPT, int P, int NC, bool SCALAR, bool REMOVAL>
-__global__ void __launch_bounds__(P == 32 ? 256 : 128, P == 32 ? 1 : 2) delta_rule_kernel(DeltaSrc ksrc, DeltaSrc rsrc, DeltaSrc vsrc, const float* __restrict__ wdec,
+__global__ void __launch_bounds__(128, 2) delta_rule_kernel(DeltaSrc ksrc, DeltaSrc rsrc, DeltaSrc vsrc, const float* __restrict__ wdec,
                                   const float* __restrict__ uvec, const float* __restrict__ auvec, const Item* __restrict__ seqs, int H, int dk,
                                   int dv, float* __restrict__ state, size_t state_slot_stride, float* __restrict__ o_raw, int vec4) {
   pdl_enter();
@@ -733,30 +733,48 @@ __global__ void __launch_bounds__(P == 32 ? 256 : 128, P == 32 ? 1 : 2) delta_ru
   for (int e = threadIdx.x; e < 2 * CH * NVEC * DKP; e += blockDim.x) (&buf[0][0][0][0])[e] = 0.f;   // the padding stays zero
   __syncthreads();
   const int HD = H * dk;
-  // A thread copies the same pieces (vector, offset) of every token of a chunk: which pieces is worked out per piece, not per copy
-  // (the divisions stay out of the token loop), and the token loop only adds the source's row stride.
+  // Staging.  A piece is one copy (16 or 4 bytes) of one vector of a token; the block's threads share pieces and, where there are threads to spare,
+  // the tokens of a chunk, so that no warp waits at the barrier for another's copies.  What a thread's piece is is worked out once.
   const int perk = vec4 ? dk / 4 : dk, perv = vec4 ? dv / 4 : dv;   // copies per key-sized vector / per value vector
   const int per_tok = (NVEC - 1) * perk + perv;
+  const int tlanes = max(1, min(CH, (int)blockDim.x / per_tok));    // threads that share a piece, each every tlanes-th token
+  auto source = [&](int piece, const float*& src, size_t& stride, int& off) {
+    // order of the pieces: v, then k, r (, w, u, au)
+    const int vec = piece < perv ? 2 : (piece - perv) / perk < 2 ? (piece - perv) / perk : (piece - perv) / perk + 1;
+    const int i = (piece < perv ? piece : (piece - perv) % perk) * (vec4 ? 4 : 1);
+    off = vec * DKP + i;
+    if (!SCALAR && !REMOVAL && vec >= 4) return false;       // no removal term
+    const size_t m0 = sq.row0;
+    if (vec == 0) { src = ksrc.p + m0 * ksrc.ld + ksrc.col + h / ksrc.rep * dk + i; stride = ksrc.ld; }
+    else if (vec == 1) { src = rsrc.p + m0 * rsrc.ld + rsrc.col + h / rsrc.rep * dk + i; stride = rsrc.ld; }
+    else if (vec == 2) { src = vsrc.p + m0 * vsrc.ld + vsrc.col + h * dv + i; stride = vsrc.ld; }
+    else { src = (vec == 3 ? wdec : vec == 4 ? uvec : auvec) + m0 * HD + h * dk + i; stride = HD; }
+    return true;
+  };
+  auto copy = [&](int c, const float* src, size_t stride, int off, int tl) {
+    const int t0 = c * CH, nt = min(CH, sq.n_rows - t0);
+    float* dst = &buf[c & 1][0][0][0] + off;
+    src += (size_t)t0 * stride;
+    if (vec4) {
+      for (int t = tl; t < nt; t += tlanes) cp_async16(dst + (size_t)t * NVEC * DKP, src + (size_t)t * stride);
+    } else {
+      for (int t = tl; t < nt; t += tlanes) cp_async4(dst + (size_t)t * NVEC * DKP, src + (size_t)t * stride);
+    }
+  };
+  const float* own_src = nullptr;                    // this thread's first piece
+  size_t own_stride = 0;
+  int own_off = 0;
+  const int own_piece = tlanes > 1 ? (int)threadIdx.x % per_tok : (int)threadIdx.x, own_tl = tlanes > 1 ? (int)threadIdx.x / per_tok : 0;
+  const bool own = own_tl < tlanes && own_piece < per_tok && source(own_piece, own_src, own_stride, own_off);
   auto issue = [&](int c) {
     const int t0 = c * CH, nt = min(CH, sq.n_rows - t0);
     const size_t m0 = (size_t)sq.row0 + t0;
-    for (int piece = threadIdx.x; piece < per_tok; piece += blockDim.x) {
-      // order of the pieces: v, then k, r (, w, u, au)
-      const int vec = piece < perv ? 2 : (piece - perv) / perk < 2 ? (piece - perv) / perk : (piece - perv) / perk + 1;
-      const int i = (piece < perv ? piece : (piece - perv) % perk) * (vec4 ? 4 : 1);
+    if (own) copy(c, own_src, own_stride, own_off, own_tl);
+    for (int piece = threadIdx.x + blockDim.x; piece < per_tok; piece += blockDim.x) {   // more pieces than threads (then tlanes is 1)
       const float* src;
       size_t stride;
-      if (!SCALAR && !REMOVAL && vec >= 4) continue;         // no removal term
-      if (vec == 0) { src = ksrc.p + m0 * ksrc.ld + ksrc.col + h / ksrc.rep * dk + i; stride = ksrc.ld; }
-      else if (vec == 1) { src = rsrc.p + m0 * rsrc.ld + rsrc.col + h / rsrc.rep * dk + i; stride = rsrc.ld; }
-      else if (vec == 2) { src = vsrc.p + m0 * vsrc.ld + vsrc.col + h * dv + i; stride = vsrc.ld; }
-      else { src = (vec == 3 ? wdec : vec == 4 ? uvec : auvec) + m0 * HD + h * dk + i; stride = HD; }
-      float* dst = &buf[c & 1][0][vec][i];
-      if (vec4) {
-        for (int t = 0; t < nt; ++t) cp_async16(dst + (size_t)t * NVEC * DKP, src + t * stride);
-      } else {
-        for (int t = 0; t < nt; ++t) cp_async4(dst + (size_t)t * NVEC * DKP, src + t * stride);
-      }
+      int off;
+      if (source(piece, src, stride, off)) copy(c, src, stride, off, 0);
     }
     if (SCALAR)
       for (int p = threadIdx.x; p < 3 * nt; p += blockDim.x) {

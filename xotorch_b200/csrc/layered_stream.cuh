@@ -56,7 +56,6 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int S = gridDim.x, split = blockIdx.x, n0 = blockIdx.y * LTC_M, z = blockIdx.z;
   const int nkb = (a.K + LTC_BK - 1) / LTC_BK, per = (nkb + S - 1) / S;
   const int kb0 = min(nkb, split * per), nk = min(nkb, kb0 + per) - kb0;
-  pdl_launch_dependents();
   int zb = z, mx = 0, zx = z;
   if (a.tile_batch) {                                        // which expert this row tile belongs to: known once the plan has been made
     pdl_wait();
@@ -75,6 +74,7 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   xb::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();   // not before: a later kernel's CTA that takes tensor memory and then waits for this kernel must not take it first
 
   if (warp == 0) {
     if (lane == 0) {

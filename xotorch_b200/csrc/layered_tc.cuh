@@ -165,7 +165,7 @@ struct LtcEpilogue {
 template <int NT, int EPI, int NS, typename TC>
 __global__ void __launch_bounds__(LTC_THREADS, 2 * ltc_smem_bytes(NT, NS) <= 226 * 1024 ? 2 : 1)
 ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LtcArgs a) {
-  pdl_enter();
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t ltc_smem[];
   constexpr int A_BYTES = LTC_M * LTC_BK * 2;
   constexpr int STAGE = ltc_stage_bytes(NT);
@@ -192,6 +192,7 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   __syncthreads();
   xb::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();   // not before: a later kernel's CTA that takes tensor memory and then waits for this kernel must not take it first
 
   if (warp == 0 && lane == 0) {
     // ===== TMA producer =====
@@ -260,7 +261,7 @@ constexpr int LTP_SMEM = LTP_STAGES * LTP_STAGE_BYTES + 1024 + 256;
 template <int EPI, typename TC>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LTP_THREADS, 1)
 ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LtcArgs a) {
-  pdl_enter();
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t ltc_smem[];
   constexpr int A_BYTES = LTC_M * LTC_BK * 2, NS = LTP_STAGES, NT = LTP_N;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ltc_smem) + 1023) & ~(uintptr_t)1023);
@@ -284,6 +285,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   xb::cluster_sync_all();                 // both CTAs' barriers are initialised before anybody signals across the pair
   xb::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();   // not before: a later kernel's CTA that takes tensor memory and then waits for this kernel must not take it first
 
   if (warp == 0 && lane == 0) {
     // ===== TMA producer (both CTAs): own rows of A, own half of B; completion is counted on the leader's barrier =====

@@ -23,6 +23,8 @@ constexpr int TC_M = 128;        // tokens per GEMM tile = UMMA M
 constexpr int TC_BK = 64;        // K elements per ring stage = one 128-byte swizzle row
 constexpr int TC_THREADS = 256;  // warp 0 TMA producer, warp 1 MMA issuer, warp 2 TMEM allocator, warps 4..7 epilogue
 
+constexpr int TC2_THREADS = 384; // CTA pairs: warps 4..11 epilogue
+
 enum { TCE_STORE = 0, TCE_RESID = 1, TCE_HEAD_LAST = 2, TCE_QKV = 3, TCE_SWIGLU = 4 };
 
 constexpr int TC_CHUNK = 1024;   // tokens per prefill pass: every weight tile is fetched from HBM once per chunk and reused
