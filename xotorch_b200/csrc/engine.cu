@@ -201,6 +201,7 @@ struct xotb200_engine {
   ActMaps tm_xn, tm_ao, tm_act;
   std::map<int, std::vector<CUtensorMap>> tm_w;   // per N-tile width: 4 per local layer (qkv, o, gu, down) + head
   int tc_cap = 0;                  // token rows the tensor-core scratch buffers currently hold
+  int tc_chunk = 0;                // token rows of a prefill chunk (0: not chosen yet)
   // sparse MoE prefill: gathered per-expert row blocks (rows_max = 2 * tc_cap + E * 128) and the device-side plan
   bf16 *moe_xg = nullptr, *moe_gu = nullptr, *moe_act = nullptr, *moe_y = nullptr;
   int *moe_route_e = nullptr, *moe_row_of = nullptr, *moe_row_token = nullptr, *moe_exp_info = nullptr;
@@ -599,18 +600,36 @@ static int ensure_tm_w(xotb200_engine* e, int nt) {
 static int prepare_tc(xotb200_engine* e, int n_tokens) {
   const xotb200_model_cfg& c = e->cfg;
   const size_t D = c.dim, F = c.ffn, qd = (size_t)c.n_heads * c.head_dim, nqkv = (size_t)(c.n_heads + 2 * c.n_kv_heads) * c.head_dim;
-  const int need = (std::min(n_tokens, TC_CHUNK) + TC_M - 1) / TC_M * TC_M;
+  const bool fused = e->tc_fuse && c.n_experts == 0;
+  if (e->tc_chunk == 0) e->tc_chunk = fused ? TC_CHUNK : TC_CHUNK_SMALL;
+  int need = (std::min(n_tokens, e->tc_chunk) + TC_M - 1) / TC_M * TC_M;
   if (need > e->tc_cap) {   // scratch for one chunk of `need` token rows (grown on demand, kept across requests)
     CK(cudaStreamSynchronize(e->stream));
     bf16** bufs[] = {&e->tc_x, &e->tc_xn, &e->tc_qkv, &e->tc_q, &e->tc_ao, &e->tc_gu, &e->tc_act};
     const size_t fdense = c.n_experts > 0 ? 8 : F;   // sparse MoE shards use the gathered buffers below instead of tc_gu / tc_act
-    const size_t cols[] = {D, D, nqkv, qd, qd, 2 * fdense, fdense};
-    for (int i = 0; i < 7; ++i) {
-      if (*bufs[i]) CK(cudaFree(*bufs[i]));
-      *bufs[i] = nullptr;
-      CK(cudaMalloc(bufs[i], (size_t)need * cols[i] * 2));
-      MEMSET_SYNC(e, *bufs[i], 0, (size_t)need * cols[i] * 2);
+    const size_t cols[] = {D, D, e->tc_fuse ? 0 : nqkv, qd, qd, fused ? 0 : 2 * fdense, fdense};   // the fused epilogues need no tc_qkv / tc_gu
+    e->tc_cap = 0;          // nothing is held until all of it is
+    auto take = [&]() {
+      for (int i = 0; i < 7; ++i) {
+        if (*bufs[i]) CK(cudaFree(*bufs[i]));
+        *bufs[i] = nullptr;
+      }
+      for (int i = 0; i < 7; ++i)
+        if (cols[i]) {
+          const cudaError_t r = cudaMalloc(bufs[i], (size_t)need * cols[i] * 2);
+          if (r == cudaErrorMemoryAllocation && need > TC_CHUNK_SMALL) { cudaGetLastError(); return 1; }
+          CK(r);
+          MEMSET_SYNC(e, *bufs[i], 0, (size_t)need * cols[i] * 2);
+        }
+      return 0;
+    };
+    int rc = take();
+    if (rc == 1) {          // no room for the large chunk: small ones from now on
+      e->tc_chunk = TC_CHUNK_SMALL;
+      need = TC_CHUNK_SMALL;
+      rc = take();
     }
+    if (rc) return rc;
     e->tc_cap = need;
     if (c.n_experts > 0) {
       const size_t rows = (size_t)2 * need + (size_t)c.n_experts * TC_M;
@@ -691,7 +710,7 @@ static int launch_tc_flash(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, 
   a.n_rows = S; a.pos0 = pos0; a.H = Hq; a.rep = R; a.head_rows = e->L; a.k2_from = HD / 64; a.scale = 1.0f / sqrtf((float)HD); a.out = e->tc_ao; a.err = &e->ctl->err;
   auto fn = e->cfg.dtype == XOTB200_DTYPE_F16 ? xf::flash_tc_kernel<HD / 64, HD / 64, false, true> : xf::flash_tc_kernel<HD / 64, HD / 64, false, false>;
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, xf::ft_smem_bytes(HD / 64, HD / 64))) return rc;
-  return launch_early(e, st, fn, dim3((S + xf::FT_Q - 1) / xf::FT_Q, Hq), xf::FT_THREADS, xf::ft_smem_bytes(HD / 64, HD / 64), 1, mq, mk, mk, mv, a);
+  return launch_early(e, st, fn, dim3(Hq, (S + xf::FT_Q - 1) / xf::FT_Q), xf::FT_THREADS, xf::ft_smem_bytes(HD / 64, HD / 64), 1, mq, mk, mk, mv, a);
 }
 
 template <int HD>
@@ -705,7 +724,7 @@ static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, i
   return launch_early(e, st, fn, dim3((S + 63) / 64, e->cfg.n_heads), 128, SMEM, 1, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
 }
 
-// Prefill n_tokens positions starting at pos0 on the tensor cores, in chunks of up to TC_CHUNK tokens (layer-major
+// Prefill n_tokens positions starting at pos0 on the tensor cores, in chunks of up to e->tc_chunk tokens (layer-major
 // inside a chunk, so a chunk streams the shard's weights once).  Inputs: stage_tokens /
 // stage_in or `in` (device memory); outputs: stage_out or `out` (non-last shard) or logits + ctl->token of the last position (last shard).
 static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st, const void* in = nullptr, void* out = nullptr) {
@@ -716,8 +735,8 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
   const int D = c.dim, F = c.ffn, Hq = c.n_heads, Hkv = c.n_kv_heads, hd = c.head_dim;
   const int qd = Hq * hd, nqkv = (Hq + 2 * Hkv) * hd, nl = e->end - e->start + 1;
   auto rmsnorm = c.dtype == XOTB200_DTYPE_F16 ? xb::fp::tc_rmsnorm_kernel : xb::bf::tc_rmsnorm_kernel;
-  for (int m0 = 0; m0 < n_tokens; m0 += TC_CHUNK) {
-    const int S = std::min(TC_CHUNK, n_tokens - m0);
+  for (int m0 = 0; m0 < n_tokens; m0 += e->tc_chunk) {
+    const int S = std::min(e->tc_chunk, n_tokens - m0);
     if (e->first) {
       if (int rc = launch_early(e, st, tc_gather_kernel, S, 128, 0, 1, e->stage_tokens + m0, e->embed, e->tc_x, D)) return rc;
     } else {
@@ -796,7 +815,7 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
     }
   }
   // the residual stream of the last position is what xotb200_post_to_next hands to the next shard
-  CK(cudaMemcpyAsync(e->x, e->tc_x + (size_t)((n_tokens - 1) % TC_CHUNK) * D, (size_t)D * 2, cudaMemcpyDeviceToDevice, st));
+  CK(cudaMemcpyAsync(e->x, e->tc_x + (size_t)((n_tokens - 1) % e->tc_chunk) * D, (size_t)D * 2, cudaMemcpyDeviceToDevice, st));
   return 0;
 }
 
@@ -1268,7 +1287,17 @@ int xotb200_begin_batch(xotb200_engine* e, int max_total_len, int n_requests) {
     e->L = std::max(e->L, max_total_len);
     e->nreq = n_requests;
     e->kv_req_stride = nl * 2 * (size_t)c.n_kv_heads * e->L * c.head_dim;
-    CK(cudaMalloc(&e->kv, (size_t)e->nreq * e->kv_req_stride * 2));
+    const size_t kv_bytes = (size_t)e->nreq * e->kv_req_stride * 2;
+    cudaError_t r = cudaMalloc(&e->kv, kv_bytes);
+    if (r == cudaErrorMemoryAllocation && e->tc_cap > TC_CHUNK_SMALL) {   // a large chunk's scratch gives way to the cache
+      cudaGetLastError();
+      for (bf16** p : {&e->tc_x, &e->tc_xn, &e->tc_q, &e->tc_ao, &e->tc_act}) { CK(cudaFree(*p)); *p = nullptr; }
+      e->tc_cap = 0;
+      e->tc_chunk = TC_CHUNK_SMALL;
+      r = cudaMalloc(&e->kv, kv_bytes);
+    }
+    if (r != cudaSuccess) e->kv = nullptr;
+    CK(r);
     if (c.n_experts > 0) {
       if (e->route_log) { CK(cudaFree(e->route_log)); e->route_log = nullptr; }
       CK(cudaMalloc(&e->route_log, (size_t)e->L * nl * 4));

@@ -143,12 +143,13 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     return;
   }
   FlashTile128 tl;
-  if (a.tiles) tl = a.tiles[gridDim.x - 1 - blockIdx.x];   // later tiles of a request see more keys: the long ones start first
+  // later tiles of a request see more keys: the long ones start first, those of all heads before any shorter one (the heads are the grid's fast side)
+  if (a.tiles) tl = a.tiles[gridDim.y - 1 - blockIdx.y];
   else {
-    const int t = gridDim.x - 1 - blockIdx.x;
+    const int t = gridDim.y - 1 - blockIdx.y;
     tl = FlashTile128{t * FT_Q, min(FT_Q, a.n_rows - t * FT_Q), a.pos0 + t * FT_Q, 0, 0};
   }
-  const int h = blockIdx.y, g = a.kv_per_query_head ? h : h / a.rep;
+  const int h = blockIdx.x, g = a.kv_per_query_head ? h : h / a.rep;
   const int last = tl.pos0 + tl.n_rows - 1;
   int jstart = ft_first_key(tl.pos0, a.window, a.chunk);
   if (a.page_table) jstart &= ~(FT_K - 1);           // a tile of paged keys lies in one page

@@ -1101,7 +1101,7 @@ template <int DKC, int DVC>
 static int launch_flash_tc(xotb200_lm* e, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mk2, const CUtensorMap& mv, const xf::FlashArgs& a, int n_tiles) {
   auto kern = xf::flash_tc_kernel<DKC, DVC, true, false>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, xf::ft_smem_bytes(DKC, DVC)));
-  TRY(launch_early(e, kern, dim3(n_tiles, a.H), xf::FT_THREADS, xf::ft_smem_bytes(DKC, DVC), 1, mq, mk, mk2, mv, a));
+  TRY(launch_early(e, kern, dim3(a.H, n_tiles), xf::FT_THREADS, xf::ft_smem_bytes(DKC, DVC), 1, mq, mk, mk2, mv, a));
   e->flash_launches++;
   return 0;
 }
