@@ -39,3 +39,24 @@ def test_chunks_equal_portions(shape_name, n):
     assert np.array_equal(whole, _logits(shape_name, prompt, [4096, n - 4096]))
   cut = _logits(shape_name, prompt, [1000, n - 1000])
   assert (np.abs(whole - cut) <= ATOL + RTOL * np.abs(whole)).all(), np.abs(whole - cut).max()
+
+
+@pytest.mark.parametrize("shift", [0, 50, -50])
+def test_output_over_the_input(shift):
+  """hidden states on the device, the result laid over the input or `shift` rows beside it: as into a buffer of its own"""
+  import torch
+  from xotorch_b200.native import NativeShard
+  shape, n = dataclasses.replace(PRESETS["tiny-llama-hd64"], max_pos=8192), 4096 + 130
+  e = NativeShard(hf_config(shape), device=0)
+  e.set_shard(1, 2)
+  e.init_synthetic(1234)
+  e.begin_request(n)
+  x = torch.randn(n, shape.dim, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+  own = torch.empty_like(x)
+  e.forward_device(None, x.data_ptr(), n, 0, own.data_ptr())
+  room = torch.zeros(n + 100, shape.dim, dtype=torch.bfloat16, device="cuda")
+  room[50:50 + n] = x
+  torch.cuda.synchronize()
+  e.forward_device(None, room[50:].data_ptr(), n, 0, room[50 + shift:].data_ptr())
+  assert torch.equal(room[50 + shift:50 + shift + n], own)
+  e.close()

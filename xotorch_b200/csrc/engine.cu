@@ -698,7 +698,7 @@ static int make_tmap_heads(CUtensorMap* m, const bf16* ptr, int cols, int heads,
   REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled(heads, %d columns) failed: %d", cols, (int)r);
   return 0;
 }
-// causal attention of a chunk on tcgen05 (flash_tc.cuh): q [S][Hq][HD], K / V [Hkv][L][HD]
+// causal attention of a chunk on tcgen05, from 64 rows on (6 rows: 244 us a pass with it, 236 with the 64-row mma.sync tiles) (flash_tc.cuh): q [S][Hq][HD], K / V [Hkv][L][HD]
 template <int HD>
 static int launch_tc_flash(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, int pos0, cudaStream_t st) {
   const int Hq = e->cfg.n_heads;
@@ -1394,7 +1394,8 @@ static int ensure_staging(xotb200_engine* e, int n) {
 }
 
 // Positions from which a call runs as GEMMs (prefill_tc) instead of one after the other through the decode kernel.  A dense shard streams its
-// weights once either way for one position, and once instead of n times for more; a sparse-MoE shard pays its per-expert launches first.
+// weights once either way for one position, and once instead of n times for more (two 8B layers, 2 positions: 364 us through the decode kernel, 239 as
+// GEMMs; 1B shape 178 and 140); a sparse-MoE shard pays its per-expert launches first.
 static bool runs_as_gemms(const xotb200_engine* e, int n_tokens) {
   return e->prefill_mode == 2 || (e->prefill_mode == 0 && n_tokens >= (e->cfg.n_experts > 0 ? 8 : 2));
 }
@@ -1469,7 +1470,13 @@ int xotb200_forward_device(xotb200_engine* e, const int32_t* tokens, const void*
   }
   const bool use_tc = runs_as_gemms(e, n_tokens);
   if (use_tc) {   // the caller's buffers are read and written in place, no copy through the staging buffers
-    if (int rc = prefill_tc(e, n_tokens, pos0, st, hidden_dev, e->last ? nullptr : out_hidden_dev)) return rc;
+    const char *in = static_cast<const char*>(hidden_dev), *out = static_cast<const char*>(e->last ? nullptr : out_hidden_dev);
+    const size_t bytes = (size_t)n_tokens * D * 2;
+    if (!tokens && out && in != out && in < out + bytes && out < in + bytes) {   // shifted over one another: a chunk's output may lie on a later chunk's input
+      CK(cudaMemcpyAsync(e->stage_in, in, bytes, cudaMemcpyDeviceToDevice, st));
+      in = nullptr;
+    }
+    if (int rc = prefill_tc(e, n_tokens, pos0, st, in, const_cast<char*>(out))) return rc;
   } else {
     if (!tokens) CK(cudaMemcpyAsync(e->stage_in, hidden_dev, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
     if (int rc = launch_mega(e, 1, n_tokens, 0, pos0, st)) return rc;

@@ -841,6 +841,8 @@ static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& 
   e->tc_launches++;
   return 0;
 }
+// Pairs where their tiles, empty rows and columns included, keep 72 % of the waves' slots busy: a pair's tile runs 1.2 .. 1.4 times as fast as its share of
+// 128 x 128 tiles (layered_tc.cuh), which lose less in the last wave.  K < 512: filling the ring is most of a tile.
 static bool pairs_pay(const xotb200_lm* e, int M, int N, int K) {
   const long tiles = (long)cdiv(M, 2 * LTC_M) * cdiv(N, LTP_N), pairs = std::max(1, e->sm_count / 2), waves = (tiles + pairs - 1) / pairs;
   return K >= 512 && (double)M * N >= 0.72 * (double)waves * pairs * (2.0 * LTC_M * LTP_N);
@@ -850,7 +852,7 @@ static bool pairs_pay(const xotb200_lm* e, int M, int N, int K) {
 template <typename TC, int EPI>
 static int product_tc(xotb200_lm* e, const bf16* A, long lda, long a_batch, const bf16* B, long ldb, long b_batch, TC* C, long ldc, long c_batch, int M,
                       int N, int K, int batch, const EpiArgs& epi) {
-  // one row tile or less: bound by reading B (measured up to 128 rows: 24.8 -> 17.8 us a launch at 64 .. 128 rows, width 2048)
+  // two row tiles or less: bound by reading B (layered_stream.cuh has both sides)
   if (M <= LST_MAX_ROWS) return product_stream<TC, EPI>(e, A, lda, a_batch, B, ldb, b_batch, batch, C, ldc, c_batch, M, N, K, batch, epi);
   const int nt = N > 64 ? 128 : 64;                            // 128: also a CTA's half of a pair's column tile
   CUtensorMap ma, mb;

@@ -14,7 +14,8 @@
 // Grouped products (`tile_batch`): row tile t = blockIdx.z holds NB rows of one expert, tile_batch[t] names it (negative: empty).
 // Measured (B200, per launch in a decode step, 128 x 64 tiles of layered_tc.cuh -> this kernel): 8 rows, a 2048-wide model: 26.4 -> 12.5 us on average
 // over the projections, 28.5 -> 11.2 for the 8192 x 2048 up product, experts' gate/up (14 of 16 experts of 4096 x 2048) 64.7 -> 39.6 us = 5.9 TB/s; 16
-// rows, width 4096: 34.6 -> 21.6 us on average, 14336 x 4096 33.1 -> 29.4 us; 64 .. 128 rows, width 2048: 24.8 -> 17.8 us.  What is left above
+// rows, width 4096: 34.6 -> 21.6 us on average, 14336 x 4096 33.1 -> 29.4 us; 64 .. 128 rows, width 2048: 24.8 -> 17.8 us.  129 .. 256 rows
+// keep one CTA per SM: two thirds of a stage are then rows, and a second CTA's would not fit.  What is left above
 // the weights' time is the launch, the first copies' latency and the cluster's exchange (6 .. 8 us a launch).
 // Every mbarrier wait is bounded: one that expires sets *err, the CTA waits for its own copies, still takes part in the cluster's barriers,
 // frees its tensor memory and returns.
@@ -28,7 +29,7 @@ constexpr int LST_THREADS = 256, LST_MAX_ROWS = 256, LST_EXPERT_ROWS = 128;   //
 // ring stages that let two CTAs share an SM (its 227 KB): the weights in flight per SM are then 2 * stages * 16 KB
 __host__ __device__ constexpr int lst_stage_bytes(int nb) { return LTC_M * LTC_BK * 2 + nb * LTC_BK * 2; }
 __host__ __device__ constexpr int lst_stages(int nb) { return nb <= 16 ? 6 : nb <= 32 ? 5 : nb <= 64 ? 4 : nb <= 128 ? 3 : 4; }
-__host__ __device__ constexpr int lst_ctas_per_sm(int nb) { return nb <= 128 ? 2 : 1; }   // 256 rows: half of a stage is rows, one CTA per SM with a deeper ring
+__host__ __device__ constexpr int lst_ctas_per_sm(int nb) { return nb <= 128 ? 2 : 1; }   // 256 rows: two thirds of a stage are rows, one CTA per SM with a deeper ring
 __host__ __device__ constexpr int lst_smem_bytes(int nb) { return lst_stages(nb) * lst_stage_bytes(nb) + 1024 + 256; }
 static_assert(lst_smem_bytes(128) <= 112 * 1024 && lst_smem_bytes(16) <= 112 * 1024 && lst_smem_bytes(32) <= 112 * 1024 && lst_smem_bytes(64) <= 112 * 1024, "two CTAs per SM");
 static_assert(LTC_M * 128 * 4 <= lst_stages(128) * lst_stage_bytes(128) && LTC_M * 256 * 4 <= lst_stages(256) * lst_stage_bytes(256), "the partial tile reuses the ring");

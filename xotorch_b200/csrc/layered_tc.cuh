@@ -255,6 +255,8 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // leader's thread issues tcgen05.mma.cta_group::2 over both CTAs' shared memory, and every CTA keeps its 128 rows of the accumulator.  Persistent: 74
 // pairs walk the tiles (row tile fastest, so that pairs running together share weight tiles in L2) with two accumulators in tensor memory (all
 // 512 columns), so the epilogue of one tile runs under the products of the next.  Plain loads, no multicast.  Every wait is bounded.
+// Measured (B200, a launch, 128 x 128 tiles -> pairs): 3500 rows, width 2048: 86 -> 62 us, the 8192-wide up product with its activation 189 -> 133 us
+// (213 with four epilogue warps: they took longer than the next tile's products); 1024 rows, width 4096, all products of a pass: 1139 -> 976 us.
 constexpr int LTP_N = 256, LTP_STAGES = 6, LTP_THREADS = 384, LTP_STAGE_BYTES = LTC_M * LTC_BK * 2 + LTP_N / 2 * LTC_BK * 2;
 constexpr int LTP_SMEM = LTP_STAGES * LTP_STAGE_BYTES + 1024 + 256;
 
