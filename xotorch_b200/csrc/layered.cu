@@ -2566,6 +2566,11 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
       const size_t need = splits > 1 ? (size_t)M * L.s.heads * splits * (2 + (latent ? L.s.kv_rank : L.s.vdim)) : 0;
       if (need > e->part_cap) { drop_graphs(e); TRY(regrow(e->part, need * 4)); e->part_cap = need; }
     }
+  // rows of the stream, each followed by the first mixing layer's values where those cross the border
+  auto copy_rows = [&](float* dst, size_t dld, const float* src, size_t sld, size_t n, cudaMemcpyKind kind) -> int {
+    CK(cudaMemcpy2DAsync(dst, dld * 4, src, sld * 4, n * 4, M, kind, e->stream));
+    return 0;
+  };
   GraphSlot* gs = nullptr;
   if (decode_shape) {
     const std::array<long, 5> key{n_seq, n_want, (logits_f32 ? 1 : 0) | (argmax_i32 ? 2 : 0), sp.max_len, (long)off};
@@ -2604,23 +2609,12 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
         f.n_reqs = kv.second.n_reqs; f.n_tiles = kv.second.n_tiles; f.n_keys = kv.second.n_keys; f.max_keys = kv.second.max_keys;
         sp.flash[kv.first] = f;
       }
-      // rows of the stream, each followed by the first mixing layer's values where those cross the border
-      auto copy_rows = [&](float* dst, size_t dld, const float* src, size_t sld, size_t n, cudaMemcpyKind kind) -> int {
-        CK(cudaMemcpy2DAsync(dst, dld * 4, src, sld * 4, n * 4, M, kind, e->stream));
-        return 0;
-      };
       if (!e->first) {
         const size_t ld = (size_t)D + e->carry_in;
         TRY(copy_rows(e->x, D, hidden_f32, ld, D, cudaMemcpyHostToDevice));
         if (e->carry_in) TRY(copy_rows(e->vfirst, e->carry_in, hidden_f32 + D, ld, e->carry_in, cudaMemcpyHostToDevice));
       }
       TRY(e->esz == 2 ? run_layers<bf16>(e, sp, n_want) : run_layers<float>(e, sp, n_want));
-      if (!e->last) {
-        const size_t ld = (size_t)D + e->carry_out;
-        float* dst = direct ? hidden_out_f32 : e->h_out;
-        TRY(copy_rows(dst, ld, e->x, D, D, cudaMemcpyDeviceToHost));
-        if (e->carry_out) TRY(copy_rows(dst + D, ld, e->vfirst, e->carry_out, e->carry_out, cudaMemcpyDeviceToHost));
-      }
       if (!results) CK(cudaMemcpyAsync(e->h_err, e->d_err, 4, cudaMemcpyDeviceToHost, e->stream));
       return 0;
     };
@@ -2641,9 +2635,14 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     }
     if (rc < 0) { cudaStreamSynchronize(e->stream); return rc; }
   }
-  if (results) {
-    // behind the (replayed) kernels, not part of a captured step: the caller's pointer is another one each time.  The argmax and the error word lie behind
-    // the logits; one copy when the logits go through the staging buffer or are not asked for.
+  // What goes to the caller is copied behind the (replayed) kernels and is not part of a captured step: the caller's pointer is another one each time.
+  if (!e->last) {
+    const size_t ld = (size_t)D + e->carry_out;
+    float* dst = direct ? hidden_out_f32 : e->h_out;
+    TRY(copy_rows(dst, ld, e->x, D, D, cudaMemcpyDeviceToHost));
+    if (e->carry_out) TRY(copy_rows(dst + D, ld, e->vfirst, e->carry_out, e->carry_out, cudaMemcpyDeviceToHost));
+  } else if (results) {
+    // the argmax and the error word lie behind the logits; one copy when the logits go through the staging buffer or are not asked for
     const size_t n = (size_t)n_want * V;
     if (direct) CK(cudaMemcpyAsync(logits_f32, e->logits, n * 4, cudaMemcpyDeviceToHost, e->stream));
     const size_t skip = direct || !logits_f32 ? n : 0;
