@@ -249,7 +249,25 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const float* rel = a.rel ? a.rel + (size_t)h * a.rel_n : nullptr;
     float m = -INFINITY, den = 0.f;                  // reference of the exponentials (units of ln 2), sum of the weights
     bool ok = true;
-    for (int j = 0; j < nt; ++j) {
+    // Tokens of a tile that no row here sees (a request's last piece of a page, the next request's keys, what lies before a window) hold anything: their
+    // weight is 0, but 0 * Inf is not.  Their rows of the value stage are zeroed before the product reads it (a row of a chunk is 128 bytes, swizzled
+    // within itself).
+    const int seen0 = ft_first_key(tl.pos0, a.window, a.chunk);
+    auto clear_unseen = [&](int j) -> bool {
+      const int j0 = jstart + j * FT_K, lead = min(max(seen0 - j0, 0), FT_K), rest = min(max(last + 1 - j0, 0), FT_K);   // rows [lead, rest) are seen
+      if (lead == 0 && rest == FT_K) return true;
+      if (!__all_sync(0xffffffffu, ft_wait(&v_full[j % VS], (j / VS) & 1, abort, a.err))) return false;
+      for (int i = r; i < (lead + FT_K - rest) * DVC * 8; i += 128) {
+        const int n = i / (DVC * 8), row = n < lead ? n : rest + n - lead, c = i / 8 % DVC;
+        *reinterpret_cast<uint4*>(vs + (j % VS) * V_BYTES + c * FT_K * 128 + row * 128 + i % 8 * 16) = make_uint4(0, 0, 0, 0);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      return true;
+    };
+    int j = 0;
+    for (; j < nt; ++j) {
+      // no row of this warp sees this tile or a later one: the warp's output is read before their products are added to it (0 * Inf again)
+      if (jstart + j * FT_K > pos - lane + 31) break;
       ok = __all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err));
       if (!ok) break;
       xb::tc_fence_after();
@@ -302,7 +320,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             uint32_t o[32];
             tmem_ld32(tm_o + lane_base + c, o);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+            for (int i = 0; i < 32; ++i) o[i] = m == -INFINITY ? 0u : __float_as_uint(__uint_as_float(o[i]) * corr);   // nothing seen yet: a plain 0
             tmem_st32(tm_o + lane_base + c, o);
           }
           tmem_st_wait();
@@ -326,10 +344,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tmem_st32(ts, hi);
       if constexpr (PAIR) tmem_st32(ts + 32, rest);
       tmem_st_wait();
+      ok = clear_unseen(j);
+      if (!ok) break;
       xb::tc_fence_before();
       mbar_arrive(&p_full[j & 1]);
     }
-    if (ok) ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(nt - 1) & 1], ((nt - 1) >> 1) & 1, abort, a.err));
+    if (ok) ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort, a.err));
     if (ok) {
       xb::tc_fence_after();
       float f = 1.0f;
@@ -367,6 +387,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(pack16<F16>(v[i], v[i + 1]), pack16<F16>(v[i + 2], v[i + 3]), pack16<F16>(v[i + 4], v[i + 5]), pack16<F16>(v[i + 6], v[i + 7]));
         }
         __syncwarp();
+      }
+      for (; j < nt; ++j) {                          // tiles this warp sees nothing of: the products wait for all four warps
+        ok = __all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err)) && clear_unseen(j);
+        if (!ok) break;
+        xb::tc_fence_before();
+        mbar_arrive(&p_full[j & 1]);
       }
     }
   }
