@@ -718,10 +718,12 @@ static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, i
   if (S >= 64 && e->cfg.n_heads > 1) return launch_tc_flash<HD>(e, S, R, kc, vc, pos0, st);
   constexpr int SMEM = (64 + 4 * 64) * HD * 2;          // Q tile + 2 x (K, V) tiles
   const bool f16 = e->cfg.dtype == XOTB200_DTYPE_F16;
-  auto fn = f16 ? xb::fp::tc_flash_attn_kernel<HD> : xb::bf::tc_flash_attn_kernel<HD>;
+  const bool few = S < TC_FEW;
+  auto fn = few ? (f16 ? xb::fp::tc_flash_attn_kernel<HD, true> : xb::bf::tc_flash_attn_kernel<HD, true>)
+                : (f16 ? xb::fp::tc_flash_attn_kernel<HD, false> : xb::bf::tc_flash_attn_kernel<HD, false>);
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, SMEM)) return rc;
   const float scale_log2 = 1.4426950408889634f / sqrtf((float)HD);
-  return launch_early(e, st, fn, dim3((S + 63) / 64, e->cfg.n_heads), 128, SMEM, 1, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
+  return launch_early(e, st, fn, dim3(few ? S : (S + 63) / 64, e->cfg.n_heads), 128, SMEM, 1, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
 }
 
 // Prefill n_tokens positions starting at pos0 on the tensor cores, in chunks of up to e->tc_chunk tokens (layer-major
@@ -1397,7 +1399,7 @@ static int ensure_staging(xotb200_engine* e, int n) {
 // weights once either way for one position, and once instead of n times for more (two 8B layers, 2 positions: 364 us through the decode kernel, 239 as
 // GEMMs; 1B shape 178 and 140); a sparse-MoE shard pays its per-expert launches first.
 static bool runs_as_gemms(const xotb200_engine* e, int n_tokens) {
-  return e->prefill_mode == 2 || (e->prefill_mode == 0 && n_tokens >= (e->cfg.n_experts > 0 ? 8 : 2));
+  return e->prefill_mode == 2 || (e->prefill_mode == 0 && n_tokens >= (e->cfg.n_experts > 0 ? TC_FEW : 2));
 }
 
 int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidden_f32, int n_tokens, int pos0,
