@@ -79,3 +79,20 @@ def test_positions_in_front_of_a_non_finite_one(at):
   got = run(eng, rows[61:].clone(), 61)
   assert np.array_equal(got[:at], ref[:at]) and not np.isfinite(got[at]).any()
   eng.close()
+
+
+def test_vocabularies_that_the_head_has_no_tile_for():
+  from dataclasses import replace
+  from xotorch_b200.native import NativeShard
+  shape = replace(PRESETS["tiny-llama-hd64"], name="tiny-odd-vocab", vocab=2050)
+  eng = NativeShard(hf_config(shape), 0)
+  eng.set_shard(0, shape.n_layers - 1)
+  eng.init_synthetic(2)
+  ids = np.arange(5, dtype=np.int32).reshape(1, -1) * 401
+  out = []
+  for mode in (1, 0):
+    eng.begin_request(8)
+    eng.set_prefill_mode(mode)
+    out.append(eng.forward(ids, 0))
+  assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
+  eng.close()

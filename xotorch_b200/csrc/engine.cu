@@ -1399,7 +1399,10 @@ static int ensure_staging(xotb200_engine* e, int n) {
 // weights once either way for one position, and once instead of n times for more (two 8B layers, 2 positions: 364 us through the decode kernel, 239 as
 // GEMMs; 1B shape 178 and 140); a sparse-MoE shard pays its per-expert launches first.
 static bool runs_as_gemms(const xotb200_engine* e, int n_tokens) {
-  return e->prefill_mode == 2 || (e->prefill_mode == 0 && n_tokens >= (e->cfg.n_experts > 0 ? TC_FEW : 2));
+  if (e->prefill_mode != 0) return e->prefill_mode == 2;
+  if (n_tokens >= TC_FEW) return true;
+  if (n_tokens < 2 || e->cfg.n_experts > 0) return false;
+  return !e->last || e->cfg.vocab % 64 == 0;   // the head as a GEMM has no tile for other vocabularies (prompts of TC_FEW positions or more are refused there)
 }
 
 int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidden_f32, int n_tokens, int pos0,
