@@ -96,3 +96,18 @@ def test_vocabularies_that_the_head_has_no_tile_for():
     out.append(eng.forward(ids, 0))
   assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1])
   eng.close()
+
+
+def test_a_long_cache_is_left_to_the_decode_kernel():
+  """one launch walks the positions where spreading the keys over the chip pays, whatever the number of positions below the general rule; the GEMMs elsewhere"""
+  eng, shape = middle_shard("tiny-llama-hd64", False)
+  h = torch.randn(8, shape.dim, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+
+  def launches(n, pos0):
+    before = eng.kernel_launches()
+    run(eng, h[:n].clone(), pos0)
+    return eng.kernel_launches() - before
+  eng.begin_request(2048)
+  for n, pos0, gemms in ((2, 0, True), (2, 300, True), (2, 2040, False), (3, 2040, False), (7, 2040, True), (8, 2040, True), (1, 0, False)):
+    assert (launches(n, pos0) > 1) == gemms, (n, pos0)
+  eng.close()

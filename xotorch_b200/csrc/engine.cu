@@ -1398,10 +1398,21 @@ static int ensure_staging(xotb200_engine* e, int n) {
 // Positions from which a call runs as GEMMs (prefill_tc) instead of one after the other through the decode kernel.  A dense shard streams its
 // weights once either way for one position, and once instead of n times for more (two 8B layers, 2 positions: 364 us through the decode kernel, 239 as
 // GEMMs; 1B shape 178 and 140); a sparse-MoE shard pays its per-expert launches first.
-static bool runs_as_gemms(const xotb200_engine* e, int n_tokens) {
+// Behind a long cache it is the other way round: the decode kernel spreads the keys over the chip, as GEMMs one block walks all keys of its query and
+// head.  Below TC_FEW positions the cheaper way is taken by a layer's time in us: constants fitted to both ways at 2 .. 7 positions behind 100 .. 16000
+// keys, layers of 122 MB with heads of 64 and 436 MB with heads of 128 (as GEMMs / one after the other: 2 positions behind 4000 keys 261 / 213 and
+// 144 / 98 us; 4 behind 4000 261 / 402 and 142 / 182; 4 behind 16000 705 / 529 and 397 / 238); the lines cross within a tenth of where the times do.
+static bool gemms_pay(const xotb200_engine* e, int n_tokens, int pos0) {
+  const xotb200_model_cfg& c = e->cfg;
+  const double keys = (double)pos0 + n_tokens, kv_bytes = 4.0 * c.n_kv_heads * c.head_dim;
+  const double weight_bytes = 2.0 * c.dim * ((2.0 * c.n_heads + 2.0 * c.n_kv_heads) * c.head_dim + 3.0 * c.ffn);
+  const int waves = (n_tokens * c.n_heads + 2 * e->sm_count - 1) / (2 * e->sm_count);
+  return 31.0 + weight_bytes / 7.4e6 + waves * keys * (0.0056 + 0.000244 * c.head_dim) <= n_tokens * (21.0 + weight_bytes / 6.9e6 + keys * kv_bytes / 1.6e6);
+}
+static bool runs_as_gemms(const xotb200_engine* e, int n_tokens, int pos0) {
   if (e->prefill_mode != 0) return e->prefill_mode == 2;
   if (n_tokens >= TC_FEW) return true;
-  if (n_tokens < 2 || e->cfg.n_experts > 0) return false;
+  if (n_tokens < 2 || e->cfg.n_experts > 0 || !gemms_pay(e, n_tokens, pos0)) return false;
   return !e->last || e->cfg.vocab % 64 == 0;   // the head as a GEMM has no tile for other vocabularies (prompts of TC_FEW positions or more are refused there)
 }
 
@@ -1430,7 +1441,7 @@ int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidde
     CK(cudaGetLastError());
     e->launches++;
   }
-  const bool use_tc = runs_as_gemms(e, n_tokens);
+  const bool use_tc = runs_as_gemms(e, n_tokens, pos0);
   if (use_tc) {
     if (int rc = prefill_tc(e, n_tokens, pos0, st)) return rc;     // GEMM-shaped: 5th-gen tensor cores
   } else {
@@ -1473,7 +1484,7 @@ int xotb200_forward_device(xotb200_engine* e, const int32_t* tokens, const void*
       REQUIRE(tokens[i] >= 0 && tokens[i] < e->cfg.vocab, "token id %d out of range", tokens[i]);
     CK(cudaMemcpyAsync(e->stage_tokens, tokens, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, st));
   }
-  const bool use_tc = runs_as_gemms(e, n_tokens);
+  const bool use_tc = runs_as_gemms(e, n_tokens, pos0);
   if (use_tc) {   // the caller's buffers are read and written in place, no copy through the staging buffers
     const char *in = static_cast<const char*>(hidden_dev), *out = static_cast<const char*>(e->last ? nullptr : out_hidden_dev);
     const size_t bytes = (size_t)n_tokens * D * 2;
@@ -1540,7 +1551,7 @@ int xotb200_forward_hop(xotb200_engine* e, const int32_t* tokens, int64_t seq_in
   e->hop_out = (!e->last && decode) ? 1 : 0;
   e->hop_seq_in = (unsigned int)seq_in;
   e->hop_seq_out = seq;
-  const bool use_tc = runs_as_gemms(e, n_tokens);
+  const bool use_tc = runs_as_gemms(e, n_tokens, pos0);
   int rc = use_tc ? prefill_tc(e, n_tokens, pos0, st) : launch_mega(e, 1, n_tokens, 0, pos0, st);
   e->hop_in = e->hop_out = 0;
   if (rc) return rc;
