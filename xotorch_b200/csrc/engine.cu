@@ -444,7 +444,8 @@ static int ensure_smem_attr(int device, const void* fn, int bytes) {
 }
 
 // A launch that may start before the kernel in front of it has finished (every kernel of the dense prompt path waits for it itself: pdl_wait), in
-// clusters of `cluster` CTAs along x (0 or 1: none, or the kernel fixes its cluster shape itself).
+// clusters of `cluster` CTAs along x (0 or 1: none, or the kernel fixes its cluster shape itself; LAUNCH_LATE: none, and the ordinary start).
+constexpr int LAUNCH_LATE = -1;
 template <typename... KA, typename... A>
 static int launch_early(xotb200_engine* e, cudaStream_t st, void (*fn)(KA...), dim3 grid, int threads, size_t smem, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -458,7 +459,7 @@ static int launch_early(xotb200_engine* e, cudaStream_t st, void (*fn)(KA...), d
   at[1].id = cudaLaunchAttributeClusterDimension;
   at[1].val.clusterDim = {(unsigned)cluster, 1, 1};
   cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cfg.numAttrs = cluster > 1 ? 2 : cluster == LAUNCH_LATE ? 0 : 1;
   CK(cudaLaunchKernelEx(&cfg, fn, static_cast<KA>(args)...));
   e->launches++;
   return 0;
@@ -723,7 +724,11 @@ static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, i
                 : (f16 ? xb::fp::tc_flash_attn_kernel<HD, false> : xb::bf::tc_flash_attn_kernel<HD, false>);
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, SMEM)) return rc;
   const float scale_log2 = 1.4426950408889634f / sqrtf((float)HD);
-  return launch_early(e, st, fn, dim3(few ? S : (S + 63) / 64, e->cfg.n_heads), 128, SMEM, 1, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
+  // 8 .. 63 rows: one block per head.  Started early they find the SMs that the product in front has left already and share them, two to an SM, while others
+  // stay empty: behind many keys that costs more than the launch (early / ordinary start, one 8B layer, 16 rows behind 500: 138 / 140 us, 1000: 154 / 158,
+  // 2000: 191 / 182, 16000: 698 / 581; two 1B layers 156 / 150, 181 / 165, 244 / 208, 1059 / 754).
+  const int late = !few && pos0 + S > 1024 ? LAUNCH_LATE : 1;
+  return launch_early(e, st, fn, dim3(few ? S : (S + 63) / 64, e->cfg.n_heads), 128, SMEM, late, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
 }
 
 // Prefill n_tokens positions starting at pos0 on the tensor cores, in chunks of up to e->tc_chunk tokens (layer-major
