@@ -1289,12 +1289,11 @@ int xotb200_begin_batch(xotb200_engine* e, int max_total_len, int n_requests) {
   CK(cudaStreamSynchronize(e->stream));
   const xotb200_model_cfg& c = e->cfg;
   const size_t nl = e->end - e->start + 1;
-  if (max_total_len > e->L || n_requests != e->nreq) {
+  if (!e->kv || max_total_len > e->L || n_requests != e->nreq) {
+    const int L = std::max(e->L, max_total_len);
+    const size_t stride = nl * 2 * (size_t)c.n_kv_heads * L * c.head_dim, kv_bytes = (size_t)n_requests * stride * 2;
+    e->L = 0;               // until the new cache is there, steps are refused
     if (e->kv) { CK(cudaFree(e->kv)); e->kv = nullptr; }
-    e->L = std::max(e->L, max_total_len);
-    e->nreq = n_requests;
-    e->kv_req_stride = nl * 2 * (size_t)c.n_kv_heads * e->L * c.head_dim;
-    const size_t kv_bytes = (size_t)e->nreq * e->kv_req_stride * 2;
     cudaError_t r = cudaMalloc(&e->kv, kv_bytes);
     if (r == cudaErrorMemoryAllocation && e->tc_cap > TC_CHUNK_SMALL) {   // a large chunk's scratch gives way to the cache
       cudaGetLastError();
@@ -1303,12 +1302,15 @@ int xotb200_begin_batch(xotb200_engine* e, int max_total_len, int n_requests) {
       e->tc_chunk = TC_CHUNK_SMALL;
       r = cudaMalloc(&e->kv, kv_bytes);
     }
-    if (r != cudaSuccess) e->kv = nullptr;
+    if (r != cudaSuccess) { e->kv = nullptr; cudaGetLastError(); }   // reported here, not by the next launch
     CK(r);
     if (c.n_experts > 0) {
       if (e->route_log) { CK(cudaFree(e->route_log)); e->route_log = nullptr; }
-      CK(cudaMalloc(&e->route_log, (size_t)e->L * nl * 4));
+      CK(cudaMalloc(&e->route_log, (size_t)L * nl * 4));
     }
+    e->L = L;
+    e->nreq = n_requests;
+    e->kv_req_stride = stride;
   }
   if (e->route_log) CK(cudaMemsetAsync(e->route_log, 0xff, (size_t)e->L * nl * 4, e->stream));
   if (max_total_len > e->rope_len) {
