@@ -445,6 +445,8 @@ static int ensure_smem_attr(int device, const void* fn, int bytes) {
 
 // A launch that may start before the kernel in front of it has finished (every kernel of the dense prompt path waits for it itself: pdl_wait), in
 // clusters of `cluster` CTAs along x (0 or 1: none, or the kernel fixes its cluster shape itself; LAUNCH_LATE: none, and the ordinary start).
+// tc_stream_kernel reads its first weights before that wait: no kernel that writes weights may be in flight when a product is launched (loading ends with a
+// synchronisation).
 constexpr int LAUNCH_LATE = -1;
 template <typename... KA, typename... A>
 static int launch_early(xotb200_engine* e, cudaStream_t st, void (*fn)(KA...), dim3 grid, int threads, size_t smem, int cluster, A&&... args) {
@@ -1818,6 +1820,7 @@ int xotb200_debug_gemm(xotb200_engine* e, const void* a_bf16, const void* w_bf16
   MEMCPY_SYNC(e, dW0, w_bf16, (size_t)N * K * 2, cudaMemcpyHostToDevice);
   relayout_rows_kernel<<<N, 128, 0, e->stream>>>(dW0, dW, N, K, 0, e->cfg.head_dim, 1, 0, N, tk);
   CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(e->stream));                  // a streaming product reads its first weights before it waits for the kernel in front
   ActMaps tA;
   CUtensorMap tB;
   const bool stream = N % TC_M == 0;                     // as tc_gemm chooses

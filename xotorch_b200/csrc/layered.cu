@@ -743,7 +743,8 @@ static bool make_map3(CUtensorMap* m, const void* ptr, long rows, long K, long l
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Launches a kernel in clusters of `cluster` CTAs along x.  In a step of few rows (e->early) it may start before the kernel in front of it has
+// Launches a kernel in clusters of `cluster` CTAs along x.  Weights are read before a kernel waits for the one in front (stream_gemm_kernel,
+// gemv_rows_kernel, the row norms), so none may be in the writing then: loading ends with a synchronisation.  In a step of few rows (e->early) it may start before the kernel in front of it has
 // finished: it waits itself (pdl_wait), its launch and what it loads ahead of that are hidden.  Such a step is a chain of some forty short
 // kernels, and the launches are most of it (one request, width 1024: 5979 -> 4913 us for 25 steps).  With many rows the kernels are long, and
 // blocks that were placed early, around a kernel still running, are spread worse over the SMs (1024 rows, width 4096: 2503 -> 2588 us).
