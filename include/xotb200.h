@@ -65,9 +65,10 @@ typedef struct xotb200_engine xotb200_engine;
 const char* xotb200_last_error(void);
 /* Library / build identification ("xotb200 <version> sm_100a"). */
 const char* xotb200_version(void);
-/* Page-locked host memory for results: a step whose output pointer lies in it is copied there directly, without a second copy on the CPU. */
-int xotb200_host_alloc(int64_t bytes, void** out);
-int xotb200_host_free(void* p);
+/* Page-locked host memory for results: a step whose output pointer lies in it is copied there directly, without a second copy on the CPU.
+ * Usable with engines on every device; `device` (the same one for both calls) owns the allocation and is the calling thread's current one afterwards. */
+int xotb200_host_alloc(int device, int64_t bytes, void** out);
+int xotb200_host_free(int device, void* p);
 
 /* ---- lifetime: replaces ShardedGeneralModel.__init__ / clear_model
  *      (xotorch/inference/torch/models/general_mha.py:144-176; sharded_inference_engine.py:85-106) ---- */

@@ -263,9 +263,10 @@ typedef struct xotb200_lm xotb200_lm;
 
 const char* xotb200_lm_last_error(void);
 const char* xotb200_lm_version(void);
-/* Page-locked host memory for results: a step whose output pointer lies in it is copied there directly, without a second copy on the CPU. */
-int xotb200_lm_host_alloc(int64_t bytes, void** out);
-int xotb200_lm_host_free(void* p);
+/* Page-locked host memory for results: a step whose output pointer lies in it is copied there directly, without a second copy on the CPU.
+ * Usable with engines on every device; `device` (the same one for both calls) owns the allocation and is the calling thread's current one afterwards. */
+int xotb200_lm_host_alloc(int device, int64_t bytes, void** out);
+int xotb200_lm_host_free(int device, void* p);
 
 /* `layers` has cfg->n_layers entries (the engine keeps those of its range). */
 int xotb200_lm_create(const xotb200_lm_cfg* cfg, const xotb200_lm_layer* layers, int device, xotb200_lm** out);

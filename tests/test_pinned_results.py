@@ -70,3 +70,35 @@ def test_threads_do_not_share_a_block():
   threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
   [t.start() for t in threads], [t.join() for t in threads]
   assert not bad
+
+
+def test_blocks_are_taken_and_freed_under_the_device_of_their_engine():
+  """an array is asked for before the step makes the engine's device current: the allocation names it, in any thread"""
+  from xotorch_b200 import _lib
+  calls = []
+
+  class Library:
+    heap = Heap()
+
+    def x_host_alloc(self, device, size, out):
+      calls.append(("alloc", device.value, threading.get_ident()))
+      out._obj.value = self.heap.alloc(size.value)
+      return 0
+
+    def x_host_free(self, device, p):
+      calls.append(("free", device.value, threading.get_ident()))
+      self.heap.free(p.value)
+      return 0
+  lib = Library()
+  pools = [_lib.results(lib, "x", d) for d in (0, 3)]
+  assert pools[0] is not pools[1] and _lib.results(lib, "x", 3) is pools[1]
+  t = threading.Thread(target=lambda: pools[1].empty((SMALLEST,)))
+  t.start(), t.join()
+  assert [c[:2] for c in calls] == [("alloc", 3)] and calls[0][2] != threading.get_ident()
+  gc.collect()
+  pools[1].limit = 8 * SMALLEST
+  pools[1].empty((8 * SMALLEST,), np.uint8)          # the smaller block makes room
+  assert [c[:2] for c in calls] == [("alloc", 3), ("free", 3), ("alloc", 3)]
+  for lm in (False, True):                           # both engines' signatures take the device first
+    for name in ("host_alloc", "host_free"):
+      assert (_lib._LM_SIGS if lm else _lib._SIGS)[("xotb200_lm_" if lm else "xotb200_") + name][1][0] is C.c_int

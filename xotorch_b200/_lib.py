@@ -36,13 +36,13 @@ class XotB200Error(RuntimeError):
 
 
 _lib = None
-_pools, _pools_lock = {}, threading.Lock()      # one per loaded library (libraries stay loaded)
+_pools, _pools_lock = {}, threading.Lock()      # one per loaded library (libraries stay loaded) and device
 
 _SIGS = {
   "xotb200_last_error": (C.c_char_p, []),
   "xotb200_version": (C.c_char_p, []),
-  "xotb200_host_alloc": (C.c_int, [C.c_int64, C.POINTER(C.c_void_p)]),
-  "xotb200_host_free": (C.c_int, [C.c_void_p]),
+  "xotb200_host_alloc": (C.c_int, [C.c_int, C.c_int64, C.POINTER(C.c_void_p)]),
+  "xotb200_host_free": (C.c_int, [C.c_int, C.c_void_p]),
   "xotb200_create": (C.c_int, [C.POINTER(ModelCfg), C.c_int, C.POINTER(C.c_void_p)]),
   "xotb200_destroy": (C.c_int, [C.c_void_p]),
   "xotb200_set_shard": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
@@ -152,8 +152,8 @@ _I32P = C.POINTER(C.c_int32)
 _LM_SIGS = {
   "xotb200_lm_last_error": (C.c_char_p, []),
   "xotb200_lm_version": (C.c_char_p, []),
-  "xotb200_lm_host_alloc": (C.c_int, [C.c_int64, C.POINTER(C.c_void_p)]),
-  "xotb200_lm_host_free": (C.c_int, [C.c_void_p]),
+  "xotb200_lm_host_alloc": (C.c_int, [C.c_int, C.c_int64, C.POINTER(C.c_void_p)]),
+  "xotb200_lm_host_free": (C.c_int, [C.c_int, C.c_void_p]),
   "xotb200_lm_create": (C.c_int, [C.POINTER(LmCfg), C.POINTER(LmLayer), C.c_int, C.POINTER(C.c_void_p)]),
   "xotb200_lm_destroy": (C.c_int, [C.c_void_p]),
   "xotb200_lm_load_dir": (C.c_int, [C.c_void_p, C.c_char_p]),
@@ -212,13 +212,13 @@ def load_lm(path: os.PathLike | None = None, build: bool = True) -> C.CDLL:
   return lib
 
 
-def results(lib, prefix: str) -> "ResultPool":
-  """the process's pool of page-locked result arrays of a loaded library"""
-  pool = _pools.get(id(lib))
+def results(lib, prefix: str, device: int) -> "ResultPool":
+  """the process's pool of page-locked result arrays of a loaded library and a device"""
+  pool = _pools.get((id(lib), device))
   if pool is None:
     from .pinned import library_pool
     with _pools_lock:
-      pool = _pools.setdefault(id(lib), library_pool(lib, prefix))
+      pool = _pools.setdefault((id(lib), device), library_pool(lib, prefix, device))
   return pool
 
 

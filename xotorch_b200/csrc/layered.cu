@@ -2026,12 +2026,14 @@ extern "C" {
 const char* xotb200_lm_last_error(void) { return g_err; }
 const char* xotb200_lm_version(void) { return "xotb200_lm 0.1.0 sm_100a"; }
 
-int xotb200_lm_host_alloc(int64_t bytes, void** out) {
+int xotb200_lm_host_alloc(int device, int64_t bytes, void** out) {
   REQUIRE(bytes > 0 && out, "bad argument");
+  CK(cudaSetDevice(device));   // a thread that has not chosen one yet would start a context on device 0
   CK(cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable));
   return 0;
 }
-int xotb200_lm_host_free(void* p) {
+int xotb200_lm_host_free(int device, void* p) {
+  CK(cudaSetDevice(device));
   if (p) CK(cudaFreeHost(p));
   return 0;
 }

@@ -453,8 +453,8 @@ class LayeredShard:
     if dtype not in ("bfloat16", "float32"):
       raise ValueError(f"dtype {dtype!r}: the layered engine serves in bfloat16 and has an all-float32 mode")
     self.lib = _lib.load_lm()
-    self.results = _lib.results(self.lib, "xotb200_lm")
     self.config, self.family, self.device, self.dtype = dict(config), fam, int(device), dtype
+    self.results = _lib.results(self.lib, "xotb200_lm", self.device)
     self.globals = LAYERED_FAMILIES[fam][1](config)
     self.n_layers = len(config["layers"])
     self.h = None

@@ -71,10 +71,10 @@ def cfg_from_hf(hf: dict) -> ModelCfg:
 class NativeShard:
   def __init__(self, hf_config: dict, device: int = 0):
     self.lib = _lib.load()
-    self.results = _lib.results(self.lib, "xotb200")
     self.hf_config = dict(hf_config)
     self.cfg = cfg_from_hf(hf_config)
     self.device = device
+    self.results = _lib.results(self.lib, "xotb200", self.device)
     h = C.c_void_p()
     check(self.lib.xotb200_create(C.byref(self.cfg), device, C.byref(h)))
     self.h = h

@@ -61,14 +61,15 @@ class ResultPool:
     return np.frombuffer(block, dtype=dtype, count=count).reshape(shape)
 
 
-def library_pool(lib, prefix: str) -> ResultPool:
-  """the pool of page-locked memory that a native library hands out through `<prefix>_host_alloc` / `<prefix>_host_free`"""
+def library_pool(lib, prefix: str, device: int = 0) -> ResultPool:
+  """the pool of page-locked memory that a native library hands out through `<prefix>_host_alloc` / `<prefix>_host_free`.  An array is asked for BEFORE the
+  step that fills it has made the engine's device the thread's current one, so the pool names it: memory taken under another would start a context there."""
   alloc_fn, free_fn = getattr(lib, prefix + "_host_alloc", None), getattr(lib, prefix + "_host_free", None)
 
   def alloc(size: int) -> Optional[int]:
     if alloc_fn is None:
       return None
     p = C.c_void_p()
-    return p.value if alloc_fn(C.c_int64(size), C.byref(p)) == 0 else None
+    return p.value if alloc_fn(C.c_int(device), C.c_int64(size), C.byref(p)) == 0 else None
 
-  return ResultPool(alloc, lambda addr: free_fn(C.c_void_p(addr)))
+  return ResultPool(alloc, lambda addr: free_fn(C.c_int(device), C.c_void_p(addr)))
