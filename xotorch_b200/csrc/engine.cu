@@ -961,8 +961,10 @@ const char* xotb200_version(void) { return "xotb200 0.1.0 sm_100a"; }
 
 int xotb200_host_alloc(int device, int64_t bytes, void** out) {
   REQUIRE(bytes > 0 && out, "bad argument");
-  CK(cudaSetDevice(device));   // a thread that has not chosen one yet would start a context on device 0
-  CK(cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable));
+  cudaError_t r = cudaSetDevice(device);   // a thread that has not chosen one yet would start a context on device 0
+  if (r == cudaSuccess) r = cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable);
+  if (r != cudaSuccess) cudaGetLastError();   // the caller goes on without: not an error of the next launch
+  CK(r);
   return 0;
 }
 int xotb200_host_free(int device, void* p) {
