@@ -1,7 +1,7 @@
 // flash_tc.cuh — prompt attention on the 5th-generation tensor cores (both engines): one CTA = 128 query rows of one request x one query head.
 //
 //   warp 0   one thread brings Q once and then the key / value tiles of 64 tokens by TMA (SWIZZLE_128B) into their rings;
-//   warp 1   one thread issues tcgen05.mma: S_j = Q K_j^T (128 x 64, fp32, tensor memory) one tile ahead, then O += P_j V_j with P read from tensor
+//   warp 1   one lane issues tcgen05.mma: S_j = Q K_j^T (128 x 64, fp32, tensor memory) one tile ahead, then O += P_j V_j with P read from tensor
 //            memory and V as it lies in memory ([token][value], the MN-major form of the B operand);
 //   warps 2-5  thread = query row: the row's 64 scores come by tcgen05.ld, so scale, soft cap, distance terms, mask, maximum and sum need no
 //            shuffle; the weights go back over the scores as the packed A operand of the value product.
@@ -156,6 +156,10 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   int jstart = ft_first_key(tl.pos0, a.window, a.chunk);
   if (a.page_table) jstart &= ~(FT_K - 1);           // a tile of paged keys lies in one page
   const int nt = (last - jstart) / FT_K + 1;
+  // Tokens of a tile that no row here sees (a request's last piece of a page, the next request's keys, what lies before a window) hold anything: their
+  // weight is 0, but 0 * Inf is not.  The rows of the value stage they lie in — `front` of the first tile, `behind` of the last — are zeroed before the
+  // product reads them (a row of a chunk is 128 bytes, swizzled within itself).
+  const int front = ft_first_key(tl.pos0, a.window, a.chunk) - jstart, behind = nt * FT_K - (last + 1 - jstart);
   if (threadIdx.x == 0) {
     *abort = 0;
     xb::mbar_init(q_full, 1);
@@ -205,16 +209,17 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ===== MMA issuer =====
-      constexpr uint32_t id_s = ft_idesc(FT_Q, FT_K, F16, false), id_o = ft_idesc(FT_Q, 64 * DVC, F16, true);
-      bool ok = ft_wait(q_full, 0, abort, a.err);
-      for (int j = 0; j <= nt && ok; ++j) {
-        if (j < nt) {
-          ok = ft_wait(&k_full[j % KS], (j / KS) & 1, abort, a.err);
-          if (ok && j >= 2) ok = ft_wait(&pv_done[j & 1], ((j - 2) >> 1) & 1, abort, a.err);   // the weights that lie over these scores have been used
-          if (!ok) break;
-          xb::tc_fence_after();
+    // ===== MMA issuer: lane 0; all lanes wait and zero unseen rows =====
+    constexpr uint32_t id_s = ft_idesc(FT_Q, FT_K, F16, false), id_o = ft_idesc(FT_Q, 64 * DVC, F16, true);
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, ft_wait(bar, parity, abort, a.err)); };
+    bool ok = wait(q_full, 0);
+    for (int j = 0; j <= nt && ok; ++j) {
+      if (j < nt) {
+        ok = wait(&k_full[j % KS], (j / KS) & 1);
+        if (ok && j >= 2) ok = wait(&pv_done[j & 1], ((j - 2) >> 1) & 1);   // the weights that lie over these scores have been used
+        if (!ok) break;
+        xb::tc_fence_after();
+        if (lane == 0) {
           const uint32_t sq = xb::smem_u32(qs), sk = xb::smem_u32(ks + (j % KS) * K_BYTES);
 #pragma unroll
           for (int c = 0; c < DKC; ++c)
@@ -224,12 +229,25 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           xb::umma_commit(&k_empty[j % KS]);
           xb::umma_commit(&s_full[j & 1]);
         }
-        if (j >= 1) {
-          const int i = j - 1;
-          ok = ft_wait(&p_full[i & 1], (i >> 1) & 1, abort, a.err) && ft_wait(&v_full[i % VS], (i / VS) & 1, abort, a.err);
-          if (!ok) break;
-          xb::tc_fence_after();
-          const uint32_t sv = xb::smem_u32(vs + (i % VS) * V_BYTES), p = tmem + (i & 1) * 64;
+        __syncwarp();
+      }
+      if (j >= 1) {
+        const int i = j - 1;
+        ok = wait(&p_full[i & 1], (i >> 1) & 1) && wait(&v_full[i % VS], (i / VS) & 1);
+        if (!ok) break;
+        uint8_t* vt = vs + (i % VS) * V_BYTES;
+        const int lead = i == 0 ? front : 0, rest = i == nt - 1 ? FT_K - behind : FT_K;   // rows [lead, rest) are seen
+        if (lead > 0 || rest < FT_K) {
+          for (int x = lane; x < (lead + FT_K - rest) * DVC * 8; x += 32) {
+            const int n = x / (DVC * 8), row = n < lead ? n : rest + n - lead;
+            *reinterpret_cast<uint4*>(vt + x / 8 % DVC * FT_K * 128 + row * 128 + x % 8 * 16) = make_uint4(0, 0, 0, 0);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+        }
+        xb::tc_fence_after();
+        if (lane == 0) {
+          const uint32_t sv = xb::smem_u32(vt), p = tmem + (i & 1) * 64;
 #pragma unroll
           for (int part = 0; part < (PAIR ? 2 : 1); ++part)
 #pragma unroll
@@ -237,6 +255,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           xb::umma_commit(&v_empty[i % VS]);
           xb::umma_commit(&pv_done[i & 1]);
         }
+        __syncwarp();
       }
     }
   } else {
@@ -249,21 +268,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const float* rel = a.rel ? a.rel + (size_t)h * a.rel_n : nullptr;
     float m = -INFINITY, den = 0.f;                  // reference of the exponentials (units of ln 2), sum of the weights
     bool ok = true;
-    // Tokens of a tile that no row here sees (a request's last piece of a page, the next request's keys, what lies before a window) hold anything: their
-    // weight is 0, but 0 * Inf is not.  Their rows of the value stage are zeroed before the product reads it (a row of a chunk is 128 bytes, swizzled
-    // within itself).
-    const int seen0 = ft_first_key(tl.pos0, a.window, a.chunk);
-    auto clear_unseen = [&](int j) -> bool {
-      const int j0 = jstart + j * FT_K, lead = min(max(seen0 - j0, 0), FT_K), rest = min(max(last + 1 - j0, 0), FT_K);   // rows [lead, rest) are seen
-      if (lead == 0 && rest == FT_K) return true;
-      if (!__all_sync(0xffffffffu, ft_wait(&v_full[j % VS], (j / VS) & 1, abort, a.err))) return false;
-      for (int i = r; i < (lead + FT_K - rest) * DVC * 8; i += 128) {
-        const int n = i / (DVC * 8), row = n < lead ? n : rest + n - lead, c = i / 8 % DVC;
-        *reinterpret_cast<uint4*>(vs + (j % VS) * V_BYTES + c * FT_K * 128 + row * 128 + i % 8 * 16) = make_uint4(0, 0, 0, 0);
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      return true;
-    };
     int j = 0;
     for (; j < nt; ++j) {
       // no row of this warp sees this tile or a later one: the warp's output is read before their products are added to it (0 * Inf again)
@@ -344,14 +348,20 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       tmem_st32(ts, hi);
       if constexpr (PAIR) tmem_st32(ts + 32, rest);
       tmem_st_wait();
-      ok = clear_unseen(j);
-      if (!ok) break;
       xb::tc_fence_before();
       mbar_arrive(&p_full[j & 1]);
     }
     if (ok) ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort, a.err));
     if (ok) {
       xb::tc_fence_after();
+      uint32_t o[2 * DVC][32];
+#pragma unroll
+      for (int c = 0; c < 2 * DVC; ++c) tmem_ld32(tm_o + lane_base + c * 32, o[c]);
+      for (; j < nt; ++j) {                          // tiles this warp sees nothing of: their products wait for all four warps
+        if (!__all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err))) break;
+        xb::tc_fence_before();
+        mbar_arrive(&p_full[j & 1]);
+      }
       float f = 1.0f;
       if (a.sink || a.sink_one) {
         const float sk = a.sink ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.sink)[h]) * LOG2E : 0.f, nm = fmaxf(m, sk);
@@ -363,14 +373,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const float* gt = a.gate_mode && r < tl.n_rows ? a.gate + row * a.gate_ld + a.gate_col0 + (a.gate_mode == 1 ? h : h * 64 * DVC) : nullptr;
       if (a.gate_mode == 1 && gt) f *= 1.0f / (1.0f + expf(-*gt));
       uint16_t* dst = static_cast<uint16_t*>(a.out) + (row * a.H + h) * (64 * DVC);
-#pragma unroll 1
-      for (int c = 0; c < 64 * DVC; c += 32) {
-        uint32_t o[32];
-        tmem_ld32(tm_o + lane_base + c, o);
-        if (r < tl.n_rows) {
+      if (r < tl.n_rows) {
+#pragma unroll
+        for (int c = 0; c < 64 * DVC; c += 32) {
           float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * f;
+          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[c / 32][i]) * f;
           if (a.gate_mode == 2) {
             const bool vec = ((reinterpret_cast<uintptr_t>(gt) | (uintptr_t)c) & 15) == 0;
 #pragma unroll
@@ -386,14 +394,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           for (int i = 0; i < 32; i += 8)
             *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(pack16<F16>(v[i], v[i + 1]), pack16<F16>(v[i + 2], v[i + 3]), pack16<F16>(v[i + 4], v[i + 5]), pack16<F16>(v[i + 6], v[i + 7]));
         }
-        __syncwarp();
       }
-      for (; j < nt; ++j) {                          // tiles this warp sees nothing of: the products wait for all four warps
-        ok = __all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err)) && clear_unseen(j);
-        if (!ok) break;
-        xb::tc_fence_before();
-        mbar_arrive(&p_full[j & 1]);
-      }
+      __syncwarp();
     }
   }
   xb::tc_fence_before();
