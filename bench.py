@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """bench.py — the driver's measurement contract for the shard-decode hot path.
 
-Metric (BASELINE.json): Llama-3-8B greedy decode tokens/sec (128-token prompt, 512 generated, batch 1) at N
+Metric: Llama-3-8B greedy decode tokens/sec (128-token prompt, 512 generated, batch 1) at N
 ring shards (one process per GPU, launched by torchrun for N>1), plus the mean inter-shard hop latency.
 
 A "step" is ONE request of the workload: a 128-token prefill (not timed, reported in `config`) followed by the timed
@@ -12,7 +12,7 @@ reference's Node drives (`forward(ids/hidden ndarray) -> ndarray`, i.e. `Inferen
 token copies its input host->device and its result (fp32 logits / hidden state) device->host inside the timed region.
 
 `python bench.py --impl reference` times the CPU restatement of the reference engine (oracle/, test infrastructure;
-the reference itself cannot be imported: torchtune is absent, SURVEY.md §8c) on the host cores — a bounded sample.
+the reference itself cannot be imported: torchtune is absent) on the host cores — a bounded sample.
 """
 from __future__ import annotations
 
@@ -31,7 +31,7 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 N_PROMPT, N_GEN = 128, 512
-TRAFFIC_FILE = ROOT / "profiles" / "r2_decode_ncu_traffic.json"   # written by tools/ncu_summarize.py from an `ncu --set full` capture of THIS build
+TRAFFIC_FILE = ROOT / "profiles" / "decode_ncu_traffic.json"   # written by tools/ncu_summarize.py from an `ncu --set full` capture of THIS build
 MODEL = "llama-3-8b"
 SEED = 1234
 
@@ -183,9 +183,9 @@ def workload_string(dtype_name: str) -> str:
 
 def run_reference(args):
   """`--impl reference`: the reference's own CPU implementation of the path.  The reference engine cannot be imported
-  (torchtune is absent here and on the box, SURVEY.md §8c), so this is the oracle port, timed on all usable host cores.
+  (torchtune is absent here and on the box), so this is the oracle port, timed on all usable host cores.
   A step = a bounded sample of the workload: `tok_per_step` consecutive decode tokens of the full-depth model (at least 32
-  timed tokens in total, BASELINE.md §4); W warm-up steps, then K timed steps; value = timed tokens / timed seconds."""
+  timed tokens in total); W warm-up steps, then K timed steps; value = timed tokens / timed seconds."""
   rank = int(os.environ.get("RANK", "0"))
   if rank != 0:
     return
@@ -198,7 +198,7 @@ def run_reference(args):
     avail = int([l for l in open("/proc/meminfo") if l.startswith("MemAvailable")][0].split()[1]) * 1024
   except Exception:
     avail = 1 << 62
-  if need > 0.7 * avail:       # 70B / Mixtral: the full model does not fit the host's RAM (SURVEY.md §8d: report n/a, do not extrapolate)
+  if need > 0.7 * avail:       # 70B / Mixtral: the full model does not fit the host's RAM (report n/a, do not extrapolate)
     print(json.dumps({"impl": "reference", "unavailable": f"{MODEL}: {need / 1e9:.0f} GB of weights do not fit the host's {avail / 1e9:.0f} GB of available RAM"}), flush=True)
     return
   steps, warm = max(1, args.steps), max(0, args.warmup)
@@ -357,7 +357,7 @@ def run_b200(args):
   d2h = (N_GEN + 1) * V * 4 + (n - 1) * N_PROMPT * D * 4
 
   # ---- requests in flight (N>1): B = N independent batch-1 requests interleaved through the ring, so every shard is busy.
-  #      Reported beside the headline, never instead of it: `value` stays the single-request metric BASELINE.json names. ----
+  #      Reported beside the headline, never instead of it: `value` stays the single-request metric. ----
   pipelined = None
   if n > 1:
     Bq, gen_q = min(n, 8), min(256, N_GEN)
@@ -371,7 +371,7 @@ def run_b200(args):
                  "unit": "tokens/s (all requests)", "per_request": round((gen_q - 1) / (ms_q * 1e-3), 2),
                  "how": "ring step s serves request s % B (own KV cache each, each still a batch-1 greedy stream); decode phase, CUDA events, max over ranks"}
 
-  # ---- roofline of the decode step (algorithmic bytes of SURVEY.md §8d / DESIGN.md, live CUDA-event time) ----
+  # ---- roofline of the decode step (algorithmic bytes, live CUDA-event time) ----
   peak, peak_src = _peaks()
   ctx_avg = N_PROMPT + (N_GEN - 1) / 2.0
   step_bytes_local = eng.step_bytes(int(round(ctx_avg)))
@@ -481,7 +481,7 @@ def main():
   ap.add_argument("--partition", default="bytes", choices=["bytes", "layers"], help="N>1: balance streamed bytes (default) or layer counts (reference rule)")
   ap.add_argument("--no-single-shard-check", action="store_true", help="N>1: skip re-running the request on ONE shard holding all layers")
   ap.add_argument("--no-ref-hop", action="store_true", help="--impl reference --gpus N>1: skip the reference gRPC hop comparator")
-  # the other BASELINE.json configs through the same contract (defaults = the headline config):
+  # the other configurations through the same contract (defaults = the headline config):
   #   --model llama-3-70b --gpus 8 --prompt 4096      (fp16, must shard to fit)     --model mixtral-8x7b --gpus 4
   from xotorch_b200.synth import PRESETS
   ap.add_argument("--model", default=MODEL, choices=sorted(k for k in PRESETS if not k.startswith("tiny")))

@@ -4,9 +4,9 @@
  * This is the drop-in boundary for xotorch's ONE hot path: the per-shard Llama-style decode/prefill step behind
  * `InferenceEngine.infer_tensor` and the inter-shard hidden-state hop behind `PeerHandle.send_tensor`.
  * The reference is pure Python and has no FFI for this path; the closest precedent is the external "Cheetah"
- * C++ service it talks to over a Unix socket (/root/reference/xotorch/inference/cheetah/sharded_inference_engine.py:331-457).
- * Each entry point below cites the reference interface it replaces (paths relative to /root/reference).
- * The ctypes binding a maintainer would add is xotorch_b200/_lib.py (shown in INTEGRATION.md).
+ * C++ service it talks to over a Unix socket (xotorch/inference/cheetah/sharded_inference_engine.py:331-457).
+ * Each entry point below cites the reference interface it replaces (paths within its project).
+ * The ctypes binding a maintainer would add is xotorch_b200/_lib.py.
  *
  * Conventions: every function returns 0 on success or a negative XOTB200_E* code; the message is available
  * from xotb200_last_error() (thread-local).  All pointers are plain host pointers unless the name says `dev`.
@@ -33,7 +33,7 @@ extern "C" {
 #define XOTB200_DTYPE_BF16 0
 #define XOTB200_DTYPE_F16 1 /* IEEE half weights / activations / KV (the 70B card upstream is fp16); fp32 accumulation as for bf16 */
 
-#define XOTB200_ROPE_PLAIN 0  /* RotaryPositionalEmbeddings (general_mha.py:57-63, and llama ids w/o rope_scaling: App. B3) */
+#define XOTB200_ROPE_PLAIN 0  /* RotaryPositionalEmbeddings (general_mha.py:57-63, and llama ids w/o rope_scaling) */
 #define XOTB200_ROPE_LLAMA3 1 /* Llama3ScaledRoPE (general_mha.py:33-40)                                              */
 
 /* Mirror of the dict built by load_model_config (xotorch/inference/llm_utils.py:79-126). */
@@ -51,7 +51,7 @@ typedef struct xotb200_model_cfg {
   int32_t tie_embeddings; /* tied lm_head (general_mha.py:42-44,125-126)  */
   int32_t dtype;          /* XOTB200_DTYPE_*                               */
   int32_t rope_kind;      /* XOTB200_ROPE_*                                */
-  float rope_factor;      /* HF rope_scaling.factor (App. B2)              */
+  float rope_factor;      /* HF rope_scaling.factor              */
   float rope_low_freq_factor;
   float rope_high_freq_factor;
   int32_t rope_old_context_len;
@@ -78,7 +78,7 @@ int xotb200_destroy(xotb200_engine* e);
 /* ---- shard selection + weights: replaces TorchDynamicShardInferenceEngine.ensure_shard -> start_model ->
  *      load_model_weights_torchtune (sharded_inference_engine.py:372-421; llm_utils.py:185-333).
  *      Inclusive layer range as in Shard (xotorch/inference/shard.py:4-39).  Embedding is held only by the first
- *      shard, final norm + lm_head only by the last (App. B6).  The loader is STRICT (App. B6). ---- */
+ *      shard, final norm + lm_head only by the last.  The loader is STRICT. ---- */
 int xotb200_set_shard(xotb200_engine* e, int start_layer, int end_layer);
 /* set_shard + read every *.safetensors in `dir` (HF names, HF layout; q/k re-laid out like _permute, llm_utils.py:175-183).
  * Streams: file mapping -> pinned double buffer (parallel copy) -> DMA -> re-layout kernel, chunk i+1 overlapping chunk i; strict:
@@ -93,11 +93,11 @@ int xotb200_check_loaded(xotb200_engine* e);
 
 /* ---- request state: replaces encode()'s state/KV reset + setup_cache
  *      (sharded_inference_engine.py:71-83,133-147) and ShardTransformerDecoder.setup_caches/reset_caches
- *      (llm_utils.py:369-414).  KV capacity comes from the request (App. B7). ---- */
+ *      (llm_utils.py:369-414).  KV capacity comes from the request. ---- */
 int xotb200_begin_request(xotb200_engine* e, int max_total_len);
 /* Several independent requests in flight through the ring (each keeps its own KV cache; each is still a batch-1 stream):
  * ring step s serves request s % n_requests at position pos0 + s / n_requests, so with n_requests >= number of shards
- * every GPU of the ring is busy all the time (SURVEY.md §8f.2; the reference keeps per-request state in Node but its engine
+ * every GPU of the ring is busy all the time (the reference keeps per-request state in Node but its engine
  * is single-request, sharded_inference_engine.py:250).  1 <= n_requests <= 8.  xotb200_forward / xotb200_post_to_next act on
  * the request chosen with xotb200_select_request (0 after begin_batch). */
 int xotb200_begin_batch(xotb200_engine* e, int max_total_len, int n_requests);
@@ -172,7 +172,7 @@ int xotb200_ring_wait(xotb200_engine* e, int32_t* tokens_out, int n_steps, float
  * existing engines, or that recovers from XOTB200_ETIMEOUT, continues from the maximum of this value over its engines. */
 int xotb200_ring_next_step(xotb200_engine* e, int* step);
 /* Per-step device timestamps (globaltimer ns) of the most recent ring run: t_in = input flag observed,
- * t_out = result posted.  Arrays of n_steps uint64 each (hop latency accounting, SURVEY.md §8d). */
+ * t_out = result posted.  Arrays of n_steps uint64 each (hop latency accounting). */
 int xotb200_ring_timestamps(xotb200_engine* e, uint64_t* t_in, uint64_t* t_out, int n_steps);
 
 /* ---- tuning / debugging ----

@@ -1,6 +1,5 @@
-"""TEST INFRASTRUCTURE: builds the oracle's C helpers (gcc only).  /root/reference is pure Python and its hot-path
-arithmetic lives in an absent third-party package (torchtune), so there is nothing to compile into oracle/_ref —
-see DESIGN.md "Oracle"."""
+"""TEST INFRASTRUCTURE: builds the oracle's C helpers (gcc only).  The reference is pure Python and its hot-path
+arithmetic lives in an absent third-party package (torchtune), so there is nothing to compile into oracle/_ref."""
 import subprocess
 from pathlib import Path
 

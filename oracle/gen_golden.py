@@ -5,7 +5,7 @@ A. oracle goldens: for each tiny preset, prompt ids, greedy ids, logits of the p
 B. reference-generated fixtures: the partitioning outputs of the REAL reference code
    (xotorch/topology/ring_memory_weighted_partitioning_strategy.py + partitioning_strategy.py), imported from
    /root/reference with a scapy stub, for the memories/layer counts our tests use.  Also the DummyInferenceEngine
-   behaviour through the reference's own InferenceEngine ABC (the boundary fixture, SURVEY.md §2 row 7).
+   behaviour through the reference's own InferenceEngine ABC (the boundary fixture).
 """
 import json
 import os
@@ -84,7 +84,7 @@ def part_b():
   sys.path.insert(0, str(ref))
   cwd = os.getcwd()
   with tempfile.TemporaryDirectory() as td:
-    os.chdir(td)   # device_capabilities.py writes a log file into the CWD (SURVEY.md §0.3)
+    os.chdir(td)   # device_capabilities.py writes a log file into the CWD
     sys.dont_write_bytecode = True
     from xotorch.topology.ring_memory_weighted_partitioning_strategy import RingMemoryWeightedPartitioningStrategy
     from xotorch.topology.partitioning_strategy import map_partitions_to_shards

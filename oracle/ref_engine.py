@@ -7,7 +7,7 @@ library.
 What this is
 ------------
 A torchtune-free restatement, in plain eager PyTorch on the CPU, of the reference's
-`TorchDynamicShardInferenceEngine` path (all citations relative to /root/reference):
+`TorchDynamicShardInferenceEngine` path (all citations by the path within its project):
 
 * config mapping            xotorch/inference/llm_utils.py:79-126          -> `load_model_config`
 * weight key map + _permute xotorch/inference/llm_utils.py:175-183,230-318 -> `permute_qk`, `RefShardModel.__init__`
@@ -20,13 +20,13 @@ A torchtune-free restatement, in plain eager PyTorch on the CPU, of the referenc
 
 The arithmetic itself lives in a third-party dependency that is absent here (torchtune >= 0.6.1, un-pinned,
 setup.py:41-68; `import torchtune` fails in this container and there is no network), so its published
-algorithm is restated from SURVEY.md Appendix A: RMSNorm (A.1), Llama3ScaledRoPE / RotaryPositionalEmbeddings
+algorithm is restated: RMSNorm (A.1), Llama3ScaledRoPE / RotaryPositionalEmbeddings
 (A.2), MultiHeadAttention with KVCache + GQA expand + masked SDPA over the whole cache (A.3-A.4),
 TransformerSelfAttentionLayer / FeedForward (A.5), `torchtune.generation.sample` (A.8).
 
 Pinning status ("how do we know the oracle is right")
 -----------------------------------------------------
-The reference holds NO golden logits / known-answer vectors for this path (SURVEY.md §4, §8c) and its own
+The reference holds NO golden logits / known-answer vectors for this path and its own
 implementation cannot be imported, so absolute numerical parity with *the reference* is **unpinned**.  What is
 pinned instead (tests/test_oracle.py, fixtures under tests/golden/, generator oracle/gen_golden.py):
   1. independent cross-check against HF transformers `LlamaForCausalLM` (half-split RoPE, un-permuted q/k) on
@@ -35,7 +35,7 @@ pinned instead (tests/test_oracle.py, fixtures under tests/golden/, generator or
      bit-exact;
   3. golden logits / ids of this oracle, committed, so later edits cannot drift silently.
 
-Deliberate deviations from reference *defects* (SURVEY.md Appendix B): B1 (a shard hands off the output of its
+Deliberate deviations from reference *defects*: B1 (a shard hands off the output of its
 last layer), B2/B3 (HF rope_scaling keys; un-scaled RoPE when rope_scaling is null so Llama-3-8B/70B build), B5
 (position is explicit).  Cost structure kept faithful for the CPU baseline: bf16 weights, KV cache of
 prompt+1024, full-length masked SDPA, per-step GQA K/V materialisation, fp32 logits, reference sampler at
@@ -104,7 +104,7 @@ def permute_qk(t: torch.Tensor, n_heads: int, head_dim: int, dim: int) -> torch.
 
 
 # --------------------------------------------------------------------------------------------------------------
-# torchtune semantics (SURVEY.md Appendix A)
+# torchtune semantics
 # --------------------------------------------------------------------------------------------------------------
 def rope_theta_llama3(dim: int, base: float, scale_factor: float, low_freq_factor: float = 1.0,
                       high_freq_factor: float = 4.0, old_context_len: int = 8192) -> torch.Tensor:
@@ -297,8 +297,8 @@ class RefShardModel:
   route_log: Optional[list] = None
 
   def _moe(self, L: dict, xm: torch.Tensor, layer: int = -1, input_pos: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Mixtral sparse-MoE MLP.  The reference has no MoE path (its `MOELayer`, llm_utils.py:502-590, is an unused stub:
-    SURVEY.md §0.10), so this restates the third-party algorithm the config names: HF transformers 5.5.0
+    """Mixtral sparse-MoE MLP.  The reference has no MoE path (its `MOELayer`, llm_utils.py:502-590, is an unused
+    stub), so this restates the third-party algorithm the config names: HF transformers 5.5.0
     models/mixtral/modeling_mixtral.py:101-116 (MixtralTopKRouter: linear -> fp32 softmax -> top-k -> renormalise) and
     :74-98 (MixtralExperts: per expert in ascending index, down(silu(gate x) * up x) * fp32 routing weight -> model dtype ->
     index_add_ into a model-dtype accumulator).  One deliberate pin: torch.topk leaves the order of EQUAL values
@@ -370,7 +370,7 @@ def ref_sample(logits: torch.Tensor, temperature: float = 1.0, top_k: Optional[i
 
 class RefEngine:
   """Synchronous mirror of TorchDynamicShardInferenceEngine (sharded_inference_engine.py:37-370) minus the
-  tokenizer/downloader: prompts are token ids (SURVEY.md §8d feeds `infer_tensor` ids directly)."""
+  tokenizer/downloader: prompts are token ids (`infer_tensor` is fed ids directly)."""
 
   def __init__(self, config: dict, weights: Dict[str, torch.Tensor], shard, dtype=None, norm_variant="old",
                max_generated_tokens: int = MAX_GENERATED_TOKENS):

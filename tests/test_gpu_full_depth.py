@@ -19,7 +19,8 @@ Greedy ids: the north star asks for bit-exact ids on the same prompt.  Two corre
 random-weight models (top-2 logit gaps below one bf16 ulp occur every few dozen steps), so the rule asserted here is the
 strongest one that is implementation-independent: at EVERY teacher-forced step whose oracle top-2 gap exceeds the logit
 tolerance the CUDA argmax equals the oracle's; the number of near-tie steps is reported; free-running ids are identical up
-to the first near-tie step.  Reports go to gpurun_out/parity_full_depth.json when that directory exists."""
+to the first near-tie step.  Reports go to parity_full_depth.json in the folder that
+XOTB200_TEST_REPORTS names, if any."""
 import json
 import os
 import time
@@ -37,9 +38,9 @@ ROOT = Path(__file__).resolve().parent.parent
 
 def _report(name: str, rec: dict):
   print(f"[parity] {name}: {json.dumps(rec)}")
-  d = ROOT / "gpurun_out"
-  if d.is_dir():
-    p = d / "parity_full_depth.json"
+  d = os.environ.get("XOTB200_TEST_REPORTS")
+  if d:
+    p = Path(d) / "parity_full_depth.json"
     try:
       cur = json.loads(p.read_text()) if p.exists() else {}
     except Exception:

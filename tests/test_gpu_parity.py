@@ -412,9 +412,9 @@ def test_streaming_loader_chunks_equal_device_synth_at_real_dims(tmp_path):
       os.environ.pop("XOTB200_LOAD_STREAM", None)
     assert np.array_equal(want[0], got[0]) and np.array_equal(want[1], got[1]), f"loader mode {mode}"
   print(f"[loader] {json.dumps(rates)}")
-  out = Path(__file__).resolve().parent.parent / "gpurun_out"
-  if out.is_dir():
-    (out / "loader_rates.json").write_text(json.dumps(rates, indent=1))
+  out = os.environ.get("XOTB200_TEST_REPORTS")
+  if out:
+    (Path(out) / "loader_rates.json").write_text(json.dumps(rates, indent=1))
 
 
 def _rewrite_safetensors(path, mutate):

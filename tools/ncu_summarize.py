@@ -1,9 +1,9 @@
 """Turn ncu output into the summaries kept under profiles/.
 
   launch list  : ncu --metrics gpu__time_duration.sum --clock-control none -c N --csv --log-file L.csv <cmd>
-                 python tools/ncu_summarize.py launches L.csv > profiles/<round>_launch_list_summary.txt
+                 python tools/ncu_summarize.py launches L.csv > profiles/<what>_launch_list_summary.txt
   full capture : ncu --set full --clock-control none -k regex:<kernels> -o R <cmd>
-                 ncu -i R.ncu-rep --page raw --csv > R.csv ; python tools/ncu_summarize.py full R.csv > profiles/<round>_ncu_full_metrics.txt
+                 ncu -i R.ncu-rep --page raw --csv > R.csv ; python tools/ncu_summarize.py full R.csv > profiles/<what>_ncu_full_metrics.txt
 (per-launch times under ncu are cold-cache and serialised: read the SHARES, not the absolutes — B200_PROFILING.md)"""
 import collections
 import csv
@@ -49,7 +49,7 @@ def full(path):
 
 
 def traffic(path, tokens, command):
-  """profiles/r2_decode_ncu_traffic.json (what bench.py reports as roofline.traffic): DRAM bytes per decoded token of the
+  """profiles/decode_ncu_traffic.json (what bench.py reports as roofline.traffic): DRAM bytes per decoded token of the
   persistent decode kernel = (dram__bytes_read.sum + dram__bytes_write.sum) of ONE launch / the tokens that launch decoded."""
   import json
   r = list(csv.reader(open(path)))
@@ -64,7 +64,7 @@ def traffic(path, tokens, command):
   out = {"bytes_per_token": int((rd + wr) / tokens), "dram_read_bytes": int(rd), "dram_write_bytes": int(wr), "tokens_in_launch": tokens,
          "kernel": row[h.index("Kernel Name")].split("(")[0], "duration_ms_under_ncu": round(dur * 1e3, 3), "command": command,
          "note": f"bytes per token = (dram__bytes_read.sum + dram__bytes_write.sum) / {tokens} tokens of one persistent-kernel launch, ncu --set full "
-                 f"--clock-control none of the committed build (profiles/r2_decode_ncu_full_metrics.txt)"}
+                 f"--clock-control none of the committed build"}
   print(json.dumps(out, indent=1))
 
 

@@ -1,5 +1,5 @@
-"""Same-box comparator for the hop number (SURVEY.md §8d last sentence): the REFERENCE's own hop —
-`GRPCPeerHandle.send_tensor` (/root/reference/xotorch/networking/grpc/grpc_peer_handle.py:111-130) into the reference's own
+"""Same-box comparator for the hop number: the REFERENCE's own hop —
+`GRPCPeerHandle.send_tensor` (xotorch/networking/grpc/grpc_peer_handle.py:111-130) into the reference's own
 `GRPCServer.SendTensor` (grpc_server.py:73-88) in a SECOND process on the same host (loopback), unmodified, from the package
 installed under baseline/_ref (or /root/reference in the build container) — timed next to the device hop bench.py reports.
 

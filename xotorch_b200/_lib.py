@@ -18,7 +18,7 @@ E_TIMEOUT = -5
 
 class ModelCfg(C.Structure):
   """xotb200_model_cfg — mirror of the dict built by load_model_config
-  (/root/reference/xotorch/inference/llm_utils.py:79-126)."""
+  (xotorch/inference/llm_utils.py:79-126)."""
   _fields_ = [
     ("n_layers", C.c_int32), ("dim", C.c_int32), ("ffn", C.c_int32), ("n_heads", C.c_int32),
     ("n_kv_heads", C.c_int32), ("head_dim", C.c_int32), ("vocab", C.c_int32), ("max_pos", C.c_int32),

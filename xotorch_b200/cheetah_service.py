@@ -1,5 +1,5 @@
-"""Cheetah-socket façade (SURVEY.md §3.5, §8f.4): a Unix-socket service that speaks the wire protocol of the reference's
-`CheetahInferenceEngine.run_cheetah` (/root/reference/xotorch/inference/cheetah/sharded_inference_engine.py:331-457) and
+"""Cheetah-socket façade: a Unix-socket service that speaks the wire protocol of the reference's
+`CheetahInferenceEngine.run_cheetah` (xotorch/inference/cheetah/sharded_inference_engine.py:331-457) and
 answers from libxotb200 — so upstream's Cheetah client can drive the B200 engine without any change on its side.  The
 reference ships only the CLIENT of that protocol (the C++ "Cheetah" service it talks to is not in the repository), so the
 server side here is written from the client's send/receive code:
@@ -17,7 +17,7 @@ server side here is written from the client's send/receive code:
 
 What the service keeps per (model_path, layer range): one engine; per session_id: the position — a hidden-state request
 carries no position at all, so the service counts the tokens each session has pushed through this shard (a token request
-states it in `input_pos`).  The mask is read and dropped: attention here touches only the valid prefix (SURVEY.md App. B7).
+states it in `input_pos`).  The mask is read and dropped: attention here touches only the valid prefix.
 Last shard: the reply is the last position's logits as [1, 1, V] (the client's `[:, -1]` yields the [1, V] it passes to
 `sample`); other shards: the hidden state [1, S, D].
 

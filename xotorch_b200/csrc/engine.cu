@@ -8,12 +8,12 @@
 // thread can issue only ~14 M bulk copies/s; with 4 KiB row-wise copies it could not outrun HBM).
 //   per layer: attn_norm[D] | Wqkv[(Hq+2Hkv)*hd, D] | Wo[D, Hq*hd] | mlp_norm[D] | Wgu[2F, D] | Wdown[D, F]
 //     Wqkv rows: q heads then k heads in interleaved-pair order (the reference's `_permute`,
-//       /root/reference/xotorch/inference/llm_utils.py:175-183) so a RoPE pair is two ADJACENT rows and the rotation
+//       xotorch/inference/llm_utils.py:175-183) so a RoPE pair is two ADJACENT rows and the rotation
 //       fuses into the GEMV epilogue; v rows unchanged.
 //     Wgu rows: gate_m, up_m interleaved so SwiGLU fuses into the epilogue.
 //     sparse MoE (Mixtral): Wgu / Wdown hold the E experts back to back (each in the same K-panel layout) + router[E, D].
 //   first shard: embed[V, D];  last shard: final_norm[D] | lm_head[V, D] (a second, K-panelled copy of embed when tied).
-//   KV cache: [request][local_layer][k|v][Hkv][L][hd] (same [Hkv, L, hd] order as torchtune KVCache, SURVEY.md App. A.4).
+//   KV cache: [request][local_layer][k|v][Hkv][L][hd] (same [Hkv, L, hd] order as torchtune KVCache).
 #include <cuda_runtime.h>
 #include <dirent.h>
 #include <fcntl.h>
@@ -42,8 +42,8 @@
 #include "flash_tc.cuh"
 #include "st_header.h"
 
-// Decode GEMV inner loop: 1 = mma.sync tensor-core path (default), 0 = the round-1 packed-FFMA2 loop (kept for A/B builds:
-// make EXTRA=-DXB_GEMV_MMA=0).  XB_TILE_STAMPS=1 adds per-tile timestamps to the debug timeline (tools/quick_bench.py).
+// Decode GEMV inner loop: 1 = mma.sync tensor-core path (default), 0 = the packed-FFMA2 loop (kept for A/B builds:
+// make EXTRA=-DXB_GEMV_MMA=0).  XB_TILE_STAMPS=1 adds per-tile timestamps to the debug timeline.
 #ifndef XB_GEMV_MMA
 #define XB_GEMV_MMA 1
 #endif
@@ -869,7 +869,7 @@ static int upload_slot(xotb200_engine* e, TensorSlot& s, const void* host) {
 }
 
 // --------------------------------------------------------------------------------------------------------------
-// Streaming shard loader (SURVEY.md §8f.4): safetensors file (mmap, page cache) -> pinned double buffer -> HBM.
+// Streaming shard loader: safetensors file (mmap, page cache) -> pinned double buffer -> HBM.
 // The reference reads every *.safetensors of the directory fully into host tensors and copies module by module
 // (llm_utils.py:205-218,230-318).  Here a tensor is cut into chunks of whole rows (<= STAGE_BYTES); worker threads copy chunk
 // i+1 from the mapping into pinned buffer B while chunk i goes pinned buffer A -> device (DMA at PCIe rate, no pageable bounce
@@ -1190,7 +1190,7 @@ int xotb200_load_shard(xotb200_engine* e, const char* dir, int start_layer, int 
   std::sort(files.begin(), files.end());
   if (files.empty()) { set_err("no *.safetensors in %s", dir); return XOTB200_EIO; }
   CK(cudaSetDevice(e->device));
-  const bool streaming = !(getenv("XOTB200_LOAD_STREAM") && atoi(getenv("XOTB200_LOAD_STREAM")) == 0);   // 0: the round-1 per-tensor path (A/B)
+  const bool streaming = !(getenv("XOTB200_LOAD_STREAM") && atoi(getenv("XOTB200_LOAD_STREAM")) == 0);   // 0: the per-tensor path (A/B)
   StreamLoader ld;
   if (streaming)
     if (int rc = ld.init(e)) return rc;
@@ -1218,7 +1218,7 @@ int xotb200_load_shard(xotb200_engine* e, const char* dir, int start_layer, int 
     for (auto it = hdr.begin(); rc == 0 && it != hdr.end(); ++it) {
       auto sl = e->slots.find(it->first);
       if (sl == e->slots.end()) {
-        // strict (SURVEY.md App. B6): a tensor of a layer this shard OWNS that has no slot (e.g. q_proj.bias of a biased-attention
+        // strict: a tensor of a layer this shard OWNS that has no slot (e.g. q_proj.bias of a biased-attention
         // checkpoint) would be silently ignored and give wrong logits -> refuse the checkpoint
         int l = -1;
         if (sscanf(it->first.c_str(), "model.layers.%d.", &l) == 1 && l >= e->start && l <= e->end &&
@@ -1320,7 +1320,7 @@ int xotb200_begin_batch(xotb200_engine* e, int max_total_len, int n_requests) {
   }
   if (e->route_log) CK(cudaMemsetAsync(e->route_log, 0xff, (size_t)e->L * nl * 4, e->stream));
   if (max_total_len > e->rope_len) {
-    // RoPE table (SURVEY.md App. A.2): theta_j in fp32, angle = fp32(pos * theta_j), cos/sin correctly rounded
+    // RoPE table: theta_j in fp32, angle = fp32(pos * theta_j), cos/sin correctly rounded
     const int half = c.head_dim / 2;
     std::vector<float> theta(half);
     for (int j = 0; j < half; ++j) {
@@ -1694,7 +1694,7 @@ int xotb200_ring_launch(xotb200_engine* e, int n_steps, int step0, int pos0) {
   return 0;
 }
 
-// Continuous batching (SURVEY.md §8f.2): a ring launch over an explicit set of ACTIVE requests, each with its own KV slot and its
+// Continuous batching: a ring launch over an explicit set of ACTIVE requests, each with its own KV slot and its
 // own position — requests join (after a prefill into a free slot) and leave between launches, the others keep their caches.
 int xotb200_ring_launch_slots(xotb200_engine* e, int n_steps, int step0, const int32_t* kv_slots, const int32_t* positions, int n_active) {
   REQUIRE(e && kv_slots && positions, "null argument");

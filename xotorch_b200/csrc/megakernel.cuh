@@ -2,8 +2,8 @@
 //
 // ONE launch runs `n_steps` consecutive steps (tokens) of a shard: for every step
 //     ingest -> { qkv -> attention -> o-proj -> gate/up -> down } x layers [-> lm_head + argmax] -> publish
-// replacing the reference's per-token Python/eager path (SURVEY.md §3.3;
-// /root/reference/xotorch/inference/llm_utils.py:416-489, general_mha.py:178-254, node.py:109-147,424-443).
+// replacing the reference's per-token Python/eager path
+// (xotorch/inference/llm_utils.py:416-489, general_mha.py:178-254, node.py:109-147,424-443).
 //
 // Why one kernel: at batch 1 every matrix is read exactly once per token, so the step is HBM-bound, but one
 // matrix is only 5-35 us of HBM time and a kernel boundary costs several us of drained memory pipe.  Here the

@@ -8,7 +8,7 @@
 //   * math: tcgen05.mma.cta_group::1.kind::f16 (bf16 x bf16 -> fp32), M=128, N=NT, K=16, issued by ONE thread,
 //     accumulator in tensor memory, completion via tcgen05.commit -> mbarrier
 //   * epilogue: 4 warps tcgen05.ld their 32 TMEM lanes (= 32 tokens), apply the fused epilogue (bf16 store / residual
-//     add / last-row logits) with the same rounding points as the decode kernel (SURVEY.md App. A.7)
+//     add / last-row logits) with the same rounding points as the decode kernel
 // Replaces the reference's prefill pass through torchtune modules (llm_utils.py:416-489 with S = prompt length;
 // sharded_inference_engine.py:108-193,230-370).  Around the GEMMs: RMSNorm, RoPE + KV append, causal attention over the
 // prompt, SwiGLU, arg-max — small row-parallel kernels.

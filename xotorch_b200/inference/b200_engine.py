@@ -1,12 +1,12 @@
 """`B200ShardInferenceEngine` — the drop-in replacement for `TorchDynamicShardInferenceEngine`
-(/root/reference/xotorch/inference/torch/sharded_inference_engine.py:37-424) on B200.
+(xotorch/inference/torch/sharded_inference_engine.py:37-424) on B200.
 
 Same public surface (`encode / sample / decode / infer_tensor / ensure_shard / load_checkpoint`, attributes `.shard`,
 `.tokenizer`, `.shard_downloader`), same ndim protocol (2 => int token ids [1,S], 3 => float32 hidden [1,S,D]; returns
 float32 hidden [1,S,D] or last-position logits [1,V]), same 1-thread executor discipline — but every FLOP runs in
 libxotb200.so through the C ABI (xotorch_b200/native.py).  There is no CPU fallback.
 
-Deliberate deviations from reference DEFECTS (SURVEY.md App. B): the inference_state that rides the ring is the tiny
+Deliberate deviations from reference DEFECTS: the inference_state that rides the ring is the tiny
 dict {"curr_pos": int} instead of the JSON-encoded L x L mask (B5/B11, §0.9); a shard hands off the output of its
 last layer (B1); KV capacity comes from the request (B7); strict weight loading (B6)."""
 from __future__ import annotations
@@ -31,7 +31,7 @@ MAX_GENERATED_TOKENS = 1024   # general_mha.py:152: KV length = prompt + 1024
 
 # Device-resident hop (xotb200_forward_hop): when the next shard's engine lives in this process (NVLinkPeerHandle), the
 # "tensor" a non-last shard returns — and PeerHandle.send_tensor carries — is this 4-word descriptor instead of the fp32
-# hidden state; the payload was stored into the next engine's HBM by the producing kernel (SURVEY.md §8b "Hop API").
+# hidden state; the payload was stored into the next engine's HBM by the producing kernel.
 HOP_MAGIC = 0x584F5442   # "XOTB"
 
 
@@ -47,7 +47,7 @@ def parse_hop_descriptor(x: np.ndarray):
 
 
 def reference_sample(logits: np.ndarray, temp: float, top_k: int, q: np.ndarray) -> np.ndarray:
-  """torchtune.generation.sample restated on host arrays (SURVEY.md App. A.8): /max(temp,1e-5), top-k mask,
+  """torchtune.generation.sample restated on host arrays: /max(temp,1e-5), top-k mask,
   softmax, argmax(probs / q).  `q` ~ Exp(1) noise.  Returns int32 [B,1]."""
   x = logits.astype(np.float32) / np.float32(max(temp, 1e-5))
   if top_k is not None:
@@ -271,7 +271,7 @@ class B200ShardInferenceEngine(InferenceEngine):
 
 def register_with_xotorch() -> bool:
   """Install this engine into an importable reference package (no plugin registry exists upstream: the factory is an
-  if/elif and model cards are keyed by engine CLASS NAME — SURVEY.md §8b).  Returns False if xotorch is absent."""
+  if/elif and model cards are keyed by engine CLASS NAME).  Returns False if xotorch is absent."""
   try:
     import xotorch.inference.inference_engine as ref_ie
     import xotorch.models as ref_models

@@ -1,5 +1,5 @@
 """Tokenizer resolution for a LOCAL model directory (no hub access on the B200 box).  Mirrors what the reference's
-engine keeps in `.tokenizer` (/root/reference/xotorch/inference/tokenizers.py:11-63): `.encode`, `.decode`,
+engine keeps in `.tokenizer` (xotorch/inference/tokenizers.py:11-63): `.encode`, `.decode`,
 `.eos_token_id`.  Synthetic model directories have no tokenizer files -> `IdTokenizer`."""
 from __future__ import annotations
 

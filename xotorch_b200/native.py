@@ -15,7 +15,7 @@ from ._lib import ModelCfg, check
 
 def cfg_from_hf(hf: dict) -> ModelCfg:
   """HF config.json dict -> xotb200_model_cfg, following load_model_config
-  (/root/reference/xotorch/inference/llm_utils.py:79-126) with App. B2/B3 fixed (HF rope_scaling keys; unscaled RoPE
+  (xotorch/inference/llm_utils.py:79-126) with two defects fixed (HF rope_scaling keys; unscaled RoPE
   when rope_scaling is null)."""
   dt = str(hf.get("torch_dtype", "bfloat16"))
   if dt in ("bfloat16", "bf16"):

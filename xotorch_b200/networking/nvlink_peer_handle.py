@@ -1,10 +1,10 @@
 """`NVLinkPeerHandle` — the PeerHandle for a peer whose engine lives in THIS process on a GPU of the same NVSwitch box
-(/root/reference/xotorch/networking/peer_handle.py:9-56; concrete signatures grpc_peer_handle.py:96-201; receiver side
+(xotorch/networking/peer_handle.py:9-56; concrete signatures grpc_peer_handle.py:96-201; receiver side
 grpc_server.py:73-88).  Injection point upstream: the `create_peer_handle` factory given to the discovery module
 (main.py:146,155).
 
 The reference moves every hop through gRPC + gzip + a JSON-encoded inference state (≈1.25 ms bare, ≈100 ms with its L x L
-mask; SURVEY.md §0.9).  Here `connect()` attaches the peer's engine to the local one (`attach_next_engine`): from then on a
+mask).  Here `connect()` attaches the peer's engine to the local one (`attach_next_engine`): from then on a
 non-last shard's `infer_tensor` runs `xotb200_forward_hop` — the last epilogue of its decode kernel stores the 16-bit hidden
 state straight into the peer engine's HBM over NVLink and releases a flag (a prompt is one peer copy) — and returns a
 4-word DESCRIPTOR instead of the hidden state.  `send_tensor` carries that descriptor to the peer `Node.process_tensor`
@@ -88,7 +88,7 @@ class NVLinkPeerHandle:
 
 
 class InProcessPeerHandle(NVLinkPeerHandle):
-  """The same handle with no local engine attached: every hop stays on host arrays (what round 1 shipped; kept for callers
+  """The same handle with no local engine attached: every hop stays on host arrays (kept for callers
   whose engines are not B200ShardInferenceEngine)."""
 
   def __init__(self, _id: str, node, desc: str = "in-process peer", device_capabilities=None, address: str = "inproc"):

@@ -1,7 +1,7 @@
 """Device-resident ring over the shards of one model on the GPUs of one box (single process, one engine per GPU).
 
 Replaces the per-token Node.forward_tensor -> PeerHandle.send_tensor hop
-(/root/reference/xotorch/orchestration/node.py:424-443) when every shard sits on the same NVSwitch box: after a
+(xotorch/orchestration/node.py:424-443) when every shard sits on the same NVSwitch box: after a
 prefill through the host API, `generate` launches ONE persistent kernel per shard; activations and the argmax token
 travel between the engines' inboxes over NVLink (peer stores + release/acquire flags), the host only collects the ids.
 bench.py does the same across processes (torchrun) with CUDA-IPC mapped inboxes."""
@@ -300,7 +300,7 @@ class DistributedRing:
       self.step = s0 + n_steps                # also on XOTB200_ETIMEOUT: the numbers of a failed run stay burnt
     return toks, ms
 
-  # -- B requests in flight (SURVEY.md §8f.2): ring step s serves request s % B; with B >= world no GPU idles ------------
+  # -- B requests in flight: ring step s serves request s % B; with B >= world no GPU idles ------------
   def generate_batch(self, prompts: np.ndarray, n_gen: int) -> Tuple[Optional[np.ndarray], float]:
     """prompts [B, S] (same on every rank).  Prefill per request through the host-array path, then ONE persistent kernel
     per rank for B*(n_gen-1) ring steps.  Returns (ids [B, n_gen] on the last rank | None, device ms of this rank)."""

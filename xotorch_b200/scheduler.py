@@ -1,8 +1,8 @@
-"""Continuous batching over the device-resident ring + the `Node.on_token` bridge (SURVEY.md §8f.2).
+"""Continuous batching over the device-resident ring + the `Node.on_token` bridge.
 
 The reference schedules every token from Python: `Node.process_inference_result` samples on the last shard, checks EOS /
 max tokens, fires `on_token.trigger_all(request_id, [token], is_finished)` and forwards the id to the first shard
-(/root/reference/xotorch/orchestration/node.py:109-147); its engine holds ONE request.  Here the per-token loop lives in the
+(xotorch/orchestration/node.py:109-147); its engine holds ONE request.  Here the per-token loop lives in the
 persistent kernels (xotorch_b200/ring.py) and this module is what remains on the host:
 
 * `ContinuousRing` — a request table over the B KV caches of `xotb200_begin_batch`.  Requests are admitted while others are

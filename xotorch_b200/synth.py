@@ -1,6 +1,6 @@
 """Synthetic Llama-style model directories (HF layout) with counter-based, bit-reproducible weights.
 
-No real checkpoints exist on the build or GPU boxes (SURVEY.md §0.4, §8d), so every parity and bench run
+No real checkpoints exist on the build or GPU boxes, so every parity and bench run
 uses weights from this generator.  The generator is *counter based* (splitmix64 of
 ``seed, tensor_id, flat_index``) and uses only integer arithmetic plus one fp32 multiply and one fp32 add,
 so the very same values can be produced on the host (here, torch int64 ops) and on the device
@@ -8,7 +8,7 @@ so the very same values can be produced on the host (here, torch int64 ops) and 
 8B bench.  Values are Irwin-Hall(4) ~ N(mean, std^2), rounded to bf16/fp16 (round-nearest-even).
 
 The HF tensor names / shapes follow what the reference's loader consumes
-(/root/reference/xotorch/inference/llm_utils.py:230-318, key map in SURVEY.md App. A.6).
+(xotorch/inference/llm_utils.py:230-318).
 """
 from __future__ import annotations
 
@@ -94,7 +94,7 @@ class ModelShape:
 _LLAMA32_SCALING = {"factor": 32.0, "high_freq_factor": 4.0, "low_freq_factor": 1.0,
                     "original_max_position_embeddings": 8192, "rope_type": "llama3"}
 
-# Constants from SURVEY.md Appendix C.
+# Published shapes of the models.
 PRESETS: Dict[str, ModelShape] = {
   # tiny parity shapes (oracle runs in milliseconds)
   "tiny-llama-hd64": ModelShape("tiny-llama-hd64", 4, 512, 1536, 8, 2, 64, 2048, max_pos=2048),
@@ -107,7 +107,7 @@ PRESETS: Dict[str, ModelShape] = {
                              rope_scaling=dict(_LLAMA32_SCALING)),
   "llama-3-8b": ModelShape("llama-3-8b", 32, 4096, 14336, 32, 8, 128, 128256),
   "llama-3-70b": ModelShape("llama-3-70b", 80, 8192, 28672, 64, 8, 128, 128256, dtype="float16"),
-  # Mixtral-style sparse MoE MLP (SURVEY.md §8f.3, App. C): router + top-2 of 8 SwiGLU experts
+  # Mixtral-style sparse MoE MLP: router + top-2 of 8 SwiGLU experts
   "tiny-mixtral": ModelShape("tiny-mixtral", 4, 512, 1024, 8, 2, 64, 2048, rope_theta=1e6, max_pos=2048, n_experts=8, top_k=2),
   "tiny-mixtral-hd128": ModelShape("tiny-mixtral-hd128", 3, 1024, 2048, 8, 2, 128, 4096, rope_theta=1e6, max_pos=2048,
                                    n_experts=4, top_k=2),
@@ -153,7 +153,7 @@ def shape_from_hf_config(cfg: dict, name: str = "model") -> ModelShape:
     n_experts=int(cfg.get("num_local_experts") or 0), top_k=int(cfg.get("num_experts_per_tok") or 0))
 
 
-W_STD = 0.02  # SURVEY.md §8(d): weights ~ N(0, 0.02^2), norm scales = 1 + N(0, 0.02^2)
+W_STD = 0.02  # weights ~ N(0, 0.02^2), norm scales = 1 + N(0, 0.02^2)
 
 
 def hf_tensor_specs(shape: ModelShape, layers: Optional[Iterable[int]] = None,
@@ -230,6 +230,6 @@ def write_hf_dir(path: os.PathLike, shape: ModelShape, seed: int = 1234, n_files
 
 
 def synth_prompt(vocab: int, n: int = 128, seed: int = 42) -> np.ndarray:
-  """SURVEY.md §8(d): prompt = n random ids from Generator(seed 42); returned as int32 [1, n]."""
+  """prompt = n random ids from Generator(seed 42); returned as int32 [1, n]."""
   g = torch.Generator().manual_seed(seed)
   return torch.randint(0, vocab, (1, n), generator=g).to(torch.int32).numpy()

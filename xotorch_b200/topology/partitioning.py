@@ -2,15 +2,15 @@
 layer ranges and the reference's golden vectors hold (tests/test_partitioning.py):
 
 * `RingMemoryWeightedPartitioningStrategy.partition`
-    /root/reference/xotorch/topology/ring_memory_weighted_partitioning_strategy.py:7-18
+    xotorch/topology/ring_memory_weighted_partitioning_strategy.py:7-18
   nodes ordered by (memory, id) descending; each gets the fraction memory/total; running end rounded to 5 decimals.
 * `map_partitions_to_shards`
-    /root/reference/xotorch/topology/partitioning_strategy.py:24-42
+    xotorch/topology/partitioning_strategy.py:24-42
   layers [int(start*n), int(end*n)-1]; the last partition is forced to end at n-1; empty ranges are dropped.
 
 `HBMWeightedRingPartitioningStrategy` is the B200 flavour: `memory` is what the GPU can actually give to weights +
 KV (free HBM from cudaMemGetInfo / NVML, in MB like DeviceCapabilities.memory), one logical node per GPU (the
-reference reports a multi-GPU host as ONE node with summed memory, device_capabilities.py:215-257 — App. B10).
+reference reports a multi-GPU host as ONE node with summed memory, device_capabilities.py:215-257).
 Works on the reference's `Topology` (duck-typed: `.all_nodes()` yielding `(node_id, caps)` with `caps.memory`)
 or on a plain `{node_id: memory}` dict.
 """
@@ -69,7 +69,7 @@ class HBMWeightedRingPartitioningStrategy(RingMemoryWeightedPartitioningStrategy
 
 def model_stream_bytes(hf_config: dict) -> Tuple[int, int]:
   """(bytes one decoder layer streams per decoded token, bytes the last shard streams on top: final norm + lm_head), 16-bit
-  weights, from an HF config.json dict — SURVEY.md §8d's per-token byte formula (sparse MoE: the active experts only)."""
+  weights, from an HF config.json dict (sparse MoE: the active experts only)."""
   D, F = hf_config["hidden_size"], hf_config["intermediate_size"]
   Hq, Hkv = hf_config["num_attention_heads"], hf_config["num_key_value_heads"]
   hd = hf_config.get("head_dim") or D // Hq
@@ -83,7 +83,7 @@ def model_stream_bytes(hf_config: dict) -> Tuple[int, int]:
 class ByteBalancedRingPartitioningStrategy(RingMemoryWeightedPartitioningStrategy):
   """Ring partition that balances the BYTES A SHARD STREAMS PER TOKEN (= its decode time on an HBM-bound engine) instead of
   the layer count: the last shard also streams final norm + lm_head (1.05 GB for Llama-3-8B = 2.4 decoder layers), so under
-  the reference rule it sets the period of a ring with several requests in flight (SURVEY.md §8e; 8B on 8 GPUs: 2.79 GB vs
+  the reference rule it sets the period of a ring with several requests in flight (8B on 8 GPUs: 2.79 GB vs
   1.74 GB elsewhere).  Same node order as the reference ((memory, id) descending) and the same `Partition` fractions ->
   `map_partitions_to_shards` pipeline, so every node still derives the same ranges; node i's share of the bytes is its share
   of the memory.  Boundaries are whole layers: cumulative byte target T_i -> the layer count nearest to it (each node keeps
@@ -142,7 +142,7 @@ def map_partitions_to_shards(partitions: List[Partition], num_layers: int, model
 
 
 def shard_for(node_id: str, topology, num_layers: int, model_id: str, strategy: PartitioningStrategy | None = None) -> Shard:
-  """What Node.get_current_shard does (/root/reference/xotorch/orchestration/node.py:455-460)."""
+  """What Node.get_current_shard does (xotorch/orchestration/node.py:455-460)."""
   parts = (strategy or RingMemoryWeightedPartitioningStrategy()).partition(topology)
   shards = map_partitions_to_shards(parts, num_layers, model_id)
   idx = [p.node_id for p in parts].index(node_id)
