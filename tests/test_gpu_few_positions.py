@@ -111,3 +111,43 @@ def test_a_long_cache_is_left_to_the_decode_kernel():
   for n, pos0, gemms in ((2, 0, True), (2, 300, True), (2, 2040, False), (3, 2040, False), (7, 2040, True), (8, 2040, True), (1, 0, False)):
     assert (launches(n, pos0) > 1) == gemms, (n, pos0)
   eng.close()
+
+
+def test_without_memory_for_the_scratch_of_the_gemms():
+  """the decode kernel takes the call, as it needs no scratch; once there is memory the GEMMs do"""
+  from dataclasses import replace
+  runtime = pytest.importorskip("cuda.bindings.runtime")
+  from xotorch_b200.native import NativeShard
+  shape = replace(PRESETS["llama-3-8b"], name="llama-3-8b-cut", n_layers=3)
+  eng = NativeShard(hf_config(shape), 0)
+  eng.set_shard(1, 1)
+  eng.init_synthetic(5)
+  eng.begin_request(16)
+  h = torch.randn(5, shape.dim, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+  out = torch.empty_like(h)
+
+  def call():
+    before = eng.kernel_launches()
+    torch.cuda.synchronize()
+    eng.forward_device(None, h.data_ptr(), 5, 0, out.data_ptr())
+    return eng.kernel_launches() - before
+  eng.set_prefill_mode(1)
+  call()
+  ref = out.clone()
+  eng.set_prefill_mode(0)
+  held = []
+  try:
+    for size in (8 << 30, 1 << 30, 64 << 20, 2 << 20):
+      while True:
+        err, p = runtime.cudaMalloc(size)
+        if err != runtime.cudaError_t.cudaSuccess:
+          runtime.cudaGetLastError()
+          break
+        held.append(p)
+    out.zero_()
+    assert call() == 1 and torch.equal(out, ref)
+  finally:
+    for p in held:
+      runtime.cudaFree(p)
+  assert call() > 1
+  eng.close()

@@ -1422,11 +1422,14 @@ static bool gemms_pay(const xotb200_engine* e, int n_tokens, int pos0) {
   const int waves = (n_tokens * c.n_heads + 2 * e->sm_count - 1) / (2 * e->sm_count);
   return 31.0 + weight_bytes / 7.4e6 + waves * keys * (0.0056 + 0.000244 * c.head_dim) <= n_tokens * (21.0 + weight_bytes / 6.9e6 + keys * kv_bytes / 1.6e6);
 }
-static bool runs_as_gemms(const xotb200_engine* e, int n_tokens, int pos0) {
+static bool runs_as_gemms(xotb200_engine* e, int n_tokens, int pos0) {
   if (e->prefill_mode != 0) return e->prefill_mode == 2;
   if (n_tokens >= TC_FEW) return true;
   if (n_tokens < 2 || e->cfg.n_experts > 0 || !gemms_pay(e, n_tokens, pos0)) return false;
-  return !e->last || e->cfg.vocab % 64 == 0;   // the head as a GEMM has no tile for other vocabularies (prompts of TC_FEW positions or more are refused there)
+  if (e->last && e->cfg.vocab % 64 != 0) return false;   // the head as a GEMM has no tile for them (prompts of TC_FEW positions or more are refused there)
+  if (prepare_tc(e, n_tokens) == 0) return true;
+  cudaGetLastError();                                    // no memory for the GEMMs' scratch: the decode kernel needs none
+  return false;
 }
 
 int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidden_f32, int n_tokens, int pos0,
