@@ -185,6 +185,8 @@ int xotb200_set_prefill_mode(xotb200_engine* e, int mode);
 /* Unit-test hook for the tensor-core GEMM: out[S,N] (bf16 bits) = A[S,K] * W[N,K]^T with fp32 accumulation, W re-laid out
  * as K-panels of width tk exactly like a model weight.  S <= 128. */
 int xotb200_debug_gemm(xotb200_engine* e, const void* a_bf16, const void* w_bf16, int S, int N, int K, int tk, void* out_bf16);
+/* Unit-test hook: the device error word, as a bounded wait that expired would leave it (1, 2: a flag or a barrier; 3 and up: a prompt's pipelines). */
+int xotb200_debug_set_error(xotb200_engine* e, int code);
 /* Sparse-MoE shards: the experts the router chose for request 0 at positions [0, n_positions) of the open request,
  * out[pos * n_local_layers + local_layer] = lower expert | higher expert << 8 (-1 = position not run).  Parity tests use it
  * to tell a routing near-tie (a discrete, legitimately implementation-dependent choice) from an arithmetic error. */

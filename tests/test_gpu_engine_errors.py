@@ -1,4 +1,5 @@
-"""A cache that does not fit leaves the engine without a request — steps are refused — and a smaller one can be begun afterwards."""
+"""Errors that an engine comes back from.  A cache that does not fit leaves it without a request — steps are refused — and a smaller one can be begun afterwards;
+page-locked memory that cannot be had; a prompt whose pipelines gave up a wait."""
 from dataclasses import replace
 
 import numpy as np
@@ -51,4 +52,29 @@ def test_page_locked_memory_that_cannot_be_had(layered):
   eng.results = library_pool(eng.lib, "xotb200_lm" if layered else "xotb200", 99)
   assert eng.results._alloc(1 << 20) is None
   assert np.isfinite(step()).all()
+  eng.close()
+
+
+@pytest.mark.parametrize("n", [5, 100])
+def test_a_pipeline_wait_that_expired_is_reported_by_the_call_it_spoilt(n):
+  """the error word is set as an expired wait would leave it; prompts whose hidden state stays on the device report it too, once"""
+  import torch
+  from xotorch_b200._lib import check
+  from xotorch_b200.native import NativeShard
+  shape = PRESETS["tiny-llama-hd64"]
+  eng = NativeShard(hf_config(shape), 0)
+  eng.set_shard(1, 2)
+  eng.init_synthetic(4)
+  eng.begin_request(128)
+  h = torch.randn(n, shape.dim, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+  out = torch.empty_like(h)
+  torch.cuda.synchronize()
+  call = lambda: eng.forward_device(None, h.data_ptr(), n, 0, out.data_ptr())
+  call()
+  ref = out.clone()
+  check(eng.lib.xotb200_debug_set_error(eng.h, 3))
+  with pytest.raises(XotB200Error, match="pipeline wait"):
+    call()
+  call()
+  assert torch.equal(out, ref)
   eng.close()

@@ -71,6 +71,7 @@ _SIGS = {
   "xotb200_ring_timestamps": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int]),
   "xotb200_set_cta_limit": (C.c_int, [C.c_void_p, C.c_int]),
   "xotb200_set_prefill_mode": (C.c_int, [C.c_void_p, C.c_int]),
+  "xotb200_debug_set_error": (C.c_int, [C.c_void_p, C.c_int]),
   "xotb200_debug_gemm": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p]),
   "xotb200_debug_routing": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32), C.c_int]),
   "xotb200_debug_timeline": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_int]),

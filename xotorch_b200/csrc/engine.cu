@@ -196,6 +196,7 @@ struct xotb200_engine {
   int max_inflight = 0;            // decode producer window (bulk copies in flight per CTA, 0 = ring depth)
   unsigned int pace_q = 0;         // decode producer pacing, 2^-16 ns per byte per CTA (0 = off)
   bool tc_fuse = true;             // RoPE/KV-append and SwiGLU fused into GEMM epilogues (XOTB200_TC_FUSE=0: separate kernels, A/B)
+  int* gemm_err = nullptr;         // page-locked word that a prompt's kernels write when a pipeline wait expires: read behind the call's own synchronisation, without a copy
   int prefill_mode = 0;            // 0 auto (runs_as_gemms), 1 always the decode kernel, 2 always TC
   bf16 *tc_x = nullptr, *tc_xn = nullptr, *tc_qkv = nullptr, *tc_q = nullptr, *tc_ao = nullptr, *tc_gu = nullptr, *tc_act = nullptr;
   ActMaps tm_xn, tm_ao, tm_act;
@@ -487,7 +488,7 @@ static int launch_tc_stream_nb(xotb200_engine* e, const CUtensorMap& tmW, const 
 }
 static int launch_tc_stream(xotb200_engine* e, const CUtensorMap& tmW, const ActMaps& x, const TcGemmArgs& a_in, int epi, cudaStream_t st) {
   TcGemmArgs a = a_in;
-  a.err = &e->ctl->err;
+  a.err = e->gemm_err;
   const int nb = epi == TCE_HEAD_LAST || a.S <= 16 ? 16 : a.S <= 32 ? 32 : a.S <= 64 ? 64 : 128, tiles = a.N / TC_M, nkb = a.K / TC_BK;
   int s = 1;
   while (s < 8 && tiles * s * 2 <= (nb >= 128 ? 1 : 2) * e->sm_count && nkb >= 4 * s) s *= 2;
@@ -532,7 +533,7 @@ static int launch_tc_gemm_persistent(xotb200_engine* e, const CUtensorMap& tmA, 
 template <int NT, int NS>
 static int launch_tc_gemm_2sm(xotb200_engine* e, const CUtensorMap& tmA, const CUtensorMap& tmB_half, const TcGemmArgs& a_in, int epi, cudaStream_t st) {
   TcGemmArgs a = a_in;
-  a.err = &e->ctl->err;
+  a.err = e->gemm_err;
   void (*fn)(CUtensorMap, CUtensorMap, TcGemmArgs) = nullptr;
   const bool f16 = e->cfg.dtype == XOTB200_DTYPE_F16;
   switch (epi) {
@@ -551,7 +552,7 @@ static int launch_tc_gemm_2sm(xotb200_engine* e, const CUtensorMap& tmA, const C
 static int launch_tc_gemm(xotb200_engine* e, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcGemmArgs& a_in, int epi, TcCfg c,
                           cudaStream_t st) {
   TcGemmArgs a = a_in;
-  a.err = &e->ctl->err;
+  a.err = e->gemm_err;
   REQUIRE(a.N % c.nt == 0 && a.K % TC_BK == 0, "tensor-core GEMM needs N %% %d == 0 and K %% 64 == 0 (N=%d K=%d)", c.nt, a.N, a.K);
   {
     static const bool persist = !(getenv("XOTB200_TC_PERSIST") && atoi(getenv("XOTB200_TC_PERSIST")) == 0);
@@ -710,7 +711,7 @@ static int launch_tc_flash(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, 
   if (int rc = make_tmap_heads(&mk, kc, HD, 1, (long)e->cfg.n_kv_heads * e->L, xf::FT_K)) return rc;
   if (int rc = make_tmap_heads(&mv, vc, HD, 1, (long)e->cfg.n_kv_heads * e->L, xf::FT_K)) return rc;
   xf::FlashArgs a = {};
-  a.n_rows = S; a.pos0 = pos0; a.H = Hq; a.rep = R; a.head_rows = e->L; a.k2_from = HD / 64; a.scale = 1.0f / sqrtf((float)HD); a.out = e->tc_ao; a.err = &e->ctl->err;
+  a.n_rows = S; a.pos0 = pos0; a.H = Hq; a.rep = R; a.head_rows = e->L; a.k2_from = HD / 64; a.scale = 1.0f / sqrtf((float)HD); a.out = e->tc_ao; a.err = e->gemm_err;
   auto fn = e->cfg.dtype == XOTB200_DTYPE_F16 ? xf::flash_tc_kernel<HD / 64, HD / 64, false, true> : xf::flash_tc_kernel<HD / 64, HD / 64, false, false>;
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, xf::ft_smem_bytes(HD / 64, HD / 64))) return rc;
   return launch_early(e, st, fn, dim3(Hq, (S + xf::FT_Q - 1) / xf::FT_Q), xf::FT_THREADS, xf::ft_smem_bytes(HD / 64, HD / 64), 1, mq, mk, mk, mv, a);
@@ -1016,6 +1017,8 @@ int xotb200_create(const xotb200_model_cfg* cfg, int device, xotb200_engine** ou
   CK(cudaMalloc(&e->bar_counter, 4));
   CK(cudaMalloc(&e->ctl, sizeof(StepCtl)));
   MEMSET_SYNC(e, e->ctl, 0, sizeof(StepCtl));
+  CK(cudaHostAlloc(&e->gemm_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+  *e->gemm_err = 0;
   const size_t inbox_bytes = sizeof(InboxHdr) + (size_t)(INBOX_SLOTS + API_SLOTS) * D * 2;
   CK(cudaMalloc(&e->inbox, inbox_bytes));
   MEMSET_SYNC(e, e->inbox, 0, inbox_bytes);
@@ -1054,6 +1057,7 @@ int xotb200_destroy(xotb200_engine* e) {
   for (bf16* p : e->hop_buf)
     if (p) cudaFree(p);
   if (e->tok_count_host) cudaFreeHost(const_cast<unsigned int*>(e->tok_count_host));
+  if (e->gemm_err) cudaFreeHost(e->gemm_err);
   void* ptrs[] = {e->d_req_map, e->d_pos_tab, e->x, e->q, e->attn_out, e->act, e->logits, e->part_ml, e->part_acc, e->tickets, e->cta_best_val,
                   e->cta_best_idx, e->ctl, e->bar_counter, e->dbg, e->inbox, e->tokens_log, e->t_in, e->t_out, e->rope, e->stage_tokens,
                   e->stage_f32, e->stage_in, e->stage_out};
@@ -1380,17 +1384,26 @@ int xotb200_select_request(xotb200_engine* e, int request) {
   return 0;
 }
 
-// sticky device-side error word -> status code (3: a bounded wait inside the persistent tensor-core GEMM expired)
+// sticky device-side error word -> status code
 static int check_device_error(xotb200_engine* e) {
   StepCtl h;
   CK(cudaMemcpyAsync(&h, e->ctl, sizeof(h), cudaMemcpyDeviceToHost, e->stream));
   CK(cudaStreamSynchronize(e->stream));
   if (h.err) {
     MEMSET_SYNC(e, &e->ctl->err, 0, 4);
-    set_err(h.err == 3 ? "tensor-core GEMM: a pipeline wait expired (device error %d)" : "device-side wait timed out (device error %d)", h.err);
+    set_err("device-side wait timed out (device error %d)", h.err);
     return XOTB200_ETIMEOUT;
   }
   return 0;
+}
+
+// the same for the kernels of a prompt, behind the synchronisation that ends the call
+static int check_gemm_error(xotb200_engine* e) {
+  const int err = *static_cast<volatile int*>(e->gemm_err);
+  if (err == 0) return 0;
+  *e->gemm_err = 0;
+  set_err("tensor-core GEMM: a pipeline wait expired (device error %d)", err);
+  return XOTB200_ETIMEOUT;
 }
 
 static int ensure_staging(xotb200_engine* e, int n) {
@@ -1472,8 +1485,10 @@ int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidde
     CK(cudaMemcpyAsync(out_f32, e->stage_f32, (size_t)n_tokens * D * 4, cudaMemcpyDeviceToHost, st));
   }
   CK(cudaStreamSynchronize(st));
-  if (use_tc)
+  if (use_tc) {
+    if (int rc = check_gemm_error(e)) return rc;
     if (int rc = check_device_error(e)) return rc;
+  }
   e->have_result = true;
   return 0;
 }
@@ -1516,6 +1531,8 @@ int xotb200_forward_device(xotb200_engine* e, const int32_t* tokens, const void*
   if (e->last) CK(cudaMemcpyAsync(logits_f32, e->logits, (size_t)e->cfg.vocab * 4, cudaMemcpyDeviceToHost, st));
   else if (!use_tc) CK(cudaMemcpyAsync(out_hidden_dev, e->stage_out, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
   CK(cudaStreamSynchronize(st));
+  if (use_tc)
+    if (int rc = check_gemm_error(e)) return rc;
   e->have_result = true;
   return 0;
 }
@@ -1574,6 +1591,8 @@ int xotb200_forward_hop(xotb200_engine* e, const int32_t* tokens, int64_t seq_in
   if (e->last) {
     CK(cudaMemcpyAsync(logits_f32, e->logits, (size_t)e->cfg.vocab * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    if (use_tc)
+      if (int r = check_gemm_error(e)) return r;
   } else {
     if (!decode) {
       xotb200_engine* nx = e->next_engine;
@@ -1591,6 +1610,8 @@ int xotb200_forward_hop(xotb200_engine* e, const int32_t* tokens, int64_t seq_in
       }
       CK(cudaMemcpyPeerAsync(nx->hop_buf[slot], nx->device, e->stage_out, e->device, (size_t)n_tokens * D * 2, st));
       CK(cudaStreamSynchronize(st));
+      if (use_tc)
+        if (int r = check_gemm_error(e)) return r;
     }
     *seq_out = (int64_t)seq;
   }
@@ -1806,6 +1827,14 @@ int xotb200_set_cta_limit(xotb200_engine* e, int max_ctas) {
 int xotb200_set_prefill_mode(xotb200_engine* e, int mode) {
   REQUIRE(e && mode >= 0 && mode <= 2, "prefill mode must be 0 (auto), 1 (decode kernel) or 2 (tensor cores)");
   e->prefill_mode = mode;
+  return 0;
+}
+
+int xotb200_debug_set_error(xotb200_engine* e, int code) {
+  REQUIRE(e, "null argument");
+  CK(cudaSetDevice(e->device));
+  if (code >= 3) *e->gemm_err = code;
+  else MEMCPY_SYNC(e, &e->ctl->err, &code, sizeof(code), cudaMemcpyHostToDevice);
   return 0;
 }
 

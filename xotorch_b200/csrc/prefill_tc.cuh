@@ -47,7 +47,7 @@ struct TcGemmArgs {
   bf16 *kc, *vc;          // K / V cache of (request, layer): [Hkv][L][hd]
   const float2* rope;     // [L][hd/2] (cos, sin)
   int q_rows, kv_rows, hd, L, pos0;
-  int* err;               // sticky device error word (StepCtl::err): 3 = a bounded wait of the persistent GEMM expired
+  int* err;               // error word in page-locked host memory: 3 = a bounded wait expired
 };
 
 __host__ __device__ constexpr int tc_stage_bytes(int nt) { return TC_M * TC_BK * 2 + nt * TC_BK * 2; }
