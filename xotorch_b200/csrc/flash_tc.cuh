@@ -270,7 +270,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     bool ok = true;
     int j = 0;
     for (; j < nt; ++j) {
-      // no row of this warp sees this tile or a later one: the warp's output is read before their products are added to it (0 * Inf again)
+      // no row of this warp sees this tile or a later one: the warp's output is taken out before their products are added to it (0 * Inf again)
       if (jstart + j * FT_K > pos - lane + 31) break;
       ok = __all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err));
       if (!ok) break;
@@ -352,16 +352,26 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       mbar_arrive(&p_full[j & 1]);
     }
     if (ok) ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort, a.err));
-    if (ok) {
+    if (ok && j < nt) {                              // tiles this warp sees nothing of: it keeps its output while their products, which wait for all four warps, run
       xb::tc_fence_after();
       uint32_t o[2 * DVC][32];
 #pragma unroll
       for (int c = 0; c < 2 * DVC; ++c) tmem_ld32(tm_o + lane_base + c * 32, o[c]);
-      for (; j < nt; ++j) {                          // tiles this warp sees nothing of: their products wait for all four warps
-        if (!__all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err))) break;
+      for (; j < nt && ok; ++j) {
+        ok = __all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err));
         xb::tc_fence_before();
-        mbar_arrive(&p_full[j & 1]);
+        if (ok) mbar_arrive(&p_full[j & 1]);
       }
+      if (ok) ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(nt - 1) & 1], ((nt - 1) >> 1) & 1, abort, a.err));
+      if (ok) {
+        xb::tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < 2 * DVC; ++c) tmem_st32(tm_o + lane_base + c * 32, o[c]);
+        tmem_st_wait();
+      }
+    }
+    if (ok) {
+      xb::tc_fence_after();
       float f = 1.0f;
       if (a.sink || a.sink_one) {
         const float sk = a.sink ? __bfloat162float(static_cast<const __nv_bfloat16*>(a.sink)[h]) * LOG2E : 0.f, nm = fmaxf(m, sk);
@@ -373,12 +383,14 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const float* gt = a.gate_mode && r < tl.n_rows ? a.gate + row * a.gate_ld + a.gate_col0 + (a.gate_mode == 1 ? h : h * 64 * DVC) : nullptr;
       if (a.gate_mode == 1 && gt) f *= 1.0f / (1.0f + expf(-*gt));
       uint16_t* dst = static_cast<uint16_t*>(a.out) + (row * a.H + h) * (64 * DVC);
-      if (r < tl.n_rows) {
-#pragma unroll
-        for (int c = 0; c < 64 * DVC; c += 32) {
+#pragma unroll 1   // with few tiles fetching the code counts (requests in portions of 64 rows: 8720 us a pass, 8990 with this loop unrolled)
+      for (int c = 0; c < 64 * DVC; c += 32) {
+        uint32_t o[32];
+        tmem_ld32(tm_o + lane_base + c, o);
+        if (r < tl.n_rows) {
           float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[c / 32][i]) * f;
+          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * f;
           if (a.gate_mode == 2) {
             const bool vec = ((reinterpret_cast<uintptr_t>(gt) | (uintptr_t)c) & 15) == 0;
 #pragma unroll
@@ -394,8 +406,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           for (int i = 0; i < 32; i += 8)
             *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(pack16<F16>(v[i], v[i + 1]), pack16<F16>(v[i + 2], v[i + 3]), pack16<F16>(v[i + 4], v[i + 5]), pack16<F16>(v[i + 6], v[i + 7]));
         }
+        __syncwarp();
       }
-      __syncwarp();
     }
   }
   xb::tc_fence_before();
