@@ -1,0 +1,85 @@
+"""The two ends of a step: index arrays and page table entries come in, logits, argmax and the error word go out through page-locked memory that the kernels
+read and write.  Wherever the caller's logits lie — a block of the library's page-locked memory, somebody else's page-locked memory, ordinary memory, nowhere —
+a step must leave the same bits there, at vocabularies that one block takes, that a cluster shares, and whose rows are not whole 16-byte pieces."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from tests import fekanex_oracle as fo, fekanex_util as fu, layered_util as lu, zokuvik_oracle as zo
+from xotorch_b200 import _lib
+
+
+def address(a):
+  return a.__array_interface__["data"][0]
+
+
+def step_into(eng, slots, rows, want, logits_at):
+  """one step through the C entry: argmax"""
+  ints = lambda v: np.ascontiguousarray(v, dtype=np.int32)               # noqa: E731
+  sl, counts, tok, wn, am = ints(slots), ints([len(r) for r in rows]), ints(np.concatenate(rows)), ints(want), np.full(len(want), -1, np.int32)
+  _lib.check_lm(eng.lib.xotb200_lm_step(eng.h, len(slots), address(sl), address(counts), address(tok), None, address(wn), len(want), logits_at, address(am), None))
+  return am
+
+
+@pytest.mark.parametrize("scaled", [False, True])
+@pytest.mark.parametrize("vocab", [70, 4095, 4096, 5003, 32004])
+def test_logits_in_every_kind_of_memory(vocab, scaled):
+  if scaled:                                           # logits are changed on their way out
+    cfg = fu.config([fu.attn(heads=2, kv_heads=1, dim=16, vdim=16)], width=64, vocab=vocab)
+    cfg["logit_scale"] = 0.25
+    eng = lu.make_engine(cfg, fo.random_weights(cfg, 3), "bfloat16", max_tokens=256, max_requests=3)
+  else:
+    cfg = lu.config([lu.attn()], vocab=vocab)
+    eng = lu.make_engine(cfg, zo.random_weights(cfg, 3), "bfloat16", max_tokens=256, max_requests=3)
+  schedule = [([0, 1, 2], [[1, 2, 3], [4, 5], [6]], [0, 2, 5])] + [([0, 1, 2], [[7 + s], [8 + s], [9 + s]], [0, 1, 2]) for s in range(4)] + [([1], [[5]], [0])]
+
+  def serve(kind):
+    for r in range(3):
+      eng.clear_request(r)
+    out = []
+    for slots, rows, want in schedule:
+      n = len(want) * vocab
+      if kind == "block":
+        p = C.c_void_p()
+        _lib.check_lm(eng.lib.xotb200_lm_host_alloc(0, n * 4 + 64, C.byref(p)))
+        buf = np.frombuffer((C.c_float * (n + 16)).from_address(p.value), dtype=np.float32)
+      else:
+        buf = torch.zeros(n + 16, pin_memory=kind == "foreign").numpy()
+      buf[:] = 7.0
+      am = step_into(eng, slots, [np.array(r) for r in rows], want, None if kind == "nowhere" else address(buf))
+      got = buf[:n].copy().reshape(len(want), vocab)
+      assert (buf[n if kind != "nowhere" else 0:] == 7.0).all()              # nothing beyond
+      if kind == "block":
+        del buf
+        _lib.check_lm(eng.lib.xotb200_lm_host_free(0, p))
+      out.append((got, am))
+    return out
+
+  ref = serve("plain")
+  for got, am in ref:
+    assert np.isfinite(got).all() and np.array_equal(am, got.argmax(axis=1))
+  for kind in ("block", "foreign", "nowhere", "block"):
+    for (a, ia), (b, ib) in zip(ref, serve(kind)):
+      assert np.array_equal(ia, ib), kind
+      assert kind == "nowhere" or np.array_equal(a, b), kind
+  eng.close()
+
+
+def test_pages_added_by_single_row_and_by_mixed_steps():
+  """pages of 4 tokens: every few steps some of the requests start a page, in steps of one row each (replayed) and in steps of several"""
+  cfg = lu.config([lu.attn(), lu.attn("latent_attention_2", window=6)])
+  w = zo.random_weights(cfg, 9)
+  out = []
+  for page in (4, 64):
+    eng = lu.make_engine(cfg, w, "float32", max_tokens=200, max_requests=3, page_size=page)
+    rng, got = np.random.default_rng(1), []
+    for s in range(24):
+      rows = [rng.integers(0, 80, size=1 if s % 5 else 1 + 3 * r) for r in range(3)]
+      got.append(eng.step([2, 0, 1], rows)[0])
+    out.append(np.stack(got))
+    eng.close()
+  assert np.array_equal(out[0], out[1])

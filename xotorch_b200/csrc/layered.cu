@@ -22,6 +22,7 @@
 #include <array>
 #include <type_traits>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -33,6 +34,7 @@
 #include "layered_tc.cuh"
 #include "layered_stream.cuh"
 #include "layered_fma.cuh"
+#include "layered_step.cuh"
 #include "flash_tc.cuh"
 #include "st_header.h"
 
@@ -147,6 +149,7 @@ struct xotb200_lm {
   std::vector<int> free_pages, slot_len, slot_pages;
   int* h_table = nullptr;                              // pinned [max_requests, pages_per_slot]
   int* d_table = nullptr;
+  bool table_stale = false;                            // a step that failed has left page table entries on the host alone
   float* state = nullptr;                              // [max_requests][state_floats]
   size_t state_floats = 0;
   // per-step staging
@@ -1031,7 +1034,7 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
     drop_graphs(e);
     const size_t w = (size_t)std::max(n_want, 16);
     TRY(regrow(e->hw, w * D * e->esz));
-    TRY(regrow(e->logits, (w * ((size_t)e->cfg.vocab + 1) + 1) * 4));   // with the rows' argmax and the error word behind them
+    TRY(regrow(e->logits, w * e->cfg.vocab * 4));
     e->want_cap = (int)w;
   }
   if (e->trace && e->trace_cap < (size_t)e->layers.size() * e->m_cap * D) {
@@ -1697,9 +1700,9 @@ static int run_mixer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
 
 static int finish_logits(xotb200_lm* e, int n_want) {
   const float scale = e->cfg.logit_scale != 0.f ? e->cfg.logit_scale : 1.0f;
-  // the rows' results and the error word lie behind the logits: [n_want, vocab] fp32, [n_want] int, one int
-  int* tail = reinterpret_cast<int*>(e->logits + (size_t)n_want * e->cfg.vocab);
-  return launch_early(e, argmax_rows_kernel, n_want, 1024, 0, 1, e->logits, e->cfg.vocab, scale, e->cfg.logit_softcap, tail, e->d_err);
+  const int parts = e->cfg.vocab >= 4096 ? 8 : 1;       // blocks (a cluster) to a row
+  return launch_early(e, finish_rows_kernel, dim3(parts, n_want), 512, 0, parts, e->logits, e->cfg.vocab, scale, e->cfg.logit_softcap,
+                      reinterpret_cast<const StepOut*>(e->d_stage), e->d_err);
 }
 
 // How a block holds a row of D entries in registers: pieces of four per thread (nv of them, 1, 2 or 4; 0 = the row is not whole pieces or too long,
@@ -2026,17 +2029,36 @@ extern "C" {
 const char* xotb200_lm_last_error(void) { return g_err; }
 const char* xotb200_lm_version(void) { return "xotb200_lm 0.1.0 sm_100a"; }
 
+// page-locked blocks handed out and not yet given back: start -> bytes
+static std::mutex g_blocks_lock;
+static std::map<uintptr_t, size_t> g_blocks;
+static bool in_host_block(const void* p, size_t bytes) {
+  std::lock_guard<std::mutex> lock(g_blocks_lock);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  auto it = g_blocks.upper_bound(a);
+  if (it == g_blocks.begin()) return false;
+  --it;
+  return a + bytes <= it->first + it->second;
+}
+
 int xotb200_lm_host_alloc(int device, int64_t bytes, void** out) {
   REQUIRE(bytes > 0 && out, "bad argument");
   cudaError_t r = cudaSetDevice(device);   // a thread that has not chosen one yet would start a context on device 0
   if (r == cudaSuccess) r = cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable);
   if (r != cudaSuccess) cudaGetLastError();   // the caller goes on without: not an error of the next launch
   CK(r);
+  std::lock_guard<std::mutex> lock(g_blocks_lock);
+  g_blocks[reinterpret_cast<uintptr_t>(*out)] = (size_t)bytes;
   return 0;
 }
 int xotb200_lm_host_free(int device, void* p) {
   CK(cudaSetDevice(device));
-  if (p) CK(cudaFreeHost(p));
+  if (!p) return 0;
+  {
+    std::lock_guard<std::mutex> lock(g_blocks_lock);
+    g_blocks.erase(reinterpret_cast<uintptr_t>(p));
+  }
+  CK(cudaFreeHost(p));
   return 0;
 }
 
@@ -2364,6 +2386,7 @@ int xotb200_lm_begin(xotb200_lm* e, int max_tokens, int max_requests, int page_s
   memset(e->h_table, 0, tab * 4);
   CK(cudaMalloc(&e->d_table, tab * 4));
   CK(cudaMemsetAsync(e->d_table, 0, tab * 4, e->stream));
+  e->table_stale = false;
   if (e->state_floats) {
     CK(cudaMalloc(&e->state, (size_t)max_requests * e->state_floats * 4));
     CK(cudaMemsetAsync(e->state, 0, (size_t)max_requests * e->state_floats * 4, e->stream));
@@ -2431,6 +2454,10 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   TRY(ensure_scratch(e, (int)M, n_want));
   e->early = M <= LST_MAX_ROWS;
   TRY(refresh_tables(e));
+  if (e->table_stale) {
+    CK(cudaMemcpy(e->d_table, e->h_table, (size_t)e->max_requests * e->pages_per_slot * 4, cudaMemcpyHostToDevice));
+    e->table_stale = false;
+  }
   // ---- commit: pages and lengths; the step's index arrays are built in one host vector and copied once
   const bool use_flash = e->esz == 2 && e->flash_on && e->flash_fits;
   std::vector<int> qpis, windows;
@@ -2445,7 +2472,13 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     }
   std::vector<int>& st = e->stage_build;
   const bool bigram = e->first && e->cfg.bigram_buckets > 0;
-  st.assign(3 * (size_t)M + n_want, 0);
+  // [StepOut][tokens M][slots M][positions M][wanted rows], lists, and last the page table entries that the step adds: at most one per request when every
+  // request brings one row, so that such steps have one layout
+  constexpr int T0 = STEP_OUT_INTS;
+  st.assign(T0 + 3 * (size_t)M + n_want, 0);
+  const int page_cap = M == n_seq ? n_seq : need_pages;
+  std::vector<int> new_pages(2 * (size_t)page_cap, -1);
+  int n_new = 0;
   std::vector<int> bg(bigram ? M : 0);
   std::vector<Item> seqs(n_seq);
   StepPlan sp;
@@ -2455,13 +2488,13 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   for (int i = 0; i < n_seq; ++i) {
     const int sl = slots[i], len0 = e->slot_len[sl], len1 = len0 + counts[i];
     const int np0 = e->slot_pages[sl], np1 = cdiv(len1, P);
-    for (int p = np0; p < np1; ++p) {
-      e->h_table[(size_t)sl * e->pages_per_slot + p] = e->free_pages.back();
+    for (int p = np0; p < np1; ++p, ++n_new) {
+      const size_t at = (size_t)sl * e->pages_per_slot + p;
+      e->h_table[at] = e->free_pages.back();
       e->free_pages.pop_back();
+      new_pages[2 * (size_t)n_new] = (int)at;
+      new_pages[2 * (size_t)n_new + 1] = e->h_table[at];
     }
-    if (np1 > np0)
-      CK(cudaMemcpyAsync(e->d_table + (size_t)sl * e->pages_per_slot + np0, e->h_table + (size_t)sl * e->pages_per_slot + np0, (size_t)(np1 - np0) * 4,
-                         cudaMemcpyHostToDevice, e->stream));
     e->slot_pages[sl] = np1;
     e->slot_len[sl] = len1;
     seqs[i] = Item{row, counts[i], sl, len0};
@@ -2472,14 +2505,15 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
         const int64_t B = e->cfg.bigram_buckets, prev = t > 0 ? tokens[row - 1] : e->slot_last[sl];
         bg[row] = len0 + t == 0 ? (int)B : (int)((prev * (e->cfg.bigram_mul_prev % B) + tokens[row] * (e->cfg.bigram_mul_cur % B)) % B);
       }
-      st[row] = e->first ? tokens[row] : 0;
-      st[M + row] = sl;
-      st[2 * M + row] = len0 + t;
+      st[T0 + row] = e->first ? tokens[row] : 0;
+      st[T0 + M + row] = sl;
+      st[T0 + 2 * M + row] = len0 + t;
     }
   }
   if (e->first)
     for (int i = 0; i < n_seq; ++i) e->slot_last[slots[i]] = tokens[seqs[i].row0 + counts[i] - 1];
-  for (int w = 0; w < n_want; ++w) st[3 * M + w] = want_rows[w];
+  for (int w = 0; w < n_want; ++w) st[T0 + 3 * M + w] = want_rows[w];
+  e->table_stale = n_new > 0;                            // until the step has run
   auto push = [&](const void* p, size_t n_ints) { const size_t o = st.size(); const int* q = static_cast<const int*>(p); st.insert(st.end(), q, q + n_ints); return o; };
   const size_t off_seqs = push(seqs.data(), 4 * (size_t)n_seq), off_bigram = push(bg.data(), bg.size());
   auto is_long = [&](int i) { return use_flash && counts[i] >= FLASH_MIN_ROWS; };
@@ -2541,6 +2575,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     TRY(regrow(e->vxx, cap * e->max_oh * 2));
     e->flash_keys_cap = cap;
   }
+  const size_t pages_off = push(new_pages.data(), new_pages.size());
   const size_t off = st.size();
   if (off > e->stage_cap) {
     drop_graphs(e);
@@ -2553,17 +2588,23 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     CK(cudaMalloc(&e->d_stage, cap * 4));
     e->stage_cap = cap;
   }
-  memcpy(e->h_stage, st.data(), off * 4);
   const bool results = e->last && n_want > 0;
-  // page-locked output memory takes the results directly
-  bool direct = false;
-  if (float* dst = e->last ? logits_f32 : hidden_out_f32) {
+  // Page-locked output memory takes the results directly: logits by the last kernel's own stores where the memory is a block of this library's (its bounds are
+  // known: a store past registered memory would fault), hidden states and logits into anybody else's by DMA.
+  const bool own_block = results && logits_f32 && in_host_block(logits_f32, (size_t)n_want * V * 4);
+  bool direct = own_block;
+  if (float* dst = own_block ? nullptr : e->last ? logits_f32 : hidden_out_f32) {
     cudaPointerAttributes at;
     direct = (results || !e->last) && cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
     cudaGetLastError();                                  // a pointer the runtime cannot classify is ordinary memory
   }
   if (results) TRY(ensure_host_out(e, (size_t)n_want * V + n_want + 1));
   else if (!e->last) TRY(ensure_host_out(e, (size_t)M * (D + e->carry_out)));
+  if (results) {
+    const StepOut so{!logits_f32 ? nullptr : own_block ? logits_f32 : direct ? e->logits : e->h_out, reinterpret_cast<int*>(e->h_out + (size_t)n_want * V)};
+    memcpy(st.data(), &so, sizeof(so));
+  }
+  memcpy(e->h_stage, st.data(), off * 4);
   // Decoding — every request brings one row — has the same launches step after step: only the contents of the index arrays and
   // the lengths differ.  Such a step is captured into a CUDA graph the second time its shape is seen and replayed from then on.
   // What the launches depend on is in the key; the key length is a bucket of the longest request (it fixes how the absorbed
@@ -2602,11 +2643,13 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     if (capture) CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed));
     int rc = 0;
     auto body = [&]() -> int {
-      CK(cudaMemcpyAsync(e->d_stage, e->h_stage, off * 4, cudaMemcpyHostToDevice, e->stream));
-      sp.tokens = e->d_stage;
-      sp.row_slot = e->d_stage + M;
-      sp.row_pos = e->d_stage + 2 * M;
-      sp.want = e->d_stage + 3 * M;
+      const int n16 = cdiv((long)off, 4);
+      TRY(launch_late(e, stage_in_kernel, cdiv(std::max(n16, page_cap), 256), 256, 0, reinterpret_cast<const int4*>(e->h_stage), reinterpret_cast<int4*>(e->d_stage), n16,
+                      (int)pages_off, page_cap, e->d_table));
+      sp.tokens = e->d_stage + T0;
+      sp.row_slot = e->d_stage + T0 + M;
+      sp.row_pos = e->d_stage + T0 + 2 * M;
+      sp.want = e->d_stage + T0 + 3 * M;
       sp.bigram_row = e->d_stage + off_bigram;
       sp.seqs = reinterpret_cast<const Item*>(e->d_stage + off_seqs);
       for (auto& kv : item_off) sp.items[kv.first] = {reinterpret_cast<const Item*>(e->d_stage + kv.second.first), kv.second.second};
@@ -2649,21 +2692,19 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     }
     if (rc < 0) { cudaStreamSynchronize(e->stream); return rc; }
   }
-  // What goes to the caller is copied behind the (replayed) kernels and is not part of a captured step: the caller's pointer is another one each time.
+  // What is copied to the caller is copied behind the (replayed) kernels and is not part of a captured step: the caller's pointer is another one each time
+  // (the last kernel of a step reads its pointers from the staged block).
   if (!e->last) {
     const size_t ld = (size_t)D + e->carry_out;
     float* dst = direct ? hidden_out_f32 : e->h_out;
     TRY(copy_rows(dst, ld, e->x, D, D, cudaMemcpyDeviceToHost));
     if (e->carry_out) TRY(copy_rows(dst + D, ld, e->vfirst, e->carry_out, e->carry_out, cudaMemcpyDeviceToHost));
-  } else if (results) {
-    // the argmax and the error word lie behind the logits; one copy when the logits go through the staging buffer or are not asked for
-    const size_t n = (size_t)n_want * V;
-    if (direct) CK(cudaMemcpyAsync(logits_f32, e->logits, n * 4, cudaMemcpyDeviceToHost, e->stream));
-    const size_t skip = direct || !logits_f32 ? n : 0;
-    CK(cudaMemcpyAsync(e->h_out + skip, e->logits + skip, (n + n_want + 1 - skip) * 4, cudaMemcpyDeviceToHost, e->stream));
+  } else if (results && direct && !own_block) {
+    CK(cudaMemcpyAsync(logits_f32, e->logits, (size_t)n_want * V * 4, cudaMemcpyDeviceToHost, e->stream));
   }
   CK(cudaEventRecord(e->ev1, e->stream));
   CK(cudaStreamSynchronize(e->stream));
+  e->table_stale = false;
   CK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
   const int err = results ? reinterpret_cast<const int*>(e->h_out)[(size_t)n_want * V + n_want] : *e->h_err;
   if (err != 0) {

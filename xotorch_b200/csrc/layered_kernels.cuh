@@ -1176,63 +1176,6 @@ gemv_rows_kernel(const TA* __restrict__ A, long lda, long a_batch, const TB* __r
   }
 }
 
-// finishes the logits of every row in place — l <- l * scale, then l <- cap * tanh(l / cap) when cap > 0 — and takes the
-// lowest-index argmax of the row (greedy sampling on the device)
-// also hands the step's error word on behind the rows' results, so that all of them reach the host in one copy
-__global__ void argmax_rows_kernel(float* __restrict__ logits, int V, float scale, float cap, int* __restrict__ out, const int* __restrict__ err) {
-  pdl_enter();
-  __shared__ float bv[32];
-  __shared__ int bi[32];
-  float* r = logits + (size_t)blockIdx.x * V;
-  float best = -INFINITY;
-  int idx = 0x7fffffff;
-  auto finish = [&](float v) { v *= scale; return cap > 0.f ? cap * tanhf(v / cap) : v; };
-  auto take = [&](float v, int i) { if (v > best || (v == best && i < idx)) { best = v; idx = i; } };
-  const bool change = scale != 1.0f || cap > 0.f;
-  constexpr int NV = 4;                                        // 16-byte loads in flight per thread: one block reads a row (32000 entries: 12 us with single loads)
-  int done = 0;
-  if (((reinterpret_cast<uintptr_t>(r)) & 15) == 0) {
-    done = V & ~3;
-    for (int i0 = threadIdx.x * 4; i0 < done; i0 += blockDim.x * 4 * NV) {
-      float4 q[NV];
-#pragma unroll
-      for (int u = 0; u < NV; ++u) {
-        const int i = i0 + u * (int)blockDim.x * 4;
-        if (i < done) q[u] = *reinterpret_cast<const float4*>(r + i);
-      }
-#pragma unroll
-      for (int u = 0; u < NV; ++u) {
-        const int i = i0 + u * (int)blockDim.x * 4;
-        if (i >= done) continue;
-        if (change) {
-          q[u] = make_float4(finish(q[u].x), finish(q[u].y), finish(q[u].z), finish(q[u].w));
-          *reinterpret_cast<float4*>(r + i) = q[u];
-        }
-        take(q[u].x, i); take(q[u].y, i + 1); take(q[u].z, i + 2); take(q[u].w, i + 3);
-      }
-    }
-  }
-  for (int i = done + threadIdx.x; i < V; i += blockDim.x) {
-    float v = r[i];
-    if (change) r[i] = v = finish(v);
-    take(v, i);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (ov > best || (ov == best && oi < idx)) { best = ov; idx = oi; }
-  }
-  if ((threadIdx.x & 31) == 0) { bv[threadIdx.x >> 5] = best; bi[threadIdx.x >> 5] = idx; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-      if (bv[w] > best || (bv[w] == best && bi[w] < idx)) { best = bv[w]; idx = bi[w]; }
-    out[blockIdx.x] = idx;
-    if (blockIdx.x == 0) out[gridDim.x] = *err;
-  }
-}
-
 // weights arrive as bf16 bit patterns: widen (or copy) rows into their place in the T-typed blob
 template <typename T>
 __global__ void store_rows_kernel(const bf16* __restrict__ src, T* __restrict__ dst, size_t n) {
