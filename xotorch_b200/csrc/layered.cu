@@ -144,6 +144,7 @@ struct xotb200_lm {
   float* pos_freqs = nullptr;                          // [ceil(width / 2)] frequencies of the computed position vector (device)
   bool tables_stale = true;                            // tables derived from weights (learned distance bias) have to be remade
   std::map<std::string, Dest> dests;
+  bool all_loaded = false;
   // request state
   int max_requests = 0, page_size = 0, n_pages = 0, pages_per_slot = 0;
   std::vector<int> free_pages, slot_len, slot_pages;
@@ -207,6 +208,7 @@ struct xotb200_lm {
   int64_t launches = 0, tc_launches = 0, flash_launches = 0;
   int* d_err = nullptr;                                // sticky device error word (3 = a bounded wait of a tensor-core product expired)
   int* h_err = nullptr;                                // pinned copy, read after every step
+  bool timed = false;                                  // ev0 and ev1 bracket the newest step, not yet read
   float last_ms = 0.f;
 };
 
@@ -2294,11 +2296,13 @@ int xotb200_lm_init_synthetic(xotb200_lm* e, uint64_t seed) {
 
 int xotb200_lm_check_loaded(xotb200_lm* e) {
   REQUIRE(e, "null engine");
+  if (e->all_loaded) return 0;                           // what has been loaded stays loaded
   for (auto& kv : e->dests)
     if (!kv.second.loaded) {
       set_err("tensor '%s' has not been loaded", kv.first.c_str());
       return XOTB200_ESTRICT;
     }
+  e->all_loaded = true;
   return 0;
 }
 
@@ -2315,6 +2319,7 @@ int xotb200_lm_load_dir(xotb200_lm* e, const char* dir) {
   closedir(dp);
   std::sort(files.begin(), files.end());
   if (files.empty()) { set_err("no *.safetensors in %s", dir); return XOTB200_EIO; }
+  e->all_loaded = false;
   for (auto& kv : e->dests) kv.second.loaded = false;
   for (const std::string& path : files) {
     const int fd = open(path.c_str(), O_RDONLY);
@@ -2631,6 +2636,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     const std::array<long, 5> key{n_seq, n_want, (logits_f32 ? 1 : 0) | (argmax_i32 ? 2 : 0), sp.max_len, (long)off};
     gs = &e->graphs[key];
   }
+  e->timed = false;
   CK(cudaEventRecord(e->ev0, e->stream));
   if (gs && gs->exec) {
     CK(cudaGraphLaunch(gs->exec, e->stream));
@@ -2705,7 +2711,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   CK(cudaEventRecord(e->ev1, e->stream));
   CK(cudaStreamSynchronize(e->stream));
   e->table_stale = false;
-  CK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
+  e->timed = true;
   const int err = results ? reinterpret_cast<const int*>(e->h_out)[(size_t)n_want * V + n_want] : *e->h_err;
   if (err != 0) {
     set_err("a kernel gave up a bounded wait (device error word %d); the step's results are not valid", err);
@@ -2805,6 +2811,10 @@ int xotb200_lm_cache_stats(xotb200_lm* e, int* pages_total, int* pages_free, int
 
 int xotb200_lm_last_step_ms(xotb200_lm* e, float* ms) {
   REQUIRE(e && ms, "null argument");
+  if (e->timed) {
+    CK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
+    e->timed = false;
+  }
   *ms = e->last_ms;
   return 0;
 }

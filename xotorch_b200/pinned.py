@@ -8,6 +8,7 @@ blocks are taken and given back by any thread, and an array outlives the engine 
 from __future__ import annotations
 
 import ctypes as C
+import math
 import threading
 import weakref
 from collections import deque
@@ -50,7 +51,7 @@ class ResultPool:
       return addr or None
 
   def empty(self, shape, dtype=np.float32) -> np.ndarray:
-    count = int(np.prod(shape, dtype=np.int64))
+    count = math.prod(shape)
     nbytes = count * np.dtype(dtype).itemsize
     size = 1 << max(nbytes - 1, 0).bit_length()
     addr = self._block(size) if nbytes >= SMALLEST else None
