@@ -35,6 +35,7 @@
 #include "layered_stream.cuh"
 #include "layered_fma.cuh"
 #include "layered_step.cuh"
+#include "layered_delta_row.cuh"
 #include "flash_tc.cuh"
 #include "st_header.h"
 
@@ -1275,12 +1276,42 @@ static int run_delta(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaSrc ks,
   return launch_delta<32, 8, 1>(e, L, sp, ks, rs, vs, dk, dv, form);
 }
 
+// Steps in which every request brings one row: everything between a delta-rule mixer's projections as one launch (layered_delta_row.cuh).  1 = launched, 0 = a
+// longer step, or sizes that the kernel does not hold (heads above 128, rows that are not whole 16-byte pieces, long filters, wide low-rank branches)
+template <typename T, bool GATED>
+static int delta_row(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaRowArgs a, T* out) {
+  const xotb200_lm_layer& s = L.s;
+  a.proj = e->proj;
+  a.H = s.heads; a.dk = s.dim; a.dv = s.vdim;
+  a.state = e->state + L.state_off;
+  a.slot_stride = e->state_floats;
+  a.col_g = L.c_g; a.col_a = L.c_a;
+  a.norm_w = at<T>(e, L.onorm);
+  a.eps = e->cfg.norm_eps;
+  a.out = out;
+  const int d = std::max(a.dk, a.dv);
+  if (sp.max_rows != 1 || d > 128 || (a.dk | a.dv | a.ld | a.col_g) % 4 != 0 || L.state_off % 4 != 0 || e->state_floats % 4 != 0) return 0;
+  if (GATED ? a.taps > DROW_TAPS || a.rep > 8 : a.low_rank > 256) return 0;
+  const int blocks = sp.n_seq * a.H;
+  if (d <= 64) TRY(launch_early(e, delta_row_kernel<T, 16, 4, GATED>, blocks, DROW_THREADS, 0, a.rep, a, sp.seqs));
+  else TRY(launch_early(e, delta_row_kernel<T, 32, 16, GATED>, blocks, DROW_THREADS, 0, a.rep, a, sp.seqs));
+  return 1;
+}
+
 template <typename T>
 static int delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   const xotb200_lm_layer& s = L.s;
   const int D = e->cfg.width, M = sp.M, HD = s.heads * s.dim;
   T* h = static_cast<T*>(e->h);
   TRY((product<T, T, float, 0>(e, h, D, 0, at<T>(e, L.w_in), D, 1, 0, e->proj, L.n_in, 0, M, L.n_in, D, 1)));
+  DeltaRowArgs ra = {};
+  ra.ld = L.n_in; ra.rep = 1;
+  ra.col_k = L.c_k; ra.col_r = L.c_r; ra.col_v = L.c_v; ra.col_w1 = L.c_w1; ra.low_rank = s.low_rank;
+  ra.w2 = at<T>(e, L.w2); ra.w0 = at<T>(e, L.w0); ra.a_b = at<T>(e, L.a_b);
+  ra.norm_stride = s.vdim;
+  const int row = delta_row<T, false>(e, L, sp, ra, static_cast<T*>(e->oh));
+  if (row < 0) return row;
+  if (row == 1) return output_product<T>(e, static_cast<T*>(e->oh), L.wo, HD, e->y, M);
   TRY(launch_early(e, tanh_cols_kernel<T>, cdiv((long)M * s.low_rank, 256), 256, 0, 1, e->proj, L.n_in, L.c_w1, s.low_rank, static_cast<T*>(e->th), M));
   TRY((product<T, T, float, 0>(e, static_cast<T*>(e->th), s.low_rank, 0, at<T>(e, L.w2), s.low_rank, 1, 0, e->wlog, HD, 0, M, HD, s.low_rank, 1)));
   TRY(launch_early(e, delta_prepare_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->proj, L.n_in, L.c_k, L.c_a, e->wlog, at<T>(e, L.w0), at<T>(e, L.a_b), e->du, e->dau,
@@ -1485,6 +1516,14 @@ template <typename T>
 static int gated_delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout, void* ohbuf) {
   const xotb200_lm_layer& s = L.s;
   const int M = sp.M, H = s.heads, G = s.kv_heads, dk = s.dim, dv = s.vdim, C = L.conv_ch;
+  DeltaRowArgs ra = {};
+  ra.ld = L.ld_in; ra.rep = H / G;
+  ra.col_c = L.c_r; ra.C = C; ra.taps = s.conv_taps; ra.col_b = L.c_b;
+  ra.conv_w = at<T>(e, L.conv_w); ra.a_log = at<T>(e, L.a_log); ra.dt_bias = at<T>(e, L.dt_bias);
+  ra.window = e->state + L.conv_off;
+  const int row = delta_row<T, true>(e, L, sp, ra, static_cast<T*>(ohbuf));
+  if (row < 0) return row;
+  if (row == 1) return output_product<T>(e, static_cast<T*>(ohbuf), L.wo, H * dv, yout, M);
   TRY(filter_channels<T>(e, L, sp, L.c_r, C, nullptr));
   TRY(launch_early(e, gated_delta_prepare_kernel<T>, cdiv((long)M * G, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
                    e->dau, e->du, e->dkk, e->drr, H, G, dk, M));
