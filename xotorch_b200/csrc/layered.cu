@@ -36,6 +36,7 @@
 #include "layered_fma.cuh"
 #include "layered_step.cuh"
 #include "layered_delta_row.cuh"
+#include "layered_delta_chunk.cuh"
 #include "flash_tc.cuh"
 #include "st_header.h"
 
@@ -188,6 +189,8 @@ struct xotb200_lm {
   void *h = nullptr, *cqn = nullptr, *qn = nullptr, *olat = nullptr, *oh = nullptr, *act = nullptr, *th = nullptr, *hw = nullptr;
   void *q16 = nullptr, *cbuf = nullptr, *knx = nullptr, *vxx = nullptr;   // expanded prompt attention (bf16)
   size_t flash_keys_cap = 0;
+  float* dch = nullptr;                                // chunked delta rule: what its first kernel leaves for the second
+  size_t dch_cap = 0;
   float* part = nullptr;                               // key-run partial results of the absorbed attention kernel
   size_t part_cap = 0;
   int max_w = 0;                                       // widest cached row (kv_rank + rot_dim)
@@ -1298,6 +1301,67 @@ static int delta_row(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaRowArgs
   return 1;
 }
 
+// Prompts: the recurrence over chunks of 32 tokens (layered_delta_chunk.cuh).  Short steps, head sizes that it does not hold, and steps for which there is no memory
+// for what its two kernels hand over stay with delta_rule_kernel.
+template <typename T, int DK, int NC, bool GATED, int THR>
+static int launch_chunks(xotb200_lm* e, const StepPlan& sp, const DeltaChunkArgs& a) {
+  const dim3 grid(cdiv(sp.max_rows, DCH), sp.n_seq, GATED ? a.H / a.rep : a.H);
+  if constexpr (GATED) {
+    TRY(opt_in_smem(delta_chunk_gated_kernel<DK>, dch_gated_smem<DK>()));
+    TRY(launch_early(e, delta_chunk_gated_kernel<DK>, grid, 128, dch_gated_smem<DK>(), 1, a, sp.seqs));
+  } else {
+    auto kern = delta_chunk_general_kernel<T, DK>;
+    TRY(opt_in_smem(kern, dch_general_smem<DK>()));
+    TRY(launch_early(e, kern, grid, DCH_THREADS, dch_general_smem<DK>(), 1, a, sp.seqs));
+  }
+  auto walk = delta_chunk_walk_kernel<DK, NC, GATED, THR>;
+  constexpr int smem = DeltaWalk<DK, NC, GATED>::SMEM;
+  TRY(opt_in_smem(walk, smem));
+  return launch_early(e, walk, dim3(sp.n_seq * a.H, cdiv(a.dv, NC)), THR, smem, 1, a, sp.seqs);
+}
+// Rows of the longest request from which the chunks pay: two launches and a chunk's three steps against 0.14 to 0.35 us a token.  (Portions of 64 rows, 32 heads of 64 x 64, beside
+// decoded rows: 7640 us a pass token by token, 7730 in chunks.)
+static const int DCH_MIN_ROWS = 96;
+struct ChunkRoom { size_t mats, vecs, rows; };         // floats of what the two kernels hand over
+static ChunkRoom chunk_floats(const LmLayer& L, const StepPlan& sp, bool gated) {
+  const size_t pieces = (size_t)(sp.M / DCH + sp.n_seq + 1) * L.s.heads;
+  return {pieces * dch_mats(gated), pieces * dch_vecs(gated, L.s.dim), gated ? 0 : (size_t)sp.M * L.s.heads * L.s.dim};
+}
+static bool takes_chunks(xotb200_lm* e, const LmLayer& L, const StepPlan& sp, bool gated) {
+  const int dk = L.s.dim;
+  if (e->stream == e->side) return false;              // the second mixer of a layer runs beside the first, which may use the buffer
+  if (sp.max_rows < DCH_MIN_ROWS || dk % 4 != 0 || dk <= 32 || dk > 128 || sp.n_seq > 65535 || (!gated && (L.n_in | L.c_k | L.c_r) % 4 != 0)) return false;
+  const ChunkRoom c = chunk_floats(L, sp, gated);
+  const size_t need = c.mats + c.vecs + 4 * c.rows;
+  if (need > e->dch_cap) {
+    cudaFree(e->dch);
+    e->dch = nullptr;
+    e->dch_cap = 0;
+    const size_t cap = need + need / 4;                // prompts of slowly growing length do not allocate each time
+    if (cudaMalloc(&e->dch, cap * 4) != cudaSuccess) {
+      cudaGetLastError();
+      e->dch = nullptr;
+      return false;
+    }
+    e->dch_cap = cap;
+  }
+  return true;
+}
+template <typename T, bool GATED>
+static int delta_chunks(xotb200_lm* e, LmLayer& L, const StepPlan& sp, DeltaChunkArgs a) {
+  const xotb200_lm_layer& s = L.s;
+  const ChunkRoom c = chunk_floats(L, sp, GATED);
+  a.H = s.heads; a.dk = s.dim; a.dv = s.vdim;
+  a.mats = e->dch;
+  a.vecs = a.mats + c.mats;
+  a.x1 = a.vecs + c.vecs; a.x2 = a.x1 + c.rows; a.y1 = a.x2 + c.rows; a.y2 = a.y1 + c.rows;
+  a.state = e->state + L.state_off;
+  a.slot_stride = e->state_floats;
+  a.o = e->oraw;
+  if (a.dk <= 64) return launch_chunks<T, 64, 16, GATED, 256>(e, sp, a);
+  return launch_chunks<T, 128, 32, GATED, 256>(e, sp, a);
+}
+
 template <typename T>
 static int delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   const xotb200_lm_layer& s = L.s;
@@ -1314,9 +1378,19 @@ static int delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   if (row == 1) return output_product<T>(e, static_cast<T*>(e->oh), L.wo, HD, e->y, M);
   TRY(launch_early(e, tanh_cols_kernel<T>, cdiv((long)M * s.low_rank, 256), 256, 0, 1, e->proj, L.n_in, L.c_w1, s.low_rank, static_cast<T*>(e->th), M));
   TRY((product<T, T, float, 0>(e, static_cast<T*>(e->th), s.low_rank, 0, at<T>(e, L.w2), s.low_rank, 1, 0, e->wlog, HD, 0, M, HD, s.low_rank, 1)));
-  TRY(launch_early(e, delta_prepare_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->proj, L.n_in, L.c_k, L.c_a, e->wlog, at<T>(e, L.w0), at<T>(e, L.a_b), e->du, e->dau,
-                                                                              s.heads, s.dim, M));
-  TRY(run_delta(e, L, sp, DeltaSrc{e->proj, L.n_in, L.c_k}, DeltaSrc{e->proj, L.n_in, L.c_r}, DeltaSrc{e->proj, L.n_in, L.c_v}, s.dim, s.vdim, DELTA_VECTOR));
+  if (takes_chunks(e, L, sp, false)) {
+    DeltaChunkArgs ca = {};
+    ca.rep = 1;
+    ca.k = ca.r = ca.v = ca.a = e->proj;
+    ca.k_ld = ca.r_ld = ca.v_ld = ca.a_ld = L.n_in;
+    ca.k_col = L.c_k; ca.r_col = L.c_r; ca.v_col = L.c_v; ca.a_col = L.c_a;
+    ca.wlog = e->wlog; ca.a_bias = at<T>(e, L.a_b); ca.w_bias = at<T>(e, L.w0);
+    TRY((delta_chunks<T, false>(e, L, sp, ca)));
+  } else {
+    TRY(launch_early(e, delta_prepare_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->proj, L.n_in, L.c_k, L.c_a, e->wlog, at<T>(e, L.w0), at<T>(e, L.a_b), e->du, e->dau,
+                     s.heads, s.dim, M));
+    TRY(run_delta(e, L, sp, DeltaSrc{e->proj, L.n_in, L.c_k}, DeltaSrc{e->proj, L.n_in, L.c_r}, DeltaSrc{e->proj, L.n_in, L.c_v}, s.dim, s.vdim, DELTA_VECTOR));
+  }
   TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), s.vdim, e->proj, L.n_in, L.c_g, 0,
                                                                                static_cast<T*>(e->oh), s.heads, s.vdim, e->cfg.norm_eps, M));
   TRY(output_product<T>(e, static_cast<T*>(e->oh), L.wo, HD, e->y, M));
@@ -1527,7 +1601,14 @@ static int gated_delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, floa
   TRY(filter_channels<T>(e, L, sp, L.c_r, C, nullptr));
   TRY(launch_early(e, gated_delta_prepare_kernel<T>, cdiv((long)M * G, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
                    e->dau, e->du, e->dkk, e->drr, H, G, dk, M));
-  TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, G * dk, 0, H / G}, DeltaSrc{e->drr, G * dk, 0, H / G}, DeltaSrc{e->cvb, C, 2 * G * dk}, dk, dv, DELTA_SCALAR));
+  if (takes_chunks(e, L, sp, true)) {
+    DeltaChunkArgs ca = {};
+    ca.rep = H / G;
+    ca.k = e->dkk; ca.r = e->drr; ca.v = e->cvb;
+    ca.k_ld = ca.r_ld = G * dk; ca.v_ld = C; ca.v_col = 2 * G * dk;
+    ca.g = e->wlog; ca.beta = e->dau;
+    TRY((delta_chunks<T, true>(e, L, sp, ca)));
+  } else TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, G * dk, 0, H / G}, DeltaSrc{e->drr, G * dk, 0, H / G}, DeltaSrc{e->cvb, C, 2 * G * dk}, dk, dv, DELTA_SCALAR));
   TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), 0, e->proj, L.ld_in, L.c_g, 1, static_cast<T*>(ohbuf),
                                                                        H, dv, e->cfg.norm_eps, M));
   TRY(output_product<T>(e, static_cast<T*>(ohbuf), L.wo, H * dv, yout, M));
@@ -2254,7 +2335,7 @@ int xotb200_lm_destroy(xotb200_lm* e) {
     if (L.rel_bucket) cudaFree(L.rel_bucket);
     if (L.rel_tab) cudaFree(L.rel_tab);
   }
-  void* ptrs[] = {e->vfirst, e->oh2, e->y2, e->h0, e->gdec, e->ginw, e->gfloor, e->gnq, e->pos_freqs, e->dist_tab, e->moe_xg, e->moe_yg, e->moe_plan, e->dkk, e->drr, e->cvb, e->moe_ids, e->moe_wts, e->mact, e->du, e->dau, e->part, e->q16, e->cbuf, e->knx, e->vxx, e->blob, e->d_stage, e->x, e->y, e->proj, e->qraw, e->qfull, e->wlog, e->oraw, e->logits, e->h, e->cqn, e->qn, e->olat, e->oh, e->act,
+  void* ptrs[] = {e->vfirst, e->oh2, e->y2, e->h0, e->gdec, e->ginw, e->gfloor, e->gnq, e->pos_freqs, e->dist_tab, e->moe_xg, e->moe_yg, e->moe_plan, e->dkk, e->drr, e->cvb, e->moe_ids, e->moe_wts, e->mact, e->du, e->dau, e->part, e->dch, e->q16, e->cbuf, e->knx, e->vxx, e->blob, e->d_stage, e->x, e->y, e->proj, e->qraw, e->qfull, e->wlog, e->oraw, e->logits, e->h, e->cqn, e->qn, e->olat, e->oh, e->act,
                   e->th, e->hw, e->trace_buf};
   for (void* p : ptrs)
     if (p) cudaFree(p);
