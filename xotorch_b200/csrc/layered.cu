@@ -1241,6 +1241,20 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   return 0;
 }
 
+// read-outs of a recurrent mixer -> head norm, gate, the operand of the output product
+template <typename T>
+static int head_norm_gate(xotb200_lm* e, const LmLayer& L, int ld, int norm_stride, int silu, T* out, int M) {
+  const xotb200_lm_layer& s = L.s;
+  const int H = s.heads, dv = s.vdim;
+  const T* w = at<T>(e, L.onorm);
+  if ((dv == 64 || dv == 128) && (ld | L.c_g) % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & (4 * sizeof(T) - 1)) == 0) {
+    const int blocks = cdiv((long)M * H * (dv / 4), 256);
+    if (dv == 64) return launch_early(e, head_norm_gate_vec_kernel<T, 16>, blocks, 256, 0, 1, e->oraw, w, norm_stride, e->proj, ld, L.c_g, silu, out, H, e->cfg.norm_eps, M);
+    return launch_early(e, head_norm_gate_vec_kernel<T, 32>, blocks, 256, 0, 1, e->oraw, w, norm_stride, e->proj, ld, L.c_g, silu, out, H, e->cfg.norm_eps, M);
+  }
+  return launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->oraw, nullptr, nullptr, w, norm_stride, e->proj, ld, L.c_g, silu, out, H, dv, e->cfg.norm_eps, M);
+}
+
 // which of the recurrence's forms a mixer uses (delta_rule_kernel)
 enum DeltaForm { DELTA_VECTOR, DELTA_VECTOR_NO_REMOVAL, DELTA_SCALAR };
 template <int KPT, int P, int NC>
@@ -1391,8 +1405,7 @@ static int delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
                      s.heads, s.dim, M));
     TRY(run_delta(e, L, sp, DeltaSrc{e->proj, L.n_in, L.c_k}, DeltaSrc{e->proj, L.n_in, L.c_r}, DeltaSrc{e->proj, L.n_in, L.c_v}, s.dim, s.vdim, DELTA_VECTOR));
   }
-  TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * s.heads, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), s.vdim, e->proj, L.n_in, L.c_g, 0,
-                                                                               static_cast<T*>(e->oh), s.heads, s.vdim, e->cfg.norm_eps, M));
+  TRY(head_norm_gate<T>(e, L, L.n_in, s.vdim, 0, static_cast<T*>(e->oh), M));
   TRY(output_product<T>(e, static_cast<T*>(e->oh), L.wo, HD, e->y, M));
   return 0;
 }
@@ -1483,10 +1496,16 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
       TRY(launch_early(e, pk, dim3(sp.n_seq, cdiv(slots, a.spc), zs), 128, psm, 1, a, sp.seqs, pg, pool, qf, q16));
     }
   } else {
+    float* qf = sp.items.at(-gqa_rows_per_item(s)).second > 0 ? e->qfull : nullptr;   // fp32 queries: read by the warp-per-(row, head) kernel alone
+    const T *bias = s.proj_bias ? at<T>(e, L.b_in) : nullptr, *qw = weighted ? at<T>(e, L.q_norm) : nullptr, *kw = weighted && own ? at<T>(e, L.k_norm) : nullptr;
+    const uintptr_t from = reinterpret_cast<uintptr_t>(bias) | reinterpret_cast<uintptr_t>(qw) | reinterpret_cast<uintptr_t>(kw);
+    if (s.rot_dims == 0 && std::max(dk, dv) <= 128 && (dk | dv | L.ld_in | L.c_q | L.c_kk | L.c_vv) % 4 == 0 && (from & (4 * sizeof(T) - 1)) == 0)
+      TRY(launch_early(e, gqa_prepare_vec_kernel<T>, cdiv((long)M * slots, 8), 256, 0, 1, e->proj, L.ld_in, L.c_q, L.c_kk, L.c_vv, bias, qw, kw, e->cfg.norm_eps, H, G, dk, dv,
+                       own ? 1 : 0, s.q_temp_coef, s.q_temp_every, sp.row_slot, sp.row_pos, pg, pool, qf, q16, M, s.qk_norm != XOTB200_LM_QKNORM_NONE ? 1 : 0));
+    else
     TRY(launch_early(e, gqa_prepare_kernel<T>, cdiv((long)M * slots, 8), 256, 0, 1,
-        e->proj, L.ld_in, L.c_q, L.c_kk, L.c_vv, s.proj_bias ? at<T>(e, L.b_in) : nullptr, weighted ? at<T>(e, L.q_norm) : nullptr,
-        weighted && own ? at<T>(e, L.k_norm) : nullptr, e->cfg.norm_eps, H, G, dk, dv, own ? 1 : 0, s.q_temp_coef, s.q_temp_every, sp.row_slot, sp.row_pos,
-        pg, pool, e->qfull, q16, M, s.qk_norm != XOTB200_LM_QKNORM_NONE ? 1 : 0, s.rot_dims > 0 ? L.freqs : nullptr, s.rot_dims, s.rot_layout));
+        e->proj, L.ld_in, L.c_q, L.c_kk, L.c_vv, bias, qw, kw, e->cfg.norm_eps, H, G, dk, dv, own ? 1 : 0, s.q_temp_coef, s.q_temp_every, sp.row_slot, sp.row_pos,
+        pg, pool, qf, q16, M, s.qk_norm != XOTB200_LM_QKNORM_NONE ? 1 : 0, s.rot_dims > 0 ? L.freqs : nullptr, s.rot_dims, s.rot_layout));
   }
   const size_t pool_rows = (size_t)e->n_pages * e->page_size;
   if (s.pool > 0) {
@@ -1598,10 +1617,22 @@ static int gated_delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, floa
   const int row = delta_row<T, true>(e, L, sp, ra, static_cast<T*>(ohbuf));
   if (row < 0) return row;
   if (row == 1) return output_product<T>(e, static_cast<T*>(ohbuf), L.wo, H * dv, yout, M);
-  TRY(filter_channels<T>(e, L, sp, L.c_r, C, nullptr));
-  TRY(launch_early(e, gated_delta_prepare_kernel<T>, cdiv((long)M * G, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
-                   e->dau, e->du, e->dkk, e->drr, H, G, dk, M));
-  if (takes_chunks(e, L, sp, true)) {
+  const bool chunks = takes_chunks(e, L, sp, true);
+  if (chunks && dk == dv && (dk == 64 || dk == 128) && s.conv_taps <= 4 && (L.ld_in | L.c_r) % 4 == 0 && L.conv_off % 4 == 0 && e->state_floats % 4 == 0) {
+    GatedConvArgs ga = {};
+    ga.proj = e->proj; ga.ld = L.ld_in; ga.col_c = L.c_r; ga.C = C; ga.taps = s.conv_taps; ga.col_b = L.c_b; ga.col_a = L.c_a; ga.H = H; ga.G = G;
+    ga.conv_w = at<T>(e, L.conv_w); ga.a_log = at<T>(e, L.a_log); ga.dt_bias = at<T>(e, L.dt_bias);
+    ga.window = e->state + L.conv_off; ga.slot_stride = e->state_floats;
+    ga.g = e->wlog; ga.beta = e->dau; ga.k = e->dkk; ga.r = e->drr; ga.v = e->cvb;
+    const dim3 grid(sp.n_seq, cdiv(2 * G + H, dk == 64 ? 16 : 8), std::min(65535, cdiv(sp.max_rows, 16)));
+    if (dk == 64) TRY(launch_early(e, gated_conv_prepare_kernel<T, 16>, grid, 256, 0, 1, ga, sp.seqs));
+    else TRY(launch_early(e, gated_conv_prepare_kernel<T, 32>, grid, 256, 0, 1, ga, sp.seqs));
+  } else {
+    TRY(filter_channels<T>(e, L, sp, L.c_r, C, nullptr));
+    TRY(launch_early(e, gated_delta_prepare_kernel<T>, cdiv((long)M * G, 8), 256, 0, 1, e->cvb, C, e->proj, L.ld_in, L.c_b, L.c_a, at<T>(e, L.a_log), at<T>(e, L.dt_bias), e->wlog,
+                     e->dau, e->du, e->dkk, e->drr, H, G, dk, M));
+  }
+  if (chunks) {
     DeltaChunkArgs ca = {};
     ca.rep = H / G;
     ca.k = e->dkk; ca.r = e->drr; ca.v = e->cvb;
@@ -1609,8 +1640,7 @@ static int gated_delta_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, floa
     ca.g = e->wlog; ca.beta = e->dau;
     TRY((delta_chunks<T, true>(e, L, sp, ca)));
   } else TRY(run_delta(e, L, sp, DeltaSrc{e->dkk, G * dk, 0, H / G}, DeltaSrc{e->drr, G * dk, 0, H / G}, DeltaSrc{e->cvb, C, 2 * G * dk}, dk, dv, DELTA_SCALAR));
-  TRY(launch_early(e, head_norm_gate_kernel<T>, cdiv((long)M * H, 8), 256, 0, 1, e->oraw, nullptr, nullptr, at<T>(e, L.onorm), 0, e->proj, L.ld_in, L.c_g, 1, static_cast<T*>(ohbuf),
-                                                                       H, dv, e->cfg.norm_eps, M));
+  TRY(head_norm_gate<T>(e, L, L.ld_in, 0, 1, static_cast<T*>(ohbuf), M));
   TRY(output_product<T>(e, static_cast<T*>(ohbuf), L.wo, H * dv, yout, M));
   return 0;
 }

@@ -252,6 +252,93 @@ __global__ void __launch_bounds__(DCH_THREADS) delta_chunk_general_kernel(const 
   }
 }
 
+// ---- what a prompt of the gated form needs per token, in one pass over the projection: the channels' convolution (its window in registers), silu, unit key, scaled
+// query, values (at v [M, C], the value channels' place), decay and write strength.  LPH lanes have the 4 LPH channels of one query, key or value head (dk = dv) and
+// walk a stretch of rows; grid (requests, groups of heads, stretches).  Stretch 0 reads the window that the slot keeps and moves it on.  Up to four taps.
+// 3500 rows of 4096 channels: 65 us (convolution) + 37 (unit vectors, decays) -> 36.
+struct GatedConvArgs {
+  const float* proj;
+  int ld, col_c, C, taps, col_b, col_a, H, G;
+  const void *conv_w, *a_log, *dt_bias;
+  float* window;
+  size_t slot_stride;
+  float *g, *beta, *k, *r, *v;
+};
+template <typename T, int LPH>
+__global__ void __launch_bounds__(256) gated_conv_prepare_kernel(const GatedConvArgs a, const Item* __restrict__ seqs) {
+  pdl_enter();
+  constexpr int DK = 4 * LPH, W = 4, NB = 4;           // taps at most, rows whose loads are in flight
+  const Item sq = seqs[blockIdx.x];
+  const int l = threadIdx.x % LPH, vec = blockIdx.y * (256 / LPH) + threadIdx.x / LPH, c = vec * DK + 4 * l;
+  const int per = max((sq.n_rows + (int)gridDim.z - 1) / (int)gridDim.z, W - 1);
+  const int t_begin = blockIdx.z * per, t_end = min(sq.n_rows, t_begin + per), skip = W - a.taps;
+  if (t_begin >= t_end) return;
+  const bool on = vec < 2 * a.G + a.H;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* src = a.proj + (size_t)sq.row0 * a.ld + a.col_c + (on ? c : 0);
+  float* st = a.window + (size_t)sq.slot * a.slot_stride + (on ? c : 0);
+  float w[W][4];
+  float4 win[W - 1], first[W - 1];                     // inputs of the three rows in front; the same at the stretch's begin
+#pragma unroll
+  for (int i = 0; i < W; ++i)
+#pragma unroll
+    for (int x = 0; x < 4; ++x) w[i][x] = on && i >= skip ? ldf(static_cast<const T*>(a.conv_w) + (size_t)(c + x) * a.taps + i - skip) : 0.f;
+#pragma unroll
+  for (int i = 0; i < W - 1; ++i) {
+    const int t = t_begin - (W - 1) + i;
+    first[i] = win[i] = !on || i < skip ? zero : t >= 0 ? ld4f(src + (size_t)t * a.ld) : ld4f(st + (size_t)(t + a.taps - 1) * a.C);
+  }
+  const float qs = vec < a.G ? sqrtf((float)DK) : 1.0f;
+  float* dst = vec < a.G ? a.r + (size_t)sq.row0 * (a.G * DK) + c : vec < 2 * a.G ? a.k + (size_t)sq.row0 * (a.G * DK) + c - a.G * DK : a.v + (size_t)sq.row0 * a.C + c;
+  const int ld_dst = vec < 2 * a.G ? a.G * DK : a.C;
+  for (int t0 = t_begin; t0 < t_end; t0 += NB) {
+    float4 cur[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) cur[b] = on && t0 + b < t_end ? ld4f(src + (size_t)(t0 + b) * a.ld) : zero;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      float4 acc = zero;
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        if (i < skip) continue;
+        const float4 in = i == W - 1 ? cur[b] : win[i < W - 1 ? i : 0];
+        acc = make_float4(fmaf(w[i][0], in.x, acc.x), fmaf(w[i][1], in.y, acc.y), fmaf(w[i][2], in.z, acc.z), fmaf(w[i][3], in.w, acc.w));
+      }
+#pragma unroll
+      for (int i = 0; i + 1 < W - 1; ++i) win[i] = win[i + 1];
+      win[W - 2] = cur[b];
+      acc = make_float4(siluf_(acc.x), siluf_(acc.y), siluf_(acc.z), siluf_(acc.w));
+      float s = sq4(acc);
+#pragma unroll
+      for (int x = LPH / 2; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+      const float f = vec < 2 * a.G ? 1.0f / (sqrtf(s + 1e-6f) * qs) : 1.0f;
+      if (on && t0 + b < t_end) st4f(dst + (size_t)(t0 + b) * ld_dst, make_float4(acc.x * f, acc.y * f, acc.z * f, acc.w * f));
+    }
+  }
+  if (!on) return;
+  if (vec >= 2 * a.G) {
+    const int h = vec - 2 * a.G;
+    const float al = expf(ldf(static_cast<const T*>(a.a_log) + h)), db = ldf(static_cast<const T*>(a.dt_bias) + h);
+    for (int t = t_begin + l; t < t_end; t += LPH) {
+      const size_t m = (size_t)sq.row0 + t;
+      a.beta[m * a.H + h] = sigmoidf_(a.proj[m * a.ld + a.col_b + h]);
+      a.g[m * a.H + h] = expf(-al * softplusf_(a.proj[m * a.ld + a.col_a + h] + db));
+    }
+  }
+  if (blockIdx.z == 0)
+#pragma unroll
+    for (int i = 0; i < W - 1; ++i) {
+      if (i < skip) continue;
+      const int t = sq.n_rows - (W - 1) + i;           // the row whose input entry i - skip of the window becomes
+      float4 v = zero;
+      if (t >= 0) v = ld4f(src + (size_t)t * a.ld);
+#pragma unroll
+      for (int x = 0; x < W - 1; ++x)
+        if (t < 0 && x == t + W - 1) v = first[x];
+      st4f(st + (size_t)(i - skip) * a.C, v);
+    }
+}
+
 // ---- the walk over the chunks.  One CTA of THR threads per (request, head, NC value columns); S^T, and everything a chunk needs, in shared memory, the next chunk on its
 // way.  A 16-byte load of a warp takes four turns of shared memory, shared addresses or not, so every product is cut into tiles of 4 x 4 to 8 x 8 results whose K
 // is shared by four lanes: two loads feed 2 to 4 times as many sums as with a 2 x 2 tile per thread (349 -> 295 us for 3500 tokens), and shuffles add the lanes' parts.
