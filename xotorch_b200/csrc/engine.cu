@@ -472,19 +472,21 @@ static int launch_early(xotb200_engine* e, cudaStream_t st, void (*fn)(KA...), d
 // while two CTAs per SM (with 128 rows, whose partial tiles are 64 KB: one) are not exceeded and each keeps two K blocks or more.  Measured on an 8B layer
 // (16 / 128 rows; 128 x 64..128 token tiles with split-K through a workspace took 36.5 us for O and down on average, 30.6 for QKV, 54.9 for
 // gate/up at 128 rows): O and down 18.3 / 28.7 us, QKV 14.5 / 23.6, gate/up 41.4 (5.7 TB/s) / 47.9.
-template <int NB>
+// With 128 rows a stage holds as many bytes of rows as of weights; where no SM has two CTAs the ring is twice as deep (two 8B layers, 128 rows: 344 -> 294 us a call; cutting K
+// over as many CTAs as fit, not a power of two of them, loses: 321; 6 rows 232 -> 243).
+template <int NB, int NS>
 static int launch_tc_stream_nb(xotb200_engine* e, const CUtensorMap& tmW, const CUtensorMap& tmX, const TcGemmArgs& a, int epi, int splits, cudaStream_t st) {
   void (*fn)(CUtensorMap, CUtensorMap, TcGemmArgs) = nullptr;
   const bool f16 = e->cfg.dtype == XOTB200_DTYPE_F16;
   switch (epi) {
-    case TCE_STORE: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_STORE> : xb::bf::tc_stream_kernel<NB, TCE_STORE>; break;
-    case TCE_RESID: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_RESID> : xb::bf::tc_stream_kernel<NB, TCE_RESID>; break;
-    case TCE_QKV: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_QKV> : xb::bf::tc_stream_kernel<NB, TCE_QKV>; break;
-    case TCE_SWIGLU: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_SWIGLU> : xb::bf::tc_stream_kernel<NB, TCE_SWIGLU>; break;
-    default: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_HEAD_LAST> : xb::bf::tc_stream_kernel<NB, TCE_HEAD_LAST>; break;
+    case TCE_STORE: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_STORE, NS> : xb::bf::tc_stream_kernel<NB, TCE_STORE, NS>; break;
+    case TCE_RESID: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_RESID, NS> : xb::bf::tc_stream_kernel<NB, TCE_RESID, NS>; break;
+    case TCE_QKV: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_QKV, NS> : xb::bf::tc_stream_kernel<NB, TCE_QKV, NS>; break;
+    case TCE_SWIGLU: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_SWIGLU, NS> : xb::bf::tc_stream_kernel<NB, TCE_SWIGLU, NS>; break;
+    default: fn = f16 ? xb::fp::tc_stream_kernel<NB, TCE_HEAD_LAST, NS> : xb::bf::tc_stream_kernel<NB, TCE_HEAD_LAST, NS>; break;
   }
-  if (int rc = ensure_smem_attr(e->device, (const void*)fn, tcs_smem_bytes(NB))) return rc;
-  return launch_early(e, st, fn, dim3(splits, a.N / TC_M), TC_THREADS, tcs_smem_bytes(NB), splits, tmW, tmX, a);
+  if (int rc = ensure_smem_attr(e->device, (const void*)fn, tcs_smem_bytes(NB, NS))) return rc;
+  return launch_early(e, st, fn, dim3(splits, a.N / TC_M), TC_THREADS, tcs_smem_bytes(NB, NS), splits, tmW, tmX, a);
 }
 static int launch_tc_stream(xotb200_engine* e, const CUtensorMap& tmW, const ActMaps& x, const TcGemmArgs& a_in, int epi, cudaStream_t st) {
   TcGemmArgs a = a_in;
@@ -492,8 +494,9 @@ static int launch_tc_stream(xotb200_engine* e, const CUtensorMap& tmW, const Act
   const int nb = epi == TCE_HEAD_LAST || a.S <= 16 ? 16 : a.S <= 32 ? 32 : a.S <= 64 ? 64 : 128, tiles = a.N / TC_M, nkb = a.K / TC_BK;
   int s = 1;
   while (s < 8 && tiles * s * 2 <= (nb >= 128 ? 1 : 2) * e->sm_count && nkb >= 4 * s) s *= 2;
-  return nb == 16 ? launch_tc_stream_nb<16>(e, tmW, x.r16, a, epi, s, st) : nb == 32 ? launch_tc_stream_nb<32>(e, tmW, x.r32, a, epi, s, st)
-       : nb == 64 ? launch_tc_stream_nb<64>(e, tmW, x.r64, a, epi, s, st) : launch_tc_stream_nb<128>(e, tmW, x.full, a, epi, s, st);
+  if (nb == 128 && tiles * s <= e->sm_count) return launch_tc_stream_nb<128, TCS_ALONE>(e, tmW, x.full, a, epi, s, st);
+  return nb == 16 ? launch_tc_stream_nb<16, tcs_stages(16)>(e, tmW, x.r16, a, epi, s, st) : nb == 32 ? launch_tc_stream_nb<32, tcs_stages(32)>(e, tmW, x.r32, a, epi, s, st)
+       : nb == 64 ? launch_tc_stream_nb<64, tcs_stages(64)>(e, tmW, x.r64, a, epi, s, st) : launch_tc_stream_nb<128, tcs_stages(128)>(e, tmW, x.full, a, epi, s, st);
 }
 
 template <int NT, int NS>

@@ -160,7 +160,9 @@ __host__ __device__ constexpr int tc2_smem_bytes(int nt, int ns) { return ns * t
 // ---- few token rows (tc_stream_kernel): 128 weight rows are the M operand, NB token rows the N side; two CTAs share an SM's shared memory
 __host__ __device__ constexpr int tcs_stage_bytes(int nb) { return TC_M * TC_BK * 2 + nb * TC_BK * 2; }
 __host__ __device__ constexpr int tcs_stages(int nb) { return nb <= 16 ? 6 : nb <= 32 ? 5 : nb <= 64 ? 4 : 3; }
-__host__ __device__ constexpr int tcs_smem_bytes(int nb) { return tcs_stages(nb) * tcs_stage_bytes(nb) + 1024 + 256; }
+constexpr int TCS_ALONE = 6;           // stages of a 128-row ring when no SM has more than one CTA
+__host__ __device__ constexpr int tcs_smem_bytes(int nb, int ns) { return ns * tcs_stage_bytes(nb) + 1024 + 256; }
+__host__ __device__ constexpr int tcs_smem_bytes(int nb) { return tcs_smem_bytes(nb, tcs_stages(nb)); }
 constexpr int TCS_LD = TC_M + 4;      // floats per row of a CTA's partial tile (16-byte pieces of neighbouring rows in different banks)
 static_assert(tcs_smem_bytes(16) <= 112 * 1024 && tcs_smem_bytes(32) <= 112 * 1024 && tcs_smem_bytes(64) <= 112 * 1024 && tcs_smem_bytes(128) <= 112 * 1024, "two CTAs per SM");
 static_assert(128 * TCS_LD * 4 <= tcs_stages(128) * tcs_stage_bytes(128), "the partial tile reuses the ring");
