@@ -37,6 +37,7 @@
 #include "layered_step.cuh"
 #include "layered_delta_row.cuh"
 #include "layered_delta_chunk.cuh"
+#include "layered_gqa_row.cuh"
 #include "flash_tc.cuh"
 #include "st_header.h"
 
@@ -785,6 +786,7 @@ static int launch_early(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threa
 // whose blocks are smaller, gain by the early start up to runs of GQA_EARLY_RUN keys (one / four requests behind 250: 162 / 176 against 167 / 178 us; behind
 // 4000: 202 / 295 against 186 / 264).
 constexpr int GQA_EARLY_RUN = 64;
+constexpr int GQA_ROW_EARLY = 128;                     // keys of a block of gqa_row_kernel up to which it starts early (no difference measured at 64; behind long caches as above)
 template <typename... KA, typename... A>
 static int launch_late(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threads, size_t smem, A&&... args) {
   kern<<<grid, threads, smem, e->stream>>>(static_cast<KA>(args)...);
@@ -1068,6 +1070,7 @@ struct StepPlan {
   const int* bigram_row = nullptr;                     // per row: its row of the hashed-pair table
   const Item* seqs = nullptr;
   std::map<int, std::pair<const Item*, int>> items;   // rows per attention work item -> (device list, count)
+  std::map<int, bool> single;                          // the same: every item of the list has one row
   // expanded prompt attention (bf16): per distinct window of the model's attention layers, the requests that bring many rows
   struct Flash {
     const GatherReq* reqs = nullptr;
@@ -1431,6 +1434,43 @@ static int gqa_key_runs(const xotb200_lm* e, const xotb200_lm_layer& s, int n_it
   return cdiv(span, *run);
 }
 
+// Lists of single rows over heads of 64 or 128 entries (keys and values alike) take gqa_row_kernel
+static bool gqa_row_fits(const xotb200_lm* e, const xotb200_lm_layer& s, bool single) { return single && s.dim == s.vdim && (s.dim == 64 || s.dim == 128); }
+static int gqa_row_heads(const xotb200_lm_layer& s) { const int rep = s.heads / s.kv_heads; return rep % 4 == 0 ? 4 : rep % 2 == 0 ? 2 : 1; }
+// its shares of the keys: about one block per SM, two turns of 32 keys or more each
+static int gqa_row_shares(const xotb200_lm* e, const xotb200_lm_layer& s, int n_items, int max_len, int* keys) {
+  int span = std::max(1, max_len);
+  if (s.window > 0) span = std::min(span, s.window);
+  if (s.chunk > 0) span = std::min(span, s.chunk);
+  if (s.keep_first > 0) span += std::min(s.keep_first, std::max(1, max_len));
+  if (s.pool > 0) span += std::max(1, max_len) / s.pool;
+  const long ctas = std::max(1L, (long)n_items * s.heads / gqa_row_heads(s));
+  const int shares = (int)std::max(1L, std::min(std::min(32L, (long)cdiv(span, 2 * GROW_KEYS)), (e->sm_count + ctas - 1) / ctas));
+  *keys = cdiv(span, shares);
+  return shares;
+}
+template <typename T, int D>
+static int launch_gqa_row(xotb200_lm* e, const GqaRowArgs& a, int rep, int keys, dim3 grid) {
+  auto kern = rep == 4 ? gqa_row_kernel<T, D, 4> : rep == 2 ? gqa_row_kernel<T, D, 2> : gqa_row_kernel<T, D, 1>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(GROW_THREADS);
+  cfg.stream = e->stream;
+  cudaLaunchAttribute at[2];
+  cfg.attrs = at;
+  if (e->early && keys <= GQA_ROW_EARLY) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (!a.part && grid.z > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs++].val.clusterDim = {1, 1, grid.z};
+  }
+  CK(cudaLaunchKernelEx(&cfg, kern, a));
+  e->launches++;
+  return 0;
+}
+
 // (the projection of the layer's mixers is in e->proj, leading dimension L.ld_in; the mixer's output goes to yout)
 template <typename T>
 static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout) {
@@ -1519,7 +1559,21 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
   const float* gate = s.out_gate ? e->proj : nullptr;
   const int qpi = gqa_rows_per_item(s);
   const auto& it = sp.items.at(-qpi);   // the lists of this mixer have negative keys
-  if (it.second > 0) {
+  if (it.second > 0 && gqa_row_fits(e, s, sp.single.at(-qpi))) {
+    GqaRowArgs a = {};
+    int keys = 0;
+    const int splits = gqa_row_shares(e, s, it.second, sp.max_len, &keys), heads = gqa_row_heads(s);
+    const bool cluster = splits <= 8;
+    REQUIRE(cluster || (size_t)M * H * splits * (2 + dv) <= e->part_cap, "internal: the key-run buffer was not sized for this step");
+    a.qf = e->qfull; a.pool = pool; a.pg = pg; a.items = it.first; a.H = H; a.G = G; a.sc = sc;
+    a.gate = gate; a.gate_mode = s.out_gate; a.gate_ld = L.ld_in; a.gate_col0 = L.c_g; a.out = e->oh; a.part = cluster ? nullptr : e->part;
+    const dim3 grid(it.second, H / heads, splits);
+    if (dk == 64) TRY((launch_gqa_row<T, 64>(e, a, heads, keys, grid)));
+    else TRY((launch_gqa_row<T, 128>(e, a, heads, keys, grid)));
+    if (!cluster)
+      TRY(launch_early(e, gqa_combine_kernel<T>, dim3(it.second, cdiv(qpi * H, 8), it.second * cdiv(qpi * H, 8) < 4 * e->sm_count ? cdiv(dv, 32) : 1), 256, 0, 1, e->part, it.first, H, dv, splits,
+                       static_cast<const T*>(sc.sink), sc.sink_one, gate, s.out_gate, L.ld_in, L.c_g, static_cast<T*>(e->oh)));
+  } else if (it.second > 0) {
     const int pairs = qpi * rep, nw = gqa_item_warps(s, pairs), ytiles = cdiv(pairs, nw);
     const size_t smem = ((size_t)32 * ((dk + dv) | 1) + (size_t)nw * dk) * 4;
     int run = 0;
@@ -2673,6 +2727,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   const size_t off_seqs = push(seqs.data(), 4 * (size_t)n_seq), off_bigram = push(bg.data(), bg.size());
   auto is_long = [&](int i) { return use_flash && counts[i] >= FLASH_MIN_ROWS; };
   std::map<int, std::pair<size_t, int>> item_off;
+  std::map<int, bool> item_single;
   sp.any_short = false;
   const bool use_gqa_flash = e->esz == 2 && e->flash_on && e->gqa_flash_fits;
   auto is_long_gqa = [&](int i) { return use_gqa_flash && counts[i] >= FLASH_MIN_ROWS; };
@@ -2683,6 +2738,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
       if (qk < 0 ? !is_long_gqa(i) : !is_long(i))
         for (int t = 0; t < counts[i]; t += q) it.push_back(Item{seqs[i].row0 + t, std::min(q, counts[i] - t), seqs[i].slot, seqs[i].pos0 + t});
     item_off[qk] = {push(it.data(), 4 * it.size()), (int)it.size()};
+    item_single[qk] = std::all_of(it.begin(), it.end(), [](const Item& i) { return i.n_rows == 1; });
     if (!it.empty() && qk > 0) sp.any_short = true;
   }
   size_t gqa_tiles_off = 0, gqa_tiles128_off = 0;
@@ -2772,6 +2828,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
       const bool latent = L.s.mixer == XOTB200_LM_MIX_LATENT_ATTN;
       int run = 0;
       const int splits = latent ? latent_key_runs(e, L.s, item_off[latent_rows_per_item(L.s)].second, sp.max_len, &run)
+                       : gqa_row_fits(e, L.s, item_single[-gqa_rows_per_item(L.s)]) ? gqa_row_shares(e, L.s, item_off[-gqa_rows_per_item(L.s)].second, sp.max_len, &run)
                                 : gqa_key_runs(e, L.s, item_off[-gqa_rows_per_item(L.s)].second, sp.max_len, &run);
       const size_t need = splits > 1 ? (size_t)M * L.s.heads * splits * (2 + (latent ? L.s.kv_rank : L.s.vdim)) : 0;
       if (need > e->part_cap) { drop_graphs(e); TRY(regrow(e->part, need * 4)); e->part_cap = need; }
@@ -2808,6 +2865,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
       sp.want = e->d_stage + T0 + 3 * M;
       sp.bigram_row = e->d_stage + off_bigram;
       sp.seqs = reinterpret_cast<const Item*>(e->d_stage + off_seqs);
+      sp.single = item_single;
       for (auto& kv : item_off) sp.items[kv.first] = {reinterpret_cast<const Item*>(e->d_stage + kv.second.first), kv.second.second};
       sp.gqa_tiles = reinterpret_cast<const GqaTile*>(e->d_stage + gqa_tiles_off);
       sp.n_gqa_tiles = n_gqa_tiles;
