@@ -38,6 +38,7 @@
 #include "layered_delta_row.cuh"
 #include "layered_delta_chunk.cuh"
 #include "layered_gqa_row.cuh"
+#include "layered_latent_row.cuh"
 #include "flash_tc.cuh"
 #include "st_header.h"
 
@@ -786,6 +787,7 @@ static int launch_early(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threa
 // whose blocks are smaller, gain by the early start up to runs of GQA_EARLY_RUN keys (one / four requests behind 250: 162 / 176 against 167 / 178 us; behind
 // 4000: 202 / 295 against 186 / 264).
 constexpr int GQA_EARLY_RUN = 64;
+constexpr int LATENT_ROW_EARLY = 64;                   // keys of a block of latent_row_kernel up to which it starts early (no difference measured up to 128)
 constexpr int GQA_ROW_EARLY = 128;                     // keys of a block of gqa_row_kernel up to which it starts early (no difference measured at 64; behind long caches as above)
 template <typename... KA, typename... A>
 static int launch_late(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threads, size_t smem, A&&... args) {
@@ -1106,6 +1108,42 @@ static int latent_key_runs(const xotb200_lm* e, const xotb200_lm_layer& s, int n
   return cdiv(span, *run);
 }
 
+// Lists of single rows over latents of 256 (or, in 16 bits, 512) entries take latent_row_kernel
+static bool latent_row_fits(const xotb200_lm* e, const xotb200_lm_layer& s, bool single) {
+  const int vec = e->esz == 2 ? 8 : 4;
+  return single && (s.kv_rank == 256 || (s.kv_rank == 512 && e->esz == 2)) && s.rot_dim % vec == 0 && s.rot_dim <= 8 * vec;
+}
+// its shares of the keys: about one block per SM, four turns of four keys or more each
+static int latent_row_shares(const xotb200_lm* e, const xotb200_lm_layer& s, int n_items, int max_len, int* keys) {
+  const int span = std::max(1, s.window > 0 ? std::min(max_len, s.window) : max_len);
+  const long ctas = std::max(1L, (long)n_items * cdiv(s.heads, 8));
+  const int shares = (int)std::max(1L, std::min(std::min(32L, (long)cdiv(span, 4 * LROW_KEYS)), (e->sm_count + ctas - 1) / ctas));
+  *keys = cdiv(span, shares);
+  return shares;
+}
+template <typename T, int R>
+static int launch_latent_row(xotb200_lm* e, const LatentRowArgs& a, int keys, dim3 grid) {
+  auto kern = latent_row_kernel<T, R>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(LROW_THREADS);
+  cfg.dynamicSmemBytes = (8 * R + 16) * 4;
+  cfg.stream = e->stream;
+  cudaLaunchAttribute at[2];
+  cfg.attrs = at;
+  if (e->early && keys <= LATENT_ROW_EARLY) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (!a.part && grid.z > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs++].val.clusterDim = {1, 1, grid.z};
+  }
+  CK(cudaLaunchKernelEx(&cfg, kern, a));
+  e->launches++;
+  return 0;
+}
+
 // ---- prompt attention on tcgen05 (flash_tc.cuh) ---------------------------------------------------------------------------------
 // queries [M][H][d] as a 3-D map {d, H, M} with a box of 64 entries of one head of 128 rows
 static bool make_query_map(CUtensorMap* m, const bf16* q, int M, int H, int d) {
@@ -1168,7 +1206,20 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
                                  dn, H)));
     const int qpi = latent_rows_per_item(s);
     const auto& it = sp.items.at(qpi);
-    if (it.second > 0) {
+    if (it.second > 0 && latent_row_fits(e, s, sp.single.at(qpi))) {
+      int keys = 0;
+      const int shares = latent_row_shares(e, s, it.second, sp.max_len, &keys);
+      REQUIRE(shares <= 8 || (size_t)M * H * shares * (2 + R) <= e->part_cap, "internal: the key-run buffer was not sized for this step");
+      LatentRowArgs a = {};
+      a.q = e->qfull; a.pool = L.pool; a.pg = pg; a.items = it.first; a.H = H; a.dr = dr; a.window = s.window; a.scale = s.scale;
+      a.gate = gate; a.gate_ld = L.n_in; a.gate_col0 = L.c_g; a.sink = sink; a.out = e->olat; a.part = shares <= 8 ? nullptr : e->part;
+      const dim3 grid(it.second, cdiv(H, 8), shares);
+      if (R == 256) TRY((launch_latent_row<T, 256>(e, a, keys, grid)));
+      else if constexpr (std::is_same<T, bf16>::value) TRY((launch_latent_row<T, 512>(e, a, keys, grid)));
+      if (shares > 8)
+        TRY(launch_early(e, latent_attention_combine_kernel<T>, dim3(it.second, cdiv(qpi * H, 8), it.second * cdiv(qpi * H, 8) < e->sm_count ? std::min(16, cdiv(R, 32)) : 1), 256, 0, 1, e->part, it.first, H, R,
+                         shares, gate, L.n_in, L.c_g, sink, static_cast<T*>(e->olat)));
+    } else if (it.second > 0) {
       const int pairs = qpi * H, nw = latent_item_warps(s, pairs);
       const int nbuf = latent_smem_bytes<T>(R + dr, nw, 2) <= 200 * 1024 ? 2 : 1;
       const size_t smem = latent_smem_bytes<T>(R + dr, nw, nbuf);
@@ -2827,7 +2878,8 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     if (L.s.mixer == XOTB200_LM_MIX_ATTENTION || L.s.mixer == XOTB200_LM_MIX_LATENT_ATTN) {
       const bool latent = L.s.mixer == XOTB200_LM_MIX_LATENT_ATTN;
       int run = 0;
-      const int splits = latent ? latent_key_runs(e, L.s, item_off[latent_rows_per_item(L.s)].second, sp.max_len, &run)
+      const int splits = latent && latent_row_fits(e, L.s, item_single[latent_rows_per_item(L.s)]) ? latent_row_shares(e, L.s, item_off[latent_rows_per_item(L.s)].second, sp.max_len, &run)
+                       : latent ? latent_key_runs(e, L.s, item_off[latent_rows_per_item(L.s)].second, sp.max_len, &run)
                        : gqa_row_fits(e, L.s, item_single[-gqa_rows_per_item(L.s)]) ? gqa_row_shares(e, L.s, item_off[-gqa_rows_per_item(L.s)].second, sp.max_len, &run)
                                 : gqa_key_runs(e, L.s, item_off[-gqa_rows_per_item(L.s)].second, sp.max_len, &run);
       const size_t need = splits > 1 ? (size_t)M * L.s.heads * splits * (2 + (latent ? L.s.kv_rank : L.s.vdim)) : 0;
