@@ -535,17 +535,26 @@ template <typename T, int RPB>
 __global__ void __launch_bounds__(1024) moe_router_kernel(const T* __restrict__ h, int D, const T* __restrict__ w_router, const T* __restrict__ bias, int kind, int E,
                                   int groups, int keep, int top, const T* __restrict__ correction, int group_best, float wscale, int* __restrict__ ids,
                                   float* __restrict__ wts, int M) {
-  pdl_enter();
   extern __shared__ __align__(16) float rsm[];                 // [RPB][D] the rows (fp32), then [RPB] scores
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int m0 = blockIdx.x * RPB, nr = min(RPB, M - m0), Dp = (D + 3) & ~3, ns = moe_router_scores(kind, E, groups);
   float* scores = rsm + RPB * Dp;
+  constexpr int VEC = 16 / sizeof(T), NB = RPB > 1 ? 2 : 4;     // NB weight pieces in flight per lane
+  const bool vec = D % VEC == 0 && (reinterpret_cast<uintptr_t>(w_router) & 15) == 0;
+  // a warp's first weights depend on nothing: on their way while the kernel in front ends and the rows are staged
+  pdl_launch_dependents();
+  uint4 ahead[NB];
+  if (vec && warp < E)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int k = (lane + b * 32) * VEC;
+      ahead[b] = k < D ? *reinterpret_cast<const uint4*>(w_router + (size_t)warp * D + k) : make_uint4(0, 0, 0, 0);
+    }
+  pdl_wait();
 #pragma unroll
   for (int r = 0; r < RPB; ++r)
     if (r < nr) stage_f32(rsm + r * Dp, h + (size_t)(m0 + r) * D, D);
   __syncthreads();
-  constexpr int VEC = 16 / sizeof(T), NB = RPB > 1 ? 2 : 4;     // NB weight pieces in flight per lane
-  const bool vec = D % VEC == 0 && (reinterpret_cast<uintptr_t>(w_router) & 15) == 0;
   for (int e = warp; e < E; e += nw) {                         // the warps share the experts; logits in fp32
     const T* w = w_router + (size_t)e * D;
     float z[RPB];
@@ -555,7 +564,8 @@ __global__ void __launch_bounds__(1024) moe_router_kernel(const T* __restrict__ 
       for (int k = lane * VEC; k < D; k += 32 * VEC * NB) {
         uint4 raw[NB];
 #pragma unroll
-        for (int b = 0; b < NB; ++b) raw[b] = k + b * 32 * VEC < D ? *reinterpret_cast<const uint4*>(w + k + b * 32 * VEC) : make_uint4(0, 0, 0, 0);
+        for (int b = 0; b < NB; ++b)
+          raw[b] = e == warp && k == lane * VEC ? ahead[b] : k + b * 32 * VEC < D ? *reinterpret_cast<const uint4*>(w + k + b * 32 * VEC) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
           const int kb = k + b * 32 * VEC < D ? k + b * 32 * VEC : k;   // past the end the weights read as zero; the index stays inside the row
@@ -652,6 +662,38 @@ __global__ void __launch_bounds__(1024) moe_router_kernel(const T* __restrict__ 
   __syncwarp();
   for (int e = lane; e < E; e += 32) s[e] = expf(s[e] - mx) / den;
   __syncwarp();
+  if (E <= 32 && E % max(groups, 1) == 0) {
+    // the same selection as below, an expert to a lane: a chain of some hundred reads of shared memory by one lane is 3 us of the step
+    const int gs = groups > 1 ? E / groups : E;
+    const float v = lane < E ? s[lane] : -1.f;
+    bool kept = lane < E;
+    if (groups > 1) {
+      float best = -1.f;
+      for (int i = 0; i < gs; ++i) best = fmaxf(best, __shfl_sync(0xffffffffu, v, min(lane / gs, groups - 1) * gs + i));
+      for (int r = 0; r < groups - keep; ++r) {
+        float worst = kept ? best : INFINITY;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) worst = fminf(worst, __shfl_xor_sync(0xffffffffu, worst, o));
+        const unsigned at = __ballot_sync(0xffffffffu, kept && best == worst);
+        if (at == 0) break;
+        if (lane / gs == (31 - __clz(at)) / gs) kept = false;    // ties: the higher index is dropped first
+      }
+    }
+    bool free_ = kept && v >= 0.f;
+    for (int k = 0; k < top; ++k) {
+      float bv = free_ ? v : -INFINITY;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) bv = fmaxf(bv, __shfl_xor_sync(0xffffffffu, bv, o));
+      const unsigned at = __ballot_sync(0xffffffffu, free_ && v == bv);
+      const int bi = at ? __ffs(at) - 1 : 0;                     // nothing left to choose: expert 0, as below
+      if (lane == 0) {
+        ids[(size_t)m * top + k] = bi;
+        wts[(size_t)m * top + k] = bv;
+      }
+      if (lane == bi) free_ = false;
+    }
+    return;
+  }
   if (lane == 0) {
     // serial selection (E and top are small next to the products).  Scores are in [0, 1]; an expert of a dropped group is marked
     // by s <- -1 - s, a chosen expert by s <- -3, so `s >= 0` means "can still be chosen".
