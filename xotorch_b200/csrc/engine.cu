@@ -720,21 +720,30 @@ static int launch_tc_flash(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, 
   return launch_early(e, st, fn, dim3(Hq, (S + xf::FT_Q - 1) / xf::FT_Q), xf::FT_THREADS, xf::ft_smem_bytes(HD / 64, HD / 64), 1, mq, mk, mk, mv, a);
 }
 
+// 2 .. 7 positions: about one CTA per SM, two turns of 32 keys or more each
+template <int HD, int REP>
+static int launch_tc_row_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, int pos0, float scale_log2, cudaStream_t st) {
+  auto fn = e->cfg.dtype == XOTB200_DTYPE_F16 ? xb::fp::tc_row_attn_kernel<HD, REP> : xb::bf::tc_row_attn_kernel<HD, REP>;
+  const int Hq = e->cfg.n_heads, ctas = S * Hq / REP;
+  const int shares = std::max(1, std::min(std::min(8, (pos0 + S) / (2 * 32)), (e->sm_count + ctas - 1) / ctas));
+  return launch_early(e, st, fn, dim3(shares, S, Hq / REP), 256, 0, shares, e->tc_q, kc, vc, e->tc_ao, Hq, R, e->L, pos0, scale_log2);
+}
 template <int HD>
 static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, int pos0, cudaStream_t st) {
   if (S >= 64 && e->cfg.n_heads > 1) return launch_tc_flash<HD>(e, S, R, kc, vc, pos0, st);
-  constexpr int SMEM = (64 + 4 * 64) * HD * 2;          // Q tile + 2 x (K, V) tiles
-  const bool f16 = e->cfg.dtype == XOTB200_DTYPE_F16;
-  const bool few = S < TC_FEW;
-  auto fn = few ? (f16 ? xb::fp::tc_flash_attn_kernel<HD, true> : xb::bf::tc_flash_attn_kernel<HD, true>)
-                : (f16 ? xb::fp::tc_flash_attn_kernel<HD, false> : xb::bf::tc_flash_attn_kernel<HD, false>);
-  if (int rc = ensure_smem_attr(e->device, (const void*)fn, SMEM)) return rc;
   const float scale_log2 = 1.4426950408889634f / sqrtf((float)HD);
+  if (S < TC_FEW)
+    return R % 4 == 0   ? launch_tc_row_attn<HD, 4>(e, S, R, kc, vc, pos0, scale_log2, st)
+           : R % 2 == 0 ? launch_tc_row_attn<HD, 2>(e, S, R, kc, vc, pos0, scale_log2, st)
+                        : launch_tc_row_attn<HD, 1>(e, S, R, kc, vc, pos0, scale_log2, st);
+  constexpr int SMEM = (64 + 4 * 64) * HD * 2;          // Q tile + 2 x (K, V) tiles
+  auto fn = e->cfg.dtype == XOTB200_DTYPE_F16 ? xb::fp::tc_flash_attn_kernel<HD> : xb::bf::tc_flash_attn_kernel<HD>;
+  if (int rc = ensure_smem_attr(e->device, (const void*)fn, SMEM)) return rc;
   // 8 .. 63 rows: one block per head.  Started early they find the SMs that the product in front has left already and share them, two to an SM, while others
   // stay empty: behind many keys that costs more than the launch (early / ordinary start, one 8B layer, 16 rows behind 500: 138 / 140 us, 1000: 154 / 158,
   // 2000: 191 / 182, 16000: 698 / 581; two 1B layers 156 / 150, 181 / 165, 244 / 208, 1059 / 754).
-  const int late = !few && pos0 + S > 1024 ? LAUNCH_LATE : 1;
-  return launch_early(e, st, fn, dim3(few ? S : (S + 63) / 64, e->cfg.n_heads), 128, SMEM, late, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
+  const int late = pos0 + S > 1024 ? LAUNCH_LATE : 1;
+  return launch_early(e, st, fn, dim3((S + 63) / 64, e->cfg.n_heads), 128, SMEM, late, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
 }
 
 // Prefill n_tokens positions starting at pos0 on the tensor cores, in chunks of up to e->tc_chunk tokens (layer-major
@@ -1427,16 +1436,16 @@ static int ensure_staging(xotb200_engine* e, int n) {
 // Positions from which a call runs as GEMMs (prefill_tc) instead of one after the other through the decode kernel.  A dense shard streams its
 // weights once either way for one position, and once instead of n times for more (two 8B layers, 2 positions: 364 us through the decode kernel, 239 as
 // GEMMs; 1B shape 178 and 140); a sparse-MoE shard pays its per-expert launches first.
-// Behind a long cache it is the other way round: the decode kernel spreads the keys over the chip, as GEMMs one block walks all keys of its query and
-// head.  Below TC_FEW positions the cheaper way is taken by a layer's time in us: constants fitted to both ways at 2 .. 7 positions behind 100 .. 16000
-// keys, layers of 122 MB with heads of 64 and 436 MB with heads of 128 (as GEMMs / one after the other: 2 positions behind 4000 keys 261 / 213 and
-// 144 / 98 us; 4 behind 4000 261 / 402 and 142 / 182; 4 behind 16000 705 / 529 and 397 / 238); the lines cross within a tenth of where the times do.
+// Behind a long cache both ways spread the keys over the chip, and below TC_FEW positions the cheaper one is taken by a layer's time in us: constants fitted to both at
+// 2 .. 7 positions behind 100 .. 16000 keys, layers of 122 MB with heads of 64 and 436 MB with heads of 128 (as GEMMs, with the call around it: 7 positions behind 2000 keys
+// 89 and 153 us, 8000 127 and 231, 16000 183 and 333; one after the other 4 behind 8000 215 and about 440).  Smaller layers keep the line that was drawn when one block walked all keys of its query and head.
 static bool gemms_pay(const xotb200_engine* e, int n_tokens, int pos0) {
   const xotb200_model_cfg& c = e->cfg;
   const double keys = (double)pos0 + n_tokens, kv_bytes = 4.0 * c.n_kv_heads * c.head_dim;
   const double weight_bytes = 2.0 * c.dim * ((2.0 * c.n_heads + 2.0 * c.n_kv_heads) * c.head_dim + 3.0 * c.ffn);
   const int waves = (n_tokens * c.n_heads + 2 * e->sm_count - 1) / (2 * e->sm_count);
-  return 31.0 + weight_bytes / 7.4e6 + waves * keys * (0.0056 + 0.000244 * c.head_dim) <= n_tokens * (21.0 + weight_bytes / 6.9e6 + keys * kv_bytes / 1.6e6);
+  const double attention = weight_bytes >= 1e8 ? keys * c.head_dim * (1.5e-5 + 4.8e-7 * n_tokens * c.n_heads) : waves * keys * (0.0056 + 0.000244 * c.head_dim);
+  return 31.0 + weight_bytes / 7.4e6 + attention <= n_tokens * (21.0 + weight_bytes / 6.9e6 + keys * kv_bytes / 1.6e6);
 }
 static bool runs_as_gemms(xotb200_engine* e, int n_tokens, int pos0) {
   if (e->prefill_mode != 0) return e->prefill_mode == 2;

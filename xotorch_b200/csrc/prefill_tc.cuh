@@ -32,7 +32,7 @@ enum { TCE_STORE = 0, TCE_RESID = 1, TCE_HEAD_LAST = 2, TCE_QKV = 3, TCE_SWIGLU 
 // all its rows fills the chip at once (two 8B layers: 2764 -> 2362 us a pass).  A shard without the fused epilogues, a sparse one, or one whose scratch does not fit beside the
 // weights and the caches takes 1024 (per-token scratch is twice as large, or more, there).
 constexpr int TC_CHUNK = 4096, TC_CHUNK_SMALL = 1024;
-constexpr int TC_FEW = 8;        // fewer positions than this keep what the decode kernel computes in 32 bits in 32 bits (tc_flash_attn_kernel)
+constexpr int TC_FEW = 8;        // fewer positions than this keep what the decode kernel computes in 32 bits in 32 bits (tc_row_attn_kernel)
 
 struct TcGemmArgs {
   int S;            // valid token rows of the chunk (grid.x = ceil(S/128) token tiles; HEAD_LAST: only the last tile)
