@@ -204,6 +204,7 @@ struct xotb200_lm {
   size_t trace_floats = 0, trace_cap = 0;
   int gemm_mode = 0;
   bool early = false;                                  // this step's kernels may start before the one in front has finished (launch_early)
+  bool staged = false;                                 // the next launch is the first behind the step's index arrays (launch_early)
   bool graphs_on = true;                               // decode steps are replayed from CUDA graphs
   std::map<std::array<long, 5>, GraphSlot> graphs;
   int64_t graph_replays = 0;
@@ -759,6 +760,8 @@ static bool make_map3(CUtensorMap* m, const void* ptr, long rows, long K, long l
 // finished: it waits itself (pdl_wait), its launch and what it loads ahead of that are hidden.  Such a step is a chain of some forty short
 // kernels, and the launches are most of it (one request, width 1024: 5979 -> 4913 us for 25 steps).  With many rows the kernels are long, and
 // blocks that were placed early, around a kernel still running, are spread worse over the SMs (1024 rows, width 4096: 2503 -> 2588 us).
+// The step's first kernel starts the ordinary way, behind a finished stage_in_kernel: whatever starts after it may read the staged index arrays ahead of its
+// wait (delta_row_kernel looks up the slot whose state it fetches), which an early start behind the staging kernel's last block would not order.
 template <typename... KA, typename... A>
 static int launch_early(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threads, size_t smem, int cluster, A&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -769,10 +772,11 @@ static int launch_early(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threa
   cudaLaunchAttribute at[2];
   cfg.attrs = at;
   cfg.numAttrs = 0;
-  if (e->early) {
+  if (e->early && !e->staged) {
     at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
   }
+  e->staged = false;
   if (cluster > 1) {
     at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
     at[cfg.numAttrs++].val.clusterDim = {(unsigned)cluster, 1, 1};
@@ -2911,6 +2915,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
       const int n16 = cdiv((long)off, 4);
       TRY(launch_late(e, stage_in_kernel, cdiv(std::max(n16, page_cap), 256), 256, 0, reinterpret_cast<const int4*>(e->h_stage), reinterpret_cast<int4*>(e->d_stage), n16,
                       (int)pages_off, page_cap, e->d_table));
+      e->staged = true;
       sp.tokens = e->d_stage + T0;
       sp.row_slot = e->d_stage + T0 + M;
       sp.row_pos = e->d_stage + T0 + 2 * M;

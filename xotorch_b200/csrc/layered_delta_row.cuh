@@ -8,7 +8,8 @@
 //
 // A token reads and writes dk x dv floats of state a head and does next to nothing else: bound by that traffic when there are many heads and by latency when
 // there are few.  One block of 256 threads has one (request, value head): a thread holds four neighbouring columns of RPT rows, so that a warp's accesses are whole
-// rows, and the state is on its way before the block waits for the kernel in front (it was last written in the step before, which has ended).  The sums over
+// rows, and the state is on its way before the block waits for the kernel in front (it was last written in the step before, which has ended; the slot that says where it
+// lies comes from the staged index arrays, which were complete before the step's first kernel started: launch_early).  The sums over
 // rows run over the thread's rows, then over the warps through shared memory, one barrier each.  The heads that share a query / key head are a cluster: all read the
 // shared channels' window before the first of them moves it on.
 // Measured (B200): 16 requests, 32 heads of 128 x 128 (67 MB of state a step): five launches of 54 us -> one step of it 31 us shorter; 8 requests, 32 heads of 64 x 64: four launches

@@ -21,7 +21,8 @@ typedef __nv_bfloat16 bf16;
 
 // Programmatic dependent launch: a kernel launched with that attribute may start while the one in front of it still runs.  It must not touch
 // memory which that kernel (or any before it) reads or writes until pdl_wait returns — then all of them have completed and their results are
-// visible, provided every kernel of the chain waits too.  pdl_launch_dependents lets the next kernel's blocks start as soon as there is room.
+// visible, provided every kernel of the chain waits too.  (Weights, and what was complete before the first kernel of the chain started — a request's state, the
+// staged index arrays: launch_early —, may be read ahead of it.)  pdl_launch_dependents lets the next kernel's blocks start as soon as there is room.
 // Both do nothing in a kernel launched the ordinary way.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
