@@ -83,3 +83,29 @@ def test_pages_added_by_single_row_and_by_mixed_steps():
     out.append(np.stack(got))
     eng.close()
   assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("short", [0, 1, 2, 3])
+@pytest.mark.parametrize("extra", [1, 2])
+def test_staged_arrays_that_end_where_their_buffer_does(extra, short):
+  """the staged block grows to twice what a step needs, in whole 16-byte pieces, which is also what a step copies: steps that need all of it, and up to three ints less"""
+  cfg = lu.config([lu.delta(heads=1, dim=8)], width=48, vocab=50)
+  w, page, rows = zo.random_weights(cfg, 2), 64, 1000
+
+  def ints(rows, want):                                # result pointers, tokens, slots and positions, wanted rows, one request, its new pages
+    return 4 + 3 * rows + want + 4 + 2 * -(-rows // page)
+
+  first = ints(rows, extra)
+  size = (2 * first + 3) // 4 * 4
+  long = max(m for m in range(rows, 4 * rows) if ints(m, 1) <= size - short)
+  want = 1 + size - short - ints(long, 1)
+  assert first > 2048 and ints(long, want) == size - short and want <= long
+  toks, got = lu.rand_tokens(50, long, 5), []
+  for grown in (False, True):
+    eng = lu.make_engine(cfg, w, "float32", max_tokens=4 * rows, max_requests=1, page_size=page)
+    if grown:
+      eng.step([0], [lu.rand_tokens(50, rows, 6)], want=list(range(extra)))
+      eng.clear_request(0)
+    got.append(eng.step([0], [toks], want=list(range(long - want, long)))[0])
+    eng.close()
+  assert np.isfinite(got[0]).all() and np.array_equal(*got)

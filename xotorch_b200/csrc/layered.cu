@@ -2849,7 +2849,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     if (e->h_stage) cudaFreeHost(e->h_stage);
     if (e->d_stage) cudaFree(e->d_stage);
     e->h_stage = nullptr; e->d_stage = nullptr; e->stage_cap = 0;
-    const size_t cap = std::max<size_t>(off * 2, 4096);
+    const size_t cap = (std::max<size_t>(off * 2, 4096) + 3) & ~(size_t)3;   // stage_in_kernel moves whole pieces of four
     CK(cudaHostAlloc(&e->h_stage, cap * 4, cudaHostAllocDefault));
     CK(cudaMalloc(&e->d_stage, cap * 4));
     e->stage_cap = cap;
