@@ -109,3 +109,17 @@ def test_staged_arrays_that_end_where_their_buffer_does(extra, short):
     got.append(eng.step([0], [toks], want=list(range(long - want, long)))[0])
     eng.close()
   assert np.isfinite(got[0]).all() and np.array_equal(*got)
+
+
+def test_more_wanted_rows_than_a_grid_is_high():
+  """scoring every token of a long text: all rows of one step against the same rows in portions.  Bound: sums over 48 terms through
+  a state that forgets within tens of tokens, 2^-24 sqrt(48 x 40) = 2.6e-6 of a row if all were as large as the result; four times that"""
+  cfg = lu.config([lu.delta(heads=1, dim=8)], width=48, vocab=70)
+  n = 70000
+  eng = lu.make_engine(cfg, zo.random_weights(cfg, 4), "float32", max_tokens=2 * n + 256, max_requests=2, page_size=64)
+  toks = lu.rand_tokens(70, n, 8)
+  whole, best = eng.step([0], [toks], want=list(range(n)))
+  assert whole.shape == (n, 70) and np.array_equal(best, whole.argmax(axis=1))
+  parts = np.concatenate([eng.step([1], [p], want=list(range(len(p))))[0] for p in np.split(toks, 5)])
+  eng.close()
+  assert np.isfinite(whole).all() and lu.row_err(whole, parts) < 1e-5

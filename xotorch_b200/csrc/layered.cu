@@ -1962,7 +1962,7 @@ static int run_mixer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
 static int finish_logits(xotb200_lm* e, int n_want) {
   const float scale = e->cfg.logit_scale != 0.f ? e->cfg.logit_scale : 1.0f;
   const int parts = e->cfg.vocab >= 4096 ? 8 : 1;       // blocks (a cluster) to a row
-  return launch_early(e, finish_rows_kernel, dim3(parts, n_want), 512, 0, parts, e->logits, e->cfg.vocab, scale, e->cfg.logit_softcap,
+  return launch_early(e, finish_rows_kernel, n_want * parts, 512, 0, parts, e->logits, e->cfg.vocab, n_want, parts, scale, e->cfg.logit_softcap,
                       reinterpret_cast<const StepOut*>(e->d_stage), e->d_err);
 }
 

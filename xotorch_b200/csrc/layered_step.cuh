@@ -25,14 +25,15 @@ __global__ void stage_in_kernel(const int4* __restrict__ src, int4* __restrict__
 }
 
 // finishes the logits of every row — l <- l * scale, then l <- cap * tanh(l / cap) when cap > 0 —, takes the lowest-index argmax of the row
-// (greedy sampling on the device) and sends both where the caller wants them, the step's error word behind the rows' results.  A cluster of gridDim.x blocks shares a row:
-// its reads and its writes over PCIe are in flight together (one row of 32000: 5.6 us by one block without the copy out).
-__global__ void __launch_bounds__(512) finish_rows_kernel(float* logits, int V, float scale, float cap, const StepOut* __restrict__ to, const int* __restrict__ err) {
+// (greedy sampling on the device) and sends both where the caller wants them, the step's error word behind the rows' results.  A cluster of `parts` blocks shares a row
+// (grid n_want * parts, along x: as many rows as a step may want): its reads and its writes over PCIe are in flight together (one row of 32000: 5.6 us by one block without the copy out).
+__global__ void __launch_bounds__(512) finish_rows_kernel(float* logits, int V, int n_want, int parts, float scale, float cap, const StepOut* __restrict__ to,
+                                                          const int* __restrict__ err) {
   pdl_enter();
   __shared__ float bv[32];
   __shared__ int bi[32];
-  const size_t m = blockIdx.y;
-  const int n_want = gridDim.y, rank = blockIdx.x, parts = gridDim.x;
+  const size_t m = blockIdx.x / parts;
+  const int rank = blockIdx.x % parts;
   const float* r = logits + m * V;
   const StepOut so = *to;
   float* w = so.logits ? so.logits + m * V : nullptr;
