@@ -1112,6 +1112,9 @@ static int latent_key_runs(const xotb200_lm* e, const xotb200_lm_layer& s, int n
   return cdiv(span, *run);
 }
 
+// shares of a request's keys that the row kernels merge in a cluster; more leave their sums in the key-run buffer
+constexpr int CLUSTER_SHARES = 8;
+
 // Lists of single rows over latents of 256 (or, in 16 bits, 512) entries take latent_row_kernel
 static bool latent_row_fits(const xotb200_lm* e, const xotb200_lm_layer& s, bool single) {
   const int vec = e->esz == 2 ? 8 : 4;
@@ -1213,14 +1216,14 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
     if (it.second > 0 && latent_row_fits(e, s, sp.single.at(qpi))) {
       int keys = 0;
       const int shares = latent_row_shares(e, s, it.second, sp.max_len, &keys);
-      REQUIRE(shares <= 8 || (size_t)M * H * shares * (2 + R) <= e->part_cap, "internal: the key-run buffer was not sized for this step");
+      REQUIRE(shares <= CLUSTER_SHARES || (size_t)M * H * shares * (2 + R) <= e->part_cap, "internal: the key-run buffer was not sized for this step");
       LatentRowArgs a = {};
       a.q = e->qfull; a.pool = L.pool; a.pg = pg; a.items = it.first; a.H = H; a.dr = dr; a.window = s.window; a.scale = s.scale;
-      a.gate = gate; a.gate_ld = L.n_in; a.gate_col0 = L.c_g; a.sink = sink; a.out = e->olat; a.part = shares <= 8 ? nullptr : e->part;
+      a.gate = gate; a.gate_ld = L.n_in; a.gate_col0 = L.c_g; a.sink = sink; a.out = e->olat; a.part = shares <= CLUSTER_SHARES ? nullptr : e->part;
       const dim3 grid(it.second, cdiv(H, 8), shares);
       if (R == 256) TRY((launch_latent_row<T, 256>(e, a, keys, grid)));
       else if constexpr (std::is_same<T, bf16>::value) TRY((launch_latent_row<T, 512>(e, a, keys, grid)));
-      if (shares > 8)
+      if (shares > CLUSTER_SHARES)
         TRY(launch_early(e, latent_attention_combine_kernel<T>, dim3(it.second, cdiv(qpi * H, 8), it.second * cdiv(qpi * H, 8) < e->sm_count ? std::min(16, cdiv(R, 32)) : 1), 256, 0, 1, e->part, it.first, H, R,
                          shares, gate, L.n_in, L.c_g, sink, static_cast<T*>(e->olat)));
     } else if (it.second > 0) {
@@ -1618,7 +1621,7 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
     GqaRowArgs a = {};
     int keys = 0;
     const int splits = gqa_row_shares(e, s, it.second, sp.max_len, &keys), heads = gqa_row_heads(s);
-    const bool cluster = splits <= 8;
+    const bool cluster = splits <= CLUSTER_SHARES;
     REQUIRE(cluster || (size_t)M * H * splits * (2 + dv) <= e->part_cap, "internal: the key-run buffer was not sized for this step");
     a.qf = e->qfull; a.pool = pool; a.pg = pg; a.items = it.first; a.H = H; a.G = G; a.sc = sc;
     a.gate = gate; a.gate_mode = s.out_gate; a.gate_ld = L.ld_in; a.gate_col0 = L.c_g; a.out = e->oh; a.part = cluster ? nullptr : e->part;
@@ -2793,7 +2796,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
       if (qk < 0 ? !is_long_gqa(i) : !is_long(i))
         for (int t = 0; t < counts[i]; t += q) it.push_back(Item{seqs[i].row0 + t, std::min(q, counts[i] - t), seqs[i].slot, seqs[i].pos0 + t});
     item_off[qk] = {push(it.data(), 4 * it.size()), (int)it.size()};
-    item_single[qk] = std::all_of(it.begin(), it.end(), [](const Item& i) { return i.n_rows == 1; });
+    item_single[qk] = !it.empty() && std::all_of(it.begin(), it.end(), [](const Item& i) { return i.n_rows == 1; });
     if (!it.empty() && qk > 0) sp.any_short = true;
   }
   size_t gqa_tiles_off = 0, gqa_tiles128_off = 0;
@@ -2881,12 +2884,13 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   for (auto& L : e->layers)
     if (L.s.mixer == XOTB200_LM_MIX_ATTENTION || L.s.mixer == XOTB200_LM_MIX_LATENT_ATTN) {
       const bool latent = L.s.mixer == XOTB200_LM_MIX_LATENT_ATTN;
+      const int qk = latent ? latent_rows_per_item(L.s) : -gqa_rows_per_item(L.s), items = item_off[qk].second;
+      if (items == 0) continue;                          // all rows go through the prompt attention
+      const bool row = latent ? latent_row_fits(e, L.s, item_single[qk]) : gqa_row_fits(e, L.s, item_single[qk]);
       int run = 0;
-      const int splits = latent && latent_row_fits(e, L.s, item_single[latent_rows_per_item(L.s)]) ? latent_row_shares(e, L.s, item_off[latent_rows_per_item(L.s)].second, sp.max_len, &run)
-                       : latent ? latent_key_runs(e, L.s, item_off[latent_rows_per_item(L.s)].second, sp.max_len, &run)
-                       : gqa_row_fits(e, L.s, item_single[-gqa_rows_per_item(L.s)]) ? gqa_row_shares(e, L.s, item_off[-gqa_rows_per_item(L.s)].second, sp.max_len, &run)
-                                : gqa_key_runs(e, L.s, item_off[-gqa_rows_per_item(L.s)].second, sp.max_len, &run);
-      const size_t need = splits > 1 ? (size_t)M * L.s.heads * splits * (2 + (latent ? L.s.kv_rank : L.s.vdim)) : 0;
+      const int splits = row ? (latent ? latent_row_shares(e, L.s, items, sp.max_len, &run) : gqa_row_shares(e, L.s, items, sp.max_len, &run))
+                             : (latent ? latent_key_runs(e, L.s, items, sp.max_len, &run) : gqa_key_runs(e, L.s, items, sp.max_len, &run));
+      const size_t need = splits > (row ? CLUSTER_SHARES : 1) ? (size_t)M * L.s.heads * splits * (2 + (latent ? L.s.kv_rank : L.s.vdim)) : 0;
       if (need > e->part_cap) { drop_graphs(e); TRY(regrow(e->part, need * 4)); e->part_cap = need; }
     }
   // rows of the stream, each followed by the first mixing layer's values where those cross the border
