@@ -56,6 +56,7 @@ static void set_err(const char* fmt, ...) {
     cudaError_t _e = (call);                                                               \
     if (_e != cudaSuccess) {                                                               \
       set_err("%s failed: %s (%s:%d)", #call, cudaGetErrorString(_e), __FILE__, __LINE__); \
+      cudaGetLastError(); /* reported here: not an error of the next launch */             \
       return XOTB200_ECUDA;                                                                \
     }                                                                                      \
   } while (0)
@@ -975,6 +976,8 @@ static int output_product(xotb200_lm* e, const T* A, size_t w, int K, float* you
 // ---------------------------------------------------------------------------------------------------------------------------
 // scratch
 // ---------------------------------------------------------------------------------------------------------------------------
+// A buffer that cannot be had leaves nothing behind: who regrows one (or several under one capacity) sets the capacity to 0 first and to the new one when
+// all of them are there, so that a smaller step after a failure makes them again.
 template <typename P> static int regrow(P*& p, size_t bytes) {
   if (p) { cudaFree(p); p = nullptr; }
   if (bytes == 0) return 0;
@@ -993,6 +996,7 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
   const int D = e->cfg.width;
   if (M > e->m_cap) {
     drop_graphs(e);
+    e->m_cap = 0;
     const size_t m = (size_t)std::max(M, 64), z = e->esz;
     TRY(regrow(e->x, m * D * 4 * (e->pre_scalar ? std::max(1, e->cfg.streams) : 1)));
     TRY(regrow(e->y, m * D * 4));
@@ -1046,14 +1050,16 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
   }
   if (n_want > e->want_cap) {
     drop_graphs(e);
+    e->want_cap = 0;
     const size_t w = (size_t)std::max(n_want, 16);
     TRY(regrow(e->hw, w * D * e->esz));
     TRY(regrow(e->logits, w * e->cfg.vocab * 4));
     e->want_cap = (int)w;
   }
   if (e->trace && e->trace_cap < (size_t)e->layers.size() * e->m_cap * D) {
+    e->trace_cap = 0;
+    TRY(regrow(e->trace_buf, (size_t)e->layers.size() * e->m_cap * D * 4));
     e->trace_cap = (size_t)e->layers.size() * e->m_cap * D;
-    TRY(regrow(e->trace_buf, e->trace_cap * 4));
   }
   return 0;
 }
@@ -1061,6 +1067,7 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
 static int ensure_host_out(xotb200_lm* e, size_t floats) {
   if (floats <= e->h_out_cap) return 0;
   drop_graphs(e);
+  e->h_out_cap = 0;
   if (e->h_out) { cudaFreeHost(e->h_out); e->h_out = nullptr; }
   CK(cudaHostAlloc(&e->h_out, floats * 4, cudaHostAllocDefault));
   e->h_out_cap = floats;
@@ -1672,7 +1679,7 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
       if (s.chunk > 0) dist_n = std::min(dist_n, s.chunk + 64);
       if (s.window > 0) dist_n = std::min(dist_n, s.window + 64);
       if (s.dist_bias) {
-        if ((size_t)H * dist_n > e->dist_cap) { TRY(regrow(e->dist_tab, (size_t)H * dist_n * 4)); e->dist_cap = (size_t)H * dist_n; }
+        if ((size_t)H * dist_n > e->dist_cap) { e->dist_cap = 0; TRY(regrow(e->dist_tab, (size_t)H * dist_n * 4)); e->dist_cap = (size_t)H * dist_n; }
         TRY(launch_early(e, gqa_dist_table_kernel, cdiv((long)H * dist_n, 256), 256, 0, 1, at<bf16>(e, L.r1), at<bf16>(e, L.r2), H, dist_n, e->dist_tab));
       }
       CUtensorMap mq, mkv;
@@ -2839,6 +2846,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   }
   if (flash_keys > e->flash_keys_cap) {
     const size_t cap = std::max<size_t>(flash_keys, 1024);
+    e->flash_keys_cap = 0;
     TRY(regrow(e->cbuf, cap * e->max_w * 2));
     TRY(regrow(e->knx, cap * e->max_hdn * 2));
     TRY(regrow(e->vxx, cap * e->max_oh * 2));
@@ -2891,7 +2899,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
       const int splits = row ? (latent ? latent_row_shares(e, L.s, items, sp.max_len, &run) : gqa_row_shares(e, L.s, items, sp.max_len, &run))
                              : (latent ? latent_key_runs(e, L.s, items, sp.max_len, &run) : gqa_key_runs(e, L.s, items, sp.max_len, &run));
       const size_t need = splits > (row ? CLUSTER_SHARES : 1) ? (size_t)M * L.s.heads * splits * (2 + (latent ? L.s.kv_rank : L.s.vdim)) : 0;
-      if (need > e->part_cap) { drop_graphs(e); TRY(regrow(e->part, need * 4)); e->part_cap = need; }
+      if (need > e->part_cap) { drop_graphs(e); e->part_cap = 0; TRY(regrow(e->part, need * 4)); e->part_cap = need; }
     }
   // rows of the stream, each followed by the first mixing layer's values where those cross the border
   auto copy_rows = [&](float* dst, size_t dld, const float* src, size_t sld, size_t n, cudaMemcpyKind kind) -> int {
