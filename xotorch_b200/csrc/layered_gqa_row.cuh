@@ -117,6 +117,8 @@ __global__ void __launch_bounds__(GROW_THREADS) gqa_row_kernel(const GqaRowArgs 
           for (int e = 0; e < VEC; ++e) acc[r][p * VEC + e] = fmaf(wr, ldf(reinterpret_cast<const T*>(&x[p]) + e), acc[r][p * VEC + e]);
     }
   }
+  // From here on sums are merged without a look at their weights: who saw no key has parked zeros, and who saw keys whose scores are all NaN (its maximum is still -inf, its
+  // weight 0) must not drop out of the denominator.
   // the warp's four keys of every turn: one maximum, sums over the groups; lane group i ends with a quarter of the entries
   float wm = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
   wm = fmaxf(wm, __shfl_xor_sync(0xffffffffu, wm, 16));
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(GROW_THREADS) gqa_row_kernel(const GqaRowArgs 
     const float fr = __shfl_sync(0xffffffffu, f, (lane & 24) + r);
     float t[DPL];
 #pragma unroll
-    for (int d = 0; d < DPL; ++d) t[d] = fr == 0.f ? 0.f : acc[r][d] * fr;
+    for (int d = 0; d < DPL; ++d) t[d] = acc[r][d] * fr;
 #pragma unroll
     for (int d = 0; d < DPL / 2; ++d) t[d] = (up16 ? t[d + DPL / 2] : t[d]) + __shfl_xor_sync(0xffffffffu, up16 ? t[d] : t[d + DPL / 2], 16);
 #pragma unroll
@@ -153,7 +155,8 @@ __global__ void __launch_bounds__(GROW_THREADS) gqa_row_kernel(const GqaRowArgs 
 #pragma unroll
     for (int w = 0; w < 8; ++w) {
       const float c = scale(sm[w][r], top);
-      if (c != 0.f) { o = fmaf(c, so[w][r][d], o); dn = fmaf(c, sd[w][r], dn); }
+      o = fmaf(c, so[w][r][d], o);
+      dn = fmaf(c, sd[w][r], dn);
     }
     so[8][r][d] = o;
     if (d == 0) { sm[8][r] = top; sd[8][r] = dn; }
@@ -190,7 +193,8 @@ __global__ void __launch_bounds__(GROW_THREADS) gqa_row_kernel(const GqaRowArgs 
       for (int c = 0; c < 8; ++c)
         if (c < nz) {
           const float w = scale(mi[c], top);
-          if (w != 0.f) { o = fmaf(w, oi[c], o); dn = fmaf(w, di[c], dn); }
+          o = fmaf(w, oi[c], o);
+          dn = fmaf(w, di[c], dn);
         }
     }
     const float corr = sc.sink || sc.sink_one ? apply_sink(gqa_sink_score<T>(sc.sink, h), top, dn) : 1.0f;

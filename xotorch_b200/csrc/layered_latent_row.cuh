@@ -88,12 +88,14 @@ __global__ void __launch_bounds__(LROW_THREADS) latent_row_kernel(const LatentRo
       if (corr != 1.f)
 #pragma unroll
         for (int d = 0; d < DPL; ++d) acc[d] *= corr;
-      if (w != 0.f)
+      if (on)
 #pragma unroll
         for (int p = 0; p < NP; ++p)
 #pragma unroll
           for (int e = 0; e < VEC; ++e) acc[p * VEC + e] = fmaf(w, ldf(reinterpret_cast<const T*>(&k[p]) + e), acc[p * VEC + e]);
     }
+    // From here on sums are merged without a look at their weights: who saw no key has parked zeros, and who saw keys whose scores are all NaN (its maximum is still
+    // -inf, its weight 0) must not drop out of the denominator.
     // the warp: one maximum, sums over the four keys of every turn; lane group i ends with a quarter of the entries
     float top = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
@@ -105,7 +107,7 @@ __global__ void __launch_bounds__(LROW_THREADS) latent_row_kernel(const LatentRo
     if (lane == 0) { sm[warp] = top; sd[warp] = den; }
     const bool up16 = lane & 16, up8 = lane & 8;
 #pragma unroll
-    for (int d = 0; d < DPL; ++d) acc[d] = f == 0.f ? 0.f : acc[d] * f;
+    for (int d = 0; d < DPL; ++d) acc[d] *= f;
 #pragma unroll
     for (int d = 0; d < DPL / 2; ++d) acc[d] = (up16 ? acc[d + DPL / 2] : acc[d]) + __shfl_xor_sync(0xffffffffu, up16 ? acc[d] : acc[d + DPL / 2], 16);
 #pragma unroll
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(LROW_THREADS) latent_row_kernel(const LatentRo
         if (c < nz) top = fmaxf(top, ms[c]);
 #pragma unroll
       for (int c = 0; c < 8; ++c)
-        if (c < nz) { ms[c] = ms[c] == -INFINITY ? 0.f : expf(ms[c] - top); dn = ms[c] == 0.f ? dn : fmaf(ms[c], ds[c], dn); }
+        if (c < nz) { ms[c] = ms[c] == -INFINITY ? 0.f : expf(ms[c] - top); dn = fmaf(ms[c], ds[c], dn); }
     } else {
       __syncwarp();
       top = sm[warp];
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(LROW_THREADS) latent_row_kernel(const LatentRo
           if (c < nz) v[c] = ld_dsmem_f32(xb::smem_u32(so + warp * R + d), c);
 #pragma unroll
         for (int c = 0; c < 8; ++c)
-          if (c < nz && ms[c] != 0.f) o = fmaf(ms[c], v[c], o);
+          if (c < nz) o = fmaf(ms[c], v[c], o);
       } else {
         o = so[warp * R + d];
       }
