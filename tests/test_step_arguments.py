@@ -48,3 +48,29 @@ def test_hidden_rows_and_a_row_list_too_short():
   assert s.lib.seen == ([1, 0], [2, 1], [0, 1, 2, 3, 4, 5, 1, 1, 1], [], False, False, True) and out.shape == (3, 3)
   with pytest.raises(ValueError):
     s.step([1, 0], [np.ones(3)])
+
+
+@pytest.mark.parametrize("want", [[[4, 0]], [[4], [0]], ((4,), (0,)), [np.int64(4), np.int32(0)], [np.array([4, 0])], np.array([[4], [0]]), [4.0, 0.0]])
+def test_wanted_rows_of_any_shape(want):
+  s = shard()
+  lg, am = s.step([7, 0, 3], [[1, 2, 3], [4], [5, 6]], want=want)
+  assert s.lib.seen[3] == [4, 0] and lg.shape == (2, 5) and am.shape == (2,)
+
+
+def test_slots_in_a_column():
+  s = shard()
+  s.step(np.array([[7], [0]]), [[1, 2, 3], [4]])
+  assert s.lib.seen[:4] == ([7, 0], [3, 1], [1, 2, 3, 4], [2, 3])
+
+
+def test_rows_beyond_the_slots_are_not_served():
+  s = shard()
+  lg, _ = s.step([7, 0], [[1, 2, 3], [4], [5, 6]], want=[3, 2])
+  assert s.lib.seen[:4] == ([7, 0], [3, 1], [1, 2, 3, 4], [3, 2]) and lg.shape == (2, 5)
+  s.step([7, 0], [[1, 2, 3], [4], [5, 6]])               # the last rows of all three: the native step refuses the one that is not there
+  assert s.lib.seen[3] == [2, 3, 5]
+  s.step([7], [[1, 2], [4]])
+  assert s.lib.seen[:3] == ([7], [2], [1, 2])
+  s = shard(first=False, last=False)
+  out = s.step([1], [np.arange(6).reshape(2, 3), np.ones(3)])
+  assert s.lib.seen[:3] == ([1], [2], [0, 1, 2, 3, 4, 5]) and out.shape == (3, 3)

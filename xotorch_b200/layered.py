@@ -571,24 +571,28 @@ class LayeredShard:
   def step(self, slots: Sequence[int], rows: Sequence[np.ndarray], want: Optional[Sequence[int]] = None, logits: bool = True,
            argmax: bool = True):
     """One batched step.  rows[i]: the next token ids (1-D int) of slot slots[i] on the first shard, else its hidden state
-    [n_i, hidden_in] float32 (the stream, `width` floats, and whatever else an earlier shard hands over: see xotb200_lm_hidden_width).  want: packed row indices whose output is asked for (default: every request's last row).
+    [n_i, hidden_in] float32 (the stream, `width` floats, and whatever else an earlier shard hands over: see xotb200_lm_hidden_width).  Entries of `rows` beyond the slots are not served
+    (the hidden rows of a middle shard keep their places for them).  want: packed row indices whose output is asked for, of any shape (default: every request's last row).
     Last shard -> (logits [n_want, vocab] float32 | None, argmax [n_want] int32 | None); other shards -> hidden [sum n_i, hidden_out]."""
     # a decode step is 150 to 600 us on the device: the arrays of this call are few, and their addresses are handed on as plain ints
     n_seq, first, last = len(slots), self.is_first, self.is_last
-    if len(rows) != n_seq:
+    if len(rows) < n_seq:
       raise ValueError(f"{n_seq} slots, but rows for {len(rows)}")
     if first:
       parts = [r if type(r) is np.ndarray and r.dtype == _INT32 and r.ndim == 1 else np.asarray(r, dtype=np.int32).reshape(-1) for r in rows]
     else:
       parts = [np.asarray(r, dtype=np.float32).reshape(-1, self.hidden_in) for r in rows]
     counts = [len(p) for p in parts]
-    data = np.ascontiguousarray(parts[0]) if n_seq == 1 else np.concatenate(parts) if parts else np.zeros(0, np.int32 if first else np.float32)
+    data = np.ascontiguousarray(parts[0]) if len(parts) == 1 else np.concatenate(parts) if parts else np.zeros(0, np.int32 if first else np.float32)
     if want is None:
       want = [w - 1 for w in accumulate(counts)]
-    elif not isinstance(want, list):
-      want = np.asarray(want).reshape(-1).tolist()
+    elif type(want) is not list or any(type(w) is not int for w in want):
+      want = np.asarray(want, dtype=np.int32).reshape(-1).tolist()
     n_want = len(want)
-    ints = np.array([*slots, *counts, *want], dtype=np.int32)
+    try:
+      ints = np.array([*slots, *counts[:n_seq], *want], dtype=np.int32)
+    except ValueError:                                   # slots in an array of more than one dimension
+      ints = np.concatenate([np.asarray(v, dtype=np.int32).reshape(-1) for v in (slots, counts[:n_seq], want)])
     at, data_at = _address(ints), _address(data)
     lg = am = ho = None
     if last:
