@@ -113,6 +113,29 @@ def test_a_long_cache_is_left_to_the_decode_kernel():
   eng.close()
 
 
+@pytest.mark.parametrize("dims", [dict(dim=1024, ffn=3072, n_heads=16, n_kv_heads=4), dict(dim=2048, ffn=5632, n_heads=32, n_kv_heads=8)])
+def test_layers_of_24_and_90_mb_behind_a_long_cache(dims):
+  """both ways spread the keys, and the GEMMs are the cheaper one: few positions run as they do, close to what the decode kernel gives"""
+  from dataclasses import replace
+  from xotorch_b200.native import NativeShard
+  shape = replace(PRESETS["tiny-llama-hd64"], name="small-llama", **dims)
+  eng = NativeShard(hf_config(shape), 0)
+  eng.set_shard(1, 1)
+  eng.init_synthetic(11)
+  eng.begin_request(2048)
+  h = torch.randn(2048, shape.dim, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+  run(eng, h[:2040].clone(), 0)
+  for n in (2, 3):
+    before, out = eng.kernel_launches(), []
+    for mode in (0, 1):
+      eng.set_prefill_mode(mode)
+      out.append(run(eng, h[2040:2040 + n].clone(), 2040))
+      if mode == 0:
+        assert eng.kernel_launches() - before > n
+    assert np.linalg.norm(out[0] - out[1]) <= 2.0 ** -6 * np.linalg.norm(out[1])   # a layer's products round to 8 bits on both sides
+  eng.close()
+
+
 def test_without_memory_for_the_scratch_of_the_gemms():
   """the decode kernel takes the call, as it needs no scratch; once there is memory the GEMMs do"""
   from dataclasses import replace

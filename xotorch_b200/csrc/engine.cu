@@ -1437,14 +1437,17 @@ static int ensure_staging(xotb200_engine* e, int n) {
 // weights once either way for one position, and once instead of n times for more (two 8B layers, 2 positions: 364 us through the decode kernel, 239 as
 // GEMMs; 1B shape 178 and 140); a sparse-MoE shard pays its per-expert launches first.
 // Behind a long cache both ways spread the keys over the chip, and below TC_FEW positions the cheaper one is taken by a layer's time in us: constants fitted to both at
-// 2 .. 7 positions behind 100 .. 16000 keys, layers of 122 MB with heads of 64 and 436 MB with heads of 128 (as GEMMs, with the call around it: 7 positions behind 2000 keys
-// 89 and 153 us, 8000 127 and 231, 16000 183 and 333; one after the other 4 behind 8000 215 and about 440).  Smaller layers keep the line that was drawn when one block walked all keys of its query and head.
+// 2 .. 7 positions behind 100 .. 16000 keys, layers of 122 MB with heads of 64 and 436 MB with heads of 128.  Measured on layers of 24 to 436 MB, 2, 4 and 7 positions
+// behind 30 .. 16000 keys, the line takes the cheaper way everywhere but at 2 positions behind 16000 keys, 46 MB with heads of 128 (GEMMs / one after the other, us a
+// layer: 2 positions behind 16000 keys, 24 MB 70 / 86, 46 MB 86 / 124, 122 MB 104 / 125, 436 MB 184 / 268; 4 behind 4000, 24 MB 50 / 128, 68 MB 63 / 171, 436 MB 145 / 391).
+// Layers under 10 MB, models of a test's size, keep the line of an attention that walked all keys of a query in one block, although GEMMs are cheaper there too (2
+// positions behind 2000 keys, 6 MB: 39 / 57): behind a long cache their few positions come out bit for bit as one after the other.
 static bool gemms_pay(const xotb200_engine* e, int n_tokens, int pos0) {
   const xotb200_model_cfg& c = e->cfg;
   const double keys = (double)pos0 + n_tokens, kv_bytes = 4.0 * c.n_kv_heads * c.head_dim;
   const double weight_bytes = 2.0 * c.dim * ((2.0 * c.n_heads + 2.0 * c.n_kv_heads) * c.head_dim + 3.0 * c.ffn);
   const int waves = (n_tokens * c.n_heads + 2 * e->sm_count - 1) / (2 * e->sm_count);
-  const double attention = weight_bytes >= 1e8 ? keys * c.head_dim * (1.5e-5 + 4.8e-7 * n_tokens * c.n_heads) : waves * keys * (0.0056 + 0.000244 * c.head_dim);
+  const double attention = weight_bytes >= 1e7 ? keys * c.head_dim * (1.5e-5 + 4.8e-7 * n_tokens * c.n_heads) : waves * keys * (0.0056 + 0.000244 * c.head_dim);
   return 31.0 + weight_bytes / 7.4e6 + attention <= n_tokens * (21.0 + weight_bytes / 6.9e6 + keys * kv_bytes / 1.6e6);
 }
 static bool runs_as_gemms(xotb200_engine* e, int n_tokens, int pos0) {
