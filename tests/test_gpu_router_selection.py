@@ -1,8 +1,10 @@
-"""Softmax routers with up to 32 experts choose with a warp, more with one lane: both must choose what the definition says (groups' best scores, ties to the lower index), bit for bit the
-same weights, for expert counts around a warp, every number of groups and of kept groups, and scores with ties."""
+"""Softmax routers with up to 32 experts choose with a warp, more with one lane: both must choose what the definition says (groups' best scores, ties to the lower index) and weigh the chosen by
+their scores, for expert counts around a warp, every number of groups and of kept groups, and scores with ties.  Every expert has matrices of its own, so a choice shows in the
+output; the oracle's own order among equals is not defined, which is why the first test cuts no pair of equals and the second states the order itself."""
 
 import numpy as np
 import pytest
+import torch
 
 pytestmark = pytest.mark.gpu
 
@@ -28,3 +30,34 @@ def test_choice(experts, groups, keep, top, ties):
   eng.close()
   ok = [lu.row_err(g, ref) < lu.TOL["float32"] for g in (whole, single)]
   assert all(ok)
+
+
+def lower_index_first(h, w_router, r):
+  """the definition with its order among equals: sorts that keep equals in place, and logits whose sums do not depend on where a row of the router lies"""
+  E, top, gr = r["experts"], r["top"], r.get("groups")
+  s = torch.softmax((h[:, None, :] * w_router[None]).sum(-1), dim=-1)
+  free = torch.ones_like(s, dtype=torch.bool)
+  if gr and gr["count"] > 1:
+    best = s.reshape(-1, gr["count"], E // gr["count"]).amax(-1)
+    kept = torch.zeros_like(best, dtype=torch.bool).scatter_(1, best.sort(dim=-1, descending=True, stable=True).indices[:, :gr["keep"]], True)
+    free = kept.repeat_interleave(E // gr["count"], dim=1)
+  idx = s.masked_fill(~free, -1.0).sort(dim=-1, descending=True, stable=True).indices[:, :top]
+  return idx, s.gather(1, idx)
+
+
+@pytest.mark.parametrize("equals", ["pairs", "groups", "all"])
+@pytest.mark.parametrize("experts,groups,keep,top", [(8, 1, 1, 3), (8, 4, 2, 3), (16, 4, 2, 5), (16, 8, 3, 1), (31, 1, 1, 5), (32, 4, 3, 7), (32, 16, 5, 3), (48, 6, 2, 5), (64, 1, 1, 3)])
+def test_ties_go_to_the_lower_index(experts, groups, keep, top, equals, monkeypatch):
+  """equal scores: an expert and its neighbour (top cuts a pair), a group and all others (kept is less than their number), all experts"""
+  cfg = bu.config([bu.attention(mlp=bu.moe(experts=experts, top=top, groups=(groups, keep), ff=16))], width=32, vocab=60)
+  w = bo.random_weights(cfg, experts + top)
+  own = {"pairs": torch.arange(experts) // 2 * 2, "groups": torch.arange(experts) % (experts // groups), "all": torch.zeros(experts, dtype=torch.long)}[equals]
+  w["l0.mlp.router"] = w["l0.mlp.router"][own].clone()
+  toks = lu.rand_tokens(60, 12, 3)
+  monkeypatch.setattr(bo, "route", lower_index_first)
+  ref = bu.oracle_logits(cfg, w, toks)[0]
+  eng = lu.make_engine(cfg, w, "float32")
+  whole = eng.step([0], [toks], want=list(range(12)))[0]
+  single = np.concatenate([eng.step([1], [toks[i:i + 1]])[0] for i in range(12)])
+  eng.close()
+  assert lu.row_err(whole, ref) < lu.TOL["float32"] and lu.row_err(single, ref) < lu.TOL["float32"]

@@ -14,14 +14,16 @@ from tests import bufulorn_oracle as bo, bufulorn_util as bu, layered_util as lu
 def test_gated_delta_in_portions(dim, vdim, conv, cut):
   cfg = bu.config([bu.delta(heads=4, kv_heads=2, dim=dim, vdim=vdim, conv=conv)], width=48, vocab=50)
   w = bo.random_weights(cfg, dim + conv)
-  toks = [lu.rand_tokens(50, sum(cut), 3 + r) for r in range(2)]
+  cuts = [cut, [cut[0] + 1, *cut[1:]]]                 # the second request is a row ahead after the first portion
+  toks = [lu.rand_tokens(50, sum(c), 3 + r) for r, c in enumerate(cuts)]
   eng = lu.make_engine(cfg, w, "float32", max_tokens=1024, max_requests=2)
-  got, at = [[], []], 0
-  for n in cut:                                        # the second request stays a row behind after the first portion
-    rows = [t[at:at + n] for t in toks]
-    lg = eng.step([1, 0], rows, want=list(range(2 * n)))[0]
-    got[0].append(lg[:n]), got[1].append(lg[n:])
-    at += n
+  got, at = [[], []], [0, 0]
+  for portion in zip(*cuts):
+    rows = [t[a:a + n] for t, a, n in zip(toks, at, portion)]
+    lg = eng.step([1, 0], rows, want=list(range(sum(portion))))[0]
+    for g, part in zip(got, np.split(lg, [portion[0]])):
+      g.append(part)
+    at = [a + n for a, n in zip(at, portion)]
   eng.close()
   for t, g in zip(toks, got):
     assert lu.row_err(np.concatenate(g), bu.oracle_logits(cfg, w, t)[0]) < 2.4e-5   # as in the chunk tests

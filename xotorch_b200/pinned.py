@@ -1,7 +1,8 @@
 """Result arrays in page-locked host memory.
 
-A step's results (logits, hidden states) reach the host by DMA.  Into an ordinary numpy array that takes a second copy on the CPU — and, for a fresh
-array, the page faults of its memory; into page-locked memory the DMA is all there is.  `ResultPool.empty` hands out ordinary numpy arrays over
+A step's results (logits, hidden states) reach the host over PCIe.  Into an ordinary numpy array that takes a staging buffer and a second copy on the CPU — and, for a
+fresh array, the page faults of its memory; into page-locked memory they go directly: hidden states, and the shard engine's logits, by DMA, the layered engine's logits
+by the stores of its last kernel, which takes blocks of this library alone (their bounds are known).  `ResultPool.empty` hands out ordinary numpy arrays over
 page-locked blocks: when the last reference to an array (or a view of it) is gone, its block goes back to the pool and is handed out again.
 The pool is bounded (`limit` bytes in use and kept together; beyond it, and where page-locked memory cannot be had, plain arrays are handed out),
 blocks are taken and given back by any thread, and an array outlives the engine that filled it."""
