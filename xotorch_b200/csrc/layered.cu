@@ -207,7 +207,7 @@ struct xotb200_lm {
   bool early = false;                                  // this step's kernels may start before the one in front has finished (launch_early)
   bool staged = false;                                 // the next launch is the first behind the step's index arrays (launch_early)
   bool graphs_on = true;                               // decode steps are replayed from CUDA graphs
-  std::map<std::array<long, 5>, GraphSlot> graphs;
+  std::map<std::array<long, 6>, GraphSlot> graphs;
   int64_t graph_replays = 0;
   bool flash_fits = true;                              // every attention layer fits the expanded kernel's tile sizes
   bool gqa_flash_fits = true;                          // every key/value-cache attention layer fits the tensor-core prompt kernel (16-byte rows)
@@ -792,8 +792,10 @@ static int launch_early(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threa
 // whose blocks are smaller, gain by the early start up to runs of GQA_EARLY_RUN keys (one / four requests behind 250: 162 / 176 against 167 / 178 us; behind
 // 4000: 202 / 295 against 186 / 264).
 constexpr int GQA_EARLY_RUN = 64;
-constexpr int LATENT_ROW_EARLY = 64;                   // keys of a block of latent_row_kernel up to which it starts early (no difference measured up to 128)
-constexpr int GQA_ROW_EARLY = 128;                     // keys of a block of gqa_row_kernel up to which it starts early (no difference measured at 64; behind long caches as above)
+// Keys of a block of a row kernel up to which it starts early.  latent_row_kernel: no difference measured beyond 1.5 us either way (one and two requests, 16 and 32 heads, behind 30 .. 16000 tokens).
+// gqa_row_kernel: none up to 128 keys; beyond, many blocks lose (32 + 8 heads of 128, a layer, early / the ordinary way: 16 requests behind 1000 tokens 99.9 / 99.3 us, 2000
+// 163.5 / 156.8, 8000 490.5 / 458.5; one request behind 8000 74.7 / 74.9).
+constexpr int LATENT_ROW_EARLY = 64, GQA_ROW_EARLY = 128;
 template <typename... KA, typename... A>
 static int launch_late(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int threads, size_t smem, A&&... args) {
   kern<<<grid, threads, smem, e->stream>>>(static_cast<KA>(args)...);
@@ -1094,6 +1096,7 @@ struct StepPlan {
   };
   std::map<int, Flash> flash;
   int max_len = 0;                                     // longest request after this step (bounds every key range)
+  int longest = 0;                                     // the same, where max_len of a captured step is rounded up
   int max_rows = 0;                                    // most rows one request brings
   const GqaTile* gqa_tiles = nullptr;                  // key/value-cache attention, long portions (bf16): 64-row tiles
   int n_gqa_tiles = 0;
@@ -1122,14 +1125,27 @@ static int latent_key_runs(const xotb200_lm* e, const xotb200_lm_layer& s, int n
 // shares of a request's keys that the row kernels merge in a cluster; more leave their sums in the key-run buffer
 constexpr int CLUSTER_SHARES = 8;
 
-// Lists of single rows over latents of 256 (or, in 16 bits, 512) entries take latent_row_kernel
-static bool latent_row_fits(const xotb200_lm* e, const xotb200_lm_layer& s, bool single) {
+static int latent_row_span(const xotb200_lm_layer& s, int max_len) { return std::max(1, s.window > 0 ? std::min(max_len, s.window) : max_len); }
+// Lists of single rows over latents of 256 (or, in 16 bits, 512) entries — the ranks it is instantiated for — take latent_row_kernel while it is the faster one: each of its
+// blocks of eight heads reads the cached rows anew, where the general kernel stages them once for up to 32 heads, so it wins by its shorter chain while blocks x keys are
+// few.  `longest`: cached tokens of the longest request, not the length that a captured step is planned for.  Measured (B200, a layer, a step, this / the general kernel):
+//   latents of 512, 32 heads:  1 request (4 blocks) behind 200 tokens 53 / 59 us, 4000 84 / 102, 16000 174 / 241;  4 requests behind 150 66 / 69, 300 73 / 69, 2000 153 / 110;
+//                              16 requests behind 16 67 / 73, 60 74 / 72, 2000 374 / 219
+//   latents of 512, 16 heads:  2 requests (4 blocks) behind 16000 178 / 244;  8 behind 150 64 / 67, 500 81 / 81;  16 behind 16 62 / 68, 300 89 / 81, 8000 821 / 636
+//   latents of 512, 64 heads:  1 request (8 blocks) behind 200 59 / 67, 2000 108 / 83;   latents of 256, 32 heads, 4 requests behind 200 61 / 66, 500 70 / 71
+//   one block per request, latents of 256, 8 heads: 1 request behind 16 .. 100 44.5 / 44.6, 2000 57 / 54;  16 behind 16 55 / 57, 150 61 / 57, 8000 302 / 179
+// Short portions at 32 heads or more, whose lists are of single rows too, follow the same line (32 heads, 512: 2 rows behind 30 62 / 73, 15 rows behind 30 109 / 96, 8 rows behind 8000 822 / 394).
+constexpr int LATENT_ROW_ALWAYS = 4, LATENT_ROW_WORK = 3200, LATENT_ROW_ONE_BLOCK = 128;   // blocks; blocks x keys; keys where a request is one block
+static bool latent_row_pays(const xotb200_lm* e, const xotb200_lm_layer& s, bool single, int n_items, int longest) {
   const int vec = e->esz == 2 ? 8 : 4;
-  return single && (s.kv_rank == 256 || (s.kv_rank == 512 && e->esz == 2)) && s.rot_dim % vec == 0 && s.rot_dim <= 8 * vec;
+  if (!single || !(s.kv_rank == 256 || (s.kv_rank == 512 && e->esz == 2)) || s.rot_dim % vec != 0 || s.rot_dim > 8 * vec) return false;
+  const long blocks = (long)n_items * cdiv(s.heads, 8), keys = latent_row_span(s, longest);
+  if (s.heads > 8) return blocks <= LATENT_ROW_ALWAYS || blocks * keys <= LATENT_ROW_WORK;
+  return keys <= LATENT_ROW_ONE_BLOCK && blocks * keys <= LATENT_ROW_WORK;
 }
 // its shares of the keys: about one block per SM, four turns of four keys or more each
 static int latent_row_shares(const xotb200_lm* e, const xotb200_lm_layer& s, int n_items, int max_len, int* keys) {
-  const int span = std::max(1, s.window > 0 ? std::min(max_len, s.window) : max_len);
+  const int span = latent_row_span(s, max_len);
   const long ctas = std::max(1L, (long)n_items * cdiv(s.heads, 8));
   const int shares = (int)std::max(1L, std::min(std::min(32L, (long)cdiv(span, 4 * LROW_KEYS)), (e->sm_count + ctas - 1) / ctas));
   *keys = cdiv(span, shares);
@@ -1220,7 +1236,7 @@ static int attention_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
                                  dn, H)));
     const int qpi = latent_rows_per_item(s);
     const auto& it = sp.items.at(qpi);
-    if (it.second > 0 && latent_row_fits(e, s, sp.single.at(qpi))) {
+    if (it.second > 0 && latent_row_pays(e, s, sp.single.at(qpi), it.second, sp.longest)) {
       int keys = 0;
       const int shares = latent_row_shares(e, s, it.second, sp.max_len, &keys);
       REQUIRE(shares <= CLUSTER_SHARES || (size_t)M * H * shares * (2 + R) <= e->part_cap, "internal: the key-run buffer was not sized for this step");
@@ -1499,16 +1515,31 @@ static int gqa_key_runs(const xotb200_lm* e, const xotb200_lm_layer& s, int n_it
   return cdiv(span, *run);
 }
 
-// Lists of single rows over heads of 64 or 128 entries (keys and values alike) take gqa_row_kernel
-static bool gqa_row_fits(const xotb200_lm* e, const xotb200_lm_layer& s, bool single) { return single && s.dim == s.vdim && (s.dim == 64 || s.dim == 128); }
-static int gqa_row_heads(const xotb200_lm_layer& s) { const int rep = s.heads / s.kv_heads; return rep % 4 == 0 ? 4 : rep % 2 == 0 ? 2 : 1; }
-// its shares of the keys: about one block per SM, two turns of 32 keys or more each
-static int gqa_row_shares(const xotb200_lm* e, const xotb200_lm_layer& s, int n_items, int max_len, int* keys) {
+// keys that a row meets at most
+static int gqa_row_span(const xotb200_lm_layer& s, int max_len) {
   int span = std::max(1, max_len);
   if (s.window > 0) span = std::min(span, s.window);
   if (s.chunk > 0) span = std::min(span, s.chunk);
   if (s.keep_first > 0) span += std::min(s.keep_first, std::max(1, max_len));
   if (s.pool > 0) span += std::max(1, max_len) / s.pool;
+  return span;
+}
+// Lists of single rows over heads of 64 or 128 entries (keys and values alike; the sizes it is instantiated for) take gqa_row_kernel, but where 16 or more heads of 128 share a
+// key head: its blocks have four heads and read the same keys four times and more, where the general kernel stages them once.  That one wins then from 256 keys on,
+// while it has enough blocks to spread (more than 2) and not so many that it runs in waves (16).  Measured (B200, a layer, a step, this / the general kernel):
+//   32 heads on 1: 1 request behind 2000 tokens 50 / 60 us, 8000 78 / 121;  4 requests behind 30 41 / 51, 300 49 / 51, 2000 78 / 64, 8000 172 / 126;  16 behind 8000 403 / 365
+//   32 heads on 2: 1 behind 8000 77 / 95;  4 behind 2000 79 / 73;  16 behind 2000 129 / 147, 8000 416 / 585
+//   16 heads on 1: 2 behind 8000 78 / 96;  8 behind 30 41 / 49, 1000 65 / 59, 8000 175 / 159
+//   4 and 8 heads on one, heads of 128: 4 requests behind 2000 79 / 120 and 82 / 93, 16 behind 8000 463 / 1590 and 460 / 964;  32 heads of 64 on 1: 4 behind 2000 55 / 55, 16 behind 8000 201 / 248
+static bool gqa_row_pays(const xotb200_lm_layer& s, bool single, int n_items, int longest) {
+  if (!single || s.dim != s.vdim || (s.dim != 64 && s.dim != 128)) return false;
+  const long tiles = (long)n_items * s.kv_heads;         // blocks of the general kernel that share out the keys
+  return s.dim == 64 || s.heads / s.kv_heads < 16 || gqa_row_span(s, longest) <= 256 || tiles <= 2 || tiles > 16;
+}
+static int gqa_row_heads(const xotb200_lm_layer& s) { const int rep = s.heads / s.kv_heads; return rep % 4 == 0 ? 4 : rep % 2 == 0 ? 2 : 1; }
+// its shares of the keys: about one block per SM, two turns of 32 keys or more each
+static int gqa_row_shares(const xotb200_lm* e, const xotb200_lm_layer& s, int n_items, int max_len, int* keys) {
+  const int span = gqa_row_span(s, max_len);
   const long ctas = std::max(1L, (long)n_items * s.heads / gqa_row_heads(s));
   const int shares = (int)std::max(1L, std::min(std::min(32L, (long)cdiv(span, 2 * GROW_KEYS)), (e->sm_count + ctas - 1) / ctas));
   *keys = cdiv(span, shares);
@@ -1624,7 +1655,7 @@ static int gqa_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yout)
   const float* gate = s.out_gate ? e->proj : nullptr;
   const int qpi = gqa_rows_per_item(s);
   const auto& it = sp.items.at(-qpi);   // the lists of this mixer have negative keys
-  if (it.second > 0 && gqa_row_fits(e, s, sp.single.at(-qpi))) {
+  if (it.second > 0 && gqa_row_pays(s, sp.single.at(-qpi), it.second, sp.longest)) {
     GqaRowArgs a = {};
     int keys = 0;
     const int splits = gqa_row_shares(e, s, it.second, sp.max_len, &keys), heads = gqa_row_heads(s);
@@ -2887,14 +2918,17 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   // What the launches depend on is in the key; the key length is a bucket of the longest request (it fixes how the absorbed
   // attention kernel cuts the keys into runs).
   const bool decode_shape = e->graphs_on && e->first && !e->trace && M == n_seq;
+  sp.longest = sp.max_len;
   sp.max_len = decode_shape ? cdiv(sp.max_len, 256) * 256 : sp.max_len;
   // the key-run buffer is sized before anything is captured: a captured step must not replace a buffer
+  int row_layers = 0;                                    // layers whose attention takes a row kernel: with the rest of the key this says which ones, as each leaves it beyond a length of its own
   for (auto& L : e->layers)
     if (L.s.mixer == XOTB200_LM_MIX_ATTENTION || L.s.mixer == XOTB200_LM_MIX_LATENT_ATTN) {
       const bool latent = L.s.mixer == XOTB200_LM_MIX_LATENT_ATTN;
       const int qk = latent ? latent_rows_per_item(L.s) : -gqa_rows_per_item(L.s), items = item_off[qk].second;
       if (items == 0) continue;                          // all rows go through the prompt attention
-      const bool row = latent ? latent_row_fits(e, L.s, item_single[qk]) : gqa_row_fits(e, L.s, item_single[qk]);
+      const bool row = latent ? latent_row_pays(e, L.s, item_single[qk], items, sp.longest) : gqa_row_pays(L.s, item_single[qk], items, sp.longest);
+      row_layers += row;
       int run = 0;
       const int splits = row ? (latent ? latent_row_shares(e, L.s, items, sp.max_len, &run) : gqa_row_shares(e, L.s, items, sp.max_len, &run))
                              : (latent ? latent_key_runs(e, L.s, items, sp.max_len, &run) : gqa_key_runs(e, L.s, items, sp.max_len, &run));
@@ -2908,7 +2942,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   };
   GraphSlot* gs = nullptr;
   if (decode_shape) {
-    const std::array<long, 5> key{n_seq, n_want, (logits_f32 ? 1 : 0) | (argmax_i32 ? 2 : 0), sp.max_len, (long)off};
+    const std::array<long, 6> key{n_seq, n_want, (logits_f32 ? 1 : 0) | (argmax_i32 ? 2 : 0), sp.max_len, row_layers, (long)off};
     gs = &e->graphs[key];
   }
   e->timed = false;

@@ -5,7 +5,8 @@
 // from the pool in 16-byte pieces, the next key's on their way meanwhile, the queries and the sums stay in registers in fp32.  Each lane of a key finishes the score of one head (soft
 // cap, distance terms, mask), keeps that head's running maximum and sum, and hands the weight round.  The shares of a request are a cluster: their sums meet in
 // shared memory and every block finishes a part of the outputs (sink, gate).  More shares than a cluster holds leave them in `part` for gqa_combine_kernel.
-// Bound by latency while the cache is short, by the cache's bytes when it is long.  Measured (B200): 8 requests of
+// Bound by latency while the cache is short, by the fp32 arithmetic on each key when it is long (16 requests behind 8000 tokens, 32 + 8 heads of 128, a layer: 525 MB in 460 us, general kernel 1590); heads
+// that share a key head beyond four read its keys again: gqa_row_pays (layered.cu) has the line.  Measured (B200): 8 requests of
 // some 40 cached tokens, 16 + 4 heads of 128, a launch and what follows it in a step: 9.3 + 3.1 us (general kernel, merge) -> 7.6; a step with two such layers 305 -> 299 us.
 #pragma once
 #include "layered_gqa.cuh"

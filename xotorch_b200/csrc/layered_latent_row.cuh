@@ -5,7 +5,7 @@
 // pieces straight from the pool, the next one's on its way meanwhile: its latent entries are the key's and, with the weight, the value's, so a row is read once a head and the
 // eight warps of a block meet in L1.  Queries and sums stay in registers in fp32.  The shares of a request are a cluster, whose blocks finish a part of the outputs
 // each (sink, gate); more shares than a cluster holds leave them in `part` for latent_attention_combine_kernel.  Measured (B200): 16 requests of
-// some 30 cached tokens, 32 heads, rows of 576, a step with two such layers: 16 + 8 us a layer (general kernel, merge) -> the step 18 us shorter (7115 -> 6877 us for 13 steps).
+// some 30 cached tokens, 32 heads, rows of 576 (bound by latency; behind more tokens every block reads the request's rows anew and the general kernel takes over: latent_row_pays, layered.cu), a step with two such layers: 16 + 8 us a layer (general kernel, merge) -> the step 18 us shorter (7115 -> 6877 us for 13 steps).
 #pragma once
 #include "layered_stream.cuh"
 
