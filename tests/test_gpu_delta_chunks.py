@@ -1,4 +1,4 @@
-"""Prompts of the delta-rule mixers over chunks of 32 tokens: head sizes at both padded ones and between, value columns that are no whole group, row counts around whole
+"""Prompts of the delta-rule mixers (from 128 rows on) over chunks of 32 tokens, and shorter ones beside them: head sizes at both padded ones and between, value columns that are no whole group, row counts around whole
 chunks, requests of very different lengths in one step, key heads shared by value heads, filters shorter than the window registers — 32-bit engine against the
 float64 oracles, and the state they leave carried on row by row.
 
@@ -54,20 +54,46 @@ def test_gated_rule_at_the_ends_of_its_decay(decay):
   check(cfg, w, bu.oracle_logits, [160])
 
 
-@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
-@pytest.mark.parametrize("at", [0, 31, 40, 95, 99])
-@pytest.mark.parametrize("general", [False, True])
-def test_tokens_in_front_of_one_that_is_not_finite(general, at, bad):
+def with_a_token_that_is_not_finite(general, n, at, bad):
   cfg = lu.config([lu.delta(heads=2, dim=64)], width=48, vocab=51) if general else bu.config([bu.delta(heads=4, kv_heads=2, dim=64, vdim=64)], width=48, vocab=51)
   w = (zo if general else bo).random_weights(cfg, 3)
   w["embed"] = w["embed"].clone()
   w["embed"][50] = bad
-  eng = lu.make_engine(cfg, w, "float32", max_tokens=512)
-  toks = lu.rand_tokens(50, 100, 5)
-  ref = eng.step([0, 1], [toks, toks], want=list(range(200)))[0]
+  eng = lu.make_engine(cfg, w, "float32", max_tokens=1024)
+  toks = lu.rand_tokens(50, n, 5)
+  ref = eng.step([0, 1], [toks, toks], want=list(range(2 * n)))[0]
   spoilt = toks.copy()
   spoilt[at] = 50
-  got = eng.step([2, 3], [spoilt, toks], want=list(range(200)))[0]
-  assert np.isfinite(got[:at]).all() and lu.row_err(np.concatenate([got[:at], got[100:]]), np.concatenate([ref[:at], ref[100:]])) < BOUND
-  assert not np.isfinite(got[at:100]).any()
+  got = eng.step([2, 3], [spoilt, toks], want=list(range(2 * n)))[0]
+  assert np.isfinite(got[:at]).all() and lu.row_err(np.concatenate([got[:at], got[n:]]), np.concatenate([ref[:at], ref[n:]])) < BOUND
+  assert not np.isfinite(got[at:n]).any()
   eng.close()
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [0, 31, 40, 95, 99])
+@pytest.mark.parametrize("general", [False, True])
+def test_tokens_in_front_of_one_that_is_not_finite(general, at, bad):
+  with_a_token_that_is_not_finite(general, 100, at, bad)
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [0, 31, 40, 127, 128, 139])
+@pytest.mark.parametrize("general", [False, True])
+def test_tokens_of_a_prompt_in_front_of_one_that_is_not_finite(general, at, bad):
+  """100 rows go token by token, 140 over chunks"""
+  with_a_token_that_is_not_finite(general, 140, at, bad)
+
+
+@pytest.mark.parametrize("others", [21, 22])
+@pytest.mark.parametrize("general", [False, True])
+def test_requests_beside_a_prompt_on_both_sides_of_the_line(general, others):
+  """a prompt of 160 rows and requests of 40: four heads of 64 x 64 are 16 blocks, 148 / 16 - 1 of whose walks are free beside the prompt's five chunks, 41 chunks, and its 32 rows beyond 128
+  pay for two more: 21 others (42 chunks) go over chunks with it, with 22 all go token by token"""
+  rows = [160] + [40] * others
+  if general:
+    cfg = lu.config([lu.delta(heads=4, dim=64)], width=48, vocab=50)
+    check(cfg, zo.random_weights(cfg, 1), lu.oracle_logits, rows, more=1)
+  else:
+    cfg = bu.config([bu.delta(heads=4, kv_heads=2, dim=64, vdim=64)], width=48, vocab=50)
+    check(cfg, bo.random_weights(cfg, 2), bu.oracle_logits, rows, more=1)

@@ -1,6 +1,6 @@
 """The element kernels around the mixers of a prompt in 16-byte pieces: convolution, unit vectors and decays in one pass (one to four taps; five take the kernels before), head norm and
-gate, query / key / value preparation — at the head sizes that they take and beside them, with steps cut so that a filter's window is carried on from every side (portions of 96 and
-more rows, of 1, 2 and 3), 32-bit engine against the float64 oracle."""
+gate, query / key / value preparation — at the head sizes that they take and beside them, with steps cut so that a filter's window is carried on from every side (portions of 128 and
+more rows, of 1, 2, 3, and some that stay under the line), 32-bit engine against the float64 oracle."""
 import numpy as np
 import pytest
 
@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 from tests import bufulorn_oracle as bo, bufulorn_util as bu, layered_util as lu
 
 
-@pytest.mark.parametrize("cut", [[96, 1, 2, 130], [1, 100, 3, 97], [2, 99, 96, 1]])
+@pytest.mark.parametrize("cut", [[128, 1, 2, 130], [1, 132, 3, 129], [2, 131, 128, 1], [96, 3, 127, 128]])
 @pytest.mark.parametrize("dim,vdim,conv", [(64, 64, 1), (64, 64, 2), (64, 64, 3), (128, 128, 4), (64, 64, 5), (64, 128, 4), (68, 68, 4)])
 def test_gated_delta_in_portions(dim, vdim, conv, cut):
   cfg = bu.config([bu.delta(heads=4, kv_heads=2, dim=dim, vdim=vdim, conv=conv)], width=48, vocab=50)

@@ -1,6 +1,6 @@
 """The lines at which single rows leave the row kernels for the general ones: behind 128 tokens for latents whose heads are one block a request, from blocks x keys = 3200 on for more, behind
 256 tokens where many heads share a key head.  Rows on both sides of a line must be the same rows — against the general kernels, which take two rows at a time — with steps
-captured and without (a captured step must be one of its own side of the line, and cuts the keys for a length rounded up).
+captured and without (a captured step must be one of its own side of the line, and cuts the keys for a length rounded up); in 32 bits they must be the float64 oracle's too.
 
 Bounds as for the row kernels themselves: sums over at most 420 keys x 288 entries in another order, 2^-24 sqrt(420 x 288) = 2.1e-5 of a row if all were as large as the result, twice
 that; in 16 bits the products around the attention round to 8 bits on both sides, 2^-8, twice."""
@@ -60,3 +60,6 @@ def test_rows_on_both_sides_of_a_line(kind, dtype):
   flat = lambda x: x.reshape(-1, x.shape[-1])            # noqa: E731
   for got in (plain, first, again):
     assert lu.row_err(flat(got), flat(ref)) < BOUND[dtype]
+  if dtype == "float32":
+    for r in range(requests):
+      assert lu.row_err(plain[r], (bu if oracle is bo else lu).oracle_logits(cfg, w, toks[r])[0][start:]) < lu.TOL[dtype]

@@ -1098,6 +1098,7 @@ struct StepPlan {
   int max_len = 0;                                     // longest request after this step (bounds every key range)
   int longest = 0;                                     // the same, where max_len of a captured step is rounded up
   int max_rows = 0;                                    // most rows one request brings
+  int chunks = 0;                                      // the requests' rows in pieces of DCH, a last piece of any size
   const GqaTile* gqa_tiles = nullptr;                  // key/value-cache attention, long portions (bf16): 64-row tiles
   int n_gqa_tiles = 0;
   const xf::FlashTile128* gqa_tiles128 = nullptr;      // the same rows in 128-row tiles
@@ -1417,9 +1418,19 @@ static int launch_chunks(xotb200_lm* e, const StepPlan& sp, const DeltaChunkArgs
   TRY(opt_in_smem(walk, smem));
   return launch_early(e, walk, dim3(sp.n_seq * a.H, cdiv(a.dv, NC)), THR, smem, 1, a, sp.seqs);
 }
-// Rows of the longest request from which the chunks pay: two launches and a chunk's three steps against 0.14 to 0.35 us a token.  (Portions of 64 rows, 32 heads of 64 x 64, beside
-// decoded rows: 7640 us a pass token by token, 7730 in chunks.)
-static const int DCH_MIN_ROWS = 96;
+// Rows of the longest request from which the chunks pay: two launches and a chunk's three steps against 0.14 to 0.35 us a token (a layer in its step, chunks / token by token: 32 heads of
+// 128 x 128, general form, 96 rows 108 / 106 us, 128 124 / 124, 256 176 / 194, 1024 492 / 560; gated 96 / 91, 104 / 102, 141 / 146, 383 / 448; 32 of 64 x 64, gated 79 / 75, 84 / 82, 105 / 112, 221 / 290).
+static const int DCH_MIN_ROWS = 128;
+// The other requests of the step: a block of the walk takes most of an SM and as long for a chunk of one row as for one of 32, so what they bring is free only where it fits beside the
+// longest request's blocks, and the rest has to be won back by that one's rows.  Rows beyond DCH_MIN_ROWS that pay for one more chunk of others (the same layers, chunks /
+// token by token; a prompt and requests of one row: general, 128: 256 + 4 293 / 276, 512 + 4 395 / 435, 1024 + 16 782 / 759, 128 + 48 694 / 263; gated, 128: 512 + 16 434 / 425,
+// 1024 + 16 620 / 712; gated, 64: 256 + 16 187 / 181, 512 + 16 236 / 273, 1024 + 48 453 / 555; 8 prompts of 100: 485 / 394, 380 / 333, 218 / 176):
+static int chunk_rows_per_other(bool gated, int dk) { return dk <= 64 ? 16 : gated ? 48 : 96; }
+static bool chunks_pay(const xotb200_lm* e, const xotb200_lm_layer& s, const StepPlan& sp, bool gated) {
+  if (sp.max_rows < DCH_MIN_ROWS) return false;
+  const double longest = cdiv(sp.max_rows, DCH), blocks = (double)s.heads * cdiv(s.vdim, s.dim <= 64 ? 16 : 32);   // of a request, one to an SM
+  return sp.chunks - longest - std::max(0.0, e->sm_count / blocks - 1) * longest <= (double)(sp.max_rows - DCH_MIN_ROWS) / chunk_rows_per_other(gated, s.dim);
+}
 struct ChunkRoom { size_t mats, vecs, rows; };         // floats of what the two kernels hand over
 static ChunkRoom chunk_floats(const LmLayer& L, const StepPlan& sp, bool gated) {
   const size_t pieces = (size_t)(sp.M / DCH + sp.n_seq + 1) * L.s.heads;
@@ -1428,7 +1439,7 @@ static ChunkRoom chunk_floats(const LmLayer& L, const StepPlan& sp, bool gated) 
 static bool takes_chunks(xotb200_lm* e, const LmLayer& L, const StepPlan& sp, bool gated) {
   const int dk = L.s.dim;
   if (e->stream == e->side) return false;              // the second mixer of a layer runs beside the first, which may use the buffer
-  if (sp.max_rows < DCH_MIN_ROWS || dk % 4 != 0 || dk <= 32 || dk > 128 || sp.n_seq > 65535 || (!gated && (L.n_in | L.c_k | L.c_r) % 4 != 0)) return false;
+  if (!chunks_pay(e, L.s, sp, gated) || dk % 4 != 0 || dk <= 32 || dk > 128 || sp.n_seq > 65535 || (!gated && (L.n_in | L.c_k | L.c_r) % 4 != 0)) return false;
   const ChunkRoom c = chunk_floats(L, sp, gated);
   const size_t need = c.mats + c.vecs + 4 * c.rows;
   if (need > e->dch_cap) {
@@ -2805,6 +2816,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     seqs[i] = Item{row, counts[i], sl, len0};
     sp.max_len = std::max(sp.max_len, len1);
     sp.max_rows = std::max(sp.max_rows, counts[i]);
+    sp.chunks += cdiv(counts[i], DCH);
     for (int t = 0; t < counts[i]; ++t, ++row) {
       if (bigram) {
         const int64_t B = e->cfg.bigram_buckets, prev = t > 0 ? tokens[row - 1] : e->slot_last[sl];
@@ -3123,6 +3135,7 @@ int xotb200_lm_cache_stats(xotb200_lm* e, int* pages_total, int* pages_free, int
 int xotb200_lm_last_step_ms(xotb200_lm* e, float* ms) {
   REQUIRE(e && ms, "null argument");
   if (e->timed) {
+    CK(cudaSetDevice(e->device));                        // a thread that has not chosen one yet would start a context on device 0
     CK(cudaEventElapsedTime(&e->last_ms, e->ev0, e->ev1));
     e->timed = false;
   }

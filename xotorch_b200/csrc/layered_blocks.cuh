@@ -663,7 +663,7 @@ __global__ void __launch_bounds__(1024) moe_router_kernel(const T* __restrict__ 
   for (int e = lane; e < E; e += 32) s[e] = expf(s[e] - mx) / den;
   __syncwarp();
   if (E <= 32 && E % max(groups, 1) == 0) {
-    // the same selection as below, an expert to a lane: a chain of some hundred reads of shared memory by one lane is 3 us of the step
+    // the same selection as below, an expert to a lane, so for up to 32 of them: a chain of some hundred reads of shared memory by one lane is 3 us of the step
     const int gs = groups > 1 ? E / groups : E;
     const float v = lane < E ? s[lane] : -1.f;
     bool kept = lane < E;
