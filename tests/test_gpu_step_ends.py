@@ -123,3 +123,22 @@ def test_more_wanted_rows_than_a_grid_is_high():
   parts = np.concatenate([eng.step([1], [p], want=list(range(len(p))))[0] for p in np.split(toks, 5)])
   eng.close()
   assert np.isfinite(whole).all() and lu.row_err(whole, parts) < 1e-5
+
+
+@pytest.mark.parametrize("vocab", [4096, 5003])
+def test_rows_shared_by_a_cluster_and_rows_of_one_block(vocab):
+  """as many wanted rows as SMs go to clusters, more to a block each; the head's product may tile 148 and 157 rows otherwise, so 2^-24 sqrt(48) = 4.1e-7 of
+  a row, twice"""
+  cfg = lu.config([lu.delta(heads=1, dim=8)], width=48, vocab=vocab)
+  sms = torch.cuda.get_device_properties(0).multi_processor_count
+  eng = lu.make_engine(cfg, zo.random_weights(cfg, 4), "float32", max_tokens=2048, max_requests=2)
+  toks, got = lu.rand_tokens(vocab, sms + 9, 8), []
+  for n in (sms, sms + 1, sms + 9):
+    eng.clear_request(0)
+    lg, best = eng.step([0], [toks], want=list(range(n)))
+    eng.clear_request(0)
+    alone = eng.step([0], [toks], want=list(range(n)), logits=False)[1]
+    assert np.array_equal(best, lg.argmax(axis=1)) and np.array_equal(best, alone)
+    got.append(lg[:sms].copy())
+  eng.close()
+  assert np.isfinite(got[0]).all() and all(lu.row_err(g, got[0]) < 1e-6 for g in got)
