@@ -1,4 +1,4 @@
-"""Prompts of the delta-rule mixers (from 128 rows on) over chunks of 32 tokens, and shorter ones beside them: head sizes at both padded ones and between, value columns that are no whole group, row counts around whole
+"""Prompts of the delta-rule mixers (from 160 rows on; gated 128, and 256 with heads above 64) over chunks of 32 tokens, and shorter ones beside them: head sizes at both padded ones and between, value columns that are no whole group, row counts around whole
 chunks, requests of very different lengths in one step, key heads shared by value heads, filters shorter than the window registers — 32-bit engine against the
 float64 oracles, and the state they leave carried on row by row.
 
@@ -30,14 +30,14 @@ def check(cfg, w, oracle, rows, more=3):
     assert lu.row_err(got, ref) < BOUND, (r, k)
 
 
-@pytest.mark.parametrize("rows", [[96], [127], [128], [129], [300], [97, 1, 130, 33]])
+@pytest.mark.parametrize("rows", [[96], [127], [128], [129], [159], [160], [161], [300], [97, 1, 130, 33], [97, 1, 190, 33]])
 @pytest.mark.parametrize("dim", [36, 64, 68, 128])
 def test_general_rule(dim, rows):
   cfg = lu.config([lu.delta(heads=2, dim=dim)], width=48, vocab=50)
   check(cfg, zo.random_weights(cfg, dim), lu.oracle_logits, rows)
 
 
-@pytest.mark.parametrize("rows", [[96], [128], [161], [2, 140, 31, 32, 1]])
+@pytest.mark.parametrize("rows", [[96], [128], [161], [2, 140, 31, 32, 1], [255], [256], [287], [2, 260, 31, 32, 1]])
 @pytest.mark.parametrize("heads,dim,vdim,conv", [(4, 64, 64, 4), (6, 64, 64, 2), (2, 128, 128, 3), (10, 64, 30, 4), (4, 36, 72, 4), (4, 128, 64, 1), (4, 64, 64, 6)])
 def test_gated_rule(heads, dim, vdim, conv, rows):
   cfg = bu.config([bu.delta(heads=heads, kv_heads=2, dim=dim, vdim=vdim, conv=conv)], width=48, vocab=50)
@@ -78,19 +78,19 @@ def test_tokens_in_front_of_one_that_is_not_finite(general, at, bad):
 
 
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
-@pytest.mark.parametrize("at", [0, 31, 40, 127, 128, 139])
+@pytest.mark.parametrize("at", [0, 31, 40, 159, 160, 171])
 @pytest.mark.parametrize("general", [False, True])
 def test_tokens_of_a_prompt_in_front_of_one_that_is_not_finite(general, at, bad):
-  """100 rows go token by token, 140 over chunks"""
-  with_a_token_that_is_not_finite(general, 140, at, bad)
+  """100 rows go token by token, these over chunks"""
+  with_a_token_that_is_not_finite(general, 172, at, bad)
 
 
 @pytest.mark.parametrize("others", [21, 22])
 @pytest.mark.parametrize("general", [False, True])
 def test_requests_beside_a_prompt_on_both_sides_of_the_line(general, others):
-  """a prompt of 160 rows and requests of 40: four heads of 64 x 64 are 16 blocks, 148 / 16 - 1 of whose walks are free beside the prompt's five chunks, 41 chunks, and its 32 rows beyond 128
-  pay for two more: 21 others (42 chunks) go over chunks with it, with 22 all go token by token"""
-  rows = [160] + [40] * others
+  """a prompt and requests of 40: four heads of 64 x 64 are 16 blocks, 148 / 16 - 1 of whose walks are free beside the prompt's chunks, and each 16 of its rows beyond the line pay for one more.
+  Gated, 160 rows: 41 + 2 chunks, 21 others (42) go over chunks with it, with 22 all go token by token.  General, 192 rows: 49 + 2, 25 others and 26"""
+  rows = [192] + [40] * (others + 4) if general else [160] + [40] * others
   if general:
     cfg = lu.config([lu.delta(heads=4, dim=64)], width=48, vocab=50)
     check(cfg, zo.random_weights(cfg, 1), lu.oracle_logits, rows, more=1)

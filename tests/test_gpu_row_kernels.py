@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 from tests import bufulorn_oracle as bo, bufulorn_util as bu, layered_util as lu
 
 
-@pytest.mark.parametrize("cut", [[128, 1, 2, 130], [1, 132, 3, 129], [2, 131, 128, 1], [96, 3, 127, 128]])
+@pytest.mark.parametrize("cut", [[128, 1, 2, 130], [1, 132, 3, 129], [2, 131, 128, 1], [96, 3, 127, 128], [256, 2, 240, 1]])
 @pytest.mark.parametrize("dim,vdim,conv", [(64, 64, 1), (64, 64, 2), (64, 64, 3), (128, 128, 4), (64, 64, 5), (64, 128, 4), (68, 68, 4)])
 def test_gated_delta_in_portions(dim, vdim, conv, cut):
   cfg = bu.config([bu.delta(heads=4, kv_heads=2, dim=dim, vdim=vdim, conv=conv)], width=48, vocab=50)

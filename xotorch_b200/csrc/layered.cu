@@ -1420,16 +1420,18 @@ static int launch_chunks(xotb200_lm* e, const StepPlan& sp, const DeltaChunkArgs
 }
 // Rows of the longest request from which the chunks pay: two launches and a chunk's three steps against 0.14 to 0.35 us a token (a layer in its step, chunks / token by token: 32 heads of
 // 128 x 128, general form, 96 rows 108 / 106 us, 128 124 / 124, 256 176 / 194, 1024 492 / 560; gated 96 / 91, 104 / 102, 141 / 146, 383 / 448; 32 of 64 x 64, gated 79 / 75, 84 / 82, 105 / 112, 221 / 290).
-static const int DCH_MIN_ROWS = 128;
+// 6 heads of 128 x 128, gated, whose token by token form has short chains: 128 rows 102 / 95, 200 131 / 132 (32-bit engine 176 / 165), 2000 501 / 531; 32 of 128, general, 32-bit engine, 128 rows 307 / 296.
+static int chunk_min_rows(bool gated, int dk) { return !gated ? 160 : dk <= 64 ? 128 : 256; }
 // The other requests of the step: a block of the walk takes most of an SM and as long for a chunk of one row as for one of 32, so what they bring is free only where it fits beside the
-// longest request's blocks, and the rest has to be won back by that one's rows.  Rows beyond DCH_MIN_ROWS that pay for one more chunk of others (the same layers, chunks /
+// longest request's blocks, and the rest has to be won back by that one's rows.  Rows beyond chunk_min_rows that pay for one more chunk of others (the same layers, chunks /
 // token by token; a prompt and requests of one row: general, 128: 256 + 4 293 / 276, 512 + 4 395 / 435, 1024 + 16 782 / 759, 128 + 48 694 / 263; gated, 128: 512 + 16 434 / 425,
 // 1024 + 16 620 / 712; gated, 64: 256 + 16 187 / 181, 512 + 16 236 / 273, 1024 + 48 453 / 555; 8 prompts of 100: 485 / 394, 380 / 333, 218 / 176):
 static int chunk_rows_per_other(bool gated, int dk) { return dk <= 64 ? 16 : gated ? 48 : 96; }
 static bool chunks_pay(const xotb200_lm* e, const xotb200_lm_layer& s, const StepPlan& sp, bool gated) {
-  if (sp.max_rows < DCH_MIN_ROWS) return false;
+  const int min_rows = chunk_min_rows(gated, s.dim);
+  if (sp.max_rows < min_rows) return false;
   const double longest = cdiv(sp.max_rows, DCH), blocks = (double)s.heads * cdiv(s.vdim, s.dim <= 64 ? 16 : 32);   // of a request, one to an SM
-  return sp.chunks - longest - std::max(0.0, e->sm_count / blocks - 1) * longest <= (double)(sp.max_rows - DCH_MIN_ROWS) / chunk_rows_per_other(gated, s.dim);
+  return sp.chunks - longest - std::max(0.0, e->sm_count / blocks - 1) * longest <= (double)(sp.max_rows - min_rows) / chunk_rows_per_other(gated, s.dim);
 }
 struct ChunkRoom { size_t mats, vecs, rows; };         // floats of what the two kernels hand over
 static ChunkRoom chunk_floats(const LmLayer& L, const StepPlan& sp, bool gated) {
