@@ -720,7 +720,9 @@ static int launch_tc_flash(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, 
   return launch_early(e, st, fn, dim3(Hq, (S + xf::FT_Q - 1) / xf::FT_Q), xf::FT_THREADS, xf::ft_smem_bytes(HD / 64, HD / 64), 1, mq, mk, mk, mv, a);
 }
 
-// 2 .. 7 positions: about one CTA per SM, two turns of 32 keys or more each
+// 2 .. 7 positions: about one CTA per SM, two turns of 32 keys or more each.  A CTA has four heads of 64 or two of 128 that share a key head: a lane's queries and sums are 64
+// registers then.  Four of 128 read the keys half as often and lose by their 128 (two 8B layers, four / two / one heads a CTA: 3 positions behind 60 214.6 / 206.5 / 207 us a
+// call, 7 behind 250 229 / 214 / 217, 4 behind 4000 290 / 258 / 288, 7 behind 8000 431 / 356 / 521).
 template <int HD, int REP>
 static int launch_tc_row_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, int pos0, float scale_log2, cudaStream_t st) {
   auto fn = e->cfg.dtype == XOTB200_DTYPE_F16 ? xb::fp::tc_row_attn_kernel<HD, REP> : xb::bf::tc_row_attn_kernel<HD, REP>;
@@ -732,10 +734,11 @@ template <int HD>
 static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, int pos0, cudaStream_t st) {
   if (S >= 64 && e->cfg.n_heads > 1) return launch_tc_flash<HD>(e, S, R, kc, vc, pos0, st);
   const float scale_log2 = 1.4426950408889634f / sqrtf((float)HD);
-  if (S < TC_FEW)
-    return R % 4 == 0   ? launch_tc_row_attn<HD, 4>(e, S, R, kc, vc, pos0, scale_log2, st)
-           : R % 2 == 0 ? launch_tc_row_attn<HD, 2>(e, S, R, kc, vc, pos0, scale_log2, st)
-                        : launch_tc_row_attn<HD, 1>(e, S, R, kc, vc, pos0, scale_log2, st);
+  if (S < TC_FEW) {
+    if constexpr (HD <= 64)
+      if (R % 4 == 0) return launch_tc_row_attn<HD, 4>(e, S, R, kc, vc, pos0, scale_log2, st);
+    return R % 2 == 0 ? launch_tc_row_attn<HD, 2>(e, S, R, kc, vc, pos0, scale_log2, st) : launch_tc_row_attn<HD, 1>(e, S, R, kc, vc, pos0, scale_log2, st);
+  }
   constexpr int SMEM = (64 + 4 * 64) * HD * 2;          // Q tile + 2 x (K, V) tiles
   auto fn = e->cfg.dtype == XOTB200_DTYPE_F16 ? xb::fp::tc_flash_attn_kernel<HD> : xb::bf::tc_flash_attn_kernel<HD>;
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, SMEM)) return rc;
