@@ -472,8 +472,14 @@ static int launch_early(xotb200_engine* e, cudaStream_t st, void (*fn)(KA...), d
 // while two CTAs per SM (with 128 rows, whose partial tiles are 64 KB: one) are not exceeded and each keeps two K blocks or more.  Measured on an 8B layer
 // (16 / 128 rows; 128 x 64..128 token tiles with split-K through a workspace took 36.5 us for O and down on average, 30.6 for QKV, 54.9 for
 // gate/up at 128 rows): O and down 18.3 / 28.7 us, QKV 14.5 / 23.6, gate/up 41.4 (5.7 TB/s) / 47.9.
-// With 128 rows a stage holds as many bytes of rows as of weights; where no SM has two CTAs the ring is twice as deep (two 8B layers, 128 rows: 344 -> 294 us a call; cutting K
-// over as many CTAs as fit, not a power of two of them, loses: 321; 6 rows 232 -> 243).
+// With 128 rows a stage holds as many bytes of rows as of weights; where no SM has two CTAs the ring is twice as deep, if a CTA has 16 K blocks or more to fill it with and its cluster is
+// at most four (a cluster of eight such CTAs needs eight empty SMs at once, and starts behind the kernel in front instead of beside it).  Two layers, a call, 65 / 128 rows, us:
+//                                       three stages   six wherever one CTA an SM   this rule
+//   8B (4096 x 14336)                   313 / 348      276 / 297                    276 / 297
+//   2048 x 8192, 32 + 8 heads of 64     203 / 253      213 / 250                    190 / 235
+//   2048 x 5632, 32 + 4 heads of 64     188 / 247      204 / 241                    187 / 237
+//   1024 x 3072                         138 / 171      131 / 157                    138 / 171
+// Cutting K over as many CTAs as fit, not a power of two of them, loses (8B, 128 rows 321; 6 rows 232 -> 243).
 template <int NB, int NS>
 static int launch_tc_stream_nb(xotb200_engine* e, const CUtensorMap& tmW, const CUtensorMap& tmX, const TcGemmArgs& a, int epi, int splits, cudaStream_t st) {
   void (*fn)(CUtensorMap, CUtensorMap, TcGemmArgs) = nullptr;
@@ -494,7 +500,7 @@ static int launch_tc_stream(xotb200_engine* e, const CUtensorMap& tmW, const Act
   const int nb = epi == TCE_HEAD_LAST || a.S <= 16 ? 16 : a.S <= 32 ? 32 : a.S <= 64 ? 64 : 128, tiles = a.N / TC_M, nkb = a.K / TC_BK;
   int s = 1;
   while (s < 8 && tiles * s * 2 <= (nb >= 128 ? 1 : 2) * e->sm_count && nkb >= 4 * s) s *= 2;
-  if (nb == 128 && tiles * s <= e->sm_count) return launch_tc_stream_nb<128, TCS_ALONE>(e, tmW, x.full, a, epi, s, st);
+  if (nb == 128 && tiles * s <= e->sm_count && s <= 4 && nkb >= 16 * s) return launch_tc_stream_nb<128, TCS_ALONE>(e, tmW, x.full, a, epi, s, st);
   return nb == 16 ? launch_tc_stream_nb<16, tcs_stages(16)>(e, tmW, x.r16, a, epi, s, st) : nb == 32 ? launch_tc_stream_nb<32, tcs_stages(32)>(e, tmW, x.r32, a, epi, s, st)
        : nb == 64 ? launch_tc_stream_nb<64, tcs_stages(64)>(e, tmW, x.r64, a, epi, s, st) : launch_tc_stream_nb<128, tcs_stages(128)>(e, tmW, x.full, a, epi, s, st);
 }
