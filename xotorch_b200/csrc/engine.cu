@@ -473,12 +473,13 @@ static int launch_early(xotb200_engine* e, cudaStream_t st, void (*fn)(KA...), d
 // (16 / 128 rows; 128 x 64..128 token tiles with split-K through a workspace took 36.5 us for O and down on average, 30.6 for QKV, 54.9 for
 // gate/up at 128 rows): O and down 18.3 / 28.7 us, QKV 14.5 / 23.6, gate/up 41.4 (5.7 TB/s) / 47.9.
 // With 128 rows a stage holds as many bytes of rows as of weights; where no SM has two CTAs the ring is twice as deep, if a CTA has 16 K blocks or more to fill it with and its cluster is
-// at most four (a cluster of eight such CTAs needs eight empty SMs at once, and starts behind the kernel in front instead of beside it).  Two layers, a call, 65 / 128 rows, us:
-//                                       three stages   six wherever one CTA an SM   this rule
-//   8B (4096 x 14336)                   313 / 348      276 / 297                    276 / 297
-//   2048 x 8192, 32 + 8 heads of 64     203 / 253      213 / 250                    190 / 235
-//   2048 x 5632, 32 + 4 heads of 64     188 / 247      204 / 241                    187 / 237
-//   1024 x 3072                         138 / 171      131 / 157                    138 / 171
+// at most four (a cluster of eight such CTAs needs eight empty SMs at once, and starts behind the kernel in front instead of beside it).  QKV always has the deep ring there: no weights
+// stream behind it that could share its SMs.  Two layers, a call, 65 / 128 rows, us:
+//                                       three stages   six wherever one CTA an SM   without QKV's exception   this rule
+//   8B (4096 x 14336)                   313 / 348      276 / 297                    276 / 298                 276 / 298
+//   2048 x 8192, 32 + 8 heads of 64     203 / 253      213 / 250                    190 / 234                 188 / 232
+//   2048 x 5632, 32 + 4 heads of 64     188 / 247      204 / 241                    187 / 237                 183 / 228
+//   1024 x 3072                         138 / 171      131 / 157                    139 / 176                 134 / 167
 // Cutting K over as many CTAs as fit, not a power of two of them, loses (8B, 128 rows 321; 6 rows 232 -> 243).
 template <int NB, int NS>
 static int launch_tc_stream_nb(xotb200_engine* e, const CUtensorMap& tmW, const CUtensorMap& tmX, const TcGemmArgs& a, int epi, int splits, cudaStream_t st) {
@@ -500,7 +501,7 @@ static int launch_tc_stream(xotb200_engine* e, const CUtensorMap& tmW, const Act
   const int nb = epi == TCE_HEAD_LAST || a.S <= 16 ? 16 : a.S <= 32 ? 32 : a.S <= 64 ? 64 : 128, tiles = a.N / TC_M, nkb = a.K / TC_BK;
   int s = 1;
   while (s < 8 && tiles * s * 2 <= (nb >= 128 ? 1 : 2) * e->sm_count && nkb >= 4 * s) s *= 2;
-  if (nb == 128 && tiles * s <= e->sm_count && s <= 4 && nkb >= 16 * s) return launch_tc_stream_nb<128, TCS_ALONE>(e, tmW, x.full, a, epi, s, st);
+  if (nb == 128 && tiles * s <= e->sm_count && (epi == TCE_QKV || (s <= 4 && nkb >= 16 * s))) return launch_tc_stream_nb<128, TCS_ALONE>(e, tmW, x.full, a, epi, s, st);
   return nb == 16 ? launch_tc_stream_nb<16, tcs_stages(16)>(e, tmW, x.r16, a, epi, s, st) : nb == 32 ? launch_tc_stream_nb<32, tcs_stages(32)>(e, tmW, x.r32, a, epi, s, st)
        : nb == 64 ? launch_tc_stream_nb<64, tcs_stages(64)>(e, tmW, x.r64, a, epi, s, st) : launch_tc_stream_nb<128, tcs_stages(128)>(e, tmW, x.full, a, epi, s, st);
 }
@@ -1448,7 +1449,7 @@ static int ensure_staging(xotb200_engine* e, int n) {
 // Behind a long cache both ways spread the keys over the chip, and below TC_FEW positions the cheaper one is taken by a layer's time in us: constants fitted to both at
 // 2 .. 7 positions behind 100 .. 16000 keys, layers of 122 MB with heads of 64 and 436 MB with heads of 128.  Measured on layers of 24 to 436 MB, 2, 4 and 7 positions
 // behind 30 .. 16000 keys, the line takes the cheaper way everywhere but at 2 positions behind 16000 keys, 46 MB with heads of 128 (GEMMs / one after the other, us a
-// layer: 2 positions behind 16000 keys, 24 MB 70 / 86, 46 MB 86 / 124, 122 MB 104 / 125, 436 MB 184 / 268; 4 behind 4000, 24 MB 50 / 128, 68 MB 63 / 171, 436 MB 145 / 391).
+// layer: 2 positions behind 16000 keys, 24 MB 70 / 87, 46 MB 84 / 125, 122 MB 104 / 125, 436 MB 165 / 267; 4 behind 4000, 24 MB 50 / 129, 68 MB 63 / 171, 436 MB 130 / 391).
 // Layers under 10 MB, models of a test's size, keep the line of an attention that walked all keys of a query in one block, although GEMMs are cheaper there too (2
 // positions behind 2000 keys, 6 MB: 39 / 57): behind a long cache their few positions come out bit for bit as one after the other.
 static bool gemms_pay(const xotb200_engine* e, int n_tokens, int pos0) {
