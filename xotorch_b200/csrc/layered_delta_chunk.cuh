@@ -14,7 +14,7 @@
 // influence of one token's value on a later correction, which the recurrence itself contracts: at most about 1.
 // Rows behind the end of a request's step count as tokens that neither decay nor write.
 // Measured (B200, a launch): 3500 tokens, 32 heads of 64 x 64 (16 key heads), gated: 495 us token by token -> 31 (matrices) + 295 (walk); 1024 tokens, 32 heads of 128 x 128, general:
-// 365 + 24 for its vectors -> 74 + 248.  The walk is bound by shared memory (wavefronts at 60 % of their rate) and by the latency of its three steps a chunk (2.7 us, 7.8 us).
+// 365 + 24 for its vectors -> 74 + 248.  The walk is bound by shared memory (wavefronts at 61 to 62 % of their rate on the SMs that have a block) and by the latency of its three steps a chunk (2.7 us, 7.8 us).
 #pragma once
 #include "layered_stream.cuh"
 
