@@ -10,7 +10,7 @@
 // against is then stale by that factor at most, which fp32 sums and floating-point weights carry without loss).  Scores are kept in units of
 // ln 2.  Two CTAs share an SM (256 of the 512 tensor-memory columns and at most 112 KB each), so one's exponentials run under the other's MMAs: bound
 // by the exponentials and the arithmetic around them, not by the tensor pipe.
-// Measured (B200, a launch, 64-row mma.sync tiles -> this kernel): grouped keys, 3500 rows x 16 heads of 128, soft cap and distance terms: 377 -> 122 us;
+// Measured (B200, a launch, 64-row mma.sync tiles -> this kernel): grouped keys, 3500 rows x 16 heads of 128, soft cap, distance terms, a gate per entry: 377 -> 122 us, -> 87 with cheap sigmoids (one portion of 64 rows 33 -> 20);
 // latent keys, 1024 rows x 32 heads of 192 / 128: 190 -> 52 us; 2701 rows in chunks x 32 heads of 128, 16-bit weights: 127 -> 79 us.
 // Every wait is bounded: one that expires sets *err, all roles of the CTA run out, it frees its tensor memory and returns.
 #pragma once
@@ -391,15 +391,15 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           float v[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * f;
-          if (a.gate_mode == 2) {
+          if (a.gate_mode == 2) {   // sigmoids with the hardware's power of two and reciprocal (2e-6 off at gates of -30, the output has 8 bits): expf and an exact division took 18 us of a 33 us launch
             const bool vec = ((reinterpret_cast<uintptr_t>(gt) | (uintptr_t)c) & 15) == 0;
 #pragma unroll
             for (int i = 0; i < 32; i += 4) {
               const float4 z = vec ? *reinterpret_cast<const float4*>(gt + c + i) : make_float4(gt[c + i], gt[c + i + 1], gt[c + i + 2], gt[c + i + 3]);
-              v[i] *= 1.0f / (1.0f + expf(-z.x));
-              v[i + 1] *= 1.0f / (1.0f + expf(-z.y));
-              v[i + 2] *= 1.0f / (1.0f + expf(-z.z));
-              v[i + 3] *= 1.0f / (1.0f + expf(-z.w));
+              v[i] *= rcp(1.0f + ex2(-LOG2E * z.x));
+              v[i + 1] *= rcp(1.0f + ex2(-LOG2E * z.y));
+              v[i + 2] *= rcp(1.0f + ex2(-LOG2E * z.z));
+              v[i + 3] *= rcp(1.0f + ex2(-LOG2E * z.w));
             }
           }
 #pragma unroll
