@@ -856,8 +856,7 @@ static int product_stream(xotb200_lm* e, const bf16* A, long lda, long a_batch, 
   return 1;
 }
 
-// Pairs of CTAs on 256 x 256 tiles: 1.4 times the rate of 128 x 128 tiles while the tiles fill the pairs, so they are taken when at least 0.72 of
-// the pairs' time goes to rows and columns that exist (a last wave that is nearly empty, and rows or columns beyond the matrix, count against it).
+// Pairs of CTAs on 256 x 256 tiles, where they pay (pairs_pay).
 template <int EPI, typename TC>
 static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& mb, const LtcArgs& a) {
   auto kern = ltc_pair_kernel<EPI, TC>;
@@ -867,11 +866,12 @@ static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& 
   e->tc_launches++;
   return 0;
 }
-// Pairs where their tiles, empty rows and columns included, keep 72 % of the waves' slots busy: a pair's tile runs 1.2 .. 1.4 times as fast as its share of
-// 128 x 128 tiles (layered_tc.cuh), which lose less in the last wave.  K < 512: filling the ring is most of a tile.
+// Pairs where their tiles, empty rows and columns included, keep 60 % of the waves' slots busy: a pair's tile runs about twice as fast as its share of 128 x 128 tiles
+// (layered_tc.cuh), which lose less in the last wave.  1024 rows, 128 x 128 tiles / pairs: 6144 columns with K = 1536 (65 %) 33 / 28 us, 6720 with 4096 (71 %) 70 / 55, 2144 with
+// 4096 (45 %) 29 / 33.  K < 512: filling the ring is most of a tile.
 static bool pairs_pay(const xotb200_lm* e, int M, int N, int K) {
   const long tiles = (long)cdiv(M, 2 * LTC_M) * cdiv(N, LTP_N), pairs = std::max(1, e->sm_count / 2), waves = (tiles + pairs - 1) / pairs;
-  return K >= 512 && (double)M * N >= 0.72 * (double)waves * pairs * (2.0 * LTC_M * LTP_N);
+  return K >= 512 && (double)M * N >= 0.6 * (double)waves * pairs * (2.0 * LTC_M * LTP_N);
 }
 
 // 1 = launched, 0 = not eligible (the caller falls back), < 0 = error

@@ -74,6 +74,21 @@ struct LtcEpilogue {
     }
     if (EPI == EPI_CLOSE && a.epi.h) alpha = __bfloat162float(*static_cast<const __nv_bfloat16*>(a.epi.alpha));
   }
+  // what is stored, CLOSE apart: 16 values, or 8 of a gated form
+  template <int N>
+  __device__ __forceinline__ void values(const LtcArgs& a, const uint32_t (&v)[16], float (&f)[N]) const {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if constexpr (epi_is_glu(EPI)) {               // 8 gate values, then their 8 up values
+        f[j] = glu_f<EPI>(__uint_as_float(v[j]), __uint_as_float(v[j + 8]), a.epi);
+      } else {
+        f[j] = __uint_as_float(v[j]);
+        if (EPI == EPI_RELU2) { f[j] = fmaxf(f[j], 0.f); f[j] *= f[j]; }
+        if (EPI == EPI_XIELU) f[j] = sizeof(TC) == 2 ? xielu16_f(f[j], ap, aq) : xielu_f(f[j], ap, aq);
+        if (EPI == EPI_GELU) f[j] = gelu_erf_f(f[j]);
+      }
+    }
+  }
   __device__ __forceinline__ void store16(const LtcArgs& a, TC* crow, int row, int n, const uint32_t (&v)[16]) const {
     float f[16];
     if constexpr (EPI == EPI_CLOSE) {
@@ -117,8 +132,8 @@ struct LtcEpilogue {
       }
     } else if constexpr (epi_is_glu(EPI)) {        // 8 gate values, then their 8 up values -> 8 outputs at columns n / 2 ..
       const int no = n >> 1;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = glu_f<EPI>(__uint_as_float(v[j]), __uint_as_float(v[j + 8]), a.epi);
+      float (&g)[8] = reinterpret_cast<float (&)[8]>(f);
+      values(a, v, g);
       if (sizeof(TC) == 2 && a.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(a.C) & 15) == 0) {
         uint32_t pk[4];
 #pragma unroll
@@ -132,13 +147,7 @@ struct LtcEpilogue {
         for (int j = 0; j < 8; ++j) ltc_store<TC>(crow + no + j, f[j]);
       }
     } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      f[j] = __uint_as_float(v[j]);
-      if (EPI == EPI_RELU2) { f[j] = fmaxf(f[j], 0.f); f[j] *= f[j]; }
-      if (EPI == EPI_XIELU) f[j] = xielu_f(f[j], ap, aq);
-      if (EPI == EPI_GELU) f[j] = gelu_erf_f(f[j]);
-    }
+    values(a, v, f);
     if (vec && n + 16 <= a.N) {
       float4* d4 = reinterpret_cast<float4*>(reinterpret_cast<float*>(crow) + n);
 #pragma unroll
@@ -159,6 +168,61 @@ struct LtcEpilogue {
         if (n + j < a.N) ltc_store<TC>(crow + n + j, f[j]);
     }
     }
+  }
+};
+
+// The accumulator of a warp's 32 rows on its way out: a thread holds 16 neighbouring columns of ONE row, and stores of that shape reach L2 in 16-byte pieces of 32 different lines
+// (a 256 x 256 fp32 tile took 20000 cycles, its products with K = 2048 17000).  Rows are put together in shared memory first, 128 bytes of each (16-byte pieces, XORed with the row: no bank
+// conflicts), and go out eight lanes to a row, whole lines.  One warp's buffer: LTC_STAGED bytes.
+constexpr int LTC_STAGED = 32 * 128;
+template <int EPI, typename TC>
+struct LtcStaged {
+  static constexpr int PER = 16 / sizeof(TC);                                  // entries of a piece
+  static constexpr int OUT = 128 / sizeof(TC);                                 // entries of a row that are put together
+  static constexpr int COLS = epi_is_glu(EPI) ? 2 * OUT : OUT;                 // their columns of the accumulator
+  // 16 columns of row `lane`, columns c .. c + 15 of the COLS
+  static __device__ __forceinline__ void put(uint8_t* buf, int lane, int c, const LtcEpilogue<EPI, TC>& ep, const LtcArgs& a, const uint32_t (&v)[16]) {
+    constexpr int N = epi_is_glu(EPI) ? 8 : 16;
+    float f[N];
+    ep.values(a, v, f);
+    const int first = (epi_is_glu(EPI) ? c / 2 : c) / PER;
+#pragma unroll
+    for (int j = 0; j < N / PER; ++j) {
+      uint4* d = reinterpret_cast<uint4*>(buf + lane * 128 + (((first + j) ^ lane) & 7) * 16);
+      if constexpr (sizeof(TC) == 4) {
+        *d = make_uint4(__float_as_uint(f[4 * j]), __float_as_uint(f[4 * j + 1]), __float_as_uint(f[4 * j + 2]), __float_as_uint(f[4 * j + 3]));
+      } else {
+        uint32_t pk[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          __nv_bfloat162 h2 = __floats2bfloat162_rn(f[8 * j + 2 * i], f[8 * j + 2 * i + 1]);
+          pk[i] = *reinterpret_cast<uint32_t*>(&h2);
+        }
+        *d = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      }
+    }
+  }
+  // the warp's rows row0 .. row0 + 31, output columns n .. n + OUT - 1 (n a multiple of OUT, N outputs in all)
+  static __device__ __forceinline__ void out(const uint8_t* buf, int lane, const LtcEpilogue<EPI, TC>& ep, const LtcArgs& a, TC* C, int row0, int n, int N) {
+    __syncwarp();
+    const int piece = lane & 7, col = n + piece * PER;
+    const bool whole = (sizeof(TC) == 4 ? ep.vec : ep.vec16) && col + PER <= N;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + (lane >> 3), row = row0 + r;
+      const uint4 q = *reinterpret_cast<const uint4*>(buf + r * 128 + ((piece ^ r) & 7) * 16);
+      if (row >= a.M) continue;
+      TC* d = C + (size_t)row * a.ldc + col;
+      if (whole) {
+        *reinterpret_cast<uint4*>(d) = q;
+      } else {
+        const TC* e = reinterpret_cast<const TC*>(&q);
+#pragma unroll
+        for (int j = 0; j < PER; ++j)
+          if (col + j < N) d[j] = e[j];
+      }
+    }
+    __syncwarp();                                                              // the buffer may be written again
   }
 };
 
@@ -234,13 +298,21 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (ltc_wait(tmem_full, 0, a.err)) {
       xb::tc_fence_after();
       const LtcEpilogue<EPI, TC> ep(a);
+      using St = LtcStaged<EPI, TC>;
+      TC* C = static_cast<TC*>(a.C) + (size_t)z * a.c_batch;
+      uint8_t* mine = base + q * LTC_STAGED;           // the ring has nothing in flight any more
 #pragma unroll 1
       for (int c0 = 0; c0 < NT; c0 += 16) {
         uint32_t v[16];
         xb::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);   // warp-collective: before any row / column test
         const int n = n0 + c0;
-        if (row >= a.M || n >= a.N) continue;
-        ep.store16(a, static_cast<TC*>(a.C) + (size_t)z * a.c_batch + (size_t)row * a.ldc, row, n, v);
+        if constexpr (EPI == EPI_CLOSE || St::COLS > NT) {
+          if (row < a.M && n < a.N) ep.store16(a, C + (size_t)row * a.ldc, row, n, v);
+        } else {
+          const int c = c0 % St::COLS, glu = epi_is_glu(EPI) ? 2 : 1;
+          St::put(mine, lane, c, ep, a, v);
+          if (c + 16 == St::COLS) St::out(mine, lane, ep, a, C, row - lane, (n - c) / glu, a.N / glu);
+        }
       }
     }
   }
@@ -256,9 +328,11 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // pairs walk the tiles (row tile fastest, so that pairs running together share weight tiles in L2) with two accumulators in tensor memory (all
 // 512 columns), so the epilogue of one tile runs under the products of the next.  Plain loads, no multicast.  Every wait is bounded.
 // Measured (B200, a launch, 128 x 128 tiles -> pairs): 3500 rows, width 2048: 86 -> 62 us, the 8192-wide up product with its activation 189 -> 133 us
-// (213 with four epilogue warps: they took longer than the next tile's products); 1024 rows, width 4096, all products of a pass: 1139 -> 976 us.
+// (213 with four epilogue warps: they took longer than the next tile's products); 1024 rows, width 4096, all products of a pass: 1139 -> 976 us.  With rows put together
+// in shared memory (LtcStaged) and a cheap xIELU: 3500 rows, 6208 columns, K = 2048 78 -> 73 us, the 8192-wide up product 131 -> 113.
 constexpr int LTP_N = 256, LTP_STAGES = 6, LTP_THREADS = 384, LTP_STAGE_BYTES = LTC_M * LTC_BK * 2 + LTP_N / 2 * LTC_BK * 2;
-constexpr int LTP_SMEM = LTP_STAGES * LTP_STAGE_BYTES + 1024 + 256;
+constexpr int LTP_SMEM = LTP_STAGES * LTP_STAGE_BYTES + 8 * LTC_STAGED + 1024 + 256;   // the ring, the epilogue warps' buffers
+static_assert(LTP_SMEM <= 227 * 1024, "shared memory of a CTA");
 
 template <int EPI, typename TC>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LTP_THREADS, 1)
@@ -267,7 +341,8 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   extern __shared__ __align__(1024) uint8_t ltc_smem[];
   constexpr int A_BYTES = LTC_M * LTC_BK * 2, NS = LTP_STAGES, NT = LTP_N;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ltc_smem) + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = reinterpret_cast<uint64_t*>(base + NS * LTP_STAGE_BYTES);   // the leader's count both CTAs' copies
+  uint8_t* staged = base + NS * LTP_STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(staged + 8 * LTC_STAGED);   // the leader's count both CTAs' copies
   uint64_t* empty = full + NS;
   uint64_t* tmem_full = empty + NS;       // [2]
   uint64_t* tmem_empty = tmem_full + 2;   // [2], the leader's: 8 warps of both CTAs
@@ -337,6 +412,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const int q = warp & 3, half = (warp - 4) >> 2;
     const uint32_t leader_empty = xb::mapa_shared(xb::smem_u32(&tmem_empty[0]), 0);
     const LtcEpilogue<EPI, TC> ep(a);
+    uint8_t* mine = staged + (warp - 4) * LTC_STAGED;
     unsigned ti = 0;
     for (int t = pair; t < total; t += npairs, ++ti) {
       const uint32_t buf = ti & 1u;
@@ -347,7 +423,14 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       for (int c0 = half * (NT / 2); c0 < (half + 1) * (NT / 2); c0 += 16) {
         uint32_t v[16];
         xb::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + buf * NT + (uint32_t)c0, v);   // warp-collective: before any row / column test
-        if (row < a.M && n0 + c0 < a.N) ep.store16(a, static_cast<TC*>(a.C) + (size_t)row * a.ldc, row, n0 + c0, v);
+        if constexpr (EPI == EPI_CLOSE) {
+          if (row < a.M && n0 + c0 < a.N) ep.store16(a, static_cast<TC*>(a.C) + (size_t)row * a.ldc, row, n0 + c0, v);
+        } else {
+          using St = LtcStaged<EPI, TC>;
+          const int c = c0 % St::COLS, glu = epi_is_glu(EPI) ? 2 : 1;
+          St::put(mine, lane, c, ep, a, v);
+          if (c + 16 == St::COLS) St::out(mine, lane, ep, a, static_cast<TC*>(a.C), row - lane, (n0 + c0 - c) / glu, a.N / glu);
+        }
       }
       xb::tc_fence_before();
       __syncwarp();
