@@ -1,0 +1,57 @@
+"""Tiles of CTA pairs that are cut along K (74 pairs): pieces of unequal length, ragged last row and column tiles, one phase and two, a second launch on the same
+slots — against the float64 oracles (layered engine) and against the same prompt in portions that take other kernels (shard engine)."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from tests import bufulorn_oracle as bo, bufulorn_util as bu, layered_util as lu
+from tests.test_gpu_parity import ATOL, RTOL
+
+
+# down products: 760 x 1280 with K = 6216, 3 x 5 tiles in four pieces of 24 and 25 blocks and a tail; 1025 x 2056 with K = 16392, 5 x 9 tiles: 37 in two pieces, 8 in four
+@pytest.mark.parametrize("rows,width,ff", [(760, 1280, 6216), (1025, 2056, 16392)])
+def test_layered_products(rows, width, ff):
+  cfg = bu.config([bu.attention(heads=2, kv_heads=1, dim=16, vdim=16, chunk=64, mlp=bu.dense(ff)), bu.attention(heads=2, kv_heads=1, dim=16, vdim=16, chunk=64, mlp=bu.dense(ff))],
+                  width=width, vocab=70, max_positions=rows + 8)
+  w = bo.random_weights(cfg, 3)
+  toks = lu.rand_tokens(70, rows, 3)
+  eng = lu.make_engine(cfg, w, "bfloat16", max_tokens=rows + 8)
+  got, _ = eng.step([0], [toks], want=list(range(rows)), argmax=False)
+  got = got.copy()
+  eng.clear_request(0)
+  again, _ = eng.step([0], [toks], want=list(range(rows)), argmax=False)
+  assert np.array_equal(got, again)
+  eng.close()
+  ref, _ = bu.oracle_logits(cfg, w, toks)
+  assert lu.row_err(got, ref) < lu.TOL["bfloat16"]
+
+
+@pytest.mark.parametrize("n", [600, 1029])
+def test_shard_engine_prompts(n):
+  """down product of a layer of 2048 x 8192, 128 K blocks: 3 x 8 tiles in three pieces each, 5 x 8 whole ones; portions of 200 take 128-wide tiles"""
+  from xotorch_b200.native import NativeShard
+  from xotorch_b200.synth import PRESETS, hf_config, synth_prompt
+  shape = dataclasses.replace(PRESETS["tiny-llama-hd64"], dim=2048, ffn=8192, n_heads=32, n_kv_heads=8, n_layers=2, max_pos=2048)
+  prompt = synth_prompt(shape.vocab, n)
+
+  def logits(cuts):
+    e = NativeShard(hf_config(shape), device=0)
+    e.set_shard(0, shape.n_layers - 1)
+    e.init_synthetic(1234)
+    e.set_prefill_mode(2)
+    e.begin_request(n + 8)
+    pos = 0
+    for c in cuts:
+      out = e.forward(prompt[:, pos:pos + c].astype(np.int32), pos)[0].copy()
+      pos += c
+    more = e.forward(np.array([[3]], dtype=np.int32), pos)[0].copy()
+    e.close()
+    return np.stack([out, more])
+
+  whole = logits([n])
+  assert np.array_equal(whole, logits([n]))
+  cut = logits([200] * (n // 200) + [n % 200] if n % 200 else [200] * (n // 200))
+  assert (np.abs(whole - cut) <= ATOL + RTOL * np.abs(whole)).all(), np.abs(whole - cut).max()

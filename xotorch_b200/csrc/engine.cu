@@ -196,6 +196,7 @@ struct xotb200_engine {
   int max_inflight = 0;            // decode producer window (bulk copies in flight per CTA, 0 = ring depth)
   unsigned int pace_q = 0;         // decode producer pacing, 2^-16 ns per byte per CTA (0 = off)
   bool tc_fuse = true;             // RoPE/KV-append and SwiGLU fused into GEMM epilogues (XOTB200_TC_FUSE=0: separate kernels, A/B)
+  float* pair_ws = nullptr;        // slots and flags of a prompt's GEMM tiles that are cut along K (prefill_tc.cuh); NULL: not needed yet, or no memory
   int* gemm_err = nullptr;         // page-locked word that a prompt's kernels write when a pipeline wait expires: read behind the call's own synchronisation, without a copy
   int prefill_mode = 0;            // 0 auto (runs_as_gemms), 1 always the decode kernel, 2 always TC
   bf16 *tc_x = nullptr, *tc_xn = nullptr, *tc_qkv = nullptr, *tc_q = nullptr, *tc_ao = nullptr, *tc_gu = nullptr, *tc_act = nullptr;
@@ -554,9 +555,14 @@ static int launch_tc_gemm_2sm(xotb200_engine* e, const CUtensorMap& tmA, const C
     default: set_err("no CTA-pair GEMM for epilogue %d", epi); return XOTB200_EINVAL;
   }
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, tc2_smem_bytes(NT, NS))) return rc;
-  const int total = ((a.S + 2 * TC_M - 1) / (2 * TC_M)) * (a.N / NT);
-  const int pairs = std::max(1, std::min(total, e->sm_count / 2));
-  return launch_early(e, st, fn, 2 * pairs, TC2_THREADS, tc2_smem_bytes(NT, NS), 0, tmA, tmB_half, a);
+  const int total = ((a.S + 2 * TC_M - 1) / (2 * TC_M)) * (a.N / NT), pairs = std::max(1, e->sm_count / 2);
+  a.split = PairSplit{};
+  if (e->pair_ws && NT == 256) {
+    a.split = pair_split(total, pairs, a.K / TC_BK);
+    a.split.ws = e->pair_ws;
+    a.split.flags = reinterpret_cast<int*>(e->pair_ws + (size_t)pair_slots(pairs) * PAIR_SLOT);
+  }
+  return launch_early(e, st, fn, 2 * pair_count(total, pairs, a.split), TC2_THREADS, tc2_smem_bytes(NT, NS), 0, tmA, tmB_half, a);
 }
 
 static int launch_tc_gemm(xotb200_engine* e, const CUtensorMap& tmA, const CUtensorMap& tmB, const TcGemmArgs& a_in, int epi, TcCfg c,
@@ -644,6 +650,11 @@ static int prepare_tc(xotb200_engine* e, int n_tokens) {
       rc = take();
     }
     if (rc) return rc;
+    if (need > 2 * TC_M && !e->pair_ws) {   // 29 MB; without them the tiles stay whole
+      const size_t slots = pair_slots(std::max(1, e->sm_count / 2)), floats = slots * PAIR_SLOT, flags = slots * PAIR_FLAGS;
+      if (cudaMalloc(&e->pair_ws, (floats + flags) * 4) != cudaSuccess) { cudaGetLastError(); e->pair_ws = nullptr; }
+      else MEMSET_SYNC(e, e->pair_ws + floats, 0, flags * 4);
+    }
     e->tc_cap = need;
     if (c.n_experts > 0) {
       const size_t rows = (size_t)2 * need + (size_t)c.n_experts * TC_M;
@@ -1072,7 +1083,7 @@ int xotb200_destroy(xotb200_engine* e) {
   cudaDeviceSynchronize();
   free_shard(e);
   if (e->next_ipc && e->next_inbox) cudaIpcCloseMemHandle(e->next_inbox);
-  void* tcp[] = {e->tc_x, e->tc_xn, e->tc_qkv, e->tc_q, e->tc_ao, e->tc_gu, e->tc_act, e->moe_xg, e->moe_gu, e->moe_act, e->moe_y,
+  void* tcp[] = {e->pair_ws, e->tc_x, e->tc_xn, e->tc_qkv, e->tc_q, e->tc_ao, e->tc_gu, e->tc_act, e->moe_xg, e->moe_gu, e->moe_act, e->moe_y,
                  e->moe_route_e, e->moe_route_w, e->moe_row_of, e->moe_row_token, e->moe_exp_info};
   for (void* p : tcp)
     if (p) cudaFree(p);
@@ -1424,6 +1435,8 @@ static int check_gemm_error(xotb200_engine* e) {
   const int err = *static_cast<volatile int*>(e->gemm_err);
   if (err == 0) return 0;
   *e->gemm_err = 0;
+  const size_t slots = pair_slots(std::max(1, e->sm_count / 2));
+  if (e->pair_ws) MEMSET_SYNC(e, e->pair_ws + slots * PAIR_SLOT, 0, slots * PAIR_FLAGS * 4);   // flags that nobody waited for any more
   set_err("tensor-core GEMM: a pipeline wait expired (device error %d)", err);
   return XOTB200_ETIMEOUT;
 }

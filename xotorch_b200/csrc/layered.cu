@@ -214,6 +214,7 @@ struct xotb200_lm {
   bool flash_on = true;                                // bf16: prompt portions of FLASH_MIN_ROWS rows or more use the expanded tensor-core attention
   std::vector<int> stage_build;
   int64_t launches = 0, tc_launches = 0, flash_launches = 0;
+  float* pair_ws = nullptr;                            // slots and flags of the products' tiles that are cut along K (layered_tc.cuh); NULL: not needed yet, or no memory
   int* d_err = nullptr;                                // sticky device error word (3 = a bounded wait of a tensor-core product expired)
   int* h_err = nullptr;                                // pinned copy, read after every step
   bool timed = false;                                  // ev0 and ev1 bracket the newest step, not yet read
@@ -857,12 +858,20 @@ static int product_stream(xotb200_lm* e, const bf16* A, long lda, long a_batch, 
 }
 
 // Pairs of CTAs on 256 x 256 tiles, where they pay (pairs_pay).
+// The slots of tiles that are cut along K (PairWalk).  The second mixer of a layer runs beside the first, which may use them: its tiles stay whole.
+static bool pair_room(const xotb200_lm* e) { return e->pair_ws && e->stream != e->side; }
 template <int EPI, typename TC>
 static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& mb, const LtcArgs& a) {
   auto kern = ltc_pair_kernel<EPI, TC>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LTP_SMEM));
-  const int tiles = cdiv(a.M, 2 * LTC_M) * cdiv(a.N, LTP_N), pairs = std::min(tiles, e->sm_count / 2);
-  TRY(launch_late(e, kern, 2 * pairs, LTP_THREADS, LTP_SMEM, ma, mb, a));
+  const int tiles = cdiv(a.M, 2 * LTC_M) * cdiv(a.N, LTP_N), pairs = std::max(1, e->sm_count / 2);
+  LtcArgs b = a;
+  if (pair_room(e)) {
+    b.split = xb::pair_split(tiles, pairs, cdiv(a.K, LTC_BK));
+    b.split.ws = e->pair_ws;
+    b.split.flags = reinterpret_cast<int*>(e->pair_ws + (size_t)xb::pair_slots(pairs) * xb::PAIR_SLOT);
+  }
+  TRY(launch_late(e, kern, 2 * xb::pair_count(tiles, pairs, b.split), LTP_THREADS, LTP_SMEM, ma, mb, b));
   e->tc_launches++;
   return 0;
 }
@@ -870,8 +879,9 @@ static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& 
 // (layered_tc.cuh), which lose less in the last wave.  1024 rows, 128 x 128 tiles / pairs: 6144 columns with K = 1536 (65 %) 33 / 28 us, 6720 with 4096 (71 %) 70 / 55, 2144 with
 // 4096 (45 %) 29 / 33.  K < 512: filling the ring is most of a tile.
 static bool pairs_pay(const xotb200_lm* e, int M, int N, int K) {
-  const long tiles = (long)cdiv(M, 2 * LTC_M) * cdiv(N, LTP_N), pairs = std::max(1, e->sm_count / 2), waves = (tiles + pairs - 1) / pairs;
-  return K >= 512 && (double)M * N >= 0.6 * (double)waves * pairs * (2.0 * LTC_M * LTP_N);
+  const int tiles = cdiv(M, 2 * LTC_M) * cdiv(N, LTP_N), pairs = std::max(1, e->sm_count / 2);
+  const double waves = pair_room(e) ? xb::pair_waves(tiles, pairs, cdiv(K, LTC_BK)) : cdiv(tiles, pairs);
+  return K >= 512 && (double)M * N >= 0.6 * waves * pairs * (2.0 * LTC_M * LTP_N);
 }
 
 // 1 = launched, 0 = not eligible (the caller falls back), < 0 = error
@@ -1047,6 +1057,11 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
     if (e->pre_scalar) TRY(regrow(e->oh2, m * e->max_oh * z));
     TRY(regrow(e->act, m * e->max_ff * z));
     TRY(regrow(e->th, m * e->max_lr * z));
+    if (z == 2 && M > LST_MAX_ROWS && !e->pair_ws) {   // 29 MB; without them the tiles stay whole
+      const size_t slots = xb::pair_slots(std::max(1, e->sm_count / 2)), floats = slots * xb::PAIR_SLOT, flags = slots * xb::PAIR_FLAGS;
+      if (cudaMalloc(&e->pair_ws, (floats + flags) * 4) != cudaSuccess) { cudaGetLastError(); e->pair_ws = nullptr; }
+      else CK(cudaMemsetAsync(e->pair_ws + floats, 0, flags * 4, e->stream));
+    }
     e->m_cap = (int)m;
     e->trace_cap = 0;
   }
@@ -2530,7 +2545,7 @@ int xotb200_lm_destroy(xotb200_lm* e) {
     if (L.rel_bucket) cudaFree(L.rel_bucket);
     if (L.rel_tab) cudaFree(L.rel_tab);
   }
-  void* ptrs[] = {e->vfirst, e->oh2, e->y2, e->h0, e->gdec, e->ginw, e->gfloor, e->gnq, e->pos_freqs, e->dist_tab, e->moe_xg, e->moe_yg, e->moe_plan, e->dkk, e->drr, e->cvb, e->moe_ids, e->moe_wts, e->mact, e->du, e->dau, e->part, e->dch, e->q16, e->cbuf, e->knx, e->vxx, e->blob, e->d_stage, e->x, e->y, e->proj, e->qraw, e->qfull, e->wlog, e->oraw, e->logits, e->h, e->cqn, e->qn, e->olat, e->oh, e->act,
+  void* ptrs[] = {e->pair_ws, e->vfirst, e->oh2, e->y2, e->h0, e->gdec, e->ginw, e->gfloor, e->gnq, e->pos_freqs, e->dist_tab, e->moe_xg, e->moe_yg, e->moe_plan, e->dkk, e->drr, e->cvb, e->moe_ids, e->moe_wts, e->mact, e->du, e->dau, e->part, e->dch, e->q16, e->cbuf, e->knx, e->vxx, e->blob, e->d_stage, e->x, e->y, e->proj, e->qraw, e->qfull, e->wlog, e->oraw, e->logits, e->h, e->cqn, e->qn, e->olat, e->oh, e->act,
                   e->th, e->hw, e->trace_buf};
   for (void* p : ptrs)
     if (p) cudaFree(p);

@@ -43,6 +43,7 @@ struct LtcArgs {
   const int* tile_batch;      // not NULL: row tile t reads B's batch tile_batch[t] (A and C are not batched); a negative entry = the tile is empty
   int cols_first;             // 1: blockIdx.x walks the column tiles and blockIdx.y the row tiles (CTAs that run together share few row tiles:
                               // a grouped product then streams an expert's matrix while only that expert's rows are in flight)
+  xb::PairSplit split;        // CTA pairs: tiles cut along K
 };
 
 template <typename TC>
@@ -351,6 +352,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   const uint32_t rank = xb::cluster_ctarank();
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const int mtiles = (a.M + 2 * LTC_M - 1) / (2 * LTC_M), total = mtiles * ((a.N + NT - 1) / NT), nkb = (a.K + LTC_BK - 1) / LTC_BK;
+  const xb::PairWalk walk(total, nkb, npairs, pair, a.split);
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) { xb::mbar_init(&full[i], 1); xb::mbar_init(&empty[i], 1); }
     for (int i = 0; i < 2; ++i) { xb::mbar_init(&tmem_full[i], 1); xb::mbar_init(&tmem_empty[i], 16); }
@@ -368,9 +370,9 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     // ===== TMA producer (both CTAs): own rows of A, own half of B; completion is counted on the leader's barrier =====
     unsigned it = 0;
     bool ok = true;
-    for (int t = pair; t < total && ok; t += npairs) {
+    for (int i = 0, t, k0, k1, slot, step; ok && walk.get(i, t, k0, k1, slot, step); ++i) {
       const int m0 = (t % mtiles) * 2 * LTC_M + (int)rank * LTC_M, n0 = (t / mtiles) * NT + (int)rank * (NT / 2);
-      for (int kb = 0; kb < nkb; ++kb, ++it) {
+      for (int kb = k0; kb < k1; ++kb, ++it) {
         const int st = it % NS;
         ok = ltc_wait(&empty[st], ((it / NS) & 1u) ^ 1u, a.err);
         if (!ok) break;
@@ -388,12 +390,12 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     constexpr uint32_t idesc = ltc_idesc(2 * LTC_M, NT);
     unsigned it = 0, ti = 0;
     bool ok = true;
-    for (int t = pair; t < total && ok; t += npairs, ++ti) {
+    for (int t, k0, k1, slot, step; ok && walk.get((int)ti, t, k0, k1, slot, step); ++ti) {
       const uint32_t buf = ti & 1u, acc = tmem_base + buf * NT;
       ok = ltc_wait(&tmem_empty[buf], ((ti >> 1) & 1u) ^ 1u, a.err);     // both CTAs' epilogues have drained it
       if (!ok) break;
       xb::tc_fence_after();
-      for (int kb = 0; kb < nkb; ++kb, ++it) {
+      for (int kb = k0; kb < k1; ++kb, ++it) {
         const int st = it % NS;
         ok = ltc_wait(&full[st], (it / NS) & 1u, a.err);
         if (!ok) break;
@@ -401,7 +403,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const uint32_t sa = xb::smem_u32(base + (size_t)st * LTP_STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
         for (int k = 0; k < LTC_BK / 16; ++k)
-          xb::umma_bf16_2sm(acc, xb::umma_desc_sw128(sa + k * 32), xb::umma_desc_sw128(sb + k * 32), idesc, (kb | k) != 0 ? 1u : 0u);
+          xb::umma_bf16_2sm(acc, xb::umma_desc_sw128(sa + k * 32), xb::umma_desc_sw128(sb + k * 32), idesc, kb != k0 || k != 0 ? 1u : 0u);
         xb::umma_commit_2sm(&empty[st], 3);                              // frees the stage in both CTAs
       }
       if (ok) xb::umma_commit_2sm(&tmem_full[buf], 3);
@@ -414,15 +416,35 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const LtcEpilogue<EPI, TC> ep(a);
     uint8_t* mine = staged + (warp - 4) * LTC_STAGED;
     unsigned ti = 0;
-    for (int t = pair; t < total; t += npairs, ++ti) {
+    for (int t, k0, k1, slot, step; walk.get((int)ti, t, k0, k1, slot, step); ++ti) {
       const uint32_t buf = ti & 1u;
       const int row = (t % mtiles) * 2 * LTC_M + (int)rank * LTC_M + q * 32 + lane, n0 = (t / mtiles) * NT;
       if (!ltc_wait(&tmem_full[buf], (ti >> 1) & 1u, a.err)) break;
       xb::tc_fence_after();
+      const bool part = k1 < nkb;
+      const int front = k0 == 0 && !part ? 0 : walk.before(t);   // pieces of the tile in front of this one
+      const bool add = !part && front > 0;
+      float4 f[4];
+      if (add) {
+        if (!xb::pair_flags_wait(a.split, slot, step, front, rank, warp - 4)) {
+          atomicExch(a.err, 3);
+          break;
+        }
+        xb::pair_fetch16(xb::pair_slot(a.split, slot, rank, warp - 4, 0), f);
+      }
 #pragma unroll 1
       for (int c0 = half * (NT / 2); c0 < (half + 1) * (NT / 2); c0 += 16) {
         uint32_t v[16];
         xb::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + buf * NT + (uint32_t)c0, v);   // warp-collective: before any row / column test
+        const int piece = c0 / 16 % 8;
+        if (part) {
+          xb::pair_leave16(xb::pair_slot(a.split, slot + front * step, rank, warp - 4, piece), v);
+          continue;
+        }
+        if (add) {
+          xb::pair_add16(a.split, slot, step, front, rank, warp - 4, piece, f, v);
+          if (piece < 7) xb::pair_fetch16(xb::pair_slot(a.split, slot, rank, warp - 4, piece + 1), f);
+        }
         if constexpr (EPI == EPI_CLOSE) {
           if (row < a.M && n0 + c0 < a.N) ep.store16(a, static_cast<TC*>(a.C) + (size_t)row * a.ldc, row, n0 + c0, v);
         } else {
@@ -435,6 +457,8 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       xb::tc_fence_before();
       __syncwarp();
       if (lane == 0) xb::mbar_arrive_cluster(leader_empty + buf * 8);
+      if (part) xb::pair_flag_set(a.split, slot + front * step, rank, warp - 4);
+      else if (add) xb::pair_flags_clear(a.split, slot, step, front, rank, warp - 4);
     }
   }
   __syncwarp();

@@ -13,6 +13,7 @@
 // sharded_inference_engine.py:108-193,230-370).  Around the GEMMs: RMSNorm, RoPE + KV append, causal attention over the
 // prompt, SwiGLU, arg-max — small row-parallel kernels.
 #pragma once
+#include <algorithm>
 #include <cuda.h>   // CUtensorMap + enums only; cuTensorMapEncodeTiled is fetched with cudaGetDriverEntryPoint (no -lcuda)
 
 #include "kernels.cuh"
@@ -34,6 +35,13 @@ enum { TCE_STORE = 0, TCE_RESID = 1, TCE_HEAD_LAST = 2, TCE_QKV = 3, TCE_SWIGLU 
 constexpr int TC_CHUNK = 4096, TC_CHUNK_SMALL = 1024;
 constexpr int TC_FEW = 8;        // fewer positions than this keep what the decode kernel computes in 32 bits in 32 bits (tc_row_attn_kernel)
 
+// tiles of a CTA-pair product that are cut along K (PairWalk)
+struct PairSplit {
+  int n[2], s[2];                      // two phases: tiles, pieces of each; n = 0: none
+  float* ws;                           // [slots][PAIR_SLOT] accumulators
+  int* flags;                          // [slots][PAIR_FLAGS], 0 between launches
+};
+
 struct TcGemmArgs {
   int S;            // valid token rows of the chunk (grid.x = ceil(S/128) token tiles; HEAD_LAST: only the last tile)
   int N, K, tk;     // output features, reduction length, K-panel width of the weight layout
@@ -48,6 +56,7 @@ struct TcGemmArgs {
   const float2* rope;     // [L][hd/2] (cos, sin)
   int q_rows, kv_rows, hd, L, pos0;
   int* err;               // error word in page-locked host memory: 3 = a bounded wait expired
+  PairSplit split;        // CTA pairs: tiles cut along K
 };
 
 __host__ __device__ constexpr int tc_stage_bytes(int nt) { return TC_M * TC_BK * 2 + nt * TC_BK * 2; }
@@ -156,6 +165,135 @@ __device__ __forceinline__ void umma_commit_2sm(uint64_t* bar, uint16_t mask) {
 }
 __host__ __device__ constexpr int tc2_stage_bytes(int nt) { return TC_M * TC_BK * 2 + (nt / 2) * TC_BK * 2; }   // per CTA: own A rows + half of B
 __host__ __device__ constexpr int tc2_smem_bytes(int nt, int ns) { return ns * tc2_stage_bytes(nt) + 1024 + 256; }
+
+// ---- CTA pairs: the tiles that do not fill a wave -----------------------------------------------------------------------
+// Persistent pairs walk `total` tiles, wave by wave.  What is left beyond whole waves would keep a few pairs busy for a whole tile while the others idle: 1024 x 14336
+// columns are 224 tiles for 74 pairs, three waves and two tiles.  Those tiles come last and are cut along K, in one phase or two: n tiles in s equal pieces, n * s <= pairs.  A
+// pair that has another piece than a tile's last leaves its fp32 accumulator in a slot and sets one flag per epilogue warp; the same warp of who has the last piece adds the
+// slots in the order of K (deterministic) and finishes the tile.  Measured (B200): 2701 rows of 4096 x 14336, 2.38 waves,
+// 140 -> 113 us; 1024 rows of 4096 x 4096 cut as well, 33 -> 43: leaving and adding a slot takes some 13 us, hence PAIR_MIN_GAIN.
+constexpr int PAIR_SLOT = 256 * 256, PAIR_FLAGS = 16;   // floats of a slot; flags: [2 CTAs][8 warps]
+__host__ __device__ constexpr int pair_slots(int pairs) { return pairs + pairs / 2; }   // a first phase of two pieces leaves pairs / 2, the second fewer than pairs
+// Pieces of a tile: the finisher's epilogue reads them all, some 1 us each (128 KB a CTA), and a K block takes 0.4 us: about sqrt(K blocks / 2) pieces are cheapest.
+// The cut has to save more K blocks of a tile than leaving and adding up a slot takes: some 13 us in all, bound by L2 (19 MB written and read by all pairs); 52 blocks saved (1024 rows of
+// 14336 x 4096, two tiles in five) made no difference, 99 -> 98 us.
+constexpr int PAIR_MAX_PIECES = 6, PAIR_MIN_KB = 4, PAIR_MIN_GAIN = 64;
+inline int pair_pieces(int n, int pairs, int nkb) {
+  int s = 1;
+  while (s < PAIR_MAX_PIECES && n * (s + 1) <= pairs && 2 * (s + 1) * (s + 1) <= nkb && nkb / (s + 1) >= PAIR_MIN_KB) ++s;
+  return s;
+}
+inline PairSplit pair_split(int total, int pairs, int nkb) {
+  PairSplit r = {};
+  const int rem = total % pairs, half = pairs / 2;
+  if (rem == 0) return r;
+  if (rem <= half) {
+    const int s = pair_pieces(rem, pairs, nkb);
+    if (nkb - nkb / s >= PAIR_MIN_GAIN) { r.n[0] = rem; r.s[0] = s; }
+  } else if (rem > half && half > 0) {               // half of the pairs' tiles in two pieces, the rest in as many as fit: pays from three pieces on
+    const int s = pair_pieces(rem - half, pairs, nkb);
+    if (nkb - nkb / 2 - nkb / s >= PAIR_MIN_GAIN) { r.n[0] = half; r.s[0] = 2; r.n[1] = rem - half; r.s[1] = s; }
+  }
+  return r;
+}
+// waves that the walk takes, in units of a tile
+inline double pair_waves(int total, int pairs, int nkb) {
+  const PairSplit r = pair_split(total, pairs, nkb);
+  return total / pairs + (r.n[0] ? 1.0 / r.s[0] + (r.n[1] ? 1.0 / r.s[1] : 0.0) : total % pairs ? 1.0 : 0.0);
+}
+// pairs that have anything to do
+inline int pair_count(int total, int pairs, const PairSplit& r) { return std::max(std::min(total, pairs), std::max(r.n[0] * r.s[0], r.n[1] * r.s[1])); }
+struct PairWalk {
+  int whole, nkb, npairs, pair;                      // tiles that are not cut: the first ones
+  const PairSplit& s;
+  __device__ __forceinline__ PairWalk(int total, int nkb_, int npairs_, int pair_, const PairSplit& s_) : whole(total - s_.n[0] - s_.n[1]), nkb(nkb_), npairs(npairs_), pair(pair_), s(s_) {}
+  // the i-th piece of this pair: K blocks [k0, k1) of tile t.  slot: where the tile's first piece is left, the next ones `step` further each
+  __device__ __forceinline__ bool get(int i, int& t, int& k0, int& k1, int& slot, int& step) const {
+    const int mine = pair < whole ? (whole - pair + npairs - 1) / npairs : 0;
+    if (i < mine) {
+      t = pair + i * npairs;
+      k0 = 0;
+      k1 = nkb;
+      return true;
+    }
+    i -= mine;
+    int from = whole, first = 0;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const int n = s.n[p], pieces = s.s[p];
+      if (pair < n * pieces) {
+        if (i == 0) {
+          const int j = pair / n;
+          t = from + pair % n;
+          k0 = j * nkb / pieces;
+          k1 = (j + 1) * nkb / pieces;
+          slot = first + pair % n;
+          step = n;
+          return true;
+        }
+        --i;
+      }
+      from += n;
+      first += n * (pieces - 1);
+    }
+    return false;
+  }
+  // which piece of its tile begins at K block k0 (its tile is cut): the number of slots in front of it
+  __device__ __forceinline__ int before(int t) const { return t < whole ? 0 : pair / (t < whole + s.n[0] ? s.n[0] : s.n[1]); }
+};
+// 16 columns (piece c of 8) of a warp's part of a slot: [2 CTAs][8 warps][8 pieces][4][32 lanes] float4
+__device__ __forceinline__ float4* pair_slot(const PairSplit& s, int slot, uint32_t rank, int w, int c) {
+  return reinterpret_cast<float4*>(s.ws + (size_t)slot * PAIR_SLOT) + (((size_t)rank * 8 + w) * 8 + c) * 128 + (threadIdx.x & 31);
+}
+__device__ __forceinline__ void pair_leave16(float4* d, const uint32_t (&v)[16]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) __stcg(d + j * 32, make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
+}
+__device__ __forceinline__ void pair_fetch16(const float4* d, float4 (&f)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) f[j] = __ldcg(d + j * 32);
+}
+// the n pieces of a tile from slot `slot` on, in the order of K, then v; f: the first piece, fetched already
+__device__ __forceinline__ void pair_add16(const PairSplit& s, int slot, int step, int n, uint32_t rank, int w, int c, float4 (&f)[4], uint32_t (&v)[16]) {
+  for (int p = 1; p < n; ++p) {
+    float4 x[4];
+    pair_fetch16(pair_slot(s, slot + p * step, rank, w, c), x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { f[j].x += x[j].x; f[j].y += x[j].y; f[j].z += x[j].z; f[j].w += x[j].w; }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[4 * j] = __float_as_uint(f[j].x + __uint_as_float(v[4 * j]));
+    v[4 * j + 1] = __float_as_uint(f[j].y + __uint_as_float(v[4 * j + 1]));
+    v[4 * j + 2] = __float_as_uint(f[j].z + __uint_as_float(v[4 * j + 2]));
+    v[4 * j + 3] = __float_as_uint(f[j].w + __uint_as_float(v[4 * j + 3]));
+  }
+}
+__device__ __forceinline__ void pair_flag_set(const PairSplit& s, int slot, uint32_t rank, int w) {   // whole warp, behind its stores
+  __threadfence();
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) asm volatile("st.release.gpu.global.s32 [%0], 1;" ::"l"(s.flags + (slot * 2 + (int)rank) * 8 + w) : "memory");
+}
+// whole warp: the n pieces from slot `slot` on are there; false: the limit was reached
+__device__ __forceinline__ bool pair_flags_wait(const PairSplit& s, int slot, int step, int n, uint32_t rank, int w) {
+  bool ok = true;
+  if ((threadIdx.x & 31) == 0)
+    for (int p = 0; p < n && ok; ++p) {
+      int* f = s.flags + ((slot + p * step) * 2 + (int)rank) * 8 + w;
+      int there = 0;
+      for (unsigned i = 0; i < (1u << 24) && !there; ++i) asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(there) : "l"(f) : "memory");
+      ok = there != 0;
+    }
+  ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+  __threadfence();
+  return ok;
+}
+// whole warp, behind its last read of the slots: the flags are down again for the next launch
+__device__ __forceinline__ void pair_flags_clear(const PairSplit& s, int slot, int step, int n, uint32_t rank, int w) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0)
+    for (int p = 0; p < n; ++p) s.flags[((slot + p * step) * 2 + (int)rank) * 8 + w] = 0;
+}
 
 // ---- few token rows (tc_stream_kernel): 128 weight rows are the M operand, NB token rows the N side; two CTAs share an SM's shared memory
 __host__ __device__ constexpr int tcs_stage_bytes(int nb) { return TC_M * TC_BK * 2 + nb * TC_BK * 2; }
