@@ -3,14 +3,16 @@
 //   warp 0   one thread brings Q once and then the key / value tiles of 64 tokens by TMA (SWIZZLE_128B) into their rings;
 //   warp 1   one lane issues tcgen05.mma: S_j = Q K_j^T (128 x 64, fp32, tensor memory) one tile ahead, then O += P_j V_j with P read from tensor
 //            memory and V as it lies in memory ([token][value], the MN-major form of the B operand);
-//   warps 2-5  thread = query row: the row's 64 scores come by tcgen05.ld, so scale, soft cap, distance terms, mask, maximum and sum need no
-//            shuffle; the weights go back over the scores as the packed A operand of the value product.
+//   warps 2-9  two threads to a query row, 32 of a tile's 64 scores each: they come by tcgen05.ld, so scale, soft cap, distance terms, mask, maximum and sum need no
+//            shuffle (the two maxima meet in shared memory); the weights go back over the scores as the packed A operand of the value product.  A row in one
+//            thread left a scheduler two warps at most, 4500 cycles a tile against the 1500 of its exponentials.
 // PAIR: the weights enter the value product as a 16-bit PAIR (high part + remainder, two MMAs), 16 mantissa bits instead of 8.
 // The output is rescaled only when a row's maximum has grown by more than 2^8 since the last time (the reference the exponentials are taken
 // against is then stale by that factor at most, which fp32 sums and floating-point weights carry without loss).  Scores are kept in units of
 // ln 2.  Two CTAs share an SM (256 of the 512 tensor-memory columns and at most 112 KB each), so one's exponentials run under the other's MMAs: bound
 // by the exponentials and the arithmetic around them, not by the tensor pipe.
-// Measured (B200, a launch, 64-row mma.sync tiles -> this kernel): grouped keys, 3500 rows x 16 heads of 128, soft cap, distance terms, a gate per entry: 377 -> 122 us, -> 87 with cheap sigmoids (one portion of 64 rows 33 -> 20);
+// Measured (B200, a launch, 64-row mma.sync tiles -> this kernel): grouped keys, 3500 rows x 16 heads of 128, soft cap, distance terms, a gate per entry: 377 -> 122 us, -> 87 with cheap sigmoids, -> 77 with
+// two threads to a row (a portion of 64 rows behind a few hundred keys 35 -> 18 us a launch in its step, half of it the gate);
 // latent keys, 1024 rows x 32 heads of 192 / 128: 190 -> 52 us; 2701 rows in chunks x 32 heads of 128, 16-bit weights: 127 -> 79 us.
 // Every wait is bounded: one that expires sets *err, all roles of the CTA run out, it frees its tensor memory and returns.
 #pragma once
@@ -18,7 +20,7 @@
 
 namespace xf {
 
-constexpr int FT_Q = 128, FT_K = 64, FT_THREADS = 192;
+constexpr int FT_Q = 128, FT_K = 64, FT_THREADS = 320;
 constexpr unsigned FT_SPIN_LIMIT = 1u << 22;   // try_wait rounds (each blocks for a while in hardware): seconds, not forever
 constexpr float LOG2E = 1.4426950408889634f;
 
@@ -53,7 +55,7 @@ struct FlashArgs {
 __host__ __device__ constexpr int ft_k_stages(int) { return 2; }
 __host__ __device__ constexpr int ft_v_stages(int dkc, int dvc) { return dkc * 2 + dvc <= 6 ? 2 : 1; }
 __host__ __device__ constexpr int ft_smem_bytes(int dkc, int dvc) {
-  return dkc * FT_Q * 128 + ft_k_stages(dkc) * dkc * FT_K * 128 + ft_v_stages(dkc, dvc) * dvc * FT_K * 128 + 256 + 512;
+  return dkc * FT_Q * 128 + ft_k_stages(dkc) * dkc * FT_K * 128 + ft_v_stages(dkc, dvc) * dvc * FT_K * 128 + 256 + FT_Q * 4;   // operands, barriers, a float per row
 }
 
 __device__ __forceinline__ bool ft_wait(uint64_t* bar, uint32_t parity, volatile int* abort, int* err) {
@@ -91,6 +93,13 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
                "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
                : "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+               "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+               : "memory");
+}
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* m) { asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // A from tensor memory (one 32-bit column = two consecutive k of a row), B from shared memory
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
@@ -139,11 +148,28 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  xb::pdl_wait();
-  if (base - ft_smem > 512) {                        // cannot be (the shared window starts on a 1 KB boundary); the sizes leave 512 bytes for it
+  float* row_sm = reinterpret_cast<float*>(vs + VS * V_BYTES + 256);
+  if (base != ft_smem) {                             // cannot be: the shared window starts on a 1 KB boundary
     if (threadIdx.x == 0 && a.err) *static_cast<volatile int*>(a.err) = 4;
     return;
   }
+  // what depends on no kernel in front, ahead of the wait
+  if (threadIdx.x == 0) {
+    *abort = 0;
+    xb::mbar_init(q_full, 1);
+    for (int i = 0; i < KS; ++i) { xb::mbar_init(&k_full[i], 1); xb::mbar_init(&k_empty[i], 1); }
+    for (int i = 0; i < VS; ++i) { xb::mbar_init(&v_full[i], 1); xb::mbar_init(&v_empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { xb::mbar_init(&s_full[i], 1); xb::mbar_init(&p_full[i], 256); xb::mbar_init(&pv_done[i], 1); }
+    xb::fence_mbar_init();
+    prefetch_map(&tmQ); prefetch_map(&tmK); prefetch_map(&tmK2); prefetch_map(&tmV);
+  }
+  if (warp == 1) xb::tmem_alloc(tmem_slot, COLS);
+  xb::tc_fence_before();
+  __syncthreads();
+  xb::tc_fence_after();
+  const uint32_t tmem = *tmem_slot, tm_o = tmem + 128;
+  xb::pdl_launch_dependents();   // not before: a later kernel's CTA that takes tensor memory and then waits for this kernel must not take it first
+  xb::pdl_wait();
   FlashTile128 tl;
   // later tiles of a request see more keys: the long ones start first, those of all heads before any shorter one (the heads are the grid's fast side)
   if (a.tiles) tl = a.tiles[gridDim.y - 1 - blockIdx.y];
@@ -160,21 +186,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   // weight is 0, but 0 * Inf is not.  The rows of the value stage they lie in — `front` of the first tile, `behind` of the last — are zeroed before the
   // product reads them (a row of a chunk is 128 bytes, swizzled within itself).
   const int front = ft_first_key(tl.pos0, a.window, a.chunk) - jstart, behind = nt * FT_K - (last + 1 - jstart);
-  if (threadIdx.x == 0) {
-    *abort = 0;
-    xb::mbar_init(q_full, 1);
-    for (int i = 0; i < KS; ++i) { xb::mbar_init(&k_full[i], 1); xb::mbar_init(&k_empty[i], 1); }
-    for (int i = 0; i < VS; ++i) { xb::mbar_init(&v_full[i], 1); xb::mbar_init(&v_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { xb::mbar_init(&s_full[i], 1); xb::mbar_init(&p_full[i], 128); xb::mbar_init(&pv_done[i], 1); }
-    xb::fence_mbar_init();
-  }
-  if (warp == 1) xb::tmem_alloc(tmem_slot, COLS);
-  xb::tc_fence_before();
-  __syncthreads();
-  xb::tc_fence_after();
-  const uint32_t tmem = *tmem_slot, tm_o = tmem + 128;
-  xb::pdl_launch_dependents();   // not before: a later kernel's CTA that takes tensor memory and then waits for this kernel must not take it first
-
   if (warp == 0) {
     if (lane == 0) {
       // ===== TMA producer =====
@@ -259,68 +270,76 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else {
-    // ===== softmax: warp w reads tensor-memory lanes 32 (w mod 4) .. =====
+    // ===== softmax: warps w and w + 4 read tensor-memory lanes 32 (w mod 4) .., scores 0 .. 31 and 32 .. 63 of a tile, the lower and the upper half of the output's columns =====
+    const int half = (warp - 2) >> 2, id = 1 + (warp & 3);
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const int r = (warp & 3) * 32 + lane, pos = tl.pos0 + r;
     const int lo = ft_first_key(pos, a.window, a.chunk), lo_last = ft_first_key(last, a.window, a.chunk);
     const float scale2 = a.scale * LOG2E, inv_cap2 = a.cap > 0.f ? 2.0f * LOG2E * a.scale / a.cap : 0.f, cap2 = a.cap * LOG2E;
     const float* dist = a.dist ? a.dist + (size_t)h * a.dist_n : nullptr;
     const float* rel = a.rel ? a.rel + (size_t)h * a.rel_n : nullptr;
-    float m = -INFINITY, den = 0.f;                  // reference of the exponentials (units of ln 2), sum of the weights
+    // one number from the two threads of a row, the same for both; what they did to tensor memory before is done for both behind it
+    auto join = [&](float v, auto op) {
+      xb::tc_fence_before();
+      if (half) row_sm[r] = v;
+      pair_sync(id);
+      if (!half) { v = op(v, row_sm[r]); row_sm[r] = v; }
+      pair_sync(id);
+      xb::tc_fence_after();
+      return half ? row_sm[r] : v;
+    };
+    float m = -INFINITY, den = 0.f;                  // reference of the exponentials (units of ln 2), this thread's sum of the weights
     bool ok = true;
     int j = 0;
     for (; j < nt; ++j) {
       // no row of this warp sees this tile or a later one: the warp's output is taken out before their products are added to it (0 * Inf again)
       if (jstart + j * FT_K > pos - lane + 31) break;
       ok = __all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err));
-      if (!ok) break;
       xb::tc_fence_after();
       const uint32_t ts = tmem + lane_base + (j & 1) * 64;
-      uint32_t raw[2][32];
-      tmem_ld32(ts, raw[0]);
-      tmem_ld32(ts + 32, raw[1]);
-      float s[64];
+      uint32_t raw[32];
+      tmem_ld32(ts + half * 32, raw);
+      float s[32];
 #pragma unroll
-      for (int c = 0; c < 64; ++c) s[c] = __uint_as_float(raw[c >> 5][c & 31]);
-      const int j0 = jstart + j * FT_K;
+      for (int c = 0; c < 32; ++c) s[c] = __uint_as_float(raw[c]);
+      const int j0 = jstart + j * FT_K + half * 32;
       if (a.cap > 0.f) {                             // cap tanh(x / cap) with tanh y = 1 - 2 / (e^2y + 1): right at both ends too (e^2y = inf, 0)
 #pragma unroll
-        for (int c = 0; c < 64; ++c) s[c] = fmaf(-2.0f * cap2, rcp(ex2(s[c] * inv_cap2) + 1.0f), cap2);
+        for (int c = 0; c < 32; ++c) s[c] = fmaf(-2.0f * cap2, rcp(ex2(s[c] * inv_cap2) + 1.0f), cap2);
       } else {
 #pragma unroll
-        for (int c = 0; c < 64; ++c) s[c] *= scale2;
+        for (int c = 0; c < 32; ++c) s[c] *= scale2;
       }
-      const bool all = j0 + FT_K - 1 <= tl.pos0 && j0 >= lo_last;   // every row of the tile sees every key of it
-      if (dist && all && pos - j0 < a.dist_n) {              // no distance outside the table: one address for the tile
+      const bool all = j0 + 31 <= tl.pos0 && j0 >= lo_last;         // every row of the tile sees every key of this half
+      if (dist && all && pos - j0 < a.dist_n) {              // no distance outside the table: one address for the half
         const float* dp = dist + (pos - j0);
 #pragma unroll
-        for (int c = 0; c < 64; ++c) s[c] = fmaf(-LOG2E, __ldg(dp - c), s[c]);
+        for (int c = 0; c < 32; ++c) s[c] = fmaf(-LOG2E, __ldg(dp - c), s[c]);
       } else if (dist) {
 #pragma unroll
-        for (int c = 0; c < 64; ++c) s[c] = fmaf(-LOG2E, __ldg(dist + min(max(pos - j0 - c, 0), a.dist_n - 1)), s[c]);
+        for (int c = 0; c < 32; ++c) s[c] = fmaf(-LOG2E, __ldg(dist + min(max(pos - j0 - c, 0), a.dist_n - 1)), s[c]);
       }
       if (rel) {
 #pragma unroll
-        for (int c = 0; c < 64; ++c) s[c] = fmaf(LOG2E, __ldg(rel + min(max(pos - j0 - c, 0), a.rel_n - 1)), s[c]);
+        for (int c = 0; c < 32; ++c) s[c] = fmaf(LOG2E, __ldg(rel + min(max(pos - j0 - c, 0), a.rel_n - 1)), s[c]);
       }
       if (!all) {
         const int clo = lo - j0, chi = pos - j0;
 #pragma unroll
-        for (int c = 0; c < 64; ++c) s[c] = c >= clo && c <= chi ? s[c] : -INFINITY;
+        for (int c = 0; c < 32; ++c) s[c] = c >= clo && c <= chi ? s[c] : -INFINITY;
       }
       float t0 = fmaxf(s[0], s[1]), t1 = fmaxf(s[2], s[3]);
 #pragma unroll
-      for (int c = 4; c < 64; c += 4) { t0 = fmaxf(t0, fmaxf(s[c], s[c + 1])); t1 = fmaxf(t1, fmaxf(s[c + 2], s[c + 3])); }
-      const float tmax = fmaxf(t0, t1);
+      for (int c = 4; c < 32; c += 4) { t0 = fmaxf(t0, fmaxf(s[c], s[c + 1])); t1 = fmaxf(t1, fmaxf(s[c + 2], s[c + 3])); }
+      const float tmax = join(fmaxf(t0, t1), [](float x, float y) { return fmaxf(x, y); });   // also: nobody writes weights over scores that the other has not read
       const bool grow = tmax > m + 8.0f || (m == -INFINITY && tmax > -INFINITY);
       if (__any_sync(0xffffffffu, grow)) {
         const float nm = fmaxf(m, tmax), corr = m == -INFINITY ? 0.f : ex2(m - nm);
         if (j > 0) {
-          ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort, a.err));   // the output as it is
-          if (!ok) break;
+          ok = ok && __all_sync(0xffffffffu, ft_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort, a.err));   // the output as it is
           xb::tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < 64 * DVC; c += 32) {
+          for (int c = half * 32 * DVC; c < (half + 1) * 32 * DVC; c += 32) {
             uint32_t o[32];
             tmem_ld32(tm_o + lane_base + c, o);
 #pragma unroll
@@ -334,9 +353,9 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const float mm = m == -INFINITY ? 0.f : m;     // a row that has not seen a key yet: every weight is ex2(-inf) = 0
       float d0 = 0.f, d1 = 0.f;
-      uint32_t hi[32], rest[32];
+      uint32_t hi[16], rest[16];
 #pragma unroll
-      for (int c = 0; c < 64; c += 2) {
+      for (int c = 0; c < 32; c += 2) {
         const float p0 = ex2(s[c] - mm), p1 = ex2(s[c + 1] - mm);
         d0 += p0;
         d1 += p1;
@@ -345,18 +364,22 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           rest[c >> 1] = pack16<F16>(p0 - __uint_as_float(hi[c >> 1] << 16), p1 - __uint_as_float(hi[c >> 1] & 0xffff0000u));
       }
       den += d0 + d1;
-      tmem_st32(ts, hi);
-      if constexpr (PAIR) tmem_st32(ts + 32, rest);
+      tmem_st16(ts + half * 16, hi);
+      if constexpr (PAIR) tmem_st16(ts + 32 + half * 16, rest);
       tmem_st_wait();
       xb::tc_fence_before();
       mbar_arrive(&p_full[j & 1]);
     }
+    den = join(den, [](float x, float y) { return x + y; });
+    // From here on a wait that expired ends the CTA's work: the two warps of a row exchange nothing more.  (Inside the loop they stay together: the exchanges take both.)
+    if (*abort) ok = false;
+    ok = __all_sync(0xffffffffu, ok);
     if (ok) ok = __all_sync(0xffffffffu, ft_wait(&pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, abort, a.err));
-    if (ok && j < nt) {                              // tiles this warp sees nothing of: it keeps its output while their products, which wait for all four warps, run
+    if (ok && j < nt) {                              // tiles this warp sees nothing of: it keeps its output while their products, which wait for all eight warps, run
       xb::tc_fence_after();
-      uint32_t o[2 * DVC][32];
+      uint32_t o[DVC][32];
 #pragma unroll
-      for (int c = 0; c < 2 * DVC; ++c) tmem_ld32(tm_o + lane_base + c * 32, o[c]);
+      for (int c = 0; c < DVC; ++c) tmem_ld32(tm_o + lane_base + (half * DVC + c) * 32, o[c]);
       for (; j < nt && ok; ++j) {
         ok = __all_sync(0xffffffffu, ft_wait(&s_full[j & 1], (j >> 1) & 1, abort, a.err));
         xb::tc_fence_before();
@@ -366,7 +389,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (ok) {
         xb::tc_fence_after();
 #pragma unroll
-        for (int c = 0; c < 2 * DVC; ++c) tmem_st32(tm_o + lane_base + c * 32, o[c]);
+        for (int c = 0; c < DVC; ++c) tmem_st32(tm_o + lane_base + (half * DVC + c) * 32, o[c]);
         tmem_st_wait();
       }
     }
@@ -384,17 +407,17 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (a.gate_mode == 1 && gt) f *= 1.0f / (1.0f + expf(-*gt));
       uint16_t* dst = static_cast<uint16_t*>(a.out) + (row * a.H + h) * (64 * DVC);
 #pragma unroll 1   // with few tiles fetching the code counts (requests in portions of 64 rows: 8720 us a pass, 8990 with this loop unrolled)
-      for (int c = 0; c < 64 * DVC; c += 32) {
-        uint32_t o[32];
-        tmem_ld32(tm_o + lane_base + c, o);
+      for (int c = half * 32 * DVC; c < (half + 1) * 32 * DVC; c += 16) {
+        uint32_t o[16];
+        xb::tmem_ld16(tm_o + lane_base + c, o);
         if (r < tl.n_rows) {
-          float v[32];
+          float v[16];
 #pragma unroll
-          for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(o[i]) * f;
+          for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(o[i]) * f;
           if (a.gate_mode == 2) {   // sigmoids with the hardware's power of two and reciprocal (2e-6 off at gates of -30, the output has 8 bits): expf and an exact division took 18 us of a 33 us launch
             const bool vec = ((reinterpret_cast<uintptr_t>(gt) | (uintptr_t)c) & 15) == 0;
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
+            for (int i = 0; i < 16; i += 4) {
               const float4 z = vec ? *reinterpret_cast<const float4*>(gt + c + i) : make_float4(gt[c + i], gt[c + i + 1], gt[c + i + 2], gt[c + i + 3]);
               v[i] *= rcp(1.0f + ex2(-LOG2E * z.x));
               v[i + 1] *= rcp(1.0f + ex2(-LOG2E * z.y));
@@ -403,7 +426,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             }
           }
 #pragma unroll
-          for (int i = 0; i < 32; i += 8)
+          for (int i = 0; i < 16; i += 8)
             *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(pack16<F16>(v[i], v[i + 1]), pack16<F16>(v[i + 2], v[i + 3]), pack16<F16>(v[i + 4], v[i + 5]), pack16<F16>(v[i + 6], v[i + 7]));
         }
         __syncwarp();
