@@ -1159,11 +1159,12 @@ static bool latent_row_pays(const xotb200_lm* e, const xotb200_lm_layer& s, bool
   if (s.heads > 8) return blocks <= LATENT_ROW_ALWAYS || blocks * keys <= LATENT_ROW_WORK;
   return keys <= LATENT_ROW_ONE_BLOCK && blocks * keys <= LATENT_ROW_WORK;
 }
-// its shares of the keys: about one block per SM, four turns of four keys or more each
+// its shares of the keys: at most one block per SM, which is what its registers allow (a second wave of blocks costs more than longer shares: 16 requests of 30 tokens, 32 heads, three layers a
+// step, 3 shares on 192 blocks 437 us, 2 on 128 417), four turns of four keys or more each
 static int latent_row_shares(const xotb200_lm* e, const xotb200_lm_layer& s, int n_items, int max_len, int* keys) {
   const int span = latent_row_span(s, max_len);
   const long ctas = std::max(1L, (long)n_items * cdiv(s.heads, 8));
-  const int shares = (int)std::max(1L, std::min(std::min(32L, (long)cdiv(span, 4 * LROW_KEYS)), (e->sm_count + ctas - 1) / ctas));
+  const int shares = (int)std::max(1L, std::min(std::min(32L, (long)cdiv(span, 4 * LROW_KEYS)), e->sm_count / ctas));
   *keys = cdiv(span, shares);
   return shares;
 }
@@ -1565,11 +1566,13 @@ static bool gqa_row_pays(const xotb200_lm_layer& s, bool single, int n_items, in
   return s.dim == 64 || s.heads / s.kv_heads < 16 || gqa_row_span(s, longest) <= 256 || tiles <= 2 || tiles > 16;
 }
 static int gqa_row_heads(const xotb200_lm_layer& s) { const int rep = s.heads / s.kv_heads; return rep % 4 == 0 ? 4 : rep % 2 == 0 ? 2 : 1; }
-// its shares of the keys: about one block per SM, two turns of 32 keys or more each
+// its shares of the keys, a turn of 32 or more each (two beyond what a cluster holds): heads of 128 at most one block per SM, which is what its registers allow (three layers a step, 16 requests, 4 key heads: behind 30 tokens 234 -> 220 us,
+// 230 259 -> 238, 900 333 -> 295; one request behind 230, shares of one turn instead of two, 179 -> 174), heads of 64 about one (16 behind 900 218 us, at most one 234)
 static int gqa_row_shares(const xotb200_lm* e, const xotb200_lm_layer& s, int n_items, int max_len, int* keys) {
   const int span = gqa_row_span(s, max_len);
   const long ctas = std::max(1L, (long)n_items * s.heads / gqa_row_heads(s));
-  const int shares = (int)std::max(1L, std::min(std::min(32L, (long)cdiv(span, 2 * GROW_KEYS)), (e->sm_count + ctas - 1) / ctas));
+  const int by_keys = std::min(32, std::min(cdiv(span, GROW_KEYS), std::max(CLUSTER_SHARES, cdiv(span, 2 * GROW_KEYS))));
+  const int shares = (int)std::max(1L, std::min((long)by_keys, s.dim == 64 ? (e->sm_count + ctas - 1) / ctas : e->sm_count / ctas));
   *keys = cdiv(span, shares);
   return shares;
 }
