@@ -2336,11 +2336,12 @@ static int run_layers(xotb200_lm* e, const StepPlan& sp, int n_want) {
       CK(cudaMemcpyAsync(e->trace_buf + li * (size_t)M * D, e->x, (size_t)M * D * 4, cudaMemcpyDeviceToDevice, e->stream));
     }
   }
-  TRY(open(nullptr));
   if (e->trace) e->trace_floats = e->layers.size() * (size_t)M * D;
-  if (e->last && n_want > 0) {
+  if (!e->last) return open(nullptr);
+  if (n_want > 0) {
+    // the last sublayer is closed by the norm in front of the head, for the rows that go through it: nobody reads the stream behind them
     T* hw = static_cast<T*>(e->hw);
-    TRY(norm_rows(nullptr, nullptr, at<T>(e, e->final_norm), hw, sp.want, n_want));
+    TRY(norm_rows(pend_y, pend_w, at<T>(e, e->final_norm), hw, sp.want, n_want));
     TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
     TRY(finish_logits(e, n_want));
   }

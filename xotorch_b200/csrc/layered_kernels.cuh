@@ -206,8 +206,8 @@ __global__ void embed_rows_kernel(const T* __restrict__ embed, const int* __rest
 // ---------------------------------------------------------------------------------------------------------------------------
 // Fused "close one sublayer, open the next":   x += groupnorm(y) * w_post ;  h = groupnorm(x) * w_pre
 // groupnorm: the row is cut into G equal consecutive parts, each divided by sqrt(mean(part^2) + eps).  A part is shared by a few warps of the row's block.  y / w_post may be NULL (first sublayer), h / w_pre may be NULL (no
-// sublayer follows).  src_rows (may be NULL) gathers: output row m reads x row src_rows[m] and does not write x (used for the
-// final norm on the rows whose logits are wanted).
+// sublayer follows).  src_rows (may be NULL) gathers: output row m reads rows src_rows[m] of x and y and does not write x (the
+// end of a step, for the rows whose logits are wanted).
 // ---------------------------------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void residual_groupnorm_kernel(float* __restrict__ x, const float* __restrict__ y, const T* __restrict__ w_post,
@@ -228,7 +228,7 @@ __global__ void residual_groupnorm_kernel(float* __restrict__ x, const float* __
     const int g = g0 + gsel;
     const bool on = gsel < gpr && g < G;
     float* xr = x + (size_t)xm * D + (size_t)(on ? g : 0) * Dg;
-    const float* yr = y ? y + (size_t)m * D + (size_t)(on ? g : 0) * Dg : nullptr;
+    const float* yr = y ? y + (size_t)xm * D + (size_t)(on ? g : 0) * Dg : nullptr;
     float ry = 0.f;
     if (y) {
       float s = 0.f;
@@ -247,7 +247,7 @@ __global__ void residual_groupnorm_kernel(float* __restrict__ x, const float* __
         float v = xr[d];
         if (y) {
           v += yr[d] * ry * ldf(w_post + (size_t)g * Dg + d);
-          xr[d] = v;
+          if (!src_rows) xr[d] = v;                  // gathered rows may repeat
         }
         s2 = fmaf(v, v, s2);
       }
@@ -259,7 +259,10 @@ __global__ void residual_groupnorm_kernel(float* __restrict__ x, const float* __
       for (int k = 0; k < wpg; ++k) t += red[1][(warp / wpg) * wpg + k];
       const float rx = 1.0f / sqrtf(t / (float)Dg + eps);
       if (on)
-        for (int d = d0 + lane; d < d1; d += 32) stf(h + (size_t)m * D + (size_t)g * Dg + d, xr[d] * rx * ldf(w_pre + (size_t)g * Dg + d));
+        for (int d = d0 + lane; d < d1; d += 32) {
+          const float v = y && src_rows ? xr[d] + yr[d] * ry * ldf(w_post + (size_t)g * Dg + d) : xr[d];
+          stf(h + (size_t)m * D + (size_t)g * Dg + d, v * rx * ldf(w_pre + (size_t)g * Dg + d));
+        }
     }
     __syncthreads();                                 // `red` is reused by the next round
   }
@@ -292,7 +295,7 @@ __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float
   for (int v = 0; v < NV; ++v) {
     const bool on = d[v] < D;
     xv[v] = on ? ld4f(x + xm * D + d[v]) : zero;
-    yv[v] = on && y ? ld4f(y + m * D + d[v]) : zero;
+    yv[v] = on && y ? ld4f(y + xm * D + d[v]) : zero;
   }
   // 1 / rms of the part that piece v of this warp lies in
   auto part_scale = [&](float* r, int v) {
@@ -313,7 +316,7 @@ __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float
       if (v * (int)blockDim.x * 4 + warp * 128 >= D) continue;  // warp-uniform: the row's pieces are whole warps
       const float r = part_scale(red[0], v);
       xv[v].x += yv[v].x * r * wo[v].x; xv[v].y += yv[v].y * r * wo[v].y; xv[v].z += yv[v].z * r * wo[v].z; xv[v].w += yv[v].w * r * wo[v].w;
-      st4f(x + xm * D + d[v], xv[v]);
+      if (!src_rows) st4f(x + xm * D + d[v], xv[v]);            // gathered rows may repeat
     }
   }
   if (!h) return;
