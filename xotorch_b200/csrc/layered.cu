@@ -197,6 +197,8 @@ struct xotb200_lm {
   float* part = nullptr;                               // key-run partial results of the absorbed attention kernel
   size_t part_cap = 0;
   int max_w = 0;                                       // widest cached row (kv_rank + rot_dim)
+  float2* seg_best = nullptr;                          // best entry per segment of the vocabulary and wanted row (head_logits)
+  bool logits_out = false;                             // this step's logits are asked for
   float* h_out = nullptr;                              // pinned staging for results
   size_t h_out_cap = 0;
   int max_in = 0, max_q = 0, max_qfull = 0, max_qr = 0, max_hdn = 0, max_olat = 0, max_oh = 0, max_ff = 0, max_hd = 0, max_lr = 0;
@@ -1004,6 +1006,7 @@ static void drop_graphs(xotb200_lm* e) {
   e->graphs.clear();
 }
 
+constexpr int HEAD_SEGMENTS = 4;                       // head_logits
 static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
   const int D = e->cfg.width;
   if (M > e->m_cap) {
@@ -1071,6 +1074,7 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
     const size_t w = (size_t)std::max(n_want, 16);
     TRY(regrow(e->hw, w * D * e->esz));
     TRY(regrow(e->logits, w * e->cfg.vocab * 4));
+    TRY(regrow(e->seg_best, w * HEAD_SEGMENTS * sizeof(float2)));
     e->want_cap = (int)w;
   }
   if (e->trace && e->trace_cap < (size_t)e->layers.size() * e->m_cap * D) {
@@ -2031,13 +2035,45 @@ static int run_mixer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
   return 0;
 }
 
-static int finish_logits(xotb200_lm* e, int n_want) {
+// hw [n_want, D] -> logits, argmax, where the caller wants them.  Results of several rows take as long over PCIe as the head's weights take from memory (16 rows of 32000: 2 MB, 40 us; 262 MB of
+// weights, 40 us), so the vocabulary is cut into segments of about 256 KB of results, four at most, and a segment is sent, on the side stream, while the next ones are computed (8 rows, width 2048: HEAD8;
+// 16 rows, width 4096: HEAD16).
+template <typename T>
+static int head_logits(xotb200_lm* e, const T* hw, int n_want) {
+  const int D = e->cfg.width, V = e->cfg.vocab;
   const float scale = e->cfg.logit_scale != 0.f ? e->cfg.logit_scale : 1.0f;
   // Blocks (a cluster) to a row.  Where the rows alone fill the chip a cluster only costs (vocabulary of 32000, argmax alone, a small step, a block of 1024 threads before / cluster / one
   // block of 512: 100 rows 99 / 98 / - us, 148 133 / 129 / -, 400 218 / 232 / 204, 1000 372 / 401 / 327).
-  const int parts = e->cfg.vocab >= 4096 && n_want <= e->sm_count ? 8 : 1;
-  return launch_early(e, finish_rows_kernel, n_want * parts, 512, 0, parts, e->logits, e->cfg.vocab, n_want, parts, scale, e->cfg.logit_softcap,
-                      reinterpret_cast<const StepOut*>(e->d_stage), e->d_err);
+  const int parts = V >= 4096 && n_want <= e->sm_count ? 8 : 1;
+  const long pieces = e->logits_out && parts > 1 && n_want > GEMV_MAX_ROWS ? std::min<long>(HEAD_SEGMENTS, ((long)n_want * V) >> 16) : 1;
+  const int per = pieces > 1 ? cdiv(cdiv(V, pieces), LTC_M) * LTC_M : V, segs = cdiv(V, per);
+  auto columns = [&](int c0, int c1) { return product<T, T, float, EPI_NONE>(e, hw, D, 0, at<T>(e, e->head) + (size_t)c0 * D, D, 1, 0, e->logits + c0, V, 0, n_want, c1 - c0, D, 1); };
+  const StepOut* to = reinterpret_cast<const StepOut*>(e->d_stage);
+  if (segs == 1) {
+    TRY(columns(0, V));
+    return launch_early(e, finish_rows_kernel, n_want * parts, 512, 0, parts, e->logits, V, n_want, parts, scale, e->cfg.logit_softcap, to, e->d_err, 0, V, 0, 1, e->seg_best);
+  }
+  int rc = 0;
+  for (int s = 0; s < segs && rc == 0; ++s) {
+    const int c0 = s * per, c1 = std::min(V, c0 + per);
+    rc = columns(c0, c1);
+    if (rc < 0) break;
+    CK(cudaEventRecord(e->ev_fork, e->stream));
+    CK(cudaStreamWaitEvent(e->side, e->ev_fork, 0));
+    cudaStream_t main_stream = e->stream;
+    const bool early = e->early;
+    e->stream = e->side;
+    e->early = false;                                    // behind an event: the ordinary start
+    rc = launch_early(e, finish_rows_kernel, n_want * parts, 512, 0, parts, e->logits, V, n_want, parts, scale, e->cfg.logit_softcap, to, e->d_err, c0, c1, s, segs, e->seg_best);
+    e->stream = main_stream;
+    e->early = early;
+  }
+  // joined also after a failed launch: a capture must not end with the side stream still forked
+  const cudaError_t j1 = cudaEventRecord(e->ev_join, e->side), j2 = cudaStreamWaitEvent(e->stream, e->ev_join, 0);
+  if (rc < 0) return rc;
+  CK(j1);
+  CK(j2);
+  return 0;
 }
 
 // How a block holds a row of D entries in registers: pieces of four per thread (nv of them, 1, 2 or 4; 0 = the row is not whole pieces or too long,
@@ -2104,8 +2140,7 @@ static int run_layers_post(xotb200_lm* e, const StepPlan& sp, int n_want) {
   if (e->last && n_want > 0) {
     T* hw = static_cast<T*>(e->hw);
     TRY(norm_rows(nullptr, nullptr, e->final_norm, e->final_norm_b, hw, sp.want, n_want));
-    TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    TRY(finish_logits(e, n_want));
+    TRY(head_logits<T>(e, hw, n_want));
   }
   return 0;
 }
@@ -2168,8 +2203,7 @@ static int run_layers_pre_scalar(xotb200_lm* e, const StepPlan& sp, int n_want) 
     T* hw = static_cast<T*>(e->hw);
     TRY(launch_early(e, okern, n_want, nt, (size_t)D * 4, 1, e->x, S, pend.y, pend.y2, pend.ya, pend.yb, mult, pend.mix, pend.out, nullptr, at<T>(e, e->final_norm), eps, sp.want,
                                                     nullptr, hw, D));
-    TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    TRY(finish_logits(e, n_want));
+    TRY(head_logits<T>(e, hw, n_want));
   }
   return 0;
 }
@@ -2221,8 +2255,7 @@ static int run_layers_pre_dyt(xotb200_lm* e, const StepPlan& sp, int n_want) {
   if (e->last && n_want > 0) {
     T* hw = static_cast<T*>(e->hw);
     TRY(launch_early(e, dyt_rows_kernel<T>, row_grid(e, n_want, D, nt), nt, 0, 1, e->x, sp.want, at<T>(e, e->final_norm_a), at<T>(e, e->final_norm), at<T>(e, e->final_norm_b), hw, D));
-    TRY((product<T, T, float, EPI_NONE>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    TRY(finish_logits(e, n_want));
+    TRY(head_logits<T>(e, hw, n_want));
   }
   return 0;
 }
@@ -2273,8 +2306,7 @@ static int run_layers_parallel(xotb200_lm* e, const StepPlan& sp, int n_want) {
   if (e->last && n_want > 0) {
     T* hw = static_cast<T*>(e->hw);
     TRY(pass(false, at<T>(e, e->final_norm), hw, sp.want, n_want));
-    TRY((product<T, T, float, EPI_NONE>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    TRY(finish_logits(e, n_want));
+    TRY(head_logits<T>(e, hw, n_want));
   }
   return 0;
 }
@@ -2342,8 +2374,7 @@ static int run_layers(xotb200_lm* e, const StepPlan& sp, int n_want) {
     // the last sublayer is closed by the norm in front of the head, for the rows that go through it: nobody reads the stream behind them
     T* hw = static_cast<T*>(e->hw);
     TRY(norm_rows(pend_y, pend_w, at<T>(e, e->final_norm), hw, sp.want, n_want));
-    TRY((product<T, T, float, 0>(e, hw, D, 0, at<T>(e, e->head), D, 1, 0, e->logits, e->cfg.vocab, 0, n_want, e->cfg.vocab, D, 1)));
-    TRY(finish_logits(e, n_want));
+    TRY(head_logits<T>(e, hw, n_want));
   }
   return 0;
 }
@@ -2549,7 +2580,7 @@ int xotb200_lm_destroy(xotb200_lm* e) {
     if (L.rel_bucket) cudaFree(L.rel_bucket);
     if (L.rel_tab) cudaFree(L.rel_tab);
   }
-  void* ptrs[] = {e->pair_ws, e->vfirst, e->oh2, e->y2, e->h0, e->gdec, e->ginw, e->gfloor, e->gnq, e->pos_freqs, e->dist_tab, e->moe_xg, e->moe_yg, e->moe_plan, e->dkk, e->drr, e->cvb, e->moe_ids, e->moe_wts, e->mact, e->du, e->dau, e->part, e->dch, e->q16, e->cbuf, e->knx, e->vxx, e->blob, e->d_stage, e->x, e->y, e->proj, e->qraw, e->qfull, e->wlog, e->oraw, e->logits, e->h, e->cqn, e->qn, e->olat, e->oh, e->act,
+  void* ptrs[] = {e->pair_ws, e->seg_best, e->vfirst, e->oh2, e->y2, e->h0, e->gdec, e->ginw, e->gfloor, e->gnq, e->pos_freqs, e->dist_tab, e->moe_xg, e->moe_yg, e->moe_plan, e->dkk, e->drr, e->cvb, e->moe_ids, e->moe_wts, e->mact, e->du, e->dau, e->part, e->dch, e->q16, e->cbuf, e->knx, e->vxx, e->blob, e->d_stage, e->x, e->y, e->proj, e->qraw, e->qfull, e->wlog, e->oraw, e->logits, e->h, e->cqn, e->qn, e->olat, e->oh, e->act,
                   e->th, e->hw, e->trace_buf};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -2792,6 +2823,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
     for (long m = 0; m < M; ++m) REQUIRE(tokens[m] >= 0 && tokens[m] < V, "token id %d outside the vocabulary of %d", tokens[m], V);
   TRY(ensure_scratch(e, (int)M, n_want));
   e->early = M <= LST_MAX_ROWS;
+  e->logits_out = logits_f32 != nullptr;
   TRY(refresh_tables(e));
   if (e->table_stale) {
     CK(cudaMemcpy(e->d_table, e->h_table, (size_t)e->max_requests * e->pages_per_slot * 4, cudaMemcpyHostToDevice));

@@ -27,8 +27,10 @@ __global__ void stage_in_kernel(const int4* __restrict__ src, int4* __restrict__
 // finishes the logits of every row — l <- l * scale, then l <- cap * tanh(l / cap) when cap > 0 —, takes the lowest-index argmax of the row
 // (greedy sampling on the device) and sends both where the caller wants them, the step's error word behind the rows' results.  A cluster of `parts` blocks shares a row
 // (grid n_want * parts, along x: as many rows as a step may want): its reads and its writes over PCIe are in flight together (one row of 32000: 5.6 us by one block without the copy out).
+// A launch has columns c0 .. c1 - 1, segment `seg` of `segs`: the segments follow one another on one stream, each leaves its best entry of a row in `seg_best` [segs][n_want] and the last
+// one has the row's.
 __global__ void __launch_bounds__(512) finish_rows_kernel(float* logits, int V, int n_want, int parts, float scale, float cap, const StepOut* __restrict__ to,
-                                                          const int* __restrict__ err) {
+                                                          const int* __restrict__ err, int c0, int c1, int seg, int segs, float2* __restrict__ seg_best) {
   pdl_enter();
   __shared__ float bv[32];
   __shared__ int bi[32];
@@ -43,7 +45,7 @@ __global__ void __launch_bounds__(512) finish_rows_kernel(float* logits, int V, 
   auto take = [&](float v, int i) { if (v > best || (v == best && i < idx)) { best = v; idx = i; } };
   const bool change = scale != 1.0f || cap > 0.f, write = w && (change || w != r);
   constexpr int NV = 4;                                        // 16-byte loads in flight per thread
-  const int per = ((V + 3) / 4 + parts - 1) / parts * 4, v0 = min(V, rank * per), v1 = min(V, v0 + per);   // this block's stretch, from a piece of four on
+  const int per = ((c1 - c0 + 3) / 4 + parts - 1) / parts * 4, v0 = min(c1, c0 + rank * per), v1 = min(c1, v0 + per);   // this block's stretch, from a piece of four on (c0 is one)
   int done = v0;
   if (((reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(w)) & 15) == 0) {
     done = v0 + ((v1 - v0) & ~3);
@@ -96,6 +98,14 @@ __global__ void __launch_bounds__(512) finish_rows_kernel(float* logits, int V, 
     xb::cluster_sync_all();                                    // nobody's shared memory goes away while it is read
   }
   if (rank == 0 && threadIdx.x == 0) {
+    if (segs > 1) {
+      if (seg + 1 < segs) { seg_best[(size_t)seg * n_want + m] = make_float2(best, __int_as_float(idx)); return; }
+      for (int u = 0; u < seg; ++u) {
+        const float2 o = __ldcg(seg_best + (size_t)u * n_want + m);
+        const int oi = __float_as_int(o.y);
+        if (o.x > best || (o.x == best && oi < idx)) { best = o.x; idx = oi; }
+      }
+    }
     so.tail[m] = idx;
     if (m == 0) so.tail[n_want] = *err;
   }
