@@ -1,0 +1,87 @@
+"""What the decode kernel takes and gives without a copy: the token by value, hidden states in the caller's device buffers, logits in page-locked blocks — against the staged
+way (buffers off a 16-byte boundary, ordinary memory, several positions at once), which computes the same bits."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from xotorch_b200.synth import PRESETS, hf_config, synth_prompt
+
+
+def shard(name, lo, hi, n):
+  from xotorch_b200.native import NativeShard
+  e = NativeShard(hf_config(PRESETS[name]), device=0)
+  e.set_shard(lo, hi)
+  e.init_synthetic(1234)
+  e.set_prefill_mode(1)                                # every call through the decode kernel
+  e.begin_request(n)
+  return e
+
+
+@pytest.mark.parametrize("name", ["tiny-llama-hd64", "tiny-llama-hd128-f16"])
+@pytest.mark.parametrize("n", [1, 3])
+def test_hidden_states_in_place(name, n):
+  import torch
+  shape = PRESETS[name]
+  dt = torch.float16 if name.endswith("f16") else torch.bfloat16
+  x = torch.randn(n, shape.dim, generator=torch.Generator().manual_seed(1)).to(dt).cuda()
+  outs = []
+  for lead_in, lead_out in ((0, 0), (1, 0), (0, 3), (8, 16)):      # entries of 2 bytes in front of the rows
+    e = shard(name, 1, 2, 16)
+    room, out = torch.zeros(lead_in + x.numel(), dtype=dt, device="cuda"), torch.zeros(lead_out + x.numel(), dtype=dt, device="cuda")
+    room[lead_in:] = x.flatten()
+    torch.cuda.synchronize()
+    for pos in (0, n):                                 # twice: the two barrier counters take turns
+      e.forward_device(None, room[lead_in:].data_ptr(), n, pos, out[lead_out:].data_ptr())
+    outs.append(out[lead_out:].clone())
+    e.close()
+  assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+@pytest.mark.parametrize("shift", [0, 8, -8])
+def test_output_over_the_input(shift):
+  import torch
+  name, n = "tiny-llama-hd64", 4
+  shape = PRESETS[name]
+  x = torch.randn(n, shape.dim, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).cuda()
+  own = torch.empty_like(x)
+  e = shard(name, 1, 2, 16)
+  e.forward_device(None, x.data_ptr(), n, 0, own.data_ptr())
+  room = torch.zeros(x.numel() + 16, dtype=torch.bfloat16, device="cuda")
+  room[8:8 + x.numel()] = x.flatten()
+  torch.cuda.synchronize()
+  e.forward_device(None, room[8:].data_ptr(), n, 0, room[8 + shift:].data_ptr())
+  assert torch.equal(room[8 + shift:8 + shift + x.numel()].reshape(x.shape), own)
+  e.close()
+
+
+@pytest.mark.parametrize("name", ["tiny-llama-hd64", "tiny-llama-hd128"])
+def test_logits_in_page_locked_and_ordinary_memory(name):
+  shape = PRESETS[name]
+  toks = synth_prompt(shape.vocab, 6)
+  e = shard(name, 0, shape.n_layers - 1, 16)
+  lib, got = e.lib, {}
+  for kind in ("page-locked", "ordinary", "results"):
+    rows = []
+    for pos in range(6):
+      t = np.ascontiguousarray(toks[:, pos:pos + 1], dtype=np.int32)
+      if kind == "results":
+        rows.append(e.forward(t, pos)[0].copy())
+        continue
+      if kind == "page-locked":
+        p = C.c_void_p()
+        assert lib.xotb200_host_alloc(0, shape.vocab * 4, C.byref(p)) == 0
+        out = np.ctypeslib.as_array((C.c_float * shape.vocab).from_address(p.value))
+      else:
+        out = np.empty(shape.vocab, dtype=np.float32)
+      assert lib.xotb200_forward(e.h, t.ctypes.data_as(C.c_void_p), None, 1, pos, out.ctypes.data_as(C.c_void_p)) == 0
+      rows.append(out.copy())
+      if kind == "page-locked":
+        lib.xotb200_host_free(0, p)
+    got[kind] = np.stack(rows)
+  assert np.array_equal(got["page-locked"], got["ordinary"]) and np.array_equal(got["results"], got["ordinary"])
+  whole = e.forward(np.ascontiguousarray(toks, dtype=np.int32), 0)[0]      # six positions in one launch: staged tokens
+  assert np.array_equal(whole, got["ordinary"][-1])
+  e.close()

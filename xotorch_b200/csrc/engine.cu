@@ -129,6 +129,7 @@ struct ActMaps {
   CUtensorMap full, r64, r32, r16;
 };
 
+constexpr int BAR_STRIDE = 64;                         // counters in different lines
 struct xotb200_engine {
   xotb200_model_cfg cfg;
   int device = 0, sm_count = 148;
@@ -186,7 +187,8 @@ struct xotb200_engine {
   bool have_result = false;
   cudaStream_t stream = nullptr;
   LayerDev* d_layers = nullptr;
-  unsigned int* bar_counter = nullptr;
+  unsigned int* bar_counter = nullptr;                 // two counters, BAR_STRIDE apart: a launch counts on one and clears the other
+  unsigned int bar_turn = 0;
   void* mega = nullptr;
   size_t mega_smem = 0;
   int mega_xbuf = 0, mega_grid = 0, mega_nstage = 0;
@@ -322,7 +324,14 @@ static size_t dbg_cap(const xotb200_engine* e) { return (size_t)(4 * e->cfg.n_la
 
 // Launch the persistent shard-step kernel for n_steps steps.  mode 0 = ring (inbox in, next inbox out),
 // mode 1 = direct (staging buffers).
-static int launch_mega(xotb200_engine* e, int mode, int n_steps, int step0, int pos0, cudaStream_t st) {
+// where a direct launch reads and writes other memory than the staging buffers
+struct DirectIo {
+  const void* in = nullptr;        // hidden state [n, D] on the device
+  void* out = nullptr;             // the same of a shard that is not the last
+  int tok1 = -1;                   // the one token of a first shard's call
+  float* logits_host = nullptr;    // page-locked logits (a block of this library: its bounds are known)
+};
+static int launch_mega(xotb200_engine* e, int mode, int n_steps, int step0, int pos0, cudaStream_t st, const DirectIo& io = DirectIo{}) {
   if (int rc = prepare_mega(e)) return rc;
   const xotb200_model_cfg& c = e->cfg;
   MegaArgs a{};
@@ -335,7 +344,8 @@ static int launch_mega(xotb200_engine* e, int mode, int n_steps, int step0, int 
   a.part_ml = e->part_ml; a.part_acc = e->part_acc; a.tickets = e->tickets;
   a.cta_best_val = e->cta_best_val; a.cta_best_idx = e->cta_best_idx; a.nsplit = e->nsplit; a.nsplit_min = e->nsplit_min;
   a.ctl = e->ctl; a.inbox = e->inbox; a.next_inbox = e->next_inbox; a.tokens_log = e->tokens_log;
-  a.t_in = e->t_in; a.t_out = e->t_out; a.bar_counter = e->bar_counter;
+  a.t_in = e->t_in; a.t_out = e->t_out;
+  a.bar_counter = e->bar_counter + BAR_STRIDE * (e->bar_turn & 1); a.bar_next = e->bar_counter + BAR_STRIDE * ((e->bar_turn + 1) & 1);
   a.mode = mode; a.n_steps = n_steps; a.step0 = step0; a.pos0 = pos0;
   const int nact = (mode == 0 && e->n_active > 0) ? e->n_active : e->nreq;
   a.nreq = nact; a.nslots = nact + 1; a.req0 = e->cur_req; a.kv_req_stride = e->kv_req_stride;
@@ -343,7 +353,8 @@ static int launch_mega(xotb200_engine* e, int mode, int n_steps, int step0, int 
   a.pos_tab = (mode == 0 && e->n_active > 0) ? e->d_pos_tab : nullptr;
   a.tok_host = (mode == 0 && e->last) ? e->tok_host_dev : nullptr;
   a.tok_count_host = e->tok_count_dev;
-  a.src_tokens = e->stage_tokens; a.src_hidden = e->stage_in; a.out_hidden = e->stage_out;
+  a.src_tokens = io.tok1 >= 0 ? nullptr : e->stage_tokens; a.tok1 = io.tok1; a.logits_host = io.logits_host;
+  a.src_hidden = io.in ? static_cast<const bf16*>(io.in) : e->stage_in; a.out_hidden = io.out ? static_cast<bf16*>(io.out) : e->stage_out;
   a.hop_in = mode == 1 ? e->hop_in : 0; a.hop_out = mode == 1 ? e->hop_out : 0;
   a.hop_seq_in = e->hop_seq_in; a.hop_seq_out = e->hop_seq_out;
   a.xbuf_bytes = e->mega_xbuf;
@@ -356,9 +367,9 @@ static int launch_mega(xotb200_engine* e, int mode, int n_steps, int step0, int 
   a.route_log = e->route_log;
   a.dbg = (mode == 0 && e->dbg_step >= 0) ? e->dbg : nullptr; a.dbg_step = e->dbg_step; a.dbg_cta = e->dbg_cta;
   a.dbg_all = a.dbg ? e->dbg + dbg_cap(e) : nullptr;
-  CK(cudaMemsetAsync(e->bar_counter, 0, 4, st));
   void* params[] = {&a};
   CK(cudaLaunchCooperativeKernel((const void*)e->mega, dim3(e->mega_grid), dim3(MK_THREADS), params, e->mega_smem, st));
+  e->bar_turn++;                   // a launch that was refused has cleared nothing
   e->launches++;
   return 0;
 }
@@ -993,16 +1004,33 @@ extern "C" {
 const char* xotb200_last_error(void) { return g_err; }
 const char* xotb200_version(void) { return "xotb200 0.1.0 sm_100a"; }
 
+// the page-locked blocks handed out, address -> bytes: what a kernel may write to (a store past registered memory would fault)
+static std::mutex g_blocks_lock;
+static std::map<uintptr_t, size_t> g_blocks;
+static bool in_host_block(const void* p, size_t bytes) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  std::lock_guard<std::mutex> lock(g_blocks_lock);
+  auto it = g_blocks.upper_bound(a);
+  if (it == g_blocks.begin()) return false;
+  --it;
+  return a + bytes <= it->first + it->second;
+}
 int xotb200_host_alloc(int device, int64_t bytes, void** out) {
   REQUIRE(bytes > 0 && out, "bad argument");
   cudaError_t r = cudaSetDevice(device);   // a thread that has not chosen one yet would start a context on device 0
   if (r == cudaSuccess) r = cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable);
   if (r != cudaSuccess) cudaGetLastError();   // the caller goes on without: not an error of the next launch
   CK(r);
+  std::lock_guard<std::mutex> lock(g_blocks_lock);
+  g_blocks[reinterpret_cast<uintptr_t>(*out)] = (size_t)bytes;
   return 0;
 }
 int xotb200_host_free(int device, void* p) {
   CK(cudaSetDevice(device));
+  {
+    std::lock_guard<std::mutex> lock(g_blocks_lock);
+    g_blocks.erase(reinterpret_cast<uintptr_t>(p));
+  }
   if (p) CK(cudaFreeHost(p));
   return 0;
 }
@@ -1047,7 +1075,8 @@ int xotb200_create(const xotb200_model_cfg* cfg, int device, xotb200_engine** ou
   MEMSET_SYNC(e, e->tickets, 0, (Hkv + 1) * 4);
   CK(cudaMalloc(&e->cta_best_val, 1024 * 4));
   CK(cudaMalloc(&e->cta_best_idx, 1024 * 4));
-  CK(cudaMalloc(&e->bar_counter, 4));
+  CK(cudaMalloc(&e->bar_counter, 2 * BAR_STRIDE * 4));
+  CK(cudaMemset(e->bar_counter, 0, 2 * BAR_STRIDE * 4));
   CK(cudaMalloc(&e->ctl, sizeof(StepCtl)));
   MEMSET_SYNC(e, e->ctl, 0, sizeof(StepCtl));
   CK(cudaHostAlloc(&e->gemm_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
@@ -1483,6 +1512,27 @@ static bool runs_as_gemms(xotb200_engine* e, int n_tokens, int pos0) {
   return false;
 }
 
+// What the decode kernel can take from the caller and give back without a copy (the copies and the clearing of a counter
+// cost some 9 us around a kernel of 179: one position of two 8B layers 200 -> 191 us, of a 1B-shaped model of two layers with its logits 209 -> 189):
+// the one token by value; hidden states on the device in place, where the kernel's 16-byte reads allow it and no position's output lies on a later position's input; logits
+// into a page-locked block of this library, stored while the rest of the head is still computed (512 KB take 12 us by DMA).
+static DirectIo direct_io(const xotb200_engine* e, const int32_t* tokens, int n_tokens, const void* in, void* out, float* logits) {
+  DirectIo io;
+  if (tokens && n_tokens == 1) io.tok1 = tokens[0];
+  const size_t bytes = (size_t)n_tokens * e->cfg.dim * 2;
+  const char *ci = static_cast<const char*>(in), *co = static_cast<const char*>(out);
+  if (in || (out && !e->last)) {
+    const bool shifted = in && out && !e->last && ci != co && ci < co + bytes && co < ci + bytes;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(in) | (e->last ? 0 : reinterpret_cast<uintptr_t>(out));
+    if (!shifted && at % 16 == 0) {
+      io.in = in;
+      io.out = e->last ? nullptr : out;
+    }
+  }
+  if (e->last && logits && in_host_block(logits, (size_t)e->cfg.vocab * 4) && reinterpret_cast<uintptr_t>(logits) % 8 == 0) io.logits_host = logits;
+  return io;
+}
+
 int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidden_f32, int n_tokens, int pos0,
                     float* out_f32) {
   REQUIRE(e && e->start >= 0, "no shard set");
@@ -1498,24 +1548,25 @@ int xotb200_forward(xotb200_engine* e, const int32_t* tokens, const float* hidde
   if (int rc = ensure_staging(e, n_tokens)) return rc;
   const size_t D = e->cfg.dim;
   cudaStream_t st = e->stream;
+  const bool use_tc = runs_as_gemms(e, n_tokens, pos0);
+  const DirectIo io = use_tc ? DirectIo{} : direct_io(e, tokens, n_tokens, nullptr, nullptr, out_f32);
   if (tokens) {
     for (int i = 0; i < n_tokens; ++i)
       REQUIRE(tokens[i] >= 0 && tokens[i] < e->cfg.vocab, "token id %d out of range", tokens[i]);
-    CK(cudaMemcpyAsync(e->stage_tokens, tokens, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, st));
+    if (io.tok1 < 0) CK(cudaMemcpyAsync(e->stage_tokens, tokens, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, st));
   } else {
     CK(cudaMemcpyAsync(e->stage_f32, hidden_f32, (size_t)n_tokens * D * 4, cudaMemcpyHostToDevice, st));
     DT_LAUNCH(e, (f32_to_bf16_kernel<<<256, 256, 0, st>>>(e->stage_f32, e->stage_in, (size_t)n_tokens * D)));
     CK(cudaGetLastError());
     e->launches++;
   }
-  const bool use_tc = runs_as_gemms(e, n_tokens, pos0);
   if (use_tc) {
     if (int rc = prefill_tc(e, n_tokens, pos0, st)) return rc;     // GEMM-shaped: 5th-gen tensor cores
   } else {
-    if (int rc = launch_mega(e, 1, n_tokens, 0, pos0, st)) return rc;   // one launch walks all n_tokens positions
+    if (int rc = launch_mega(e, 1, n_tokens, 0, pos0, st, io)) return rc;   // one launch walks all n_tokens positions
   }
   if (e->last) {
-    CK(cudaMemcpyAsync(out_f32, e->logits, (size_t)e->cfg.vocab * 4, cudaMemcpyDeviceToHost, st));
+    if (!io.logits_host) CK(cudaMemcpyAsync(out_f32, e->logits, (size_t)e->cfg.vocab * 4, cudaMemcpyDeviceToHost, st));
   } else {
     DT_LAUNCH(e, (bf16_to_f32_kernel<<<256, 256, 0, st>>>(e->stage_out, e->stage_f32, (size_t)n_tokens * D)));
     CK(cudaGetLastError());
@@ -1548,12 +1599,13 @@ int xotb200_forward_device(xotb200_engine* e, const int32_t* tokens, const void*
   if (int rc = ensure_staging(e, n_tokens)) return rc;
   const size_t D = e->cfg.dim;
   cudaStream_t st = e->stream;
+  const bool use_tc = runs_as_gemms(e, n_tokens, pos0);
+  const DirectIo io = use_tc ? DirectIo{} : direct_io(e, tokens, n_tokens, hidden_dev, out_hidden_dev, logits_f32);
   if (tokens) {
     for (int i = 0; i < n_tokens; ++i)
       REQUIRE(tokens[i] >= 0 && tokens[i] < e->cfg.vocab, "token id %d out of range", tokens[i]);
-    CK(cudaMemcpyAsync(e->stage_tokens, tokens, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, st));
+    if (io.tok1 < 0) CK(cudaMemcpyAsync(e->stage_tokens, tokens, (size_t)n_tokens * 4, cudaMemcpyHostToDevice, st));
   }
-  const bool use_tc = runs_as_gemms(e, n_tokens, pos0);
   if (use_tc) {   // the caller's buffers are read and written in place, no copy through the staging buffers
     const char *in = static_cast<const char*>(hidden_dev), *out = static_cast<const char*>(e->last ? nullptr : out_hidden_dev);
     const size_t bytes = (size_t)n_tokens * D * 2;
@@ -1563,11 +1615,14 @@ int xotb200_forward_device(xotb200_engine* e, const int32_t* tokens, const void*
     }
     if (int rc = prefill_tc(e, n_tokens, pos0, st, in, const_cast<char*>(out))) return rc;
   } else {
-    if (!tokens) CK(cudaMemcpyAsync(e->stage_in, hidden_dev, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
-    if (int rc = launch_mega(e, 1, n_tokens, 0, pos0, st)) return rc;
+    if (!tokens && !io.in) CK(cudaMemcpyAsync(e->stage_in, hidden_dev, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
+    if (int rc = launch_mega(e, 1, n_tokens, 0, pos0, st, io)) return rc;
   }
-  if (e->last) CK(cudaMemcpyAsync(logits_f32, e->logits, (size_t)e->cfg.vocab * 4, cudaMemcpyDeviceToHost, st));
-  else if (!use_tc) CK(cudaMemcpyAsync(out_hidden_dev, e->stage_out, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
+  if (e->last) {
+    if (!io.logits_host) CK(cudaMemcpyAsync(logits_f32, e->logits, (size_t)e->cfg.vocab * 4, cudaMemcpyDeviceToHost, st));
+  } else if (!use_tc && !io.out) {
+    CK(cudaMemcpyAsync(out_hidden_dev, e->stage_out, (size_t)n_tokens * D * 2, cudaMemcpyDeviceToDevice, st));
+  }
   CK(cudaStreamSynchronize(st));
   if (use_tc)
     if (int rc = check_gemm_error(e)) return rc;

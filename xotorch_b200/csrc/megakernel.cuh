@@ -71,7 +71,8 @@ struct MegaArgs {
   InboxHdr *inbox, *next_inbox;
   int* tokens_log;
   unsigned long long *t_in, *t_out;
-  unsigned int* bar_counter; // grid barrier counter (host zeroes it before every launch)
+  unsigned int* bar_counter; // grid barrier counter, 0 when the launch begins
+  unsigned int* bar_next;    // the next launch's: zeroed by this one (two take turns, so that no copy engine has to clear one in front of a launch)
   int mode;                  // 0 ring, 1 direct
   // direct mode, one step (the API hop, xotb200_forward_hop): the hidden state arrives in / leaves through the inbox's API slots
   // — the same fused peer store + release/acquire flag as ring mode, but one engine call per shard per token
@@ -86,7 +87,9 @@ struct MegaArgs {
   int* tok_host;             // last shard, optional: host-mapped token log [MAX_RING_STEPS] + counter, readable while the kernel runs
   unsigned int* tok_count_host;
   size_t kv_req_stride;      // elements between the KV caches of consecutive requests
-  const int* src_tokens;     // direct, first shard: [n_steps]
+  const int* src_tokens;     // direct, first shard: [n_steps]; NULL: one position, token tok1
+  int tok1;
+  float* logits_host;        // direct, last shard: the caller's page-locked array, written as the logits are made; NULL: they stay on the device
   const bf16* src_hidden;    // direct, other shards: [n_steps, D]
   bf16* out_hidden;          // direct, non-last shard: [n_steps, D]
   // Mixtral-style sparse MoE MLP (E == 0: dense).  Every CTA evaluates the router redundantly from the normalised x it
