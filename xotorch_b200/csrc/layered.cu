@@ -2329,11 +2329,12 @@ static int run_layers(xotb200_lm* e, const StepPlan& sp, int n_want) {
   T* h = static_cast<T*>(e->h);
   const float* pend_y = nullptr;
   const T* pend_w = nullptr;
-  const RowShape rs = (D / G) % 128 == 0 ? row_shape(D) : RowShape{0, 0};   // parts of whole 128-entry pieces: the row stays in registers
+  const RowShape rs = (D / G) % 128 == 0 && G <= 65535 ? row_shape(D / G) : RowShape{0, 0};   // parts of whole 128-entry pieces: the row stays in registers
   auto norm_rows = [&](const float* y, const T* w_post, const T* w_pre, T* out, const int* rows, int n) -> int {
     if (rs.nv) {
+      // a block to a part (the parts know nothing of one another): fewer warps at its barriers (1024 rows of 4096 in 4 parts 18.5 -> 14.8 us a launch; a step of 16 such rows 5 us less)
       auto vk = rs.nv == 1 ? residual_groupnorm_vec_kernel<T, 1> : rs.nv == 2 ? residual_groupnorm_vec_kernel<T, 2> : residual_groupnorm_vec_kernel<T, 4>;
-      TRY(launch_early(e, vk, n, rs.threads, 0, 1, e->x, y, w_post, w_pre, out, rows, D, G, eps));
+      TRY(launch_early(e, vk, dim3(n, G), rs.threads, 0, 1, e->x, y, w_post, w_pre, out, rows, D / G, 1, eps, D));
     } else {
       TRY(launch_early(e, residual_groupnorm_kernel<T>, n, norm_threads(D, G), 0, 1, e->x, y, w_post, w_pre, out, rows, D, G, eps));
     }

@@ -274,13 +274,16 @@ __global__ void residual_groupnorm_kernel(float* __restrict__ x, const float* __
 // A single row is one chain of latencies (weights, row, two block-wide sums): 1 row of 1024 entries 6.2 us with the kernel above.
 template <typename T, int NV>
 __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const T* __restrict__ w_post, const T* __restrict__ w_pre,
-                                              T* __restrict__ h, const int* __restrict__ src_rows, int D, int G, float eps) {
+                                              T* __restrict__ h, const int* __restrict__ src_rows, int D, int G, float eps, int ld) {
   __shared__ float red[2][32 * NV];
   const size_t m = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, Dg = D / G, ppg = Dg / 128;   // pieces of a part
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
   float4 xv[NV], yv[NV], wo[NV], wp[NV];
   int d[NV];
+  x += (size_t)blockIdx.y * D;                                   // this block's stretch of the row, D entries in G parts; rows are ld apart
+  if (y) { y += (size_t)blockIdx.y * D; w_post += (size_t)blockIdx.y * D; }
+  if (h) { h += (size_t)blockIdx.y * D; w_pre += (size_t)blockIdx.y * D; }
   pdl_launch_dependents();
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
@@ -294,8 +297,8 @@ __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
     const bool on = d[v] < D;
-    xv[v] = on ? ld4f(x + xm * D + d[v]) : zero;
-    yv[v] = on && y ? ld4f(y + xm * D + d[v]) : zero;
+    xv[v] = on ? ld4f(x + xm * ld + d[v]) : zero;
+    yv[v] = on && y ? ld4f(y + xm * ld + d[v]) : zero;
   }
   // 1 / rms of the part that piece v of this warp lies in
   auto part_scale = [&](float* r, int v) {
@@ -316,7 +319,7 @@ __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float
       if (v * (int)blockDim.x * 4 + warp * 128 >= D) continue;  // warp-uniform: the row's pieces are whole warps
       const float r = part_scale(red[0], v);
       xv[v].x += yv[v].x * r * wo[v].x; xv[v].y += yv[v].y * r * wo[v].y; xv[v].z += yv[v].z * r * wo[v].z; xv[v].w += yv[v].w * r * wo[v].w;
-      if (!src_rows) st4f(x + xm * D + d[v], xv[v]);            // gathered rows may repeat
+      if (!src_rows) st4f(x + xm * ld + d[v], xv[v]);            // gathered rows may repeat
     }
   }
   if (!h) return;
@@ -330,7 +333,7 @@ __global__ void residual_groupnorm_vec_kernel(float* __restrict__ x, const float
   for (int v = 0; v < NV; ++v) {
     if (v * (int)blockDim.x * 4 + warp * 128 >= D) continue;
     const float r = part_scale(red[1], v);
-    st4f(h + m * D + d[v], make_float4(xv[v].x * r * wp[v].x, xv[v].y * r * wp[v].y, xv[v].z * r * wp[v].z, xv[v].w * r * wp[v].w));
+    st4f(h + m * ld + d[v], make_float4(xv[v].x * r * wp[v].x, xv[v].y * r * wp[v].y, xv[v].z * r * wp[v].z, xv[v].w * r * wp[v].w));
   }
 }
 
