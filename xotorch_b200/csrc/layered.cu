@@ -1007,6 +1007,7 @@ static void drop_graphs(xotb200_lm* e) {
 }
 
 constexpr int HEAD_SEGMENTS = 4;                       // head_logits
+static bool experts_in_pairs(size_t pairs, int experts) { return pairs >= (size_t)experts * 2 * LTC_M; }
 static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
   const int D = e->cfg.width;
   if (M > e->m_cap) {
@@ -1040,7 +1041,8 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
       TRY(regrow(e->moe_ids, m * e->max_top * 4));
       TRY(regrow(e->moe_wts, m * e->max_top * 4));
       // the grouped form pads every expert's run to whole 128-row tiles
-      const size_t tiles = (m * e->max_top + LTC_M - 1) / LTC_M + e->max_experts, pairs_pad = tiles * LTC_M;
+      const size_t tiles = (m * e->max_top + LTC_M - 1) / LTC_M + e->max_experts;
+      const size_t pairs_pad = std::max(tiles * LTC_M, experts_in_pairs(m * e->max_top, 1) ? ((m * e->max_top + 2 * LTC_M - 1) / (2 * LTC_M) + e->max_experts) * 2 * LTC_M : 0);
       TRY(regrow(e->mact, pairs_pad * e->max_eff * z));
       if (z == 2) {
         TRY(regrow(e->moe_xg, pairs_pad * D * 2));
@@ -1873,13 +1875,17 @@ static int mamba2_layer(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
 // 1 = launched, 0 = the operands cannot be described to TMA
 template <int EPI, typename TC>
 static int grouped_product(xotb200_lm* e, const bf16* A, long lda, const bf16* B, long ldb, long b_batch, int n_batch, TC* C, long ldc, int M, int m_pad, int N,
-                           int K, const int* tile_batch, const EpiArgs& epi = EpiArgs{}) {
+                           int K, const int* tile_batch, int tile_rows, const EpiArgs& epi = EpiArgs{}) {
   if (M <= LST_EXPERT_ROWS)
     return product_stream<TC, EPI>(e, A, lda, 0, B, ldb, b_batch, n_batch, C, ldc, 0, M, N, K, m_pad / stream_tile_rows(M), epi, tile_batch);
   const int nt = N > 64 ? 128 : 64;
   CUtensorMap ma, mb;
   if (!make_map3(&ma, A, m_pad, K, lda, 0, 1, LTC_M) || !make_map3(&mb, B, N, K, ldb, b_batch, n_batch, nt)) return 0;
   LtcArgs a{m_pad, N, K, C, ldc, 0, e->d_err, epi, tile_batch, 1};
+  if (tile_rows == 2 * LTC_M) {
+    TRY((launch_pair<EPI, TC>(e, ma, mb, a)));
+    return 1;
+  }
   if (nt == 128) TRY((launch_ltc<128, EPI, TC>(e, ma, mb, a, 1)));
   else TRY((launch_ltc<64, EPI, TC>(e, ma, mb, a, 1)));
   return 1;
@@ -1934,8 +1940,9 @@ static int feed_forward(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
     if constexpr (std::is_same<T, bf16>::value) {
       if (grouped_ok) {
         // few rows: an expert has at most M of them (a row picks an expert once), one row tile each, and the products stream the chosen experts
-        const int tile_rows = M <= LST_EXPERT_ROWS ? stream_tile_rows(M) : LTC_M;
-        const int pairs = M * top, tiles = M <= LST_EXPERT_ROWS ? std::min(E, pairs) : cdiv(pairs, LTC_M) + E, m_pad = tiles * tile_rows;
+        // many: 256-row tiles of CTA pairs where an expert has that many rows on average (3500 rows, 4 of 16 experts of 4096 x 2048: gate and up 277 -> 224 us), else 128-row tiles
+        const int tile_rows = M <= LST_EXPERT_ROWS ? stream_tile_rows(M) : experts_in_pairs(M * top, E) && D >= 512 && F >= 512 ? 2 * LTC_M : LTC_M;
+        const int pairs = M * top, tiles = M <= LST_EXPERT_ROWS ? std::min(E, pairs) : cdiv(pairs, tile_rows) + E, m_pad = tiles * tile_rows;
         REQUIRE(tiles <= e->moe_tiles_cap, "internal: the expert tile list was not sized for this step");
         int *counts = e->moe_plan, *starts = counts + e->max_experts, *cursor = starts + e->max_experts + 1, *place = cursor + e->max_experts,
             *tile_expert = place + (size_t)e->m_cap * e->max_top;
@@ -1949,11 +1956,11 @@ static int feed_forward(xotb200_lm* e, LmLayer& L, const StepPlan& sp, float* yo
         }
         bf16* ma = static_cast<bf16*>(e->mact);
         int r = s.expert_act == XOTB200_LM_EXPERT_CLAMPED_GLU
-                    ? grouped_product<EPI_CLAMPED_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, M, m_pad, 2 * F, D, tile_expert, glu)
-                : gated ? grouped_product<EPI_SILU_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, M, m_pad, 2 * F, D, tile_expert, glu)
-                        : grouped_product<EPI_RELU2, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)F * D, E, ma, F, M, m_pad, F, D, tile_expert);
+                    ? grouped_product<EPI_CLAMPED_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, M, m_pad, 2 * F, D, tile_expert, tile_rows, glu)
+                : gated ? grouped_product<EPI_SILU_GLU, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)2 * F * D, E, ma, F, M, m_pad, 2 * F, D, tile_expert, tile_rows, glu)
+                        : grouped_product<EPI_RELU2, bf16>(e, xg, D, at<bf16>(e, L.w_gu), D, (long)F * D, E, ma, F, M, m_pad, F, D, tile_expert, tile_rows);
         if (r < 0) return r;
-        if (r == 1) r = grouped_product<EPI_NONE, float>(e, ma, F, at<bf16>(e, L.w_edown), F, (long)D * F, E, e->moe_yg, D, M, m_pad, D, F, tile_expert);
+        if (r == 1) r = grouped_product<EPI_NONE, float>(e, ma, F, at<bf16>(e, L.w_edown), F, (long)D * F, E, e->moe_yg, D, M, m_pad, D, F, tile_expert, tile_rows);
         if (r < 0) return r;
         if (r == 1) {
           TRY(launch_early(e, moe_combine_kernel<bf16>, row_grid(e, M, D, 256), 256, 0, 1, e->moe_yg, place, e->moe_wts, top, D, shared, yout, close));
@@ -2036,8 +2043,8 @@ static int run_mixer(xotb200_lm* e, LmLayer& L, const StepPlan& sp) {
 }
 
 // hw [n_want, D] -> logits, argmax, where the caller wants them.  Results of several rows take as long over PCIe as the head's weights take from memory (16 rows of 32000: 2 MB, 40 us; 262 MB of
-// weights, 40 us), so the vocabulary is cut into segments of about 256 KB of results, four at most, and a segment is sent, on the side stream, while the next ones are computed (8 rows, width 2048: HEAD8;
-// 16 rows, width 4096: HEAD16).
+// weights, 40 us), so the vocabulary is cut into segments of about 256 KB of results, four at most, and a segment is sent, on the side stream, while the next ones are computed (a step of 8 rows, width 2048,
+// 4 us less; 16 rows, width 4096, 12 us: each segment streams its weights a little slower beside the copy).
 template <typename T>
 static int head_logits(xotb200_lm* e, const T* hw, int n_want) {
   const int D = e->cfg.width, V = e->cfg.vocab;

@@ -81,7 +81,7 @@ struct LtcEpilogue {
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       if constexpr (epi_is_glu(EPI)) {               // 8 gate values, then their 8 up values
-        f[j] = glu_f<EPI>(__uint_as_float(v[j]), __uint_as_float(v[j + 8]), a.epi);
+        f[j] = sizeof(TC) == 2 && EPI == EPI_SILU_GLU ? silu16_f(__uint_as_float(v[j])) * __uint_as_float(v[j + 8]) : glu_f<EPI>(__uint_as_float(v[j]), __uint_as_float(v[j + 8]), a.epi);
       } else {
         f[j] = __uint_as_float(v[j]);
         if (EPI == EPI_RELU2) { f[j] = fmaxf(f[j], 0.f); f[j] *= f[j]; }
@@ -327,7 +327,7 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // Here two CTAs share one 256 x 256 tile: each stages its own 128 rows of A and HALF of the B tile (32 KB per 4.2 MFLOP of its own), the
 // leader's thread issues tcgen05.mma.cta_group::2 over both CTAs' shared memory, and every CTA keeps its 128 rows of the accumulator.  Persistent: 74
 // pairs walk the tiles (row tile fastest, so that pairs running together share weight tiles in L2) with two accumulators in tensor memory (all
-// 512 columns), so the epilogue of one tile runs under the products of the next.  Plain loads, no multicast.  Every wait is bounded.
+// 512 columns), so the epilogue of one tile runs under the products of the next.  With `tile_batch` a 256-row tile names its matrix (experts).  Plain loads, no multicast.  Every wait is bounded.
 // Measured (B200, a launch, 128 x 128 tiles -> pairs): 3500 rows, width 2048: 86 -> 62 us, the 8192-wide up product with its activation 189 -> 133 us
 // (213 with four epilogue warps: they took longer than the next tile's products); 1024 rows, width 4096, all products of a pass: 1139 -> 976 us.  With rows put together
 // in shared memory (LtcStaged) and a cheap xIELU: 3500 rows, 6208 columns, K = 2048 78 -> 73 us, the 8192-wide up product 131 -> 113.
@@ -371,6 +371,8 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     unsigned it = 0;
     bool ok = true;
     for (int i = 0, t, k0, k1, slot, step; ok && walk.get(i, t, k0, k1, slot, step); ++i) {
+      const int zb = a.tile_batch ? a.tile_batch[t % mtiles] : 0;
+      if (zb < 0) continue;
       const int m0 = (t % mtiles) * 2 * LTC_M + (int)rank * LTC_M, n0 = (t / mtiles) * NT + (int)rank * (NT / 2);
       for (int kb = k0; kb < k1; ++kb, ++it) {
         const int st = it % NS;
@@ -380,7 +382,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         if (rank == 0) xb::mbar_expect_tx(&full[st], 2 * LTP_STAGE_BYTES);
         const uint32_t bar = xb::mapa_shared(xb::smem_u32(&full[st]), 0);
         xb::tma_load_3d_2sm(sa, &tmA, kb * LTC_BK, m0, 0, bar);
-        xb::tma_load_3d_2sm(sa + A_BYTES, &tmB, kb * LTC_BK, n0, 0, bar);
+        xb::tma_load_3d_2sm(sa + A_BYTES, &tmB, kb * LTC_BK, n0, zb, bar);
       }
     }
     if (rank == 0)   // the copies still in flight (there are any only after giving up) land before the pair's shared memory goes away
@@ -390,7 +392,8 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     constexpr uint32_t idesc = ltc_idesc(2 * LTC_M, NT);
     unsigned it = 0, ti = 0;
     bool ok = true;
-    for (int t, k0, k1, slot, step; ok && walk.get((int)ti, t, k0, k1, slot, step); ++ti) {
+    for (int i = 0, t, k0, k1, slot, step; ok && walk.get(i, t, k0, k1, slot, step); ++i) {
+      if (a.tile_batch && a.tile_batch[t % mtiles] < 0) continue;
       const uint32_t buf = ti & 1u, acc = tmem_base + buf * NT;
       ok = ltc_wait(&tmem_empty[buf], ((ti >> 1) & 1u) ^ 1u, a.err);     // both CTAs' epilogues have drained it
       if (!ok) break;
@@ -407,6 +410,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         xb::umma_commit_2sm(&empty[st], 3);                              // frees the stage in both CTAs
       }
       if (ok) xb::umma_commit_2sm(&tmem_full[buf], 3);
+      ++ti;
     }
   } else if (warp >= 4) {
     // ===== epilogue (both CTAs): warps q and q + 4 hold tensor-memory lanes 32q .. 32q+31 = this CTA's rows of the tile, half of the columns each
@@ -416,7 +420,8 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const LtcEpilogue<EPI, TC> ep(a);
     uint8_t* mine = staged + (warp - 4) * LTC_STAGED;
     unsigned ti = 0;
-    for (int t, k0, k1, slot, step; walk.get((int)ti, t, k0, k1, slot, step); ++ti) {
+    for (int i = 0, t, k0, k1, slot, step; walk.get(i, t, k0, k1, slot, step); ++i) {
+      if (a.tile_batch && a.tile_batch[t % mtiles] < 0) continue;
       const uint32_t buf = ti & 1u;
       const int row = (t % mtiles) * 2 * LTC_M + (int)rank * LTC_M + q * 32 + lane, n0 = (t / mtiles) * NT;
       if (!ltc_wait(&tmem_full[buf], (ti >> 1) & 1u, a.err)) break;
@@ -459,6 +464,7 @@ ltc_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       if (lane == 0) xb::mbar_arrive_cluster(leader_empty + buf * 8);
       if (part) xb::pair_flag_set(a.split, slot + front * step, rank, warp - 4);
       else if (add) xb::pair_flags_clear(a.split, slot, step, front, rank, warp - 4);
+      ++ti;
     }
   }
   __syncwarp();
