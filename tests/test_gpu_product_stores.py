@@ -1,4 +1,4 @@
-"""Products of many rows, their way out through shared memory: 128 x 128 tiles and CTA pairs, row and column remainders of a warp's 32 rows and of a 128-byte
+"""Products of many rows — 128 x 128 tiles, whole or with K cut over a cluster, and CTA pairs —, their way out through shared memory: 128 x 128 tiles and CTA pairs, row and column remainders of a warp's 32 rows and of a 128-byte
 piece of a row, leading dimensions that are no whole pieces, 32-bit and 16-bit outputs, xIELU and gated epilogues — against the float64 oracles."""
 import pytest
 
@@ -8,7 +8,8 @@ from tests import bufulorn_oracle as bo, zokuvik_oracle as zo
 from tests import bufulorn_util as bu, layered_util as lu
 
 
-@pytest.mark.parametrize("rows,ff", [(257, 40), (260, 1000), (289, 2056), (383, 136), (700, 5904), (1030, 3592)])
+# down products with K = ff: 2056 and 2120 in two shares, 4168 in four (the last shares shorter)
+@pytest.mark.parametrize("rows,ff", [(257, 40), (260, 1000), (289, 2056), (300, 2120), (390, 4168), (383, 136), (700, 5904), (1030, 3592)])
 def test_xielu_products(rows, ff):
   """700 x 5904 and 1030 x 3592 on CTA pairs; the projections have 5 * 16 + 2 * 2 * 17 = 148 columns and more"""
   cfg = bu.config([bu.attention(heads=6, kv_heads=3, dim=16, vdim=17, chunk=64, mlp=bu.dense(ff))], width=520, vocab=331, max_positions=1200)

@@ -807,13 +807,30 @@ static int launch_late(xotb200_lm* e, void (*kern)(KA...), dim3 grid, int thread
   return 0;
 }
 
+// CTAs of a cluster that share a 128-row tile by cutting K: where the tiles leave SMs with one CTA or none (two fit), and a CTA keeps 16 K blocks or more
+static int ltc_splits(const xotb200_lm* e, long tiles, int K) {
+  int s = 1;
+  while (s < 4 && tiles * s * 2 <= 2L * e->sm_count && cdiv(K, LTC_BK) >= 32 * s) s *= 2;
+  return s;
+}
 template <int NT, int EPI, typename TC>
 static int launch_ltc(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& mb, const LtcArgs& a, int batch) {
   constexpr int NS = 3;
   auto kern = ltc_gemm_kernel<NT, EPI, NS, TC>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ltc_smem_bytes(NT, NS)));
   const dim3 grid = a.cols_first ? dim3(cdiv(a.N, NT), cdiv(a.M, LTC_M), batch) : dim3(cdiv(a.M, LTC_M), cdiv(a.N, NT), batch);
-  TRY(launch_late(e, kern, grid, LTC_THREADS, ltc_smem_bytes(NT, NS), ma, mb, a));
+  const int s = a.tile_batch ? 1 : ltc_splits(e, (long)grid.x * grid.y * grid.z, a.K);
+  if (s > 1) {
+    auto cut = ltc_gemm_kernel<NT, EPI, NS, TC, true>;
+    CK(cudaFuncSetAttribute(cut, cudaFuncAttributeMaxDynamicSharedMemorySize, ltc_smem_bytes(NT, NS)));
+    const bool early = e->early;
+    e->early = false;
+    const int rc = launch_early(e, cut, dim3(grid.x * s, grid.y, grid.z), LTC_THREADS, ltc_smem_bytes(NT, NS), s, ma, mb, a);
+    e->early = early;
+    TRY(rc);
+  } else {
+    TRY(launch_late(e, kern, grid, LTC_THREADS, ltc_smem_bytes(NT, NS), ma, mb, a));
+  }
   e->tc_launches++;
   return 0;
 }

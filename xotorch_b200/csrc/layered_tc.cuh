@@ -34,6 +34,12 @@ __device__ __forceinline__ bool ltc_wait(uint64_t* bar, uint32_t parity, int* er
   return false;
 }
 
+__device__ __forceinline__ uint32_t cluster_size_x() {
+  uint32_t n;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return n;
+}
+
 struct LtcArgs {
   int M, N, K;
   void* C;          // fp32 or bf16 [*, ldc]
@@ -227,7 +233,10 @@ struct LtcStaged {
   }
 };
 
-template <int NT, int EPI, int NS, typename TC>
+// CUT: the CTAs of a cluster (1, 2 or 4 along x) have a share of K each and leave their fp32 partial tiles in the ring's memory; CTA r adds rows r * 128 / S .. of all of them through
+// distributed shared memory, in the order of K (deterministic), and finishes those.  290 rows, 4096 columns, K = 14336: 96 CTAs 89 us, 192 in
+// clusters of two 56; 2144 columns, K = 4096: 51 CTAs 29 us, 204 17.
+template <int NT, int EPI, int NS, typename TC, bool CUT = false>
 __global__ void __launch_bounds__(LTC_THREADS, 2 * ltc_smem_bytes(NT, NS) <= 226 * 1024 ? 2 : 1)
 ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const LtcArgs a) {
   pdl_wait();
@@ -241,11 +250,12 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   uint64_t* tmem_full = empty + NS;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mt = a.cols_first ? blockIdx.y : blockIdx.x, ntile = a.cols_first ? blockIdx.x : blockIdx.y;
+  const int S = CUT ? (int)cluster_size_x() : 1, split = CUT ? (int)xb::cluster_ctarank() : 0, bx = blockIdx.x / S;
+  const int mt = a.cols_first ? blockIdx.y : bx, ntile = a.cols_first ? bx : blockIdx.y;
   const int m0 = mt * LTC_M, n0 = ntile * NT, z = blockIdx.z;
-  const int nkb = (a.K + LTC_BK - 1) / LTC_BK;
+  const int all = (a.K + LTC_BK - 1) / LTC_BK, kb0 = all * split / S, nkb = all * (split + 1) / S - kb0;   // this CTA's K blocks: kb0 ..
   const int zb = a.tile_batch ? a.tile_batch[mt] : z;
-  if (zb < 0) return;                                  // an empty tile of a grouped product: the whole CTA leaves before anything is set up
+  if (zb < 0) return;                                  // an empty tile of a grouped product: the whole CTA leaves before anything is set up (never CUT)
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < NS; ++i) { xb::mbar_init(&full[i], 1); xb::mbar_init(&empty[i], 1); }
@@ -269,8 +279,8 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       if (!ok) break;
       uint8_t* sa = base + (size_t)st * STAGE;
       xb::mbar_expect_tx(&full[st], STAGE);
-      xb::tma_load_3d(sa, &tmA, kb * LTC_BK, m0, z, &full[st]);
-      xb::tma_load_3d(sa + A_BYTES, &tmB, kb * LTC_BK, n0, zb, &full[st]);
+      xb::tma_load_3d(sa, &tmA, (kb0 + kb) * LTC_BK, m0, z, &full[st]);
+      xb::tma_load_3d(sa + A_BYTES, &tmB, (kb0 + kb) * LTC_BK, n0, zb, &full[st]);
       issued = kb + 1;
     }
     if (!ok)   // gave up: let the copies still in flight land before the CTA's shared memory goes away
@@ -292,7 +302,7 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       xb::umma_commit(&empty[st]);
     }
     if (ok) xb::umma_commit(tmem_full);
-  } else if (warp >= 4) {
+  } else if (!CUT && warp >= 4) {
     // ===== epilogue: warp q reads tensor-memory lanes 32q .. 32q+31 = output rows =====
     const int q = warp - 4;
     const int row = m0 + q * 32 + lane;
@@ -317,8 +327,62 @@ ltc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
       }
     }
   }
+  if constexpr (CUT) {
+    // piece c (16 columns) of row m of the partial tile: four float4 at [c][j][m], so that a warp's accesses are whole lines
+    float4* part = reinterpret_cast<float4*>(base);
+    static_assert(NT * LTC_M * 4 + 8 * LTC_STAGED <= NS * STAGE, "the partial tile and the warps' buffers reuse the ring");
+    if (warp >= 4) {
+      const int q = warp - 4;
+      const bool there = ltc_wait(tmem_full, 0, a.err);
+      xb::tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < NT / 16; ++c) {
+        uint32_t v[16] = {};
+        if (there) xb::tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c * 16, v);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) part[(c * 4 + j) * LTC_M + q * 32 + lane] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+      }
+    }
+    __syncthreads();
+    xb::cluster_sync_all();
+    const LtcEpilogue<EPI, TC> ep(a);
+    using St = LtcStaged<EPI, TC>;
+    constexpr bool STAGED = EPI != EPI_CLOSE && St::COLS <= NT;
+    constexpr int UNIT = STAGED ? St::COLS : 16;                 // columns that a warp takes at a time
+    TC* C = static_cast<TC*>(a.C) + (size_t)z * a.c_batch;
+    uint8_t* mine = base + NT * LTC_M * 4 + warp * LTC_STAGED;
+    const int groups = LTC_M / 32 / S;                           // 32-row groups of this CTA
+    const uint32_t part_addr = xb::smem_u32(part);
+    for (int u = warp; u < groups * (NT / UNIT); u += LTC_THREADS / 32) {
+      const int r0 = (split * groups + u % groups) * 32, cu = u / groups * UNIT, row = m0 + r0 + lane;
+#pragma unroll 1
+      for (int c0 = cu; c0 < cu + UNIT; c0 += 16) {
+        float f[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = 0.f;
+        for (int p = 0; p < S; ++p)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 x = xb::ld_dsmem_f4(part_addr + (uint32_t)((c0 / 4 + j) * LTC_M + r0 + lane) * 16, p);
+            f[4 * j] += x.x; f[4 * j + 1] += x.y; f[4 * j + 2] += x.z; f[4 * j + 3] += x.w;
+          }
+        uint32_t v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(f[i]);
+        const int n = n0 + c0;
+        if constexpr (!STAGED) {
+          if (row < a.M && n < a.N) ep.store16(a, C + (size_t)row * a.ldc, row, n, v);
+        } else {
+          const int c = c0 % St::COLS, glu = epi_is_glu(EPI) ? 2 : 1;
+          St::put(mine, lane, c, ep, a, v);
+          if (c + 16 == St::COLS) St::out(mine, lane, ep, a, C, row - lane, (n - c) / glu, a.N / glu);
+        }
+      }
+    }
+  }
   xb::tc_fence_before();
   __syncthreads();
+  if (CUT) xb::cluster_sync_all();                               // nobody's shared memory goes away while a peer reads it
   if (warp == 2) xb::tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
