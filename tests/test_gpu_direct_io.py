@@ -85,3 +85,32 @@ def test_logits_in_page_locked_and_ordinary_memory(name):
   whole = e.forward(np.ascontiguousarray(toks, dtype=np.int32), 0)[0]      # six positions in one launch: staged tokens
   assert np.array_equal(whole, got["ordinary"][-1])
   e.close()
+
+
+@pytest.mark.parametrize("name", ["tiny-llama-hd64", "tiny-llama-hd128-f16"])
+@pytest.mark.parametrize("n", [2, 17, 128, 129, 300])
+def test_prompts_in_place(name, n):
+  """prompts as GEMMs: rows on and off a 16-byte boundary, into another buffer and over the input; the next position after them (a shard's last row goes on)"""
+  import torch
+  from xotorch_b200.native import NativeShard
+  shape = PRESETS[name]
+  dt = torch.float16 if name.endswith("f16") else torch.bfloat16
+  x = torch.randn(n, shape.dim, generator=torch.Generator().manual_seed(1)).to(dt).cuda()
+  outs = []
+  for lead_in, lead_out, same in ((0, 0, False), (1, 0, False), (0, 3, False), (8, 16, False), (0, 0, True), (1, 1, True)):
+    e = NativeShard(hf_config(shape), device=0)
+    e.set_shard(1, 2)
+    e.init_synthetic(1234)
+    e.set_prefill_mode(2)
+    e.begin_request(2 * n + 1)
+    room, out = torch.zeros(lead_in + x.numel(), dtype=dt, device="cuda"), torch.zeros(lead_out + x.numel(), dtype=dt, device="cuda")
+    rows = []
+    for pos in (0, n):
+      room[lead_in:] = x.flatten()
+      torch.cuda.synchronize()
+      to = room[lead_in:] if same else out[lead_out:]
+      e.forward_device(None, room[lead_in:].data_ptr(), n, pos, to.data_ptr())
+      rows.append(to.clone())
+    outs.append(torch.cat(rows))
+    e.close()
+  assert all(torch.equal(o, outs[0]) for o in outs[1:])

@@ -789,18 +789,22 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
   const int D = c.dim, F = c.ffn, Hq = c.n_heads, Hkv = c.n_kv_heads, hd = c.head_dim;
   const int qd = Hq * hd, nqkv = (Hq + 2 * Hkv) * hd, nl = e->end - e->start + 1;
   auto rmsnorm = c.dtype == XOTB200_DTYPE_F16 ? xb::fp::tc_rmsnorm_kernel : xb::bf::tc_rmsnorm_kernel;
+  // The rows come in with the first norm and go out with one launch behind the last product: copies by the copy engine cost some 10 us around five launches a layer (two 8B
+  // layers, 6 positions 220 -> 209 us, 128 287 -> 281).  Rows off a 16-byte boundary are copied.
+  const bool in_place = (reinterpret_cast<uintptr_t>(hidden_in) & 15) == 0, out_place = (reinterpret_cast<uintptr_t>(hidden_out) & 15) == 0;
   for (int m0 = 0; m0 < n_tokens; m0 += e->tc_chunk) {
     const int S = std::min(e->tc_chunk, n_tokens - m0);
     if (e->first) {
       if (int rc = launch_early(e, st, tc_gather_kernel, S, 128, 0, 1, e->stage_tokens + m0, e->embed, e->tc_x, D)) return rc;
-    } else {
+    } else if (!in_place) {
       CK(cudaMemcpyAsync(e->tc_x, hidden_in + (size_t)m0 * D, (size_t)S * D * 2, cudaMemcpyDeviceToDevice, st));
     }
     for (int li = 0; li < nl; ++li) {
       const LayerW& w = e->layers[li];
       bf16* kc = e->kv + (size_t)e->cur_req * e->kv_req_stride + ((size_t)li * 2 + 0) * Hkv * e->L * hd;
       bf16* vc = e->kv + (size_t)e->cur_req * e->kv_req_stride + ((size_t)li * 2 + 1) * Hkv * e->L * hd;
-      if (int rc = launch_early(e, st, rmsnorm, S, 256, 0, 1, e->tc_x, w.attn_norm, e->tc_xn, D, c.norm_eps)) return rc;
+      const bool from_caller = li == 0 && !e->first && in_place;
+      if (int rc = launch_early(e, st, rmsnorm, S, 256, 0, 1, from_caller ? hidden_in + (size_t)m0 * D : e->tc_x, w.attn_norm, e->tc_xn, D, c.norm_eps, from_caller ? e->tc_x : nullptr)) return rc;
       if (e->tc_fuse) {     // RoPE + KV append in the QKV GEMM's epilogue: rotated q -> tc_q, k / v -> the cache rows of this chunk
         TcGemmArgs g{S, nqkv, D, e->tk, e->tc_q, nullptr, qd, 0};
         g.kc = kc; g.vc = vc; g.rope = e->rope; g.q_rows = qd; g.kv_rows = Hkv * hd; g.hd = hd; g.L = e->L; g.pos0 = pos0 + m0;
@@ -817,7 +821,7 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
         return rc;
       TcGemmArgs o{S, D, qd, e->tk, e->tc_x, nullptr, D, 0};
       if (int rc = tc_gemm(e, e->tm_ao, 4 * li + 1, o, TCE_RESID, st)) return rc;
-      if (int rc = launch_early(e, st, rmsnorm, S, 256, 0, 1, e->tc_x, w.mlp_norm, e->tc_xn, D, c.norm_eps)) return rc;
+      if (int rc = launch_early(e, st, rmsnorm, S, 256, 0, 1, e->tc_x, w.mlp_norm, e->tc_xn, D, c.norm_eps, nullptr)) return rc;
       if (c.n_experts > 0) {
         // ---- sparse MoE MLP: router -> plan -> gather -> per-expert gate/up -> SwiGLU -> per-expert down -> combine ----
         const int E = c.n_experts, rows = e->moe_rows, max_tiles = (S + TC_M - 1) / TC_M, avg_rows = std::max(1, 2 * S / E);
@@ -859,17 +863,22 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
     if (e->last) {
       if (m0 + S == n_tokens) {   // logits of the last position only (sharded_inference_engine.py:365-368)
         const int mt_last = (S - 1) / TC_M, r0 = c.vocab % TC_M == 0 ? S - 1 : mt_last * TC_M;   // the last position, or the tile holding it
-        if (int rc = launch_early(e, st, rmsnorm, S - r0, 256, 0, 1, e->tc_x + (size_t)r0 * D, e->final_norm, e->tc_xn + (size_t)r0 * D, D, c.norm_eps)) return rc;
+        if (int rc = launch_early(e, st, rmsnorm, S - r0, 256, 0, 1, e->tc_x + (size_t)r0 * D, e->final_norm, e->tc_xn + (size_t)r0 * D, D, c.norm_eps, nullptr)) return rc;
         TcGemmArgs h{S, c.vocab, D, e->tk, nullptr, e->logits, 0, mt_last};
         if (int rc = tc_gemm(e, e->tm_xn, 4 * nl, h, TCE_HEAD_LAST, st)) return rc;
         if (int rc = launch_early(e, st, tc_argmax_kernel, 1, 1024, 0, 1, e->logits, c.vocab, e->ctl)) return rc;
       }
-    } else {
+    } else if (!out_place) {
       CK(cudaMemcpyAsync(hidden_out + (size_t)m0 * D, e->tc_x, (size_t)S * D * 2, cudaMemcpyDeviceToDevice, st));
     }
+    // the residual stream of the last position is what xotb200_post_to_next hands to the next shard
+    const bool end = m0 + S == n_tokens, rows = !e->last && out_place;
+    const int row0 = rows ? 0 : S - 1;
+    if (rows || end)
+      if (int rc = launch_early(e, st, tc_rows_out_kernel, S - row0, 128, 0, 1, reinterpret_cast<const uint4*>(e->tc_x + (size_t)row0 * D), rows ? reinterpret_cast<uint4*>(hidden_out + (size_t)m0 * D) : nullptr,
+                                end ? reinterpret_cast<uint4*>(e->x) : nullptr, D / 8, S - 1 - row0))
+        return rc;
   }
-  // the residual stream of the last position is what xotb200_post_to_next hands to the next shard
-  CK(cudaMemcpyAsync(e->x, e->tc_x + (size_t)((n_tokens - 1) % e->tc_chunk) * D, (size_t)D * 2, cudaMemcpyDeviceToDevice, st));
   return 0;
 }
 

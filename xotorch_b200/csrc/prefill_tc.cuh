@@ -321,6 +321,17 @@ __global__ void tc_gather_kernel(const int* tokens, const bf16* embed, bf16* x, 
   for (int c = threadIdx.x; c < D / 8; c += blockDim.x) d4[c] = s4[c];
 }
 
+// the residual stream's rows (d8 pieces of 16 bytes) to `out` (may be NULL), row `last_row` to `last` as well (may be NULL)
+__global__ void tc_rows_out_kernel(const uint4* x, uint4* out, uint4* last, int d8, int last_row) {
+  pdl_enter();
+  const size_t at = (size_t)blockIdx.x * d8;
+  for (int c = threadIdx.x; c < d8; c += blockDim.x) {
+    const uint4 v = x[at + c];
+    if (out) out[at + c] = v;
+    if (last && (int)blockIdx.x == last_row) last[c] = v;
+  }
+}
+
 // lowest-index arg-max of logits[0..V) -> ctl->token   (single block of 1024 threads)
 __global__ void __launch_bounds__(1024) tc_argmax_kernel(const float* logits, int V, StepCtl* ctl) {
   pdl_enter();
