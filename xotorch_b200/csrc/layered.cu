@@ -923,14 +923,18 @@ static int product_tc(xotb200_lm* e, const bf16* A, long lda, long a_batch, cons
 }
 
 // 32-bit product of more rows than the decode kernel takes; 1 = launched, 0 = operands that are not whole 16-byte pieces
+// CTAs that share a tile by cutting K
+static int fma_splits(const xotb200_lm* e, long tiles, int K) {
+  int s = 1;
+  while (s < 8 && tiles * s * 2 <= 2L * e->sm_count && cdiv(K, FMA_BK) >= 4 * s) s *= 2;
+  return s;
+}
 template <int RM, int EPI>
 static int launch_fma(xotb200_lm* e, const float* A, long lda, long a_batch, const float* B, long ldb, long b_batch, float* C, long ldc, long c_batch, int M, int N, int K,
                       int batch, const EpiArgs& epi) {
   auto kern = gemm_fma_kernel<RM, EPI>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fma_smem_bytes(RM)));
-  const int n_tiles = cdiv(N, FMA_BN), tiles = n_tiles * cdiv(M, 8 * RM), nkb = cdiv(K, FMA_BK);
-  int s = 1;
-  while (s < 8 && (long)tiles * batch * s * 2 <= 2L * e->sm_count && nkb >= 4 * s) s *= 2;
+  const int n_tiles = cdiv(N, FMA_BN), tiles = n_tiles * cdiv(M, 8 * RM), s = fma_splits(e, (long)tiles * batch, K);
   return launch_early(e, kern, dim3(s, tiles, batch), FMA_THREADS, fma_smem_bytes(RM), s, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, n_tiles, epi);
 }
 template <int EPI>
@@ -938,10 +942,17 @@ static int product_fma(xotb200_lm* e, const float* A, long lda, long a_batch, co
                        int batch, const EpiArgs& epi) {
   if (((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) || (lda | ldb | K) % 4 || (batch > 1 && (a_batch | b_batch) % 4) || (long)cdiv(N, FMA_BN) * cdiv(M, 16) > 65535)
     return 0;
-  // rows per tile: the height that leaves the fewest empty rows in all, the taller one when equal (B is read once per row tile)
-  int best = 2;
-  for (int rm : {4, 6, 8, 10, 12})
-    if (cdiv(M, 8 * rm) * rm <= cdiv(M, 8 * best) * best) best = rm;
+  // rows per tile (8 rm): the height with the least time on the busiest SM, the taller one when about equal.  A K block takes a CTA as long as rm + 8 says (its loads and barriers are
+  // there for any height), and one alone on its SM, a warp to a scheduler, is no faster than two (85 rows, K = 4096, 1024 columns: heights of 96 rows on 16 x 8 CTAs 68 us, of 48 on
+  // 32 x 8 50; 5184 columns, K = 1024: 96 rows 53 us, 32 rows 84)
+  int best = 12;
+  double least = 0;
+  for (int rm : {12, 10, 8, 6, 4, 2}) {
+    const long tiles = (long)cdiv(N, FMA_BN) * cdiv(M, 8 * rm);
+    const int s = fma_splits(e, tiles * batch, K), per_sm = cdiv(tiles * batch * s, e->sm_count);
+    const double cost = (rm + 8.0) * cdiv(cdiv(K, FMA_BK), s) * std::max(1.6, (double)per_sm);
+    if (rm == 12 || cost < 0.95 * least) { best = rm; least = cost; }
+  }
   const int r = best == 2   ? launch_fma<2, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi)
                 : best == 4 ? launch_fma<4, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi)
                 : best == 6 ? launch_fma<6, EPI>(e, A, lda, a_batch, B, ldb, b_batch, C, ldc, c_batch, M, N, K, batch, epi)

@@ -102,10 +102,15 @@ gemm_fma_kernel(const float* __restrict__ A, long lda, long a_batch, const float
   float ap = 0.f, aq = 0.f;
   if (EPI == EPI_XIELU) { ap = softplusf_(static_cast<const float*>(epi.p)[0]); aq = 0.5f + softplusf_(static_cast<const float*>(epi.p)[1]); }
   const uint32_t part_addr = xb::smem_u32(part);
-  auto total = [&](int m, int c) {                             // sum of the cluster's partial tiles, in the order of K
+  auto total = [&](int m, int c) {                             // sum of the cluster's partial tiles, in the order of K: all loads under way before the first sum
     if (S == 1) return part[m * FMA_PLD + c];
-    float v = 0.f;
-    for (int r = 0; r < S; ++r) v += ld_dsmem_f32(part_addr + (uint32_t)(m * FMA_PLD + c) * 4, r);
+    float p[8], v = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < S) p[r] = ld_dsmem_f32(part_addr + (uint32_t)(m * FMA_PLD + c) * 4, r);
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      if (r < S) v += p[r];
     return v;
   };
   const int rows = min(BM, M - m0);
