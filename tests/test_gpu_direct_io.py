@@ -20,7 +20,7 @@ def shard(name, lo, hi, n):
   return e
 
 
-@pytest.mark.parametrize("name", ["tiny-llama-hd64", "tiny-llama-hd128-f16"])
+@pytest.mark.parametrize("name", ["tiny-llama-hd64", "tiny-llama-hd64-f16"])
 @pytest.mark.parametrize("n", [1, 3])
 def test_hidden_states_in_place(name, n):
   import torch
@@ -87,7 +87,7 @@ def test_logits_in_page_locked_and_ordinary_memory(name):
   e.close()
 
 
-@pytest.mark.parametrize("name", ["tiny-llama-hd64", "tiny-llama-hd128-f16"])
+@pytest.mark.parametrize("name", ["tiny-llama-hd64", "tiny-llama-hd64-f16"])
 @pytest.mark.parametrize("n", [2, 17, 128, 129, 300])
 def test_prompts_in_place(name, n):
   """prompts as GEMMs: rows on and off a 16-byte boundary, into another buffer and over the input; the next position after them (a shard's last row goes on)"""

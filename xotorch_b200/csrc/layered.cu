@@ -726,6 +726,10 @@ static const size_t GEMV_SMEM_MAX = 160 * 1024;
 // Rows up to which 16-bit products run on the one-warp-per-row-group kernel.  Beyond two rows its fp32 FMAs (8 per weight at 8
 // rows) fall behind the weight stream, and the tensor-core tiles — mostly empty, but they read each weight once — are faster.
 static const int GEMV_MAX_ROWS = 2;
+// ... and below this many weights, where a launch is over before the streams' copies are at full rate: long streams fill memory better (three layers and a head of 32000, one request, products
+// from here on streamed / none: width 4096 371 -> 330 us a step, 2048 198 -> 193.5, 1024 130.3 -> 129.8; two requests 468 -> 341, 237 -> 202.5, 148.8 -> 146.5; from 50 million
+// on only, width 4096 341 and 365; one request of another family, width 2048, from 15 / 6 million on 169.2 / 171.3).
+static long gemv_max_weights(int M) { return M == 1 ? 15000000 : 6000000; }
 
 template <typename K>
 static int opt_in_smem(K kernel, size_t bytes) {
@@ -969,7 +973,7 @@ static int product(xotb200_lm* e, const TA* A, long lda, long a_batch, const TB*
   const size_t smem = (size_t)M * K * 4;
   if constexpr (std::is_same<TA, bf16>::value && std::is_same<TB, bf16>::value && (EPI == EPI_NONE || EPI == EPI_CLOSE || !std::is_same<TC, float>::value)) {
     // 16-bit operands with more rows than the decode kernel takes: the tensor cores, when the operands can be described to TMA
-    if (sbk == 1 && (!epi_is_glu(EPI) || epi.il8) && ((e->gemm_mode == 0 && M > GEMV_MAX_ROWS) || e->gemm_mode == 2)) {
+    if (sbk == 1 && (!epi_is_glu(EPI) || epi.il8) && ((e->gemm_mode == 0 && (M > GEMV_MAX_ROWS || (long)N * K * batch >= gemv_max_weights(M))) || e->gemm_mode == 2)) {
       const int r = product_tc<TC, EPI>(e, A, lda, a_batch, B, sbn, b_batch, C, ldc, c_batch, M, N, K, batch, epi);
       if (r != 0) return r < 0 ? r : 0;
     }
