@@ -778,6 +778,14 @@ static int launch_tc_attn(xotb200_engine* e, int S, int R, bf16* kc, bf16* vc, i
   return launch_early(e, st, fn, dim3((S + 63) / 64, e->cfg.n_heads), 128, SMEM, late, e->tc_q, kc, vc, e->tc_ao, S, e->cfg.n_heads, R, e->L, pos0, scale_log2);
 }
 
+// memory of the engine's own GPU: what its kernels may touch whatever the caller has set up (another GPU's or the host's goes through a copy)
+static bool own_memory(const xotb200_engine* e, const void* p) {
+  cudaPointerAttributes at;
+  const bool own = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeDevice && at.device == e->device;
+  cudaGetLastError();
+  return own;
+}
+
 // Prefill n_tokens positions starting at pos0 on the tensor cores, in chunks of up to e->tc_chunk tokens (layer-major
 // inside a chunk, so a chunk streams the shard's weights once).  Inputs: stage_tokens /
 // stage_in or `in` (device memory); outputs: stage_out or `out` (non-last shard) or logits + ctl->token of the last position (last shard).
@@ -790,8 +798,9 @@ static int prefill_tc(xotb200_engine* e, int n_tokens, int pos0, cudaStream_t st
   const int qd = Hq * hd, nqkv = (Hq + 2 * Hkv) * hd, nl = e->end - e->start + 1;
   auto rmsnorm = c.dtype == XOTB200_DTYPE_F16 ? xb::fp::tc_rmsnorm_kernel : xb::bf::tc_rmsnorm_kernel;
   // The rows come in with the first norm and go out with one launch behind the last product: copies by the copy engine cost some 10 us around five launches a layer (two 8B
-  // layers, 6 positions 220 -> 209 us, 128 287 -> 281).  Rows off a 16-byte boundary are copied.
-  const bool in_place = (reinterpret_cast<uintptr_t>(hidden_in) & 15) == 0, out_place = (reinterpret_cast<uintptr_t>(hidden_out) & 15) == 0;
+  // layers, 6 positions 220 -> 209 us, 128 287 -> 281).  Rows off a 16-byte boundary or in other memory than this GPU's are copied.
+  auto direct = [&](const void* p, bool callers) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (!callers || own_memory(e, p)); };
+  const bool in_place = !e->first && direct(hidden_in, in != nullptr), out_place = !e->last && direct(hidden_out, out != nullptr);
   for (int m0 = 0; m0 < n_tokens; m0 += e->tc_chunk) {
     const int S = std::min(e->tc_chunk, n_tokens - m0);
     if (e->first) {
@@ -1533,7 +1542,7 @@ static DirectIo direct_io(const xotb200_engine* e, const int32_t* tokens, int n_
   if (in || (out && !e->last)) {
     const bool shifted = in && out && !e->last && ci != co && ci < co + bytes && co < ci + bytes;
     const uintptr_t at = reinterpret_cast<uintptr_t>(in) | (e->last ? 0 : reinterpret_cast<uintptr_t>(out));
-    if (!shifted && at % 16 == 0) {
+    if (!shifted && at % 16 == 0 && (!in || own_memory(e, in)) && (e->last || own_memory(e, out))) {
       io.in = in;
       io.out = e->last ? nullptr : out;
     }
