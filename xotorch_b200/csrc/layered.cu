@@ -206,7 +206,7 @@ struct xotb200_lm {
   float* trace_buf = nullptr;
   size_t trace_floats = 0, trace_cap = 0;
   int gemm_mode = 0;
-  bool early = false;                                  // this step's kernels may start before the one in front has finished (launch_early)
+  bool early = true;                                   // kernels may start before the one in front has finished (launch_early)
   bool staged = false;                                 // the next launch is the first behind the step's index arrays (launch_early)
   bool graphs_on = true;                               // decode steps are replayed from CUDA graphs
   std::map<std::array<long, 6>, GraphSlot> graphs;
@@ -764,10 +764,10 @@ static bool make_map3(CUtensorMap* m, const void* ptr, long rows, long K, long l
 }
 
 // Launches a kernel in clusters of `cluster` CTAs along x.  Weights are read before a kernel waits for the one in front (stream_gemm_kernel,
-// gemv_rows_kernel, the row norms), so none may be in the writing then: loading ends with a synchronisation.  In a step of few rows (e->early) it may start before the kernel in front of it has
-// finished: it waits itself (pdl_wait), its launch and what it loads ahead of that are hidden.  Such a step is a chain of some forty short
-// kernels, and the launches are most of it (one request, width 1024: 5979 -> 4913 us for 25 steps).  With many rows the kernels are long, and
-// blocks that were placed early, around a kernel still running, are spread worse over the SMs (1024 rows, width 4096: 2503 -> 2588 us).
+// gemv_rows_kernel, the row norms), so none may be in the writing then: loading ends with a synchronisation.  With e->early it may start before the kernel in front of it has
+// finished: it waits itself (pdl_wait), its launch and what it loads ahead of that are hidden.  A step is a chain of some forty kernels, and the launches are most of a short one (one request,
+// width 1024: 5979 -> 4913 us for 25 steps) and 30 to 50 us of a long one (three layers, prompts of 260 rows 577 -> 531 us, 600 764 -> 726, 1000 923 -> 878, 2500 1675 -> 1630).  Products of many
+// rows, whose blocks would be placed around a kernel still running and spread worse over the SMs, start the ordinary way (launch_late; gemm_fma_kernel).
 // The step's first kernel starts the ordinary way, behind a finished stage_in_kernel: whatever starts after it may read the staged index arrays ahead of its
 // wait (delta_row_kernel looks up the slot whose state it fetches), which an early start behind the staging kernel's last block would not order.
 template <typename... KA, typename... A>
@@ -2868,7 +2868,7 @@ int xotb200_lm_step(xotb200_lm* e, int n_seq, const int32_t* slots, const int32_
   if (e->first)
     for (long m = 0; m < M; ++m) REQUIRE(tokens[m] >= 0 && tokens[m] < V, "token id %d outside the vocabulary of %d", tokens[m], V);
   TRY(ensure_scratch(e, (int)M, n_want));
-  e->early = M <= LST_MAX_ROWS;
+  e->early = true;
   e->logits_out = logits_f32 != nullptr;
   TRY(refresh_tables(e));
   if (e->table_stale) {
