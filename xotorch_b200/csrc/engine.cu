@@ -198,6 +198,7 @@ struct xotb200_engine {
   int max_inflight = 0;            // decode producer window (bulk copies in flight per CTA, 0 = ring depth)
   unsigned int pace_q = 0;         // decode producer pacing, 2^-16 ns per byte per CTA (0 = off)
   bool tc_fuse = true;             // RoPE/KV-append and SwiGLU fused into GEMM epilogues (XOTB200_TC_FUSE=0: separate kernels, A/B)
+  int pair_cap = 0;                // slots in pair_ws
   float* pair_ws = nullptr;        // slots and flags of a prompt's GEMM tiles that are cut along K (prefill_tc.cuh); NULL: not needed yet, or no memory
   int* gemm_err = nullptr;         // page-locked word that a prompt's kernels write when a pipeline wait expires: read behind the call's own synchronisation, without a copy
   int prefill_mode = 0;            // 0 auto (runs_as_gemms), 1 always the decode kernel, 2 always TC
@@ -567,11 +568,26 @@ static int launch_tc_gemm_2sm(xotb200_engine* e, const CUtensorMap& tmA, const C
   }
   if (int rc = ensure_smem_attr(e->device, (const void*)fn, tc2_smem_bytes(NT, NS))) return rc;
   const int total = ((a.S + 2 * TC_M - 1) / (2 * TC_M)) * (a.N / NT), pairs = std::max(1, e->sm_count / 2);
-  a.split = PairSplit{};
-  if (e->pair_ws && NT == 256) {
-    a.split = pair_split(total, pairs, a.K / TC_BK);
-    a.split.ws = e->pair_ws;
-    a.split.flags = reinterpret_cast<int*>(e->pair_ws + (size_t)pair_slots(pairs) * PAIR_SLOT);
+  a.split = NT == 256 ? pair_split(total, pairs, a.K / TC_BK) : PairSplit{};
+  if (a.split.n[0] > 0) {
+    const int slots = a.split.n[0] * (a.split.s[0] - 1) + a.split.n[1] * (a.split.s[1] - 1);
+    if (slots > e->pair_cap) {           // as many as this product leaves; without memory for them its tiles stay whole
+      CK(cudaStreamSynchronize(st));
+      if (e->pair_ws) cudaFree(e->pair_ws);
+      e->pair_ws = nullptr;
+      e->pair_cap = 0;
+      if (cudaMalloc(&e->pair_ws, (size_t)slots * (PAIR_SLOT + PAIR_FLAGS) * 4) != cudaSuccess) { cudaGetLastError(); e->pair_ws = nullptr; }
+      else {
+        e->pair_cap = slots;
+        MEMSET_SYNC(e, e->pair_ws + (size_t)slots * PAIR_SLOT, 0, (size_t)slots * PAIR_FLAGS * 4);
+      }
+    }
+    if (e->pair_cap >= slots) {
+      a.split.ws = e->pair_ws;
+      a.split.flags = reinterpret_cast<int*>(e->pair_ws + (size_t)e->pair_cap * PAIR_SLOT);
+    } else {
+      a.split = PairSplit{};
+    }
   }
   return launch_early(e, st, fn, 2 * pair_count(total, pairs, a.split), TC2_THREADS, tc2_smem_bytes(NT, NS), 0, tmA, tmB_half, a);
 }
@@ -661,11 +677,6 @@ static int prepare_tc(xotb200_engine* e, int n_tokens) {
       rc = take();
     }
     if (rc) return rc;
-    if (need > 2 * TC_M && !e->pair_ws) {   // 29 MB; without them the tiles stay whole
-      const size_t slots = pair_slots(std::max(1, e->sm_count / 2)), floats = slots * PAIR_SLOT, flags = slots * PAIR_FLAGS;
-      if (cudaMalloc(&e->pair_ws, (floats + flags) * 4) != cudaSuccess) { cudaGetLastError(); e->pair_ws = nullptr; }
-      else MEMSET_SYNC(e, e->pair_ws + floats, 0, flags * 4);
-    }
     e->tc_cap = need;
     if (c.n_experts > 0) {
       const size_t rows = (size_t)2 * need + (size_t)c.n_experts * TC_M;
@@ -1482,8 +1493,7 @@ static int check_gemm_error(xotb200_engine* e) {
   const int err = *static_cast<volatile int*>(e->gemm_err);
   if (err == 0) return 0;
   *e->gemm_err = 0;
-  const size_t slots = pair_slots(std::max(1, e->sm_count / 2));
-  if (e->pair_ws) MEMSET_SYNC(e, e->pair_ws + slots * PAIR_SLOT, 0, slots * PAIR_FLAGS * 4);   // flags that nobody waited for any more
+  if (e->pair_ws) MEMSET_SYNC(e, e->pair_ws + (size_t)e->pair_cap * PAIR_SLOT, 0, (size_t)e->pair_cap * PAIR_FLAGS * 4);   // flags that nobody waited for any more
   set_err("tensor-core GEMM: a pipeline wait expired (device error %d)", err);
   return XOTB200_ETIMEOUT;
 }

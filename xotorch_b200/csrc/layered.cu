@@ -216,7 +216,8 @@ struct xotb200_lm {
   bool flash_on = true;                                // bf16: prompt portions of FLASH_MIN_ROWS rows or more use the expanded tensor-core attention
   std::vector<int> stage_build;
   int64_t launches = 0, tc_launches = 0, flash_launches = 0;
-  float* pair_ws = nullptr;                            // slots and flags of the products' tiles that are cut along K (layered_tc.cuh); NULL: not needed yet, or no memory
+  float* pair_ws = nullptr;                            // slots and flags of the products' tiles that are cut along K (pair_room); NULL: not needed yet, or no memory
+  bool pair_refused = false;
   int* d_err = nullptr;                                // sticky device error word (3 = a bounded wait of a tensor-core product expired)
   int* h_err = nullptr;                                // pinned copy, read after every step
   bool timed = false;                                  // ev0 and ev1 bracket the newest step, not yet read
@@ -881,16 +882,31 @@ static int product_stream(xotb200_lm* e, const bf16* A, long lda, long a_batch, 
 }
 
 // Pairs of CTAs on 256 x 256 tiles, where they pay (pairs_pay).
-// The slots of tiles that are cut along K (PairWalk).  The second mixer of a layer runs beside the first, which may use them: its tiles stay whole.
-static bool pair_room(const xotb200_lm* e) { return e->pair_ws && e->stream != e->side; }
+// The slots of tiles that are cut along K (PairWalk), 29 MB, made when a product first needs them.  False, and the tiles stay whole: no memory; the second mixer of a layer, which runs beside the
+// first, which may use them; a step that is being captured (its products have run once before that).
+static bool pair_room(xotb200_lm* e) {
+  if (e->stream == e->side || e->pair_refused) return false;
+  if (e->pair_ws) return true;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(e->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) { cudaGetLastError(); return false; }
+  const size_t slots = xb::pair_slots(std::max(1, e->sm_count / 2)), floats = slots * xb::PAIR_SLOT, flags = slots * xb::PAIR_FLAGS;
+  if (cudaMalloc(&e->pair_ws, (floats + flags) * 4) != cudaSuccess || cudaMemsetAsync(e->pair_ws + floats, 0, flags * 4, e->stream) != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(e->pair_ws);
+    e->pair_ws = nullptr;
+    e->pair_refused = true;
+  }
+  return e->pair_ws != nullptr;
+}
 template <int EPI, typename TC>
 static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& mb, const LtcArgs& a) {
   auto kern = ltc_pair_kernel<EPI, TC>;
   CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LTP_SMEM));
   const int tiles = cdiv(a.M, 2 * LTC_M) * cdiv(a.N, LTP_N), pairs = std::max(1, e->sm_count / 2);
   LtcArgs b = a;
-  if (pair_room(e)) {
-    b.split = xb::pair_split(tiles, pairs, cdiv(a.K, LTC_BK));
+  const xb::PairSplit cut = xb::pair_split(tiles, pairs, cdiv(a.K, LTC_BK));
+  if (cut.n[0] > 0 && pair_room(e)) {
+    b.split = cut;
     b.split.ws = e->pair_ws;
     b.split.flags = reinterpret_cast<int*>(e->pair_ws + (size_t)xb::pair_slots(pairs) * xb::PAIR_SLOT);
   }
@@ -901,10 +917,12 @@ static int launch_pair(xotb200_lm* e, const CUtensorMap& ma, const CUtensorMap& 
 // Pairs where their tiles, empty rows and columns included, keep 60 % of the waves' slots busy: a pair's tile runs about twice as fast as its share of 128 x 128 tiles
 // (layered_tc.cuh), which lose less in the last wave.  1024 rows, 128 x 128 tiles / pairs: 6144 columns with K = 1536 (65 %) 33 / 28 us, 6720 with 4096 (71 %) 70 / 55, 2144 with
 // 4096 (45 %) 29 / 33.  K < 512: filling the ring is most of a tile.
-static bool pairs_pay(const xotb200_lm* e, int M, int N, int K) {
+static bool pairs_pay(xotb200_lm* e, int M, int N, int K) {
   const int tiles = cdiv(M, 2 * LTC_M) * cdiv(N, LTP_N), pairs = std::max(1, e->sm_count / 2);
-  const double waves = pair_room(e) ? xb::pair_waves(tiles, pairs, cdiv(K, LTC_BK)) : cdiv(tiles, pairs);
-  return K >= 512 && (double)M * N >= 0.6 * waves * pairs * (2.0 * LTC_M * LTP_N);
+  auto pays = [&](double waves) { return (double)M * N >= 0.6 * waves * pairs * (2.0 * LTC_M * LTP_N); };
+  if (K < 512) return false;
+  const double cut = xb::pair_waves(tiles, pairs, cdiv(K, LTC_BK));
+  return pays(cdiv(tiles, pairs)) || (pays(cut) && pair_room(e));
 }
 
 // 1 = launched, 0 = not eligible (the caller falls back), < 0 = error
@@ -1100,11 +1118,6 @@ static int ensure_scratch(xotb200_lm* e, int M, int n_want) {
     if (e->pre_scalar) TRY(regrow(e->oh2, m * e->max_oh * z));
     TRY(regrow(e->act, m * e->max_ff * z));
     TRY(regrow(e->th, m * e->max_lr * z));
-    if (z == 2 && M > LST_MAX_ROWS && !e->pair_ws) {   // 29 MB; without them the tiles stay whole
-      const size_t slots = xb::pair_slots(std::max(1, e->sm_count / 2)), floats = slots * xb::PAIR_SLOT, flags = slots * xb::PAIR_FLAGS;
-      if (cudaMalloc(&e->pair_ws, (floats + flags) * 4) != cudaSuccess) { cudaGetLastError(); e->pair_ws = nullptr; }
-      else CK(cudaMemsetAsync(e->pair_ws + floats, 0, flags * 4, e->stream));
-    }
     e->m_cap = (int)m;
     e->trace_cap = 0;
   }
